@@ -5,7 +5,8 @@
 // Routing on sm_100a:
 //   n <= kGemvMaxN (or k == 0)                          -> streaming split-k GEMV (gemv.cu) when it takes the operand types
 //   NVFP4 x NVFP4, E4M3 scales on both                  -> tcgen05 kind::mxf4nvf4 block-scaled GEMM (gemm_w4a4.cu)
-//   NVFP4 (E4M3 scales) x BF16                          -> tcgen05 kind::f16 GEMM on weights expanded to exact BF16 (gemm_w4a16.cu)
+//   NVFP4 x BF16                                        -> tcgen05 kind::f16 GEMM on weights expanded to exact BF16 (gemm_w4a16.cu)
+//   NVFP4 (E4M3 scales) x FP16, 16-bit D, any n         -> the same kernel on weights expanded to exact FP16
 //   anything else                                       -> exact CUDA-core GEMM (gemm_generic.cu)
 #include <stdio.h>
 #include <stdlib.h>
@@ -123,7 +124,7 @@ static nvfp4a_status dispatch(const char *fn, const GemmArgs &g, cudaStream_t st
   else if (gemv && gemv_supports(g)) { g_last_route = 2; err = launch_gemv(g, stream); }
   else if (gemv && g.k > 0 && gemv_blocked_supports(g)) { g_last_route = 6; err = launch_gemv_blocked(g, stream); }
   else if (!gemv && gemm_w4a4_supports(g)) { g_last_route = 4; err = launch_gemm_w4a4(g, stream); }
-  else if (!gemv && gemm_w4a16_supports(g)) { g_last_route = 5; err = launch_gemm_w4a16(g, stream); }
+  else if ((!gemv || g.B.dtype == NVFP4A_FP16) && gemm_w4a16_supports(g)) { g_last_route = 5; err = launch_gemm_w4a16(g, stream); }
   else if (!gemv && forced_route() != 3 && gemm_w4a8_tc_supports(g)) { g_last_route = 8; err = launch_gemm_w4a8_tc(g, stream); }
   else if (!gemv && gemm_dp4a_supports(g)) { g_last_route = 7; err = launch_gemm_dp4a(g, stream); }
   else { g_last_route = 1; err = launch_gemm_generic(g, stream); }

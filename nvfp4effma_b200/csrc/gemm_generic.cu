@@ -4,7 +4,7 @@
 // per MAC, k ascending.  Outputs are therefore bit-identical to the reference's tiled CUDA-core kernels.
 //
 // This is the library's correctness anchor and the route for operand formats that have no tensor-core form on sm_100a
-// (UE5M3 block scales, FP32 / FP16 activations, INT8 activations with FP32 block scales).  It carries the plain and the
+// (UE5M3 block scales, FP32 activations, FP16 activations with an FP32 D, INT8 activations with FP32 block scales).  It carries the plain and the
 // extended epilogue.  One CTA computes a 16-row slice x 16 columns; it is not a fast path.
 #include "operands.cuh"
 

@@ -5,25 +5,43 @@
 // cores then form exact products with the BF16 activations and accumulate in FP32 -- the reference's "exact" W4A16
 // definition (include/nvfp4effma.h:82-92 there) up to the order of the FP32 additions, like its own tensor-core path.
 //
-// Tile: 128 weight rows (MMA M) x BN tokens (MMA N) x 64 values of k per stage; a stage in shared memory is
-// [A 128 rows x 128 B | B BN rows x 128 B], both K-major with the 128-byte swizzle.
-//   warp 0      TMA producer of the activation tiles (2-D tensor map over B, no multicast)
-//   warp 1      MMA issuer (4 x K16 per stage), owner of the tensor memory: 2 accumulators of BN columns
-//   warps 2-5   epilogue, one 32-lane quadrant each: plain or extended (RMSNorm column scale, SwiGLU, second output + sums
-//               of squares), D through a shared-memory staging tile and TMA stores when its layout allows
-//   warps 6-13  weight expansion, two groups of four warps on alternate stages: each thread owns a row of its stage (64
-//               nibbles + 4 scale bytes, fetched from global memory ahead of use), decodes them with shifts and masks to BF16 pairs (value * 2^-126, the
-//               subnormal trick), multiplies by the block scale in BF16 (exact) and stores 64 bytes into the swizzled
-//               A tile.  To keep scale * 2^126 inside BF16, weights are carried as a * sa * 2^-Z (Z = 8 for E4M3, 16 for
-//               UE5M3 scales) and the accumulator is multiplied by 2^Z in the epilogue.
+// CTA pairs (tcgen05.mma.cta_group::2): a tile is 256 weight rows (MMA M, 128 per CTA) x up to 256 tokens (MMA N, half of them in
+// each CTA's shared memory), a stage covers 64 values of k.  The expanded weights are the MMA's A operand IN TENSOR MEMORY: an
+// expansion thread owns a weight row = a tensor memory lane and writes its 64 values with two tcgen05.st, so that the expansion costs
+// no shared-memory traffic, no swizzled addressing and no proxy fence, and shared memory is left to the activations (read once per
+// pair and stage).  Tensor memory: columns [0, 256) one accumulator of 256 columns or two of 128, [256, 512) eight weight stages.
+// Roles, 20 warps per CTA:
+//   warp 0      TMA producer of the activations: this CTA's half of the tile's tokens (no multicast); the bytes of both CTAs are
+//               counted on the even CTA's barrier
+//   warp 1      MMA issuer (even CTA; 4 x K16 per stage, one elected lane), owner of the tensor memory
+//   warp 2      TMA producer of the weight nibbles: [128 rows][128 bytes] = 256 values of k per slot, so that the expansion
+//               reads shared memory and never waits for a trip to L2
+//   warps 4-11  epilogue (160 registers each, taken from the others by setmaxnreg), one 32-lane quadrant and one half of the columns
+//               each: the accumulator block goes into registers at once and back to the MMA warp before any arithmetic; then
+//               plain or extended epilogue (RMSNorm column scale, SwiGLU, second output + sums of squares), D through
+//               shared-memory staging tiles and TMA stores when its layout allows
+//   warps 12-19 weight expansion, two groups of four warps on alternate stages.  The eight magnitudes of E2M1 times a block scale
+//               are eight 16-bit floats (exact: 2 x 4 significant bits); a 4 KiB table holds their high and low bytes for each of
+//               the 256 scale codes, so a block costs one 16-byte table read and four values cost three byte permutes (the packed
+//               nibbles ARE the permute's selectors: high bytes, low bytes, signs), two of them again to interleave, and two
+//               logical operations -- 2 instructions per value where shifts, masks, the multiply and reordering took 3.
+// Instruction issue, not the tensor pipe, bounded the former kernel (a thread-per-row expansion through shared memory with a proxy
+// fence per stage: 1240 cycles per stage of 512 cycles of MMAs, 41 % of the tensor pipe).
+// The last round of tiles over the SM pairs is cut along the tokens when it would leave pairs idle, and a tile at the end of the
+// tokens is only as wide (in steps of 64) as the tokens left.
 // Every wait is bounded; a wait that gives up raises the CTA's abort flag and the kernel status word.
+//
+// FP16 activations (F16): e2m1 x E4M3 is a multiple of 2^-10 up to 2880 with at most 6 significant bits, exact in FP16, so the same
+// kernel runs on FP16 operands.
+//
+// Grouped (mixture of experts): A stacks the weights of all groups, a group owns the tokens [seg[q], seg[q + 1]); the CTAs read seg
+// (device memory) into a table of tile counts and find a tile's group there.
 //
 // INT8 activations (W4A8, FP32 scale per 16 values) run on the same kernel with PLANES = 3: an activation is the FP32 value
 // x = q * s_b (one rounding: within the accumulation bound of the exact definition, not bit-identical to the integer block sums
 // of the DP4A kernels), split exactly into three BF16 terms x = t1 + t2 + t3 (8 + 8 + 8 significant bits) by a small kernel
-// that runs first.  The terms lie side by side as [token][3][k]; a stage then holds one expanded weight tile and the three
-// activation tiles of its 64 values of k, and the MMA issuer accumulates weight x t1, weight x t2, weight x t3 into the same
-// accumulator -- three times the tensor-core work per expanded weight tile, which is what this kernel otherwise lacks.
+// that runs first.  The terms lie side by side as [token][3][k]; the activation ring holds one plane of a stage per slot, and the
+// MMA issuer accumulates weight x t1, weight x t2, weight x t3 from one expanded weight tile into the same accumulator.
 #include <atomic>
 #include <cuda_bf16.h>
 #include "operands.cuh"
@@ -42,7 +60,11 @@ struct W4A16Args {
   EpilogueEx x;
   unsigned *status;
   unsigned tag;  // this launch's tag in the status word
-  int d_tma;     // the output goes through the staging tile and TMA stores (SwiGLU: 64 output rows per tile)
+  int d_tma;     // the output goes through the staging tiles and TMA stores (SwiGLU: 64 output rows per tile)
+  int width;     // tokens per tile: 64, 128 or 256
+  int nfull, cut;   // tiles 0 .. nfull - 1 are `width` tokens wide; the rest (to `tiles`) are parts of width / cut tokens
+  int tiles;
+  const int *seg; int groups;   // GROUPED: m is the rows of ONE group's weight, n the bound on seg[groups]
 };
 
 // tensor maps of D in the peers' buffers (tensor-parallel all-gather fused into the epilogue's TMA stores); n = 0: none
@@ -51,95 +73,115 @@ struct alignas(64) PeerMaps {
   int n;
 };
 
-template <int BN, int PLANES = 1>
+template <int PLANES>
 struct Cfg {
-  static constexpr int kStages = PLANES == 3 ? 3 : BN == 256 ? 4 : 6;
-  static constexpr int kABytes = 128 * 128, kPlaneBytes = BN * 128, kBBytes = PLANES * kPlaneBytes, kStageBytes = kABytes + kBBytes;
-  static constexpr int kStagingBytes = 8192;
-  static constexpr int kSmemBytes = 1024 + kStages * kStageBytes + kStagingBytes + 1024 /* scale table */ + BN * 4 /* column scales */ + 256;
+  // PLANES = 1: the weight and the activation ring advance together and share their `empty` barriers (one commit per stage)
+  static constexpr int kA = 8, kB = 8, kRaw = 2;
+  static constexpr int kBBytes = 128 * 128, kRawBytes = 128 * 128, kStagingBytes = 8192;
+  static constexpr int kSmemBytes = 1024 + kB * kBBytes + kRaw * kRawBytes + 4 * kStagingBytes + 4096 /* expansion table */ + 256 * 4 /* column scales */ +
+                                    512 /* barriers */ + 2 * 257 * 4 + 8 /* groups */;
 };
+static_assert(Cfg<1>::kSmemBytes <= 232448, "shared memory budget");
+constexpr int kACols = 256;   // first tensor memory column of the weight stages (32 columns each)
 
-constexpr int kThreads = 448, kConvWarps = 8;
+constexpr int kThreads = 640, kRegsRest = 40, kRegsEpi = 160, kRegsConv = 56;
+static_assert(128 * kRegsRest + 256 * kRegsEpi + 256 * kRegsConv <= kThreads * 96, "the split draws on the registers of the launch: 96 per thread");
 constexpr unsigned kStWaitFullA = 0x301, kStWaitFullB = 0x302, kStWaitEmpty = 0x303, kStWaitTmemFull = 0x304, kStWaitTmemEmpty = 0x305,
-                   kStWaitConv = 0x306;
+                   kStWaitConv = 0x306, kStWaitRaw = 0x307;
 
-__device__ __forceinline__ uint32_t bf16x2_mul(uint32_t a, uint32_t b) {
-  uint32_t d;
-  asm("mul.rn.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
-  return d;
-}
 __device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t sel) {
   uint32_t d;
   asm("prmt.b32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(sel));
   return d;
 }
-// nibbles p and p + 4 of w -> BF16 pair (low half: nibble p), each value * 2^-126: magnitude bits to [6, 9), sign to 15
-template <int P>
-__device__ __forceinline__ uint32_t decode_pair(uint32_t w) {
-  const uint32_t mag = (P < 2 ? w << (6 - 4 * P) : w >> (4 * P - 6)) & 0x01C001C0u;
-  const uint32_t sgn = (w << (12 - 4 * P)) & 0x80008000u;
-  return mag | sgn;
+// Four nibbles (the low 16 bits of w) of a block -> four 16-bit floats in two registers, value 0 in the low half of the first.  `t` holds
+// the block's eight products: high bytes in x (codes 0-3) and y (4-7), low bytes in z and w.  A permute's selector nibble picks a byte with
+// its low three bits; with its top bit set -- here the sign -- it gives that byte's sign replicated instead: 0x80 becomes 0xFF, so
+// that bit 6 of each byte of `s` is the value's sign.
+__device__ __forceinline__ void expand4(uint32_t w, const uint4 &t, uint32_t &o0, uint32_t &o1) {
+  const uint32_t sel = w & 0x7777u;
+  const uint32_t s = prmt(0x80808080u, 0x80808080u, w);
+  const uint32_t hi = prmt(t.x, t.y, sel) | ((s << 1) & 0x80808080u), lo = prmt(t.z, t.w, sel);
+  o0 = prmt(lo, hi, 0x5140u);
+  o1 = prmt(lo, hi, 0x7362u);
 }
 
-// four MMAs of K = 16 over one 128-byte-row stage without a commit (elected lane of a converged warp): the first and second
-// activation plane of a stage; the third goes through mma4_f16_commit_elect
-__device__ __forceinline__ void mma4_f16_elect(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+// one stage's four MMAs (K = 16 each: 8 tensor memory columns of A, 32 bytes along B's 128-byte rows) over a CTA pair and the commit that hands the activation slot
+// back in both CTAs, in one statement issued by one elected lane of a converged warp
+__device__ __forceinline__ void mma4_f16_commit_pair_elect(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate,
+                                                           uint64_t *bar) {
   asm volatile("{\n\t.reg .pred p, q, t;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.eq.u32 t, %3, %3;\n\telect.sync _|q, 0xFFFFFFFF;\n\t"
-               "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t"
-               "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %5, %6, %3, t;\n\t"
-               "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %7, %8, %3, t;\n\t"
-               "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %9, %10, %3, t;\n\t}"
-               ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "l"(a_desc + 2), "l"(b_desc + 2), "l"(a_desc + 4), "l"(b_desc + 4),
-                 "l"(a_desc + 6), "l"(b_desc + 6) : "memory");
+               "@q tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n\t"
+               "@q tcgen05.mma.cta_group::2.kind::f16 [%0], [%5], %6, %3, t;\n\t"
+               "@q tcgen05.mma.cta_group::2.kind::f16 [%0], [%7], %8, %3, t;\n\t"
+               "@q tcgen05.mma.cta_group::2.kind::f16 [%0], [%9], %10, %3, t;\n\t"
+               "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%11], %12;\n\t}"
+               ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(a_tmem + 8), "l"(b_desc + 2), "r"(a_tmem + 16), "l"(b_desc + 4),
+                 "r"(a_tmem + 24), "l"(b_desc + 6), "r"(smem_u32(bar)), "h"((uint16_t)3) : "memory");
 }
 
-// what a conversion thread fetches for one stage: the 64 nibbles and 4 scale bytes of its row
-struct RawRow {
-  uint4 w0, w1;
-  uint32_t sc;
-};
+// A tile of the schedule: 128-row tiles 2 * tm and 2 * tm + 1 (one per CTA of the pair) against the tokens [j0, j0 + width), of which
+// those below jend exist (width: a multiple of 64; 0: nothing to do).  Grouped: ro = the group's first row in the stacked weights.
+struct Tile { int tm, j0, jend, width, ro; };
+constexpr int kMaxGroups = 256;
 
-template <int BN, int PLANES>
+template <int PLANES, bool F16, bool GROUPED>
 __global__ void __launch_bounds__(kThreads, 1)
-gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_constant__ CUtensorMap tmap_d, const __grid_constant__ PeerMaps peers,
-                  const W4A16Args g) {
-  using C = Cfg<BN, PLANES>;
-  constexpr int kStages = C::kStages;
+gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_b, const __grid_constant__ CUtensorMap tmap_d,
+                  const __grid_constant__ PeerMaps peers, const W4A16Args g) {
+  using C = Cfg<PLANES>;
+  constexpr int kA = C::kA, kB = C::kB, kRaw = C::kRaw;
   extern __shared__ uint8_t smem_raw[];
   uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-  uint8_t *staging = smem + kStages * C::kStageBytes;
-  uint32_t *lut = (uint32_t *)(staging + C::kStagingBytes);      // scale code -> BF16 pair (sa * 2^(126 - Z), twice)
+  uint8_t *const sB = smem, *const sRaw = sB + kB * C::kBBytes, *const staging = sRaw + kRaw * C::kRawBytes;
+  uint4 *lut = (uint4 *)(staging + 4 * C::kStagingBytes);           // scale code -> bytes of the eight products (see expand4)
   float *colscale = (float *)(lut + 256);                           // RMSNorm column scales of the current token tile
-  uint64_t *bars = (uint64_t *)(colscale + BN);
-  uint64_t *full = bars, *empty = bars + kStages, *tmem_full = bars + 2 * kStages, *tmem_empty = tmem_full + 2;
+  uint64_t *bars = (uint64_t *)(colscale + 256);
+  uint64_t *a_full = bars, *b_full = a_full + kA, *b_empty = b_full + kB, *a_empty = PLANES == 1 ? b_empty : b_empty + kB,
+           *raw_full = b_empty + kB + kA, *raw_empty = raw_full + kRaw, *tmem_full = raw_empty + kRaw, *tmem_empty = tmem_full + 2;
   uint32_t *tmem_slot = (uint32_t *)(tmem_empty + 2);
   volatile int *abort_flag = (volatile int *)(tmem_slot + 1);
+  int *gseg = (int *)((uint8_t *)bars + 512), *gcum = gseg + kMaxGroups + 1;   // GROUPED: seg, and the token tiles of the groups before each
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int rank = (int)cluster_ctarank();
   const int gm = g.m, gn = g.n, gk = g.k;
-  const int tiles_m = (gm + 127) / 128, tiles_n = (gn + BN - 1) / BN, ntiles = tiles_m * tiles_n;
-  const int nk = gk / 64;
+  const int tiles_m = (gm + 255) / 256, nk = gk / 64, nslots = (nk + 3) / 4;   // 256-row tiles
+  const int tile_first = blockIdx.x >> 1, tile_step = gridDim.x >> 1;
   const bool ue = g.A.ue != 0;
   unsigned *const status_word = g.status;
 
+  // The set-up touches no global memory: under programmatic dependent launch it runs while the stream's previous kernel drains.
+  pdl_launch_dependents();
   if (threadIdx.x == 0) {
-    // one `full` barrier per stage: the four conversion warps of the stage's group and the producer's expect-tx arrival
-    for (int s = 0; s < kStages; ++s) { mbar_init(&full[s], kConvWarps / 2 + 1); mbar_init(&empty[s], 1); }
-    for (int a = 0; a < 2; ++a) { mbar_init(&tmem_full[a], 1); mbar_init(&tmem_empty[a], 4); }
+    for (int s = 0; s < kA; ++s) mbar_init(&a_full[s], 8);   // the stage's four expansion warps of both CTAs
+    if (PLANES != 1) for (int s = 0; s < kA; ++s) mbar_init(&a_empty[s], 1);
+    for (int s = 0; s < kB; ++s) { mbar_init(&b_full[s], 1); mbar_init(&b_empty[s], 1); }
+    for (int s = 0; s < kRaw; ++s) { mbar_init(&raw_full[s], 1); mbar_init(&raw_empty[s], 8); }
+    for (int a = 0; a < 2; ++a) { mbar_init(&tmem_full[a], 1); mbar_init(&tmem_empty[a], 16); }
     *abort_flag = 0;
     fence_barrier_init();
+    prefetch_tensormap(&tmap_w);
     prefetch_tensormap(&tmap_b);
   }
   if (threadIdx.x < 256) {
-    const float s = scale_to_f32((uint32_t)threadIdx.x, ue) * (ue ? 0x1p110f : 0x1p118f);  // exact: 4 significant bits
-    const uint32_t h = __float_as_uint(s) >> 16;
-    lut[threadIdx.x] = h | (h << 16);
+    const float sc = scale_to_f32((uint32_t)threadIdx.x, ue);
+    uint32_t hi[2] = {0, 0}, lo[2] = {0, 0};
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+      const float v = __fmul_rn(e2m1_to_f32(c), sc);   // exact in 16 bits
+      const uint32_t h = F16 ? (uint32_t)__half_as_ushort(__float2half_rn(v)) : __float_as_uint(v) >> 16;
+      hi[c >> 2] |= (h >> 8) << (8 * (c & 3));
+      lo[c >> 2] |= (h & 0xFFu) << (8 * (c & 3));
+    }
+    lut[threadIdx.x] = make_uint4(hi[0], hi[1], lo[0], lo[1]);
   }
-  if (warp == 1) tmem_alloc(tmem_slot, 512);
+  if (warp == 1) tmem_alloc_pair(tmem_slot, 512);
   tc_fence_before();
-  __syncthreads();
+  cluster_sync_all();   // the peer's barriers are initialised before anything arrives on them
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_wait();   // from here on the previous kernel has completed and its writes are visible
 
   const unsigned tag = g.tag;
   auto wait = [abort_flag, status_word, tag](uint64_t *bar, uint32_t parity, unsigned code) -> bool {
@@ -150,120 +192,182 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_const
     atomicCAS(status_word, 0u, code | tag);
     return false;
   };
-
-  if (warp == 0) {
-    // ---------------- producer: activation tiles ----------------
-    // (the whole warp runs the loop, one elected lane issues: see tma_load_2d_elect)
-    uint32_t it = 0;
-    for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
-      const int tn = t / tiles_m;
-      for (int ks = 0; ks < nk; ++ks, ++it) {
-        const int s = it % kStages;
-        if (!__all_sync(0xFFFFFFFFu, wait(&empty[s], ((it / kStages) & 1) ^ 1, kStWaitEmpty))) goto done;
-        mbar_arrive_expect_tx_elect(&full[s], C::kBBytes);
+  const int W = g.width, nfull = g.nfull, cut = g.cut;
+  int ntiles = g.tiles;
+  if (GROUPED) {   // token tiles per group, then their running sum; a group whose rows are not inside [0, n) has none
+    const int groups = g.groups;
+    for (int q = threadIdx.x; q <= groups; q += kThreads) gseg[q] = g.seg[q];
+    __syncthreads();
+    if (warp == 0) {
+      int base = 0;
+      for (int q0 = 0; q0 < groups; q0 += 32) {
+        const int q = q0 + lane;
+        const int lo = q < groups ? gseg[q] : 0, hi = q < groups ? gseg[q + 1] : 0;
+        int v = (lo >= 0 && hi > lo && hi <= gn) ? (hi - lo + W - 1) / W : 0;
 #pragma unroll
-        for (int p = 0; p < PLANES; ++p)   // plane p of a token's row starts 2 k bytes after plane p - 1
-          tma_load_2d_elect(smem_u32(smem + (size_t)s * C::kStageBytes + C::kABytes + p * C::kPlaneBytes), &tmap_b, p * 2 * gk + ks * 128, tn * BN,
-                            smem_u32(&full[s]));
+        for (int o = 1; o < 32; o <<= 1) { const int u = __shfl_up_sync(0xFFFFFFFFu, v, o); if (lane >= o) v += u; }
+        if (q < groups) gcum[q + 1] = base + v;
+        base += __shfl_sync(0xFFFFFFFFu, v, 31);
+      }
+      if (lane == 0) gcum[0] = 0;
+    }
+    __syncthreads();
+    ntiles = gcum[groups] * tiles_m;
+  }
+  auto tile_of = [=](int t) -> Tile {
+    if (GROUPED) {
+      const int tt = t / tiles_m;
+      int q = 0, hi = g.groups;   // the last q with gcum[q] <= tt (the group holding token tile tt has gcum[q + 1] > tt)
+      while (hi - q > 1) { const int mid = (q + hi) >> 1; if (gcum[mid] <= tt) q = mid; else hi = mid; }
+      const int j0 = gseg[q] + (tt - gcum[q]) * W, left = gseg[q + 1] - j0;
+      return Tile{t % tiles_m, j0, gseg[q + 1], left < W ? (left + 63) & ~63 : W, q * gm};
+    }
+    int w = W, part = 0;
+    if (t >= nfull) { w = W / cut; part = (t - nfull) % cut; t = nfull + (t - nfull) / cut; }
+    const int j0 = t / tiles_m * W + part * w, left = gn - j0;
+    return Tile{t % tiles_m, j0, gn, left <= 0 ? 0 : left < w ? (left + 63) & ~63 : w, 0};
+  };
+  // accumulators: two of 128 columns while tiles are that narrow, else one of 256
+  const int nacc = W > 128 ? 1 : 2;
+
+  if (warp < 4) {
+  asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsRest));
+  if (warp == 0) {
+    // ---------------- producer: this CTA's half of the tile's tokens, one plane of one stage per slot ----------------
+    // (the whole warp runs the loop, one elected lane issues: see tma_load_3d_pair_elect)
+    const uint32_t stage_bytes = 2u * (uint32_t)(W / 2) * 128u;   // a box is always W / 2 rows per CTA, however many of them the tile uses
+    uint32_t it = 0;
+    for (int t = tile_first; t < ntiles; t += tile_step) {
+      const Tile p = tile_of(t);
+      if (p.width == 0) continue;
+      const int row0 = p.j0 + rank * (p.width >> 1);
+      for (int ks = 0; ks < nk; ++ks) {
+#pragma unroll
+        for (int pl = 0; pl < PLANES; ++pl, ++it) {   // plane pl of a token's row starts 2 k bytes after plane pl - 1
+          const int s = it % kB;
+          if (!__all_sync(0xFFFFFFFFu, wait(&b_empty[s], ((it / kB) & 1) ^ 1, kStWaitEmpty))) goto done;
+          if (rank == 0) mbar_arrive_expect_tx_elect(&b_full[s], stage_bytes);
+          tma_load_3d_pair_elect(smem_u32(sB + (size_t)s * C::kBBytes), &tmap_b, pl * 2 * gk + ks * 128, row0, 0, mbar_addr_rank(&b_full[s], 0));
+        }
       }
     }
   } else if (warp == 1) {
-    // ---------------- MMA issuer ----------------
-    // The whole warp runs the loop and one elected lane issues a stage's four MMAs (K = 16 each: 32 bytes along the row) and the
-    // commit in one statement; from inside a one-lane branch every tcgen05.mma costs ~150 cycles, more than the 128 the tensor
-    // pipe needs for 128 x 256 x 16.
-    constexpr uint32_t idesc = idesc_f16(128, BN, 1);
-    const uint64_t da0 = smem_desc_sw128(smem_u32(smem));
-    uint32_t it = 0, tile_i = 0;
-    for (int t = blockIdx.x; t < ntiles; t += gridDim.x, ++tile_i) {
-      const int acc = tile_i & 1;
-      if (!__all_sync(0xFFFFFFFFu, wait(&tmem_empty[acc], ((tile_i >> 1) & 1) ^ 1, kStWaitTmemEmpty))) goto done;
-      tc_fence_after();
-      const uint32_t d_tmem = tmem_base + acc * BN;
-      for (int ks = 0; ks < nk; ++ks, ++it) {
-        const int s = it % kStages;
-        if (!__all_sync(0xFFFFFFFFu, wait(&full[s], (it / kStages) & 1, kStWaitFullA))) goto done;
+    // ---------------- MMA issuer (even CTA) ----------------
+    // The whole warp runs the loop and one elected lane issues a stage's four MMAs and the commit in one statement; from inside a
+    // one-lane branch every tcgen05.mma costs ~150 cycles, more than the 128 the tensor pipe needs for 256 x 256 x 16 on a pair.
+    if (rank == 0) {
+      const uint64_t db0 = smem_desc_sw128(smem_u32(sB));
+      uint32_t ia = 0, ib = 0, tile_i = 0;
+      for (int t = tile_first; t < ntiles; t += tile_step) {
+        const Tile p = tile_of(t);
+        if (p.width == 0) continue;
+        const int acc = nacc == 2 ? tile_i & 1 : 0;
+        const uint32_t idesc = idesc_f16(256, p.width, F16 ? 0 : 1), acc_par = (nacc == 2 ? tile_i >> 1 : tile_i) & 1;
+        if (!__all_sync(0xFFFFFFFFu, wait(&tmem_empty[acc], acc_par ^ 1, kStWaitTmemEmpty))) goto done;
         tc_fence_after();
-        const uint64_t da = da0 + (uint32_t)s * (uint32_t)(C::kStageBytes >> 4), db = da + (C::kABytes >> 4);
-        if (PLANES == 3) {
-          mma4_f16_elect(d_tmem, da, db, idesc, (uint32_t)(ks != 0));
-          mma4_f16_elect(d_tmem, da, db + (C::kPlaneBytes >> 4), idesc, 1u);
-          mma4_f16_commit_elect(d_tmem, da, db + 2 * (C::kPlaneBytes >> 4), idesc, 1u, &empty[s]);
-        } else {
-          mma4_f16_commit_elect(d_tmem, da, db, idesc, (uint32_t)(ks != 0), &empty[s]);
+        const uint32_t d_tmem = tmem_base + acc * 128;
+        for (int ks = 0; ks < nk; ++ks, ++ia) {
+          const int sa = ia % kA;
+          if (!__all_sync(0xFFFFFFFFu, wait(&a_full[sa], (ia / kA) & 1, kStWaitFullA))) goto done;
+          const uint32_t a_tmem = tmem_base + kACols + sa * 32;
+#pragma unroll
+          for (int pl = 0; pl < PLANES; ++pl, ++ib) {
+            const int sb = ib % kB;
+            if (!__all_sync(0xFFFFFFFFu, wait(&b_full[sb], (ib / kB) & 1, kStWaitFullB))) goto done;
+            tc_fence_after();
+            mma4_f16_commit_pair_elect(d_tmem, a_tmem, db0 + (uint32_t)sb * (uint32_t)(C::kBBytes >> 4), idesc, (uint32_t)((ks | pl) != 0), &b_empty[sb]);
+          }
+          if (PLANES != 1) tc_commit_pair_elect(&a_empty[sa]);
         }
+        tc_commit_pair_elect(&tmem_full[acc]);
+        ++tile_i;
       }
-      tc_commit_elect(&tmem_full[acc]);
     }
-  } else if (warp < 6) {
+  } else if (warp == 2) {
+    // ---------------- producer: this CTA's 128 weight rows, 256 values of k per slot ----------------
+    const bool img = g.A.image;
+    const int ktiles = g.A.ktiles;
+    uint32_t it = 0;
+    for (int t = tile_first; t < ntiles; t += tile_step) {
+      const Tile p = tile_of(t);
+      if (p.width == 0) continue;
+      const int row_tile = 2 * p.tm + rank;
+      for (int sl = 0; sl < nslots; ++sl, ++it) {
+        const int s = it % kRaw;
+        if (!__all_sync(0xFFFFFFFFu, wait(&raw_empty[s], ((it / kRaw) & 1) ^ 1, kStWaitRaw))) goto done;
+        mbar_arrive_expect_tx_elect(&raw_full[s], C::kRawBytes);
+        const uint32_t dst = smem_u32(sRaw + (size_t)s * C::kRawBytes), bar = smem_u32(&raw_full[s]);
+        // (rows past the matrix read zeros; their scales are those of its last row, and no row past it is stored)
+        if (img) tma_load_3d_elect(dst, &tmap_w, 0, 0, row_tile * ktiles + sl, bar);
+        else tma_load_3d_elect(dst, &tmap_w, sl * 128, p.ro + row_tile * 128, 0, bar);
+      }
+    }
+  }
+  } else if (warp < 12) {
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kRegsEpi));
     // ---------------- epilogue ----------------
-    const int quad = warp & 3;
-    const float *const ga = g.e.ga;
-    const int ga_stride = g.e.ga_stride;
-    const float gf = g.e.gf, alpha = g.e.alpha, beta = g.e.beta;
+    const int quad = warp & 3, half = (warp - 4) >> 2, bar_id = 2 + half;   // barrier 1: all eight warps; 2 and 3: the four of a half
+    // (rarely used parameters are read from the constant bank where they are needed: the registers belong to the accumulator block)
     const float gb0 = g.e.gb ? __ldg(g.e.gb) : 1.f;   // B's global: dense B has none, INT8 B one for the tensor (a multiply by 1 is exact)
-    const void *const cptr = g.e.c, *const biasptr = g.e.bias;
-    const int ldc = g.e.ldc, c_dtype = g.e.c_dtype, bias_dtype = g.e.bias_dtype;
     uint8_t *const dptr = (uint8_t *)g.e.d;
-    const int ldd = g.e.ldd, d_dtype = g.e.d_dtype;
-    float *const amax_out = g.e.amax;
-    const int mask = g.x.mask;
-    const float *const norm_parts = g.x.norm_parts;
-    const int norm_nparts = g.x.norm_nparts, norm_ld = g.x.norm_ld;
-    const float norm_inv_n = g.x.norm_inv_n, norm_eps = g.x.norm_eps;
-    const float *const colscales = g.x.colscales;
-    uint8_t *const d2ptr = (uint8_t *)g.x.d2;
-    const int d2_dtype = g.x.d2_dtype, ldd2 = g.x.ldd2, w2_dtype = g.x.w2_dtype, ld_sq = g.x.ld_sq;
-    const void *const w2ptr = g.x.w2;
-    float *const sqptr = g.x.sq;
+    const int d_dtype = g.e.d_dtype, mask = g.x.mask;
     const bool d_tma = g.d_tma;
     const int esz = dense_bytes(d_dtype);
     const int cw = esz == 2 ? 32 : 16;
-    const bool leader = warp == 2 && lane == 0;
-    const float zf = ue ? 65536.f : 256.f;
+    const bool leader = quad == 0 && lane == 0;
+    uint8_t *const boxes = staging + half * 2 * C::kStagingBytes;
     float amax = 0.f;
-    uint32_t tile_i = 0;
-    for (int t = blockIdx.x; t < ntiles; t += gridDim.x, ++tile_i) {
-      const int tm = t % tiles_m, tn = t / tiles_m, acc = tile_i & 1;
+    uint32_t tile_i = 0, box = 0;
+    // a staging tile is free when the store before the last one has been read (the two tiles alternate)
+    auto next_box = [&]() -> uint8_t * {
+      if (leader) bulk_wait_read_one();
+      named_barrier(bar_id, 128);
+      return boxes + (box++ & 1) * C::kStagingBytes;
+    };
+    for (int t = tile_first; t < ntiles; t += tile_step) {
+      const Tile p = tile_of(t);
+      if (p.width == 0) continue;
+      const int tm = 2 * p.tm + rank, jt = p.j0, jend = min(p.j0 + p.width, p.jend), acc = nacc == 2 ? tile_i & 1 : 0;
+      const uint32_t acc_par = (nacc == 2 ? tile_i >> 1 : tile_i) & 1;
       const int i = tm * 128 + quad * 32 + lane;
-      const bool row_ok = i < gm;
-      const float rowp = row_ok ? __fmul_rn(alpha, ga ? ga[(size_t)i * ga_stride] : 1.f) : 0.f;
-      const float bias = (row_ok && biasptr) ? load_dense(bias_dtype, biasptr, i) : 0.f;
-      const float w2 = (row_ok && (mask & kExOut2)) ? load_dense(w2_dtype, w2ptr, i) : 0.f;
-      const float s_plain = __fmul_rn(__fmul_rn(rowp, gb0), gf);   // ((alpha gA) * gB) * gf
+      const bool row_ok = i < gm, tile_ok = tm * 128 < gm;   // (an odd number of 128-row tiles leaves the last pair's second CTA without rows)
+      const float rowp = row_ok ? __fmul_rn(g.e.alpha, g.e.ga ? g.e.ga[(size_t)(p.ro + i) * g.e.ga_stride] : 1.f) : 0.f;
+      const float bias = (row_ok && g.e.bias) ? load_dense(g.e.bias_dtype, g.e.bias, p.ro + i) : 0.f;
+      const float w2 = (row_ok && (mask & kExOut2)) ? load_dense(g.x.w2_dtype, g.x.w2, i) : 0.f;
+      const float s_plain = __fmul_rn(__fmul_rn(rowp, gb0), g.e.gf);   // ((g.e.alpha gA) * gB) * g.e.gf
       if (mask & kExNorm) {  // column scales of this token tile (the previous tile's are no longer in use: see the barrier below)
-        named_barrier(1, 128);
-        if (colscales) {  // computed before the launch, one float per token
-          for (int jj = quad * 32 + lane; jj < BN; jj += 128) colscale[jj] = __ldcg(colscales + min(tn * BN + jj, gn - 1));
+        named_barrier(1, 256);
+        if (g.x.colscales) {  // computed before the launch, one float per token
+          for (int jj = (warp - 4) * 32 + lane; jj < p.width; jj += 256) colscale[jj] = __ldcg(g.x.colscales + min(jt + jj, gn - 1));
         }
         // The defining order (reference include/nvfp4effma.h:224-226 there): lane l adds parts l, l + 32, ... in ascending
         // order, then an xor butterfly 16..1.  A warp takes 8 tokens at a time so that their loads fly together.
-        for (int j8 = quad * 8; j8 < BN && !colscales; j8 += 32) {
+        for (int j8 = (warp - 4) * 8; j8 < p.width && !g.x.colscales; j8 += 64) {
           float sum[8];
-          if (norm_nparts <= 256) {
+          if (g.x.norm_nparts <= 256) {
             float v[8][8];
 #pragma unroll
             for (int u = 0; u < 8; ++u) {
-              const int j = min(tn * BN + j8 + u, gn - 1);
-              const float *p = norm_parts + (size_t)j * norm_ld + lane;
+              const int j = min(jt + j8 + u, gn - 1);
+              const float *p = g.x.norm_parts + (size_t)j * g.x.norm_ld + lane;
 #pragma unroll
-              for (int q = 0; q < 8; ++q) v[u][q] = (32 * q + lane < norm_nparts) ? __ldcg(p + 32 * q) : 0.f;
+              for (int q = 0; q < 8; ++q) v[u][q] = (32 * q + lane < g.x.norm_nparts) ? __ldcg(p + 32 * q) : 0.f;
             }
 #pragma unroll
             for (int u = 0; u < 8; ++u) {
               float a = 0.f;
 #pragma unroll
               for (int q = 0; q < 8; ++q)
-                if (32 * q + lane < norm_nparts) a = __fadd_rn(a, v[u][q]);
+                if (32 * q + lane < g.x.norm_nparts) a = __fadd_rn(a, v[u][q]);
               sum[u] = a;
             }
           } else {
 #pragma unroll
             for (int u = 0; u < 8; ++u) {
-              const int j = min(tn * BN + j8 + u, gn - 1);
-              const float *p = norm_parts + (size_t)j * norm_ld;
+              const int j = min(jt + j8 + u, gn - 1);
+              const float *p = g.x.norm_parts + (size_t)j * g.x.norm_ld;
               float a = 0.f;
-              for (int q = lane; q < norm_nparts; q += 32) a = __fadd_rn(a, __ldcg(p + q));
+              for (int q = lane; q < g.x.norm_nparts; q += 32) a = __fadd_rn(a, __ldcg(p + q));
               sum[u] = a;
             }
           }
@@ -272,46 +376,55 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_const
             float a = sum[u];
 #pragma unroll
             for (int o = 16; o; o >>= 1) a = __fadd_rn(a, __shfl_xor_sync(0xFFFFFFFFu, a, o));
-            if (lane == 0) colscale[j8 + u] = __frsqrt_rn(__fadd_rn(__fmul_rn(a, norm_inv_n), norm_eps));
+            if (lane == 0) colscale[j8 + u] = __frsqrt_rn(__fadd_rn(__fmul_rn(a, g.x.norm_inv_n), g.x.norm_eps));
           }
         }
       }
-      if (!wait(&tmem_full[acc], (tile_i >> 1) & 1, kStWaitTmemFull)) *abort_flag = 1;
-      named_barrier(1, 128);   // the four epilogue warps go on together or not at all
+      if (!wait(&tmem_full[acc], acc_par, kStWaitTmemFull)) *abort_flag = 1;
+      named_barrier(1, 256);   // the eight epilogue warps go on together or not at all
       if (*abort_flag) goto done;
       tc_fence_after();
-      const int nchunks = min(BN / 32, (gn - tn * BN + 31) / 32);
+      // this warp's block (width / 2 columns: one, two or four chunks of 32) into registers, and the accumulator back to the MMA warp
+      const int hw = p.width >> 1, nchunks = hw >> 5;
+      const uint32_t acc_addr = tmem_base + ((uint32_t)(quad * 32) << 16) + acc * 128 + half * hw;
+      uint32_t r[32], r1[32], r2[32], r3[32];
+      tmem_ld32(acc_addr, r);
+      if (nchunks > 1) tmem_ld32(acc_addr + 32, r1);
+      if (nchunks > 2) { tmem_ld32(acc_addr + 64, r2); tmem_ld32(acc_addr + 96, r3); }
+      tmem_ld_wait();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive_rank(&tmem_empty[acc], 0);
       for (int c = 0; c < nchunks; ++c) {
-        uint32_t r[32];
-        tmem_ld32(tmem_base + ((uint32_t)(quad * 32) << 16) + acc * BN + c * 32, r);
-        tmem_ld_wait();
-        if (c == nchunks - 1) {
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(&tmem_empty[acc]);
+        if (c) {   // the next chunk moves into r
+#pragma unroll
+          for (int q = 0; q < 32; ++q) { r[q] = r1[q]; r1[q] = r2[q]; r2[q] = r3[q]; }
         }
-        const int j0 = tn * BN + c * 32;
-        const int nvalid = min(32, gn - j0);
+        const int cc = half * hw + c * 32;   // first column of the chunk in the tile
+        if (jt + cc >= jend) break;
+        const int j0 = jt + cc;
+        const int nvalid = min(32, jend - j0);
+        const bool tma = d_tma && (!GROUPED || nvalid == 32);   // (a group's last box would reach into the next group's tokens)
         // values before the output rounding, kept in r[] as FP32 bits
 #pragma unroll
         for (int jj = 0; jj < 32; ++jj) {
-          const float a = __fmul_rn(__uint_as_float(r[jj]), zf);
-          const float s = (mask & kExNorm) ? __fmul_rn(__fmul_rn(rowp, __fmul_rn(gb0, colscale[c * 32 + jj])), gf) : s_plain;
+          const float a = __uint_as_float(r[jj]);
+          const float s = (mask & kExNorm) ? __fmul_rn(__fmul_rn(rowp, __fmul_rn(gb0, colscale[cc + jj])), g.e.gf) : s_plain;
           float v = __fmul_rn(a, s);
-          if (biasptr) v = __fadd_rn(v, bias);
-          if (beta != 0.f && row_ok && jj < nvalid) v = __fmaf_rn(beta, load_dense(c_dtype, cptr, (size_t)(j0 + jj) * ldc + i), v);
+          if (g.e.bias) v = __fadd_rn(v, bias);
+          if (g.e.beta != 0.f && row_ok && jj < nvalid) v = __fmaf_rn(g.e.beta, load_dense(g.e.c_dtype, g.e.c, (size_t)(j0 + jj) * g.e.ldc + i), v);
           r[jj] = __float_as_uint(v);
         }
         if (mask & kExOut2) {  // second output v * w2[i] and the slice's sum of squares (rows 16 q .. 16 q + 15 in ascending order)
 #pragma unroll
           for (int jj = 0; jj < 32; ++jj) {
             const float v = __uint_as_float(r[jj]);
-            if (row_ok && jj < nvalid) store_dense(d2_dtype, d2ptr, (size_t)(j0 + jj) * ldd2 + i, __fmul_rn(v, w2));
+            if (row_ok && jj < nvalid) store_dense(g.x.d2_dtype, g.x.d2, (size_t)(j0 + jj) * g.x.ldd2 + i, __fmul_rn(v, w2));
             const float vv = __fmul_rn(v, v);
             float sq = 0.f;
 #pragma unroll
             for (int q = 0; q < 16; ++q) sq = __fadd_rn(sq, __shfl_sync(0xFFFFFFFFu, vv, (lane & 16) + q));
-            if (row_ok && !(lane & 15) && jj < nvalid) sqptr[(size_t)(j0 + jj) * ld_sq + (i >> 4)] = sq;
+            if (row_ok && !(lane & 15) && jj < nvalid) g.x.sq[(size_t)(j0 + jj) * g.x.ld_sq + (i >> 4)] = sq;
           }
         }
         if (mask & kExSwiglu) {  // rows 16 q + r (gate) and 16 q + 8 + r (up) -> output row 8 q + r: 64 output rows per tile
@@ -330,39 +443,38 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_const
             else if (d_dtype == NVFP4A_FP16) r[q] = (uint32_t)__half_as_ushort(__float2half_rn(h));
             else r[q] = __float_as_uint(h);
           }
-          if (!d_tma) {
+          if (!tma) {
             if (row_ok) {
 #pragma unroll
               for (int q = 0; q < 16; ++q)
                 if (2 * q + odd < nvalid) {
-                  if (esz == 2) ((uint16_t *)dptr)[(size_t)(j0 + 2 * q + odd) * ldd + io] = (uint16_t)r[q];
-                  else ((uint32_t *)dptr)[(size_t)(j0 + 2 * q + odd) * ldd + io] = r[q];
+                  if (esz == 2) ((uint16_t *)dptr)[(size_t)(j0 + 2 * q + odd) * g.e.ldd + io] = (uint16_t)r[q];
+                  else ((uint32_t *)dptr)[(size_t)(j0 + 2 * q + odd) * g.e.ldd + io] = r[q];
                 }
             }
             continue;
           }
           const int lr = quad * 16 + (lane >> 4) * 8 + (lane & 7);  // output row inside the tile's 64
           for (int half = 0; half < 32 / cw; ++half) {
-            if (leader) bulk_wait_read_all();
-            named_barrier(1, 128);
+            uint8_t *const st = next_box();
             if (esz == 2) {
 #pragma unroll
-              for (int q = 0; q < 16; ++q) ((uint16_t *)staging)[(2 * q + odd) * 64 + lr] = (uint16_t)r[q];
+              for (int q = 0; q < 16; ++q) ((uint16_t *)st)[(2 * q + odd) * 64 + lr] = (uint16_t)r[q];
             } else {
 #pragma unroll
-              for (int q = 0; q < 8; ++q) ((uint32_t *)staging)[(2 * q + odd) * 64 + lr] = half ? r[8 + q] : r[q];
+              for (int q = 0; q < 8; ++q) ((uint32_t *)st)[(2 * q + odd) * 64 + lr] = half ? r[8 + q] : r[q];
             }
             fence_proxy_async_smem();
-            named_barrier(1, 128);
-            if (leader) {
-              tma_store_2d(&tmap_d, staging, tm * 64, j0 + half * cw);
-              for (int p = 0; p < peers.n; ++p) tma_store_2d(&peers.map[p], staging, tm * 64, j0 + half * cw);   // the same tile into every peer's buffer
+            named_barrier(bar_id, 128);
+            if (leader && tile_ok) {
+              tma_store_2d(&tmap_d, st, tm * 64, j0 + half * cw);
+              for (int q = 0; q < peers.n; ++q) tma_store_2d(&peers.map[q], st, tm * 64, j0 + half * cw);   // the same tile into every peer's buffer
               bulk_commit();
             }
           }
           continue;
         }
-        if (amax_out && row_ok) {
+        if (g.e.amax && row_ok) {
 #pragma unroll
           for (int jj = 0; jj < 32; ++jj)
             if (jj < nvalid) amax = fmaxf(amax, fabsf(__uint_as_float(r[jj])));
@@ -373,137 +485,196 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_const
 #pragma unroll
           for (int jj = 0; jj < 32; ++jj) r[jj] = (uint32_t)__half_as_ushort(__float2half_rn(__uint_as_float(r[jj])));
         }
-        if (!d_tma) {
+        if (!tma) {
           if (row_ok) {
             if (esz == 2) {
-              uint16_t *d16 = (uint16_t *)dptr + (size_t)j0 * ldd + i;
+              uint16_t *d16 = (uint16_t *)dptr + (size_t)j0 * g.e.ldd + i;
 #pragma unroll
               for (int jj = 0; jj < 32; ++jj)
-                if (jj < nvalid) d16[(size_t)jj * ldd] = (uint16_t)r[jj];
+                if (jj < nvalid) d16[(size_t)jj * g.e.ldd] = (uint16_t)r[jj];
             } else {
-              uint32_t *d32 = (uint32_t *)dptr + (size_t)j0 * ldd + i;
+              uint32_t *d32 = (uint32_t *)dptr + (size_t)j0 * g.e.ldd + i;
 #pragma unroll
               for (int jj = 0; jj < 32; ++jj)
-                if (jj < nvalid) d32[(size_t)jj * ldd] = r[jj];
+                if (jj < nvalid) d32[(size_t)jj * g.e.ldd] = r[jj];
             }
           }
           continue;
         }
         for (int half = 0; half < 32 / cw; ++half) {
-          if (leader) bulk_wait_read_all();
-          named_barrier(1, 128);
+          uint8_t *const st = next_box();
           const int rr = quad * 32 + lane;
           if (esz == 2) {
 #pragma unroll
-            for (int jj = 0; jj < 32; ++jj) ((uint16_t *)staging)[jj * 128 + rr] = (uint16_t)r[jj];
+            for (int jj = 0; jj < 32; ++jj) ((uint16_t *)st)[jj * 128 + rr] = (uint16_t)r[jj];
           } else {
 #pragma unroll
-            for (int jj = 0; jj < 16; ++jj) ((uint32_t *)staging)[jj * 128 + rr] = half ? r[16 + jj] : r[jj];
+            for (int jj = 0; jj < 16; ++jj) ((uint32_t *)st)[jj * 128 + rr] = half ? r[16 + jj] : r[jj];
           }
           fence_proxy_async_smem();
-          named_barrier(1, 128);
-          if (leader) {
-            tma_store_2d(&tmap_d, staging, tm * 128, j0 + half * cw);
-            for (int p = 0; p < peers.n; ++p) tma_store_2d(&peers.map[p], staging, tm * 128, j0 + half * cw);   // the same tile into every peer's buffer
+          named_barrier(bar_id, 128);
+          if (leader && tile_ok) {
+            tma_store_2d(&tmap_d, st, tm * 128, j0 + half * cw);
+            for (int q = 0; q < peers.n; ++q) tma_store_2d(&peers.map[q], st, tm * 128, j0 + half * cw);   // the same tile into every peer's buffer
             bulk_commit();
           }
         }
       }
+      ++tile_i;
     }
     if (leader) bulk_wait_all();
-    if (amax_out) warp_amax_commit(amax_out, amax);
+    if (g.e.amax) warp_amax_commit(g.e.amax, amax);
   } else {
-    // ---------------- weight expansion: NVFP4 -> BF16 into the swizzled A tile ----------------
-    // Two groups of four warps take alternate stages; inside a group thread r owns row r of the stage: 64 nibbles (32
-    // contiguous bytes) and their 4 scale bytes, fetched one of its own stages (two pipeline stages) ahead.
-    const int cwarp = warp - 6, group = cwarp >> 2;
-    const int row = (cwarp & 3) * 32 + lane;
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsConv));
+    // ---------------- weight expansion: NVFP4 -> 16-bit floats in tensor memory ----------------
+    // Two groups of four warps take the even and the odd stages of a tile; inside a group thread r owns row r of the CTA's 128 (and
+    // tensor memory lane r: warp % 4 is its quadrant): a stage's 64 nibbles are two 16-byte words of the slot's swizzled row, its 4 scale bytes one word fetched a slot (four stages)
+    // ahead.  A slot goes back to the producer as soon as its words are in registers.
+    const int cwarp = warp - 12, group = cwarp >> 2;
+    const int row = (cwarp & 3) * 32 + lane, r7 = row & 7;
     const Fp4Operand A = g.A;
     const ScalePos sp{A.sld};
-    // source pointers of (tile t, k step 0) for this thread's row; a k step advances nibbles by 32 bytes and scales by 4
-    auto tile_ptrs = [&](int t, const uint8_t *&wp, const uint8_t *&scp) {
-      const int r = min((t % tiles_m) * 128 + row, gm - 1);
-      if (A.image) {
-        const uint8_t *tile = A.data + (size_t)(r >> 7) * A.ktiles * kImgTileBytes;
-        const int rr = r & 127;
-        wp = tile + rr * 128;
-        scp = tile + kImgDataBytes + (rr & 31) * 16 + (rr >> 5) * 4;
-      } else {
-        wp = A.data + (size_t)r * (A.ld >> 1);
-        scp = A.sc + sp.row(r);
+    const bool img = A.image, swz = A.sld < 0;
+    // scale words of this group's two stages of slot sl (stages past the end of k: zeros)
+    auto fetch_scales = [&](const uint8_t *scp, int sl, uint32_t (&v)[2]) {
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int ks = 4 * sl + group + 2 * h;
+        const size_t off = img ? (size_t)sl * kImgTileBytes + (ks & 3) * 512 : swz ? (size_t)ks * 512 : (size_t)ks * 4;
+        v[h] = ks < nk ? __ldg((const uint32_t *)(scp + off)) : 0u;
       }
     };
-    const bool img = A.image, swz = A.sld < 0;
-    auto fetch = [&](const uint8_t *wp, const uint8_t *scp, int ks, RawRow &v) {
-      size_t woff, soff;
-      if (img) { woff = (size_t)(ks >> 2) * kImgTileBytes + (ks & 3) * 32; soff = (size_t)(ks >> 2) * kImgTileBytes + (ks & 3) * 512; }
-      else { woff = (size_t)ks * 32; soff = swz ? (size_t)ks * 512 : (size_t)ks * 4; }
-      v.w0 = __ldg((const uint4 *)(wp + woff));
-      v.w1 = __ldg((const uint4 *)(wp + woff + 16));
-      v.sc = __ldg((const uint32_t *)(scp + soff));
-    };
-    // prefetch cursor: this group's next stage (tile pf_t, k step pf_ks)
-    int pf_t = blockIdx.x, pf_ks = group;
-    const uint8_t *pf_w = nullptr, *pf_s = nullptr;
-    auto advance = [&]() {  // to the group's following stage
-      pf_ks += 2;
-      while (pf_ks >= nk && pf_t < ntiles) { pf_ks -= nk; pf_t += gridDim.x; if (pf_t < ntiles) tile_ptrs(pf_t, pf_w, pf_s); }
-    };
-    RawRow cur, nxt;
-    cur.w0 = cur.w1 = nxt.w0 = nxt.w1 = make_uint4(0, 0, 0, 0); cur.sc = nxt.sc = 0;
-    if (pf_t < ntiles) tile_ptrs(pf_t, pf_w, pf_s);
-    while (pf_ks >= nk && pf_t < ntiles) { pf_ks -= nk; pf_t += gridDim.x; if (pf_t < ntiles) tile_ptrs(pf_t, pf_w, pf_s); }
-    if (pf_t < ntiles) { fetch(pf_w, pf_s, pf_ks, cur); advance(); }
-    uint32_t it = 0;
-    for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
-      for (int ks = 0; ks < nk; ++ks, ++it) {
-        if ((int)(it & 1) != group) continue;
-        if (pf_t < ntiles) { fetch(pf_w, pf_s, pf_ks, nxt); advance(); }
-        const int s = it % kStages;
-        if (!wait(&empty[s], ((it / kStages) & 1) ^ 1, kStWaitConv)) goto done;
-        uint8_t *sA = smem + (size_t)s * C::kStageBytes + row * 128;
-        const uint32_t wv[8] = {cur.w0.x, cur.w0.y, cur.w0.z, cur.w0.w, cur.w1.x, cur.w1.y, cur.w1.z, cur.w1.w};
+    uint32_t isl = 0, it0 = 0;   // slots so far; stages of the finished tiles
+    for (int t = tile_first; t < ntiles; t += tile_step, it0 += nk) {
+      const Tile p = tile_of(t);
+      if (p.width == 0) { it0 -= nk; continue; }
+      const int r = min((2 * p.tm + rank) * 128 + row, gm - 1);
+      const uint8_t *scp = img ? A.data + (size_t)(r >> 7) * A.ktiles * kImgTileBytes + kImgDataBytes + (r & 31) * 16 + ((r & 127) >> 5) * 4
+                               : A.sc + sp.row(p.ro + r);
+      uint32_t sc[2], sc_next[2] = {0, 0};
+      fetch_scales(scp, 0, sc);
+      for (int sl = 0; sl < nslots; ++sl, ++isl) {
+        if (sl + 1 < nslots) fetch_scales(scp, sl + 1, sc_next);
+        const int rs = isl % kRaw;
+        if (!wait(&raw_full[rs], (isl / kRaw) & 1, kStWaitRaw)) goto done;
+        const uint8_t *src = sRaw + (size_t)rs * C::kRawBytes + row * 128;
+        uint4 w[4];
 #pragma unroll
-        for (int q = 0; q < 8; ++q) {  // word q: k = 8 q .. 8 q + 7 of the stage, block q / 2
-          const uint32_t sc = lut[(cur.sc >> (8 * (q >> 1))) & 0xFF];
-          const uint32_t d0 = bf16x2_mul(decode_pair<0>(wv[q]), sc), d1 = bf16x2_mul(decode_pair<1>(wv[q]), sc);
-          const uint32_t d2 = bf16x2_mul(decode_pair<2>(wv[q]), sc), d3 = bf16x2_mul(decode_pair<3>(wv[q]), sc);
-          // (n0 n4)(n1 n5)(n2 n6)(n3 n7) -> (n0 n1)(n2 n3)(n4 n5)(n6 n7)
-          const uint4 o = make_uint4(prmt(d0, d1, 0x5410), prmt(d2, d3, 0x5410), prmt(d0, d1, 0x7632), prmt(d2, d3, 0x7632));
-          *(uint4 *)(sA + ((q ^ (row & 7)) << 4)) = o;
-        }
-        fence_proxy_async_smem();
+        for (int q = 0; q < 4; ++q) w[q] = *(const uint4 *)(src + (((2 * group + 4 * (q >> 1) + (q & 1)) ^ r7) << 4));
         __syncwarp();
-        if (lane == 0) mbar_arrive(&full[s]);
-        cur = nxt;
+        if (lane == 0) mbar_arrive(&raw_empty[rs]);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int ks = 4 * sl + group + 2 * h;
+          if (ks >= nk) break;
+          const uint32_t it = it0 + ks;
+          const int s = it % kA;
+          if (!wait(&a_empty[s], ((it / kA) & 1) ^ 1, kStWaitConv)) goto done;
+          tc_fence_after();   // the MMAs of the stage's previous round have read it
+          const uint32_t dst = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + kACols + s * 32;
+#pragma unroll
+          for (int u = 0; u < 2; ++u) {   // 32 values: two blocks, 16 columns
+            const uint32_t wv[4] = {w[2 * h + u].x, w[2 * h + u].y, w[2 * h + u].z, w[2 * h + u].w};
+            uint32_t o[16];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {  // 8 values per word
+              const uint4 t4 = lut[(sc[h] >> (16 * u + 8 * (q >> 1))) & 0xFF];
+              expand4(wv[q], t4, o[4 * q], o[4 * q + 1]);
+              expand4(wv[q] >> 16, t4, o[4 * q + 2], o[4 * q + 3]);
+            }
+            tmem_st16(dst + 16 * u, o);
+          }
+          tmem_st_wait();
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive_rank(&a_full[s], 0);
+        }
+        sc[0] = sc_next[0]; sc[1] = sc_next[1];
       }
     }
   }
 done:
   __syncwarp();
   tc_fence_before();
-  __syncthreads();
+  cluster_sync_all();   // neither CTA leaves (or frees tensor memory) while the other may still arrive on its barriers
   if (warp == 1) {
     tc_fence_after();
-    tmem_dealloc(tmem_base, 512);
+    tmem_dealloc_pair(tmem_base, 512);
   }
 }
 
-template <int BN, int PLANES = 1>
-cudaError_t launch_cfg(const CUtensorMap &tb, const CUtensorMap &td, const PeerMaps &pm, const W4A16Args &a, cudaStream_t s) {
-  using C = Cfg<BN, PLANES>;
+// Tile width and cut for a problem of `rows256` 256-row tiles and n tokens: the width whose rounds over the SM pairs cost least, a stage
+// costing what its MMAs take (2 cycles per token and plane) but not less than its weight expansion (about 300 cycles); the tiles of
+// the last round are cut into 2 or 4 parts while the pairs can take them all at once.
+struct Plan { int width, nfull, cut, tiles; };
+Plan make_plan(int rows256, int n, int planes, int pairs) {
+  Plan best = {0, 0, 1, 0};
+  long long best_cost = 0;
+  for (int w = 256; w >= 64; w /= 2) {
+    if (w > 64 && w / 2 >= n) continue;   // half of the width covers every token
+    const int tiles = rows256 * ((n + w - 1) / w), rest = tiles % pairs;
+    auto cost = [&](int width) { return (long long)(2 * width * planes > 300 ? 2 * width * planes : 300); };
+    int cut = 1;
+    while (tiles > pairs && rest && w / (2 * cut) >= 64 && rest * 2 * cut <= pairs) cut *= 2;
+    const long long c = tiles / pairs * cost(w) + (rest ? cost(w / cut) : 0);
+    if (!best.width || c < best_cost) {
+      best_cost = c;
+      best = Plan{w, cut > 1 ? tiles - rest : tiles, cut, cut > 1 ? tiles - rest + rest * cut : tiles};
+    }
+  }
+  return best;
+}
+
+template <int PLANES, bool F16, bool GROUPED = false>
+cudaError_t launch_cfg(const CUtensorMap &tw, const CUtensorMap &tb, const CUtensorMap &td, const PeerMaps &pm, const W4A16Args &a, cudaStream_t s) {
+  using C = Cfg<PLANES>;
   static std::atomic<bool> attr_set[64];   // zero-initialised; set once per device (a repeated cudaFuncSetAttribute is harmless)
   int dev = 0;
   cudaGetDevice(&dev);
   if (!attr_set[dev & 63]) {
-    const cudaError_t e = cudaFuncSetAttribute(gemm_w4a16_kernel<BN, PLANES>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes);
+    const cudaError_t e = cudaFuncSetAttribute(gemm_w4a16_kernel<PLANES, F16, GROUPED>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes);
     if (e != cudaSuccess) return e;
     attr_set[dev & 63] = true;
   }
-  const int tiles = ((a.m + 127) / 128) * ((a.n + BN - 1) / BN);
-  const int grid = tiles < device_sms() ? tiles : device_sms();
-  gemm_w4a16_kernel<BN, PLANES><<<grid, kThreads, C::kSmemBytes, s>>>(tb, td, pm, a);
-  return cudaGetLastError();
+  const int pairs = device_sms() / 2;
+  cudaLaunchConfig_t cfg;
+  memset(&cfg, 0, sizeof cfg);
+  cfg.gridDim = dim3(2 * (a.tiles < pairs ? a.tiles : pairs), 1, 1);
+  cfg.blockDim = dim3(kThreads, 1, 1);
+  cfg.dynamicSmemBytes = C::kSmemBytes;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr; cfg.numAttrs = pdl_enabled() ? 2 : 1;
+  return cudaLaunchKernelEx(&cfg, gemm_w4a16_kernel<PLANES, F16, GROUPED>, tw, tb, td, pm, a);
+}
+
+// what every launch of the kernel shares: arguments, the schedule, the maps of the weights, of the activations (`row_bytes` bytes per
+// token, `pitch` between tokens) and of D
+bool set_up(const GemmArgs &g, int planes, const void *act, uint64_t row_bytes, uint64_t pitch, W4A16Args *a, CUtensorMap *tw, CUtensorMap *tb, CUtensorMap *td) {
+  memset(a, 0, sizeof *a);
+  a->m = g.m; a->n = g.n; a->k = g.k;
+  a->A = g.A;
+  a->e = g.e; a->x = g.x;
+  a->status = kernel_status_device_ptr();
+  a->tag = next_launch_tag();
+  const Plan p = make_plan((g.m + 255) / 256, g.n, planes, device_sms() / 2);
+  a->width = p.width; a->nfull = p.nfull; a->cut = p.cut; a->tiles = p.tiles;
+  const uint64_t wtiles = (uint64_t)((g.m + 127) / 128) * g.A.ktiles;
+  if (g.A.image ? !make_tmap_bytes(tw, g.A.data, 128, 128, 128, 128, wtiles, kImgTileBytes)
+                : !make_tmap_bytes(tw, g.A.data, (uint64_t)g.k / 2, (uint64_t)g.m, (uint64_t)g.A.ld / 2, 128, 1, (uint64_t)g.A.ld / 2 * g.m))
+    return false;
+  if (!make_tmap_bytes(tb, act, row_bytes, (uint64_t)g.n, pitch, p.width / 2, 1, pitch * g.n)) return false;
+  memset(td, 0, sizeof *td);
+  const int esz = dense_bytes(g.e.d_dtype);
+  const bool glu = (g.x.mask & kExSwiglu) != 0;
+  const int drows = glu ? g.m / 2 : g.m;   // SwiGLU: the output has m / 2 rows, 64 per 128-row tile
+  a->d_tma = ((uintptr_t)g.e.d & 15) == 0 && ((size_t)g.e.ldd * esz) % 16 == 0 && ((size_t)drows * esz) % 16 == 0 &&
+             make_tmap_dense(td, g.e.d, esz, (uint64_t)drows, (uint64_t)g.n, (uint64_t)g.e.ldd * esz, glu ? 64 : 128, esz == 2 ? 32 : 16);
+  return true;
 }
 
 // INT8 activations q [n][ld] with one FP32 scale per 16 values -> three BF16 planes [n][3][k] with t1 + t2 + t3 = fl(q * s) exactly.
@@ -545,7 +716,10 @@ bool gemm_w4a16_pushes(const GemmArgs &g) {
 }
 
 bool gemm_w4a16_supports(const GemmArgs &g) {
-  if (g.B.dtype != NVFP4A_BF16 || g.k < 64 || ((uintptr_t)g.B.data & 15) || g.B.ld % 8) return false;
+  // FP16 activations: E4M3 scales (UE5M3 products leave FP16's range) and a 16-bit D -- with an FP32 D the CUDA-core kernel's ordered
+  // FP32 sums are closer to the exact value than the tensor cores'
+  const bool f16 = g.B.dtype == NVFP4A_FP16 && !g.A.ue && g.e.d_dtype != NVFP4A_FP32;
+  if ((g.B.dtype != NVFP4A_BF16 && !f16) || g.k < 64 || ((uintptr_t)g.B.data & 15) || g.B.ld % 8) return false;
   if (!g.A.image && (((uintptr_t)g.A.data & 15) || g.A.ld % 32 || ((uintptr_t)g.A.sc & 1))) return false;
   return true;
 }
@@ -598,13 +772,6 @@ bool gemm_w4a8_tc_supports(const GemmArgs &g) {
 }
 
 cudaError_t launch_gemm_w4a8_tc(const GemmArgs &g, cudaStream_t s) {
-  W4A16Args a;
-  memset(&a, 0, sizeof a);
-  a.m = g.m; a.n = g.n; a.k = g.k;
-  a.A = g.A;
-  a.e = g.e; a.x = g.x;
-  a.status = kernel_status_device_ptr();
-  a.tag = next_launch_tag();
   uint16_t *planes = nullptr;
   cudaMemPool_t pool;
   cudaError_t e = planes_pool(&pool);
@@ -614,18 +781,12 @@ cudaError_t launch_gemm_w4a8_tc(const GemmArgs &g, cudaStream_t s) {
   const long long groups = (long long)g.n * (g.k >> 3);
   w4a8_planes_kernel<<<(unsigned)((groups + 255) / 256), 256, 0, s>>>((const int8_t *)g.B.data, g.B.ld, g.B.s8, g.B.lds8, g.n, g.k, planes);
   e = cudaGetLastError();
-  CUtensorMap tb, td;
-  memset(&td, 0, sizeof td);
-  if (e == cudaSuccess && !make_tmap_bytes(&tb, planes, (uint64_t)g.k * 6, (uint64_t)g.n, (uint64_t)g.k * 6, 128)) e = cudaErrorInvalidValue;
   if (e == cudaSuccess) {
-    const int esz = dense_bytes(g.e.d_dtype);
-    const bool glu = (g.x.mask & kExSwiglu) != 0;
-    const int drows = glu ? g.m / 2 : g.m;
-    a.d_tma = ((uintptr_t)g.e.d & 15) == 0 && ((size_t)g.e.ldd * esz) % 16 == 0 && ((size_t)drows * esz) % 16 == 0 &&
-              make_tmap_dense(&td, g.e.d, esz, (uint64_t)drows, (uint64_t)g.n, (uint64_t)g.e.ldd * esz, glu ? 64 : 128, esz == 2 ? 32 : 16);
+    W4A16Args a;
+    CUtensorMap tw, tb, td;
     PeerMaps pm;
     memset(&pm, 0, sizeof pm);
-    e = launch_cfg<128, 3>(tb, td, pm, a, s);
+    e = set_up(g, 3, planes, (uint64_t)g.k * 6, (uint64_t)g.k * 6, &a, &tw, &tb, &td) ? launch_cfg<3, false>(tw, tb, td, pm, a, s) : cudaErrorInvalidValue;
   }
   const cudaError_t ef = cudaFreeAsync(planes, s);
   return e != cudaSuccess ? e : ef;
@@ -633,24 +794,14 @@ cudaError_t launch_gemm_w4a8_tc(const GemmArgs &g, cudaStream_t s) {
 
 cudaError_t launch_gemm_w4a16(const GemmArgs &g, cudaStream_t s) {
   W4A16Args a;
-  memset(&a, 0, sizeof a);
-  a.m = g.m; a.n = g.n; a.k = g.k;
-  a.A = g.A;
-  a.e = g.e; a.x = g.x;
-  a.status = kernel_status_device_ptr();
-  a.tag = next_launch_tag();
-  const int bn = g.n > 128 ? 256 : 128;
-  CUtensorMap tb, td;
-  if (!make_tmap_bytes(&tb, g.B.data, (uint64_t)g.k * 2, (uint64_t)g.n, (uint64_t)g.B.ld * 2, bn)) return cudaErrorInvalidValue;
-  memset(&td, 0, sizeof td);
-  const int esz = dense_bytes(g.e.d_dtype);
-  const bool glu = (g.x.mask & kExSwiglu) != 0;
-  const int drows = glu ? g.m / 2 : g.m;   // SwiGLU: the output has m / 2 rows, 64 per tile
-  a.d_tma = ((uintptr_t)g.e.d & 15) == 0 && ((size_t)g.e.ldd * esz) % 16 == 0 && ((size_t)drows * esz) % 16 == 0 &&
-            make_tmap_dense(&td, g.e.d, esz, (uint64_t)drows, (uint64_t)g.n, (uint64_t)g.e.ldd * esz, glu ? 64 : 128, esz == 2 ? 32 : 16);
+  CUtensorMap tw, tb, td;
+  if (!set_up(g, 1, g.B.data, (uint64_t)g.k * 2, (uint64_t)g.B.ld * 2, &a, &tw, &tb, &td)) return cudaErrorInvalidValue;
   PeerMaps pm;
   memset(&pm, 0, sizeof pm);
   if (gemm_w4a16_pushes(g)) {   // tensor parallel: the epilogue's TMA stores also go to every peer's copy of D
+    const int esz = dense_bytes(g.e.d_dtype);
+    const bool glu = (g.x.mask & kExSwiglu) != 0;
+    const int drows = glu ? g.m / 2 : g.m;
     for (int p = 0; p < g.tp.world; ++p) {
       if (p == g.tp.rank) continue;
       if (!make_tmap_dense(&pm.map[pm.n], (uint8_t *)g.e.d + g.tp.delta[p], esz, (uint64_t)drows, (uint64_t)g.n, (uint64_t)g.e.ldd * esz, glu ? 64 : 128,
@@ -659,7 +810,7 @@ cudaError_t launch_gemm_w4a16(const GemmArgs &g, cudaStream_t s) {
       ++pm.n;
     }
   }
-  return bn == 256 ? launch_cfg<256>(tb, td, pm, a, s) : launch_cfg<128>(tb, td, pm, a, s);
+  return g.B.dtype == NVFP4A_FP16 ? launch_cfg<1, true>(tw, tb, td, pm, a, s) : launch_cfg<1, false>(tw, tb, td, pm, a, s);
 }
 
 }  // namespace nvb

@@ -722,3 +722,17 @@ def test_blocked_gemv_with_sixteen_and_thirty_two_rows_per_cta():
         hs = dict(h, A=As)
         got_short, _ = run_gemm(cs, hs)
         assert np.array_equal(values(got_tall, c, h)[:, :160], values(got_short, cs, hs))
+
+
+@pytest.mark.parametrize("m,n,k", [(1, 1, 64), (128, 8, 192), (129, 9, 320), (257, 63, 256), (300, 65, 1088), (520, 257, 576), (1100, 700, 512)])
+def test_fp16_activations_on_the_tensor_cores(m, n, k):
+    """FP16 activations with a 16-bit D run on the tcgen05 kernel (route 5; weights expanded to exact FP16) for every n; an FP32 D or
+    UE5M3 scales keep the CUDA-core kernel.  Edges of the 256-row / 64-token tiles and of the 256-value slots of k, every epilogue input."""
+    for i, (dt, fa, route) in enumerate([(L.FP16, 0, 5), (L.BF16, SW, 5), (L.FP16, AM | PR, 5), (L.FP32, 0, 1), (L.FP16, UE, 1)]):
+        c = Case(m, n, k, L.FP16, dt, dt if i % 2 else -1, L.BF16 if i % 2 else -1, 1.25 if i % 2 else 1.0, 0.5 if i % 2 else 0.0, fa=fa)
+        h = build_case(c, 5200 + 10 * m + i)
+        exp = oracle_case(c, h, want_ref=True)
+        got, amax = run_gemm(c, h)
+        assert L.lib.nvfp4a_b200_last_route() == route, c
+        check_bound(c, h, got, amax, exp)
+    assert kernel_status() == 0
