@@ -76,7 +76,7 @@ struct alignas(64) PeerMaps {
 template <int PLANES>
 struct Cfg {
   // PLANES = 1: the weight and the activation ring advance together and share their `empty` barriers (one commit per stage)
-  static constexpr int kA = 8, kB = 8, kRaw = 2;
+  static constexpr int kA = 8, kB = 8, kRaw = 3;
   static constexpr int kBBytes = 128 * 128, kRawBytes = 128 * 128, kStagingBytes = 8192;
   static constexpr int kSmemBytes = 1024 + kB * kBBytes + kRaw * kRawBytes + 4 * kStagingBytes + 4096 /* expansion table */ + 256 * 4 /* column scales */ +
                                     512 /* barriers */ + 2 * 257 * 4 + 8 /* groups */;
@@ -84,7 +84,7 @@ struct Cfg {
 static_assert(Cfg<1>::kSmemBytes <= 232448, "shared memory budget");
 constexpr int kACols = 256;   // first tensor memory column of the weight stages (32 columns each)
 
-constexpr int kThreads = 640, kRegsRest = 40, kRegsEpi = 160, kRegsConv = 56;
+constexpr int kThreads = 640, kRegsRest = 40, kRegsEpi = 128, kRegsConv = 72;
 static_assert(128 * kRegsRest + 256 * kRegsEpi + 256 * kRegsConv <= kThreads * 96, "the split draws on the registers of the launch: 96 per thread");
 constexpr unsigned kStWaitFullA = 0x301, kStWaitFullB = 0x302, kStWaitEmpty = 0x303, kStWaitTmemFull = 0x304, kStWaitTmemEmpty = 0x305,
                    kStWaitConv = 0x306, kStWaitRaw = 0x307;
@@ -104,6 +104,17 @@ __device__ __forceinline__ void expand4(uint32_t w, const uint4 &t, uint32_t &o0
   const uint32_t hi = prmt(t.x, t.y, sel) | ((s << 1) & 0x80808080u), lo = prmt(t.z, t.w, sel);
   o0 = prmt(lo, hi, 0x5140u);
   o1 = prmt(lo, hi, 0x7362u);
+}
+
+__device__ __forceinline__ uint32_t bf16x2_rn(float lo, float hi) {
+  uint32_t d;
+  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(d) : "f"(hi), "f"(lo));
+  return d;
+}
+// four 8 x 8 blocks of 16-bit values in MMA fragment layout, each stored transposed: lane 8 q + j gives the address of row j (16 bytes,
+// the fragment's column j) of block q
+__device__ __forceinline__ void stmatrix_x4_trans(void *row, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+  asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1, %2, %3, %4};" ::"r"(smem_u32(row)), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
 }
 
 // one stage's four MMAs (K = 16 each: 8 tensor memory columns of A, 32 bytes along B's 128-byte rows) over a CTA pair and the commit that hands the activation slot
@@ -312,8 +323,12 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
     uint8_t *const dptr = (uint8_t *)g.e.d;
     const int d_dtype = g.e.d_dtype, mask = g.x.mask;
     const bool d_tma = g.d_tma;
-    const int esz = dense_bytes(d_dtype);
-    const int cw = esz == 2 ? 32 : 16;
+    // The accumulator is read as MMA fragments (16 lanes x 8 columns per register quad): a thread holds rows rb + 16 hh + 8 u (hh, u in
+    // {0, 1}) of columns 8 gq + cp + e (e in {0, 1}) of a chunk of 32, register 16 hh + 4 gq + 2 u + e.  Gate and up rows of SwiGLU (8
+    // apart) then meet in one thread, neighbouring columns pack into one conversion, and stmatrix transposes 8 x 8 blocks on their
+    // way into the staging box: 4 instructions per chunk where a lane per row took 32 two-byte stores (and a shuffle per SwiGLU pair).
+    // With SwiGLU the epilogue, which shares issue slots with the expansion, took 140 of 490 us at 28672 x 2048 x 4096.
+    const int cp = 2 * (lane & 3), l7 = lane & 7, mi = lane >> 3;
     const bool leader = quad == 0 && lane == 0;
     uint8_t *const boxes = staging + half * 2 * C::kStagingBytes;
     float amax = 0.f;
@@ -329,12 +344,16 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
       if (p.width == 0) continue;
       const int tm = 2 * p.tm + rank, jt = p.j0, jend = min(p.j0 + p.width, p.jend), acc = nacc == 2 ? tile_i & 1 : 0;
       const uint32_t acc_par = (nacc == 2 ? tile_i >> 1 : tile_i) & 1;
-      const int i = tm * 128 + quad * 32 + lane;
-      const bool row_ok = i < gm, tile_ok = tm * 128 < gm;   // (an odd number of 128-row tiles leaves the last pair's second CTA without rows)
-      const float rowp = row_ok ? __fmul_rn(g.e.alpha, g.e.ga ? g.e.ga[(size_t)(p.ro + i) * g.e.ga_stride] : 1.f) : 0.f;
-      const float bias = (row_ok && g.e.bias) ? load_dense(g.e.bias_dtype, g.e.bias, p.ro + i) : 0.f;
-      const float w2 = (row_ok && (mask & kExOut2)) ? load_dense(g.x.w2_dtype, g.x.w2, i) : 0.f;
-      const float s_plain = __fmul_rn(__fmul_rn(rowp, gb0), g.e.gf);   // ((g.e.alpha gA) * gB) * g.e.gf
+      const int rb = tm * 128 + quad * 32 + (lane >> 2);
+      const bool tile_ok = tm * 128 < gm;   // (an odd number of 128-row tiles leaves the last pair's second CTA without rows)
+      float rowp[4], bias[4];               // row 8 q of this thread's four: alpha gA, bias
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int i = rb + 8 * q;
+        rowp[q] = i < gm ? __fmul_rn(g.e.alpha, g.e.ga ? g.e.ga[(size_t)(p.ro + i) * g.e.ga_stride] : 1.f) : 0.f;
+        bias[q] = (i < gm && g.e.bias) ? load_dense(g.e.bias_dtype, g.e.bias, p.ro + i) : 0.f;
+        if (!(mask & kExNorm)) rowp[q] = __fmul_rn(__fmul_rn(rowp[q], gb0), g.e.gf);   // ((alpha gA) * gB) * gf
+      }
       if (mask & kExNorm) {  // column scales of this token tile (the previous tile's are no longer in use: see the barrier below)
         named_barrier(1, 256);
         if (g.x.colscales) {  // computed before the launch, one float per token
@@ -382,141 +401,172 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
       }
       if (!wait(&tmem_full[acc], acc_par, kStWaitTmemFull)) *abort_flag = 1;
       named_barrier(1, 256);   // the eight epilogue warps go on together or not at all
-      if (*abort_flag) goto done;
+      if (__any_sync(0xFFFFFFFFu, *abort_flag)) goto done;
       tc_fence_after();
-      // this warp's block (width / 2 columns: one, two or four chunks of 32) into registers, and the accumulator back to the MMA warp
-      const int hw = p.width >> 1, nchunks = hw >> 5;
+      // this warp's block: width / 2 columns, one, two or four chunks of 32.  The chunk after the next is requested while one is processed;
+      // the accumulator goes back to the MMA warp with the last chunk's load.  (A 256-column accumulator is alone in tensor memory: until
+      // then the weight stages fill up behind it, eight deep, and the MMAs catch up from there.)
+      const int hw = p.width >> 1, nchunks = min(hw, jend - jt - half * hw + 31) >> 5;   // (chunks past the last token are left alone)
       const uint32_t acc_addr = tmem_base + ((uint32_t)(quad * 32) << 16) + acc * 128 + half * hw;
-      uint32_t r[32], r1[32], r2[32], r3[32];
-      tmem_ld32(acc_addr, r);
-      if (nchunks > 1) tmem_ld32(acc_addr + 32, r1);
-      if (nchunks > 2) { tmem_ld32(acc_addr + 64, r2); tmem_ld32(acc_addr + 96, r3); }
-      tmem_ld_wait();
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive_rank(&tmem_empty[acc], 0);
+      uint32_t r[32], rn[32];
+      auto load_chunk = [&](int c, uint32_t (&v)[32]) {
+        tmem_ld_16x256b_x4(acc_addr + 32 * c, v);
+        tmem_ld_16x256b_x4(acc_addr + (16u << 16) + 32 * c, v + 16);
+      };
+      auto release = [&]() {
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_rank(&tmem_empty[acc], 0);
+      };
+      if (nchunks > 0) load_chunk(0, rn);
+      else release();
       for (int c = 0; c < nchunks; ++c) {
-        if (c) {   // the next chunk moves into r
+        __syncwarp();   // (the tensor memory loads and waits are warp-wide)
+        tmem_ld_wait32(rn);
 #pragma unroll
-          for (int q = 0; q < 32; ++q) { r[q] = r1[q]; r1[q] = r2[q]; r2[q] = r3[q]; }
+        for (int q = 0; q < 32; ++q) r[q] = rn[q];
+        if (c + 1 < nchunks) load_chunk(c + 1, rn);
+        if (c == (nchunks > 1 ? nchunks - 2 : 0)) {   // every column of this warp's block is in registers
+          if (nchunks > 1) tmem_ld_wait32(rn);
+          release();
         }
         const int cc = half * hw + c * 32;   // first column of the chunk in the tile
-        if (jt + cc >= jend) break;
         const int j0 = jt + cc;
         const int nvalid = min(32, jend - j0);
         const bool tma = d_tma && (!GROUPED || nvalid == 32);   // (a group's last box would reach into the next group's tokens)
         // values before the output rounding, kept in r[] as FP32 bits
 #pragma unroll
-        for (int jj = 0; jj < 32; ++jj) {
-          const float a = __uint_as_float(r[jj]);
-          const float s = (mask & kExNorm) ? __fmul_rn(__fmul_rn(rowp, __fmul_rn(gb0, colscale[cc + jj])), g.e.gf) : s_plain;
-          float v = __fmul_rn(a, s);
-          if (g.e.bias) v = __fadd_rn(v, bias);
-          if (g.e.beta != 0.f && row_ok && jj < nvalid) v = __fmaf_rn(g.e.beta, load_dense(g.e.c_dtype, g.e.c, (size_t)(j0 + jj) * g.e.ldc + i), v);
-          r[jj] = __float_as_uint(v);
+        for (int gq = 0; gq < 4; ++gq) {
+          float2 cs = make_float2(0.f, 0.f);
+          if (mask & kExNorm) cs = *(const float2 *)&colscale[cc + 8 * gq + cp];
+#pragma unroll
+          for (int q = 0; q < 4; ++q)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+              uint32_t &x = r[16 * (q >> 1) + 4 * gq + 2 * (q & 1) + e];
+              const float sc = (mask & kExNorm) ? __fmul_rn(__fmul_rn(rowp[q], __fmul_rn(gb0, e ? cs.y : cs.x)), g.e.gf) : rowp[q];
+              float v = __fmul_rn(__uint_as_float(x), sc);
+              if (g.e.bias) v = __fadd_rn(v, bias[q]);
+              const int jj = 8 * gq + cp + e;
+              if (g.e.beta != 0.f && rb + 8 * q < gm && jj < nvalid)
+                v = __fmaf_rn(g.e.beta, load_dense(g.e.c_dtype, g.e.c, (size_t)(j0 + jj) * g.e.ldc + rb + 8 * q), v);
+              x = __float_as_uint(v);
+            }
         }
         if (mask & kExOut2) {  // second output v * w2[i] and the slice's sum of squares (rows 16 q .. 16 q + 15 in ascending order)
 #pragma unroll
-          for (int jj = 0; jj < 32; ++jj) {
-            const float v = __uint_as_float(r[jj]);
-            if (row_ok && jj < nvalid) store_dense(g.x.d2_dtype, g.x.d2, (size_t)(j0 + jj) * g.x.ldd2 + i, __fmul_rn(v, w2));
-            const float vv = __fmul_rn(v, v);
-            float sq = 0.f;
+          for (int hh = 0; hh < 2; ++hh) {
+            const int i = rb + 16 * hh;   // (m is a multiple of 16: rows i and i + 8 exist together)
+            const float w20 = i < gm ? load_dense(g.x.w2_dtype, g.x.w2, i) : 0.f, w21 = i < gm ? load_dense(g.x.w2_dtype, g.x.w2, i + 8) : 0.f;
 #pragma unroll
-            for (int q = 0; q < 16; ++q) sq = __fadd_rn(sq, __shfl_sync(0xFFFFFFFFu, vv, (lane & 16) + q));
-            if (row_ok && !(lane & 15) && jj < nvalid) g.x.sq[(size_t)(j0 + jj) * g.x.ld_sq + (i >> 4)] = sq;
+            for (int ce = 0; ce < 8; ++ce) {
+              const int jj = 8 * (ce >> 1) + cp + (ce & 1);
+              const float v0 = __uint_as_float(r[16 * hh + 4 * (ce >> 1) + (ce & 1)]), v1 = __uint_as_float(r[16 * hh + 4 * (ce >> 1) + 2 + (ce & 1)]);
+              if (i < gm && jj < nvalid) {
+                store_dense(g.x.d2_dtype, g.x.d2, (size_t)(j0 + jj) * g.x.ldd2 + i, __fmul_rn(v0, w20));
+                store_dense(g.x.d2_dtype, g.x.d2, (size_t)(j0 + jj) * g.x.ldd2 + i + 8, __fmul_rn(v1, w21));
+              }
+              const float vv0 = __fmul_rn(v0, v0), vv1 = __fmul_rn(v1, v1);
+              float sq = 0.f;
+#pragma unroll
+              for (int q = 0; q < 8; ++q) sq = __fadd_rn(sq, __shfl_sync(0xFFFFFFFFu, vv0, 4 * q + (lane & 3)));
+#pragma unroll
+              for (int q = 0; q < 8; ++q) sq = __fadd_rn(sq, __shfl_sync(0xFFFFFFFFu, vv1, 4 * q + (lane & 3)));
+              if (i < gm && lane < 4 && jj < nvalid) g.x.sq[(size_t)(j0 + jj) * g.x.ld_sq + (i >> 4)] = sq;
+            }
           }
         }
-        if (mask & kExSwiglu) {  // rows 16 q + r (gate) and 16 q + 8 + r (up) -> output row 8 q + r: 64 output rows per tile
-          // The gate lane and its up lane (lane ^ 8) share the work: the gate lane forms the even columns of their output
-          // row, the up lane the odd ones; one shuffle per column pair carries what each needs from the other.
-          const int io = (i >> 4) * 8 + (i & 7);
-          const bool gate = !(lane & 8);
-          const int odd = gate ? 0 : 1;
+        const bool glu = (mask & kExSwiglu) != 0;
+        if (glu) {  // rows 16 q + r (gate) and 16 q + 8 + r (up) -> output row 8 q + r: 64 output rows per 128-row tile
+          // (the results take the gate's registers: 16 hh + 4 gq + e)
 #pragma unroll
-          for (int q = 0; q < 16; ++q) {
-            const float v0 = __uint_as_float(r[2 * q]), v1 = __uint_as_float(r[2 * q + 1]);
-            const float got = __shfl_xor_sync(0xFFFFFFFFu, gate ? v1 : v0, 8);
-            const float h = gate ? silu_mul(v0, got) : silu_mul(got, v1);
-            if (row_ok && 2 * q + odd < nvalid) amax = fmaxf(amax, fabsf(h));
-            if (d_dtype == NVFP4A_BF16) r[q] = f32_to_bf16_bits(h);
-            else if (d_dtype == NVFP4A_FP16) r[q] = (uint32_t)__half_as_ushort(__float2half_rn(h));
-            else r[q] = __float_as_uint(h);
-          }
-          if (!tma) {
-            if (row_ok) {
+          for (int hh = 0; hh < 2; ++hh)
 #pragma unroll
-              for (int q = 0; q < 16; ++q)
-                if (2 * q + odd < nvalid) {
-                  if (esz == 2) ((uint16_t *)dptr)[(size_t)(j0 + 2 * q + odd) * g.e.ldd + io] = (uint16_t)r[q];
-                  else ((uint32_t *)dptr)[(size_t)(j0 + 2 * q + odd) * g.e.ldd + io] = r[q];
-                }
+            for (int ce = 0; ce < 8; ++ce) {
+              const int at = 16 * hh + 4 * (ce >> 1) + (ce & 1);
+              r[at] = __float_as_uint(silu_mul(__uint_as_float(r[at]), __uint_as_float(r[at + 2])));
             }
-            continue;
-          }
-          const int lr = quad * 16 + (lane >> 4) * 8 + (lane & 7);  // output row inside the tile's 64
-          for (int half = 0; half < 32 / cw; ++half) {
-            uint8_t *const st = next_box();
-            if (esz == 2) {
+        }
+        if (g.e.amax) {
 #pragma unroll
-              for (int q = 0; q < 16; ++q) ((uint16_t *)st)[(2 * q + odd) * 64 + lr] = (uint16_t)r[q];
-            } else {
+          for (int q = 0; q < 4; ++q)
 #pragma unroll
-              for (int q = 0; q < 8; ++q) ((uint32_t *)st)[(2 * q + odd) * 64 + lr] = half ? r[8 + q] : r[q];
-            }
-            fence_proxy_async_smem();
-            named_barrier(bar_id, 128);
-            if (leader && tile_ok) {
-              tma_store_2d(&tmap_d, st, tm * 64, j0 + half * cw);
-              for (int q = 0; q < peers.n; ++q) tma_store_2d(&peers.map[q], st, tm * 64, j0 + half * cw);   // the same tile into every peer's buffer
-              bulk_commit();
+            for (int ce = 0; ce < 8; ++ce)
+              if (rb + 8 * q < gm && 8 * (ce >> 1) + cp + (ce & 1) < nvalid && !(glu && (q & 1)))
+                amax = fmaxf(amax, fabsf(__uint_as_float(r[16 * (q >> 1) + 4 * (ce >> 1) + 2 * (q & 1) + (ce & 1)])));
+        }
+        const int orow = glu ? tm * 64 : tm * 128, orows = glu ? gm >> 1 : gm;   // the tile's first output row, rows of D
+        if (d_dtype == NVFP4A_FP32) {   // eight lanes write 32 contiguous bytes of a column
+          float *const d32 = (float *)dptr + (size_t)j0 * g.e.ldd + orow + (lane >> 2);
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            if (glu && (q & 1)) continue;
+            const int o = glu ? quad * 16 + 4 * q : quad * 32 + 8 * q;   // output row inside the tile, less lane / 4
+            if (rb + 8 * q < gm) {
+#pragma unroll
+              for (int ce = 0; ce < 8; ++ce) {
+                const int jj = 8 * (ce >> 1) + cp + (ce & 1);
+                if (jj < nvalid) d32[(size_t)jj * g.e.ldd + o] = __uint_as_float(r[16 * (q >> 1) + 4 * (ce >> 1) + 2 * (q & 1) + (ce & 1)]);
+              }
             }
           }
           continue;
         }
-        if (g.e.amax && row_ok) {
-#pragma unroll
-          for (int jj = 0; jj < 32; ++jj)
-            if (jj < nvalid) amax = fmaxf(amax, fabsf(__uint_as_float(r[jj])));
-        }
+        // 16-bit D: neighbouring columns into one register (in place of column 0), then 8 x 8 blocks transposed into a box of
+        // [32 tokens][64 rows] with the 128-byte swizzle (two boxes without SwiGLU)
         if (d_dtype == NVFP4A_BF16) {
-          round32_to_bf16(r);
-        } else if (d_dtype == NVFP4A_FP16) {
+          uint32_t nan = 0;
 #pragma unroll
-          for (int jj = 0; jj < 32; ++jj) r[jj] = (uint32_t)__half_as_ushort(__float2half_rn(__uint_as_float(r[jj])));
-        }
-        if (!tma) {
-          if (row_ok) {
-            if (esz == 2) {
-              uint16_t *d16 = (uint16_t *)dptr + (size_t)j0 * g.e.ldd + i;
+          for (int q = 0; q < 32; q += 2) {
+            r[q] = bf16x2_rn(__uint_as_float(r[q]), __uint_as_float(r[q + 1]));
+            nan |= (r[q] & 0x7FFF7FFFu) + 0x00010001u;   // (the hardware rounds every NaN to 0x7FFF, which nothing else gives)
+          }
+          if (nan & 0x80008000u) {
 #pragma unroll
-              for (int jj = 0; jj < 32; ++jj)
-                if (jj < nvalid) d16[(size_t)jj * g.e.ldd] = (uint16_t)r[jj];
-            } else {
-              uint32_t *d32 = (uint32_t *)dptr + (size_t)j0 * g.e.ldd + i;
-#pragma unroll
-              for (int jj = 0; jj < 32; ++jj)
-                if (jj < nvalid) d32[(size_t)jj * g.e.ldd] = r[jj];
+            for (int q = 0; q < 32; q += 2) {
+              if ((r[q] & 0x7FFFu) == 0x7FFFu) r[q] = (r[q] & 0xFFFF0000u) | 0x7FC0u;
+              if ((r[q] & 0x7FFF0000u) == 0x7FFF0000u) r[q] = (r[q] & 0xFFFFu) | 0x7FC00000u;
             }
           }
-          continue;
-        }
-        for (int half = 0; half < 32 / cw; ++half) {
-          uint8_t *const st = next_box();
-          const int rr = quad * 32 + lane;
-          if (esz == 2) {
+        } else {
 #pragma unroll
-            for (int jj = 0; jj < 32; ++jj) ((uint16_t *)st)[jj * 128 + rr] = (uint16_t)r[jj];
-          } else {
-#pragma unroll
-            for (int jj = 0; jj < 16; ++jj) ((uint32_t *)st)[jj * 128 + rr] = half ? r[16 + jj] : r[jj];
+          for (int q = 0; q < 32; q += 2) {
+            const __half2 h = __floats2half2_rn(__uint_as_float(r[q]), __uint_as_float(r[q + 1]));
+            r[q] = *reinterpret_cast<const uint32_t *>(&h);
           }
+        }
+        uint8_t *const st = next_box();
+        __syncwarp();
+        if (glu) {
+#pragma unroll
+          for (int gp = 0; gp < 2; ++gp)   // matrices: column groups 2 gp and 2 gp + 1, each 16-row half
+            stmatrix_x4_trans(st + (8 * (2 * gp + (mi >> 1)) + l7) * 128 + (((2 * quad + (mi & 1)) ^ l7) << 4), r[8 * gp], r[16 + 8 * gp], r[4 + 8 * gp],
+                              r[20 + 8 * gp]);
+        } else {
+#pragma unroll
+          for (int gq = 0; gq < 4; ++gq)   // matrices: the four 8-row groups of the warp's 32 rows
+            stmatrix_x4_trans(st + (quad >> 1) * 4096 + (8 * gq + l7) * 128 + (((4 * (quad & 1) + mi) ^ l7) << 4), r[4 * gq], r[4 * gq + 2], r[16 + 4 * gq],
+                              r[18 + 4 * gq]);
+        }
+        if (tma) {
           fence_proxy_async_smem();
           named_barrier(bar_id, 128);
           if (leader && tile_ok) {
-            tma_store_2d(&tmap_d, st, tm * 128, j0 + half * cw);
-            for (int q = 0; q < peers.n; ++q) tma_store_2d(&peers.map[q], st, tm * 128, j0 + half * cw);   // the same tile into every peer's buffer
+            for (int b = 0; b < (glu ? 1 : 2); ++b) {
+              const int o = orow + 64 * b;
+              if (o >= orows) break;
+              tma_store_2d(&tmap_d, st + b * 4096, o, j0);
+              for (int q = 0; q < peers.n; ++q) tma_store_2d(&peers.map[q], st + b * 4096, o, j0);   // the same box into every peer's buffer
+            }
             bulk_commit();
+          }
+        } else {   // D that TMA cannot store, or a group's last tokens: a thread per row
+          named_barrier(bar_id, 128);
+          const int th = quad * 32 + lane, row = glu ? th & 63 : th, step = glu ? 2 : 1;
+          if (orow + row < orows) {
+            const uint8_t *src = st + (row >> 6) * 4096 + (row & 7) * 2;
+            for (int jj = glu ? th >> 6 : 0; jj < nvalid; jj += step)
+              ((uint16_t *)dptr)[(size_t)(j0 + jj) * g.e.ldd + orow + row] = *(const uint16_t *)(src + jj * 128 + ((((row >> 3) & 7) ^ (jj & 7)) << 4));
           }
         }
       }
@@ -529,7 +579,7 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
     // ---------------- weight expansion: NVFP4 -> 16-bit floats in tensor memory ----------------
     // Two groups of four warps take the even and the odd stages of a tile; inside a group thread r owns row r of the CTA's 128 (and
     // tensor memory lane r: warp % 4 is its quadrant): a stage's 64 nibbles are two 16-byte words of the slot's swizzled row, its 4 scale bytes one word fetched a slot (four stages)
-    // ahead.  A slot goes back to the producer as soon as its words are in registers.
+    // ahead.
     const int cwarp = warp - 12, group = cwarp >> 2;
     const int row = (cwarp & 3) * 32 + lane, r7 = row & 7;
     const Fp4Operand A = g.A;
@@ -556,20 +606,19 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
       for (int sl = 0; sl < nslots; ++sl, ++isl) {
         if (sl + 1 < nslots) fetch_scales(scp, sl + 1, sc_next);
         const int rs = isl % kRaw;
-        if (!wait(&raw_full[rs], (isl / kRaw) & 1, kStWaitRaw)) goto done;
+        if (!__all_sync(0xFFFFFFFFu, wait(&raw_full[rs], (isl / kRaw) & 1, kStWaitRaw))) goto done;
         const uint8_t *src = sRaw + (size_t)rs * C::kRawBytes + row * 128;
         uint4 w[4];
 #pragma unroll
         for (int q = 0; q < 4; ++q) w[q] = *(const uint4 *)(src + (((2 * group + 4 * (q >> 1) + (q & 1)) ^ r7) << 4));
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&raw_empty[rs]);
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
           const int ks = 4 * sl + group + 2 * h;
           if (ks >= nk) break;
           const uint32_t it = it0 + ks;
           const int s = it % kA;
-          if (!wait(&a_empty[s], ((it / kA) & 1) ^ 1, kStWaitConv)) goto done;
+          // (the vote also brings the warp together again: lanes whose first poll failed come later, and the stores below are warp-wide)
+          if (!__all_sync(0xFFFFFFFFu, wait(&a_empty[s], ((it / kA) & 1) ^ 1, kStWaitConv))) goto done;
           tc_fence_after();   // the MMAs of the stage's previous round have read it
           const uint32_t dst = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + kACols + s * 32;
 #pragma unroll
@@ -589,6 +638,10 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
           __syncwarp();
           if (lane == 0) mbar_arrive_rank(&a_full[s], 0);
         }
+        // The slot goes back only now that its words have been USED: a load that is merely issued may still be queued behind the epilogue's
+        // stores when the producer's next copy lands (seen as words of the following slot in a handful of rows).
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&raw_empty[rs]);
         sc[0] = sc_next[0]; sc[1] = sc_next[1];
       }
     }
@@ -672,8 +725,8 @@ bool set_up(const GemmArgs &g, int planes, const void *act, uint64_t row_bytes, 
   const int esz = dense_bytes(g.e.d_dtype);
   const bool glu = (g.x.mask & kExSwiglu) != 0;
   const int drows = glu ? g.m / 2 : g.m;   // SwiGLU: the output has m / 2 rows, 64 per 128-row tile
-  a->d_tma = ((uintptr_t)g.e.d & 15) == 0 && ((size_t)g.e.ldd * esz) % 16 == 0 && ((size_t)drows * esz) % 16 == 0 &&
-             make_tmap_dense(td, g.e.d, esz, (uint64_t)drows, (uint64_t)g.n, (uint64_t)g.e.ldd * esz, glu ? 64 : 128, esz == 2 ? 32 : 16);
+  a->d_tma = esz == 2 && ((uintptr_t)g.e.d & 15) == 0 && ((size_t)g.e.ldd * esz) % 16 == 0 && ((size_t)drows * esz) % 16 == 0 &&
+             make_tmap_dense(td, g.e.d, esz, (uint64_t)drows, (uint64_t)g.n, (uint64_t)g.e.ldd * esz, 64, 32, 128);
   return true;
 }
 
@@ -712,7 +765,7 @@ bool gemm_w4a16_pushes(const GemmArgs &g) {
   if (g.tp.world <= 1) return false;
   const int esz = dense_bytes(g.e.d_dtype);
   const int drows = (g.x.mask & kExSwiglu) ? g.m / 2 : g.m;
-  return ((uintptr_t)g.e.d & 15) == 0 && ((size_t)g.e.ldd * esz) % 16 == 0 && ((size_t)drows * esz) % 16 == 0;
+  return esz == 2 && ((uintptr_t)g.e.d & 15) == 0 && ((size_t)g.e.ldd * esz) % 16 == 0 && ((size_t)drows * esz) % 16 == 0;
 }
 
 bool gemm_w4a16_supports(const GemmArgs &g) {
@@ -804,8 +857,7 @@ cudaError_t launch_gemm_w4a16(const GemmArgs &g, cudaStream_t s) {
     const int drows = glu ? g.m / 2 : g.m;
     for (int p = 0; p < g.tp.world; ++p) {
       if (p == g.tp.rank) continue;
-      if (!make_tmap_dense(&pm.map[pm.n], (uint8_t *)g.e.d + g.tp.delta[p], esz, (uint64_t)drows, (uint64_t)g.n, (uint64_t)g.e.ldd * esz, glu ? 64 : 128,
-                           esz == 2 ? 32 : 16))
+      if (!make_tmap_dense(&pm.map[pm.n], (uint8_t *)g.e.d + g.tp.delta[p], esz, (uint64_t)drows, (uint64_t)g.n, (uint64_t)g.e.ldd * esz, 64, 32, 128))
         return cudaErrorInvalidValue;
       ++pm.n;
     }
