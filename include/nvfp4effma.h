@@ -94,7 +94,9 @@ nvfp4a_status nvfp4a_gemm_dual(int m, int n, int k, float alpha, const nvfp4a_du
                                int ldc, const nvfp4a_tensor *D, int ldd, const nvfp4a_tensor *bias,
                                cudaStream_t stream);
 
-/* Grouped (mixture-of-experts) GEMM.  Declared for link compatibility; this build returns NVFP4A_NOT_SUPPORTED.
+/* Grouped (mixture-of-experts) GEMM: A stacks `groups` weights of m rows, group q owns the rows [seg[q], seg[q + 1]) of B and D (seg:
+ * device memory, groups + 1 non-decreasing offsets, none above `rows`); bias is stacked like A.  INT8 activations with a 16-bit D and
+ * k >= 512 run the tcgen05 kernel (the accumulation bound of nvfp4a_gemm), everything else the exact tiled order.
  * ref include/nvfp4effma.h:114 */
 nvfp4a_status nvfp4a_gemm_grouped(int groups, int m, int k, int rows, float alpha, const nvfp4a_tensor *A, int lda,
                                   const nvfp4a_tensor *B, int ldb, float beta, const nvfp4a_tensor *C, int ldc,

@@ -125,7 +125,7 @@ static nvfp4a_status dispatch(const char *fn, const GemmArgs &g, cudaStream_t st
   else if (gemv && g.k > 0 && gemv_blocked_supports(g)) { g_last_route = 6; err = launch_gemv_blocked(g, stream); }
   else if (!gemv && gemm_w4a4_supports(g)) { g_last_route = 4; err = launch_gemm_w4a4(g, stream); }
   else if ((!gemv || g.B.dtype == NVFP4A_FP16) && gemm_w4a16_supports(g)) { g_last_route = 5; err = launch_gemm_w4a16(g, stream); }
-  else if (!gemv && forced_route() != 3 && gemm_w4a8_tc_supports(g)) { g_last_route = 8; err = launch_gemm_w4a8_tc(g, stream); }
+  else if (!gemv && forced_route() != 3 && gemm_w4a8_tc_supports(g)) { g_last_route = 8; err = launch_gemm_w4a8_tc(g, nullptr, 0, stream); }
   else if (!gemv && gemm_dp4a_supports(g)) { g_last_route = 7; err = launch_gemm_dp4a(g, stream); }
   else { g_last_route = 1; err = launch_gemm_generic(g, stream); }
   if (err == cudaSuccess && g.tp.world > 1 && g_last_route != 2) {
@@ -403,8 +403,13 @@ extern "C" nvfp4a_status nvfp4a_gemm_grouped(int groups, int m, int k, int rows,
   // the checks of nvfp4a_gemm with A taken as [groups * m][k]; an empty problem returns before anything is filled in
   if (nvfp4a_status st = gemm_run(fn, m, rows, k, alpha, A, lda, B, ldb, beta, C, ldc, D, ldd, bias, none, stream, false, groups, &g)) return st;
   if (m == 0 || rows == 0) return NVFP4A_OK;
-  // Every group runs a CUDA-core kernel in the reference's tiled order: the bytes of nvfp4a_gemm's tiled kernel for that group.
-  // INT8 activations take the 128 x 128 DP4A kernel, everything else the generic one.
+  // INT8 activations with a 16-bit D and a long reduction run on the tensor cores, like nvfp4a_gemm's (within the FP32 accumulation bound;
+  // nvfp4a_b200_set_route(3) keeps them on the exact kernel).  Everything else runs a CUDA-core kernel in the reference's tiled order,
+  // the bytes of nvfp4a_gemm's tiled kernel for each group: other INT8 problems the 128 x 128 DP4A kernel, the rest the generic one.
+  if (forced_route() != 1 && forced_route() != 3 && gemm_w4a8_grouped_supports(g, groups)) {
+    g_last_route = 8;
+    return cuda_fail(launch_gemm_w4a8_tc(g, seg, groups, stream), "nvfp4a_gemm_grouped: kernel launch");
+  }
   if (forced_route() != 1 && gemm_dp4a_supports(g)) {
     g_last_route = 7;
     return cuda_fail(launch_gemm_dp4a_grouped(g, seg, groups, stream), "nvfp4a_gemm_grouped: kernel launch");

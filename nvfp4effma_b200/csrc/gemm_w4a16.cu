@@ -678,6 +678,24 @@ Plan make_plan(int rows256, int n, int planes, int pairs) {
   return best;
 }
 
+// Grouped: only the average number of tokens per group is known here; each group ends in a partial tile, half a tile on average.
+// `tiles` bounds the grid, the kernel counts the tiles itself.
+Plan make_grouped_plan(int rows256, int n, int groups, int planes, int pairs) {
+  Plan best = {0, 0, 1, 0};
+  double best_cost = 0;
+  const double avg = (double)n / groups;
+  for (int w = 256; w >= 64; w /= 2) {
+    const double tiles = rows256 * (double)groups * (avg <= w ? 1.0 : avg / w + 0.5), per = 2.0 * w * planes > 300 ? 2.0 * w * planes : 300.0;
+    const double c = (tiles <= pairs ? 1.0 : tiles / pairs + 0.5) * per;
+    if (!best.width || c < best_cost) {
+      const long long bound = (long long)rows256 * ((n + w - 1) / w + groups);
+      best_cost = c;
+      best = Plan{w, 0, 1, (int)(bound < (1 << 30) ? bound : 1 << 30)};
+    }
+  }
+  return best;
+}
+
 template <int PLANES, bool F16, bool GROUPED = false>
 cudaError_t launch_cfg(const CUtensorMap &tw, const CUtensorMap &tb, const CUtensorMap &td, const PeerMaps &pm, const W4A16Args &a, cudaStream_t s) {
   using C = Cfg<PLANES>;
@@ -707,18 +725,20 @@ cudaError_t launch_cfg(const CUtensorMap &tw, const CUtensorMap &tb, const CUten
 
 // what every launch of the kernel shares: arguments, the schedule, the maps of the weights, of the activations (`row_bytes` bytes per
 // token, `pitch` between tokens) and of D
-bool set_up(const GemmArgs &g, int planes, const void *act, uint64_t row_bytes, uint64_t pitch, W4A16Args *a, CUtensorMap *tw, CUtensorMap *tb, CUtensorMap *td) {
+bool set_up(const GemmArgs &g, int planes, int groups, const void *act, uint64_t row_bytes, uint64_t pitch, W4A16Args *a, CUtensorMap *tw, CUtensorMap *tb,
+            CUtensorMap *td) {
   memset(a, 0, sizeof *a);
   a->m = g.m; a->n = g.n; a->k = g.k;
   a->A = g.A;
   a->e = g.e; a->x = g.x;
   a->status = kernel_status_device_ptr();
   a->tag = next_launch_tag();
-  const Plan p = make_plan((g.m + 255) / 256, g.n, planes, device_sms() / 2);
+  const Plan p = groups ? make_grouped_plan((g.m + 255) / 256, g.n, groups, planes, device_sms() / 2) : make_plan((g.m + 255) / 256, g.n, planes, device_sms() / 2);
+  const uint64_t wrows = (uint64_t)g.m * (groups ? groups : 1);
   a->width = p.width; a->nfull = p.nfull; a->cut = p.cut; a->tiles = p.tiles;
   const uint64_t wtiles = (uint64_t)((g.m + 127) / 128) * g.A.ktiles;
   if (g.A.image ? !make_tmap_bytes(tw, g.A.data, 128, 128, 128, 128, wtiles, kImgTileBytes)
-                : !make_tmap_bytes(tw, g.A.data, (uint64_t)g.k / 2, (uint64_t)g.m, (uint64_t)g.A.ld / 2, 128, 1, (uint64_t)g.A.ld / 2 * g.m))
+                : !make_tmap_bytes(tw, g.A.data, (uint64_t)g.k / 2, wrows, (uint64_t)g.A.ld / 2, 128, 1, (uint64_t)g.A.ld / 2 * wrows))
     return false;
   if (!make_tmap_bytes(tb, act, row_bytes, (uint64_t)g.n, pitch, p.width / 2, 1, pitch * g.n)) return false;
   memset(td, 0, sizeof *td);
@@ -824,22 +844,34 @@ bool gemm_w4a8_tc_supports(const GemmArgs &g) {
   return true;
 }
 
-cudaError_t launch_gemm_w4a8_tc(const GemmArgs &g, cudaStream_t s) {
+// The same for nvfp4a_gemm_grouped: problems whose D is 16-bit (its rounding hides the order of the sums; an FP32 D keeps the exact block
+// sums of the DP4A kernel) and whose reduction is long enough to pay for the planes.  8 experts of 2048 x 4096 on 1100 tokens, INT8
+// quantization of the tokens included: 600 us on the DP4A kernel, 158 us here.
+bool gemm_w4a8_grouped_supports(const GemmArgs &g, int groups) {
+  return gemm_w4a8_tc_supports(g) && !g.A.image && groups <= kMaxGroups && g.k >= 512 && g.e.d_dtype != NVFP4A_FP32;
+}
+
+// seg == NULL: one weight; else `groups` stacked weights of g.m rows
+cudaError_t launch_gemm_w4a8_tc(const GemmArgs &g, const int *seg, int groups, cudaStream_t s) {
   uint16_t *planes = nullptr;
   cudaMemPool_t pool;
   cudaError_t e = planes_pool(&pool);
   if (e != cudaSuccess) return e;
   e = cudaMallocFromPoolAsync((void **)&planes, (size_t)g.n * 3 * g.k * sizeof(uint16_t), pool, s);
   if (e != cudaSuccess) return e;
-  const long long groups = (long long)g.n * (g.k >> 3);
-  w4a8_planes_kernel<<<(unsigned)((groups + 255) / 256), 256, 0, s>>>((const int8_t *)g.B.data, g.B.ld, g.B.s8, g.B.lds8, g.n, g.k, planes);
+  const long long vecs = (long long)g.n * (g.k >> 3);
+  w4a8_planes_kernel<<<(unsigned)((vecs + 255) / 256), 256, 0, s>>>((const int8_t *)g.B.data, g.B.ld, g.B.s8, g.B.lds8, g.n, g.k, planes);
   e = cudaGetLastError();
   if (e == cudaSuccess) {
     W4A16Args a;
     CUtensorMap tw, tb, td;
     PeerMaps pm;
     memset(&pm, 0, sizeof pm);
-    e = set_up(g, 3, planes, (uint64_t)g.k * 6, (uint64_t)g.k * 6, &a, &tw, &tb, &td) ? launch_cfg<3, false>(tw, tb, td, pm, a, s) : cudaErrorInvalidValue;
+    if (!set_up(g, 3, seg ? groups : 0, planes, (uint64_t)g.k * 6, (uint64_t)g.k * 6, &a, &tw, &tb, &td)) e = cudaErrorInvalidValue;
+    else if (seg) {
+      a.seg = seg; a.groups = groups;
+      e = launch_cfg<3, false, true>(tw, tb, td, pm, a, s);
+    } else e = launch_cfg<3, false>(tw, tb, td, pm, a, s);
   }
   const cudaError_t ef = cudaFreeAsync(planes, s);
   return e != cudaSuccess ? e : ef;
@@ -848,7 +880,7 @@ cudaError_t launch_gemm_w4a8_tc(const GemmArgs &g, cudaStream_t s) {
 cudaError_t launch_gemm_w4a16(const GemmArgs &g, cudaStream_t s) {
   W4A16Args a;
   CUtensorMap tw, tb, td;
-  if (!set_up(g, 1, g.B.data, (uint64_t)g.k * 2, (uint64_t)g.B.ld * 2, &a, &tw, &tb, &td)) return cudaErrorInvalidValue;
+  if (!set_up(g, 1, 0, g.B.data, (uint64_t)g.k * 2, (uint64_t)g.B.ld * 2, &a, &tw, &tb, &td)) return cudaErrorInvalidValue;
   PeerMaps pm;
   memset(&pm, 0, sizeof pm);
   if (gemm_w4a16_pushes(g)) {   // tensor parallel: the epilogue's TMA stores also go to every peer's copy of D

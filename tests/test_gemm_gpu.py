@@ -760,3 +760,52 @@ def test_w4a16_gemm_gives_the_same_bytes_every_time():
             differs.append((D != first).any())
     assert not bool(torch.stack(differs).any())
     assert kernel_status() == 0
+
+
+@pytest.mark.parametrize("seg,m,k", [([0, 1, 1, 64], 128, 512), ([0, 65, 130, 131], 130, 576), ([0, 0, 0, 257], 300, 1088), ([3, 3, 100, 400], 257, 512)])
+def test_grouped_w4a8_on_the_tensor_cores(seg, m, k):
+    """INT8 activations, 16-bit D, k >= 512: nvfp4a_gemm_grouped runs the tcgen05 kernel (route 8), every group within the bound of its own
+    GEMM; nvfp4a_b200_set_route(3) gives the DP4A kernel's bytes.  Empty groups, groups of one token, partial 64-token tiles, row tiles
+    that cross into the next group's weight, rows before seg[0] and past seg[groups] left alone, per-row globals, bias, beta * C."""
+    groups, rows = len(seg) - 1, seg[-1] + 5
+    rng = np.random.default_rng(6100 + m + k)
+    lda, ldb, ldd = k + 64, k + 64, m + 8
+    A = rand_fp4(rng, groups * m, k, ld=lda, ld_scale=k // 16 + 4, flags=O.PER_ROW, glob=0.375)
+    B = rand_q8(rng, rows, k, ld=ldb, ld_scale=k // 16 + 8)
+    bias = rand_dense(rng, L.BF16, groups * m, 3.0)
+    dA, dB, dS, dbias, dseg = DevFp4(A), dev(B.data), dev(B.scales), dev(bias), dev(np.array(seg, np.int32))
+    for dt, pad, alpha, beta in ((L.BF16, 8, 1.25, 0.5), (L.FP16, 3, 0.0078125, 0.0)):   # ldd = m + 3: D that TMA cannot store; FP16: stays in range
+        ldd = m + pad
+        Dinit = rand_dense(rng, dt, ldd * rows, 4.0)
+        for route in (0, 3):
+            old = L.lib.nvfp4a_b200_set_route(route)
+            try:
+                dD, damax = dev(Dinit), dev(np.zeros(1, np.float32))
+                tA, tB, tD, tb = dA.tensor(), tensor(dB, L.INT8, dS, B.ld_scale), tensor(dD, dt, amax=damax), tensor(dbias, L.BF16)
+                st = L.lib.nvfp4a_gemm_grouped(groups, m, k, rows, alpha, ctypes.byref(tA), lda, ctypes.byref(tB), ldb, beta, ctypes.byref(tD), ldd,
+                                               ctypes.byref(tD), ldd, ctypes.byref(tb), ctypes.c_void_p(dseg.data_ptr()), stream())
+                assert st == 0, L.lib.nvfp4a_last_error()
+                assert L.lib.nvfp4a_b200_last_route() == (8 if route == 0 else 7)
+            finally:
+                L.lib.nvfp4a_b200_set_route(old)
+            torch.cuda.synchronize()
+            raw = host(dD).view(np.uint16).reshape(rows, ldd)
+            init = Dinit.reshape(rows, ldd)
+            assert np.array_equal(raw[:, m:], init[:, m:]) and np.array_equal(raw[seg[-1]:], init[seg[-1]:]) and np.array_equal(raw[:seg[0]], init[:seg[0]])
+            for q in range(groups):
+                lo, hi = seg[q], seg[q + 1]
+                if hi == lo:
+                    continue
+                Aq = O.Fp4(m, k, ld=lda, ld_scale=A.ld_scale, flags=A.flags, scale_max=A.scale_max, glob=0.0)
+                Aq.data[:], Aq.scales[:] = A.data[q * m * lda // 2:(q + 1) * m * lda // 2], A.scales[q * m * A.ld_scale:(q + 1) * m * A.ld_scale]
+                Aq.glob[:] = A.glob[q * m:(q + 1) * m]
+                Bq = O.Q8(hi - lo, k, ld=ldb, ld_scale=B.ld_scale)
+                Bq.data[:], Bq.scales[:] = B.data[lo * ldb:hi * ldb], B.scales[lo * B.ld_scale:hi * B.ld_scale]
+                exp = O.gemm(m, hi - lo, k, Aq, Bq, D_dtype=dt, alpha=alpha, beta=beta, C=Dinit[lo * ldd:hi * ldd], C_dtype=dt, ldc=ldd, ldd=ldd,
+                             bias=bias[q * m:(q + 1) * m], bias_dtype=L.BF16, lda=lda, ldb=ldb, D_init=Dinit[lo * ldd:hi * ldd], want_ref=True)
+                got = O.to_f32(np.ascontiguousarray(raw[lo:hi, :m]).reshape(-1), dt).reshape(hi - lo, m).astype(np.float64)
+                if route == 3:
+                    assert np.array_equal(raw[lo:hi], exp["D"].reshape(hi - lo, ldd))
+                else:
+                    assert np.all(np.abs(got - exp["ref64"]) <= exp["bound"]), (q, np.max(np.abs(got - exp["ref64"]) / exp["bound"]))
+    assert kernel_status() == 0
