@@ -102,6 +102,24 @@ __device__ __forceinline__ void round32_to_bf16(uint32_t (&r)[32]) {
   }
 }
 
+// Four nibbles (the low 16 bits of w) of a block -> four 16-bit floats in two registers, value 0 in the low half of the first.  `t` holds
+// what the block's eight magnitudes become: high bytes in x (codes 0-3) and y (4-7), low bytes in z and w.  A byte permute's selector
+// nibble picks a byte with its low three bits; with its top bit set -- here the sign -- it gives that byte's sign replicated instead: 0x80
+// becomes 0xFF, so that bit 6 of each byte of `s` is the value's sign.  The sign is applied by XOR: the table's own signs (negative block
+// scales) multiply.
+__device__ __forceinline__ uint32_t byte_perm(uint32_t a, uint32_t b, uint32_t sel) {
+  uint32_t d;
+  asm("prmt.b32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(sel));
+  return d;
+}
+__device__ __forceinline__ void e2m1_expand4(uint32_t w, const uint4 &t, uint32_t &o0, uint32_t &o1) {
+  const uint32_t sel = w & 0x7777u;
+  const uint32_t s = byte_perm(0x80808080u, 0x80808080u, w);
+  const uint32_t hi = byte_perm(t.x, t.y, sel) ^ ((s << 1) & 0x80808080u), lo = byte_perm(t.z, t.w, sel);
+  o0 = byte_perm(lo, hi, 0x5140u);
+  o1 = byte_perm(lo, hi, 0x7362u);
+}
+
 // ---- block scale addressing ----------------------------------------------------------------------------------------
 // ld > 0: linear, ld scales per row.  ld < 0: swizzled 128 x 4 tiles, -ld = padded scale columns.
 struct ScalePos {

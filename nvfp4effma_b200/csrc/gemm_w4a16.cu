@@ -89,23 +89,6 @@ static_assert(128 * kRegsRest + 256 * kRegsEpi + 256 * kRegsConv <= kThreads * 9
 constexpr unsigned kStWaitFullA = 0x301, kStWaitFullB = 0x302, kStWaitEmpty = 0x303, kStWaitTmemFull = 0x304, kStWaitTmemEmpty = 0x305,
                    kStWaitConv = 0x306, kStWaitRaw = 0x307;
 
-__device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t sel) {
-  uint32_t d;
-  asm("prmt.b32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(sel));
-  return d;
-}
-// Four nibbles (the low 16 bits of w) of a block -> four 16-bit floats in two registers, value 0 in the low half of the first.  `t` holds
-// the block's eight products: high bytes in x (codes 0-3) and y (4-7), low bytes in z and w.  A permute's selector nibble picks a byte with
-// its low three bits; with its top bit set -- here the sign -- it gives that byte's sign replicated instead: 0x80 becomes 0xFF, so
-// that bit 6 of each byte of `s` is the value's sign.
-__device__ __forceinline__ void expand4(uint32_t w, const uint4 &t, uint32_t &o0, uint32_t &o1) {
-  const uint32_t sel = w & 0x7777u;
-  const uint32_t s = prmt(0x80808080u, 0x80808080u, w);
-  const uint32_t hi = prmt(t.x, t.y, sel) | ((s << 1) & 0x80808080u), lo = prmt(t.z, t.w, sel);
-  o0 = prmt(lo, hi, 0x5140u);
-  o1 = prmt(lo, hi, 0x7362u);
-}
-
 __device__ __forceinline__ uint32_t bf16x2_rn(float lo, float hi) {
   uint32_t d;
   asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(d) : "f"(hi), "f"(lo));
@@ -145,7 +128,7 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
   extern __shared__ uint8_t smem_raw[];
   uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint8_t *const sB = smem, *const sRaw = sB + kB * C::kBBytes, *const staging = sRaw + kRaw * C::kRawBytes;
-  uint4 *lut = (uint4 *)(staging + 4 * C::kStagingBytes);           // scale code -> bytes of the eight products (see expand4)
+  uint4 *lut = (uint4 *)(staging + 4 * C::kStagingBytes);           // scale code -> bytes of the eight products (see e2m1_expand4)
   float *colscale = (float *)(lut + 256);                           // RMSNorm column scales of the current token tile
   uint64_t *bars = (uint64_t *)(colscale + 256);
   uint64_t *a_full = bars, *b_full = a_full + kA, *b_empty = b_full + kB, *a_empty = PLANES == 1 ? b_empty : b_empty + kB,
@@ -628,8 +611,8 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
 #pragma unroll
             for (int q = 0; q < 4; ++q) {  // 8 values per word
               const uint4 t4 = lut[(sc[h] >> (16 * u + 8 * (q >> 1))) & 0xFF];
-              expand4(wv[q], t4, o[4 * q], o[4 * q + 1]);
-              expand4(wv[q] >> 16, t4, o[4 * q + 2], o[4 * q + 3]);
+              e2m1_expand4(wv[q], t4, o[4 * q], o[4 * q + 1]);
+              e2m1_expand4(wv[q] >> 16, t4, o[4 * q + 2], o[4 * q + 3]);
             }
             tmem_st16(dst + 16 * u, o);
           }

@@ -809,3 +809,18 @@ def test_grouped_w4a8_on_the_tensor_cores(seg, m, k):
                 else:
                     assert np.all(np.abs(got - exp["ref64"]) <= exp["bound"]), (q, np.max(np.abs(got - exp["ref64"]) / exp["bound"]))
     assert kernel_status() == 0
+
+
+@pytest.mark.parametrize("bt", [L.BF16, L.FP16])
+def test_w4a16_gemm_decodes_signed_block_scales(bt):
+    """Negative E4M3 block-scale codes are legal for the reference; the expansion to 16-bit weights keeps their sign."""
+    for i, (m, n, k) in enumerate([(200, 150, 256), (300, 33, 576)]):
+        c = Case(m, n, k, bt, L.BF16, -1, L.BF16, 1.25, 0.0, fa=SW if i else 0)
+        h = build_case(c, 6600 + i)
+        rng = np.random.default_rng(6600 + i)
+        flip = rng.integers(0, 3, h["A"].scales.size) == 0
+        h["A"].scales[flip & (h["A"].scales != 0)] |= 0x80
+        exp = oracle_case(c, h, want_ref=True)
+        got, amax = run_gemm(c, h)
+        assert L.lib.nvfp4a_b200_last_route() == 5
+        check_bound(c, h, got, amax, exp)
