@@ -639,9 +639,15 @@ done:
   }
 }
 
-// Tile width and cut for a problem of `rows256` 256-row tiles and n tokens: the width whose rounds over the SM pairs cost least, a stage
-// costing what its MMAs take (2 cycles per token and plane) but not less than its weight expansion (about 300 cycles); the tiles of
-// the last round are cut into 2 or 4 parts while the pairs can take them all at once.
+// What a stage of a tile costs in SM cycles: four MMAs per plane, measured at about 190 cycles for 256 tokens and, because the weights
+// have to reach the tensor cores whatever the tokens, no less than about 110 for 128 and for 64; never less than the expansion.
+constexpr int kNarrow = 128;   // a tile narrower than this saves nothing
+long long stage_cost(int width, int planes) {
+  const long long mma = 4ll * planes * (width > 149 ? width * 190 / 256 : 110);
+  return mma > 400 ? mma : 400;
+}
+// Tile width and cut for a problem of `rows256` 256-row tiles and n tokens: the width whose rounds over the SM pairs cost least; the tiles of
+// the last round are cut in two while the pairs can take the halves all at once.
 struct Plan { int width, nfull, cut, tiles; };
 Plan make_plan(int rows256, int n, int planes, int pairs) {
   Plan best = {0, 0, 1, 0};
@@ -649,10 +655,9 @@ Plan make_plan(int rows256, int n, int planes, int pairs) {
   for (int w = 256; w >= 64; w /= 2) {
     if (w > 64 && w / 2 >= n) continue;   // half of the width covers every token
     const int tiles = rows256 * ((n + w - 1) / w), rest = tiles % pairs;
-    auto cost = [&](int width) { return (long long)(2 * width * planes > 300 ? 2 * width * planes : 300); };
     int cut = 1;
-    while (tiles > pairs && rest && w / (2 * cut) >= 64 && rest * 2 * cut <= pairs) cut *= 2;
-    const long long c = tiles / pairs * cost(w) + (rest ? cost(w / cut) : 0);
+    while (tiles > pairs && rest && w / (2 * cut) >= kNarrow && rest * 2 * cut <= pairs) cut *= 2;
+    const long long c = tiles / pairs * stage_cost(w, planes) + (rest ? stage_cost(w / cut, planes) : 0);
     if (!best.width || c < best_cost) {
       best_cost = c;
       best = Plan{w, cut > 1 ? tiles - rest : tiles, cut, cut > 1 ? tiles - rest + rest * cut : tiles};
@@ -661,15 +666,17 @@ Plan make_plan(int rows256, int n, int planes, int pairs) {
   return best;
 }
 
-// Grouped: only the average number of tokens per group is known here; each group ends in a partial tile, half a tile on average.
-// `tiles` bounds the grid, the kernel counts the tiles itself.
+// Grouped: only the average number of tokens per group is known here, and each group ends in a tile as wide as its last tokens (in steps
+// of 64).  `tiles` bounds the grid, the kernel counts the tiles itself.
 Plan make_grouped_plan(int rows256, int n, int groups, int planes, int pairs) {
   Plan best = {0, 0, 1, 0};
-  double best_cost = 0;
-  const double avg = (double)n / groups;
+  long long best_cost = 0;
+  const int avg = (n + groups - 1) / groups;
   for (int w = 256; w >= 64; w /= 2) {
-    const double tiles = rows256 * (double)groups * (avg <= w ? 1.0 : avg / w + 0.5), per = 2.0 * w * planes > 300 ? 2.0 * w * planes : 300.0;
-    const double c = (tiles <= pairs ? 1.0 : tiles / pairs + 0.5) * per;
+    const int whole = (avg - 1) / w, last = avg - whole * w;
+    const long long tiles = (long long)rows256 * groups * (whole + 1);
+    const long long cost = whole * stage_cost(w, planes) + stage_cost((last + 63) & ~63, planes);   // of a group's tiles in one row of tiles
+    const long long c = tiles <= pairs ? stage_cost(whole ? w : (last + 63) & ~63, planes) : (long long)rows256 * groups * cost / pairs;
     if (!best.width || c < best_cost) {
       const long long bound = (long long)rows256 * ((n + w - 1) / w + groups);
       best_cost = c;
