@@ -542,7 +542,7 @@ gemm_w4a4_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
         if (PAIR) {   // the slot is free again; the tensor memory buffer must have been read by the MMAs that last used it
           __syncwarp();
           if (lane == 0) mbar_arrive(&sfs_empty[slot]);
-          if (!wait(&sf_free[b], ((it / NSF) & 1) ^ 1, kStatusWaitGather)) goto done;
+          if (!__all_sync(0xFFFFFFFFu, wait(&sf_free[b], ((it / NSF) & 1) ^ 1, kStatusWaitGather))) goto done;   // (together again for the warp-wide stores)
           tc_fence_after();
         }
         uint32_t r[16];

@@ -1,5 +1,5 @@
 // NVFP4 x NVFP4 (W4A4) GEMM on CTA pairs: tcgen05.mma.cta_group::2 kind::mxf4nvf4 on 256 x 256 tiles, the fast form of the
-// W4A4 route for large problems whose D is a 16-bit matrix that TMA can store and whose block scales lie in aligned
+// W4A4 route for large problems whose D TMA can store and whose block scales lie in aligned
 // 512-byte tiles (the GEMM-swizzled layout, or images).  Everything else runs on the single-CTA kernel (gemm_w4a4.cu).
 //
 // Why pairs: one MMA of 128 x 256 x 64 keeps an SM's tensor pipe busy for 128 cycles (measured: nvfp4a_b200_mma_ceiling), so
@@ -26,8 +26,10 @@
 //               about 27 cycles per 512-byte tile: measured)
 //   warps 8-15  epilogue (168 registers each, taken from the other eight warps by setmaxnreg): quadrant = warp % 4, column
 //               half = (warp - 8) / 4.  A warp pulls its whole 32 x 128 accumulator block into registers with four loads and
-//               hands the accumulator back at once; scaling, rounding and the two 32 x 64 box stores from its 4 KiB staging
-//               tile (128-byte TMA swizzle: conflict-free 16-byte shared-memory stores) run under the next tile's MMAs.
+//               hands the accumulator back at once; scaling, rounding and the box stores (32 tokens x 128 bytes: two for a 16-bit D,
+//               four for an FP32 one, as of weight gradients) from its 4 KiB staging tile (128-byte TMA swizzle: conflict-free 16-byte
+//               shared-memory stores) run under the next tile's MMAs.  FP32 D at 4096 x 4096 x 2048: 48 us on the
+//               single-CTA kernel, 25 here.
 // Tiles that would fill at most half of the SM pairs in the last round are cut into two 128-wide halves.
 // Every wait is bounded; a wait that gives up raises the CTA's abort flag and the kernel status word.
 //
@@ -77,6 +79,7 @@ __device__ __forceinline__ PairTile pair_tile(int t, int tiles_x, int nfull) {
 
 
 
+template <bool F32>   // FP32 D
 __global__ void __launch_bounds__(kPairThreads, 1)
 gemm_w4a4_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_y,
                       const __grid_constant__ CUtensorMap tmap_y64, const __grid_constant__ CUtensorMap tmap_sx, const __grid_constant__ CUtensorMap tmap_sy,
@@ -228,9 +231,9 @@ gemm_w4a4_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_c
     bool wide = total > 0 && pair_tile(tile_first, tiles_x, nfull).width == 256;
     for (int it = 0; it < total; ++it) {
       const int q = it % SD, s = it % S;
-      if (!wait(&sfs_full[q], (it / SD) & 1, kPStatScale)) break;
+      if (!__all_sync(0xFFFFFFFFu, wait(&sfs_full[q], (it / SD) & 1, kPStatScale))) break;   // (the vote also brings the warp together for the warp-wide stores)
       const uint8_t *src = scale_ring + q * kSlotBytes + lane * 16;
-      if (!wait(&empty[s], ((it / S) & 1) ^ 1, kPStatScale)) break;   // scale buffer s: the MMAs of the stage's previous round have read it
+      if (!__all_sync(0xFFFFFFFFu, wait(&empty[s], ((it / S) & 1) ^ 1, kPStatScale))) break;   // scale buffer s: the MMAs of the stage's previous round have read it
       tc_fence_after();
       const uint32_t sf = tmem_base + kPAccCols + s * kPSfCols + lane_base;
       // groups of four 512-byte tiles -> 16 scale columns each: the M side's; then the N side's -- 256 rows: k groups 0-1 and 2-3, per
@@ -275,14 +278,18 @@ gemm_w4a4_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_c
       const uint32_t acc_addr = acc_lanes + half * (p.width >> 1);
       const float tokp = (g_tok && tok < xm) ? g_tok[(size_t)tok * g_tok_stride] : 1.f;
       const float s_tok = __fmul_rn(__fmul_rn(s_uniform, tokp), gf);
-      // scale, amax, round, pack: 32 accumulator columns -> 64 bytes of the lane's row of the box, as four swizzled 16-byte stores
-      auto stage32 = [&](uint32_t (&r)[32], int chunk0) {
+      // scale and amax; then 32 accumulator columns -> 64 bytes (16-bit D: rounded and packed, half a box row) or 128 bytes (FP32 D: the
+      // whole box row) of the lane's row of the box, as four or eight swizzled 16-byte stores
+      auto scale32 = [&](uint32_t (&r)[32]) {
 #pragma unroll
         for (int jj = 0; jj < 32; ++jj) r[jj] = __float_as_uint(__fmul_rn(__uint_as_float(r[jj]), s_tok));
         if (amax_out) {
 #pragma unroll
           for (int jj = 0; jj < 32; ++jj) amax = fmaxf(amax, fabsf(__uint_as_float(r[jj])));
         }
+      };
+      auto stage32 = [&](uint32_t (&r)[32], int chunk0) {
+        scale32(r);
         if (d_dtype == NVFP4A_BF16) {
           round32_to_bf16(r);
         } else {
@@ -295,6 +302,11 @@ gemm_w4a4_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_c
           *(uint4 *)(row + (((chunk0 + q) ^ sw) << 4)) = make_uint4(r[b] | (r[b + 1] << 16), r[b + 2] | (r[b + 3] << 16), r[b + 4] | (r[b + 5] << 16),
                                                                   r[b + 6] | (r[b + 7] << 16));
         }
+      };
+      auto stage32_f32 = [&](uint32_t (&r)[32]) {
+        scale32(r);
+#pragma unroll
+        for (int q = 0; q < 8; ++q) *(uint4 *)(row + ((q ^ sw) << 4)) = make_uint4(r[4 * q], r[4 * q + 1], r[4 * q + 2], r[4 * q + 3]);
       };
       auto store_box = [&](int col) {   // (a box that lies outside D altogether is not stored; one that straddles the edge is clipped)
         fence_proxy_async_smem();
@@ -324,6 +336,22 @@ gemm_w4a4_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_c
       __syncwarp();
       if (lane == 0) mbar_arrive_rank(tmem_empty, 0);
       box_free();
+      if constexpr (F32) {
+        stage32_f32(r0);
+        store_box(col0);
+        box_free();
+        stage32_f32(r1);
+        store_box(col0 + 32);
+        if (wide) {
+          box_free();
+          stage32_f32(r2);
+          store_box(col0 + 64);
+          box_free();
+          stage32_f32(r3);
+          store_box(col0 + 96);
+        }
+        continue;
+      }
       stage32(r0, 0);
       stage32(r1, 4);
       store_box(col0);
@@ -353,7 +381,7 @@ static bool pair_tiled_ok(const Fp4Operand &o) { return o.image || (o.sld < 0 &&
 // Does the problem qualify, and is the pair kernel the faster choice?  (`force`: take it wherever it applies.)
 bool gemm_w4a4_pair_applies(const GemmArgs &g, bool force) {
   const int esz = dense_bytes(g.e.d_dtype);
-  if (esz != 2 || ((uintptr_t)g.e.d & 15) || ((size_t)g.e.ldd * esz) % 16 || ((size_t)g.m * esz) % 16) return false;
+  if (((uintptr_t)g.e.d & 15) || ((size_t)g.e.ldd * esz) % 16 || ((size_t)g.m * esz) % 16) return false;
   if (g.e.beta != 0.f || g.e.bias || g.e.ga_stride) return false;
   if (!pair_tiled_ok(g.A) || !pair_tiled_ok(g.B.q)) return false;
   if (force) return true;
@@ -390,12 +418,16 @@ cudaError_t launch_gemm_w4a4_pair(const GemmArgs &g, cudaStream_t s) {
   if (!nibble_map(X, a.xm, 128, &tx) || !nibble_map(Y, a.yn, 128, &ty) || !nibble_map(Y, a.yn, 64, &ty64) || !scale_map(X, a.xm, &tsx) ||
       !scale_map(Y, a.yn, &tsy))
     return cudaErrorInvalidValue;
-  if (!make_tmap_dense(&td, g.e.d, 2, (uint64_t)g.m, (uint64_t)g.n, (uint64_t)g.e.ldd * 2, 64, 32, 128)) return cudaErrorInvalidValue;
-  static std::atomic<unsigned long long> attr_set{0};
+  const int esz = dense_bytes(g.e.d_dtype);   // a box row is 128 bytes: 64 values of a 16-bit D, 32 of an FP32 one
+  if (!make_tmap_dense(&td, g.e.d, esz, (uint64_t)g.m, (uint64_t)g.n, (uint64_t)g.e.ldd * esz, 128 / esz, 32, 128)) return cudaErrorInvalidValue;
+  static std::atomic<unsigned long long> attr_sets[2];   // zero-initialised
+  const bool f32 = esz == 4;
+  auto *const kern = f32 ? gemm_w4a4_pair_kernel<true> : gemm_w4a4_pair_kernel<false>;
+  std::atomic<unsigned long long> &attr_set = attr_sets[f32];
   int dev = 0;
   cudaGetDevice(&dev);
   if (!(attr_set.load() >> (dev & 63) & 1)) {
-    const cudaError_t e = cudaFuncSetAttribute(gemm_w4a4_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairSmem);
+    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairSmem);
     if (e != cudaSuccess) return e;
     attr_set.fetch_or(1ull << (dev & 63));
   }
@@ -416,7 +448,7 @@ cudaError_t launch_gemm_w4a4_pair(const GemmArgs &g, cudaStream_t s) {
   attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr; cfg.numAttrs = pdl_enabled() ? 2 : 1;
-  return cudaLaunchKernelEx(&cfg, gemm_w4a4_pair_kernel, tx, ty, ty64, tsx, tsy, td, a);
+  return cudaLaunchKernelEx(&cfg, kern, tx, ty, ty64, tsx, tsy, td, a);
 }
 
 }  // namespace nvb
