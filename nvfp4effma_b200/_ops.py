@@ -67,6 +67,11 @@ def _scale_shape(rows, cols, flags):
     return A.padded_scale_shape(rows, cols) if flags & L.SCALES_SWIZZLED else (rows, cols // 16)
 
 
+def _has_scale_padding(rows, cols, flags):
+    """Whether the scale buffer holds entries no kernel writes (they have to read zero)."""
+    return bool(flags & L.SCALES_SWIZZLED) and (rows % 128 != 0 or (cols // 16) % 4 != 0)
+
+
 def _need_cols16(cols):
     if cols % 16:
         raise ValueError(f"{cols} values per row: NVFP4 / INT8 blocks hold 16, so the last dimension must be a multiple of 16")
@@ -84,13 +89,13 @@ def _quantize_ex_outputs(x, rowwise, columnwise, flags, compute_amax, want_amax,
     per_row = bool(flags & L.GLOBAL_PER_ROW)
     out = [None] * 7
     if rowwise:
-        out[0], out[1] = _u8((rows, cols // 2), x), _u8(_scale_shape(rows, cols, flags), x, zero=fill)
-        if compute_amax:
-            out[4] = torch.zeros(rows if per_row else 1, dtype=torch.float32, device=x.device)
+        out[0], out[1] = _u8((rows, cols // 2), x), _u8(_scale_shape(rows, cols, flags), x, zero=fill and _has_scale_padding(rows, cols, flags))
+        if compute_amax:   # (stored by the call, unless there is nothing to measure)
+            out[4] = (torch.empty if rows * cols else torch.zeros)(rows if per_row else 1, dtype=torch.float32, device=x.device)
     if columnwise:
-        out[2], out[3] = _u8((cols, rows16 // 2), x, zero=fill and rows16 != rows), _u8(_scale_shape(cols, rows16, flags), x, zero=fill)
+        out[2], out[3] = _u8((cols, rows16 // 2), x, zero=fill and rows16 != rows), _u8(_scale_shape(cols, rows16, flags), x, zero=fill and _has_scale_padding(cols, rows16, flags))
         if compute_amax:
-            out[5] = _one_float(x)
+            out[5] = (torch.empty if rows * cols else torch.zeros)(1, dtype=torch.float32, device=x.device)
     if want_amax:
         out[6] = _one_float(x)
     return out, rows16
@@ -163,7 +168,7 @@ def _transpose_meta(data, scales, flags, scale_max, cols):
 @_op("transpose").cuda
 def _transpose(data, scales, flags, scale_max, cols):
     rows = data.shape[0]
-    out, out_scales = _u8((cols, rows // 2), data), _u8(_scale_shape(cols, rows, flags), data, zero=True)
+    out, out_scales = _u8((cols, rows // 2), data), _u8(_scale_shape(cols, rows, flags), data, zero=_has_scale_padding(cols, rows, flags))
     f = flags & ~L.GLOBAL_PER_ROW
     src, ld, _keep = A.fp4_tensor(data, scales, None, f, scale_max)
     dst = L.Tensor(A.addr(out), L.NVFP4, A.addr(out_scales), 0, None, None, f, scale_max)

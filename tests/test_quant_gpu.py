@@ -238,3 +238,14 @@ def test_one_read_kernel_equals_the_two_launch_path(dtype, flags, lds_pad, rows,
         assert np.array_equal(outs[0][0], other[0]) and np.array_equal(outs[0][1], other[1]) and outs[0][2:] == other[2:]
     xr = O.to_f32(O.from_f32(x, dtype), dtype).reshape(rows, lds)[:, :cols]
     assert outs[0][2] == float(np.abs(xr).max()) == outs[0][3]
+
+
+@pytest.mark.parametrize("flags,compute", [(0, False), (AM | SW, True), (UE | AM, True)])
+@pytest.mark.parametrize("dtype", [L.BF16, L.FP16, L.FP32])
+def test_both_directions_from_one_read_at_the_edges_of_its_tiles(dtype, flags, compute):
+    """Rowwise and columnwise 1 x 16 blocks without 4over6 take the one-read kernel: 64-row and (the last shape) 256-row tiles of 64
+    columns, with every kind of remainder, against the oracle byte for byte."""
+    for i, (rows, cols) in enumerate([(1, 16), (16, 48), (63, 64), (65, 80), (80, 1040), (257, 128), (2064 + 5, 2320)]):
+        if i == 6 and dtype != L.BF16 and flags:
+            continue
+        run_quant(dtype, rows, cols, ("one read", 1, 0, flags, 0, compute, True), 700 + i)
