@@ -795,6 +795,69 @@ __global__ void __launch_bounds__(256) dequant_kernel(QOut q, uint8_t *__restric
   if (stat) warp_amax_commit(stat, mx);
 }
 
+// 16-bit destination, no amax requested: a block's eight magnitudes become eight 16-bit results (the same products, rounded once), whose
+// bytes the nibbles then select (e2m1_expand4): 3.7 instructions per value where decoding, two multiplies and the rounding of every
+// value took about 12, and no division per block.  A warp takes 32 neighbouring blocks of four rows, so that four 8-byte loads per lane
+// are in flight and a row's 1 KiB leaves as two 16-byte stores per lane.  4096 x 14336 -> BF16: 54 us before, 32 us (4.7 TB/s) here.
+template <int T>
+__global__ void __launch_bounds__(256) dequant_rows_kernel(QOut q, uint8_t *__restrict__ dst, int ldd, int rows, int bpr) {
+  const int lane = threadIdx.x & 31, upr = (bpr + 31) >> 5, groups = (rows + 3) >> 2;
+  const int nwarps = gridDim.x * (blockDim.x >> 5);
+  const ScalePos sp{q.sld};
+  const bool ue = q.ue != 0, amax_mode = q.amax_mode != 0;
+  const float finv = 1.0f / (6.f * q.smax);
+  const float g0 = q.g ? q.g[0] : (amax_mode ? 6.f * q.smax : 1.f);
+  for (long long u = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); u < (long long)groups * upr; u += nwarps) {
+    const int rg = (int)(u / upr), c = (int)(u - (long long)rg * upr) * 32 + lane, r0 = 4 * rg;
+    if (c >= bpr) continue;
+    uint2 w[4];
+    uint32_t code[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int r = min(r0 + i, rows - 1);
+      w[i] = __ldcs((const uint2 *)(q.data + (size_t)r * (q.ld >> 1) + 8 * c));
+      code[i] = q.sc[sp.at(r, c)];
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int r = r0 + i;
+      if (r >= rows) break;
+      const float sb = scale_to_f32(code[i], ue), gv = q.per_row ? q.g[r] : g0;
+      const float f = amax_mode ? __fmul_rn(__fmul_rn(sb, gv), finv) : gv;   // amax: e * f; decode factor: (e * sb) * f
+      uint32_t h[4];
+#pragma unroll
+      for (int p = 0; p < 4; ++p) {
+        const float e0 = p == 0 ? 0.f : p == 1 ? 1.f : p == 2 ? 2.f : 4.f, e1 = p == 0 ? 0.5f : p == 1 ? 1.5f : p == 2 ? 3.f : 6.f;
+        const float v0 = __fmul_rn(amax_mode ? e0 : __fmul_rn(e0, sb), f), v1 = __fmul_rn(amax_mode ? e1 : __fmul_rn(e1, sb), f);
+        if (T == NVFP4A_BF16) asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(h[p]) : "f"(v1), "f"(v0));
+        else { const __half2 t = __floats2half2_rn(v0, v1); h[p] = *reinterpret_cast<const uint32_t *>(&t); }
+      }
+      const uint4 t = make_uint4(byte_perm(h[0], h[1], 0x7531u), byte_perm(h[2], h[3], 0x7531u), byte_perm(h[0], h[1], 0x6420u), byte_perm(h[2], h[3], 0x6420u));
+      uint32_t o[8];
+      e2m1_expand4(w[i].x, t, o[0], o[1]);
+      e2m1_expand4(w[i].x >> 16, t, o[2], o[3]);
+      e2m1_expand4(w[i].y, t, o[4], o[5]);
+      e2m1_expand4(w[i].y >> 16, t, o[6], o[7]);
+      if (!(fabsf(f) <= kFltMax)) {   // a global of Inf or NaN makes NaNs, whose encoding has no sign: value by value, as dequant_kernel
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          uint32_t hv[2];
+#pragma unroll
+          for (int j = 0; j < 2; ++j) {
+            const float e = e2m1_to_f32(((k < 4 ? w[i].x : w[i].y) >> (4 * (2 * (k & 3) + j))) & 15u);
+            const float v = __fmul_rn(amax_mode ? e : __fmul_rn(e, sb), f);
+            hv[j] = T == NVFP4A_BF16 ? f32_to_bf16_bits(v) : (uint32_t)__half_as_ushort(__float2half_rn(v));
+          }
+          o[k] = hv[0] | (hv[1] << 16);
+        }
+      }
+      uint4 *p = (uint4 *)(dst + ((size_t)r * ldd + 16 * c) * 2);
+      __stcs(p, make_uint4(o[0], o[1], o[2], o[3]));
+      __stcs(p + 1, make_uint4(o[4], o[5], o[6], o[7]));
+    }
+  }
+}
+
 // ---- scale layout conversion: one thread per scale of the padded swizzled matrix ----------------------------------------------
 __global__ void swizzle_kernel(const uint8_t *__restrict__ src, uint8_t *__restrict__ dst, int ld, int rows, int cols16, int sc, int to_swz) {
   const ScalePos sp{-sc};
@@ -1073,6 +1136,12 @@ extern "C" nvfp4a_status nvfp4a_dequantize(const nvfp4a_tensor *src, int lds, co
   if (nvfp4a_status st = check_device()) return st;
   const QOut q = make_qout(src, lds, sld);
   const int bpr = cols / 16;
+  if (dst->dtype != NVFP4A_FP32 && !dst->amax) {
+    const int grid = grid_for((long long)((rows + 3) / 4) * ((bpr + 31) / 32) * 32);
+    if (dst->dtype == NVFP4A_BF16) dequant_rows_kernel<NVFP4A_BF16><<<grid, 256, 0, stream>>>(q, (uint8_t *)dst->data, ldd, rows, bpr);
+    else dequant_rows_kernel<NVFP4A_FP16><<<grid, 256, 0, stream>>>(q, (uint8_t *)dst->data, ldd, rows, bpr);
+    return cuda_fail(cudaGetLastError(), "nvfp4a_dequantize: kernel launch");
+  }
   by_dense(dst->dtype, [&](auto tc) {
     dequant_kernel<decltype(tc)::value><<<grid_for((long long)rows * bpr), 256, 0, stream>>>(q, (uint8_t *)dst->data, ldd, rows, bpr, dst->amax);
   });

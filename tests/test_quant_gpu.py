@@ -249,3 +249,33 @@ def test_both_directions_from_one_read_at_the_edges_of_its_tiles(dtype, flags, c
         if i == 6 and dtype != L.BF16 and flags:
             continue
         run_quant(dtype, rows, cols, ("one read", 1, 0, flags, 0, compute, True), 700 + i)
+
+
+@pytest.mark.parametrize("flags", [0, AM | SW, UE | AM, PR])
+@pytest.mark.parametrize("dtype", [L.BF16, L.FP16])
+def test_dequantize_by_table_equals_dequantize_value_by_value(dtype, flags):
+    """A 16-bit destination without amax takes the table kernel; with amax the value-by-value one.  Same bytes for every nibble under every
+    scale code (negative E4M3 codes included) and globals from 0 over subnormal to Inf and NaN, at the edges of the 4-row,
+    32-block units; the finite case also against the oracle."""
+    rng = np.random.default_rng(77)
+    from util import rand_fp4, DevFp4
+    for rows, cols, pad in ((1, 16, 0), (4, 512, 16), (5, 528, 0), (130, 1056, 48)):
+        for gv in (0.375, 0.0, 1e-40, 3e38, float("inf"), float("nan"), -2.5):
+            h = rand_fp4(rng, rows, cols, ld=cols + 32, ld_scale=cols // 16 + 3, flags=flags, glob=0.375)
+            if not flags & UE:
+                h.scales[:] = rng.integers(0, 256, h.scales.size)
+                h.scales[(h.scales & 0x7F) == 0x7F] = 0x01   # no NaN codes
+            h.glob[:] = gv
+            d = DevFp4(h)
+            out = []
+            for with_amax in (False, True):
+                y = torch.full((rows * (cols + pad),), 0x55, dtype=torch.int16, device="cuda")
+                am = dev(np.zeros(1, np.float32))
+                src, dst = d.tensor(), tensor(y, dtype, amax=am if with_amax else None)
+                L.check(L.lib.nvfp4a_dequantize(ctypes.byref(src), h.ld, ctypes.byref(dst), cols + pad, rows, cols, stream()))
+                torch.cuda.synchronize()
+                out.append(host(y).view(np.uint16).reshape(rows, cols + pad))
+            assert np.array_equal(out[0], out[1]), (rows, cols, gv)
+            if gv == 0.375 and flags & UE:
+                want, _ = O.dequantize(h, dtype)
+                assert np.array_equal(O.to_f32(np.ascontiguousarray(out[0][:, :cols]).reshape(-1), dtype).reshape(rows, cols), want)
