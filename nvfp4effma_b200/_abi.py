@@ -75,27 +75,6 @@ def fp4_tensor(data, scales, glob, flags, scale_max, amax=None):
     return L.Tensor(addr(data), L.NVFP4, addr(scales), pitch, addr(glob), addr(amax), flags, scale_max), 2 * data.stride(0), (data, scales, glob)
 
 
-def int8_tensor(q, scales):
-    """(struct, pitch, keep-alive) of INT8 activations with an FP32 scale per 16 values."""
-    q = matrix(q, 64, "int8 activations")
-    scales = scales.contiguous()
-    if scales.data_ptr() & 15 or scales.stride(0) % 4:
-        wide = torch.zeros((scales.shape[0], -(-scales.shape[1] // 4) * 4), dtype=torch.float32, device=scales.device)
-        wide[:, :scales.shape[1]] = scales
-        scales = wide
-    return L.Tensor(addr(q), L.INT8, addr(scales), scales.stride(0), None, None, 0, 0), q.stride(0), (q, scales)
-
-
-def activation_tensor(x, scales, glob, flags, scale_max):
-    """The B operand of a GEMM call from whatever the caller holds: uint8 = NVFP4, int8 = INT8 + FP32 scales, else dense."""
-    if x.dtype == torch.uint8:
-        return fp4_tensor(x, scales, glob, flags, scale_max)
-    if x.dtype == torch.int8:
-        return int8_tensor(x, scales)
-    x = matrix(x, 64, "activations")
-    return dense_tensor(x), x.stride(0), (x,)
-
-
 _workspace_of = {}
 
 

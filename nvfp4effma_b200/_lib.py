@@ -45,6 +45,15 @@ if not os.path.exists(LIB_PATH):
     raise ImportError(f"{LIB_PATH} is missing: build it with `python -m nvfp4effma_b200.build` (nvcc, sm_100a). "
                       "There is no CPU or PyTorch fallback.")
 lib = C.CDLL(LIB_PATH)
+_TORCH_LIB_PATH = os.path.join(_HERE, "libnvfp4effma_torch.so")
+
+
+def torch_lib_path():
+    """The library with the torch operators' CUDA kernels; there is no fallback for it either."""
+    if not os.path.exists(_TORCH_LIB_PATH):
+        raise ImportError(f"{_TORCH_LIB_PATH} is missing: build it with `python -m nvfp4effma_b200.build`.")
+    return _TORCH_LIB_PATH
+
 
 _T, _E, _i, _f, _v, _s = C.POINTER(Tensor), C.POINTER(Epilogue), C.c_int, C.c_float, C.c_void_p, C.c_void_p
 _GEMM = [_i, _i, _i, _f, _T, _i, _T, _i, _f, _T, _i, _T, _i, _T]

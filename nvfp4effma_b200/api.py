@@ -97,8 +97,10 @@ def quantize(x: torch.Tensor, global_scale: Optional[torch.Tensor] = None, *, am
         extra = {"amax": glob} if measured else {"global_scale": glob}
         return NVFP4Tensor(data, codes, scale_max=bound, swizzled=swizzled, ue5m3=ue5m3, cols=ncols, block=_BLOCKS[block], **extra)
 
-    lead = tuple(x.shape[:-1])
-    result = build(d_row.reshape(*lead, cols // 2), s_row if swizzled else s_row.reshape(*lead, cols // 16), g_row if measured else given, cols)
+    if x.dim() != 2:
+        lead = tuple(x.shape[:-1])
+        d_row, s_row = d_row.reshape(*lead, cols // 2), s_row if swizzled else s_row.reshape(*lead, cols // 16)
+    result = build(d_row, s_row, g_row if measured else given, cols)
     if columnwise:
         result.columnwise = build(d_col, s_col, g_col if measured else given, rows)
     return result
@@ -168,9 +170,11 @@ def _activations(x, K: int, mode: str) -> _Activations:
     if isinstance(x, Int8Tensor):
         return _from_int8(x, K)
     lead = tuple(x.shape[:-1])
-    matrix = x.reshape(-1, K)
+    matrix = _as_matrix(x)
     if mode == "int8":
-        return _from_int8(quantize_int8(matrix), K)._replace(lead=lead, result_dtype=x.dtype)
+        _dense_input(matrix)
+        q, s = ops.quantize_int8(matrix)
+        return _Activations("int8", q, s, None, 0, 0, lead, x.dtype)
     if mode == "nvfp4":
         return _from_fp4(quantize(matrix), K, lead, x.dtype)
     return _Activations("dense", matrix, None, None, 0, 0, lead, x.dtype)
@@ -221,7 +225,7 @@ def _run(a: _Activations, w: Fp4Operand, image, N, K, bias, out_dtype, out, alph
         else:
             y, seen = out2d, ops.linear_out(*head, out2d, alpha, beta, want, image)
     _raise_amax(amax_out, seen)
-    return out if out is not None else y.reshape(*a.lead, N)
+    return out if out is not None else y if len(a.lead) == 1 else y.reshape(*a.lead, N)
 
 
 def linear(x: Union[torch.Tensor, NVFP4Tensor, Int8Tensor], weight, bias: Optional[torch.Tensor] = None, *, act: str = "auto",
