@@ -116,11 +116,13 @@ static nvfp4a_status dispatch(const char *fn, const GemmArgs &g, cudaStream_t st
     // GEMV only waits, so with bit 1 unset either may run and the caller's nvfp4a_b200_tp_gather_post follows.
     if (!(gemv && gemv_supports(g))) return fail(NVFP4A_NOT_SUPPORTED, "%s: the deferred tensor-parallel form takes 1 to 8 BF16 activation vectors", fn);
     if (!(g.tp.deferred & 2) && g.k > 0 && forced_route() != 2 && gemv_fp4_supports(g)) { g_last_route = 3; return cuda_fail(launch_gemv_fp4(g, stream), fn); }
+    if (!(g.tp.deferred & 2) && g.k > 0 && forced_route() != 2 && gemv_fp4_n8_supports(g)) { g_last_route = 3; return cuda_fail(launch_gemv_fp4_n8(g, stream), fn); }
     g_last_route = 2;
     return cuda_fail(launch_gemv(g, stream), fn);
   }
   if (forced_route() == 1) { g_last_route = 1; err = launch_gemm_generic(g, stream); }
   else if (gemv && g.k > 0 && forced_route() != 2 && gemv_fp4_supports(g)) { g_last_route = 3; err = launch_gemv_fp4(g, stream); }
+  else if (gemv && g.k > 0 && forced_route() != 2 && gemv_fp4_n8_supports(g)) { g_last_route = 3; err = launch_gemv_fp4_n8(g, stream); }
   else if (gemv && gemv_supports(g)) { g_last_route = 2; err = launch_gemv(g, stream); }
   else if (gemv && g.k > 0 && gemv_blocked_supports(g)) { g_last_route = 6; err = launch_gemv_blocked(g, stream); }
   else if (!gemv && gemm_w4a4_supports(g)) { g_last_route = 4; err = launch_gemm_w4a4(g, stream); }

@@ -508,6 +508,7 @@ gemv_fp4_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
 
 static std::atomic<int> g_gemv_splits{0};  // 0 = automatic
 void set_gemv_fp4_splits(int s) { g_gemv_splits = s; }
+int gemv_fp4_pinned_splits() { return g_gemv_splits.load(); }
 
 // splits: power of two, at most 8 and nk; every CTA's k range is at most kMaxChunks chunks (its pieces' shared memory).
 // Pinned (nvfp4a_b200_set_gemv_splits): that value if the problem can use it.  Automatic: this kernel pays about 5 us of

@@ -69,6 +69,8 @@ cudaError_t launch_gemv(const GemmArgs &g, cudaStream_t s);          // n <= 8: 
 bool gemv_supports(const GemmArgs &g);
 cudaError_t launch_gemv_fp4(const GemmArgs &g, cudaStream_t s);      // n <= 2: weights straight into tcgen05 kind::mxf4nvf4, activations as FP4 digit planes
 bool gemv_fp4_supports(const GemmArgs &g);
+cudaError_t launch_gemv_fp4_n8(const GemmArgs &g, cudaStream_t s);   // the same for 3 <= n <= 8
+bool gemv_fp4_n8_supports(const GemmArgs &g);
 void set_gemv_fp4_splits(int s);
 cudaError_t launch_gemv_blocked(const GemmArgs &g, cudaStream_t s);  // n <= 8, INT8 or NVFP4 activations: exact DP4A block sums
 bool gemv_blocked_supports(const GemmArgs &g);

@@ -1,4 +1,4 @@
-"""The FP4 tensor-core GEMV (n <= 2 BF16 activation vectors, weights fed to tcgen05 as stored, activations as FP4 digit
+"""The FP4 tensor-core GEMV (BF16 activation vectors: a kernel for n <= 2, another for 3 <= n <= 8; weights fed to tcgen05 as stored, activations as FP4 digit
 planes) against the CPU oracle: plain epilogue within the FP32-accumulation bound, extended epilogue bit for bit given the
 kernel's own accumulators -- the checks of test_gemm_gpu / test_epilogue_gpu, with the kernel pinned by
 nvfp4a_b200_set_gemv_splits and its use confirmed by nvfp4a_b200_last_route."""
@@ -181,6 +181,90 @@ def test_plain_operand_with_linear_scales(pin):
         h["A"] = rand_fp4(rng, m, k, ld=h["lda"], ld_scale=k // 16, glob=0.375)   # compact scale rows: pitch k / 16, a multiple of 16
         exp = oracle_case(c, h, want_ref=True)
         got, amax = run_gemm(c, h)
+        assert L.lib.nvfp4a_b200_last_route() == FP4_GEMV, c
+        check_bound(c, h, got, amax, exp)
+    assert kernel_status() == 0
+
+
+@pytest.mark.parametrize("splits", [1, 2, 4, 8])
+@pytest.mark.parametrize("layout", ["image", "swizzled", "linear"])
+def test_three_to_eight_activation_vectors(pin, splits, layout):
+    """The digit planes of up to eight tokens fill the MMA's 128 rows: every n from 3 to 8, all cuts of k (at most seven or fourteen 256-value
+    chunks per CTA), row remainders, and matrices with more 256-row tiles than clusters run at once, whose clusters take two tiles."""
+    from util import rand_fp4
+    pin(splits)
+    sizes = [(77, 3, 2048), (300, 8, 256 * splits), (515, 5, 1536 if splits < 8 else 2048), (1100, 4, 256 * (14 if splits == 1 else splits + 1)), (256, 7, 256 * 7 * splits),
+             (33, 6, 2304 if splits > 1 else 1792)]
+    if splits == 8:
+        sizes.append((4096 + 300, 8, 2048))       # 18 tiles on 15 clusters
+    if splits == 4:
+        sizes.append((8704 + 200, 6, 1024))       # 35 tiles on 33 clusters
+    for i, (m, n, k) in enumerate(sizes):
+        c = Case(m, n, k, L.BF16, OUTS[i % 3], OUTS[i % 3] if i % 2 else -1, L.BF16 if i % 2 else -1, 1.25 if i % 2 else 1.0, 0.5 if i % 2 else 0.0,
+                 fa=SW if layout == "swizzled" else 0)
+        h = build_case(c, 1200 + 10 * splits + i)
+        if layout == "linear":
+            h["A"] = rand_fp4(np.random.default_rng(i), m, k, ld=h["lda"], ld_scale=-(-k // 256) * 16, glob=0.375)
+        exp = oracle_case(c, h, want_ref=True)
+        got, amax = run_tc(c, h, gemv=True) if layout == "image" else run_gemm(c, h)
+        assert L.lib.nvfp4a_b200_last_route() == FP4_GEMV, c
+        check_bound(c, h, got, amax, exp)
+    assert kernel_status() == 0
+
+
+@pytest.mark.parametrize("linear", [False, True])
+def test_eight_vectors_of_which_one_does_not_fit_the_digit_planes(pin, linear):
+    """One token spread over 2^-60 .. 1: the CTAs that meet it consume the weight ring on the CUDA cores, two tiles each."""
+    from util import rand_fp4
+    pin(8)
+    m, n, k = 4096 + 300, 8, 2048
+    c = Case(m, n, k, L.BF16, L.FP32, L.FP32, -1, 1.0, 0.0, fa=0 if linear else SW)
+    h = build_case(c, 1300)
+    rng = np.random.default_rng(1301)
+    if linear:
+        h["A"] = rand_fp4(rng, m, k, ld=h["lda"], ld_scale=k // 16, glob=0.375)
+    x = rng.standard_normal((n, h["ldb"])).astype(np.float32)
+    x[5, :700] *= np.exp2(-rng.integers(0, 61, 700)).astype(np.float32)
+    h["B"] = O.Dense(L.BF16, O.from_f32(x.reshape(-1), L.BF16), h["ldb"])
+    exp = oracle_case(c, h, want_ref=True)
+    got, amax = run_gemm(c, h)
+    assert L.lib.nvfp4a_b200_last_route() == FP4_GEMV
+    check_bound(c, h, got, amax, exp)
+    assert kernel_status() == 0
+
+
+def test_extended_epilogue_of_several_vectors(pin):
+    v = 0
+    for splits, (m, n, k) in [(2, (64, 3, 512)), (4, (1024, 8, 1024)), (8, (528, 5, 2304)), (1, (4096, 4, 1024)), (8, (4096 + 256, 8, 2048))]:
+        pin(splits)
+        for mask in range(1, 6):
+            glu = bool(mask & 2)
+            run_case(m, n, k, L.BF16, L.FP32 if v % 2 else L.BF16, mask, (not glu) and v % 3 == 1, (not glu) and v % 4 == 2, True)
+            assert L.lib.nvfp4a_b200_last_route() == FP4_GEMV
+            v += 1
+    assert kernel_status() == 0
+
+
+@pytest.mark.parametrize("layout", ["image", "swizzled", "linear"])
+def test_negative_block_scales_of_several_vectors(pin, layout):
+    """Negative E4M3 block scales are legal for the reference: they keep their sign on the FP4 tensor cores, whose scales are unsigned, and
+    where the CUDA cores take over (the last size, a token spread over 2^-60 .. 1)."""
+    from util import rand_fp4
+    for i, (splits, m, n, k) in enumerate([(1, 300, 5, 768), (2, 515, 3, 1024), (8, 4096 + 300, 8, 2048), (4, 300, 4, 1024)]):
+        pin(splits)
+        c = Case(m, n, k, L.BF16, L.FP32, -1, L.BF16, 1.25, 0.0, fa=SW if layout == "swizzled" else 0)
+        h = build_case(c, 1400 + i)
+        rng = np.random.default_rng(1400 + i)
+        if layout == "linear":
+            h["A"] = rand_fp4(rng, m, k, ld=h["lda"], ld_scale=k // 16, glob=0.375)
+        flip = rng.integers(0, 3 if i else 200, h["A"].scales.size) == 0
+        h["A"].scales[flip & (h["A"].scales != 0)] |= 0x80
+        if i == 3:
+            x = rng.standard_normal((n, h["ldb"])).astype(np.float32)
+            x[2, :700] *= np.exp2(-rng.integers(0, 61, 700)).astype(np.float32)
+            h["B"] = O.Dense(L.BF16, O.from_f32(x.reshape(-1), L.BF16), h["ldb"])
+        exp = oracle_case(c, h, want_ref=True)
+        got, amax = run_tc(c, h, gemv=True) if layout == "image" else run_gemm(c, h)
         assert L.lib.nvfp4a_b200_last_route() == FP4_GEMV, c
         check_bound(c, h, got, amax, exp)
     assert kernel_status() == 0
