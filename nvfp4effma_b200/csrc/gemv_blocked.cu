@@ -1,14 +1,23 @@
 // Decode GEMV for block-scaled activations: D[m x n] = A[m x k] (NVFP4) * B[n x k]^T with 1 <= n <= 8 and B either INT8 with one
 // FP32 scale per 16 values (W4A8) or NVFP4 (W4A4).  Per output and 16-block the kernel forms the EXACT integer sum of
-// (2 a) * b (DP4A on weights expanded to 2 * e2m1, activations as int8 / 2 * e2m1), then acc = fma(p * sa, sb, acc) in FP32
+// (2 a) * b (weights expanded to 2 * e2m1, activations as int8 / 2 * e2m1), then acc = fma(p * sa, sb, acc) in FP32
 // and a final * 1/2 (INT8) or * 1/4 (NVFP4) -- the arithmetic of the reference's blocked GEMV
 // (src/gemv_nvfp4effma.cuh:26-234 there); the order of the FP32 additions over k is this kernel's own, so results agree
 // with the exact definition within the FP32 accumulation bound.
 //
-// One CTA owns 32 (or, for matrices of few rows, 16) consecutive rows; the activations (int8, n x k bytes) and their block scales (FP32) are staged once per
-// CTA in shared memory.  A warp takes a row at a time: lane l reads the 16-byte weight chunks l, l + 32, ... of the row
-// (two blocks each), so a warp load covers 512 contiguous bytes; the n <= 8 dot products of a chunk reuse its decoded
-// weights.  The lanes' sums are added by an xor butterfly; the CTA's 32 x n results then run the plain or extended epilogue.
+// The integer sums come from mma.sync.m16n8k32 (s8): sixteen weight rows against eight columns.  So that every 16-block keeps a sum of its own
+// while the weights are read as they lie (lane l of a quad holds 16-byte chunk l -- two blocks -- of rows g and g + 8), the columns are
+// (quad lane, vector) pairs: column 2 l + j holds vector j's values in the k positions of lane l's chunk and zeros in the other lanes'.
+// Two MMAs (a block is two words of eight nibbles) then give lane l the sums of ITS block for two vectors, and its own block scales apply.
+// (DP4A instead: eight times as many instructions at a fraction of the rate: 14336 x 4096, four vectors, same loads: 26.5 us.)
+//
+// A tile is G groups of 16 rows; S warps (at most 8) share a group and take its 256-value units in turn.  CTAs are persistent: the activations (int8,
+// n x k bytes) and their block scales (FP32) are staged once per CTA, and a warp's next unit (2 KiB) -- of the next tile, at a tile's end -- is in
+// flight while it computes one.  The lanes' and warps' sums are added in a fixed order, then the tile runs the plain or extended epilogue.
+//
+// What bounds it: instruction issue (decoding: 11 instructions per 8 weights) and the loads in flight (registers: 16 warps per SM).
+// 14336 x 4096 with 1 / 4 / 8 vectors: 27.5 / 32.1 / 39.0 us with a warp per four rows, DP4A and no prefetch; 15.9 / 19.9 / 28.2 us here
+// (HBM time 5.1 us).  1024 x 1024 pays 0.1 to 0.4 us for the longer code (4 / 8 vectors: 3.6 / 4.2 -> 3.8 / 4.6 us; a call's host work is above 10 us).
 #include <atomic>
 #include "operands.cuh"
 
@@ -16,11 +25,13 @@ namespace nvb {
 
 namespace {
 
-constexpr int kWarps = 8, kMaxN = 8;   // a CTA owns kWarps * R rows: R = 4 rows per warp, or 2 when the matrix has few rows
+constexpr int kMaxN = 8, kMaxWarps = 16;   // warps of a CTA
 constexpr int kSmemLimit = 200 * 1024;
 
 struct GemvQArgs {
   int m, n, k;
+  int ksplit;          // warps that share a group of 16 rows
+  int halves;          // 128-value halves per unit: 2, or 1 (only if no warp has more than one unit of a row)
   Fp4Operand A;
   BOperand B;
   Epilogue e;
@@ -32,37 +43,88 @@ __device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t sel) {
   asm("prmt.b32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(sel));
   return d;
 }
-// four E2M1 nibbles (the low 16 bits of h) -> four int8 values 2 * e2m1 (bytes in nibble order)
-__device__ __forceinline__ uint32_t dec4(uint32_t h) {
-  const uint32_t sel = h & 0x7777u;
-  const uint32_t pos = prmt(0x03020100u, 0x0C080604u, sel);           // 0 1 2 3 | 4 6 8 12
-  const uint32_t neg = prmt(0xFDFEFF00u, 0xF4F8FAFCu, sel);           // 0 -1 -2 -3 | -4 -6 -8 -12
-  // sign bits (3, 7, 11, 15) -> byte masks: nibbles 1, 3 have theirs at the top of bytes 0, 1; nibbles 0, 2 after << 4
-  const uint32_t x = ((h << 4) & 0x8080u) | ((h & 0x8080u) << 16);
-  const uint32_t mask = prmt(x, 0u, 0xB9A8u);                         // replicate the top bit of bytes 0, 2, 1, 3
-  return (pos & ~mask) | (neg & mask);
+// eight E2M1 nibbles -> eight int8 values 2 * e2m1 (lo: nibbles 0-3, hi: 4-7).  A set bit 3 of a PRMT selector nibble returns the looked-up
+// byte's sign (0 here) instead of the byte: w picks the magnitudes of the positive nibbles, w ^ 0x88888888 those of the negative ones.
+__device__ __forceinline__ void dec8(uint32_t w, uint32_t &lo, uint32_t &hi) {
+  const uint32_t n = w ^ 0x88888888u;                                 // magnitudes 0 1 2 3 | 4 6 8 12
+  lo = (prmt(0x03020100u, 0x0C080604u, w) - prmt(0x03020100u, 0x0C080604u, n) + 0x80808080u) ^ 0x80808080u;   // no borrow between bytes
+  hi = (prmt(0x03020100u, 0x0C080604u, w >> 16) - prmt(0x03020100u, 0x0C080604u, n >> 16) + 0x80808080u) ^ 0x80808080u;
 }
-__device__ __forceinline__ int dp4a(uint32_t a, uint32_t b, int c) { return __dp4a((int)a, (int)b, c); }
 
-template <int R>
-__global__ void __launch_bounds__(kWarps * 32) gemv_blocked_kernel(const GemvQArgs g) {
-  constexpr int kRows = kWarps * R;
+__device__ __forceinline__ void mma_s8(int (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+      : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+
+template <int P>   // pairs of activation vectors
+__global__ void __launch_bounds__(32 * kMaxWarps, 1) gemv_blocked_kernel(const GemvQArgs g) {
   extern __shared__ __align__(16) uint8_t smem[];
-  __shared__ float vtile[kMaxN][32];
-  __shared__ float colscale[kMaxN];
+  __shared__ float colscale[2 * P];
   const int gm = g.m, gn = g.n, gk = g.k, nb = gk >> 4;
   int8_t *xq = (int8_t *)smem;                       // [n][k]
   float *xs = (float *)(smem + (size_t)gn * gk);     // [n][k / 16]
+  float *part = xs + gn * nb;                        // [2][warp][n][16 rows]: the warps' sums of a tile
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const bool fp4b = g.B.dtype == NVFP4A_NVFP4;
   const bool ue_a = g.A.ue != 0;
 
-  // ---- stage the activations: int8 values and FP32 block scales ----
+  // ---- rows ----
+  const int T = blockDim.x, W = T >> 5, S = g.ksplit, G = W / S, kRows = 16 * G;   // S warps share a group of 16 rows, G groups are a tile
+  const int tiles = (gm + kRows - 1) / kRows;
+  const int nchunks = gk >> 5, halves = g.halves, units = (nchunks + 4 * halves - 1) / (4 * halves);   // a chunk: 32 values = 16 bytes = two blocks; a unit: 8 chunks (or 4)
+  const int grp = warp / S, ws = warp - grp * S, gq = lane >> 2, tq = lane & 3;
+  // A unit of a row: 128 bytes of nibbles, `du` bytes from the row's previous unit, and sixteen scale codes, `ds` from the previous ones
+  // (linear: in sequence; swizzled and image: four to each 512-byte tile).
+  const bool img = g.A.image, swz = img || g.A.sld <= 0;
+  const int du = img ? kImgTileBytes : 128, ds = img ? kImgTileBytes : swz ? 2048 : 16;
+  const int sc_half = swz ? 1024 : 8;
+  const uint8_t *pw[2], *ps[2];
+  int c_next = 0;
+  auto start_row = [&](int tile, int v) {   // the lane's pointers to unit v of its two rows of a tile
+    const int u = halves == 2 ? v : v >> 1, odd = halves == 2 ? 0 : v & 1;   // 256-value unit, its second half
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+      const int row = min(tile * kRows + 16 * grp + gq + 8 * r, gm - 1), rr = row & 127;
+      const size_t in_tile = (size_t)odd * 1024 + (tq >> 1) * 512 + (rr & 31) * 16 + (rr >> 5) * 4 + (tq & 1) * 2;
+      if (img) {
+        const uint8_t *t = g.A.data + ((size_t)(row >> 7) * g.A.ktiles + u) * kImgTileBytes;
+        pw[r] = t + rr * 128 + odd * 64 + tq * 16;
+        ps[r] = t + kImgDataBytes + in_tile;
+      } else {
+        pw[r] = g.A.data + (size_t)row * (g.A.ld >> 1) + (size_t)u * 128 + odd * 64 + tq * 16;
+        ps[r] = swz ? g.A.sc + (size_t)(row >> 7) * ((size_t)((-g.A.sld) >> 2) * 512) + (size_t)u * 2048 + in_tile
+                    : g.A.sc + (size_t)row * g.A.sld + (size_t)u * 16 + odd * 8 + tq * 2;
+      }
+    }
+    c_next = 8 * u + 4 * odd + tq;
+  };
+  uint4 w_next[2][2];        // [chunk of the lane][row gq, gq + 8]
+  uint32_t sc_next[2][2];
+  auto prefetch = [&]() {
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+      if (h < halves && c_next + 4 * h < nchunks)
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+          w_next[h][r] = __ldg((const uint4 *)(pw[r] + 64 * h));
+          sc_next[h][r] = __ldg((const uint16_t *)(ps[r] + (h ? sc_half : 0)));
+        }
+  };
+#pragma unroll
+  for (int h = 0; h < 2; ++h)
+#pragma unroll
+    for (int r = 0; r < 2; ++r) { w_next[h][r] = make_uint4(0, 0, 0, 0); sc_next[h][r] = 0; }
+  start_row(blockIdx.x, ws);   // (the grid has no more CTAs than tiles)
+  prefetch();
+
+  // ---- stage the activations: int8 values and FP32 block scales (the first weights are on their way) ----
   if (fp4b) {
     for (int idx = tid; idx < gn * nb; idx += blockDim.x) {
       const int j = idx / nb, kb = idx - j * nb;
       const uint2 w = g.B.q.block(j, kb);
-      *(uint4 *)(xq + (size_t)j * gk + 16 * kb) = make_uint4(dec4(w.x), dec4(w.x >> 16), dec4(w.y), dec4(w.y >> 16));
+      uint4 d;
+      dec8(w.x, d.x, d.y); dec8(w.y, d.z, d.w);
+      *(uint4 *)(xq + (size_t)j * gk + 16 * kb) = d;
       xs[idx] = g.B.q.scale(j, kb);
     }
   } else {
@@ -78,112 +140,142 @@ __global__ void __launch_bounds__(kWarps * 32) gemv_blocked_kernel(const GemvQAr
   }
   __syncthreads();
 
-  // ---- rows: warp w takes rows w, w + 8, w + 16, w + 24 of the CTA's 32, all four at once so that their loads fly together ----
-  const int i0 = blockIdx.x * kRows;
-  const int nchunks = gk >> 5;   // 32 values = 16 bytes = two blocks
-  const ScalePos sp{g.A.sld};
-  const bool img = g.A.image;
-  const uint8_t *const adata = g.A.data, *const asc = g.A.sc;
-  const int ald2 = g.A.ld >> 1, aktiles = g.A.ktiles;
-  auto load_chunk = [&](int row, int c, uint4 &w, uint32_t &sc) {   // 32 nibbles and the two scale codes of chunk c of a row
-    if (img) {
-      const uint8_t *tile = adata + ((size_t)(row >> 7) * aktiles + (c >> 3)) * kImgTileBytes;
-      const int rr = row & 127, cc = c & 7;
-      w = __ldg((const uint4 *)(tile + rr * 128 + cc * 16));
-      sc = __ldg((const uint16_t *)(tile + kImgDataBytes + (cc >> 1) * 512 + (rr & 31) * 16 + (rr >> 5) * 4 + (cc & 1) * 2));
-    } else {
-      w = __ldg((const uint4 *)(adata + (size_t)row * ald2 + (size_t)c * 16));
-      sc = __ldg((const uint16_t *)(asc + sp.at(row, 2 * c)));
-    }
-  };
-  float acc[R][kMaxN];
+  const bool diag = (gq >> 1) == tq;   // this lane's column of B is its own chunk's (see the head of the file)
+  const Epilogue &e = g.e;
+  float amax = 0.f;
+  int buf = 0;
+#pragma unroll 1
+  for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x, buf ^= 1) {
+  const int i0 = tile * kRows;
+  float acc[2][2 * P];
 #pragma unroll
-  for (int q = 0; q < R; ++q)
+  for (int j = 0; j < 2 * P; ++j) acc[0][j] = acc[1][j] = 0.f;
+#pragma unroll 1
+  for (int u = ws; u < units; u += S) {
+    uint4 w[2][2];
+    uint32_t sc[2][2];
+    const int c_unit = c_next;
 #pragma unroll
-    for (int j = 0; j < kMaxN; ++j) acc[q][j] = 0.f;
-  int rows4[R];
+    for (int h = 0; h < 2; ++h)
 #pragma unroll
-  for (int q = 0; q < R; ++q) rows4[q] = min(i0 + warp + kWarps * q, gm - 1);
-  for (int c = lane; c < nchunks; c += 32) {
-    uint4 w[R];
-    uint32_t sc[R];
+      for (int r = 0; r < 2; ++r) { w[h][r] = w_next[h][r]; sc[h][r] = sc_next[h][r]; }
+    if (u + S < units) {
 #pragma unroll
-    for (int q = 0; q < R; ++q) load_chunk(rows4[q], c, w[q], sc[q]);
-    // decode the four rows' chunks once, then walk the activation vectors: a vector's 32 values and two scales are read from
-    // shared memory once per chunk and serve all four rows (read per row, shared memory set the pace: 16 bytes of it per weight byte)
-    float sa[R][2];
-    uint32_t a0[R][4], a1[R][4];
-#pragma unroll
-    for (int q = 0; q < R; ++q) {
-      sa[q][0] = scale_to_f32(sc[q] & 0xFFu, ue_a); sa[q][1] = scale_to_f32(sc[q] >> 8, ue_a);
-      a0[q][0] = dec4(w[q].x); a0[q][1] = dec4(w[q].x >> 16); a0[q][2] = dec4(w[q].y); a0[q][3] = dec4(w[q].y >> 16);
-      a1[q][0] = dec4(w[q].z); a1[q][1] = dec4(w[q].z >> 16); a1[q][2] = dec4(w[q].w); a1[q][3] = dec4(w[q].w >> 16);
+      for (int r = 0; r < 2; ++r) { pw[r] += (size_t)S * du; ps[r] += (size_t)S * ds; }
+      c_next += 8 * S;
+      prefetch();
+    } else if (tile + (int)gridDim.x < tiles) {
+      start_row(tile + gridDim.x, ws);
+      prefetch();
     }
 #pragma unroll
-    for (int j = 0; j < kMaxN; ++j) {
-      if (j >= gn) break;
-      const uint4 x0 = *(const uint4 *)(xq + (size_t)j * gk + 32 * c), x1 = *(const uint4 *)(xq + (size_t)j * gk + 32 * c + 16);
-      const float xs0 = xs[j * nb + 2 * c], xs1 = xs[j * nb + 2 * c + 1];
+    for (int h = 0; h < 2; ++h) {
+      if (h == halves) break;
+      const int c = c_unit + 4 * h;
+      const bool in = c < nchunks;       // (a lane past the end multiplies zeros and leaves its sums alone)
+      uint32_t a[4][4];                  // [word][MMA operand register]
 #pragma unroll
-      for (int q = 0; q < R; ++q) {
-        const int p0 = dp4a(a0[q][3], x0.w, dp4a(a0[q][2], x0.z, dp4a(a0[q][1], x0.y, dp4a(a0[q][0], x0.x, 0))));
-        const int p1 = dp4a(a1[q][3], x1.w, dp4a(a1[q][2], x1.z, dp4a(a1[q][1], x1.y, dp4a(a1[q][0], x1.x, 0))));
-        acc[q][j] = __fmaf_rn(__fmul_rn((float)p0, sa[q][0]), xs0, acc[q][j]);
-        acc[q][j] = __fmaf_rn(__fmul_rn((float)p1, sa[q][1]), xs1, acc[q][j]);
+      for (int i = 0; i < 4; ++i) {
+        dec8(((const uint32_t *)&w[h][0])[i], a[i][0], a[i][2]);
+        dec8(((const uint32_t *)&w[h][1])[i], a[i][1], a[i][3]);
+      }
+      float sa[2][2];
+#pragma unroll
+      for (int r = 0; r < 2; ++r) { sa[r][0] = scale_to_f32(sc[h][r] & 0xFFu, ue_a); sa[r][1] = scale_to_f32(sc[h][r] >> 8, ue_a); }
+#pragma unroll
+      for (int p = 0; p < P; ++p) {
+        if (2 * p >= gn) break;
+        const int jb = 2 * p + (gq & 1);
+        uint4 x0 = make_uint4(0, 0, 0, 0), x1 = x0;
+        if (diag && in && jb < gn) {
+          x0 = *(const uint4 *)(xq + (size_t)jb * gk + 32 * c);
+          x1 = *(const uint4 *)(xq + (size_t)jb * gk + 32 * c + 16);
+        }
+        // (an integer sum of at most 16 x 12 x 128 added to the bits of 1.5 * 2^23 is that float's value plus the sum)
+        int c0[4] = {0x4B400000, 0x4B400000, 0x4B400000, 0x4B400000}, c1[4] = {0x4B400000, 0x4B400000, 0x4B400000, 0x4B400000};
+        mma_s8(c0, a[0], x0.x, x0.y);
+        mma_s8(c1, a[2], x1.x, x1.y);
+        mma_s8(c0, a[1], x0.z, x0.w);
+        mma_s8(c1, a[3], x1.z, x1.w);
+#pragma unroll
+        for (int jj = 0; jj < 2; ++jj) {
+          const int j = 2 * p + jj;
+          float2 xsv = make_float2(0.f, 0.f);
+          if (in) xsv = *(const float2 *)(xs + min(j, gn - 1) * nb + 2 * c);
+#pragma unroll
+          for (int r = 0; r < 2; ++r) {
+            acc[r][j] = __fmaf_rn(__fmul_rn(__fadd_rn(__int_as_float(c0[2 * r + jj]), -12582912.f), sa[r][0]), xsv.x, acc[r][j]);
+            acc[r][j] = __fmaf_rn(__fmul_rn(__fadd_rn(__int_as_float(c1[2 * r + jj]), -12582912.f), sa[r][1]), xsv.y, acc[r][j]);
+          }
+        }
       }
     }
   }
+  float *const mine = part + ((size_t)buf * W + warp) * gn * 16;
 #pragma unroll
-  for (int q = 0; q < R; ++q)
+  for (int j = 0; j < 2 * P; ++j) {
+    if (j >= gn) break;
 #pragma unroll
-    for (int j = 0; j < kMaxN; ++j) {
-      float a = acc[q][j];
-#pragma unroll
-      for (int o = 16; o; o >>= 1) a = __fadd_rn(a, __shfl_xor_sync(0xFFFFFFFFu, a, o));
-      if (lane == 0 && j < gn) vtile[j][warp + kWarps * q] = __fmul_rn(a, fp4b ? 0.25f : 0.5f);
+    for (int r = 0; r < 2; ++r) {
+      float v = acc[r][j];
+      v = __fadd_rn(v, __shfl_xor_sync(0xFFFFFFFFu, v, 1));
+      v = __fadd_rn(v, __shfl_xor_sync(0xFFFFFFFFu, v, 2));
+      if (tq == 0) mine[j * 16 + gq + 8 * r] = v;
     }
+  }
   __syncthreads();
 
-  // ---- epilogue: thread t owns (row t % 32, column t / 32) ----
-  const Epilogue &e = g.e;
-  const int ri = tid & 31, cj = tid >> 5, i = i0 + ri;
-  const bool live = ri < kRows && i < gm && cj < gn;
-  float v = 0.f, amax = 0.f;
-  if (live) {
-    float colp = epi_col_part(e, cj);
-    if (g.ex.mask & kExNorm) colp = __fmul_rn(colp, colscale[cj]);
-    v = epi_value(e, i, cj, vtile[cj][ri], epi_scale(e, epi_row_part(e, i), colp));
+  // ---- epilogue: a thread per (row, column) of the tile; the S warps' sums are added in order ----
+  const bool neighbours = (g.ex.mask & (kExSwiglu | kExOut2)) != 0;
+  const int outs = kRows * gn;
+  for (int o = tid; o < outs; o += T) {
+    const int ri = o % kRows, cj = o / kRows, i = i0 + ri;
+    float *const p0 = part + ((size_t)buf * W + (ri >> 4) * S) * gn * 16 + cj * 16 + (ri & 15);
+    float sum = *p0;
+    for (int q = 1; q < S; ++q) sum = __fadd_rn(sum, p0[q * gn * 16]);
+    float v = 0.f;
+    if (i < gm) {
+      float colp = epi_col_part(e, cj);
+      if (g.ex.mask & kExNorm) colp = __fmul_rn(colp, colscale[cj]);
+      v = epi_value(e, i, cj, __fmul_rn(sum, fp4b ? 0.25f : 0.5f), epi_scale(e, epi_row_part(e, i), colp));
+      if (!neighbours) { store_dense(e.d_dtype, e.d, (size_t)cj * e.ldd + i, v); amax = fmaxf(amax, fabsf(v)); }
+    }
+    if (neighbours) *p0 = v;   // (in the place of the first sum, which only this thread reads)
   }
-  if (!(g.ex.mask & (kExSwiglu | kExOut2))) {
-    if (live) { store_dense(e.d_dtype, e.d, (size_t)cj * e.ldd + i, v); amax = fabsf(v); }
-  } else {
+  if (neighbours) {
     __syncthreads();
-    if (cj < kMaxN) vtile[cj][ri] = v;
-    __syncthreads();
-    if (g.ex.mask & kExSwiglu) {
-      if (live && !(ri & 8)) {
-        const float h = silu_mul(v, vtile[cj][ri + 8]);
-        store_dense(e.d_dtype, e.d, (size_t)cj * e.ldd + (i >> 4) * 8 + (i & 7), h);
-        amax = fabsf(h);
+    for (int o = tid; o < outs; o += T) {
+      const int ri = o % kRows, cj = o / kRows, i = i0 + ri;
+      const float *const p0 = part + ((size_t)buf * W + (ri >> 4) * S) * gn * 16 + cj * 16 + (ri & 15);
+      const float v = *p0;
+      const bool live = i < gm;
+      if (g.ex.mask & kExSwiglu) {
+        if (live && !(ri & 8)) {
+          const float h = silu_mul(v, p0[8]);
+          store_dense(e.d_dtype, e.d, (size_t)cj * e.ldd + (i >> 4) * 8 + (i & 7), h);
+          amax = fmaxf(amax, fabsf(h));
+        }
+      } else if (live) {
+        store_dense(e.d_dtype, e.d, (size_t)cj * e.ldd + i, v);
+        amax = fmaxf(amax, fabsf(v));
       }
-    } else if (live) {
-      store_dense(e.d_dtype, e.d, (size_t)cj * e.ldd + i, v);
-      amax = fabsf(v);
-    }
-    if (g.ex.mask & kExOut2) {
-      if (live) store_dense(g.ex.d2_dtype, g.ex.d2, (size_t)cj * g.ex.ldd2 + i, __fmul_rn(v, load_dense(g.ex.w2_dtype, g.ex.w2, i)));
-      if (live && !(ri & 15)) {
-        float sq = 0.f;
+      if (g.ex.mask & kExOut2) {
+        if (live) store_dense(g.ex.d2_dtype, g.ex.d2, (size_t)cj * g.ex.ldd2 + i, __fmul_rn(v, load_dense(g.ex.w2_dtype, g.ex.w2, i)));
+        if (live && !(ri & 15)) {
+          float sq = 0.f;
 #pragma unroll
-        for (int r = 0; r < 16; ++r) sq = __fadd_rn(sq, __fmul_rn(vtile[cj][ri + r], vtile[cj][ri + r]));
-        g.ex.sq[(size_t)cj * g.ex.ld_sq + (i >> 4)] = sq;
+          for (int r = 0; r < 16; ++r) sq = __fadd_rn(sq, __fmul_rn(p0[r], p0[r]));
+          g.ex.sq[(size_t)cj * g.ex.ld_sq + (i >> 4)] = sq;
+        }
       }
     }
+  }
   }
   if (e.amax) warp_amax_commit(e.amax, amax);
 }
 
-size_t smem_bytes(const GemmArgs &g) { return (size_t)g.n * g.k + (size_t)g.n * (g.k / 16) * sizeof(float); }
+size_t smem_bytes(int n, int k) { return (size_t)n * k + (size_t)n * (k / 16) * sizeof(float); }   // the activations
+int part_bytes(int warps, int n) { return 2 * warps * n * 16 * (int)sizeof(float); }
 
 }  // namespace
 
@@ -191,28 +283,42 @@ bool gemv_blocked_supports(const GemmArgs &g) {
   if (!(g.n >= 1 && g.n <= kMaxN && g.k >= 64 && (g.B.dtype == NVFP4A_INT8 || g.B.dtype == NVFP4A_NVFP4))) return false;
   if (g.B.dtype == NVFP4A_NVFP4 && g.B.q.image) return false;
   if (g.B.dtype == NVFP4A_INT8 && (((uintptr_t)g.B.data & 15) || g.B.ld % 16)) return false;
-  return smem_bytes(g) <= (size_t)kSmemLimit;
+  return smem_bytes(g.n, g.k) <= (size_t)kSmemLimit;
+}
+
+template <int P>
+static cudaError_t launch_pairs(GemvQArgs &a, int warps, cudaStream_t s) {
+  static std::atomic<bool> attr_set[64];   // zero-initialised; set once per device (a repeated cudaFuncSetAttribute is harmless)
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (!attr_set[dev & 63]) {
+    if (cudaError_t e = cudaFuncSetAttribute(gemv_blocked_kernel<P>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit + part_bytes(kMaxWarps, kMaxN))) return e;
+    attr_set[dev & 63] = true;
+  }
+  const int rows = 16 * (warps / a.ksplit), tiles = (a.m + rows - 1) / rows, smem = (int)smem_bytes(a.n, a.k) + part_bytes(warps, a.n);
+  int per_sm = kMaxWarps / warps;   // (by its registers)
+  while (per_sm > 1 && per_sm * (smem + 2048) > 227 * 1024) --per_sm;
+  const int grid = tiles < per_sm * device_sms() ? tiles : per_sm * device_sms();
+  gemv_blocked_kernel<P><<<grid, warps * 32, smem, s>>>(a);
+  return cudaGetLastError();
 }
 
 cudaError_t launch_gemv_blocked(const GemmArgs &g, cudaStream_t s) {
   GemvQArgs a;
   a.m = g.m; a.n = g.n; a.k = g.k;
   a.A = g.A; a.B = g.B; a.e = g.e; a.ex = g.x;
-  static std::atomic<bool> attr_set[64];   // zero-initialised; set once per device (a repeated cudaFuncSetAttribute is harmless)
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (!attr_set[dev & 63]) {
-    cudaError_t e = cudaFuncSetAttribute(gemv_blocked_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(gemv_blocked_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit);
-    if (e != cudaSuccess) return e;
-    attr_set[dev & 63] = true;
-  }
-  // 32 rows per CTA give every SM a CTA from about 4700 rows up; below that, 16 rows per CTA put twice as many warps on the
-  // SMs (4096 x 4096, 8 vectors: 17.2 -> 14.1 us; at 8192 rows the doubled staging of the activations costs more than it brings).
-  // A row's sum does not depend on the choice: a warp walks its rows' chunks in the same order either way.
-  if ((g.m + 31) / 32 >= device_sms()) gemv_blocked_kernel<4><<<(g.m + 31) / 32, kWarps * 32, smem_bytes(g), s>>>(a);
-  else gemv_blocked_kernel<2><<<(g.m + 15) / 16, kWarps * 32, smem_bytes(g), s>>>(a);
-  return cudaGetLastError();
+  // How a row's k is dealt to warps depends on k alone, so that a row's bits do not depend on the matrix around it (or on n): eight warps in
+  // 256-value units, or up to 1024 values a 128-value half unit to a warp (1024 x 1024, 4 / 8 vectors: 3.9 / 4.8 -> 3.8 / 4.6 us).
+  // CTAs of eight warps, two per SM; of sixteen (two groups) where a CTA gets one tile at most or the activations leave room for one CTA:
+  // 4096 x 14336, 4 / 8 vectors 21.0 / 34.7 -> 18.8 / 26.0 us, 4096 x 4096, 8 vectors 11.8 -> 11.0 us.  Fewer than eight only if that gives more CTAs.
+  const int groups = (g.m + 15) / 16, sms = device_sms();
+  a.halves = g.k <= 1024 ? 1 : 2;
+  a.ksplit = 8;
+  while (a.ksplit > 1 && a.ksplit * 64 >= g.k) a.ksplit >>= 1;
+  int warps = 8;
+  if (a.ksplit < 8 && groups <= 2 * sms) warps = a.ksplit < 4 ? 4 : a.ksplit;
+  if (g.k > 1024 && ((groups > sms && groups <= 2 * sms) || 2 * (smem_bytes(g.n, g.k) + part_bytes(8, g.n) + 2048) > 227 * 1024)) warps = 16;
+  return g.n <= 2 ? launch_pairs<1>(a, warps, s) : g.n <= 4 ? launch_pairs<2>(a, warps, s) : launch_pairs<4>(a, warps, s);
 }
 
 }  // namespace nvb

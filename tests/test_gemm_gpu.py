@@ -472,6 +472,30 @@ def test_gemv_with_block_scaled_activations_uses_the_dp4a_kernel(bt):
             check_bound(c, h, got, amax, exp)
 
 
+@pytest.mark.parametrize("bt", [L.INT8, L.NVFP4])
+@pytest.mark.parametrize("layout", ["image", "swizzled", "linear"])
+def test_blocked_gemv_at_the_edges_of_its_tiles_and_k_ranges(bt, layout):
+    """Units of 128 and 256 values with remainders, one to eight warps per group of 16 rows, CTAs of 4, 8 and 16 warps (the last also because
+    the activations fill shared memory), more tiles than CTAs, odd n; negative block scales; and a row's bits do not depend on the matrix around it."""
+    for i, (m, n, k) in enumerate([(33, 1, 64), (77, 2, 192), (200, 3, 320), (130, 5, 576), (4900, 4, 128), (100, 7, 1088), (2500, 8, 2112), (5000, 2, 1344), (50, 8, 14400),
+                                   (9700, 6, 256)]):
+        c = Case(m, n, k, bt, L.FP32, -1, -1, 1.0, 0.0, fa=SW if layout == "swizzled" else 0)
+        h = build_case(c, 7300 + i)
+        flip = np.random.default_rng(i).integers(0, 4, h["A"].scales.size) == 0
+        h["A"].scales[flip & (h["A"].scales != 0)] |= 0x80
+        exp = oracle_case(c, h, want_ref=True)
+        got, amax = run_tc(c, h, gemv=True) if layout == "image" else run_gemm(c, h)
+        assert L.lib.nvfp4a_b200_last_route() == 6, c
+        check_bound(c, h, got, amax, exp)
+        if layout == "linear" and m > 160:
+            A = h["A"]
+            top = O.Fp4(160, k, ld=A.ld, ld_scale=A.ld_scale, flags=A.flags, scale_max=A.scale_max, glob=0.0)
+            top.data[:], top.scales[:], top.glob[:] = A.data[:160 * A.ld // 2], A.scales[:160 * A.ld_scale], A.glob
+            ct, ht = Case(160, n, k, bt, L.FP32, -1, -1, 1.0, 0.0), dict(h, A=top)
+            got_top, _ = run_gemm(ct, ht)
+            assert np.array_equal(values(got_top, ct, ht), values(got, c, h)[:, :160])
+
+
 def test_w4a8_dp4a_gemm_is_bit_exact_in_the_tiled_order():
     """INT8 activations, n > 8, with the tensor-core W4A8 GEMM switched off (nvfp4a_b200_set_route(3)): the DP4A GEMM (route 7)
     sums blocks in the reference's tiled order, so D and amax equal the oracle's bit for bit; tails in m and n, padded leading
