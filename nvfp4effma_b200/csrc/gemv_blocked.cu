@@ -134,9 +134,11 @@ __global__ void __launch_bounds__(32 * kMaxWarps, 1) gemv_blocked_kernel(const G
       xs[idx] = g.B.s8[(size_t)j * g.B.lds8 + kb];
     }
   }
-  if ((g.ex.mask & kExNorm) && warp < gn) {
-    const float s = warp_norm_scale(g.ex, warp, lane);
-    if (lane == 0) colscale[warp] = s;
+  if (g.ex.mask & kExNorm) {   // a warp per vector in turn: a CTA may have fewer warps (four) than there are vectors
+    for (int j = warp; j < gn; j += W) {
+      const float s = warp_norm_scale(g.ex, j, lane);
+      if (lane == 0) colscale[j] = s;
+    }
   }
   __syncthreads();
 

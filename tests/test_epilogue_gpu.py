@@ -110,6 +110,15 @@ def run_case(m, n, k, bt, dt, mask, use_bias, use_c, tc):
 
 
 @pytest.mark.parametrize("tc", [False, True])
+@pytest.mark.parametrize("m,n,k", [(528, 5, 64), (528, 8, 256), (1024, 7, 512), (4736, 8, 512), (1024, 8, 576)])
+def test_extended_epilogue_with_fewer_warps_than_vectors(m, n, k, tc):
+    """Short reductions run the GEMV of INT8 vectors with four or eight warps per CTA: every vector still gets its RMSNorm scale.  (Shared
+    memory keeps what earlier kernels left there; the scales of a call with other parts come first.)"""
+    for mask in (1, 3, 5):
+        run_case(m, n, k, L.INT8, L.FP32, mask, False, False, tc)
+
+
+@pytest.mark.parametrize("tc", [False, True])
 @pytest.mark.parametrize("bt", [L.BF16, L.INT8])
 def test_extended_epilogue(tc, bt):
     v = 0
