@@ -316,7 +316,8 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
     uint8_t *const boxes = staging + half * 2 * C::kStagingBytes;
     float amax = 0.f;
     uint32_t tile_i = 0, box = 0;
-    // a staging tile is free when the store before the last one has been read (the two tiles alternate)
+    // A staging tile is free when the store before the last one has been read (the two tiles alternate).  Every turn commits a group, an empty
+    // one where nothing was stored by TMA (a group's last tokens, a CTA without rows): "all but the last group" is then the tile's own.
     auto next_box = [&]() -> uint8_t * {
       if (leader) bulk_wait_read_one();
       named_barrier(bar_id, 128);
@@ -541,7 +542,6 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
               tma_store_2d(&tmap_d, st + b * 4096, o, j0);
               for (int q = 0; q < peers.n; ++q) tma_store_2d(&peers.map[q], st + b * 4096, o, j0);   // the same box into every peer's buffer
             }
-            bulk_commit();
           }
         } else {   // D that TMA cannot store, or a group's last tokens: a thread per row
           named_barrier(bar_id, 128);
@@ -552,6 +552,7 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
               ((uint16_t *)dptr)[(size_t)(j0 + jj) * g.e.ldd + orow + row] = *(const uint16_t *)(src + jj * 128 + ((((row >> 3) & 7) ^ (jj & 7)) << 4));
           }
         }
+        if (leader) bulk_commit();
       }
       ++tile_i;
     }

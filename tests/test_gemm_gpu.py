@@ -786,6 +786,50 @@ def test_w4a16_gemm_gives_the_same_bytes_every_time():
     assert kernel_status() == 0
 
 
+@pytest.mark.parametrize("case", ["odd_row_tiles", "swiglu", "grouped"])
+def test_tma_stored_tiles_equal_plain_stores_on_every_launch(case):
+    """A 16-bit D leaves through two alternating staging tiles and TMA stores.  Short reductions (the next tile's results arrive soon), several
+    tiles per CTA pair and turns that store nothing by TMA -- an odd number of 128-row tiles, the last tokens of a group -- against the
+    same launch with a leading dimension that TMA cannot store (plain stores, no staging tile in flight), 60 launches each."""
+    m, k = (2048, 512) if case == "grouped" else (33 * 128, 64)
+    gen = torch.Generator(device="cuda").manual_seed(11)
+    ints = lambda lo, hi, shape: torch.randint(lo, hi, shape, generator=gen, device="cuda", dtype=torch.uint8)
+    if case == "grouped":
+        sizes = torch.randint(1, 250, (40,), generator=torch.Generator().manual_seed(3))
+        seg = torch.cat([torch.zeros(1, dtype=torch.int64), sizes.cumsum(0)]).to(torch.int32).cuda()
+        groups, n = 40, int(sizes.sum())
+        x, xs = ints(0, 256, (n, k)).view(torch.int8), torch.rand(n, k // 16, generator=gen, device="cuda") + 0.5
+        tb = tensor(x, L.INT8, xs, k // 16)
+    else:
+        groups, n = 1, 2048
+        x = torch.randn(n, k, generator=gen, device="cuda").to(torch.bfloat16)
+        tb = tensor(x, L.BF16)
+    w, ws = ints(0, 256, (groups * m, k // 2)), ints(0x30, 0x48, (groups * m, k // 16))
+    ta = tensor(w, L.NVFP4, ws, k // 16)
+    mo = m // 2 if case == "swiglu" else m
+    ex = L.Epilogue()
+    ex.swiglu = int(case == "swiglu")
+
+    def launch(out):
+        td, ld = tensor(out, L.BF16), out.stride(0)
+        if case == "grouped":
+            return L.lib.nvfp4a_gemm_grouped(groups, m, k, n, 2.0 ** -10, ctypes.byref(ta), k, ctypes.byref(tb), k, 0.0, None, 0, ctypes.byref(td), ld, None,
+                                             ctypes.c_void_p(seg.data_ptr()), stream())
+        return L.lib.nvfp4a_gemm_ex(m, n, k, 0.25, ctypes.byref(ta), k, ctypes.byref(tb), k, 0.0, None, 0, ctypes.byref(td), ld, None, ctypes.byref(ex), stream())
+
+    plain, out = torch.zeros(n, mo + 1, dtype=torch.bfloat16, device="cuda"), torch.zeros(n, mo, dtype=torch.bfloat16, device="cuda")
+    L.check(launch(plain))
+    assert L.lib.nvfp4a_b200_last_route() == (8 if case == "grouped" else 5)
+    assert bool(torch.isfinite(plain.float()).all()) and bool(plain.any())
+    want, differs = plain[:, :mo].contiguous().view(torch.int16), []
+    for _ in range(60):
+        out.zero_()
+        L.check(launch(out))
+        differs.append((out.view(torch.int16) != want).any())
+    assert not bool(torch.stack(differs).any())
+    assert kernel_status() == 0
+
+
 @pytest.mark.parametrize("seg,m,k", [([0, 1, 1, 64], 128, 512), ([0, 65, 130, 131], 130, 576), ([0, 0, 0, 257], 300, 1088), ([3, 3, 100, 400], 257, 512)])
 def test_grouped_w4a8_on_the_tensor_cores(seg, m, k):
     """INT8 activations, 16-bit D, k >= 512: nvfp4a_gemm_grouped runs the tcgen05 kernel (route 8), every group within the bound of its own
