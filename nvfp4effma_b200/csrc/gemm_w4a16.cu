@@ -1,5 +1,5 @@
 // NVFP4 weights x BF16 activations (W4A16) GEMM on the 5th-generation tensor cores: tcgen05.mma kind::f16 (BF16 in, FP32
-// accumulators in tensor memory) on weights expanded to exact BF16 in shared memory.
+// accumulators in tensor memory) on weights expanded to exact BF16 in tensor memory.
 //
 // An NVFP4 value times its block scale has at most 2 + 4 significant bits, so e2m1 * scale is exact in BF16; the tensor
 // cores then form exact products with the BF16 activations and accumulate in FP32 -- the reference's "exact" W4A16
@@ -9,14 +9,15 @@
 // each CTA's shared memory), a stage covers 64 values of k.  The expanded weights are the MMA's A operand IN TENSOR MEMORY: an
 // expansion thread owns a weight row = a tensor memory lane and writes its 64 values with two tcgen05.st, so that the expansion costs
 // no shared-memory traffic, no swizzled addressing and no proxy fence, and shared memory is left to the activations (read once per
-// pair and stage).  Tensor memory: columns [0, 256) one accumulator of 256 columns or two of 128, [256, 512) eight weight stages.
+// pair and stage).  Tensor memory: columns [0, 256) one accumulator of 256 columns or two of 128, [256, 512) eight weight stages (grouped: a
+// third accumulator of 128 columns, then four stages).
 // Roles, 20 warps per CTA:
 //   warp 0      TMA producer of the activations: this CTA's half of the tile's tokens (no multicast); the bytes of both CTAs are
 //               counted on the even CTA's barrier
 //   warp 1      MMA issuer (even CTA; 4 x K16 per stage, one elected lane), owner of the tensor memory
 //   warp 2      TMA producer of the weight nibbles: [128 rows][128 bytes] = 256 values of k per slot, so that the expansion
 //               reads shared memory and never waits for a trip to L2
-//   warps 4-11  epilogue (160 registers each, taken from the others by setmaxnreg), one 32-lane quadrant and one half of the columns
+//   warps 4-11  epilogue (144 registers each, taken from the others by setmaxnreg), one 32-lane quadrant and one half of the columns
 //               each: the accumulator block goes into registers at once and back to the MMA warp before any arithmetic; then
 //               plain or extended epilogue (RMSNorm column scale, SwiGLU, second output + sums of squares), D through
 //               shared-memory staging tiles and TMA stores when its layout allows
@@ -34,8 +35,19 @@
 // FP16 activations (F16): e2m1 x E4M3 is a multiple of 2^-10 up to 2880 with at most 6 significant bits, exact in FP16, so the same
 // kernel runs on FP16 operands.
 //
+// Segments.  The tensor cores truncate the running sum at every instruction, so that one chain over all of k drifts towards zero: at k = 4096 its
+// error against 64 bits is 1.3e-6 (BF16 / FP16 activations) and 9.9e-6 (INT8, three chains in one) where the ordered FP32 sums of the
+// CUDA-core kernels have 2.2e-7 and 2.9e-7.  The calls that those kernels would take otherwise -- FP16 activations, INT8 groups -- are therefore
+// summed in segments: 4 stages (256 values of k) go into one of two accumulators, the epilogue warps add each to running FP32 sums in
+// their registers (64 per thread: tiles of at most 128 tokens) while the next one fills, and INT8's two small planes, whose drift does
+// not matter, have an accumulator of their own for all of k.  Error: 1.05e-7 and 9.8e-8 at k = 4096 (normal data; 2.9e-7 and 1.4e-7 against
+// 6.9e-7 and 2.9e-7 with activations spread over ten binades).  Below k = 1024 segments are 2 stages, below 512 one (INT8 at k = 512:
+// 6.2e-8 against 1.08e-7; FP16 at k = 512, 128 and 64: 6.3e-8, 4.2e-8 and 4.0e-8 against 6.9e-8, 4.1e-8 and 3.7e-8).
+// Cost: 8 experts of 2048 x 4096 on 1100 tokens 132 us instead of 102 (125 with tiles of 128 tokens in one chain), FP16 4096 x 4096 on 333
+// tokens 38.5 instead of 36.3 us; the CUDA-core kernels take 602 and 1932 us.
+//
 // Grouped (mixture of experts): A stacks the weights of all groups, a group owns the tokens [seg[q], seg[q + 1]); the CTAs read seg
-// (device memory) into a table of tile counts and find a tile's group there.
+// (device memory) into a table of tile counts and find a tile's group there.  (INT8 activations only, plain epilogue, 16-bit D.)
 //
 // INT8 activations (W4A8, FP32 scale per 16 values) run on the same kernel with PLANES = 3: an activation is the FP32 value
 // x = q * s_b (one rounding: within the accumulation bound of the exact definition, not bit-identical to the integer block sums
@@ -64,6 +76,7 @@ struct W4A16Args {
   int width;     // tokens per tile: 64, 128 or 256
   int nfull, cut;   // tiles 0 .. nfull - 1 are `width` tokens wide; the rest (to `tiles`) are parts of width / cut tokens
   int tiles;
+  int seg_stages;   // F16, GROUPED: stages per segment of k
   const int *seg; int groups;   // GROUPED: m is the rows of ONE group's weight, n the bound on seg[groups]
 };
 
@@ -73,18 +86,19 @@ struct alignas(64) PeerMaps {
   int n;
 };
 
-template <int PLANES>
+template <int PLANES, bool GROUPED>
 struct Cfg {
   // PLANES = 1: the weight and the activation ring advance together and share their `empty` barriers (one commit per stage)
-  static constexpr int kA = 8, kB = 8, kRaw = 3;
+  static constexpr int kA = GROUPED ? 4 : 8, kB = 8, kRaw = 3;
+  static constexpr int kACols = 512 - 32 * kA;   // first tensor memory column of the weight stages (32 columns each)
   static constexpr int kBBytes = 128 * 128, kRawBytes = 128 * 128, kStagingBytes = 8192;
   static constexpr int kSmemBytes = 1024 + kB * kBBytes + kRaw * kRawBytes + 4 * kStagingBytes + 4096 /* expansion table */ + 256 * 4 /* column scales */ +
                                     512 /* barriers */ + 2 * 257 * 4 + 8 /* groups */;
 };
-static_assert(Cfg<1>::kSmemBytes <= 232448, "shared memory budget");
-constexpr int kACols = 256;   // first tensor memory column of the weight stages (32 columns each)
+static_assert(Cfg<1, false>::kSmemBytes <= 232448, "shared memory budget");
+constexpr int kSegmentWidth = 128;   // tokens per tile where k is summed in segments: the running sums have to fit the epilogue's registers
 
-constexpr int kThreads = 640, kRegsRest = 40, kRegsEpi = 128, kRegsConv = 72;
+constexpr int kThreads = 640, kRegsRest = 40, kRegsEpi = 144, kRegsConv = 72;
 static_assert(128 * kRegsRest + 256 * kRegsEpi + 256 * kRegsConv <= kThreads * 96, "the split draws on the registers of the launch: 96 per thread");
 constexpr unsigned kStWaitFullA = 0x301, kStWaitFullB = 0x302, kStWaitEmpty = 0x303, kStWaitTmemFull = 0x304, kStWaitTmemEmpty = 0x305,
                    kStWaitConv = 0x306, kStWaitRaw = 0x307;
@@ -123,8 +137,9 @@ template <int PLANES, bool F16, bool GROUPED>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_b, const __grid_constant__ CUtensorMap tmap_d,
                   const __grid_constant__ PeerMaps peers, const W4A16Args g) {
-  using C = Cfg<PLANES>;
-  constexpr int kA = C::kA, kB = C::kB, kRaw = C::kRaw;
+  using C = Cfg<PLANES, GROUPED>;
+  constexpr bool SEG = F16 || GROUPED;   // k is summed in segments: see the head of the file
+  constexpr int kA = C::kA, kB = C::kB, kRaw = C::kRaw, kACols = C::kACols, kSmallCols = 256;
   extern __shared__ uint8_t smem_raw[];
   uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint8_t *const sB = smem, *const sRaw = sB + kB * C::kBBytes, *const staging = sRaw + kRaw * C::kRawBytes;
@@ -139,7 +154,7 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int rank = (int)cluster_ctarank();
-  const int gm = g.m, gn = g.n, gk = g.k;
+  const int gm = g.m, gn = g.n, gk = g.k, seg_stages = SEG ? g.seg_stages : 0;
   const int tiles_m = (gm + 255) / 256, nk = gk / 64, nslots = (nk + 3) / 4;   // 256-row tiles
   const int tile_first = blockIdx.x >> 1, tile_step = gridDim.x >> 1;
   const bool ue = g.A.ue != 0;
@@ -251,30 +266,36 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
     // one-lane branch every tcgen05.mma costs ~150 cycles, more than the 128 the tensor pipe needs for 256 x 256 x 16 on a pair.
     if (rank == 0) {
       const uint64_t db0 = smem_desc_sw128(smem_u32(sB));
-      uint32_t ia = 0, ib = 0, tile_i = 0;
+      uint32_t ia = 0, ib = 0, acc_i = 0;
       for (int t = tile_first; t < ntiles; t += tile_step) {
         const Tile p = tile_of(t);
         if (p.width == 0) continue;
-        const int acc = nacc == 2 ? tile_i & 1 : 0;
-        const uint32_t idesc = idesc_f16(256, p.width, F16 ? 0 : 1), acc_par = (nacc == 2 ? tile_i >> 1 : tile_i) & 1;
-        if (!__all_sync(0xFFFFFFFFu, wait(&tmem_empty[acc], acc_par ^ 1, kStWaitTmemEmpty))) goto done;
-        tc_fence_after();
-        const uint32_t d_tmem = tmem_base + acc * 128;
-        for (int ks = 0; ks < nk; ++ks, ++ia) {
-          const int sa = ia % kA;
-          if (!__all_sync(0xFFFFFFFFu, wait(&a_full[sa], (ia / kA) & 1, kStWaitFullA))) goto done;
-          const uint32_t a_tmem = tmem_base + kACols + sa * 32;
+        const uint32_t idesc = idesc_f16(256, p.width, F16 ? 0 : 1);
+        for (int ks0 = 0; ks0 < nk; ks0 += SEG ? seg_stages : nk, ++acc_i) {
+          const int acc = nacc == 2 ? acc_i & 1 : 0, ks1 = SEG ? min(ks0 + seg_stages, nk) : nk;
+          const uint32_t acc_par = (nacc == 2 ? acc_i >> 1 : acc_i) & 1;
+          if (!__all_sync(0xFFFFFFFFu, wait(&tmem_empty[acc], acc_par ^ 1, kStWaitTmemEmpty))) goto done;
+          // (the small terms' accumulator was read together with the previous tile's last segment, whose accumulator is the next one's)
+          if (SEG && PLANES != 1 && ks0 == 0 && !__all_sync(0xFFFFFFFFu, wait(&tmem_empty[acc ^ 1], (((acc_i + 1) >> 1) & 1) ^ 1, kStWaitTmemEmpty))) goto done;
+          tc_fence_after();
+          const uint32_t d_tmem = tmem_base + acc * 128;
+          for (int ks = ks0; ks < ks1; ++ks, ++ia) {
+            const int sa = ia % kA;
+            if (!__all_sync(0xFFFFFFFFu, wait(&a_full[sa], (ia / kA) & 1, kStWaitFullA))) goto done;
+            const uint32_t a_tmem = tmem_base + kACols + sa * 32;
 #pragma unroll
-          for (int pl = 0; pl < PLANES; ++pl, ++ib) {
-            const int sb = ib % kB;
-            if (!__all_sync(0xFFFFFFFFu, wait(&b_full[sb], (ib / kB) & 1, kStWaitFullB))) goto done;
-            tc_fence_after();
-            mma4_f16_commit_pair_elect(d_tmem, a_tmem, db0 + (uint32_t)sb * (uint32_t)(C::kBBytes >> 4), idesc, (uint32_t)((ks | pl) != 0), &b_empty[sb]);
+            for (int pl = 0; pl < PLANES; ++pl, ++ib) {
+              const int sb = ib % kB;
+              if (!__all_sync(0xFFFFFFFFu, wait(&b_full[sb], (ib / kB) & 1, kStWaitFullB))) goto done;
+              tc_fence_after();
+              const bool small = SEG && pl > 0;   // (summed over all of k, apart from the segments)
+              mma4_f16_commit_pair_elect(small ? tmem_base + kSmallCols : d_tmem, a_tmem, db0 + (uint32_t)sb * (uint32_t)(C::kBBytes >> 4), idesc,
+                                         (uint32_t)((small ? ks | (pl - 1) : (ks - ks0) | pl) != 0), &b_empty[sb]);
+            }
+            if (PLANES != 1) tc_commit_pair_elect(&a_empty[sa]);
           }
-          if (PLANES != 1) tc_commit_pair_elect(&a_empty[sa]);
+          tc_commit_pair_elect(&tmem_full[acc]);
         }
-        tc_commit_pair_elect(&tmem_full[acc]);
-        ++tile_i;
       }
     }
   } else if (warp == 2) {
@@ -304,7 +325,7 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
     // (rarely used parameters are read from the constant bank where they are needed: the registers belong to the accumulator block)
     const float gb0 = g.e.gb ? __ldg(g.e.gb) : 1.f;   // B's global: dense B has none, INT8 B one for the tensor (a multiply by 1 is exact)
     uint8_t *const dptr = (uint8_t *)g.e.d;
-    const int d_dtype = g.e.d_dtype, mask = g.x.mask;
+    const int d_dtype = g.e.d_dtype, mask = SEG ? 0 : g.x.mask;   // (segments: a 16-bit D and the plain epilogue)
     const bool d_tma = g.d_tma;
     // The accumulator is read as MMA fragments (16 lanes x 8 columns per register quad): a thread holds rows rb + 16 hh + 8 u (hh, u in
     // {0, 1}) of columns 8 gq + cp + e (e in {0, 1}) of a chunk of 32, register 16 hh + 4 gq + 2 u + e.  Gate and up rows of SwiGLU (8
@@ -315,7 +336,7 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
     const bool leader = quad == 0 && lane == 0;
     uint8_t *const boxes = staging + half * 2 * C::kStagingBytes;
     float amax = 0.f;
-    uint32_t tile_i = 0, box = 0;
+    uint32_t acc_i = 0, box = 0;
     // A staging tile is free when the store before the last one has been read (the two tiles alternate).  Every turn commits a group, an empty
     // one where nothing was stored by TMA (a group's last tokens, a CTA without rows): "all but the last group" is then the tile's own.
     auto next_box = [&]() -> uint8_t * {
@@ -326,8 +347,43 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
     for (int t = tile_first; t < ntiles; t += tile_step) {
       const Tile p = tile_of(t);
       if (p.width == 0) continue;
-      const int tm = 2 * p.tm + rank, jt = p.j0, jend = min(p.j0 + p.width, p.jend), acc = nacc == 2 ? tile_i & 1 : 0;
-      const uint32_t acc_par = (nacc == 2 ? tile_i >> 1 : tile_i) & 1;
+      const int tm = 2 * p.tm + rank, jt = p.j0, jend = min(p.j0 + p.width, p.jend);
+      // this warp's block: width / 2 columns, one, two or four chunks of 32
+      const int hw = p.width >> 1, nchunks = min(hw, jend - jt - half * hw + 31) >> 5;   // (chunks past the last token are left alone)
+      uint32_t r[32], rn[32];
+      auto load_chunk = [&](uint32_t col, int c, uint32_t (&v)[32]) {
+        const uint32_t a = tmem_base + ((uint32_t)(quad * 32) << 16) + col + half * hw + 32 * c;
+        tmem_ld_16x256b_x4(a, v);
+        tmem_ld_16x256b_x4(a + (16u << 16), v + 16);
+      };
+      auto release = [&](int acc) {
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_rank(&tmem_empty[acc], 0);
+      };
+      if constexpr (SEG) {   // the running sums of chunk 0 are kept in r, those of chunk 1 in rn
+#pragma unroll
+        for (int q = 0; q < 32; ++q) r[q] = rn[q] = 0;
+        auto join = [&](uint32_t col, int c, uint32_t (&sum)[32]) {
+          uint32_t v[32];
+          load_chunk(col, c, v);
+          tmem_ld_wait32(v);
+#pragma unroll
+          for (int q = 0; q < 32; ++q) sum[q] = __float_as_uint(__fadd_rn(__uint_as_float(sum[q]), __uint_as_float(v[q])));
+        };
+        for (int ks = 0; ks < nk; ks += seg_stages, ++acc_i) {
+          const int acc = acc_i & 1;
+          if (!__all_sync(0xFFFFFFFFu, wait(&tmem_full[acc], (acc_i >> 1) & 1, kStWaitTmemFull))) { *abort_flag = 1; break; }
+          tc_fence_after();
+          if (nchunks > 0) join(acc * 128, 0, r);
+          if (nchunks > 1) join(acc * 128, 1, rn);
+          if (PLANES != 1 && ks + seg_stages >= nk) {
+            if (nchunks > 0) join(kSmallCols, 0, r);
+            if (nchunks > 1) join(kSmallCols, 1, rn);
+          }
+          release(acc);
+        }
+      }
       const int rb = tm * 128 + quad * 32 + (lane >> 2);
       const bool tile_ok = tm * 128 < gm;   // (an odd number of 128-row tiles leaves the last pair's second CTA without rows)
       float rowp[4], bias[4];               // row 8 q of this thread's four: alpha gA, bias
@@ -383,36 +439,34 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
           }
         }
       }
-      if (!wait(&tmem_full[acc], acc_par, kStWaitTmemFull)) *abort_flag = 1;
+      const int acc = nacc == 2 ? acc_i & 1 : 0;
+      if constexpr (!SEG) {
+        if (!wait(&tmem_full[acc], (nacc == 2 ? acc_i >> 1 : acc_i) & 1, kStWaitTmemFull)) *abort_flag = 1;
+        ++acc_i;
+      }
       named_barrier(1, 256);   // the eight epilogue warps go on together or not at all
       if (__any_sync(0xFFFFFFFFu, *abort_flag)) goto done;
       tc_fence_after();
-      // this warp's block: width / 2 columns, one, two or four chunks of 32.  The chunk after the next is requested while one is processed;
-      // the accumulator goes back to the MMA warp with the last chunk's load.  (A 256-column accumulator is alone in tensor memory: until
-      // then the weight stages fill up behind it, eight deep, and the MMAs catch up from there.)
-      const int hw = p.width >> 1, nchunks = min(hw, jend - jt - half * hw + 31) >> 5;   // (chunks past the last token are left alone)
-      const uint32_t acc_addr = tmem_base + ((uint32_t)(quad * 32) << 16) + acc * 128 + half * hw;
-      uint32_t r[32], rn[32];
-      auto load_chunk = [&](int c, uint32_t (&v)[32]) {
-        tmem_ld_16x256b_x4(acc_addr + 32 * c, v);
-        tmem_ld_16x256b_x4(acc_addr + (16u << 16) + 32 * c, v + 16);
-      };
-      auto release = [&]() {
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive_rank(&tmem_empty[acc], 0);
-      };
-      if (nchunks > 0) load_chunk(0, rn);
-      else release();
+      // One sum over k: the chunk after the next is requested while one is processed; the accumulator goes back to the MMA warp with the last
+      // chunk's load.  (A 256-column accumulator is alone in tensor memory: until then the weight stages fill up behind it, eight deep, and
+      // the MMAs catch up from there.)
+      if constexpr (!SEG) {
+        if (nchunks > 0) load_chunk(acc * 128, 0, rn);
+        else release(acc);
+      }
       for (int c = 0; c < nchunks; ++c) {
         __syncwarp();   // (the tensor memory loads and waits are warp-wide)
-        tmem_ld_wait32(rn);
+        if constexpr (!SEG) tmem_ld_wait32(rn);
+        if (!SEG || c != 0) {
 #pragma unroll
-        for (int q = 0; q < 32; ++q) r[q] = rn[q];
-        if (c + 1 < nchunks) load_chunk(c + 1, rn);
-        if (c == (nchunks > 1 ? nchunks - 2 : 0)) {   // every column of this warp's block is in registers
-          if (nchunks > 1) tmem_ld_wait32(rn);
-          release();
+          for (int q = 0; q < 32; ++q) r[q] = rn[q];
+        }
+        if constexpr (!SEG) {
+          if (c + 1 < nchunks) load_chunk(acc * 128, c + 1, rn);
+          if (c == (nchunks > 1 ? nchunks - 2 : 0)) {   // every column of this warp's block is in registers
+            if (nchunks > 1) tmem_ld_wait32(rn);
+            release(acc);
+          }
         }
         const int cc = half * hw + c * 32;   // first column of the chunk in the tile
         const int j0 = jt + cc;
@@ -480,7 +534,7 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
                 amax = fmaxf(amax, fabsf(__uint_as_float(r[16 * (q >> 1) + 4 * (ce >> 1) + 2 * (q & 1) + (ce & 1)])));
         }
         const int orow = glu ? tm * 64 : tm * 128, orows = glu ? gm >> 1 : gm;   // the tile's first output row, rows of D
-        if (d_dtype == NVFP4A_FP32) {   // eight lanes write 32 contiguous bytes of a column
+        if (!SEG && d_dtype == NVFP4A_FP32) {   // eight lanes write 32 contiguous bytes of a column
           float *const d32 = (float *)dptr + (size_t)j0 * g.e.ldd + orow + (lane >> 2);
 #pragma unroll
           for (int q = 0; q < 4; ++q) {
@@ -554,7 +608,6 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
         }
         if (leader) bulk_commit();
       }
-      ++tile_i;
     }
     if (leader) bulk_wait_all();
     if (g.e.amax) warp_amax_commit(g.e.amax, amax);
@@ -650,10 +703,10 @@ long long stage_cost(int width, int planes) {
 // Tile width and cut for a problem of `rows256` 256-row tiles and n tokens: the width whose rounds over the SM pairs cost least; the tiles of
 // the last round are cut in two while the pairs can take the halves all at once.
 struct Plan { int width, nfull, cut, tiles; };
-Plan make_plan(int rows256, int n, int planes, int pairs) {
+Plan make_plan(int rows256, int n, int planes, int pairs, int widest) {
   Plan best = {0, 0, 1, 0};
   long long best_cost = 0;
-  for (int w = 256; w >= 64; w /= 2) {
+  for (int w = widest; w >= 64; w /= 2) {
     if (w > 64 && w / 2 >= n) continue;   // half of the width covers every token
     const int tiles = rows256 * ((n + w - 1) / w), rest = tiles % pairs;
     int cut = 1;
@@ -669,11 +722,11 @@ Plan make_plan(int rows256, int n, int planes, int pairs) {
 
 // Grouped: only the average number of tokens per group is known here, and each group ends in a tile as wide as its last tokens (in steps
 // of 64).  `tiles` bounds the grid, the kernel counts the tiles itself.
-Plan make_grouped_plan(int rows256, int n, int groups, int planes, int pairs) {
+Plan make_grouped_plan(int rows256, int n, int groups, int planes, int pairs, int widest) {
   Plan best = {0, 0, 1, 0};
   long long best_cost = 0;
   const int avg = (n + groups - 1) / groups;
-  for (int w = 256; w >= 64; w /= 2) {
+  for (int w = widest; w >= 64; w /= 2) {
     const int whole = (avg - 1) / w, last = avg - whole * w;
     const long long tiles = (long long)rows256 * groups * (whole + 1);
     const long long cost = whole * stage_cost(w, planes) + stage_cost((last + 63) & ~63, planes);   // of a group's tiles in one row of tiles
@@ -689,7 +742,7 @@ Plan make_grouped_plan(int rows256, int n, int groups, int planes, int pairs) {
 
 template <int PLANES, bool F16, bool GROUPED = false>
 cudaError_t launch_cfg(const CUtensorMap &tw, const CUtensorMap &tb, const CUtensorMap &td, const PeerMaps &pm, const W4A16Args &a, cudaStream_t s) {
-  using C = Cfg<PLANES>;
+  using C = Cfg<PLANES, GROUPED>;
   static std::atomic<bool> attr_set[64];   // zero-initialised; set once per device (a repeated cudaFuncSetAttribute is harmless)
   int dev = 0;
   cudaGetDevice(&dev);
@@ -716,7 +769,7 @@ cudaError_t launch_cfg(const CUtensorMap &tw, const CUtensorMap &tb, const CUten
 
 // what every launch of the kernel shares: arguments, the schedule, the maps of the weights, of the activations (`row_bytes` bytes per
 // token, `pitch` between tokens) and of D
-bool set_up(const GemmArgs &g, int planes, int groups, const void *act, uint64_t row_bytes, uint64_t pitch, W4A16Args *a, CUtensorMap *tw, CUtensorMap *tb,
+bool set_up(const GemmArgs &g, int planes, bool f16, int groups, const void *act, uint64_t row_bytes, uint64_t pitch, W4A16Args *a, CUtensorMap *tw, CUtensorMap *tb,
             CUtensorMap *td) {
   memset(a, 0, sizeof *a);
   a->m = g.m; a->n = g.n; a->k = g.k;
@@ -724,8 +777,10 @@ bool set_up(const GemmArgs &g, int planes, int groups, const void *act, uint64_t
   a->e = g.e; a->x = g.x;
   a->status = kernel_status_device_ptr();
   a->tag = next_launch_tag();
-  const Plan p = groups ? make_grouped_plan((g.m + 255) / 256, g.n, groups, planes, device_sms() / 2) : make_plan((g.m + 255) / 256, g.n, planes, device_sms() / 2);
+  const int rows256 = (g.m + 255) / 256, pairs = device_sms() / 2, widest = f16 || groups ? kSegmentWidth : 256;
+  const Plan p = groups ? make_grouped_plan(rows256, g.n, groups, planes, pairs, widest) : make_plan(rows256, g.n, planes, pairs, widest);
   const uint64_t wrows = (uint64_t)g.m * (groups ? groups : 1);
+  a->seg_stages = g.k >= 1024 ? 4 : g.k >= 512 ? 2 : 1;
   a->width = p.width; a->nfull = p.nfull; a->cut = p.cut; a->tiles = p.tiles;
   const uint64_t wtiles = (uint64_t)((g.m + 127) / 128) * g.A.ktiles;
   if (g.A.image ? !make_tmap_bytes(tw, g.A.data, 128, 128, 128, 128, wtiles, kImgTileBytes)
@@ -780,8 +835,7 @@ bool gemm_w4a16_pushes(const GemmArgs &g) {
 }
 
 bool gemm_w4a16_supports(const GemmArgs &g) {
-  // FP16 activations: E4M3 scales (UE5M3 products leave FP16's range) and a 16-bit D -- with an FP32 D the CUDA-core kernel's ordered
-  // FP32 sums are closer to the exact value than the tensor cores'
+  // FP16 activations: E4M3 scales (UE5M3 products leave FP16's range) and a 16-bit D (the kernel's FP32 stores are for one sum over k)
   const bool f16 = g.B.dtype == NVFP4A_FP16 && !g.A.ue && g.e.d_dtype != NVFP4A_FP32;
   if ((g.B.dtype != NVFP4A_BF16 && !f16) || g.k < 64 || ((uintptr_t)g.B.data & 15) || g.B.ld % 8) return false;
   if (!g.A.image && (((uintptr_t)g.A.data & 15) || g.A.ld % 32 || ((uintptr_t)g.A.sc & 1))) return false;
@@ -835,9 +889,9 @@ bool gemm_w4a8_tc_supports(const GemmArgs &g) {
   return true;
 }
 
-// The same for nvfp4a_gemm_grouped: problems whose D is 16-bit (its rounding hides the order of the sums; an FP32 D keeps the exact block
-// sums of the DP4A kernel) and whose reduction is long enough to pay for the planes.  8 experts of 2048 x 4096 on 1100 tokens, INT8
-// quantization of the tokens included: 600 us on the DP4A kernel, 158 us here.
+// The same for nvfp4a_gemm_grouped: problems whose D is 16-bit (an FP32 D keeps the exact block sums of the DP4A kernel) and whose reduction
+// is long enough to pay for the planes and for segments no less exact than the DP4A kernel's ordered sums (see the head of the file).  8
+// experts of 2048 x 4096 on 1100 tokens, INT8 quantization of the tokens included: 602 us on the DP4A kernel, 132 us here.
 bool gemm_w4a8_grouped_supports(const GemmArgs &g, int groups) {
   return gemm_w4a8_tc_supports(g) && !g.A.image && groups <= kMaxGroups && g.k >= 512 && g.e.d_dtype != NVFP4A_FP32;
 }
@@ -858,7 +912,7 @@ cudaError_t launch_gemm_w4a8_tc(const GemmArgs &g, const int *seg, int groups, c
     CUtensorMap tw, tb, td;
     PeerMaps pm;
     memset(&pm, 0, sizeof pm);
-    if (!set_up(g, 3, seg ? groups : 0, planes, (uint64_t)g.k * 6, (uint64_t)g.k * 6, &a, &tw, &tb, &td)) e = cudaErrorInvalidValue;
+    if (!set_up(g, 3, false, seg ? groups : 0, planes, (uint64_t)g.k * 6, (uint64_t)g.k * 6, &a, &tw, &tb, &td)) e = cudaErrorInvalidValue;
     else if (seg) {
       a.seg = seg; a.groups = groups;
       e = launch_cfg<3, false, true>(tw, tb, td, pm, a, s);
@@ -871,7 +925,7 @@ cudaError_t launch_gemm_w4a8_tc(const GemmArgs &g, const int *seg, int groups, c
 cudaError_t launch_gemm_w4a16(const GemmArgs &g, cudaStream_t s) {
   W4A16Args a;
   CUtensorMap tw, tb, td;
-  if (!set_up(g, 1, 0, g.B.data, (uint64_t)g.k * 2, (uint64_t)g.B.ld * 2, &a, &tw, &tb, &td)) return cudaErrorInvalidValue;
+  if (!set_up(g, 1, g.B.dtype == NVFP4A_FP16, 0, g.B.data, (uint64_t)g.k * 2, (uint64_t)g.B.ld * 2, &a, &tw, &tb, &td)) return cudaErrorInvalidValue;
   PeerMaps pm;
   memset(&pm, 0, sizeof pm);
   if (gemm_w4a16_pushes(g)) {   // tensor parallel: the epilogue's TMA stores also go to every peer's copy of D

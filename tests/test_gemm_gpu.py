@@ -786,6 +786,42 @@ def test_w4a16_gemm_gives_the_same_bytes_every_time():
     assert kernel_status() == 0
 
 
+@pytest.mark.parametrize("k", [512, 576, 1024, 4096])
+@pytest.mark.parametrize("kind", ["fp16", "grouped_int8"])
+def test_long_sums_on_the_tensor_cores_are_joined_in_fp32(kind, k):
+    """The tensor cores truncate the running sum at every instruction, so that one chain over k = 4096 loses about 1e-5 of a sum of positive
+    terms, always downwards; the ordered CUDA-core kernels lose a few 1e-7.  FP16 activations and INT8 groups therefore sum segments of 256
+    values (128 below k = 1024).  The largest result before its rounding (amax) against 64 bits: at most one unit in the last place (2^-23)
+    of the segment's running sum, on average half of the segment's, for each of its 16 instructions, as much again for the FP32
+    additions of up to 16 segments, four more for the small terms, scales and the quantities rounded on the way."""
+    m, n = 300, 70
+    gen = torch.Generator(device="cuda").manual_seed(k)
+    w = torch.randint(1, 8, (m, k), generator=gen, device="cuda", dtype=torch.uint8)             # positive codes
+    ws = torch.randint(0x28, 0x48, (m, k // 16), generator=gen, device="cuda", dtype=torch.uint8)
+    packed = (w[:, 0::2] | (w[:, 1::2] << 4)).contiguous()
+    W = torch.tensor([0.0, 0.5, 1.0, 1.5, 2.0, 3.0, 4.0, 6.0], dtype=torch.float64, device="cuda")[w.long()]
+    W = (W.view(m, k // 16, 16) * ws.view(torch.float8_e4m3fn).double().unsqueeze(-1)).view(m, k)
+    ta, amax = tensor(packed, L.NVFP4, ws, k // 16), torch.zeros(1, dtype=torch.float32, device="cuda")
+    D = torch.zeros(n, m, dtype=torch.bfloat16, device="cuda")
+    td = tensor(D, L.BF16, amax=amax)
+    if kind == "fp16":
+        x = (torch.rand(n, k, generator=gen, device="cuda") + 0.01).half()
+        X, tb = x.double(), tensor(x, L.FP16)
+        L.check(L.lib.nvfp4a_gemm(m, n, k, 1.0, ctypes.byref(ta), k, ctypes.byref(tb), k, 0.0, None, 0, ctypes.byref(td), m, None, stream()))
+        assert L.lib.nvfp4a_b200_last_route() == 5
+    else:
+        x, xs = torch.randint(1, 128, (n, k), generator=gen, device="cuda", dtype=torch.int8), torch.rand(n, k // 16, generator=gen, device="cuda") + 0.01
+        X = (x.double().view(n, k // 16, 16) * xs.double().unsqueeze(-1)).view(n, k)
+        tb, seg = tensor(x, L.INT8, xs, k // 16), torch.tensor([0, n], dtype=torch.int32, device="cuda")
+        L.check(L.lib.nvfp4a_gemm_grouped(1, m, k, n, 1.0, ctypes.byref(ta), k, ctypes.byref(tb), k, 0.0, None, 0, ctypes.byref(td), m, None,
+                                          ctypes.c_void_p(seg.data_ptr()), stream()))
+        assert L.lib.nvfp4a_b200_last_route() == 8
+    want = X @ W.t()
+    assert abs(float(amax.double()) / float(want.max()) - 1.0) <= (16 + 16 + 4) * 2.0 ** -24
+    assert torch.allclose(D.double(), want, rtol=2.0 ** -8, atol=0.0)
+    assert kernel_status() == 0
+
+
 @pytest.mark.parametrize("case", ["odd_row_tiles", "swiglu", "grouped"])
 def test_tma_stored_tiles_equal_plain_stores_on_every_launch(case):
     """A 16-bit D leaves through two alternating staging tiles and TMA stores.  Short reductions (the next tile's results arrive soon), several
