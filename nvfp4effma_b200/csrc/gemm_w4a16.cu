@@ -444,8 +444,9 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
         if (!wait(&tmem_full[acc], (nacc == 2 ? acc_i >> 1 : acc_i) & 1, kStWaitTmemFull)) *abort_flag = 1;
         ++acc_i;
       }
-      named_barrier(1, 256);   // the eight epilogue warps go on together or not at all
-      if (__any_sync(0xFFFFFFFFu, *abort_flag)) goto done;
+      // the eight epilogue warps go on together or not at all (another role may raise the flag between two warps' looks at it, and a warp that
+      // leaves alone would keep the others at their next barrier)
+      if (named_barrier_or(1, 256, *abort_flag != 0)) goto done;
       tc_fence_after();
       // One sum over k: the chunk after the next is requested while one is processed; the accumulator goes back to the MMA warp with the last
       // chunk's load.  (A 256-column accumulator is alone in tensor memory: until then the weight stages fill up behind it, eight deep, and

@@ -326,8 +326,7 @@ gemm_w4a4_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
       bool okw;
       okw = wait(&tmem_full[acc], (tile_i / ACC) & 1, kStatusWaitTmemFull);
       if (!okw) *abort_flag = 1;
-      named_barrier(bar_id, 128);
-      if (*abort_flag) goto done;
+      if (named_barrier_or(bar_id, 128, *abort_flag != 0)) goto done;   // (one answer for the four warps, whoever raises the flag in between)
       tc_fence_after();
       const int nchunks = min(BN / 32, (gn - tn * BN + 31) / 32);
       // Swapped operands: this lane is token jt and the accumulator's columns are 32 consecutive rows of D, which lie side by

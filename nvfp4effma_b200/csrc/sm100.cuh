@@ -171,6 +171,14 @@ __device__ __forceinline__ void bulk_wait_read_one() { asm volatile("cp.async.bu
 __device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 // barrier among `threads` threads of the CTA (id 1..15; 0 is __syncthreads)
 __device__ __forceinline__ void named_barrier(int id, int threads) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
+// the same, and whether `pred` held in any of them: one answer for all
+__device__ __forceinline__ bool named_barrier_or(int id, int threads, bool pred) {
+  uint32_t any;
+  __syncwarp();   // (lanes may come from a wait of their own)
+  asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %3, 0;\n\tbar.red.or.pred q, %1, %2, p;\n\tselp.u32 %0, 1, 0, q;\n\t}"
+               : "=r"(any) : "r"(id), "r"(threads), "r"((uint32_t)pred) : "memory");
+  return any != 0;
+}
 __device__ __forceinline__ void prefetch_tensormap(const CUtensorMap *map) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(map) : "memory");
 }
