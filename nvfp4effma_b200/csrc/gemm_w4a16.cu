@@ -686,6 +686,8 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
   }
 done:
   __syncwarp();
+  if (*abort_flag) { bulk_wait_all(); settle_after_abort(); }
+  __syncwarp();
   tc_fence_before();
   cluster_sync_all();   // neither CTA leaves (or frees tensor memory) while the other may still arrive on its barriers
   if (warp == 1) {

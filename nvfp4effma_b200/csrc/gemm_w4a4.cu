@@ -606,6 +606,8 @@ gemm_w4a4_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
   }
 done:
   __syncwarp();   // lanes that left a role's loop early rejoin their warp before the aligned barriers below
+  if (*abort_flag) { bulk_wait_all(); settle_after_abort(); }
+  __syncwarp();
   tc_fence_before();
   if (PAIR) cluster_sync_all();   // neither CTA leaves (or frees tensor memory) while the other may still arrive on its barriers
   else __syncthreads();

@@ -367,6 +367,8 @@ gemm_w4a4_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_c
   }
 done:
   __syncwarp();
+  if (*abort_flag) { bulk_wait_all(); settle_after_abort(); }
+  __syncwarp();
   tc_fence_before();
   cluster_sync_all();   // neither CTA leaves (or frees tensor memory) while the other may still arrive on its barriers
   if (warp == 1) {

@@ -169,6 +169,11 @@ __device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.comm
 __device__ __forceinline__ void bulk_wait_read_all() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
 __device__ __forceinline__ void bulk_wait_read_one() { asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory"); }
 __device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
+// After a wait that gave up: copies and MMAs that were already issued land within microseconds; the CTA keeps its shared and tensor memory for
+// 0.1 ms more (a fixed time: their barriers may never complete).
+__device__ __forceinline__ void settle_after_abort() {
+  for (const long long t0 = clock64(); clock64() - t0 < 200000;) {}
+}
 // barrier among `threads` threads of the CTA (id 1..15; 0 is __syncthreads)
 __device__ __forceinline__ void named_barrier(int id, int threads) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
 // the same, and whether `pred` held in any of them: one answer for all
