@@ -120,6 +120,19 @@ __device__ __forceinline__ void e2m1_expand4(uint32_t w, const uint4 &t, uint32_
   o1 = byte_perm(lo, hi, 0x7362u);
 }
 
+// Data that another kernel (programmatic dependent launch) or a peer writes until a wait of this kernel returns: `p` after the wait is a value the
+// compiler cannot have known before, so no load through it moves up across the wait.  ld16 is an ordinary load (not ld.global.nc, which
+// promises that nobody writes during the kernel's lifetime) that the compiler may otherwise schedule as freely as a read-only one.
+template <typename V> __device__ __forceinline__ const V *behind_wait(const V *p) {
+  asm volatile("" : "+l"(p) :: "memory");
+  return p;
+}
+__device__ __forceinline__ uint4 ld16(const uint4 *p) {
+  uint4 v;
+  asm("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  return v;
+}
+
 // ---- block scale addressing ----------------------------------------------------------------------------------------
 // ld > 0: linear, ld scales per row.  ld < 0: swizzled 128 x 4 tiles, -ld = padded scale columns.
 struct ScalePos {

@@ -323,7 +323,7 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
     // ---------------- epilogue ----------------
     const int quad = warp & 3, half = (warp - 4) >> 2, bar_id = 2 + half;   // barrier 1: all eight warps; 2 and 3: the four of a half
     // (rarely used parameters are read from the constant bank where they are needed: the registers belong to the accumulator block)
-    const float gb0 = g.e.gb ? __ldg(g.e.gb) : 1.f;   // B's global: dense B has none, INT8 B one for the tensor (a multiply by 1 is exact)
+    const float gb0 = g.e.gb ? *g.e.gb : 1.f;   // B's global: dense B has none, INT8 B one for the tensor (a multiply by 1 is exact)
     uint8_t *const dptr = (uint8_t *)g.e.d;
     const int d_dtype = g.e.d_dtype, mask = SEG ? 0 : g.x.mask;   // (segments: a 16-bit D and the plain epilogue)
     const bool d_tma = g.d_tma;
@@ -629,7 +629,7 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
       for (int h = 0; h < 2; ++h) {
         const int ks = 4 * sl + group + 2 * h;
         const size_t off = img ? (size_t)sl * kImgTileBytes + (ks & 3) * 512 : swz ? (size_t)ks * 512 : (size_t)ks * 4;
-        v[h] = ks < nk ? __ldg((const uint32_t *)(scp + off)) : 0u;
+        v[h] = ks < nk ? *(const uint32_t *)(scp + off) : 0u;
       }
     };
     uint32_t isl = 0, it0 = 0;   // slots so far; stages of the finished tiles

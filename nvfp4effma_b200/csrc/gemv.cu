@@ -103,7 +103,7 @@ __global__ void __launch_bounds__(kGemvWarps * 32, 3) gemv_kernel(const GemvArgs
   // rows of this lane (clamped for the loads; rows past m are never stored)
   const int r0 = min(i0 + gq, gm - 1), r1 = min(i0 + gq + 8, gm - 1);
   const bool has_col = gq < gn;
-  const uint4 *xrow = (const uint4 *)(g.x + (size_t)(has_col ? gq : 0) * g.ldx);
+  const uint4 *xrow = (const uint4 *)(behind_wait(g.x) + (size_t)(has_col ? gq : 0) * g.ldx);
   const uint8_t *a0p, *a1p, *s0p, *s1p;
   if (LAYOUT != 2) {
     const ScalePos sp{g.A.sld};
@@ -142,7 +142,7 @@ __global__ void __launch_bounds__(kGemvWarps * 32, 3) gemv_kernel(const GemvArgs
       v.sc1 = __ldg((const uint16_t *)(s1p + soff));
     }
 #pragma unroll
-    for (int i = 0; i < 4; ++i) v.x[i] = (in && has_col) ? __ldg(xrow + 4 * c + i) : make_uint4(0, 0, 0, 0);
+    for (int i = 0; i < 4; ++i) v.x[i] = (in && has_col) ? ld16(xrow + 4 * c + i) : make_uint4(0, 0, 0, 0);
     return v;
   };
 

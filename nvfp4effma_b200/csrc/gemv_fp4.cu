@@ -156,6 +156,7 @@ gemv_fp4_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
   pdl_wait();
   // tensor-parallel layers in the deferred form: the activations are complete once every peer has posted the previous gather
   if (g.tp_world > 1) tp_wait_posts(g.tp_flags, g.tp_world, g.tp_rank, g.status, g.tag, g.tp_wait_cycles);
+  const uint16_t *const x = behind_wait(g.x);
   // the decomposition warps ask for their activations first: the loads fly while the barrier below gathers the CTA
   const int t2 = threadIdx.x - 64, nvec = nloc * 32;  // vectors of 8 consecutive k; at most 2 per thread and token
   uint4 xq[NTOK][2];
@@ -165,7 +166,7 @@ gemv_fp4_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
 #pragma unroll
       for (int u = 0; u < 2; ++u) {
         const int v = t2 + u * kDecompThreads;
-        xq[t][u] = (t < gn && v < nvec) ? __ldg((const uint4 *)(g.x + (size_t)t * g.ldx + (size_t)c0 * 256) + v) : make_uint4(0, 0, 0, 0);
+        xq[t][u] = (t < gn && v < nvec) ? ld16((const uint4 *)(x + (size_t)t * g.ldx + (size_t)c0 * 256) + v) : make_uint4(0, 0, 0, 0);
       }
   }
 

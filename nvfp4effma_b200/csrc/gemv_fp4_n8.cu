@@ -201,12 +201,13 @@ gemv_fp4_n8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
     tp_wait_posts(g.tp_flags, g.tp_world, g.tp_rank, g.status, g.tag, g.tp_wait_cycles);
     __syncthreads();
   }
+  const uint16_t *const x = behind_wait(g.x);
   // The decomposition warps ask for their activations first.  The CTA's activations are gn x nvec vectors of 8 consecutive k, dealt to the 256 threads in one run (a warp's vectors belong to one token).
   const int t2 = threadIdx.x - 64, nvec = nloc * 32, items = gn * nvec;
   uint4 xq[NI];
   auto load_x = [&](int idx) {
     const int t = idx / nvec, v = idx - t * nvec;
-    return __ldg((const uint4 *)(g.x + (size_t)t * g.ldx + (size_t)c0 * 256) + v);
+    return ld16((const uint4 *)(x + (size_t)t * g.ldx + (size_t)c0 * 256) + v);
   };
   if (warp >= 2 && warp < 10) {
 #pragma unroll

@@ -81,6 +81,7 @@ __device__ __forceinline__ void fence_proxy_async_smem() { asm volatile("fence.p
 // before it touches any memory the predecessor reads or writes: the wait returns when the predecessor has completed and its
 // writes are visible.  Both are no-ops in a launch without the attribute or without a predecessor.
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// (What the previous kernel wrote is read with ordinary loads: see behind_wait.)
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // ---- thread-block clusters: rank, barrier, loads from a peer CTA's shared memory ---------------------------------------------

@@ -25,6 +25,23 @@ def test_every_declared_symbol_is_exported():
         assert n in L.EXPORTS, f"{n} has no ctypes prototype"
 
 
+def test_kernels_that_start_before_their_producer_ends_use_no_read_only_loads():
+    """`ld.global.nc` (`__ldg`) is for data that nobody writes during the kernel's lifetime.  A kernel under programmatic dependent launch begins
+    while its predecessor writes, and a deferred tensor-parallel GEMV while the peers do."""
+    csrc = os.path.join(ROOT, "nvfp4effma_b200", "csrc")
+    early = []
+    for name in sorted(os.listdir(csrc)):
+        if not name.endswith(".cu"):
+            continue
+        text = re.sub(r"//.*", "", open(os.path.join(csrc, name)).read())
+        if "pdl_wait()" in text:
+            early.append(name)
+            assert "__ldg(" not in text and "ld.global.nc" not in text, name
+        elif "tp_wait_posts(" in text:
+            assert "__ldg(xrow" not in text and "__ldg(g.x" not in text, name
+    assert len(early) >= 4, early
+
+
 def test_struct_layouts_match_the_reference_abi():
     # field order / offsets of nvfp4a_tensor on LP64 (reference include/nvfp4effma.h:46-57)
     T = L.Tensor
