@@ -155,7 +155,10 @@ gemv_fp4_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
   if (warp == 1) tmem_alloc(tmem_slot, kTmemCols);
   pdl_wait();
   // tensor-parallel layers in the deferred form: the activations are complete once every peer has posted the previous gather
-  if (g.tp_world > 1) tp_wait_posts(g.tp_flags, g.tp_world, g.tp_rank, g.status, g.tag, g.tp_wait_cycles);
+  if (g.tp_world > 1) {
+    tp_wait_posts(g.tp_flags, g.tp_world, g.tp_rank, g.status, g.tag, g.tp_wait_cycles);
+    __syncthreads();   // (a few threads wait for all)
+  }
   const uint16_t *const x = behind_wait(g.x);
   // the decomposition warps ask for their activations first: the loads fly while the barrier below gathers the CTA
   const int t2 = threadIdx.x - 64, nvec = nloc * 32;  // vectors of 8 consecutive k; at most 2 per thread and token

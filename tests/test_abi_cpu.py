@@ -42,6 +42,15 @@ def test_kernels_that_start_before_their_producer_ends_use_no_read_only_loads():
     assert len(early) >= 4, early
 
 
+def test_deferred_tensor_parallel_gemvs_read_activations_behind_a_cta_barrier():
+    """tp_wait_posts is executed by `world` threads of a CTA; the others know that the peers have posted only after a CTA barrier."""
+    csrc = os.path.join(ROOT, "nvfp4effma_b200", "csrc")
+    for name in ("gemv.cu", "gemv_fp4.cu", "gemv_fp4_n8.cu"):
+        text = re.sub(r"//.*", "", open(os.path.join(csrc, name)).read())
+        after = text[text.index("tp_wait_posts("):]
+        assert after.index("__syncthreads()") < after.index("behind_wait(") <= after.index("ld16("), name
+
+
 def test_struct_layouts_match_the_reference_abi():
     # field order / offsets of nvfp4a_tensor on LP64 (reference include/nvfp4effma.h:46-57)
     T = L.Tensor
