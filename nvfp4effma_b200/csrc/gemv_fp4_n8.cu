@@ -52,6 +52,7 @@ namespace {
 struct GemvN8Args {
   int m, n, k;
   int a_image;
+  Fp4Operand A;        // (for code_7f_sum)
   const uint8_t *sa;   // plain: block scale base; image: image base
   int sa_ld, ktiles;
   int linear;          // plain operand with linear block scales: a TMA box brings [256 rows][16 bytes], four warps re-tile it
@@ -106,6 +107,21 @@ __device__ __forceinline__ void transpose_nibbles(const uint32_t (&x)[8], uint32
     out[4 + h] = byte_perm(c01, c23, 0x5410u);
     out[6 + h] = byte_perm(c01, c23, 0x7632u);
   }
+}
+
+// Block scale code 0x7F (with either sign) is 480 everywhere in this library, as in the reference's decode; the tensor cores take it for a NaN, which
+// reaches the partial sums of that weight row and of no other (activations and weights are finite here).  Such a row's sum over the CTA's
+// blocks [b0, b1) on the CUDA cores, from memory, in the order of the CUDA-core consumer below; never met in a matrix that a quantizer made from finite
+// values.  (Inlined: as a function it costs every launch 4 us.)
+__device__ __forceinline__ float code_7f_sum(const Fp4Operand &A, const uint16_t *x, int row, int b0, int b1) {
+  float acc = 0.f;
+  for (int b = b0; b < b1; ++b) {
+    const uint2 w = A.block(row, b);
+    float part = 0.f;
+    for (int i = 0; i < 16; ++i) part = __fmaf_rn((float)e2m1_x2(((i < 8 ? w.x : w.y) >> (4 * (i & 7))) & 15u), __uint_as_float((uint32_t)x[16 * b + i] << 16), part);
+    acc = __fmaf_rn(__fmul_rn(A.scale(row, b), 0.5f), part, acc);
+  }
+  return acc;
 }
 
 template <int NTOK>
@@ -429,6 +445,7 @@ gemv_fp4_n8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
           ok = __all_sync(0xFFFFFFFFu, wait(acc_full, ti & 1, kStWaitAcc));
           tc_fence_after();
           const int ntq = min(gn - 2 * quad, 2);   // tokens in this quadrant's lanes
+          uint32_t nans = 0;   // this lane's sums that are not numbers, two per turn
 #pragma unroll 1
           for (int tq = 0; tq < 2 * ntq; ++tq) {     // 64 columns of one token per turn
             const int tok = 2 * quad + (tq >> 1), q = tq & 1;
@@ -457,10 +474,18 @@ gemv_fp4_n8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
             float *d = slot + tok * rows_per + row % rows_per;
             st_peer_f32(d, owner, __fmul_rn(__fmul_rn(v[0], s1), s2));
             st_peer_f32(d + 1, owner, __fmul_rn(__fmul_rn(v[1], s1), s2));
+            nans |= (uint32_t)(v[0] != v[0]) << (2 * tq) | (uint32_t)(v[1] != v[1]) << (2 * tq + 1);
           }
           tc_fence_before();
           __syncwarp();
           if (lane == 0) mbar_arrive(acc_empty);   // the MMA warp may start the next tile
+          if (nans) {
+            for (int b = 0; b < 8; ++b) {
+              const int tok = 2 * quad + (b >> 2), row = half * 128 + ((b >> 1) & 1) * 64 + 2 * lane + (b & 1), i = tm * 256 + row;
+              if ((nans >> b & 1u) && i < gm)
+                st_peer_f32(slot + tok * rows_per + row % rows_per, row / rows_per, code_7f_sum(g.A, x + (size_t)tok * g.ldx, i, 16 * c0, 16 * c1));
+            }
+          }
         }
       } else {
         float acc[NTOK];
@@ -636,6 +661,7 @@ cudaError_t launch_gemv_fp4_n8(const GemmArgs &g, cudaStream_t s) {
   }
   a.ktiles = (g.k + kImgK - 1) / kImgK;
   a.a_image = g.A.image;
+  a.A = g.A;
   CUtensorMap ta, ts;
   memset(&ts, 0, sizeof ts);
   if (g.A.image) {

@@ -268,3 +268,28 @@ def test_negative_block_scales_of_several_vectors(pin, layout):
         assert L.lib.nvfp4a_b200_last_route() == FP4_GEMV, c
         check_bound(c, h, got, amax, exp)
     assert kernel_status() == 0
+
+
+@pytest.mark.parametrize("layout", ["image", "swizzled", "linear"])
+def test_block_scale_code_7f_of_several_vectors(pin, layout):
+    """Codes 0x7F and 0xFF decode as +-480 (a NaN to the tensor cores) in a few blocks, in the first and last row and in the last block of a row."""
+    from util import rand_fp4
+    for i, (splits, m, n, k) in enumerate([(1, 300, 5, 768), (2, 515, 3, 1024), (8, 4096 + 300, 8, 2048)]):
+        pin(splits)
+        c = Case(m, n, k, L.BF16, L.FP32, -1, L.BF16, 1.25, 0.0, fa=SW if layout == "swizzled" else 0)
+        h = build_case(c, 1500 + i)
+        rng = np.random.default_rng(1500 + i)
+        if layout == "linear":
+            h["A"] = rand_fp4(rng, m, k, ld=h["lda"], ld_scale=k // 16, glob=0.375)
+        sc = h["A"].scales
+        sc[rng.integers(0, sc.size, 1 + sc.size // 500)] = 0x7F
+        sc[rng.integers(0, sc.size, 1 + sc.size // 500)] = 0xFF
+        sc[0] = 0x7F
+        if layout == "linear":
+            sc[(m - 1) * (k // 16) + k // 16 - 1] = 0xFF
+        exp = oracle_case(c, h, want_ref=True)
+        got, amax = run_tc(c, h, gemv=True) if layout == "image" else run_gemm(c, h)
+        assert L.lib.nvfp4a_b200_last_route() == FP4_GEMV, c
+        assert np.isfinite(exp["ref64"]).all()
+        check_bound(c, h, got, amax, exp)
+    assert kernel_status() == 0
