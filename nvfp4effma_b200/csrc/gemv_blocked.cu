@@ -16,8 +16,9 @@
 // flight while it computes one.  The lanes' and warps' sums are added in a fixed order, then the tile runs the plain or extended epilogue.
 //
 // What bounds it: instruction issue (decoding: 11 instructions per 8 weights) and the loads in flight (registers: 16 warps per SM).
-// 14336 x 4096 with 1 / 4 / 8 vectors: 27.5 / 32.1 / 39.0 us with a warp per four rows, DP4A and no prefetch; 15.9 / 19.9 / 28.2 us here
-// (HBM time 5.1 us).  1024 x 1024 pays 0.1 to 0.4 us for the longer code (4 / 8 vectors: 3.6 / 4.2 -> 3.8 / 4.6 us; a call's host work is above 10 us).
+// 14336 x 4096 with 1 / 4 / 8 vectors: 27.5 / 32.1 / 39.0 us with a warp per four rows, DP4A and no prefetch; 16.1 / 19.7 / 27.9 us here
+// (HBM time 5.1 us).  Small matrices are bound by fetching the code: 1024 x 1024 with 1 / 4 / 8 vectors 3.0 / 3.55 / 4.1 us then, 3.1 / 3.6 / 4.4
+// unrolled, 2.7 / 3.1 / 3.7 in the form for one unit per warp (CUDA graph); 256 x 64 with eight 3.6, 4.5, 3.1.
 #include <atomic>
 #include "operands.cuh"
 
@@ -31,7 +32,6 @@ constexpr int kSmemLimit = 200 * 1024;
 struct GemvQArgs {
   int m, n, k;
   int ksplit;          // warps that share a group of 16 rows
-  int halves;          // 128-value halves per unit: 2, or 1 (only if no warp has more than one unit of a row)
   Fp4Operand A;
   BOperand B;
   Epilogue e;
@@ -56,7 +56,10 @@ __device__ __forceinline__ void mma_s8(int (&c)[4], const uint32_t (&a)[4], uint
       : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
-template <int P>   // pairs of activation vectors
+// P: pairs of activation vectors.  HALVES: 128-value halves per unit of a warp, 2 or 1.  ONE: a warp has one unit of a tile at most (any n up to 8),
+// whose pairs go through one short loop and leave for the epilogue at once -- the unrolled form of eight vectors is bound by fetching its
+// code there.
+template <int P, int HALVES, bool ONE>
 __global__ void __launch_bounds__(32 * kMaxWarps, 1) gemv_blocked_kernel(const GemvQArgs g) {
   extern __shared__ __align__(16) uint8_t smem[];
   __shared__ float colscale[2 * P];
@@ -71,7 +74,7 @@ __global__ void __launch_bounds__(32 * kMaxWarps, 1) gemv_blocked_kernel(const G
   // ---- rows ----
   const int T = blockDim.x, W = T >> 5, S = g.ksplit, G = W / S, kRows = 16 * G;   // S warps share a group of 16 rows, G groups are a tile
   const int tiles = (gm + kRows - 1) / kRows;
-  const int nchunks = gk >> 5, halves = g.halves, units = (nchunks + 4 * halves - 1) / (4 * halves);   // a chunk: 32 values = 16 bytes = two blocks; a unit: 8 chunks (or 4)
+  const int nchunks = gk >> 5, units = (nchunks + 4 * HALVES - 1) / (4 * HALVES);   // a chunk: 32 values = 16 bytes = two blocks; a unit: 8 chunks (or 4)
   const int grp = warp / S, ws = warp - grp * S, gq = lane >> 2, tq = lane & 3;
   // A unit of a row: 128 bytes of nibbles, `du` bytes from the row's previous unit, and sixteen scale codes, `ds` from the previous ones
   // (linear: in sequence; swizzled and image: four to each 512-byte tile).
@@ -81,7 +84,7 @@ __global__ void __launch_bounds__(32 * kMaxWarps, 1) gemv_blocked_kernel(const G
   const uint8_t *pw[2], *ps[2];
   int c_next = 0;
   auto start_row = [&](int tile, int v) {   // the lane's pointers to unit v of its two rows of a tile
-    const int u = halves == 2 ? v : v >> 1, odd = halves == 2 ? 0 : v & 1;   // 256-value unit, its second half
+    const int u = HALVES == 2 ? v : v >> 1, odd = HALVES == 2 ? 0 : v & 1;   // 256-value unit, its second half
 #pragma unroll
     for (int r = 0; r < 2; ++r) {
       const int row = min(tile * kRows + 16 * grp + gq + 8 * r, gm - 1), rr = row & 127;
@@ -103,7 +106,7 @@ __global__ void __launch_bounds__(32 * kMaxWarps, 1) gemv_blocked_kernel(const G
   auto prefetch = [&]() {
 #pragma unroll
     for (int h = 0; h < 2; ++h)
-      if (h < halves && c_next + 4 * h < nchunks)
+      if (h < HALVES && c_next + 4 * h < nchunks)
 #pragma unroll
         for (int r = 0; r < 2; ++r) {
           w_next[h][r] = __ldg((const uint4 *)(pw[r] + 64 * h));
@@ -143,12 +146,68 @@ __global__ void __launch_bounds__(32 * kMaxWarps, 1) gemv_blocked_kernel(const G
   __syncthreads();
 
   const bool diag = (gq >> 1) == tq;   // this lane's column of B is its own chunk's (see the head of the file)
+  // two vectors j0, j0 + 1 against the lane's chunk c: use(row r, vector jj, the two blocks' sums times the weight scales, their activation scales)
+  auto block_sums = [&](const uint32_t (&a)[4][4], const float (&sa)[2][2], int j0, int c, bool in, auto use) {
+    const int jb = j0 + (gq & 1);
+    uint4 x0 = make_uint4(0, 0, 0, 0), x1 = x0;
+    if (diag && in && jb < gn) {
+      x0 = *(const uint4 *)(xq + (size_t)jb * gk + 32 * c);
+      x1 = *(const uint4 *)(xq + (size_t)jb * gk + 32 * c + 16);
+    }
+    // (an integer sum of at most 16 x 12 x 128 added to the bits of 1.5 * 2^23 is that float's value plus the sum)
+    int c0[4] = {0x4B400000, 0x4B400000, 0x4B400000, 0x4B400000}, c1[4] = {0x4B400000, 0x4B400000, 0x4B400000, 0x4B400000};
+    mma_s8(c0, a[0], x0.x, x0.y);
+    mma_s8(c1, a[2], x1.x, x1.y);
+    mma_s8(c0, a[1], x0.z, x0.w);
+    mma_s8(c1, a[3], x1.z, x1.w);
+#pragma unroll
+    for (int jj = 0; jj < 2; ++jj) {
+      float2 xsv = make_float2(0.f, 0.f);
+      if (in) xsv = *(const float2 *)(xs + min(j0 + jj, gn - 1) * nb + 2 * c);
+#pragma unroll
+      for (int r = 0; r < 2; ++r)
+        use(r, jj, __fmul_rn(__fadd_rn(__int_as_float(c0[2 * r + jj]), -12582912.f), sa[r][0]),
+            __fmul_rn(__fadd_rn(__int_as_float(c1[2 * r + jj]), -12582912.f), sa[r][1]), xsv.x, xsv.y);
+    }
+  };
   const Epilogue &e = g.e;
   float amax = 0.f;
   int buf = 0;
 #pragma unroll 1
   for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x, buf ^= 1) {
   const int i0 = tile * kRows;
+  if constexpr (ONE) {
+    float *const mine = part + ((size_t)buf * W + warp) * gn * 16;
+    const int c = c_next;
+    const bool in = c < nchunks;   // (a lane past the end multiplies zeros)
+    uint32_t a[4][4];              // [word][MMA operand register]
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      dec8(((const uint32_t *)&w_next[0][0])[i], a[i][0], a[i][2]);
+      dec8(((const uint32_t *)&w_next[0][1])[i], a[i][1], a[i][3]);
+    }
+    float sa[2][2];
+#pragma unroll
+    for (int r = 0; r < 2; ++r) { sa[r][0] = scale_to_f32(sc_next[0][r] & 0xFFu, ue_a); sa[r][1] = scale_to_f32(sc_next[0][r] >> 8, ue_a); }
+    if (tile + (int)gridDim.x < tiles) {
+      start_row(tile + gridDim.x, ws);
+      prefetch();
+    }
+#pragma unroll 1
+    for (int j0 = 0; j0 < gn; j0 += 2) {
+      float v[2][2];
+      block_sums(a, sa, j0, c, in, [&](int r, int jj, float s0, float s1, float x0, float x1) { v[r][jj] = __fmaf_rn(s1, x1, __fmul_rn(s0, x0)); });
+#pragma unroll
+      for (int jj = 0; jj < 2; ++jj)
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+          float t = v[r][jj];
+          t = __fadd_rn(t, __shfl_xor_sync(0xFFFFFFFFu, t, 1));
+          t = __fadd_rn(t, __shfl_xor_sync(0xFFFFFFFFu, t, 2));
+          if (tq == 0 && j0 + jj < gn) mine[(j0 + jj) * 16 + gq + 8 * r] = t;
+        }
+    }
+  } else {
   float acc[2][2 * P];
 #pragma unroll
   for (int j = 0; j < 2 * P; ++j) acc[0][j] = acc[1][j] = 0.f;
@@ -163,16 +222,16 @@ __global__ void __launch_bounds__(32 * kMaxWarps, 1) gemv_blocked_kernel(const G
       for (int r = 0; r < 2; ++r) { w[h][r] = w_next[h][r]; sc[h][r] = sc_next[h][r]; }
     if (u + S < units) {
 #pragma unroll
-      for (int r = 0; r < 2; ++r) { pw[r] += (size_t)S * du; ps[r] += (size_t)S * ds; }
-      c_next += 8 * S;
+      for (int r = 0; r < 2; ++r) { pw[r] += (size_t)(S * HALVES / 2) * du; ps[r] += (size_t)(S * HALVES / 2) * ds; }   // (several 128-value units: S is 8)
+      c_next += 4 * HALVES * S;
       prefetch();
     } else if (tile + (int)gridDim.x < tiles) {
       start_row(tile + gridDim.x, ws);
       prefetch();
     }
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      if (h == halves) break;
+    for (int h = 0; h < HALVES; ++h) {
+      if (P == 4 && h) __syncwarp();   // (keeps the compiler from interleaving the halves, for which the registers do not suffice)
       const int c = c_unit + 4 * h;
       const bool in = c < nchunks;       // (a lane past the end multiplies zeros and leaves its sums alone)
       uint32_t a[4][4];                  // [word][MMA operand register]
@@ -187,29 +246,10 @@ __global__ void __launch_bounds__(32 * kMaxWarps, 1) gemv_blocked_kernel(const G
 #pragma unroll
       for (int p = 0; p < P; ++p) {
         if (2 * p >= gn) break;
-        const int jb = 2 * p + (gq & 1);
-        uint4 x0 = make_uint4(0, 0, 0, 0), x1 = x0;
-        if (diag && in && jb < gn) {
-          x0 = *(const uint4 *)(xq + (size_t)jb * gk + 32 * c);
-          x1 = *(const uint4 *)(xq + (size_t)jb * gk + 32 * c + 16);
-        }
-        // (an integer sum of at most 16 x 12 x 128 added to the bits of 1.5 * 2^23 is that float's value plus the sum)
-        int c0[4] = {0x4B400000, 0x4B400000, 0x4B400000, 0x4B400000}, c1[4] = {0x4B400000, 0x4B400000, 0x4B400000, 0x4B400000};
-        mma_s8(c0, a[0], x0.x, x0.y);
-        mma_s8(c1, a[2], x1.x, x1.y);
-        mma_s8(c0, a[1], x0.z, x0.w);
-        mma_s8(c1, a[3], x1.z, x1.w);
-#pragma unroll
-        for (int jj = 0; jj < 2; ++jj) {
-          const int j = 2 * p + jj;
-          float2 xsv = make_float2(0.f, 0.f);
-          if (in) xsv = *(const float2 *)(xs + min(j, gn - 1) * nb + 2 * c);
-#pragma unroll
-          for (int r = 0; r < 2; ++r) {
-            acc[r][j] = __fmaf_rn(__fmul_rn(__fadd_rn(__int_as_float(c0[2 * r + jj]), -12582912.f), sa[r][0]), xsv.x, acc[r][j]);
-            acc[r][j] = __fmaf_rn(__fmul_rn(__fadd_rn(__int_as_float(c1[2 * r + jj]), -12582912.f), sa[r][1]), xsv.y, acc[r][j]);
-          }
-        }
+        block_sums(a, sa, 2 * p, c, in, [&](int r, int jj, float s0, float s1, float x0, float x1) {
+          acc[r][2 * p + jj] = __fmaf_rn(s0, x0, acc[r][2 * p + jj]);
+          acc[r][2 * p + jj] = __fmaf_rn(s1, x1, acc[r][2 * p + jj]);
+        });
       }
     }
   }
@@ -224,6 +264,7 @@ __global__ void __launch_bounds__(32 * kMaxWarps, 1) gemv_blocked_kernel(const G
       v = __fadd_rn(v, __shfl_xor_sync(0xFFFFFFFFu, v, 2));
       if (tq == 0) mine[j * 16 + gq + 8 * r] = v;
     }
+  }
   }
   __syncthreads();
 
@@ -290,20 +331,20 @@ bool gemv_blocked_supports(const GemmArgs &g) {
   return smem_bytes(g.n, g.k) <= (size_t)kSmemLimit;
 }
 
-template <int P>
+template <int P, int HALVES, bool ONE = false>
 static cudaError_t launch_pairs(GemvQArgs &a, int warps, cudaStream_t s) {
   static std::atomic<bool> attr_set[64];   // zero-initialised; set once per device (a repeated cudaFuncSetAttribute is harmless)
   int dev = 0;
   cudaGetDevice(&dev);
   if (!attr_set[dev & 63]) {
-    if (cudaError_t e = cudaFuncSetAttribute(gemv_blocked_kernel<P>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit + part_bytes(kMaxWarps, kMaxN))) return e;
+    if (cudaError_t e = cudaFuncSetAttribute(gemv_blocked_kernel<P, HALVES, ONE>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit + part_bytes(kMaxWarps, kMaxN))) return e;
     attr_set[dev & 63] = true;
   }
   const int rows = 16 * (warps / a.ksplit), tiles = (a.m + rows - 1) / rows, smem = (int)smem_bytes(a.n, a.k) + part_bytes(warps, a.n);
   int per_sm = kMaxWarps / warps;   // (by its registers)
   while (per_sm > 1 && per_sm * (smem + 2048) > 227 * 1024) --per_sm;
   const int grid = tiles < per_sm * device_sms() ? tiles : per_sm * device_sms();
-  gemv_blocked_kernel<P><<<grid, warps * 32, smem, s>>>(a);
+  gemv_blocked_kernel<P, HALVES, ONE><<<grid, warps * 32, smem, s>>>(a);
   return cudaGetLastError();
 }
 
@@ -312,17 +353,17 @@ cudaError_t launch_gemv_blocked(const GemmArgs &g, cudaStream_t s) {
   a.m = g.m; a.n = g.n; a.k = g.k;
   a.A = g.A; a.B = g.B; a.e = g.e; a.ex = g.x;
   // How a row's k is dealt to warps depends on k alone, so that a row's bits do not depend on the matrix around it (or on n): eight warps in
-  // 256-value units, or up to 1024 values a 128-value half unit to a warp (1024 x 1024, 4 / 8 vectors: 3.9 / 4.8 -> 3.8 / 4.6 us).
+  // 256-value units, or up to 1024 values a 128-value half unit to a warp.
   // CTAs of eight warps, two per SM; of sixteen (two groups) where a CTA gets one tile at most or the activations leave room for one CTA:
   // 4096 x 14336, 4 / 8 vectors 21.0 / 34.7 -> 18.8 / 26.0 us, 4096 x 4096, 8 vectors 11.8 -> 11.0 us.  Fewer than eight only if that gives more CTAs.
   const int groups = (g.m + 15) / 16, sms = device_sms();
-  a.halves = g.k <= 1024 ? 1 : 2;
   a.ksplit = 8;
   while (a.ksplit > 1 && a.ksplit * 64 >= g.k) a.ksplit >>= 1;
   int warps = 8;
-  if (a.ksplit < 8 && groups <= 2 * sms) warps = a.ksplit < 4 ? 4 : a.ksplit;
+  if (a.ksplit < 8 && groups <= 2 * sms) a.ksplit = warps = 4;   // (a warp without a unit adds zeros)
   if (g.k > 1024 && ((groups > sms && groups <= 2 * sms) || 2 * (smem_bytes(g.n, g.k) + part_bytes(8, g.n) + 2048) > 227 * 1024)) warps = 16;
-  return g.n <= 2 ? launch_pairs<1>(a, warps, s) : g.n <= 4 ? launch_pairs<2>(a, warps, s) : launch_pairs<4>(a, warps, s);
+  if (g.k <= 1024) return launch_pairs<4, 1, true>(a, warps, s);
+  return g.n <= 2 ? launch_pairs<1, 2>(a, warps, s) : g.n <= 4 ? launch_pairs<2, 2>(a, warps, s) : launch_pairs<4, 2>(a, warps, s);
 }
 
 }  // namespace nvb

@@ -496,6 +496,24 @@ def test_blocked_gemv_at_the_edges_of_its_tiles_and_k_ranges(bt, layout):
             assert np.array_equal(values(got_top, ct, ht), values(got, c, h)[:, :160])
 
 
+@pytest.mark.parametrize("m,n,k", [(300, 8, 1024), (9700, 5, 1024), (130, 8, 1984), (5000, 3, 1536), (70, 6, 2048), (40, 8, 960), (4800, 7, 64), (64, 4, 2112)])
+def test_blocked_gemv_where_its_units_change(m, n, k):
+    """One 128-value unit per warp (k <= 1024: pairs of vectors in a loop), two of them (k < 2048), 256-value units from there on: within the bound,
+    and a vector's bits are those of the vector alone."""
+    c = Case(m, n, k, L.INT8, L.FP32, -1, L.BF16, 1.0, 0.0)
+    h = build_case(c, 7500 + m)
+    got, amax = run_gemm(c, h)
+    assert L.lib.nvfp4a_b200_last_route() == 6
+    check_bound(c, h, got, amax, oracle_case(c, h, want_ref=True))
+    B = h["B"]
+    one = O.Q8(1, k, ld=B.ld, ld_scale=B.ld_scale)
+    one.data[:], one.scales[:] = B.data[:B.ld], B.scales[:B.ld_scale]
+    one.glob = B.glob
+    c1, h1 = Case(m, 1, k, L.INT8, L.FP32, -1, L.BF16, 1.0, 0.0), dict(h, B=one, Dinit=h["Dinit"][:h["ldd"]])
+    got1, _ = run_gemm(c1, h1)
+    assert np.array_equal(values(got1, c1, h1)[0], values(got, c, h)[0])
+
+
 def test_w4a8_dp4a_gemm_is_bit_exact_in_the_tiled_order():
     """INT8 activations, n > 8, with the tensor-core W4A8 GEMM switched off (nvfp4a_b200_set_route(3)): the DP4A GEMM (route 7)
     sums blocks in the reference's tiled order, so D and amax equal the oracle's bit for bit; tails in m and n, padded leading
