@@ -353,7 +353,8 @@ cudaError_t launch_gemv_blocked(const GemmArgs &g, cudaStream_t s) {
   a.m = g.m; a.n = g.n; a.k = g.k;
   a.A = g.A; a.B = g.B; a.e = g.e; a.ex = g.x;
   // How a row's k is dealt to warps depends on k alone, so that a row's bits do not depend on the matrix around it (or on n): eight warps in
-  // 256-value units, or up to 1024 values a 128-value half unit to a warp.
+  // 256-value units, or below 2048 values in 128-value half units (every warp has one: as many roundings on the way to a sum as a lane per
+  // chunk and a butterfly; in 256-value units 1088 values are up to 3 % less exact).
   // CTAs of eight warps, two per SM; of sixteen (two groups) where a CTA gets one tile at most or the activations leave room for one CTA:
   // 4096 x 14336, 4 / 8 vectors 21.0 / 34.7 -> 18.8 / 26.0 us, 4096 x 4096, 8 vectors 11.8 -> 11.0 us.  Fewer than eight only if that gives more CTAs.
   const int groups = (g.m + 15) / 16, sms = device_sms();
@@ -363,6 +364,7 @@ cudaError_t launch_gemv_blocked(const GemmArgs &g, cudaStream_t s) {
   if (a.ksplit < 8 && groups <= 2 * sms) a.ksplit = warps = 4;   // (a warp without a unit adds zeros)
   if (g.k > 1024 && ((groups > sms && groups <= 2 * sms) || 2 * (smem_bytes(g.n, g.k) + part_bytes(8, g.n) + 2048) > 227 * 1024)) warps = 16;
   if (g.k <= 1024) return launch_pairs<4, 1, true>(a, warps, s);
+  if (g.k < 2048) return g.n <= 2 ? launch_pairs<1, 1>(a, warps, s) : g.n <= 4 ? launch_pairs<2, 1>(a, warps, s) : launch_pairs<4, 1>(a, warps, s);
   return g.n <= 2 ? launch_pairs<1, 2>(a, warps, s) : g.n <= 4 ? launch_pairs<2, 2>(a, warps, s) : launch_pairs<4, 2>(a, warps, s);
 }
 
