@@ -45,14 +45,16 @@ if not os.path.exists(LIB_PATH):
     raise ImportError(f"{LIB_PATH} is missing: build it with `python -m nvfp4effma_b200.build` (nvcc, sm_100a). "
                       "There is no CPU or PyTorch fallback.")
 lib = C.CDLL(LIB_PATH)
-_TORCH_LIB_PATH = os.path.join(_HERE, "libnvfp4effma_torch.so")
 
 
 def torch_lib_path():
-    """The library with the torch operators' CUDA kernels; there is no fallback for it either."""
-    if not os.path.exists(_TORCH_LIB_PATH):
-        raise ImportError(f"{_TORCH_LIB_PATH} is missing: build it with `python -m nvfp4effma_b200.build`.")
-    return _TORCH_LIB_PATH
+    """The library with the torch operators' CUDA kernels; there is no fallback for it either.  It links against torch's C++ ABI, so its name
+    carries the version of torch that it was built with: after a change of torch it is missing, not wrong."""
+    import torch
+    path = os.path.join(_HERE, f"libnvfp4effma_torch-{torch.__version__}.so")
+    if not os.path.exists(path):
+        raise ImportError(f"{path} is missing: build it with `python -m nvfp4effma_b200.build` (it is built for one version of torch).")
+    return path
 
 
 _T, _E, _i, _f, _v, _s = C.POINTER(Tensor), C.POINTER(Epilogue), C.c_int, C.c_float, C.c_void_p, C.c_void_p

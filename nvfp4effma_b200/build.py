@@ -1,5 +1,5 @@
-"""Builds ``libnvfp4effma.so`` (the C-ABI shared library) in-tree from ``csrc/*.cu`` for sm_100a, and ``libnvfp4effma_torch.so`` (the
-torch operators' CUDA kernels, host code that calls the C ABI) from ``csrc/torch_ops.cpp``.
+"""Builds ``libnvfp4effma.so`` (the C-ABI shared library) in-tree from ``csrc/*.cu`` for sm_100a, and
+``libnvfp4effma_torch-<version of torch>.so`` (the torch operators' CUDA kernels, host code that calls the C ABI) from ``csrc/torch_ops.cpp``.
 
     python -m nvfp4effma_b200.build [--force]
 
@@ -16,7 +16,6 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OBJ = os.path.join(CSRC, "_obj")
 LIB = os.path.join(HERE, "libnvfp4effma.so")
-TORCH_LIB = os.path.join(HERE, "libnvfp4effma_torch.so")
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-gencode", "arch=compute_100a,code=sm_100a", "-Xcompiler", "-fPIC,-ffp-contract=off",
          "-Xptxas", "-v", "--expt-relaxed-constexpr"] + os.environ.get("NVFP4A_NVCC_FLAGS", "").split()
@@ -41,17 +40,18 @@ def _build_torch(force):
     """The torch operators' library; its C-ABI calls resolve to LIB beside it."""
     src = os.path.join(CSRC, "torch_ops.cpp")
     newest = max(os.path.getmtime(src), os.path.getmtime(os.path.join(HERE, "..", "include", "nvfp4effma.h")))
-    if not force and os.path.exists(TORCH_LIB) and os.path.getmtime(TORCH_LIB) > newest:
-        return
     import torch
+    out = os.path.join(HERE, f"libnvfp4effma_torch-{torch.__version__}.so")
+    if not force and os.path.exists(out) and os.path.getmtime(out) > newest:
+        return
     base = os.path.dirname(os.path.abspath(torch.__file__))
     cuda = os.path.dirname(os.path.dirname(NVCC))
     r = subprocess.run(["g++", "-O2", "-std=c++17", "-shared", "-fPIC", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
-                        f"-I{base}/include", f"-I{base}/include/torch/csrc/api/include", f"-I{cuda}/include", "-o", TORCH_LIB, src,
+                        f"-I{base}/include", f"-I{base}/include/torch/csrc/api/include", f"-I{cuda}/include", "-o", out, src,
                         f"-L{base}/lib", "-ltorch", "-ltorch_cpu", "-lc10", "-lc10_cuda", f"-L{HERE}", "-lnvfp4effma", "-Wl,-rpath,$ORIGIN"],
                        capture_output=True, text=True)
     if r.returncode:
-        raise RuntimeError(f"building {TORCH_LIB} failed:\n{r.stdout}\n{r.stderr}")
+        raise RuntimeError(f"building {out} failed:\n{r.stdout}\n{r.stderr}")
 
 
 def build(force=False, verbose=False):

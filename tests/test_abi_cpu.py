@@ -51,6 +51,15 @@ def test_deferred_tensor_parallel_gemvs_read_activations_behind_a_cta_barrier():
         assert after.index("__syncthreads()") < after.index("behind_wait(") <= after.index("ld16("), name
 
 
+def test_the_torch_operators_library_belongs_to_one_version_of_torch(monkeypatch):
+    """It links against torch's C++ ABI: one built with another torch must not be loaded."""
+    import torch
+    assert torch.__version__ in os.path.basename(L.torch_lib_path())
+    monkeypatch.setattr(torch, "__version__", "0.0.1")
+    with pytest.raises(ImportError, match="one version of torch"):
+        L.torch_lib_path()
+
+
 def test_struct_layouts_match_the_reference_abi():
     # field order / offsets of nvfp4a_tensor on LP64 (reference include/nvfp4effma.h:46-57)
     T = L.Tensor
