@@ -32,10 +32,26 @@ void check(nvfp4a_status st) {
 
 cudaStream_t stream() { return c10::cuda::getCurrentCUDAStream().stream(); }
 
+// the element type as Python spells it
+const char *dtype_name(ScalarType t) {
+  switch (t) {
+    case at::kByte: return "uint8";
+    case at::kChar: return "int8";
+    case at::kShort: return "int16";
+    case at::kInt: return "int32";
+    case at::kLong: return "int64";
+    case at::kHalf: return "float16";
+    case at::kBFloat16: return "bfloat16";
+    case at::kFloat: return "float32";
+    case at::kDouble: return "float64";
+    case at::kBool: return "bool";
+    default: return c10::toString(t);
+  }
+}
 nvfp4a_dtype dense_code(ScalarType t) {
   if (t == at::kBFloat16) return NVFP4A_BF16;
   if (t == at::kHalf) return NVFP4A_FP16;
-  TORCH_CHECK_TYPE(t == at::kFloat, "torch.", c10::toString(t), " is not one of the dense element types (bfloat16, float16, float32)");
+  TORCH_CHECK_TYPE(t == at::kFloat, "torch.", dtype_name(t), " is not one of the dense element types (bfloat16, float16, float32)");
   return NVFP4A_FP32;
 }
 bool is_dense(ScalarType t) { return t == at::kBFloat16 || t == at::kHalf || t == at::kFloat; }
@@ -228,7 +244,7 @@ Tensor tc_image(int64_t operand, const Tensor &x, const OptTensor &scales, int64
   const c10::cuda::CUDAGuard guard(x.device());
   const Operand s = activation(x, scales, std::nullopt, flags & (NVFP4A_SCALES_SWIZZLED | NVFP4A_SCALES_UE5M3), 0);
   const size_t size = nvfp4a_tc_image_bytes((int)operand, s.t.dtype, (int)x.size(0), (int)k);
-  TORCH_CHECK_NOT_IMPLEMENTED(size != 0, "no image of kind ", operand, " for a torch.", c10::toString(x.scalar_type()), " operand with k = ", k);
+  TORCH_CHECK_NOT_IMPLEMENTED(size != 0, "no image of kind ", operand, " for a torch.", dtype_name(x.scalar_type()), " operand with k = ", k);
   const Tensor image = empty({(int64_t)size}, at::kByte, x);
   check(nvfp4a_tc_image((int)operand, &s.t, (int)s.ld, (int)x.size(0), (int)k, image.data_ptr(), stream()));
   return image;

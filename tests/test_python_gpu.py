@@ -421,3 +421,10 @@ def test_operators_pass_opcheck_and_trace_without_graph_breaks():
 
     compiled = torch.compile(fn, backend="aot_eager", fullgraph=True)
     assert torch.allclose(compiled(x), fn(x))
+
+
+def test_operator_errors_name_element_types_as_python_does():
+    w = nf.quantize(normal((128, 128), seed=45))
+    for dtype in (torch.int32, torch.float64, torch.bool):
+        with pytest.raises(TypeError, match=f"{dtype} is not one of the dense element types"):
+            nf.linear(normal((4, 128), torch.bfloat16, seed=46), w, torch.zeros(128, dtype=dtype, device=GPU))
