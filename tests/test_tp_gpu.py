@@ -94,6 +94,26 @@ def test_a_barrier_whose_peer_never_arrives_gives_up_and_reports_it():
     assert st.value == 0 and bool(torch.isfinite(y.float()).all())
 
 
+@pytest.mark.parametrize("T", [1, 4, 8])
+def test_shard_rows_are_the_rows_of_the_whole_on_the_same_kernel(T):
+    """A shard's decode outputs equal the whole matrix's bit for bit where both run one kernel: on the mma.sync GEMV (nvfp4a_b200_set_route(2)),
+    whose sums depend on k alone.  (By default the whole may take an FP4 tensor-core GEMV that its shards are too small for.)"""
+    import nvfp4effma_b200 as nf
+    from nvfp4effma_b200 import _lib as L
+    from nvfp4effma_b200.tp import shard_rows
+    w = nf.quantize(rand((8192, 8192), seed=11, scale=0.02), torch.tensor([0.0001], device="cuda"))
+    x = rand((T, 8192), torch.bfloat16, seed=12)
+    old = L.lib.nvfp4a_b200_set_route(2)
+    try:
+        whole = nf.linear(x, nf.TCWeight(w, "exact"))
+        for rank in range(4):
+            part = nf.linear(x, nf.TCWeight(shard_rows(w, 4, rank), "exact"))
+            assert L.lib.nvfp4a_b200_last_route() == 2
+            assert torch.equal(part, whole[:, rank * 2048:(rank + 1) * 2048])
+    finally:
+        L.lib.nvfp4a_b200_set_route(old)
+
+
 RANK_SCRIPT = r"""
 import os, sys, torch, torch.distributed as dist
 sys.path.insert(0, os.environ["NVB_ROOT"])
