@@ -309,7 +309,6 @@ gemm_w4a4_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
     const int ldd = g.e.ldd, d_dtype = g.e.d_dtype;
     float *const amax_out = g.e.amax;
     const int esz = dense_bytes(d_dtype);
-    const int cw = esz == 2 ? 16 : 8;           // columns per staging round: 128 rows x cw columns = 4 KiB
     const bool leader = (warp == 2 || warp == 10) && lane == 0; // issues and tracks its group's TMA stores
     const bool fast = beta == 0.f && gb_stride == 0;  // one scale per lane, no C: the common case
     const float colp0 = (gb && !gb_stride) ? gb[0] : 1.f;

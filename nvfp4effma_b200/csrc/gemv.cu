@@ -58,11 +58,6 @@ __device__ __forceinline__ uint32_t decode_pair(uint32_t w) {
   const uint32_t sgn = (w << (12 - 4 * P)) & 0x80008000u;
   return mag | sgn;
 }
-__device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t sel) {
-  uint32_t d;
-  asm("prmt.b32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(sel));
-  return d;
-}
 
 // One step of one lane: 32 values of k (one 16-byte word of nibbles) for rows gq and gq + 8, two scale codes per row,
 // and -- for the lanes that carry an activation column -- the 32 matching activations.
@@ -154,8 +149,8 @@ __global__ void __launch_bounds__(kGemvWarps * 32, 3) gemv_kernel(const GemvArgs
     for (int i = 0; i < 4; ++i) {  // word i: 8 values, k = 32 c + 8 i ..; block i / 2 of the chunk
       const uint32_t a = ww0[i], b = ww1[i], sa = S0[i >> 1], sb = S1[i >> 1];
       // B pairs (x[p], x[p + 4]) to match the decode's pairing
-      const uint32_t x04 = prmt(cur.x[i].x, cur.x[i].z, 0x5410), x15 = prmt(cur.x[i].x, cur.x[i].z, 0x7632);
-      const uint32_t x26 = prmt(cur.x[i].y, cur.x[i].w, 0x5410), x37 = prmt(cur.x[i].y, cur.x[i].w, 0x7632);
+      const uint32_t x04 = byte_perm(cur.x[i].x, cur.x[i].z, 0x5410), x15 = byte_perm(cur.x[i].x, cur.x[i].z, 0x7632);
+      const uint32_t x26 = byte_perm(cur.x[i].y, cur.x[i].w, 0x5410), x37 = byte_perm(cur.x[i].y, cur.x[i].w, 0x7632);
       mma_bf16_16816(acc, bf16x2_mul(decode_pair<0>(a), sa), bf16x2_mul(decode_pair<0>(b), sb), bf16x2_mul(decode_pair<1>(a), sa),
                      bf16x2_mul(decode_pair<1>(b), sb), x04, x15);
       mma_bf16_16816(acc, bf16x2_mul(decode_pair<2>(a), sa), bf16x2_mul(decode_pair<2>(b), sb), bf16x2_mul(decode_pair<3>(a), sa),

@@ -38,17 +38,12 @@ struct GemvQArgs {
   EpilogueEx ex;
 };
 
-__device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t sel) {
-  uint32_t d;
-  asm("prmt.b32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(sel));
-  return d;
-}
 // eight E2M1 nibbles -> eight int8 values 2 * e2m1 (lo: nibbles 0-3, hi: 4-7).  A set bit 3 of a PRMT selector nibble returns the looked-up
 // byte's sign (0 here) instead of the byte: w picks the magnitudes of the positive nibbles, w ^ 0x88888888 those of the negative ones.
 __device__ __forceinline__ void dec8(uint32_t w, uint32_t &lo, uint32_t &hi) {
   const uint32_t n = w ^ 0x88888888u;                                 // magnitudes 0 1 2 3 | 4 6 8 12
-  lo = (prmt(0x03020100u, 0x0C080604u, w) - prmt(0x03020100u, 0x0C080604u, n) + 0x80808080u) ^ 0x80808080u;   // no borrow between bytes
-  hi = (prmt(0x03020100u, 0x0C080604u, w >> 16) - prmt(0x03020100u, 0x0C080604u, n >> 16) + 0x80808080u) ^ 0x80808080u;
+  lo = (byte_perm(0x03020100u, 0x0C080604u, w) - byte_perm(0x03020100u, 0x0C080604u, n) + 0x80808080u) ^ 0x80808080u;   // no borrow between bytes
+  hi = (byte_perm(0x03020100u, 0x0C080604u, w >> 16) - byte_perm(0x03020100u, 0x0C080604u, n >> 16) + 0x80808080u) ^ 0x80808080u;
 }
 
 __device__ __forceinline__ void mma_s8(int (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {

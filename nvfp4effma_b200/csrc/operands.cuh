@@ -72,13 +72,13 @@ bool gemv_fp4_supports(const GemmArgs &g);
 cudaError_t launch_gemv_fp4_n8(const GemmArgs &g, cudaStream_t s);   // the same for 3 <= n <= 8
 bool gemv_fp4_n8_supports(const GemmArgs &g);
 void set_gemv_fp4_splits(int s);
-cudaError_t launch_gemv_blocked(const GemmArgs &g, cudaStream_t s);  // n <= 8, INT8 or NVFP4 activations: exact DP4A block sums
+cudaError_t launch_gemv_blocked(const GemmArgs &g, cudaStream_t s);  // n <= 8, INT8 or NVFP4 activations: exact integer block sums (mma.sync s8)
 bool gemv_blocked_supports(const GemmArgs &g);
 cudaError_t launch_gemm_w4a4(const GemmArgs &g, cudaStream_t s);     // tcgen05 kind::mxf4nvf4 (E4M3 scales)
 bool gemm_w4a4_supports(const GemmArgs &g);
 cudaError_t launch_gemm_dp4a(const GemmArgs &g, cudaStream_t s);     // W4A8, n > 8: DP4A block sums in the reference's tiled order
 bool gemm_dp4a_supports(const GemmArgs &g);
-cudaError_t launch_gemm_w4a16(const GemmArgs &g, cudaStream_t s);    // tcgen05 kind::f16 with weights expanded to BF16 in smem
+cudaError_t launch_gemm_w4a16(const GemmArgs &g, cudaStream_t s);    // tcgen05 kind::f16 with weights expanded to 16-bit values in tensor memory
 bool gemm_w4a16_supports(const GemmArgs &g);
 bool gemm_w4a16_pushes(const GemmArgs &g);
 cudaError_t launch_gemm_w4a8_tc(const GemmArgs &g, const int *seg, int groups, cudaStream_t s);  // INT8 activations as three BF16 planes on the same tcgen05 kernel

@@ -1011,7 +1011,6 @@ extern "C" nvfp4a_status nvfp4a_quantize_ex(const nvfp4a_tensor *src, int lds, i
 
   const uint8_t *s = (const uint8_t *)src->data;
   const int bpr = cols / 16;
-  const long long blocks = (long long)rows * bpr;
   // One-read path: the common recipe (rowwise 1 x 16 blocks, one amax for the tensor, no 4over6, 16-bit source) on a matrix large
   // enough to occupy every SM runs as ONE cooperative kernel that reads most of the source once (quant_fused_kernel).
   if (c.compute_amax && rowwise && !columnwise && c.tile_rows == 1 && c.four_over_six == NVFP4A_4OVER6_OFF &&

@@ -11,11 +11,6 @@ namespace nvb {
 namespace sm100 {
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ bool elect_one() {
-  uint32_t pred;
-  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xFFFFFFFF;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(pred));
-  return pred != 0;
-}
 
 // ---- mbarrier ---------------------------------------------------------------------------------------------------------
 __device__ __forceinline__ void mbar_init(uint64_t *bar, uint32_t count) {
@@ -84,7 +79,7 @@ __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepc
 // (What the previous kernel wrote is read with ordinary loads: see behind_wait.)
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
-// ---- thread-block clusters: rank, barrier, loads from a peer CTA's shared memory ---------------------------------------------
+// ---- thread-block clusters: rank, barrier, stores to a peer CTA's shared memory ---------------------------------------------
 __device__ __forceinline__ uint32_t cluster_ctarank() {
   uint32_t r;
   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
@@ -102,22 +97,11 @@ __device__ __forceinline__ void st_peer_f32(void *own_smem, uint32_t peer_rank, 
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(addr) : "r"(smem_u32(own_smem)), "r"(peer_rank));
   asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory");
 }
-__device__ __forceinline__ float ld_peer_f32(const void *own_smem, uint32_t peer_rank) {
-  uint32_t addr;
-  float v;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(addr) : "r"(smem_u32(own_smem)), "r"(peer_rank));
-  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
-  return v;
-}
 
 // ---- TMA (no multicast anywhere) -----------------------------------------------------------------------------------------
 __device__ __forceinline__ void tma_load_2d(void *dst, const CUtensorMap *map, int x, int y, uint64_t *bar) {
   asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
                ::"r"(smem_u32(dst)), "l"(map), "r"(x), "r"(y), "r"(smem_u32(bar)) : "memory");
-}
-__device__ __forceinline__ void tma_load_3d(void *dst, const CUtensorMap *map, int x, int y, int z, uint64_t *bar) {
-  asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
-               ::"r"(smem_u32(dst)), "l"(map), "r"(x), "r"(y), "r"(z), "r"(smem_u32(bar)) : "memory");
 }
 __device__ __forceinline__ void tma_load_4d(void *dst, const CUtensorMap *map, int x, int y, int z, int w, uint64_t *bar) {
   asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];"
@@ -227,14 +211,6 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t *r) {
         "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
       : "r"(taddr) : "memory");
 }
-// 32 lanes x 16 consecutive columns -> 16 registers per thread
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t *r) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
-        "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-      : "r"(taddr) : "memory");
-}
 // 16 lanes x 64 consecutive columns -> 32 registers per thread.  For every group of 8 columns (registers 4 g .. 4 g + 3):
 // thread t holds (lane t / 4, columns 2 (t % 4) and 2 (t % 4) + 1) in the first two and (lane t / 4 + 8, same columns) in the
 // last two -- the fragment layout of an MMA accumulator.
@@ -272,12 +248,6 @@ __device__ __forceinline__ void tmem_ld_wait32(uint32_t (&r)[32]) {
                  "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15]), "+r"(r[16]), "+r"(r[17]), "+r"(r[18]), "+r"(r[19]), "+r"(r[20]),
                  "+r"(r[21]), "+r"(r[22]), "+r"(r[23]), "+r"(r[24]), "+r"(r[25]), "+r"(r[26]), "+r"(r[27]), "+r"(r[28]), "+r"(r[29]), "+r"(r[30]),
                  "+r"(r[31])
-               :: "memory");
-}
-__device__ __forceinline__ void tmem_ld_wait16(uint32_t (&r)[16]) {
-  asm volatile("tcgen05.wait::ld.sync.aligned;"
-               : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]), "+r"(r[8]), "+r"(r[9]), "+r"(r[10]),
-                 "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15])
                :: "memory");
 }
 // shared memory (32 rows x 16 bytes, described by sdesc) -> 4 columns of all 128 lanes (the 32 rows replicated per quadrant)
@@ -361,10 +331,6 @@ __device__ __forceinline__ void mma4_commit_pair_elect(uint32_t d_tmem, uint64_t
                                                        uint32_t sfb_step, uint32_t accumulate, uint64_t *bar) {
   NVB_MMA4_BODY("2", "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%19], %20;");
 }
-__device__ __forceinline__ void mma4_commit_elect(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t sfa, uint32_t sfb,
-                                                  uint32_t sfb_step, uint32_t accumulate, uint64_t *bar) {
-  NVB_MMA4_BODY("1", "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%19];");
-}
 // One 64-value k group of the FP4 GEMV in one statement (elected lane of a converged warp): the two 512-byte scale tiles of the
 // group's 256 weight rows copied into tensor memory (tcgen05.cp), then the MMA that reads them.
 __device__ __forceinline__ void cp2_mma_mxf4nvf4_elect(uint32_t sfb_tmem, uint64_t sf_desc0, uint64_t sf_desc1, uint32_t d_tmem, uint64_t a_desc,
@@ -380,22 +346,6 @@ __device__ __forceinline__ void tmem_cp_32x128b_warpx4_elect(uint32_t taddr, uin
   asm volatile("{\n\t.reg .pred q;\n\telect.sync _|q, 0xFFFFFFFF;\n\t@q tcgen05.cp.cta_group::1.32x128b.warpx4 [%0], %1;\n\t}"
                ::"r"(taddr), "l"(sdesc) : "memory");
 }
-// The same for kind::f16 (K = 16 per instruction: four MMAs cover the 64 values of k of a 128-byte-row stage).
-__device__ __forceinline__ void mma4_f16_commit_elect(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate, uint64_t *bar) {
-  asm volatile("{\n\t.reg .pred p, q, t;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.eq.u32 t, %3, %3;\n\telect.sync _|q, 0xFFFFFFFF;\n\t"
-               "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t"
-               "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %5, %6, %3, t;\n\t"
-               "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %7, %8, %3, t;\n\t"
-               "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %9, %10, %3, t;\n\t"
-               "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%11];\n\t}"
-               ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "l"(a_desc + 2), "l"(b_desc + 2), "l"(a_desc + 4), "l"(b_desc + 4),
-                 "l"(a_desc + 6), "l"(b_desc + 6), "r"(smem_u32(bar)) : "memory");
-}
-__device__ __forceinline__ void tma_load_2d_elect(uint32_t dst, const CUtensorMap *map, int x, int y, uint32_t bar_addr) {
-  asm volatile("{\n\t.reg .pred q;\n\telect.sync _|q, 0xFFFFFFFF;\n\t"
-               "@q cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];\n\t}"
-               ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(bar_addr) : "memory");
-}
 __device__ __forceinline__ void tc_commit_elect(uint64_t *bar) {
   asm volatile("{\n\t.reg .pred q;\n\telect.sync _|q, 0xFFFFFFFF;\n\t"
                "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(smem_u32(bar)) : "memory");
@@ -404,11 +354,6 @@ __device__ __forceinline__ void tc_commit_pair_elect(uint64_t *bar) {
   asm volatile("{\n\t.reg .pred q;\n\telect.sync _|q, 0xFFFFFFFF;\n\t"
                "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n\t}"
                ::"r"(smem_u32(bar)), "h"((uint16_t)3) : "memory");
-}
-__device__ __forceinline__ void mma_f16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
-  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-               "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-               ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
 }
 
 }  // namespace sm100
