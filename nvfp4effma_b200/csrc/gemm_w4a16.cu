@@ -53,7 +53,8 @@
 // x = q * s_b (one rounding: within the accumulation bound of the exact definition, not bit-identical to the integer block sums
 // of the DP4A kernels), split exactly into three BF16 terms x = t1 + t2 + t3 (8 + 8 + 8 significant bits) by a small kernel
 // that runs first.  The terms lie side by side as [token][3][k]; the activation ring holds one plane of a stage per slot, and the
-// MMA issuer accumulates weight x t1, weight x t2, weight x t3 from one expanded weight tile into the same accumulator.
+// MMA issuer accumulates weight x t1, weight x t2, weight x t3 from one expanded weight tile into the same accumulator (grouped: the last two
+// into one of their own, see Segments).
 #include <atomic>
 #include <cuda_bf16.h>
 #include "operands.cuh"
@@ -783,7 +784,7 @@ bool set_up(const GemmArgs &g, int planes, bool f16, int groups, const void *act
   const int rows256 = (g.m + 255) / 256, pairs = device_sms() / 2, widest = f16 || groups ? kSegmentWidth : 256;
   const Plan p = groups ? make_grouped_plan(rows256, g.n, groups, planes, pairs, widest) : make_plan(rows256, g.n, planes, pairs, widest);
   const uint64_t wrows = (uint64_t)g.m * (groups ? groups : 1);
-  a->seg_stages = g.k >= 1024 ? 4 : g.k >= 512 ? 2 : 1;
+  a->seg_stages = g.k >= 1024 ? 4 : g.k >= 512 ? 2 : 1;   // (the longest that keep the sums no less exact than the CUDA-core kernels': see the head of the file)
   a->width = p.width; a->nfull = p.nfull; a->cut = p.cut; a->tiles = p.tiles;
   const uint64_t wtiles = (uint64_t)((g.m + 127) / 128) * g.A.ktiles;
   if (g.A.image ? !make_tmap_bytes(tw, g.A.data, 128, 128, 128, 128, wtiles, kImgTileBytes)
