@@ -18,8 +18,12 @@ def stream():
 
 
 def addr(t):
-    """Device address of ``t`` (``None`` stays NULL)."""
-    return None if t is None else ctypes.c_void_p(t.data_ptr())
+    """Device address of ``t`` (``None`` stays NULL).  A kernel would fault on ordinary host memory (pinned memory is mapped on the GPU)."""
+    if t is None:
+        return None
+    if not t.is_cuda and not t.is_pinned():
+        raise ValueError(f"a tensor of shape {tuple(t.shape)} lives on {t.device}; the library works on CUDA memory only")
+    return ctypes.c_void_p(t.data_ptr())
 
 
 def ref(struct):

@@ -57,7 +57,12 @@ nvfp4a_dtype dense_code(ScalarType t) {
 bool is_dense(ScalarType t) { return t == at::kBFloat16 || t == at::kHalf || t == at::kFloat; }
 
 bool misaligned(const Tensor &t, uintptr_t mask) { return ((uintptr_t)t.data_ptr() & mask) != 0; }
-void *addr(const OptTensor &t) { return t ? t->data_ptr() : nullptr; }
+// the address of a tensor that a kernel will use: one of host memory would fault on the GPU (pinned memory is mapped there)
+void *device_ptr(const Tensor &t, const char *name) {
+  TORCH_CHECK_VALUE(t.is_cuda() || t.is_pinned(), name, " lives on ", t.device(), "; the library works on CUDA memory only");
+  return t.data_ptr();
+}
+void *addr(const OptTensor &t, const char *name) { return t ? device_ptr(*t, name) : nullptr; }
 
 // a 2-D matrix the library can address: unit stride along rows, a pitch that is a multiple of `mult` and not below the row length, a
 // 16-byte aligned base; anything else is copied once
@@ -67,11 +72,11 @@ Tensor matrix(const Tensor &t, int64_t mult, const char *name) {
   return t.stride(1) != 1 || pitch < t.size(1) || pitch % mult || misaligned(t, 15) ? t.contiguous() : t;
 }
 
-nvfp4a_tensor dense_tensor(const Tensor &t, const OptTensor &amax = std::nullopt) {
+nvfp4a_tensor dense_tensor(const Tensor &t, const char *name, const OptTensor &amax = std::nullopt) {
   nvfp4a_tensor r = {};
-  r.data = t.data_ptr();
+  r.data = device_ptr(t, name);
   r.dtype = dense_code(t.scalar_type());
-  r.amax = (float *)addr(amax);
+  r.amax = (float *)addr(amax, "amax");
   return r;
 }
 
@@ -103,10 +108,10 @@ Operand fp4_operand(const Tensor &data, const Tensor &scales, const OptTensor &g
     }
     o.t.ld_scale = (int)o.scales.stride(0);
   }
-  o.t.data = o.data.data_ptr();
+  o.t.data = device_ptr(o.data, "NVFP4 data");
   o.t.dtype = NVFP4A_NVFP4;
-  o.t.block_scale = o.scales.data_ptr();
-  o.t.global_scale = (const float *)addr(glob);
+  o.t.block_scale = device_ptr(o.scales, "block scales");
+  o.t.global_scale = (const float *)addr(glob, "global");
   o.t.flags = (unsigned)flags;
   o.t.scale_max = (int)smax;
   o.ld = 2 * o.data.stride(0);
@@ -125,13 +130,13 @@ Operand activation(const Tensor &x, const OptTensor &scales, const OptTensor &gl
     o.data = matrix(x, 64, "int8 activations");
     o.scales = scales->contiguous();
     if (misaligned(o.scales, 15) || o.scales.stride(0) % 4) o.scales = padded_rows(o.scales);
-    o.t.data = o.data.data_ptr();
+    o.t.data = device_ptr(o.data, "int8 activations");
     o.t.dtype = NVFP4A_INT8;
-    o.t.block_scale = o.scales.data_ptr();
+    o.t.block_scale = device_ptr(o.scales, "block scales");
     o.t.ld_scale = (int)o.scales.stride(0);
   } else {
     o.data = matrix(x, 64, "activations");
-    o.t = dense_tensor(o.data);
+    o.t = dense_tensor(o.data, "x");
   }
   o.ld = o.data.stride(0);
   return o;
@@ -155,7 +160,7 @@ struct Bias {
     if (!b) return;
     TORCH_CHECK_VALUE(b->numel() == n, "bias has ", b->numel(), " elements for ", n, " output features");
     keep = b->contiguous();
-    t = dense_tensor(keep);
+    t = dense_tensor(keep, "bias");
     p = &t;
   }
 };
@@ -171,16 +176,16 @@ OptTensor gemm_into(const Tensor &out, const Tensor &x, const OptTensor &xs, con
   check_out(out, T, N);
   const OptTensor amax = amax_buffer(want_amax, out);
   const Operand b = activation(x, xs, xg, xf, xm);
-  const nvfp4a_tensor d = dense_tensor(out, amax);
+  const nvfp4a_tensor d = dense_tensor(out, "out", amax);
   const Bias bi(bias, N);
   const int ldd = (int)out.stride(0);
   const nvfp4a_tensor *c = beta != 0.0 ? &d : nullptr;   // beta accumulates into out itself
   const int ldc = beta != 0.0 ? ldd : 0;
   if (w_img && T <= 8) {
     nvfp4a_tensor a = {};
-    a.data = w_img->data_ptr();
+    a.data = device_ptr(*w_img, "the weight's image");
     a.dtype = NVFP4A_NVFP4;
-    a.global_scale = (const float *)addr(wg);
+    a.global_scale = (const float *)addr(wg, "global");
     a.flags = (unsigned)wf;
     a.scale_max = (int)wm;
     check(nvfp4a_gemv_tc((int)N, (int)T, (int)k, (float)alpha, &a, &b.t, (int)b.ld, (float)beta, c, ldc, &d, ldd, bi.p, stream()));
@@ -216,12 +221,12 @@ OptTensor grouped_into(const Tensor &out, const Tensor &x, const OptTensor &xs, 
   check_out(out, T, N);
   const OptTensor amax = amax_buffer(want_amax, out);
   const Operand b = activation(x, xs, xg, xf, xm), a = fp4_operand(w, ws, wg, wf, wm);
-  const nvfp4a_tensor d = dense_tensor(out, amax);
+  const nvfp4a_tensor d = dense_tensor(out, "out", amax);
   const Bias bi(bias, w.size(0));
   const int ldd = (int)out.stride(0);
   const Tensor sg = seg.contiguous();
   check(nvfp4a_gemm_grouped((int)groups, (int)N, (int)k, (int)T, (float)alpha, &a.t, (int)a.ld, &b.t, (int)b.ld, (float)beta, beta != 0.0 ? &d : nullptr,
-                            beta != 0.0 ? ldd : 0, &d, ldd, bi.p, (const int *)sg.data_ptr(), stream()));
+                            beta != 0.0 ? ldd : 0, &d, ldd, bi.p, (const int *)device_ptr(sg, "seg"), stream()));
   return amax;
 }
 std::tuple<Tensor, OptTensor> grouped_linear(const Tensor &x, const OptTensor &xs, const OptTensor &xg, int64_t xf, int64_t xm, const Tensor &seg,
@@ -267,19 +272,19 @@ OptTensor image_gemm_into(const Tensor &out, const Tensor &x_img, int64_t x_dtyp
   check_out(out, T, N);
   const OptTensor amax = amax_buffer(want_amax, out);
   nvfp4a_tensor a = {}, b = {};
-  a.data = w_img.data_ptr();
+  a.data = device_ptr(w_img, "the weight's image");
   a.dtype = NVFP4A_NVFP4;
-  a.global_scale = (const float *)addr(wg);
+  a.global_scale = (const float *)addr(wg, "global");
   a.flags = (unsigned)wf;
   a.scale_max = (int)wm;
-  b.data = x_img.data_ptr();
+  b.data = device_ptr(x_img, "the activations' image");
   b.dtype = x_dtype == 0 ? NVFP4A_NVFP4 : x_dtype == 1 ? NVFP4A_INT8 : NVFP4A_BF16;
   if (x_dtype == 0) {
-    b.global_scale = (const float *)addr(xg);
+    b.global_scale = (const float *)addr(xg, "global");
     b.flags = (unsigned)xf;
     b.scale_max = (int)xm;
   }
-  const nvfp4a_tensor d = dense_tensor(out, amax);
+  const nvfp4a_tensor d = dense_tensor(out, "out", amax);
   const Bias bi(bias, N);
   const int ldd = (int)out.stride(0);
   const cudaStream_t s = stream();
@@ -337,15 +342,15 @@ Quantized quantize_ex(const Tensor &x0, bool rowwise, bool columnwise, const Opt
   }
   if (want_amax) out[6] = zeros({1}, at::kFloat, x0);
   const Tensor x = matrix(x0, 16, "x");
-  const nvfp4a_tensor src = dense_tensor(x);
+  const nvfp4a_tensor src = dense_tensor(x, "x");
   nvfp4a_tensor half[2] = {};
   for (int h = 0; h < 2; ++h) {
     if (!out[2 * h]) continue;
     half[h].data = out[2 * h]->data_ptr();
     half[h].dtype = NVFP4A_NVFP4;
     half[h].block_scale = out[2 * h + 1]->data_ptr();
-    half[h].global_scale = (const float *)addr(compute_amax ? out[4 + h] : h ? g_col : g_row);
-    half[h].amax = (float *)addr(out[6]);
+    half[h].global_scale = (const float *)addr(compute_amax ? out[4 + h] : h ? g_col : g_row, "global");
+    half[h].amax = (float *)addr(out[6], "amax");
     half[h].flags = (unsigned)(h ? flags & ~(int64_t)NVFP4A_GLOBAL_PER_ROW : flags);
     half[h].scale_max = (int)smax;
   }
@@ -360,7 +365,7 @@ std::tuple<Tensor, Tensor> quantize_int8(const Tensor &x0) {
   const c10::cuda::CUDAGuard guard(x0.device());
   const int64_t rows = x0.size(0), cols = x0.size(1);
   const Tensor q = empty({rows, cols}, at::kChar, x0), s = empty({rows, cols / 16}, at::kFloat, x0), x = matrix(x0, 16, "x");
-  const nvfp4a_tensor src = dense_tensor(x);
+  const nvfp4a_tensor src = dense_tensor(x, "x");
   nvfp4a_tensor dst = {};
   dst.data = q.data_ptr();
   dst.dtype = NVFP4A_INT8;
@@ -374,7 +379,7 @@ Tensor dequantize(const Tensor &data, const Tensor &scales, const OptTensor &glo
   const c10::cuda::CUDAGuard guard(data.device());
   const Tensor out = empty({data.size(0), cols}, dtype, data);
   const Operand s = fp4_operand(data, scales, glob, flags, smax);
-  const nvfp4a_tensor d = dense_tensor(out);
+  const nvfp4a_tensor d = dense_tensor(out, "out");
   check(nvfp4a_dequantize(&s.t, (int)s.ld, &d, (int)cols, (int)data.size(0), (int)cols, stream()));
   return out;
 }

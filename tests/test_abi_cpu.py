@@ -60,6 +60,15 @@ def test_the_torch_operators_library_belongs_to_one_version_of_torch(monkeypatch
         L.torch_lib_path()
 
 
+def test_addresses_of_host_tensors_are_not_passed_on():
+    """A kernel would fault on them."""
+    import torch
+    from nvfp4effma_b200 import _abi as A
+    assert A.addr(None) is None
+    with pytest.raises(ValueError, match="lives on cpu"):
+        A.addr(torch.zeros(4))
+
+
 def test_struct_layouts_match_the_reference_abi():
     # field order / offsets of nvfp4a_tensor on LP64 (reference include/nvfp4effma.h:46-57)
     T = L.Tensor

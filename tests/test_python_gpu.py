@@ -428,3 +428,24 @@ def test_operator_errors_name_element_types_as_python_does():
     for dtype in (torch.int32, torch.float64, torch.bool):
         with pytest.raises(TypeError, match=f"{dtype} is not one of the dense element types"):
             nf.linear(normal((4, 128), torch.bfloat16, seed=46), w, torch.zeros(128, dtype=dtype, device=GPU))
+
+
+def test_host_tensors_are_refused_before_any_launch():
+    """A kernel would fault on ordinary host memory.  (Every address that the operators pass on goes through one check.)"""
+    w = nf.quantize(normal((128, 128), seed=47))
+    img = nf.TCWeight(w, "exact")
+    x, xh = normal((4, 128), torch.bfloat16, seed=48), torch.zeros(4, 128, dtype=torch.bfloat16)
+    op, ops = w._operand(), torch.ops.nvfp4effma
+    tail = (op.glob, op.flags, op.scale_max, 128, None, torch.bfloat16, 1.0, False)
+    calls = [lambda: nf.linear(xh, w, act="exact"), lambda: nf.linear(xh, img), lambda: nf.linear(xh, w, act="int8"), lambda: nf.linear(xh, w, act="nvfp4"),
+             lambda: nf.linear(x, w, torch.zeros(128)), lambda: nf.linear(x, w, out=torch.zeros(4, 128)),
+             lambda: nf.grouped_linear(x, w, torch.tensor([0, 4], dtype=torch.int32), 1), lambda: nf.quantize(x, torch.tensor([0.5])),
+             lambda: ops.linear(x, None, None, 0, 0, op.data, op.scales.cpu(), *tail, None),
+             lambda: ops.linear(x, None, None, 0, 0, op.data, op.scales, torch.ones(1), *tail[1:], None),
+             lambda: ops.linear(x, None, None, 0, 0, op.data, op.scales, *tail, img.image.cpu()),
+             lambda: ops.linear(xh.to(torch.int8), torch.ones(4, 8), None, 0, 0, op.data, op.scales, *tail, None),
+             lambda: ops.transpose(op.data, op.scales.cpu(), op.flags, op.scale_max, 128)]
+    for call in calls:
+        with pytest.raises(ValueError, match="lives on cpu"):
+            call()
+    assert torch.isfinite(nf.linear(x, w)).all()
