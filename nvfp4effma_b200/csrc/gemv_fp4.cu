@@ -37,6 +37,7 @@
 #include "operands.cuh"
 #include "sm100.cuh"
 #include "tp_barrier.cuh"
+#include "fp4_planes.cuh"
 
 namespace nvb {
 
@@ -248,15 +249,8 @@ gemv_fp4_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
     uint32_t lost = 0;
 #pragma unroll
     for (int t = 0; t < NTOK; ++t) {
-      uint32_t a = 0;
-#pragma unroll
-      for (int u = 0; u < 2; ++u) {
-        const uint32_t w[4] = {xq[t][u].x, xq[t][u].y, xq[t][u].z, xq[t][u].w};
-#pragma unroll
-        for (int i = 0; i < 4; ++i) a = max(a, max(w[i] & 0x7FFFu, (w[i] >> 16) & 0x7FFFu));
-      }
-#pragma unroll
-      for (int o = 16; o; o >>= 1) a = max(a, __shfl_xor_sync(0xFFFFFFFFu, a, o));
+      uint32_t a = max(bf16x8_max(xq[t][0]), bf16x8_max(xq[t][1]));
+      a = __reduce_max_sync(0xFFFFFFFFu, a);
       if (lane == 0) wmax[w2 * NTOK + t] = a;
     }
     named_barrier(2, kDecompThreads);
@@ -265,36 +259,20 @@ gemv_fp4_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
       uint32_t a = 0;
 #pragma unroll
       for (int w = 0; w < 8; ++w) a = max(a, wmax[w * NTOK + t]);
-      const int eb = max((int)(a >> 7), 1);
-      ebs[t] = eb;
-      if (eb == 255) lost = 1;   // Inf or NaN: IEEE arithmetic on the CUDA cores gives each output its own Inf or NaN
-#pragma unroll
-      for (int u = 0; u < 2; ++u) {
-        const int v = t2 + u * kDecompThreads;
-        if (v >= nvec) break;
-        uint32_t X[8], sgn = 0;
-        const uint32_t w[4] = {xq[t][u].x, xq[t][u].y, xq[t][u].z, xq[t][u].w};
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          const uint32_t h = (w[i >> 1] >> (16 * (i & 1))) & 0xFFFFu;
-          const uint32_t e = (h >> 7) & 0xFFu;
-          const uint32_t mant = (h & 0x7Fu) | (e ? 0x80u : 0u);
-          const int sh = (int)max(e, 1u) - eb + 24;  // <= 24
-          X[i] = sh >= 0 ? mant << sh : (sh > -8 ? mant >> (-sh) : 0u);
-          if (sh < 0) lost |= mant & ((1u << min(-sh, 8)) - 1u);   // bits of this element below the last digit plane
-          sgn |= (h >> 15) << (4 * i + 3);
-        }
-        const int chunk = v >> 5, b = (v & 31) * 4;
-        uint8_t *base = pieces + (size_t)chunk * (PR * 128);
-#pragma unroll
-        for (int d = 0; d < 16; ++d) {
-          uint32_t word = sgn;
-#pragma unroll
-          for (int i = 0; i < 8; ++i) word |= ((X[i] >> (2 * d)) & 3u) << (4 * i);
-          const int row = t * 16 + d;
-          *(uint32_t *)(base + (row >> 3) * 1024 + (row & 7) * 128 + ((((b >> 4) ^ (row & 7)) << 4) | (b & 15))) = word;
-        }
-      }
+      ebs[t] = max((int)(a >> 7), kPlaneMinExp);
+      if (ebs[t] == 255) lost = 1;   // Inf or NaN: IEEE arithmetic on the CUDA cores gives each output its own Inf or NaN
+    }
+    // (not unrolled: the code is cold in every launch)
+#pragma unroll 1
+    for (int i = 0; i < 2 * NTOK; ++i) {
+      const int t = i >> 1, v = t2 + (i & 1) * kDecompThreads;
+      if (v >= nvec) continue;
+      const uint4 xv = i == 0 ? xq[0][0] : i == 1 ? xq[0][1] : i == 2 ? xq[NTOK - 1][0] : xq[NTOK - 1][1];
+      const int eb = t ? ebs[NTOK - 1] : ebs[0];
+      uint32_t word[16];
+      planes_of_8(xv, pow2f(158 - eb), word);
+      lost |= planes_lost_bits(xv, eb);
+      store_planes(pieces + (size_t)(v >> 5) * (PR * 128) + t * 2048, (v & 31) * 4, word);
     }
     if (lost) *inexact = 1;
     fence_proxy_async_smem();

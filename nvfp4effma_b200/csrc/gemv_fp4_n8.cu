@@ -34,14 +34,15 @@
 // (reference include/nvfp4effma.h:82-92 there), as the reference's own tensor-core GEMV (src/tensors/gemv_tc.cuh there).
 // Against 64-bit sums the results are about twice as close as the mma.sync GEMV's (28672 x 4096, eight vectors, FP32 D: 6.7e-8 relative
 // against 1.3e-7; activations spread over 2^-17 .. 1: 1.6e-7 against 6.2e-7).
-// What bounds it: 28672 x 4096 takes 20.3 us for four vectors and 23.2 us for eight (66 MB, 10.2 us of HBM time; mma.sync: 30.2 and 32.6 us,
-// which decodes every weight on the CUDA cores); past the stream it is the pieces (0.14 us per chunk and vector) and the tiles' ends.
+// What bounds it: 28672 x 4096 takes 20.1 us for four vectors and 22.8 us for eight (66 MB, 10.6 us of HBM time; mma.sync: 30.6 and 33.6 us,
+// which decodes every weight on the CUDA cores); past the stream it is the pieces (0.11 us per chunk and vector; 0.14 with digits taken one by one and the activations read twice) and the tiles' ends.
 // Negative block scales keep their sign, as in the mma.sync GEMV (gemv.cu) that takes the calls this kernel leaves.
 #include <math.h>
 #include <atomic>
 #include "operands.cuh"
 #include "sm100.cuh"
 #include "tp_barrier.cuh"
+#include "fp4_planes.cuh"
 
 namespace nvb {
 
@@ -87,27 +88,6 @@ __host__ __device__ constexpr int max_chunks(int ntok) { return ntok == 4 ? 14 :
 __host__ __device__ constexpr int fixed_bytes(int ntok, int buffers) { return 512 + buffers * ntok * 1024 + 512; }
 
 __device__ __forceinline__ float pow2f(int e) { return __int_as_float((e + 127) << 23); }  // -126 <= e <= 127
-
-// Digits of eight 32-bit integers whose nibbles hold one base-4 digit each: word j of the result is nibble j of x[0], x[1], .. x[7]
-// (an 8 x 8 transposition of nibbles: two logical steps, then byte permutes).
-__device__ __forceinline__ void transpose_nibbles(const uint32_t (&x)[8], uint32_t (&out)[8]) {
-  uint32_t lo[4], hi[4];   // byte t of lo[p] / hi[p]: nibble 2 t / 2 t + 1 of x[2 p] (low) and x[2 p + 1] (high)
-#pragma unroll
-  for (int p = 0; p < 4; ++p) {
-    lo[p] = (x[2 * p] & 0x0F0F0F0Fu) | ((x[2 * p + 1] << 4) & 0xF0F0F0F0u);
-    hi[p] = ((x[2 * p] >> 4) & 0x0F0F0F0Fu) | (x[2 * p + 1] & 0xF0F0F0F0u);
-  }
-#pragma unroll
-  for (int h = 0; h < 2; ++h) {
-    const uint32_t *b = h ? hi : lo;
-    const uint32_t a01 = byte_perm(b[0], b[1], 0x5140u), a23 = byte_perm(b[2], b[3], 0x5140u);   // bytes 0, 1
-    const uint32_t c01 = byte_perm(b[0], b[1], 0x7362u), c23 = byte_perm(b[2], b[3], 0x7362u);   // bytes 2, 3
-    out[h] = byte_perm(a01, a23, 0x5410u);
-    out[2 + h] = byte_perm(a01, a23, 0x7632u);
-    out[4 + h] = byte_perm(c01, c23, 0x5410u);
-    out[6 + h] = byte_perm(c01, c23, 0x7632u);
-  }
-}
 
 // Block scale code 0x7F (with either sign) is 480 everywhere in this library, as in the reference's decode; the tensor cores take it for a NaN, which
 // reaches the partial sums of that weight row and of no other (activations and weights are finite here).  Such a row's sum over the CTA's
@@ -352,50 +332,28 @@ gemv_fp4_n8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
     for (int u = 0; u < NI; ++u) {
       const int idx = t2 + u * kDecompThreads;
       if (idx >= items) break;
-      const uint32_t w[4] = {xq[u].x, xq[u].y, xq[u].z, xq[u].w};
-      uint32_t a = 0;
-#pragma unroll
-      for (int i = 0; i < 4; ++i) a = max(a, max(w[i] & 0x7FFFu, (w[i] >> 16) & 0x7FFFu));
+      uint32_t a = bf16x8_max(xq[u]);
       a = __reduce_max_sync(0xFFFFFFFFu, a);
       if (lane == 0) atomicMax(&wmax[idx / nvec], a);
     }
     named_barrier(2, kDecompThreads);
-    auto eb_of = [&](int t) { return max((int)(wmax[t] >> 7), 1); };   // biased exponent the token's pieces refer to
+    auto eb_of = [&](int t) { return max((int)(wmax[t] >> 7), kPlaneMinExp); };   // biased exponent the token's pieces refer to
     uint32_t lost = 0;
-    uint4 x_next = xq[0];
 #pragma unroll 1
-    for (int idx = t2; idx < items; idx += kDecompThreads) {
-      const uint4 x = x_next;
-      if (idx + kDecompThreads < items) x_next = load_x(idx + kDecompThreads);   // (in L2 since the maximum was taken; the ring leaves L1 next to nothing)
+    for (int u = 0; u < NI; ++u) {
+      const int idx = t2 + u * kDecompThreads;
+      if (idx >= items) break;
+      uint4 x = xq[0];   // (selects, not a reload: from L2 it cost each turn its latency)
+#pragma unroll
+      for (int q = 1; q < NI; ++q)
+        if (u == q) x = xq[q];
       const int t = idx / nvec, v = idx - t * nvec;
       const int eb = eb_of(t);
       if (eb == 255) lost = 1;   // Inf or NaN: IEEE arithmetic on the CUDA cores gives each output its own Inf or NaN
-      uint32_t X[8], sgn = 0;
-      const uint32_t w[4] = {x.x, x.y, x.z, x.w};
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const uint32_t h = (w[i >> 1] >> (16 * (i & 1))) & 0xFFFFu;
-        const uint32_t e = (h >> 7) & 0xFFu;
-        const uint32_t mant = (h & 0x7Fu) | (e ? 0x80u : 0u);
-        const int sh = (int)max(e, 1u) - eb + 24;  // <= 24
-        X[i] = sh >= 0 ? mant << sh : (sh > -8 ? mant >> (-sh) : 0u);
-        if (sh < 0) lost |= mant & ((1u << min(-sh, 8)) - 1u);   // bits of this element below the last digit plane
-        sgn |= (h >> 15) << (4 * i + 3);
-      }
-      const int chunk = v >> 5, b = (v & 31) * 4;
-      uint8_t *base = pieces + (size_t)chunk * (PR * 128) + t * 2048;
-#pragma unroll
-      for (int odd = 0; odd < 2; ++odd) {   // even digits, then odd ones: one digit per nibble, nibbles transposed
-        uint32_t dig[8], word[8];
-#pragma unroll
-        for (int i = 0; i < 8; ++i) dig[i] = (odd ? X[i] >> 2 : X[i]) & 0x33333333u;
-        transpose_nibbles(dig, word);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          const int row = 2 * j + odd;   // piece d = 2 j + odd of the token
-          *(uint32_t *)(base + (row >> 3) * 1024 + (row & 7) * 128 + ((((b >> 4) ^ (row & 7)) << 4) | (b & 15))) = word[j] | sgn;
-        }
-      }
+      uint32_t word[16];
+      planes_of_8(x, pow2f(158 - eb), word);
+      lost |= planes_lost_bits(x, eb);
+      store_planes(pieces + (size_t)(v >> 5) * (PR * 128) + t * 2048, (v & 31) * 4, word);
     }
     if (lost) *inexact = 1;
     fence_proxy_async_smem();
@@ -612,7 +570,7 @@ int gemv_fp4_pinned_splits();   // (gemv_fp4.cu) nvfp4a_b200_set_gemv_splits: 0 
 // takes an SM; 148, 74, 33 and 15 clusters of 1, 2, 4 and 8 by cudaOccupancyMaxActiveClusters): more are not launched, a cluster takes
 // several tiles instead.  Automatic: the cut with the shortest estimate, fitted to CUDA-graph timings of 12 shapes from 1024 x 1024 to 28672 x
 // 4096 and up to 8 vectors (within about 10 %): 4.4 us of set-up and tail (4.8 in a cluster), the stream (36 KiB per chunk at 61 GB/s
-// per CTA or 5.4 TB/s in all), the pieces (0.14 us per chunk and vector past the first) and the tiles' ends, which clusters of eight pay most for.
+// per CTA or 5.4 TB/s in all), the pieces (0.11 us per chunk and vector past the first) and the tiles' ends, which clusters of eight pay most for.
 struct GemvCut { int splits, clusters, rounds; double us; };
 static int ntok_of(int n) { return n <= 4 ? 4 : 8; }   // tokens of the kernel instance
 static GemvCut cut_for(int m, int k, int n, int splits) {
@@ -623,7 +581,7 @@ static GemvCut cut_for(int m, int k, int n, int splits) {
   const int rounds = (tiles + cap - 1) / cap, clusters = (tiles + rounds - 1) / rounds, ctas = clusters * splits;
   const double chunk = fmax(0.6, ctas * 36.9e3 / 5.4e6);
   const int more = ntok_of(n) - 1;
-  return {splits, clusters, rounds, (splits > 1 ? 4.8 : 4.4) + (0.1 + 0.14 * nloc) * more + (0.06 * more + (splits == 8 ? 1.2 : 0.05)) * (rounds - 1) + rounds * nloc * chunk};
+  return {splits, clusters, rounds, (splits > 1 ? 4.8 : 4.4) + (0.1 + 0.11 * nloc) * more + (0.06 * more + (splits == 8 ? 1.2 : 0.05)) * (rounds - 1) + rounds * nloc * chunk};
 }
 static GemvCut choose_cut(int m, int k, int n) {
   if (const int f = gemv_fp4_pinned_splits()) return cut_for(m, k, n, f);   // pinned (nvfp4a_b200_set_gemv_splits): that value if the problem can use it
@@ -633,8 +591,8 @@ static GemvCut choose_cut(int m, int k, int n) {
     if (c.splits && (!best.splits || c.us < best.us)) best = c;
   }
   // The mma.sync GEMV has less to set up and takes 3 us and 0.4 us per megabyte (same timings): it keeps small matrices, and middling ones
-  // as the number of vectors grows (28672 x 4096: 30.2 against 20.3 us for four vectors, 32.6 against 23.2 us for eight; 8192 x 8192, eight:
-  // 22.0 against 18.5, which the estimate misses; 4096 x 14336: 17.7 against 16.9 and 18.5 against 23.7; 4096 x 4096, eight: 7.6 against 11.6).
+  // as the number of vectors grows (28672 x 4096: 30.6 against 20.1 us for four vectors, 33.6 against 22.8 us for eight; 8192 x 8192, eight:
+  // 22.0 against 18.5, which the estimate misses; 4096 x 14336: 17.7 against 16.9 and 18.5 against 23.7; 4096 x 4096, eight: 7.6 against 10.8).
   if (best.us > 3.0 + 0.405 * (m * (k * 0.5625e-6)) * (1.0 + 0.012 * (n - 1))) best.splits = 0;
   return best;
 }

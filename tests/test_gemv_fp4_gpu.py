@@ -293,3 +293,26 @@ def test_block_scale_code_7f_of_several_vectors(pin, layout):
         assert np.isfinite(exp["ref64"]).all()
         check_bound(c, h, got, amax, exp)
     assert kernel_status() == 0
+
+
+@pytest.mark.parametrize("spread", [0, 23, 24, 25, 31, 200])
+def test_digit_planes_at_the_edges_of_their_range(pin, spread):
+    """Activations whose largest and smallest magnitudes are 2^spread apart, around the last digit plane, with subnormals, signed zeros and a token of
+    zeros; and tokens too small for the planes' scale to be a float (eb < 31)."""
+    for i, (n, top) in enumerate([(1, 1.0), (2, 2.0 ** -100), (8, 2.0 ** 100), (5, 2.0 ** -120)]):
+        pin(2)
+        m, k = 300, 1024
+        c = Case(m, n, k, L.BF16, L.FP32, -1, -1, 1.0, 0.0, fa=SW)
+        h = build_case(c, 1700 + i)
+        rng = np.random.default_rng(1700 + spread + i)
+        x = (rng.uniform(1, 2, (n, h["ldb"])) * rng.choice([-1.0, 1.0], (n, h["ldb"]))).astype(np.float32) * np.float32(top)
+        x[:, ::3] *= np.float32(2.0) ** -spread
+        x[:, 5] = -0.0
+        if n == 5:
+            x[2] = 0.0
+        h["B"] = O.Dense(L.BF16, O.from_f32(x.reshape(-1), L.BF16), h["ldb"])
+        exp = oracle_case(c, h, want_ref=True)
+        got, amax = run_gemm(c, h)
+        assert L.lib.nvfp4a_b200_last_route() == FP4_GEMV, c
+        check_bound(c, h, got, amax, exp)
+    assert kernel_status() == 0
