@@ -134,7 +134,12 @@ __device__ __forceinline__ void mma4_f16_commit_pair_elect(uint32_t d_tmem, uint
 struct Tile { int tm, j0, jend, width, ro; };
 constexpr int kMaxGroups = 256;
 
-template <int PLANES, bool F16, bool GROUPED>
+// EPI: what the epilogue is compiled for.  0: everything; 1: a 16-bit D, alpha, globals and bias; 2: the same and SwiGLU.  The whole of it is 150 KiB of code in
+// which a plain call's instructions lie far apart: fetching them made a chunk of 32 columns take 5000 cycles, in which the tensor cores wait for the
+// accumulator or, at the end, the caller for the result.  28672 x 4096 with SwiGLU on 2048 tokens: 412 -> 344 us; FP16 4096 x 4096 on 333
+// tokens 37.5 -> 35.2; 5504 x 3584 with SwiGLU on 121 tokens 32.1 -> 27.0.
+enum { kEpiAny = 0, kEpiPlain = 1, kEpiSwiglu = 2 };
+template <int PLANES, bool F16, bool GROUPED, int EPI>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_b, const __grid_constant__ CUtensorMap tmap_d,
                   const __grid_constant__ PeerMaps peers, const W4A16Args g) {
@@ -326,7 +331,7 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
     // (rarely used parameters are read from the constant bank where they are needed: the registers belong to the accumulator block)
     const float gb0 = g.e.gb ? *g.e.gb : 1.f;   // B's global: dense B has none, INT8 B one for the tensor (a multiply by 1 is exact)
     uint8_t *const dptr = (uint8_t *)g.e.d;
-    const int d_dtype = g.e.d_dtype, mask = SEG ? 0 : g.x.mask;   // (segments: a 16-bit D and the plain epilogue)
+    const int d_dtype = g.e.d_dtype, mask = EPI == kEpiSwiglu ? kExSwiglu : SEG || EPI == kEpiPlain ? 0 : g.x.mask;   // (segments: a 16-bit D and the plain epilogue)
     const bool d_tma = g.d_tma;
     // The accumulator is read as MMA fragments (16 lanes x 8 columns per register quad): a thread holds rows rb + 16 hh + 8 u (hh, u in
     // {0, 1}) of columns 8 gq + cp + e (e in {0, 1}) of a chunk of 32, register 16 hh + 4 gq + 2 u + e.  Gate and up rows of SwiGLU (8
@@ -392,7 +397,7 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
       for (int q = 0; q < 4; ++q) {
         const int i = rb + 8 * q;
         rowp[q] = i < gm ? __fmul_rn(g.e.alpha, g.e.ga ? g.e.ga[(size_t)(p.ro + i) * g.e.ga_stride] : 1.f) : 0.f;
-        bias[q] = (i < gm && g.e.bias) ? load_dense(g.e.bias_dtype, g.e.bias, p.ro + i) : 0.f;
+        bias[q] = (i < gm && g.e.bias) ? load_dense(g.e.bias_dtype, g.e.bias, p.ro + i) : -0.f;   // (adding -0 changes nothing)
         if (!(mask & kExNorm)) rowp[q] = __fmul_rn(__fmul_rn(rowp[q], gb0), g.e.gf);   // ((alpha gA) * gB) * gf
       }
       if (mask & kExNorm) {  // column scales of this token tile (the previous tile's are no longer in use: see the barrier below)
@@ -486,9 +491,9 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
               uint32_t &x = r[16 * (q >> 1) + 4 * gq + 2 * (q & 1) + e];
               const float sc = (mask & kExNorm) ? __fmul_rn(__fmul_rn(rowp[q], __fmul_rn(gb0, e ? cs.y : cs.x)), g.e.gf) : rowp[q];
               float v = __fmul_rn(__uint_as_float(x), sc);
-              if (g.e.bias) v = __fadd_rn(v, bias[q]);
+              v = __fadd_rn(v, bias[q]);
               const int jj = 8 * gq + cp + e;
-              if (g.e.beta != 0.f && rb + 8 * q < gm && jj < nvalid)
+              if (EPI == kEpiAny && g.e.beta != 0.f && rb + 8 * q < gm && jj < nvalid)
                 v = __fmaf_rn(g.e.beta, load_dense(g.e.c_dtype, g.e.c, (size_t)(j0 + jj) * g.e.ldc + rb + 8 * q), v);
               x = __float_as_uint(v);
             }
@@ -527,7 +532,7 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
               r[at] = __float_as_uint(silu_mul(__uint_as_float(r[at]), __uint_as_float(r[at + 2])));
             }
         }
-        if (g.e.amax) {
+        if (EPI == kEpiAny && g.e.amax) {
 #pragma unroll
           for (int q = 0; q < 4; ++q)
 #pragma unroll
@@ -536,7 +541,7 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
                 amax = fmaxf(amax, fabsf(__uint_as_float(r[16 * (q >> 1) + 4 * (ce >> 1) + 2 * (q & 1) + (ce & 1)])));
         }
         const int orow = glu ? tm * 64 : tm * 128, orows = glu ? gm >> 1 : gm;   // the tile's first output row, rows of D
-        if (!SEG && d_dtype == NVFP4A_FP32) {   // eight lanes write 32 contiguous bytes of a column
+        if (!SEG && EPI == kEpiAny && d_dtype == NVFP4A_FP32) {   // eight lanes write 32 contiguous bytes of a column
           float *const d32 = (float *)dptr + (size_t)j0 * g.e.ldd + orow + (lane >> 2);
 #pragma unroll
           for (int q = 0; q < 4; ++q) {
@@ -612,7 +617,7 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
       }
     }
     if (leader) bulk_wait_all();
-    if (g.e.amax) warp_amax_commit(g.e.amax, amax);
+    if (EPI == kEpiAny && g.e.amax) warp_amax_commit(g.e.amax, amax);
   } else {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsConv));
     // ---------------- weight expansion: NVFP4 -> 16-bit floats in tensor memory ----------------
@@ -744,14 +749,14 @@ Plan make_grouped_plan(int rows256, int n, int groups, int planes, int pairs, in
   return best;
 }
 
-template <int PLANES, bool F16, bool GROUPED = false>
-cudaError_t launch_cfg(const CUtensorMap &tw, const CUtensorMap &tb, const CUtensorMap &td, const PeerMaps &pm, const W4A16Args &a, cudaStream_t s) {
+template <int PLANES, bool F16, bool GROUPED, int EPI>
+cudaError_t launch_epi(const CUtensorMap &tw, const CUtensorMap &tb, const CUtensorMap &td, const PeerMaps &pm, const W4A16Args &a, cudaStream_t s) {
   using C = Cfg<PLANES, GROUPED>;
   static std::atomic<bool> attr_set[64];   // zero-initialised; set once per device (a repeated cudaFuncSetAttribute is harmless)
   int dev = 0;
   cudaGetDevice(&dev);
   if (!attr_set[dev & 63]) {
-    const cudaError_t e = cudaFuncSetAttribute(gemm_w4a16_kernel<PLANES, F16, GROUPED>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes);
+    const cudaError_t e = cudaFuncSetAttribute(gemm_w4a16_kernel<PLANES, F16, GROUPED, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes);
     if (e != cudaSuccess) return e;
     attr_set[dev & 63] = true;
   }
@@ -768,7 +773,16 @@ cudaError_t launch_cfg(const CUtensorMap &tw, const CUtensorMap &tb, const CUten
   attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr; cfg.numAttrs = pdl_enabled() ? 2 : 1;
-  return cudaLaunchKernelEx(&cfg, gemm_w4a16_kernel<PLANES, F16, GROUPED>, tw, tb, td, pm, a);
+  return cudaLaunchKernelEx(&cfg, gemm_w4a16_kernel<PLANES, F16, GROUPED, EPI>, tw, tb, td, pm, a);
+}
+
+template <int PLANES, bool F16, bool GROUPED = false>
+cudaError_t launch_cfg(const CUtensorMap &tw, const CUtensorMap &tb, const CUtensorMap &td, const PeerMaps &pm, const W4A16Args &a, cudaStream_t s) {
+  const bool plain = a.e.beta == 0.f && !a.e.amax && a.e.d_dtype != NVFP4A_FP32;
+  if constexpr (!F16 && !GROUPED)
+    if (plain && a.x.mask == kExSwiglu) return launch_epi<PLANES, F16, GROUPED, kEpiSwiglu>(tw, tb, td, pm, a, s);
+  if (plain && a.x.mask == 0) return launch_epi<PLANES, F16, GROUPED, kEpiPlain>(tw, tb, td, pm, a, s);
+  return launch_epi<PLANES, F16, GROUPED, kEpiAny>(tw, tb, td, pm, a, s);
 }
 
 // what every launch of the kernel shares: arguments, the schedule, the maps of the weights, of the activations (`row_bytes` bytes per

@@ -946,3 +946,50 @@ def test_w4a16_gemm_decodes_signed_block_scales(bt):
         got, amax = run_gemm(c, h)
         assert L.lib.nvfp4a_b200_last_route() == 5
         check_bound(c, h, got, amax, exp)
+
+
+@pytest.mark.parametrize("bt", [L.BF16, L.FP16, L.INT8])
+@pytest.mark.parametrize("case", ["plain", "bias", "swiglu", "grouped"])
+def test_w4a16_epilogues_compiled_for_plain_calls_equal_the_general_one(bt, case):
+    """Calls with a 16-bit D and nothing but scales, bias and SwiGLU take an epilogue of their own; an amax wish brings the general one: the same bytes.
+    D that TMA stores and D that it does not, ragged tiles, -0 results without a bias."""
+    if (case == "swiglu" and bt == L.FP16) or (case == "grouped" and bt != L.INT8):
+        pytest.skip("not a combination the entry points take")
+    m, n, k = 528, 300, 640
+    gen = torch.Generator(device="cuda").manual_seed(17)
+    ints = lambda lo, hi, shape, t=torch.uint8: torch.randint(lo, hi, shape, generator=gen, device="cuda", dtype=t)
+    groups = 3 if case == "grouped" else 1
+    w, ws = ints(0, 256, (groups * m, k // 2)), ints(0x28, 0x48, (groups * m, k // 16))
+    ta, x, xs = tensor(w, L.NVFP4, ws, k // 16), None, None
+    if bt == L.INT8:
+        x, xs = ints(-127, 128, (n, k), torch.int8), torch.rand(n, k // 16, generator=gen, device="cuda") + 0.1
+        x[7] = 0
+        tb = tensor(x, L.INT8, xs, k // 16)
+    else:
+        x = torch.randn(n, k, generator=gen, device="cuda").to(torch.bfloat16 if bt == L.BF16 else torch.float16)
+        x[7] = -0.0
+        tb = tensor(x, bt)
+    bias = torch.randn(groups * m, generator=gen, device="cuda").to(torch.bfloat16)
+    tbias = tensor(bias, L.BF16) if case in ("bias", "grouped") else None
+    seg = torch.tensor([0, 65, 66, n], dtype=torch.int32, device="cuda")
+    ex = L.Epilogue()
+    ex.swiglu = int(case == "swiglu")
+    mo = m // 2 if case == "swiglu" else m
+    for dt in (torch.bfloat16, torch.float16):
+        for ld in (mo, mo + 3):
+            outs = []
+            for amax in (None, torch.zeros(1, dtype=torch.float32, device="cuda")):
+                D = torch.zeros(n, ld, dtype=dt, device="cuda")
+                td = tensor(D, L.BF16 if dt == torch.bfloat16 else L.FP16, amax=amax)
+                pb = ctypes.byref(tbias) if tbias is not None else None
+                if case == "grouped":
+                    L.check(L.lib.nvfp4a_gemm_grouped(groups, m, k, n, -0.01, ctypes.byref(ta), k, ctypes.byref(tb), k, 0.0, None, 0, ctypes.byref(td), ld, pb,
+                                                      ctypes.c_void_p(seg.data_ptr()), stream()))
+                elif case == "swiglu":
+                    L.check(L.lib.nvfp4a_gemm_ex(m, n, k, -0.01, ctypes.byref(ta), k, ctypes.byref(tb), k, 0.0, None, 0, ctypes.byref(td), ld, pb, ctypes.byref(ex), stream()))
+                else:
+                    L.check(L.lib.nvfp4a_gemm(m, n, k, -0.01, ctypes.byref(ta), k, ctypes.byref(tb), k, 0.0, None, 0, ctypes.byref(td), ld, pb, stream()))
+                assert L.lib.nvfp4a_b200_last_route() == (8 if bt == L.INT8 else 5)
+                outs.append(D.view(torch.int16))
+            assert bool(outs[0].any()) and torch.equal(outs[0], outs[1])
+    assert kernel_status() == 0
