@@ -691,7 +691,7 @@ def bench_mlp(args, L, W, dev, rank, world, dist, stream, peaks, traffic):
             "gate_up": {"m": 2 * I, "k": H, "epilogue": "RMSNorm column scale + bias + SwiGLU + amax", "ms": ms_gu, "tflops": tf(f_gu, ms_gu)},
             "down": {"m": H, "k": I, "epilogue": "bias + second output * w2 + sums of squares + amax", "ms": ms_dn, "tflops": tf(f_dn, ms_dn)},
             "gate_up_w4a8": {"entry": "nvfp4a_gemm_ex, INT8 activations",
-                             "kernel": {8: "W4A16 tcgen05 kernel on three BF16 planes of the activations (within the accumulation bound)",
+                             "kernel": {8: "W4A16 tcgen05 kernel on two FP16 planes of the activations (within the accumulation bound)",
                                         7: "DP4A tiled GEMM (exact block sums, CUDA cores)"}.get(route8, str(route8)),
                              "ms": ms_gu8, "tflops": tf(f_gu, ms_gu8), "includes": "the planes' allocation from the stream's pool and their conversion kernel",
                              "exact_dp4a": {"ms": ms_gu8x, "tflops": tf(f_gu, ms_gu8x), "how": "nvfp4a_b200_set_route(3): bit-identical to the reference's tiled order"}},

@@ -85,7 +85,7 @@ int nvfp4a_b200_set_swap(int mode);
 
 /* The kernel the calling thread's last GEMM / GEMV call launched: 1 CUDA cores, 2 mma.sync GEMV, 3 FP4 tensor-core GEMV, 4 W4A4
  * tcgen05 GEMM, 5 W4A16 tcgen05 GEMM, 6 GEMV for INT8 / NVFP4 activations, 7 DP4A GEMM for INT8
- * activations, 8 W4A8 on the W4A16 tcgen05 kernel (INT8 activations as three BF16 planes); 0 before any call.  Test aid, no
+ * activations, 8 W4A8 on the W4A16 tcgen05 kernel (INT8 activations as two FP16 or three BF16 planes); 0 before any call.  Test aid, no
  * counterpart in the reference. */
 int nvfp4a_b200_last_route(void);
 

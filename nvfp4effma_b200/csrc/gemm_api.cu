@@ -94,7 +94,7 @@ static nvfp4a_status check_epilogue_operands(const char *fn, int m, float beta, 
 
 // kernel the last GEMM call of this thread launched (nvfp4a_b200_last_route): 1 CUDA cores, 2 mma.sync GEMV, 3 FP4 tensor-core
 // GEMV, 4 W4A4 tcgen05 GEMM, 5 W4A16 tcgen05 GEMM, 6 GEMV for INT8 / NVFP4 activations, 7 DP4A GEMM for INT8 activations,
-// 8 W4A8 on the W4A16 tcgen05 kernel (INT8 activations as three BF16 planes)
+// 8 W4A8 on the W4A16 tcgen05 kernel (INT8 activations as two FP16 or three BF16 planes)
 static thread_local int g_last_route = 0;
 // (defined in gemm_dp4a.cu) the DP4A GEMM over groups of tokens: nvfp4a_gemm_grouped with INT8 activations
 cudaError_t launch_gemm_dp4a_grouped(const GemmArgs &g, const int *seg, int groups, cudaStream_t s);

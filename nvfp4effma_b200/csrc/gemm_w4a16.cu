@@ -14,7 +14,7 @@
 // Roles, 20 warps per CTA:
 //   warp 0      TMA producer of the activations: this CTA's half of the tile's tokens (no multicast); the bytes of both CTAs are
 //               counted on the even CTA's barrier
-//   warp 1      MMA issuer (even CTA; 4 x K16 per stage, one elected lane), owner of the tensor memory
+//   warp 1      MMA issuer (even CTA; 8 or 12 x K16 per unit of work, one elected lane), owner of the tensor memory
 //   warp 2      TMA producer of the weight nibbles: [128 rows][128 bytes] = 256 values of k per slot, so that the expansion
 //               reads shared memory and never waits for a trip to L2
 //   warps 4-11  epilogue (144 registers each, taken from the others by setmaxnreg), one 32-lane quadrant and one half of the columns
@@ -43,18 +43,22 @@
 // not matter, have an accumulator of their own for all of k.  Error: 1.05e-7 and 9.8e-8 at k = 4096 (normal data; 2.9e-7 and 1.4e-7 against
 // 6.9e-7 and 2.9e-7 with activations spread over ten binades).  Below k = 1024 segments are 2 stages, below 512 one (INT8 at k = 512:
 // 6.2e-8 against 1.08e-7; FP16 at k = 512, 128 and 64: 6.3e-8, 4.2e-8 and 4.0e-8 against 6.9e-8, 4.1e-8 and 3.7e-8).
-// Cost: 8 experts of 2048 x 4096 on 1100 tokens 132 us instead of 102 (125 with tiles of 128 tokens in one chain), FP16 4096 x 4096 on 333
-// tokens 38.5 instead of 36.3 us; the CUDA-core kernels take 602 and 1932 us.
+// 8 experts of 2048 x 4096 on 1100 tokens take 96 us, FP16 4096 x 4096 on 333 tokens 35; the CUDA-core kernels 602 and 1932 us.
 //
 // Grouped (mixture of experts): A stacks the weights of all groups, a group owns the tokens [seg[q], seg[q + 1]); the CTAs read seg
 // (device memory) into a table of tile counts and find a tile's group there.  (INT8 activations only, plain epilogue, 16-bit D.)
 //
-// INT8 activations (W4A8, FP32 scale per 16 values) run on the same kernel with PLANES = 3: an activation is the FP32 value
-// x = q * s_b (one rounding: within the accumulation bound of the exact definition, not bit-identical to the integer block sums
-// of the DP4A kernels), split exactly into three BF16 terms x = t1 + t2 + t3 (8 + 8 + 8 significant bits) by a small kernel
-// that runs first.  The terms lie side by side as [token][3][k]; the activation ring holds one plane of a stage per slot, and the
-// MMA issuer accumulates weight x t1, weight x t2, weight x t3 from one expanded weight tile into the same accumulator (grouped: the last two
-// into one of their own, see Segments).
+// INT8 activations (W4A8, FP32 scale s_b per 16 values) run on the same kernel as planes [token][3][k] that a small kernel makes first.
+// PLANES = 2 (one weight): x = q * s_b is t1 + t2, two FP16 terms of 11 bits each, on a grid that puts the token's largest below 2^15 (the epilogue
+// takes that power of two back).  t2 is the exact remainder's rounding: together they are x to within 2^-23 of it, or 2^-25 on the grid, which the
+// (k + 2) 2^-24 of the accumulation bound covers for every value while a token's scales lie within 2^12 of each other.  If some token's do not, or its
+// scales are not near enough to one for the grid's power of two to be a float, or the weights' scales are UE5M3 (products leave FP16's range), all
+// tokens are three BF16 planes instead, t1 + t2 + t3 = fl(q * s_b) exactly (8 + 8 + 8 bits), and a word in memory tells this kernel so.  One chain in the
+// tensor cores, 2-norm error at k = 512 / 1024 / 4096 / 8192: 0.97e-6, 1.9e-6, 8.2e-6, 1.69e-5 (three planes: 1.4e-6, 2.6e-6, 9.9e-6, 1.91e-5).
+// 6144 x 4096 on 1000 tokens 125 us with three planes and an MMA issue per plane, 93 with two.
+// PLANES = 3 (grouped): always three BF16 planes, the last two in an accumulator of their own (see Segments).  Two FP16 planes would be 94 us instead of 96
+// (8 experts of 2048 x 4096 on 1100 tokens), but 11-bit terms lose more to the truncation in the tensor cores than 8-bit ones, whose sums stay
+// on a coarse grid: 1.6e-7 instead of 0.74e-7 at k = 4096.
 #include <atomic>
 #include <cuda_bf16.h>
 #include "operands.cuh"
@@ -78,7 +82,9 @@ struct W4A16Args {
   int nfull, cut;   // tiles 0 .. nfull - 1 are `width` tokens wide; the rest (to `tiles`) are parts of width / cut tokens
   int tiles;
   int seg_stages;   // F16, GROUPED: stages per segment of k
+  int unit;         // stages per unit: 1 or 2 (see the MMA issuer)
   const int *seg; int groups;   // GROUPED: m is the rows of ONE group's weight, n the bound on seg[groups]
+  const float *tscale;          // PLANES = 2: what each token's sums are multiplied by, then (word n) non-zero for three planes
 };
 
 // tensor maps of D in the peers' buffers (tensor-parallel all-gather fused into the epilogue's TMA stores); n = 0: none
@@ -93,13 +99,13 @@ struct Cfg {
   static constexpr int kA = GROUPED ? 4 : 8, kB = 8, kRaw = 3;
   static constexpr int kACols = 512 - 32 * kA;   // first tensor memory column of the weight stages (32 columns each)
   static constexpr int kBBytes = 128 * 128, kRawBytes = 128 * 128, kStagingBytes = 8192;
-  static constexpr int kSmemBytes = 1024 + kB * kBBytes + kRaw * kRawBytes + 4 * kStagingBytes + 4096 /* expansion table */ + 256 * 4 /* column scales */ +
+  static constexpr int kSmemBytes = 1024 + kB * kBBytes + kRaw * kRawBytes + 4 * kStagingBytes + (PLANES == 2 ? 8192 : 4096) /* expansion tables */ + 256 * 4 /* column scales */ +
                                     512 /* barriers */ + 2 * 257 * 4 + 8 /* groups */;
 };
-static_assert(Cfg<1, false>::kSmemBytes <= 232448, "shared memory budget");
+static_assert(Cfg<1, false>::kSmemBytes <= 232448 && Cfg<2, false>::kSmemBytes <= 232448, "shared memory budget");
 constexpr int kSegmentWidth = 128;   // tokens per tile where k is summed in segments: the running sums have to fit the epilogue's registers
 
-constexpr int kThreads = 640, kRegsRest = 40, kRegsEpi = 144, kRegsConv = 72;
+constexpr int kThreads = 640, kRegsRest = 48, kRegsEpi = 144, kRegsConv = 72;
 static_assert(128 * kRegsRest + 256 * kRegsEpi + 256 * kRegsConv <= kThreads * 96, "the split draws on the registers of the launch: 96 per thread");
 constexpr unsigned kStWaitFullA = 0x301, kStWaitFullB = 0x302, kStWaitEmpty = 0x303, kStWaitTmemFull = 0x304, kStWaitTmemEmpty = 0x305,
                    kStWaitConv = 0x306, kStWaitRaw = 0x307;
@@ -115,8 +121,24 @@ __device__ __forceinline__ void stmatrix_x4_trans(void *row, uint32_t a, uint32_
   asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1, %2, %3, %4};" ::"r"(smem_u32(row)), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
 }
 
-// one stage's four MMAs (K = 16 each: 8 tensor memory columns of A, 32 bytes along B's 128-byte rows) over a CTA pair and the commit that hands the activation slot
-// back in both CTAs, in one statement issued by one elected lane of a converged warp
+// Four MMAs (K = 16 each: 8 tensor memory columns of A, 32 bytes along B's 128-byte rows) over a CTA pair, twice, and the commit that hands the
+// slots back in both CTAs, in one statement issued by one elected lane of a converged warp.
+__device__ __forceinline__ void mma8_f16_commit_pair_elect(uint32_t d0, uint32_t a0, uint64_t b0, uint32_t acc0, uint32_t d1, uint32_t a1, uint64_t b1, uint32_t acc1,
+                                                           uint32_t idesc, uint64_t *bar) {
+  asm volatile("{\n\t.reg .pred p, u, q, t;\n\tsetp.ne.b32 p, %3, 0;\n\tsetp.ne.b32 u, %7, 0;\n\tsetp.eq.u32 t, %8, %8;\n\telect.sync _|q, 0xFFFFFFFF;\n\t"
+               "@q tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %8, p;\n\t"
+               "@q tcgen05.mma.cta_group::2.kind::f16 [%0], [%9], %10, %8, t;\n\t"
+               "@q tcgen05.mma.cta_group::2.kind::f16 [%0], [%11], %12, %8, t;\n\t"
+               "@q tcgen05.mma.cta_group::2.kind::f16 [%0], [%13], %14, %8, t;\n\t"
+               "@q tcgen05.mma.cta_group::2.kind::f16 [%4], [%5], %6, %8, u;\n\t"
+               "@q tcgen05.mma.cta_group::2.kind::f16 [%4], [%15], %16, %8, t;\n\t"
+               "@q tcgen05.mma.cta_group::2.kind::f16 [%4], [%17], %18, %8, t;\n\t"
+               "@q tcgen05.mma.cta_group::2.kind::f16 [%4], [%19], %20, %8, t;\n\t"
+               "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%21], %22;\n\t}"
+               ::"r"(d0), "r"(a0), "l"(b0), "r"(acc0), "r"(d1), "r"(a1), "l"(b1), "r"(acc1), "r"(idesc), "r"(a0 + 8), "l"(b0 + 2), "r"(a0 + 16), "l"(b0 + 4),
+                 "r"(a0 + 24), "l"(b0 + 6), "r"(a1 + 8), "l"(b1 + 2), "r"(a1 + 16), "l"(b1 + 4), "r"(a1 + 24), "l"(b1 + 6), "r"(smem_u32(bar)), "h"((uint16_t)3)
+               : "memory");
+}
 __device__ __forceinline__ void mma4_f16_commit_pair_elect(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate,
                                                            uint64_t *bar) {
   asm volatile("{\n\t.reg .pred p, q, t;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.eq.u32 t, %3, %3;\n\telect.sync _|q, 0xFFFFFFFF;\n\t"
@@ -127,6 +149,27 @@ __device__ __forceinline__ void mma4_f16_commit_pair_elect(uint32_t d_tmem, uint
                "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%11], %12;\n\t}"
                ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(a_tmem + 8), "l"(b_desc + 2), "r"(a_tmem + 16), "l"(b_desc + 4),
                  "r"(a_tmem + 24), "l"(b_desc + 6), "r"(smem_u32(bar)), "h"((uint16_t)3) : "memory");
+}
+
+// one weight stage against three planes: the first into d0, the others into d1
+__device__ __forceinline__ void mma12_f16_commit_pair_elect(uint32_t d0, uint32_t a, uint64_t b0, uint32_t acc0, uint32_t d1, uint64_t b1, uint32_t acc1, uint64_t b2,
+                                                            uint32_t idesc, uint64_t *bar) {
+  asm volatile("{\n\t.reg .pred p, u, q, t;\n\tsetp.ne.b32 p, %3, 0;\n\tsetp.ne.b32 u, %6, 0;\n\tsetp.eq.u32 t, %8, %8;\n\telect.sync _|q, 0xFFFFFFFF;\n\t"
+               "@q tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %8, p;\n\t"
+               "@q tcgen05.mma.cta_group::2.kind::f16 [%0], [%9], %12, %8, t;\n\t"
+               "@q tcgen05.mma.cta_group::2.kind::f16 [%0], [%10], %13, %8, t;\n\t"
+               "@q tcgen05.mma.cta_group::2.kind::f16 [%0], [%11], %14, %8, t;\n\t"
+               "@q tcgen05.mma.cta_group::2.kind::f16 [%4], [%1], %5, %8, u;\n\t"
+               "@q tcgen05.mma.cta_group::2.kind::f16 [%4], [%9], %15, %8, t;\n\t"
+               "@q tcgen05.mma.cta_group::2.kind::f16 [%4], [%10], %16, %8, t;\n\t"
+               "@q tcgen05.mma.cta_group::2.kind::f16 [%4], [%11], %17, %8, t;\n\t"
+               "@q tcgen05.mma.cta_group::2.kind::f16 [%4], [%1], %7, %8, t;\n\t"
+               "@q tcgen05.mma.cta_group::2.kind::f16 [%4], [%9], %18, %8, t;\n\t"
+               "@q tcgen05.mma.cta_group::2.kind::f16 [%4], [%10], %19, %8, t;\n\t"
+               "@q tcgen05.mma.cta_group::2.kind::f16 [%4], [%11], %20, %8, t;\n\t"
+               "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%21], %22;\n\t}"
+               ::"r"(d0), "r"(a), "l"(b0), "r"(acc0), "r"(d1), "l"(b1), "r"(acc1), "l"(b2), "r"(idesc), "r"(a + 8), "r"(a + 16), "r"(a + 24), "l"(b0 + 2), "l"(b0 + 4),
+                 "l"(b0 + 6), "l"(b1 + 2), "l"(b1 + 4), "l"(b1 + 6), "l"(b2 + 2), "l"(b2 + 4), "l"(b2 + 6), "r"(smem_u32(bar)), "h"((uint16_t)3) : "memory");
 }
 
 // A tile of the schedule: 128-row tiles 2 * tm and 2 * tm + 1 (one per CTA of the pair) against the tokens [j0, j0 + width), of which
@@ -150,7 +193,7 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
   uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint8_t *const sB = smem, *const sRaw = sB + kB * C::kBBytes, *const staging = sRaw + kRaw * C::kRawBytes;
   uint4 *lut = (uint4 *)(staging + 4 * C::kStagingBytes);           // scale code -> bytes of the eight products (see e2m1_expand4)
-  float *colscale = (float *)(lut + 256);                           // RMSNorm column scales of the current token tile
+  float *colscale = (float *)(lut + (PLANES == 2 ? 512 : 256));                           // RMSNorm column scales of the current token tile
   uint64_t *bars = (uint64_t *)(colscale + 256);
   uint64_t *a_full = bars, *b_full = a_full + kA, *b_empty = b_full + kB, *a_empty = PLANES == 1 ? b_empty : b_empty + kB,
            *raw_full = b_empty + kB + kA, *raw_empty = raw_full + kRaw, *tmem_full = raw_empty + kRaw, *tmem_empty = tmem_full + 2;
@@ -161,6 +204,11 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int rank = (int)cluster_ctarank();
   const int gm = g.m, gn = g.n, gk = g.k, seg_stages = SEG ? g.seg_stages : 0;
+  const int unit = PLANES != 1 ? 1 : F16 ? g.unit : 2;   // stages per unit
+  const int lgA = PLANES != 1 ? (kA == 8 ? 3 : 2) : unit == 2 ? 2 : 3, lgB = unit == 2 || PLANES != 1 ? 2 : 3;   // the rings' slots, as powers of two
+  const int nA = 1 << lgA, nB = 1 << lgB, subA = kA >> lgA;
+  constexpr int kSub = PLANES == 3 ? C::kBBytes / 2 : C::kBBytes;   // bytes of a stage of one plane (three planes: tiles of at most 128 tokens)
+  const int slot_bytes = (kB * C::kBBytes) >> lgB;
   const int tiles_m = (gm + 255) / 256, nk = gk / 64, nslots = (nk + 3) / 4;   // 256-row tiles
   const int tile_first = blockIdx.x >> 1, tile_step = gridDim.x >> 1;
   const bool ue = g.A.ue != 0;
@@ -169,7 +217,7 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
   // The set-up touches no global memory: under programmatic dependent launch it runs while the stream's previous kernel drains.
   pdl_launch_dependents();
   if (threadIdx.x == 0) {
-    for (int s = 0; s < kA; ++s) mbar_init(&a_full[s], 8);   // the stage's four expansion warps of both CTAs
+    for (int s = 0; s < kA; ++s) mbar_init(&a_full[s], 8 * unit);   // the expansion warps of the unit's stages, in both CTAs
     if (PLANES != 1) for (int s = 0; s < kA; ++s) mbar_init(&a_empty[s], 1);
     for (int s = 0; s < kB; ++s) { mbar_init(&b_full[s], 1); mbar_init(&b_empty[s], 1); }
     for (int s = 0; s < kRaw; ++s) { mbar_init(&raw_full[s], 1); mbar_init(&raw_empty[s], 8); }
@@ -179,28 +227,37 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
     prefetch_tensormap(&tmap_w);
     prefetch_tensormap(&tmap_b);
   }
-  if (threadIdx.x < 256) {
-    const float sc = scale_to_f32((uint32_t)threadIdx.x, ue);
+  for (int i = threadIdx.x; i < (PLANES == 2 ? 512 : 256); i += kThreads) {   // (PLANES = 2: a table for FP16, then one for BF16)
+    const bool half = PLANES == 2 ? i < 256 : F16;
+    const float sc = scale_to_f32((uint32_t)i & 255u, ue);
     uint32_t hi[2] = {0, 0}, lo[2] = {0, 0};
 #pragma unroll
     for (int c = 0; c < 8; ++c) {
       const float v = __fmul_rn(e2m1_to_f32(c), sc);   // exact in 16 bits
-      const uint32_t h = F16 ? (uint32_t)__half_as_ushort(__float2half_rn(v)) : __float_as_uint(v) >> 16;
+      const uint32_t h = half ? (uint32_t)__half_as_ushort(__float2half_rn(v)) : __float_as_uint(v) >> 16;
       hi[c >> 2] |= (h >> 8) << (8 * (c & 3));
       lo[c >> 2] |= (h & 0xFFu) << (8 * (c & 3));
     }
-    lut[threadIdx.x] = make_uint4(hi[0], hi[1], lo[0], lo[1]);
+    lut[i] = make_uint4(hi[0], hi[1], lo[0], lo[1]);
   }
   if (warp == 1) tmem_alloc_pair(tmem_slot, 512);
   tc_fence_before();
   cluster_sync_all();   // the peer's barriers are initialised before anything arrives on them
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  // (all of the tensor memory is this CTA's, so that it begins at address 0; as a constant it leaves the MMA issuer's operands in uniform registers)
+  const uint32_t tmem_base = 0;
   pdl_wait();   // from here on the previous kernel has completed and its writes are visible
+  const float *tscale = nullptr;
+  bool wide = false;   // three BF16 planes instead of two FP16 ones (see the head of the file)
+  if constexpr (PLANES == 2) {
+    tscale = behind_wait(g.tscale);
+    wide = tscale[g.n] != 0.f;
+  }
+  const int planes = PLANES == 2 && wide ? 3 : PLANES, per_slot = PLANES == 3 ? 3 : 2;   // planes of an activation, planes in a ring slot
 
   const unsigned tag = g.tag;
   auto wait = [abort_flag, status_word, tag](uint64_t *bar, uint32_t parity, unsigned code) -> bool {
-    if (mbar_try(bar, parity)) return true;   // the common case: no flag read, no clock read
+    if (__builtin_expect(mbar_try(bar, parity), 1)) return true;   // the common case: no flag read, no clock read
     if (*abort_flag) return false;
     if (mbar_wait(bar, parity)) return true;
     *abort_flag = 1;
@@ -250,33 +307,39 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
   if (warp == 0) {
     // ---------------- producer: this CTA's half of the tile's tokens, one plane of one stage per slot ----------------
     // (the whole warp runs the loop, one elected lane issues: see tma_load_3d_pair_elect)
-    const uint32_t stage_bytes = 2u * (uint32_t)(W / 2) * 128u;   // a box is always W / 2 rows per CTA, however many of them the tile uses
+    const uint32_t sub_bytes = 2u * (uint32_t)(W / 2) * 128u;   // a box is always W / 2 rows per CTA, however many of them the tile uses
     uint32_t it = 0;
     for (int t = tile_first; t < ntiles; t += tile_step) {
       const Tile p = tile_of(t);
       if (p.width == 0) continue;
       const int row0 = p.j0 + rank * (p.width >> 1);
-      for (int ks = 0; ks < nk; ++ks) {
-#pragma unroll
-        for (int pl = 0; pl < PLANES; ++pl, ++it) {   // plane pl of a token's row starts 2 k bytes after plane pl - 1
-          const int s = it % kB;
-          if (!__all_sync(0xFFFFFFFFu, wait(&b_empty[s], ((it / kB) & 1) ^ 1, kStWaitEmpty))) goto done;
-          if (rank == 0) mbar_arrive_expect_tx_elect(&b_full[s], stage_bytes);
-          tma_load_3d_pair_elect(smem_u32(sB + (size_t)s * C::kBBytes), &tmap_b, pl * 2 * gk + ks * 128, row0, 0, mbar_addr_rank(&b_full[s], 0));
+#pragma unroll 1
+      for (int ks = 0; ks < nk; ks += unit) {
+#pragma unroll 1
+        for (int pl = 0; pl < planes; pl += per_slot, ++it) {   // a slot: two stages, or two or three planes of one (plane pl of a token's row starts 2 k bytes after plane pl - 1)
+          const int s = it & (nB - 1), nsub = PLANES == 1 ? min(unit, nk - ks) : min(per_slot, planes - pl);
+          if (!__all_sync(0xFFFFFFFFu, wait(&b_empty[s], (it >> lgB & 1) ^ 1, kStWaitEmpty))) goto done;
+          if (rank == 0) mbar_arrive_expect_tx_elect(&b_full[s], nsub * sub_bytes);
+          const uint32_t dst = smem_u32(sB) + (uint32_t)(s * slot_bytes), bar = mbar_addr_rank(&b_full[s], 0);
+          for (int i = 0; i < nsub; ++i)
+            tma_load_3d_pair_elect(dst + i * kSub, &tmap_b, PLANES == 1 ? (ks + i) * 128 : (pl + i) * 2 * gk + ks * 128, row0, 0, bar);
         }
       }
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer (even CTA) ----------------
-    // The whole warp runs the loop and one elected lane issues a stage's four MMAs and the commit in one statement; from inside a
-    // one-lane branch every tcgen05.mma costs ~150 cycles, more than the 128 the tensor pipe needs for 256 x 256 x 16 on a pair.
+    // The whole warp runs the loop and one elected lane issues; from inside a one-lane branch every tcgen05.mma costs ~150 cycles.  Alone, a pair
+    // takes 64 cycles for 256 x 128 x 16 and 128 for twice the tokens, but this warp shares its scheduler and its instruction cache with 18 others: with two
+    // waits, four MMAs and a commit per plane of a stage an MMA took about 180 cycles whatever the tile's width.  A unit of work is therefore two stages,
+    // or all planes of one, behind one wait for the weights and one for the activations, with one commit, in one statement, its operands in uniform
+    // registers: now 94 - 165 cycles for 128 tokens and 127 for 256.  With the planes above, 8 experts of 2048 x 4096 on 1100 tokens: 123 -> 96 us.
     if (rank == 0) {
       const uint64_t db0 = smem_desc_sw128(smem_u32(sB));
       uint32_t ia = 0, ib = 0, acc_i = 0;
       for (int t = tile_first; t < ntiles; t += tile_step) {
         const Tile p = tile_of(t);
         if (p.width == 0) continue;
-        const uint32_t idesc = idesc_f16(256, p.width, F16 ? 0 : 1);
+        const uint32_t idesc = idesc_f16(256, p.width, PLANES == 2 ? (wide ? 1 : 0) : F16 ? 0 : 1);
         for (int ks0 = 0; ks0 < nk; ks0 += SEG ? seg_stages : nk, ++acc_i) {
           const int acc = nacc == 2 ? acc_i & 1 : 0, ks1 = SEG ? min(ks0 + seg_stages, nk) : nk;
           const uint32_t acc_par = (nacc == 2 ? acc_i >> 1 : acc_i) & 1;
@@ -285,20 +348,34 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
           if (SEG && PLANES != 1 && ks0 == 0 && !__all_sync(0xFFFFFFFFu, wait(&tmem_empty[acc ^ 1], (((acc_i + 1) >> 1) & 1) ^ 1, kStWaitTmemEmpty))) goto done;
           tc_fence_after();
           const uint32_t d_tmem = tmem_base + acc * 128;
-          for (int ks = ks0; ks < ks1; ++ks, ++ia) {
-            const int sa = ia % kA;
-            if (!__all_sync(0xFFFFFFFFu, wait(&a_full[sa], (ia / kA) & 1, kStWaitFullA))) goto done;
-            const uint32_t a_tmem = tmem_base + kACols + sa * 32;
-#pragma unroll
-            for (int pl = 0; pl < PLANES; ++pl, ++ib) {
-              const int sb = ib % kB;
-              if (!__all_sync(0xFFFFFFFFu, wait(&b_full[sb], (ib / kB) & 1, kStWaitFullB))) goto done;
-              tc_fence_after();
-              const bool small = SEG && pl > 0;   // (summed over all of k, apart from the segments)
-              mma4_f16_commit_pair_elect(small ? tmem_base + kSmallCols : d_tmem, a_tmem, db0 + (uint32_t)sb * (uint32_t)(C::kBBytes >> 4), idesc,
-                                         (uint32_t)((small ? ks | (pl - 1) : (ks - ks0) | pl) != 0), &b_empty[sb]);
+#pragma unroll 1
+          for (int ks = ks0; ks < ks1; ks += unit, ++ia, ++ib) {
+            const int sa = ia & (nA - 1);
+            int sb = ib & (nB - 1);
+            if (!__all_sync(0xFFFFFFFFu, wait(&a_full[sa], ia >> lgA & 1, kStWaitFullA) && wait(&b_full[sb], ib >> lgB & 1, kStWaitFullB))) goto done;
+            tc_fence_after();
+            const uint32_t a_tmem = tmem_base + kACols + sa * subA * 32;
+            uint64_t db = db0 + (uint32_t)(sb * (slot_bytes >> 4));
+            if (PLANES == 1) {
+              if (ks + 1 < ks1 && unit == 2)
+                mma8_f16_commit_pair_elect(d_tmem, a_tmem, db, ks != ks0, d_tmem, a_tmem + 32, db + (kSub >> 4), 1, idesc, &b_empty[sb]);
+              else
+                mma4_f16_commit_pair_elect(d_tmem, a_tmem, db, idesc, ks != ks0, &b_empty[sb]);
+            } else if (PLANES == 3) {   // (the small planes are summed over all of k, apart from the segments)
+              mma12_f16_commit_pair_elect(d_tmem, a_tmem, db, ks != ks0, tmem_base + kSmallCols, db + (kSub >> 4), ks != 0, db + 2 * (kSub >> 4), idesc, &b_empty[sb]);
+              tc_commit_pair_elect(&a_empty[sa]);
+            } else {
+              mma8_f16_commit_pair_elect(d_tmem, a_tmem, db, ks != ks0, d_tmem, a_tmem, db + (kSub >> 4), 1, idesc, &b_empty[sb]);
+              if (wide) {
+                ++ib;
+                sb = ib & (nB - 1);
+                if (!__all_sync(0xFFFFFFFFu, wait(&b_full[sb], ib >> lgB & 1, kStWaitFullB))) goto done;
+                tc_fence_after();
+                db = db0 + (uint32_t)(sb * (slot_bytes >> 4));
+                mma4_f16_commit_pair_elect(d_tmem, a_tmem, db, idesc, 1, &b_empty[sb]);
+              }
+              tc_commit_pair_elect(&a_empty[sa]);
             }
-            if (PLANES != 1) tc_commit_pair_elect(&a_empty[sa]);
           }
           tc_commit_pair_elect(&tmem_full[acc]);
         }
@@ -313,6 +390,7 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
       const Tile p = tile_of(t);
       if (p.width == 0) continue;
       const int row_tile = 2 * p.tm + rank;
+#pragma unroll 1
       for (int sl = 0; sl < nslots; ++sl, ++it) {
         const int s = it % kRaw;
         if (!__all_sync(0xFFFFFFFFu, wait(&raw_empty[s], ((it / kRaw) & 1) ^ 1, kStWaitRaw))) goto done;
@@ -484,13 +562,18 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
         for (int gq = 0; gq < 4; ++gq) {
           float2 cs = make_float2(0.f, 0.f);
           if (mask & kExNorm) cs = *(const float2 *)&colscale[cc + 8 * gq + cp];
+          float ts[2] = {1.f, 1.f};
+          if constexpr (PLANES == 2) {   // (powers of two)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) ts[e] = tscale[min(j0 + 8 * gq + cp + e, gn - 1)];
+          }
 #pragma unroll
           for (int q = 0; q < 4; ++q)
 #pragma unroll
             for (int e = 0; e < 2; ++e) {
               uint32_t &x = r[16 * (q >> 1) + 4 * gq + 2 * (q & 1) + e];
               const float sc = (mask & kExNorm) ? __fmul_rn(__fmul_rn(rowp[q], __fmul_rn(gb0, e ? cs.y : cs.x)), g.e.gf) : rowp[q];
-              float v = __fmul_rn(__uint_as_float(x), sc);
+              float v = __fmul_rn(PLANES == 2 ? __fmul_rn(__uint_as_float(x), ts[e]) : __uint_as_float(x), sc);
               v = __fadd_rn(v, bias[q]);
               const int jj = 8 * gq + cp + e;
               if (EPI == kEpiAny && g.e.beta != 0.f && rb + 8 * q < gm && jj < nvalid)
@@ -629,6 +712,7 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
     const Fp4Operand A = g.A;
     const ScalePos sp{A.sld};
     const bool img = A.image, swz = A.sld < 0;
+    const uint4 *const table = lut + (wide ? 256 : 0);
     // scale words of this group's two stages of slot sl (stages past the end of k: zeros)
     auto fetch_scales = [&](const uint8_t *scp, int sl, uint32_t (&v)[2]) {
 #pragma unroll
@@ -638,15 +722,17 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
         v[h] = ks < nk ? *(const uint32_t *)(scp + off) : 0u;
       }
     };
-    uint32_t isl = 0, it0 = 0;   // slots so far; stages of the finished tiles
-    for (int t = tile_first; t < ntiles; t += tile_step, it0 += nk) {
+    const int tile_units = (nk + unit - 1) / unit;
+    uint32_t isl = 0, it0 = 0;   // slots so far; units of the finished tiles
+    for (int t = tile_first; t < ntiles; t += tile_step, it0 += tile_units) {
       const Tile p = tile_of(t);
-      if (p.width == 0) { it0 -= nk; continue; }
+      if (p.width == 0) { it0 -= tile_units; continue; }
       const int r = min((2 * p.tm + rank) * 128 + row, gm - 1);
       const uint8_t *scp = img ? A.data + (size_t)(r >> 7) * A.ktiles * kImgTileBytes + kImgDataBytes + (r & 31) * 16 + ((r & 127) >> 5) * 4
                                : A.sc + sp.row(p.ro + r);
       uint32_t sc[2], sc_next[2] = {0, 0};
       fetch_scales(scp, 0, sc);
+#pragma unroll 1
       for (int sl = 0; sl < nslots; ++sl, ++isl) {
         if (sl + 1 < nslots) fetch_scales(scp, sl + 1, sc_next);
         const int rs = isl % kRaw;
@@ -658,20 +744,24 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
           const int ks = 4 * sl + group + 2 * h;
-          if (ks >= nk) break;
-          const uint32_t it = it0 + ks;
-          const int s = it % kA;
+          if (ks >= nk && !(unit == 2 && ks == nk && (nk & 1))) break;
+          const uint32_t it = it0 + (unit == 2 ? ks >> 1 : ks);
+          const int s = it & (nA - 1);
           // (the vote also brings the warp together again: lanes whose first poll failed come later, and the stores below are warp-wide)
-          if (!__all_sync(0xFFFFFFFFu, wait(&a_empty[s], ((it / kA) & 1) ^ 1, kStWaitConv))) goto done;
+          if (!__all_sync(0xFFFFFFFFu, wait(&a_empty[s], (it >> lgA & 1) ^ 1, kStWaitConv))) goto done;
+          if (ks == nk) {   // an odd number of stages: the last unit has one
+            if (lane == 0) mbar_arrive_rank(&a_full[s], 0);
+            break;
+          }
           tc_fence_after();   // the MMAs of the stage's previous round have read it
-          const uint32_t dst = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + kACols + s * 32;
+          const uint32_t dst = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + kACols + (unit == 2 ? 2 * s + group : s) * 32;
 #pragma unroll
           for (int u = 0; u < 2; ++u) {   // 32 values: two blocks, 16 columns
             const uint32_t wv[4] = {w[2 * h + u].x, w[2 * h + u].y, w[2 * h + u].z, w[2 * h + u].w};
             uint32_t o[16];
 #pragma unroll
             for (int q = 0; q < 4; ++q) {  // 8 values per word
-              const uint4 t4 = lut[(sc[h] >> (16 * u + 8 * (q >> 1))) & 0xFF];
+              const uint4 t4 = table[(sc[h] >> (16 * u + 8 * (q >> 1))) & 0xFF];
               e2m1_expand4(wv[q], t4, o[4 * q], o[4 * q + 1]);
               e2m1_expand4(wv[q] >> 16, t4, o[4 * q + 2], o[4 * q + 3]);
             }
@@ -798,6 +888,7 @@ bool set_up(const GemmArgs &g, int planes, bool f16, int groups, const void *act
   const int rows256 = (g.m + 255) / 256, pairs = device_sms() / 2, widest = f16 || groups ? kSegmentWidth : 256;
   const Plan p = groups ? make_grouped_plan(rows256, g.n, groups, planes, pairs, widest) : make_plan(rows256, g.n, planes, pairs, widest);
   const uint64_t wrows = (uint64_t)g.m * (groups ? groups : 1);
+  a->unit = planes == 1 && !(f16 && g.k < 512) ? 2 : 1;
   a->seg_stages = g.k >= 1024 ? 4 : g.k >= 512 ? 2 : 1;   // (the longest that keep the sums no less exact than the CUDA-core kernels': see the head of the file)
   a->width = p.width; a->nfull = p.nfull; a->cut = p.cut; a->tiles = p.tiles;
   const uint64_t wtiles = (uint64_t)((g.m + 127) / 128) * g.A.ktiles;
@@ -814,32 +905,93 @@ bool set_up(const GemmArgs &g, int planes, bool f16, int groups, const void *act
   return true;
 }
 
-// INT8 activations q [n][ld] with one FP32 scale per 16 values -> three BF16 planes [n][3][k] with t1 + t2 + t3 = fl(q * s) exactly.
-// One thread per 8 values: 8 bytes in, three 16-byte stores out.
-__global__ void __launch_bounds__(256) w4a8_planes_kernel(const int8_t *__restrict__ q, int ld, const float *__restrict__ sc, int lds, int n, int k,
-                                                          uint16_t *__restrict__ planes) {
-  const long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x, per_row = k >> 3;
-  if (v >= per_row * n) return;
-  const int j = (int)(v / per_row), c = (int)(v - (long long)j * per_row);   // token, group of 8 values
-  const uint2 raw = *(const uint2 *)(q + (size_t)j * ld + 8 * c);
-  const float s = sc[(size_t)j * lds + (c >> 1)];
-  uint32_t t[3][4];
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const int qi = (int)(int8_t)(((i < 4 ? raw.x : raw.y) >> (8 * (i & 3))) & 0xFFu);
-    float r = __fmul_rn((float)qi, s);
-#pragma unroll
-    for (int p = 0; p < 3; ++p) {
-      const float tp = __bfloat162float(__float2bfloat16_rn(r));   // 8 significant bits, round to nearest even
-      const uint32_t h = __float_as_uint(tp) >> 16;
-      if (i & 1) t[p][i >> 1] |= h << 16;
-      else t[p][i >> 1] = h;
-      r = __fsub_rn(r, tp);   // exact: the remainder has at most 16, then 8 significant bits
-    }
+// INT8 activations q [n][ld] with one FP32 scale s per 16 values -> two FP16 planes [n][3][k] (the third is left alone): t1 + t2 is q * s * 2^(7 - E) to
+// within 2^-23 of itself or 2^-25, E the exponent of the token's largest scale; tscale[token] = 2^(E - 7).  A token whose scales two planes do not
+// take (see the head of the file) is marked in wide[token].  One CTA per token, a thread per 8 values: 8 bytes in, two 16-byte stores out.
+constexpr int kPlanesThreads = 256, kPlanesSpread = 12;
+__global__ void __launch_bounds__(kPlanesThreads) w4a8_planes_kernel(const int8_t *__restrict__ q, int ld, const float *__restrict__ sc, int lds, int k,
+                                                                     uint16_t *__restrict__ planes, float *__restrict__ tscale, uint8_t *__restrict__ wide) {
+  pdl_launch_dependents();
+  __shared__ uint32_t red[2][kPlanesThreads / 32];
+  const int j = blockIdx.x;
+  const float *const srow = sc + (size_t)j * lds;
+  uint32_t hi = 0, lo = 0xFFFFFFFFu;   // largest and smallest non-zero |s| (less one), as bits
+  for (int b = threadIdx.x; b < (k >> 4); b += kPlanesThreads) {
+    const uint32_t u = __float_as_uint(srow[b]) & 0x7FFFFFFFu;
+    hi = max(hi, u);
+    lo = min(lo, u - 1u);
   }
-  uint16_t *row = planes + (size_t)j * 3 * k + 8 * c;
+  hi = __reduce_max_sync(0xFFFFFFFFu, hi);
+  lo = __reduce_min_sync(0xFFFFFFFFu, lo);
+  if ((threadIdx.x & 31) == 0) { red[0][threadIdx.x >> 5] = hi; red[1][threadIdx.x >> 5] = lo; }
+  __syncthreads();
 #pragma unroll
-  for (int p = 0; p < 3; ++p) *(uint4 *)(row + (size_t)p * k) = make_uint4(t[p][0], t[p][1], t[p][2], t[p][3]);
+  for (int w = 0; w < kPlanesThreads / 32; ++w) { hi = max(hi, red[0][w]); lo = min(lo, red[1][w]); }
+  const int eh = hi ? (int)(hi >> 23) : 127, el = hi ? (int)((lo + 1u) >> 23) : 127;   // biased exponents (Inf, NaN: 255)
+  const bool narrow = eh >= 27 && eh <= 227 && eh - el <= kPlanesSpread;
+  if (threadIdx.x == 0) {
+    tscale[j] = __uint_as_float((uint32_t)(narrow ? eh - 7 : 127) << 23);
+    wide[j] = !narrow;
+  }
+  if (!narrow) return;
+  const float up = __uint_as_float((uint32_t)(261 - eh) << 23);   // 2^(7 - E), a normal number
+  for (int c = threadIdx.x; c < (k >> 3); c += kPlanesThreads) {
+    const uint2 raw = *(const uint2 *)(q + (size_t)j * ld + 8 * c);
+    const float s = __fmul_rn(srow[c >> 1], up);   // exact
+    uint32_t t[2][4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      float v[2];
+#pragma unroll
+      for (int e = 0; e < 2; ++e) v[e] = (float)(int)(int8_t)(((i < 2 ? raw.x : raw.y) >> (16 * (i & 1) + 8 * e)) & 0xFFu);
+      const __half2 t1 = __floats2half2_rn(__fmul_rn(v[0], s), __fmul_rn(v[1], s));
+      const float2 f1 = __half22float2(t1);
+      const __half2 t2 = __floats2half2_rn(__fmaf_rn(v[0], s, -f1.x), __fmaf_rn(v[1], s, -f1.y));   // (the remainders are exact)
+      t[0][i] = *reinterpret_cast<const uint32_t *>(&t1);
+      t[1][i] = *reinterpret_cast<const uint32_t *>(&t2);
+    }
+    uint16_t *const row = planes + (size_t)j * 3 * k + 8 * c;
+#pragma unroll
+    for (int p = 0; p < 2; ++p) *(uint4 *)(row + (size_t)p * k) = make_uint4(t[p][0], t[p][1], t[p][2], t[p][3]);
+  }
+}
+
+// Runs behind it: tells the GEMM which planes there are (tscale[n]), and if some token is wide (or all count as such: `force`) writes three BF16
+// planes [n][3][k] of every token instead, t1 + t2 + t3 = fl(q * s) exactly, tscale 1.
+__global__ void __launch_bounds__(256) w4a8_wide_planes_kernel(const int8_t *q, int ld, const float *sc, int lds, int n, int k, uint16_t *planes, float *tscale,
+                                                               const uint8_t *wide_in, int force) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const uint8_t *const wide = behind_wait(wide_in);
+  int any = force;
+  for (int j = threadIdx.x; j < n && !force; j += blockDim.x) any |= wide[j];
+  any = __syncthreads_or(any);
+  if (blockIdx.x == 0 && threadIdx.x == 0) tscale[n] = any ? 1.f : 0.f;
+  if (!any) return;
+  const long long per_row = k >> 3;
+  for (long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x; v < per_row * n; v += (long long)gridDim.x * blockDim.x) {
+    const int j = (int)(v / per_row), c = (int)(v - (long long)j * per_row);   // token, group of 8 values
+    if (c == 0) tscale[j] = 1.f;
+    const uint2 raw = *(const uint2 *)(q + (size_t)j * ld + 8 * c);
+    const float s = sc[(size_t)j * lds + (c >> 1)];
+    uint32_t t[3][4];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int qi = (int)(int8_t)(((i < 4 ? raw.x : raw.y) >> (8 * (i & 3))) & 0xFFu);
+      float r = __fmul_rn((float)qi, s);
+#pragma unroll
+      for (int p = 0; p < 3; ++p) {
+        const float tp = __bfloat162float(__float2bfloat16_rn(r));   // 8 significant bits, round to nearest even
+        const uint32_t h = __float_as_uint(tp) >> 16;
+        if (i & 1) t[p][i >> 1] |= h << 16;
+        else t[p][i >> 1] = h;
+        r = __fsub_rn(r, tp);   // exact: the remainder has at most 16, then 8 significant bits
+      }
+    }
+    uint16_t *row = planes + (size_t)j * 3 * k + 8 * c;
+#pragma unroll
+    for (int p = 0; p < 3; ++p) *(uint4 *)(row + (size_t)p * k) = make_uint4(t[p][0], t[p][1], t[p][2], t[p][3]);
+  }
 }
 
 }  // namespace
@@ -909,7 +1061,7 @@ bool gemm_w4a8_tc_supports(const GemmArgs &g) {
 
 // The same for nvfp4a_gemm_grouped: problems whose D is 16-bit (an FP32 D keeps the exact block sums of the DP4A kernel) and whose reduction
 // is long enough to pay for the planes and for segments no less exact than the DP4A kernel's ordered sums (see the head of the file).  8
-// experts of 2048 x 4096 on 1100 tokens, INT8 quantization of the tokens included: 602 us on the DP4A kernel, 132 us here.
+// experts of 2048 x 4096 on 1100 tokens, INT8 quantization of the tokens included: 602 us on the DP4A kernel, 96 us here.
 bool gemm_w4a8_grouped_supports(const GemmArgs &g, int groups) {
   return gemm_w4a8_tc_supports(g) && !g.A.image && groups <= kMaxGroups && g.k >= 512 && g.e.d_dtype != NVFP4A_FP32;
 }
@@ -920,21 +1072,40 @@ cudaError_t launch_gemm_w4a8_tc(const GemmArgs &g, const int *seg, int groups, c
   cudaMemPool_t pool;
   cudaError_t e = planes_pool(&pool);
   if (e != cudaSuccess) return e;
-  e = cudaMallocFromPoolAsync((void **)&planes, (size_t)g.n * 3 * g.k * sizeof(uint16_t), pool, s);
+  // planes [n][3][k], n token scales and the word behind them, n marks
+  const size_t plane_bytes = (size_t)g.n * 3 * g.k * sizeof(uint16_t);
+  e = cudaMallocFromPoolAsync((void **)&planes, plane_bytes + (size_t)(g.n + 1) * sizeof(float) + g.n, pool, s);
   if (e != cudaSuccess) return e;
-  const long long vecs = (long long)g.n * (g.k >> 3);
-  w4a8_planes_kernel<<<(unsigned)((vecs + 255) / 256), 256, 0, s>>>((const int8_t *)g.B.data, g.B.ld, g.B.s8, g.B.lds8, g.n, g.k, planes);
-  e = cudaGetLastError();
+  float *const tscale = (float *)((uint8_t *)planes + plane_bytes);
+  uint8_t *const wide = (uint8_t *)(tscale + g.n + 1);
+  const bool force = seg || g.A.ue;   // three planes whatever the scales: groups (see Segments), and UE5M3 weights, whose products leave FP16's range
+  if (!force) {
+    w4a8_planes_kernel<<<(unsigned)g.n, kPlanesThreads, 0, s>>>((const int8_t *)g.B.data, g.B.ld, g.B.s8, g.B.lds8, g.k, planes, tscale, wide);
+    e = cudaGetLastError();
+  }
+  if (e == cudaSuccess) {
+    cudaLaunchConfig_t cfg;
+    memset(&cfg, 0, sizeof cfg);
+    cfg.gridDim = dim3(force ? (unsigned)(((long long)g.n * (g.k >> 3) + 255) / 256) : (unsigned)device_sms(), 1, 1);
+    cfg.blockDim = dim3(256, 1, 1);
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr; cfg.numAttrs = pdl_enabled() && !force ? 1 : 0;   // (`force`: what it overwrites may still be in use by the kernel before)
+    e = cudaLaunchKernelEx(&cfg, w4a8_wide_planes_kernel, (const int8_t *)g.B.data, g.B.ld, g.B.s8, g.B.lds8, g.n, g.k, planes, tscale, (const uint8_t *)wide, force ? 1 : 0);
+  }
   if (e == cudaSuccess) {
     W4A16Args a;
     CUtensorMap tw, tb, td;
     PeerMaps pm;
     memset(&pm, 0, sizeof pm);
-    if (!set_up(g, 3, false, seg ? groups : 0, planes, (uint64_t)g.k * 6, (uint64_t)g.k * 6, &a, &tw, &tb, &td)) e = cudaErrorInvalidValue;
-    else if (seg) {
+    if (!set_up(g, seg ? 3 : 2, false, seg ? groups : 0, planes, (uint64_t)g.k * 6, (uint64_t)g.k * 6, &a, &tw, &tb, &td)) e = cudaErrorInvalidValue;
+    else {
+      a.tscale = tscale;
       a.seg = seg; a.groups = groups;
-      e = launch_cfg<3, false, true>(tw, tb, td, pm, a, s);
-    } else e = launch_cfg<3, false>(tw, tb, td, pm, a, s);
+      e = seg ? launch_cfg<3, false, true>(tw, tb, td, pm, a, s) : launch_cfg<2, false>(tw, tb, td, pm, a, s);
+    }
   }
   const cudaError_t ef = cudaFreeAsync(planes, s);
   return e != cudaSuccess ? e : ef;

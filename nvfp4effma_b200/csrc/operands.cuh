@@ -81,7 +81,7 @@ bool gemm_dp4a_supports(const GemmArgs &g);
 cudaError_t launch_gemm_w4a16(const GemmArgs &g, cudaStream_t s);    // tcgen05 kind::f16 with weights expanded to 16-bit values in tensor memory
 bool gemm_w4a16_supports(const GemmArgs &g);
 bool gemm_w4a16_pushes(const GemmArgs &g);
-cudaError_t launch_gemm_w4a8_tc(const GemmArgs &g, const int *seg, int groups, cudaStream_t s);  // INT8 activations as three BF16 planes on the same tcgen05 kernel
+cudaError_t launch_gemm_w4a8_tc(const GemmArgs &g, const int *seg, int groups, cudaStream_t s);  // INT8 activations as two FP16 or three BF16 planes on the same tcgen05 kernel
 bool gemm_w4a8_tc_supports(const GemmArgs &g);
 bool gemm_w4a8_grouped_supports(const GemmArgs &g, int groups);
 cudaError_t trim_planes_pool();   // gives the W4A8 planes' pool memory of the current device back to the system

@@ -948,6 +948,74 @@ def test_w4a16_gemm_decodes_signed_block_scales(bt):
         check_bound(c, h, got, amax, exp)
 
 
+@pytest.mark.parametrize("spread,exponent", [(0, 0), (11, 0), (12, 0), (13, 0), (40, 0), (5, 100), (5, 101), (5, -94), (5, -102)])
+@pytest.mark.parametrize("grouped", [False, True])
+def test_w4a8_planes_at_the_edges_of_their_range(grouped, spread, exponent):
+    """INT8 activations are two FP16 planes while a token's scales lie within 2^12 of each other (and near enough to one for the planes' scale to be a
+    float), else three BF16 planes for every token: scales 2^spread apart around a power of two, q = -128 .. 127, a token of zeros, one whose large
+    blocks meet zero weights only, negative scales.  Against 64 bits: (k + 2) 2^-24 of the sum of the terms' magnitudes (the FP32 accumulation bound)
+    and half a unit of the 16-bit result."""
+    m, n, k = 256, 96, 512
+    gen = torch.Generator(device="cuda").manual_seed(100 + spread)
+    ints = lambda lo, hi, shape, t: torch.randint(lo, hi, shape, generator=gen, device="cuda", dtype=t)
+    w, ws = ints(0, 16, (m, k), torch.uint8), ints(0x28, 0x48, (m, k // 16), torch.uint8)
+    w[:, :32] = 0
+    x = ints(-128, 128, (n, k), torch.int8)
+    s = (1.0 + torch.rand(n, k // 16, generator=gen, device="cuda", dtype=torch.float64) * (1 - 2.0 ** -23)).float()
+    s[:, 1] = 2.0 - 2.0 ** -23
+    x[:, 16] = -128
+    s = (s.double() * 2.0 ** (exponent - spread * ints(0, 2, (n, k // 16), torch.int32).double())).float()
+    s[:, 5] *= -1.0
+    s[3] = 0.0
+    s[4] *= 2.0 ** -9
+    s[4, :2] = 2.0 ** exponent        # meets zero weights
+    W = torch.tensor([0.0, 0.5, 1.0, 1.5, 2.0, 3.0, 4.0, 6.0], dtype=torch.float64, device="cuda")[(w & 7).long()] * (1.0 - 2.0 * (w >> 3).double())
+    W = (W.view(m, k // 16, 16) * ws.view(torch.float8_e4m3fn).double().unsqueeze(-1)).view(m, k)
+    packed = (w[:, 0::2] | (w[:, 1::2] << 4)).contiguous()
+    X = (x.double().view(n, k // 16, 16) * s.double().unsqueeze(-1)).view(n, k)
+    alpha = 2.0 ** -exponent   # the results near one
+    D = torch.zeros(n, m, dtype=torch.bfloat16, device="cuda")
+    ta, tb, td = tensor(packed, L.NVFP4, ws, k // 16), tensor(x, L.INT8, s, k // 16), tensor(D, L.BF16)
+    if grouped:
+        seg = torch.tensor([0, 40, n], dtype=torch.int32, device="cuda")
+        packed2, ws2 = torch.cat([packed, packed]), torch.cat([ws, ws])
+        ta = tensor(packed2, L.NVFP4, ws2, k // 16)
+        L.check(L.lib.nvfp4a_gemm_grouped(2, m, k, n, alpha, ctypes.byref(ta), k, ctypes.byref(tb), k, 0.0, None, 0, ctypes.byref(td), m, None,
+                                          ctypes.c_void_p(seg.data_ptr()), stream()))
+    else:
+        L.check(L.lib.nvfp4a_gemm(m, n, k, alpha, ctypes.byref(ta), k, ctypes.byref(tb), k, 0.0, None, 0, ctypes.byref(td), m, None, stream()))
+    assert L.lib.nvfp4a_b200_last_route() == 8
+    want, size = X @ W.t() * alpha, X.abs() @ W.abs().t() * alpha
+    assert bool(((D.double() - want).abs() <= (k + 2) * 2.0 ** -24 * size + 2.0 ** -8 * want.abs()).all())
+    assert kernel_status() == 0
+
+
+def test_w4a8_planes_with_ue5m3_weight_scales():
+    """Products with UE5M3 scales do not fit FP16: three BF16 planes."""
+    c = Case(256, 96, 512, L.INT8, L.FP32, -1, L.BF16, 1.25, 0.0, fa=UE)
+    h = build_case(c, 4395)
+    exp = oracle_case(c, h, want_ref=True)
+    got, amax = run_gemm(c, h)
+    assert L.lib.nvfp4a_b200_last_route() == 8
+    check_bound(c, h, got, amax, exp)
+    assert kernel_status() == 0
+
+
+@pytest.mark.parametrize("bt", [L.BF16, L.FP16, L.INT8])
+def test_w4a16_units_of_two_stages_at_the_ends_of_k(bt):
+    """The tcgen05 kernel works in units of eight MMAs: two stages of 64 values of k (one where FP16 sums segments of 64), or two planes of one stage.  Odd
+    numbers of stages, a single one, segments that end in half a unit; one tile and several per CTA pair."""
+    for i, k in enumerate([64, 128, 192, 448, 512, 576, 960, 1088, 1344]):
+        for m, n in [(300, 70), (130, 700)] + ([(4500, 1100)] if k in (192, 576) else []):
+            c = Case(m, n, k, bt, L.FP16 if i % 2 else L.BF16, -1, L.BF16 if i % 3 == 1 else -1, 1.25, 0.0, fa=SW if i % 2 else 0)
+            h = build_case(c, 4800 + i)
+            exp = oracle_case(c, h, want_ref=True)
+            got, amax = run_gemm(c, h)
+            assert L.lib.nvfp4a_b200_last_route() == (8 if bt == L.INT8 else 5), c
+            check_bound(c, h, got, amax, exp)
+    assert kernel_status() == 0
+
+
 @pytest.mark.parametrize("bt", [L.BF16, L.FP16, L.INT8])
 @pytest.mark.parametrize("case", ["plain", "bias", "swiglu", "grouped"])
 def test_w4a16_epilogues_compiled_for_plain_calls_equal_the_general_one(bt, case):
