@@ -96,7 +96,7 @@ struct alignas(64) PeerMaps {
 template <int PLANES, bool GROUPED>
 struct Cfg {
   // PLANES = 1: the weight and the activation ring advance together and share their `empty` barriers (one commit per stage)
-  static constexpr int kA = GROUPED ? 4 : 8, kB = 8, kRaw = 3;
+  static constexpr int kA = PLANES == 3 ? 4 : 8, kB = 8, kRaw = 3;
   static constexpr int kACols = 512 - 32 * kA;   // first tensor memory column of the weight stages (32 columns each)
   static constexpr int kBBytes = 128 * 128, kRawBytes = 128 * 128, kStagingBytes = 8192;
   static constexpr int kSmemBytes = 1024 + kB * kBBytes + kRaw * kRawBytes + 4 * kStagingBytes + (PLANES == 2 ? 8192 : 4096) /* expansion tables */ + 256 * 4 /* column scales */ +
@@ -187,7 +187,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_b, const __grid_constant__ CUtensorMap tmap_d,
                   const __grid_constant__ PeerMaps peers, const W4A16Args g) {
   using C = Cfg<PLANES, GROUPED>;
-  constexpr bool SEG = F16 || GROUPED;   // k is summed in segments: see the head of the file
+  constexpr bool SEG = F16 || PLANES == 3;   // k is summed in segments: see the head of the file
   constexpr int kA = C::kA, kB = C::kB, kRaw = C::kRaw, kACols = C::kACols, kSmallCols = 256;
   extern __shared__ uint8_t smem_raw[];
   uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -885,7 +885,7 @@ bool set_up(const GemmArgs &g, int planes, bool f16, int groups, const void *act
   a->e = g.e; a->x = g.x;
   a->status = kernel_status_device_ptr();
   a->tag = next_launch_tag();
-  const int rows256 = (g.m + 255) / 256, pairs = device_sms() / 2, widest = f16 || groups ? kSegmentWidth : 256;
+  const int rows256 = (g.m + 255) / 256, pairs = device_sms() / 2, widest = f16 || planes == 3 ? kSegmentWidth : 256;
   const Plan p = groups ? make_grouped_plan(rows256, g.n, groups, planes, pairs, widest) : make_plan(rows256, g.n, planes, pairs, widest);
   const uint64_t wrows = (uint64_t)g.m * (groups ? groups : 1);
   a->unit = planes == 1 && !(f16 && g.k < 512) ? 2 : 1;
@@ -1050,10 +1050,15 @@ cudaError_t trim_planes_pool() {
   return p ? cudaMemPoolTrimTo(p, 0) : cudaSuccess;
 }
 
-// W4A8 on the tensor cores (see the header): from 64 tokens and 128 weight rows up, where the planes' set-up pays.  The call
+// W4A8 on the tensor cores (see the header): from 64 tokens and 128 weight rows up, where the planes' set-up pays whatever the rest.  The call
 // takes the planes from the pool above (stream-ordered: capturable, no synchronisation) and gives them back after the GEMM.
+// Fewer tokens came from the DP4A kernel, whose ordered sums are more exact than one chain: they are summed in segments (three planes, a 16-bit D, the
+// plain epilogue), and only where the reduction is long enough for that and for the planes to pay: 835 x 2176 on 30 tokens 158 us there, 30 here,
+// 640 x 3840 on 10 tokens 267 and 41, 1024 x 512 on 32 tokens 49 and 17.
+constexpr int kW4A8ChainMinN = 64;
 bool gemm_w4a8_tc_supports(const GemmArgs &g) {
-  if (g.B.dtype != NVFP4A_INT8 || g.k < 64 || g.n < 64 || g.m < 128 || g.no_alloc || g.tp.world > 1 || g.e.gb_stride) return false;
+  if (g.B.dtype != NVFP4A_INT8 || g.k < 64 || g.m < 128 || g.no_alloc || g.tp.world > 1 || g.e.gb_stride) return false;
+  if (g.n < kW4A8ChainMinN && (g.n <= 8 || g.k < 512 || g.e.d_dtype == NVFP4A_FP32 || g.x.mask || g.A.ue)) return false;
   if (((uintptr_t)g.B.data & 7) || g.B.ld % 8 || !g.B.s8 || ((uintptr_t)g.B.s8 & 3)) return false;
   if (!g.A.image && (((uintptr_t)g.A.data & 15) || g.A.ld % 32 || ((uintptr_t)g.A.sc & 1))) return false;
   return true;
@@ -1063,7 +1068,7 @@ bool gemm_w4a8_tc_supports(const GemmArgs &g) {
 // is long enough to pay for the planes and for segments no less exact than the DP4A kernel's ordered sums (see the head of the file).  8
 // experts of 2048 x 4096 on 1100 tokens, INT8 quantization of the tokens included: 602 us on the DP4A kernel, 96 us here.
 bool gemm_w4a8_grouped_supports(const GemmArgs &g, int groups) {
-  return gemm_w4a8_tc_supports(g) && !g.A.image && groups <= kMaxGroups && g.k >= 512 && g.e.d_dtype != NVFP4A_FP32;
+  return g.n >= kW4A8ChainMinN && gemm_w4a8_tc_supports(g) && !g.A.image && groups <= kMaxGroups && g.k >= 512 && g.e.d_dtype != NVFP4A_FP32;
 }
 
 // seg == NULL: one weight; else `groups` stacked weights of g.m rows
@@ -1078,7 +1083,8 @@ cudaError_t launch_gemm_w4a8_tc(const GemmArgs &g, const int *seg, int groups, c
   if (e != cudaSuccess) return e;
   float *const tscale = (float *)((uint8_t *)planes + plane_bytes);
   uint8_t *const wide = (uint8_t *)(tscale + g.n + 1);
-  const bool force = seg || g.A.ue;   // three planes whatever the scales: groups (see Segments), and UE5M3 weights, whose products leave FP16's range
+  const bool three = seg || g.n < kW4A8ChainMinN;   // in segments
+  const bool force = three || g.A.ue;   // three planes whatever the scales (products with UE5M3 scales leave FP16's range)
   if (!force) {
     w4a8_planes_kernel<<<(unsigned)g.n, kPlanesThreads, 0, s>>>((const int8_t *)g.B.data, g.B.ld, g.B.s8, g.B.lds8, g.k, planes, tscale, wide);
     e = cudaGetLastError();
@@ -1100,11 +1106,11 @@ cudaError_t launch_gemm_w4a8_tc(const GemmArgs &g, const int *seg, int groups, c
     CUtensorMap tw, tb, td;
     PeerMaps pm;
     memset(&pm, 0, sizeof pm);
-    if (!set_up(g, seg ? 3 : 2, false, seg ? groups : 0, planes, (uint64_t)g.k * 6, (uint64_t)g.k * 6, &a, &tw, &tb, &td)) e = cudaErrorInvalidValue;
+    if (!set_up(g, three ? 3 : 2, false, seg ? groups : 0, planes, (uint64_t)g.k * 6, (uint64_t)g.k * 6, &a, &tw, &tb, &td)) e = cudaErrorInvalidValue;
     else {
       a.tscale = tscale;
       a.seg = seg; a.groups = groups;
-      e = seg ? launch_cfg<3, false, true>(tw, tb, td, pm, a, s) : launch_cfg<2, false>(tw, tb, td, pm, a, s);
+      e = seg ? launch_cfg<3, false, true>(tw, tb, td, pm, a, s) : three ? launch_cfg<3, false>(tw, tb, td, pm, a, s) : launch_cfg<2, false>(tw, tb, td, pm, a, s);
     }
   }
   const cudaError_t ef = cudaFreeAsync(planes, s);

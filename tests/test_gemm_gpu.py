@@ -1061,3 +1061,32 @@ def test_w4a16_epilogues_compiled_for_plain_calls_equal_the_general_one(bt, case
                 outs.append(D.view(torch.int16))
             assert bool(outs[0].any()) and torch.equal(outs[0], outs[1])
     assert kernel_status() == 0
+
+
+@pytest.mark.parametrize("k", [512, 576, 1088, 4096])
+def test_w4a8_of_9_to_63_tokens_is_summed_in_segments(k):
+    """INT8 activations of fewer than 64 tokens (k >= 512, 16-bit D, plain epilogue): the tcgen05 kernel in segments (route 8), within the bound; sums of
+    positive terms as close to 64 bits as test_long_sums_on_the_tensor_cores_are_joined_in_fp32 asks.  Plain operands and images."""
+    for i, (m, n) in enumerate([(128, 9), (300, 33), (515, 63), (130, 16)]):
+        c = Case(m, n, k, L.INT8, L.FP16 if i % 2 else L.BF16, -1, L.BF16 if i % 2 else -1, 1.25, 0.0, fa=SW if i == 1 else 0)
+        h = build_case(c, 4900 + i)
+        exp = oracle_case(c, h, want_ref=True)
+        for run in (run_gemm, lambda c, h: run_tc(c, h, gemv=False)):
+            got, amax = run(c, h)
+            assert L.lib.nvfp4a_b200_last_route() == 8, c
+            check_bound(c, h, got, amax, exp)
+    m, n = 300, 40
+    gen = torch.Generator(device="cuda").manual_seed(k)
+    w = torch.randint(1, 8, (m, k), generator=gen, device="cuda", dtype=torch.uint8)
+    ws = torch.randint(0x28, 0x48, (m, k // 16), generator=gen, device="cuda", dtype=torch.uint8)
+    W = torch.tensor([0.0, 0.5, 1.0, 1.5, 2.0, 3.0, 4.0, 6.0], dtype=torch.float64, device="cuda")[w.long()]
+    W = (W.view(m, k // 16, 16) * ws.view(torch.float8_e4m3fn).double().unsqueeze(-1)).view(m, k)
+    packed, D, amax = (w[:, 0::2] | (w[:, 1::2] << 4)).contiguous(), torch.zeros(n, m, dtype=torch.bfloat16, device="cuda"), torch.zeros(1, device="cuda")
+    x, xs = torch.randint(1, 128, (n, k), generator=gen, device="cuda", dtype=torch.int8), torch.rand(n, k // 16, generator=gen, device="cuda") + 0.01
+    ta, tb, td = tensor(packed, L.NVFP4, ws, k // 16), tensor(x, L.INT8, xs, k // 16), tensor(D, L.BF16, amax=amax)
+    L.check(L.lib.nvfp4a_gemm(m, n, k, 1.0, ctypes.byref(ta), k, ctypes.byref(tb), k, 0.0, None, 0, ctypes.byref(td), m, None, stream()))
+    assert L.lib.nvfp4a_b200_last_route() == 8
+    want = (x.double().view(n, k // 16, 16) * xs.double().unsqueeze(-1)).view(n, k) @ W.t()
+    assert abs(float(amax.double()) / float(want.max()) - 1.0) <= (16 + 16 + 4) * 2.0 ** -24
+    assert torch.allclose(D.double(), want, rtol=2.0 ** -8, atol=0.0)
+    assert kernel_status() == 0
