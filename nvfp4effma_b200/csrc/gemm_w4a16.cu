@@ -21,7 +21,7 @@
 //               each: the accumulator block goes into registers at once and back to the MMA warp before any arithmetic; then
 //               plain or extended epilogue (RMSNorm column scale, SwiGLU, second output + sums of squares), D through
 //               shared-memory staging tiles and TMA stores when its layout allows
-//   warps 12-19 weight expansion, two groups of four warps on alternate stages.  The eight magnitudes of E2M1 times a block scale
+//   warps 12-19 weight expansion, two groups of four warps on alternate pairs of stages.  The eight magnitudes of E2M1 times a block scale
 //               are eight 16-bit floats (exact: 2 x 4 significant bits); a 4 KiB table holds their high and low bytes for each of
 //               the 256 scale codes, so a block costs one 16-byte table read and four values cost three byte permutes (the packed
 //               nibbles ARE the permute's selectors: high bytes, low bytes, signs), two of them again to interleave, and two
@@ -43,7 +43,7 @@
 // not matter, have an accumulator of their own for all of k.  Error: 1.05e-7 and 9.8e-8 at k = 4096 (normal data; 2.9e-7 and 1.4e-7 against
 // 6.9e-7 and 2.9e-7 with activations spread over ten binades).  Below k = 1024 segments are 2 stages, below 512 one (INT8 at k = 512:
 // 6.2e-8 against 1.08e-7; FP16 at k = 512, 128 and 64: 6.3e-8, 4.2e-8 and 4.0e-8 against 6.9e-8, 4.1e-8 and 3.7e-8).
-// 8 experts of 2048 x 4096 on 1100 tokens take 96 us, FP16 4096 x 4096 on 333 tokens 35; the CUDA-core kernels 602 and 1932 us.
+// 8 experts of 2048 x 4096 on 1100 tokens take 94 us, FP16 4096 x 4096 on 333 tokens 31; the CUDA-core kernels 602 and 1932 us.
 //
 // Grouped (mixture of experts): A stacks the weights of all groups, a group owns the tokens [seg[q], seg[q + 1]); the CTAs read seg
 // (device memory) into a table of tile counts and find a tile's group there.  (INT8 activations only, plain epilogue, 16-bit D.)
@@ -217,7 +217,7 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
   // The set-up touches no global memory: under programmatic dependent launch it runs while the stream's previous kernel drains.
   pdl_launch_dependents();
   if (threadIdx.x == 0) {
-    for (int s = 0; s < kA; ++s) mbar_init(&a_full[s], 8 * unit);   // the expansion warps of the unit's stages, in both CTAs
+    for (int s = 0; s < kA; ++s) mbar_init(&a_full[s], 8);   // the unit's four expansion warps of both CTAs
     if (PLANES != 1) for (int s = 0; s < kA; ++s) mbar_init(&a_empty[s], 1);
     for (int s = 0; s < kB; ++s) { mbar_init(&b_full[s], 1); mbar_init(&b_empty[s], 1); }
     for (int s = 0; s < kRaw; ++s) { mbar_init(&raw_full[s], 1); mbar_init(&raw_empty[s], 8); }
@@ -704,7 +704,8 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
   } else {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsConv));
     // ---------------- weight expansion: NVFP4 -> 16-bit floats in tensor memory ----------------
-    // Two groups of four warps take the even and the odd stages of a tile; inside a group thread r owns row r of the CTA's 128 (and
+    // Two groups of four warps take the even and the odd pairs of stages of a tile (a slot's halves; on alternate stages every wait and hand-over came
+    // twice as often: 28672 x 4096 with SwiGLU on 2048 tokens 340 us instead of 318, FP16 4096 x 4096 on 333 tokens 34.3 instead of 31.2); inside a group thread r owns row r of the CTA's 128 (and
     // tensor memory lane r: warp % 4 is its quadrant): a stage's 64 nibbles are two 16-byte words of the slot's swizzled row, its 4 scale bytes one word fetched a slot (four stages)
     // ahead.
     const int cwarp = warp - 12, group = cwarp >> 2;
@@ -717,7 +718,7 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
     auto fetch_scales = [&](const uint8_t *scp, int sl, uint32_t (&v)[2]) {
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
-        const int ks = 4 * sl + group + 2 * h;
+        const int ks = 4 * sl + 2 * group + h;
         const size_t off = img ? (size_t)sl * kImgTileBytes + (ks & 3) * 512 : swz ? (size_t)ks * 512 : (size_t)ks * 4;
         v[h] = ks < nk ? *(const uint32_t *)(scp + off) : 0u;
       }
@@ -740,21 +741,17 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
         const uint8_t *src = sRaw + (size_t)rs * C::kRawBytes + row * 128;
         uint4 w[4];
 #pragma unroll
-        for (int q = 0; q < 4; ++q) w[q] = *(const uint4 *)(src + (((2 * group + 4 * (q >> 1) + (q & 1)) ^ r7) << 4));
+        for (int q = 0; q < 4; ++q) w[q] = *(const uint4 *)(src + (((4 * group + q) ^ r7) << 4));
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
-          const int ks = 4 * sl + group + 2 * h;
-          if (ks >= nk && !(unit == 2 && ks == nk && (nk & 1))) break;
+          const int ks = 4 * sl + 2 * group + h;
+          if (ks >= nk) break;
           const uint32_t it = it0 + (unit == 2 ? ks >> 1 : ks);
           const int s = it & (nA - 1);
           // (the vote also brings the warp together again: lanes whose first poll failed come later, and the stores below are warp-wide)
-          if (!__all_sync(0xFFFFFFFFu, wait(&a_empty[s], (it >> lgA & 1) ^ 1, kStWaitConv))) goto done;
-          if (ks == nk) {   // an odd number of stages: the last unit has one
-            if (lane == 0) mbar_arrive_rank(&a_full[s], 0);
-            break;
-          }
+          if ((h == 0 || unit == 1) && !__all_sync(0xFFFFFFFFu, wait(&a_empty[s], (it >> lgA & 1) ^ 1, kStWaitConv))) goto done;
           tc_fence_after();   // the MMAs of the stage's previous round have read it
-          const uint32_t dst = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + kACols + (unit == 2 ? 2 * s + group : s) * 32;
+          const uint32_t dst = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + kACols + (unit == 2 ? 2 * s + h : s) * 32;
 #pragma unroll
           for (int u = 0; u < 2; ++u) {   // 32 values: two blocks, 16 columns
             const uint32_t wv[4] = {w[2 * h + u].x, w[2 * h + u].y, w[2 * h + u].z, w[2 * h + u].w};
@@ -767,6 +764,7 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
             }
             tmem_st16(dst + 16 * u, o);
           }
+          if (unit == 2 && h == 0 && ks + 1 < nk) continue;   // the unit's second stage follows
           tmem_st_wait();
           tc_fence_before();
           __syncwarp();
