@@ -790,12 +790,12 @@ done:
   }
 }
 
-// What a stage of a tile costs in SM cycles: four MMAs per plane, measured at about 190 cycles for 256 tokens and, because the weights
-// have to reach the tensor cores whatever the tokens, no less than about 110 for 128 and for 64; never less than the expansion.
+// What a stage of a tile costs, in nanoseconds (64 tiles of one round, k = 8192 less k = 2048).  One plane: the expansion, almost whatever the
+// tokens (32 to 128: 280 - 300; 192: 320; 256: 323).  Two planes: the MMAs (64 and 128: 440 - 450; 192: 497; 256: 623).  Three: 470 - 500.
 constexpr int kNarrow = 128;   // a tile narrower than this saves nothing
 long long stage_cost(int width, int planes) {
-  const long long mma = 4ll * planes * (width > 149 ? width * 190 / 256 : 110);
-  return mma > 400 ? mma : 400;
+  if (planes == 1) return width > 128 ? 322 : 295;
+  return planes == 3 ? 480 : width > 192 ? 623 : width > 128 ? 497 : 445;
 }
 // Tile width and cut for a problem of `rows256` 256-row tiles and n tokens: the width whose rounds over the SM pairs cost least; the tiles of
 // the last round are cut in two while the pairs can take the halves all at once.
@@ -803,11 +803,11 @@ struct Plan { int width, nfull, cut, tiles; };
 Plan make_plan(int rows256, int n, int planes, int pairs, int widest) {
   Plan best = {0, 0, 1, 0};
   long long best_cost = 0;
-  for (int w = widest; w >= 64; w /= 2) {
-    if (w > 64 && w / 2 >= n) continue;   // half of the width covers every token
+  for (int w = widest; w >= 64; w -= w > 128 ? 64 : w / 2) {   // 256, 192, 128, 64
+    if (w > 64 && (w > 128 ? w - 64 : w / 2) >= n) continue;   // the next width covers every token
     const int tiles = rows256 * ((n + w - 1) / w), rest = tiles % pairs;
     int cut = 1;
-    while (tiles > pairs && rest && w / (2 * cut) >= kNarrow && rest * 2 * cut <= pairs) cut *= 2;
+    while (w != 192 && tiles > pairs && rest && w / (2 * cut) >= kNarrow && rest * 2 * cut <= pairs) cut *= 2;
     const long long c = tiles / pairs * stage_cost(w, planes) + (rest ? stage_cost(w / cut, planes) : 0);
     if (!best.width || c < best_cost) {
       best_cost = c;
