@@ -907,12 +907,16 @@ bool set_up(const GemmArgs &g, int planes, bool f16, int groups, const void *act
 // within 2^-23 of itself or 2^-25, E the exponent of the token's largest scale; tscale[token] = 2^(E - 7).  A token whose scales two planes do not
 // take (see the head of the file) is marked in wide[token].  One CTA per token, a thread per 8 values: 8 bytes in, two 16-byte stores out.
 constexpr int kPlanesThreads = 256, kPlanesSpread = 12;
-__global__ void __launch_bounds__(kPlanesThreads) w4a8_planes_kernel(const int8_t *__restrict__ q, int ld, const float *__restrict__ sc, int lds, int k,
-                                                                     uint16_t *__restrict__ planes, float *__restrict__ tscale, uint8_t *__restrict__ wide) {
+__global__ void __launch_bounds__(kPlanesThreads) w4a8_planes_kernel(const int8_t *q_in, int ld, const float *sc_in, int lds, int k, uint16_t *planes, float *tscale,
+                                                                     uint8_t *wide) {
   pdl_launch_dependents();
+  pdl_wait();
   __shared__ uint32_t red[2][kPlanesThreads / 32];
   const int j = blockIdx.x;
-  const float *const srow = sc + (size_t)j * lds;
+  const float *const srow = behind_wait(sc_in) + (size_t)j * lds;
+  const int8_t *const qrow = behind_wait(q_in) + (size_t)j * ld;
+  uint2 raw_next = make_uint2(0, 0);   // this thread's first values: on their way while the scales are looked through
+  if ((int)threadIdx.x < (k >> 3)) raw_next = *(const uint2 *)(qrow + 8 * threadIdx.x);
   uint32_t hi = 0, lo = 0xFFFFFFFFu;   // largest and smallest non-zero |s| (less one), as bits
   for (int b = threadIdx.x; b < (k >> 4); b += kPlanesThreads) {
     const uint32_t u = __float_as_uint(srow[b]) & 0x7FFFFFFFu;
@@ -934,7 +938,8 @@ __global__ void __launch_bounds__(kPlanesThreads) w4a8_planes_kernel(const int8_
   if (!narrow) return;
   const float up = __uint_as_float((uint32_t)(261 - eh) << 23);   // 2^(7 - E), a normal number
   for (int c = threadIdx.x; c < (k >> 3); c += kPlanesThreads) {
-    const uint2 raw = *(const uint2 *)(q + (size_t)j * ld + 8 * c);
+    const uint2 raw = raw_next;
+    if (c + kPlanesThreads < (k >> 3)) raw_next = *(const uint2 *)(qrow + 8 * (c + kPlanesThreads));
     const float s = __fmul_rn(srow[c >> 1], up);   // exact
     uint32_t t[2][4];
 #pragma unroll
@@ -956,11 +961,13 @@ __global__ void __launch_bounds__(kPlanesThreads) w4a8_planes_kernel(const int8_
 
 // Runs behind it: tells the GEMM which planes there are (tscale[n]), and if some token is wide (or all count as such: `force`) writes three BF16
 // planes [n][3][k] of every token instead, t1 + t2 + t3 = fl(q * s) exactly, tscale 1.
-__global__ void __launch_bounds__(256) w4a8_wide_planes_kernel(const int8_t *q, int ld, const float *sc, int lds, int n, int k, uint16_t *planes, float *tscale,
+__global__ void __launch_bounds__(256) w4a8_wide_planes_kernel(const int8_t *q_in, int ld, const float *sc_in, int lds, int n, int k, uint16_t *planes, float *tscale,
                                                                const uint8_t *wide_in, int force) {
   pdl_launch_dependents();
   pdl_wait();
   const uint8_t *const wide = behind_wait(wide_in);
+  const int8_t *const q = behind_wait(q_in);
+  const float *const sc = behind_wait(sc_in);
   int any = force;
   for (int j = threadIdx.x; j < n && !force; j += blockDim.x) any |= wide[j];
   any = __syncthreads_or(any);
@@ -1083,20 +1090,23 @@ cudaError_t launch_gemm_w4a8_tc(const GemmArgs &g, const int *seg, int groups, c
   uint8_t *const wide = (uint8_t *)(tscale + g.n + 1);
   const bool three = seg || g.n < kW4A8ChainMinN;   // in segments
   const bool force = three || g.A.ue;   // three planes whatever the scales (products with UE5M3 scales leave FP16's range)
+  // Each kernel starts while the one before it ends (a quantizer, usually) and waits for its results; the planes may still be in use by the GEMM before the
+  // quantizer, which that one has waited for.
+  cudaLaunchConfig_t cfg;
+  memset(&cfg, 0, sizeof cfg);
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr; cfg.numAttrs = pdl_enabled() ? 1 : 0;
   if (!force) {
-    w4a8_planes_kernel<<<(unsigned)g.n, kPlanesThreads, 0, s>>>((const int8_t *)g.B.data, g.B.ld, g.B.s8, g.B.lds8, g.k, planes, tscale, wide);
-    e = cudaGetLastError();
+    cfg.gridDim = dim3((unsigned)g.n, 1, 1);
+    cfg.blockDim = dim3(kPlanesThreads, 1, 1);
+    e = cudaLaunchKernelEx(&cfg, w4a8_planes_kernel, (const int8_t *)g.B.data, g.B.ld, g.B.s8, g.B.lds8, g.k, planes, tscale, wide);
   }
   if (e == cudaSuccess) {
-    cudaLaunchConfig_t cfg;
-    memset(&cfg, 0, sizeof cfg);
     cfg.gridDim = dim3(force ? (unsigned)(((long long)g.n * (g.k >> 3) + 255) / 256) : (unsigned)device_sms(), 1, 1);
     cfg.blockDim = dim3(256, 1, 1);
-    cfg.stream = s;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr; cfg.numAttrs = pdl_enabled() && !force ? 1 : 0;   // (`force`: what it overwrites may still be in use by the kernel before)
     e = cudaLaunchKernelEx(&cfg, w4a8_wide_planes_kernel, (const int8_t *)g.B.data, g.B.ld, g.B.s8, g.B.lds8, g.n, g.k, planes, tscale, (const uint8_t *)wide, force ? 1 : 0);
   }
   if (e == cudaSuccess) {

@@ -730,25 +730,54 @@ __global__ void __launch_bounds__(256) quant_dual_kernel(const uint8_t *__restri
 }
 
 // ---- INT8 destination (W4A8 activations): sb = bmax / 127, q = clamp(rint(x / sb), +-127), 0 where sb == 0 -------------------
+// Sixteen divisions by one divisor: with the correctly rounded inv = 1 / sb and y = x * inv, the quotient is fma(fma(-y, sb, x), inv, y), correctly
+// rounded (Markstein's theorem; nothing may underflow or overflow, which the range of sb below sees to, and where x is so small that the
+// remainder does, the quotient is nowhere near 1 / 2).  Adding 1.5 * 2^23 then rounds to an integer, whose low byte is q: |x / sb| <= 127 (1 + 2^-23) needs no
+// clamp.  Blocks with a NaN or a scale outside the range take the IEEE divisions.  2048 x 4096 BF16: 6.8 us (11.5 with a division per
+// value), four rows 1.8 (2.9).
 template <int T>
 __global__ void __launch_bounds__(256) quant_int8_kernel(const uint8_t *__restrict__ src, int lds, int8_t *__restrict__ dst, int ldd,
                                                          float *__restrict__ scales, int ld_scale, int rows, int bpr, float *stat) {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // (the W4A8 GEMM's planes kernel may be launched meanwhile)
   const long long total = (long long)rows * bpr, stride = (long long)gridDim.x * blockDim.x;
   float mx = 0.f;
   for (long long b = (long long)blockIdx.x * blockDim.x + threadIdx.x; b < total; b += stride) {
     const int r = (int)(b / bpr), c = (int)(b - (long long)r * bpr);
     float v[16];
     load16<T>(src + ((size_t)r * lds + 16 * c) * ElemBytes<T>::value, v);
-    float bmax = 0.f;
+    uint32_t top = 0;   // the largest magnitude's bits; above Inf's: a NaN
 #pragma unroll
-    for (int i = 0; i < 16; ++i) bmax = fmaxf(bmax, fabsf(v[i]));
+    for (int i = 0; i < 16; ++i) top = max(top, __float_as_uint(v[i]) & 0x7FFFFFFFu);
+    float bmax = __uint_as_float(top);
+    if (top > 0x7F800000u) {
+      bmax = 0.f;
+#pragma unroll
+      for (int i = 0; i < 16; ++i) bmax = fmaxf(bmax, fabsf(v[i]));
+    }
     mx = fmaxf(mx, bmax);
     const float sb = __fdiv_rn(bmax, 127.f);
     uint32_t w[4] = {0, 0, 0, 0};
+    if (top >= 0x20000000u && top < 0x60000000u) {   // 2^-63 <= bmax < 2^65
+      const float inv = __frcp_rn(sb);
 #pragma unroll
-    for (int i = 0; i < 16; ++i) {
-      const int q = sb > 0.f ? (int)fminf(fmaxf(rintf(__fdiv_rn(v[i], sb)), -127.f), 127.f) : 0;
-      w[i >> 2] |= (uint32_t)(uint8_t)(int8_t)q << (8 * (i & 3));
+      for (int i = 0; i < 4; ++i) {
+        uint32_t q[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const float x = v[4 * i + e], y = __fmul_rn(x, inv);
+          q[e] = __float_as_uint(__fadd_rn(__fmaf_rn(__fmaf_rn(-y, sb, x), inv, y), 12582912.f));
+        }
+        w[i] = byte_perm(byte_perm(q[0], q[1], 0x0040u), byte_perm(q[2], q[3], 0x0040u), 0x5410u);
+      }
+    } else {
+#pragma unroll 1
+      for (int i = 0; i < 16; ++i) {
+        const int q = sb > 0.f ? (int)fminf(fmaxf(rintf(__fdiv_rn(v[0], sb)), -127.f), 127.f) : 0;
+        w[0] = __funnelshift_r(w[0], w[1], 8); w[1] = __funnelshift_r(w[1], w[2], 8); w[2] = __funnelshift_r(w[2], w[3], 8);
+        w[3] = (w[3] >> 8) | ((uint32_t)q << 24);
+#pragma unroll
+        for (int e = 0; e < 15; ++e) v[e] = v[e + 1];
+      }
     }
     *(uint4 *)(dst + (size_t)r * ldd + 16 * c) = make_uint4(w[0], w[1], w[2], w[3]);
     scales[(size_t)r * ld_scale + c] = sb;

@@ -278,3 +278,33 @@ def test_dequantize_by_table_equals_dequantize_value_by_value(dtype, flags):
             if gv == 0.375 and flags & UE:
                 want, _ = O.dequantize(h, dtype)
                 assert np.array_equal(O.to_f32(np.ascontiguousarray(out[0][:, :cols]).reshape(-1), dtype).reshape(rows, cols), want)
+
+
+@pytest.mark.parametrize("lo,hi", [(-10, 10), (-61, -66), (62, 67), (-126, -100), (100, 127), (-149, 127)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+def test_quantize_int8_without_divisions_equals_ieee_divisions(dtype, lo, hi):
+    """q = clamp(rint(x / sb), +-127) by a reciprocal and two fused multiply-adds, or by IEEE divisions where a block's scale is too far from one or a value is a
+    NaN: torch's IEEE division gives the same bytes.  Quotients at and beside every half integer, random significands, zeros, infinities, NaNs."""
+    import nvfp4effma_b200.api as nf
+    gen = torch.Generator(device="cuda").manual_seed(5)
+    n = 1 << 20
+    e = torch.randint(min(lo, hi), max(lo, hi) + 1, (n, 1), generator=gen, device="cuda").float()
+    x = (torch.rand(n, 16, generator=gen, device="cuda") * 2 - 1).double()
+    x[: n // 2, 0] = 1.0 - torch.rand(n // 2, generator=gen, device="cuda").double() / 4
+    half = (torch.randint(0, 127, (n // 2, 15), generator=gen, device="cuda").double() + 0.5) / 127.0 * x[: n // 2, :1]   # quotients near k + 1/2
+    x[: n // 2, 1:] = half * (1 + torch.randint(-2, 3, half.shape, generator=gen, device="cuda").double() * 2.0 ** -24)
+    x = (x * torch.exp2(e.double())).to(dtype)
+    x[7] = 0.0
+    if hi - lo > 200:
+        x[8:1000:9, 3] = float("nan")
+        x[9:1000:9, 5] = float("inf")
+    x = x.view(-1, 512)
+    got = nf.quantize_int8(x)
+    v = x.float().view(n, 16)
+    bmax = torch.where(v.isnan(), torch.zeros_like(v), v.abs()).amax(-1, keepdim=True)
+    sb = bmax / torch.tensor(127.0, device="cuda")
+    q = (v / sb).round()
+    q = torch.where(q.isnan(), torch.full_like(q, -127.0), q.clamp(-127, 127))   # (fmax(NaN, -127) = -127)
+    q = torch.where(sb > 0, q, torch.zeros_like(q)).to(torch.int8)
+    assert torch.equal(got.scales.view(n, 1).view(torch.int32), sb.view(torch.int32))
+    assert torch.equal(got.data.view(n, 16), q)
