@@ -308,3 +308,36 @@ def test_quantize_int8_without_divisions_equals_ieee_divisions(dtype, lo, hi):
     q = torch.where(sb > 0, q, torch.zeros_like(q)).to(torch.int8)
     assert torch.equal(got.scales.view(n, 1).view(torch.int32), sb.view(torch.int32))
     assert torch.equal(got.data.view(n, 16), q)
+
+
+@pytest.mark.parametrize("offset,pad", [(0, 0), (16, 0), (0, 16), (16, 48)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+def test_blocks_of_32_bytes_at_every_alignment(dtype, offset, pad):
+    """32-byte loads and stores where base and row pitch allow them, 16-byte ones elsewhere: the same bytes from the quantizer (amax computed, in one launch
+    and in two, and given) and from the dequantizer (padding untouched)."""
+    import nvfp4effma_b200.api as nf
+    esz = torch.empty(0, dtype=dtype).element_size()
+    for rows, cols in ((37, 1040), (1031, 8192)):
+        ld = cols + pad
+        gen = torch.Generator(device="cuda").manual_seed(rows)
+        base = torch.randn(rows * ld + 64, generator=gen, device="cuda").to(dtype)
+        x = base[offset // esz:][: rows * ld].view(rows, ld)
+        xc = x[:, :cols].contiguous()
+        want = nf.quantize(xc)
+        for compute in (1, 0):
+            data = torch.zeros(rows, cols // 2, dtype=torch.uint8, device="cuda")
+            sc = torch.zeros(rows, cols // 16, dtype=torch.uint8, device="cuda")
+            glob = want.amax.clone().float().reshape(1) if not compute else torch.zeros(1, device="cuda")
+            S, Q = tensor(x, {torch.bfloat16: L.BF16, torch.float16: L.FP16, torch.float32: L.FP32}[dtype]), tensor(data, L.NVFP4, sc, cols // 16, glob, None, L.GLOBAL_AMAX)
+            cfg = L.QuantConfig(1, 0, compute)
+            L.check(L.lib.nvfp4a_quantize_ex(ctypes.byref(S), ld, rows, cols, ctypes.byref(Q), cols, None, 0, ctypes.byref(cfg), stream()))
+            assert torch.equal(data, want.data.view(torch.uint8)) and torch.equal(sc, want.scales.view(torch.uint8).reshape(rows, -1)[:, : cols // 16])
+        if dtype == torch.float32:
+            continue
+        back = torch.full((rows * ld + 64,), 7.0, dtype=dtype, device="cuda")
+        out = back[offset // esz:][: rows * ld].view(rows, ld)
+        Dt = tensor(out, L.BF16 if dtype == torch.bfloat16 else L.FP16)
+        Q = tensor(want.data, L.NVFP4, want.scales, want.scales.shape[-1], want.amax, None, L.GLOBAL_AMAX)
+        L.check(L.lib.nvfp4a_dequantize(ctypes.byref(Q), cols, ctypes.byref(Dt), ld, rows, cols, stream()))
+        assert torch.equal(out[:, :cols], nf.dequantize(want, dtype))
+        assert bool((back[: offset // esz] == 7).all()) and bool((out[:, cols:] == 7).all()) and bool((back[offset // esz + rows * ld:] == 7).all())
