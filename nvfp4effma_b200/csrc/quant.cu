@@ -332,12 +332,14 @@ __global__ void __launch_bounds__(256, 3) quant_rows_kernel(const uint8_t *__res
 // Measured on 8192 x 8192: HBM traffic 159 MB against 287 MB for the two launches, the same 55 us -- the encode arithmetic (about
 // 170 instructions per block of 16) at 16 warps per SM, not memory, is what bounds the second visit.
 // Per-CTA maxima meet in a device array (no atomics on floats, no memset launch): every CTA reads all of them after the barrier.
+// (A launch on another stream may begin while this one's last CTAs run -- a CTA takes a whole SM, so its own barrier opens only when they have left.  Launches
+// therefore alternate between two arrays of maxima: nobody writes what a late CTA of the launch before is still to read.)
 // The barrier's wait is bounded like every wait of this library; on expiry the status word gets 0x601 and the kernel goes on
 // (with whatever maxima have arrived) so that it always terminates.
 constexpr int kQfSmemBytes = 96 * 2048;            // 96 units of 2 KiB stay in shared memory per CTA
 constexpr int kQfMaxGrid = 1024;
 static __device__ unsigned long long g_qf_arrivals;   // arrivals of every launch so far on this device (each launch adds its grid size, which never changes)
-static __device__ float g_qf_max[kQfMaxGrid];      // per-CTA maxima of the current launch
+static __device__ float g_qf_max[2][kQfMaxGrid];   // per-CTA maxima of the current launch and of the one before it
 
 // max |x| of a block of 16-bit values taken on the packed words (bit patterns of non-negative BF16 / FP16 values order like the values)
 template <int T>
@@ -429,6 +431,10 @@ quant_fused_kernel(const uint8_t *__restrict__ src, int lds, int rows, int bpr, 
     return pm;
   };
 
+  // which launch this is on the device: no CTA of it has passed the barrier yet, and every launch before it has
+  unsigned long long arrived = 0;
+  if (threadIdx.x == 0) asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(arrived) : "l"(&g_qf_arrivals) : "memory");
+
   // ---- visit 1: amax; the last units stay on chip ----
   uint32_t pm = 0;
   int j = 0;
@@ -473,11 +479,12 @@ quant_fused_kernel(const uint8_t *__restrict__ src, int lds, int rows, int bpr, 
   // the arrival (which publishes this CTA's maximum), the poll that sees the last arrival, the read of all CTAs' maxima by ONE warp
   // per CTA (a line that thousands of warps read at once is served one request at a time).
   if (warp == 0) {
+    float *const maxima = g_qf_max[__shfl_sync(0xFFFFFFFFu, (unsigned)(arrived / gridDim.x), 0) & 1u];
     float cm = lane < kQfWarps ? warp_max[lane] : 0.f;
 #pragma unroll
     for (int of = 16; of; of >>= 1) cm = fmaxf(cm, __shfl_xor_sync(0xFFFFFFFFu, cm, of));
     if (lane == 0) {
-      g_qf_max[blockIdx.x] = cm;
+      maxima[blockIdx.x] = cm;
       unsigned long long old, now;
       asm volatile("atom.add.acq_rel.gpu.global.u64 %0, [%1], 1;" : "=l"(old) : "l"(&g_qf_arrivals) : "memory");
       const unsigned long long target = (old / gridDim.x + 1) * gridDim.x;
@@ -490,7 +497,7 @@ quant_fused_kernel(const uint8_t *__restrict__ src, int lds, int rows, int bpr, 
     }
     __syncwarp();
     float all = 0.f;
-    for (unsigned i = lane; i < gridDim.x; i += 32) all = fmaxf(all, __ldcg(&g_qf_max[i]));
+    for (unsigned i = lane; i < gridDim.x; i += 32) all = fmaxf(all, __ldcg(&maxima[i]));
 #pragma unroll
     for (int of = 16; of; of >>= 1) all = fmaxf(all, __shfl_xor_sync(0xFFFFFFFFu, all, of));
     if (lane == 0) gmax_s = all;
@@ -1062,10 +1069,11 @@ extern "C" nvfp4a_status nvfp4a_quantize_ex(const nvfp4a_tensor *src, int lds, i
 
   const uint8_t *s = (const uint8_t *)src->data;
   const int bpr = cols / 16;
-  // One-read path: the common recipe (rowwise 1 x 16 blocks, one amax for the tensor, no 4over6, 16-bit source) on a matrix large
-  // enough to occupy every SM runs as ONE cooperative kernel that reads most of the source once (quant_fused_kernel).
+  // One-read path: the common recipe (rowwise 1 x 16 blocks, one amax for the tensor, no 4over6, 16-bit source) runs as ONE cooperative kernel
+  // that reads most of the source once (quant_fused_kernel) -- all of it up to 9.7 M values, and one launch where there were a fill, the amax pass and
+  // the encode: 256 x 1024 7.9 -> 6.2 us, 1024 x 2048 9.8 -> 7.2, 1500 x 4096 12.5 -> 10.3 (2048 x 4096 and up as before).
   if (c.compute_amax && rowwise && !columnwise && c.tile_rows == 1 && c.four_over_six == NVFP4A_4OVER6_OFF &&
-      !(rowwise->flags & NVFP4A_GLOBAL_PER_ROW) && src->dtype != NVFP4A_FP32 && (bpr & 3) == 0 && (long long)rows * cols >= (8ll << 20) &&
+      !(rowwise->flags & NVFP4A_GLOBAL_PER_ROW) && src->dtype != NVFP4A_FP32 && (bpr & 3) == 0 && (long long)rows * cols >= (1ll << 16) &&
       quant_fused_enabled()) {
     const QOut o = make_qout(rowwise, ld_row, sld[0]);
     cudaError_t e = cudaSuccess;

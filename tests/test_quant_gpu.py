@@ -341,3 +341,29 @@ def test_blocks_of_32_bytes_at_every_alignment(dtype, offset, pad):
         L.check(L.lib.nvfp4a_dequantize(ctypes.byref(Q), cols, ctypes.byref(Dt), ld, rows, cols, stream()))
         assert torch.equal(out[:, :cols], nf.dequantize(want, dtype))
         assert bool((back[: offset // esz] == 7).all()) and bool((out[:, cols:] == 7).all()) and bool((back[offset // esz + rows * ld:] == 7).all())
+
+
+def test_small_matrices_quantize_in_one_launch_on_several_streams():
+    """The cooperative kernel from 65536 values up, many launches on four streams at once (launches of it share a barrier counter and alternate between two
+    arrays of maxima): every result has the bytes of the two-launch path."""
+    import nvfp4effma_b200.api as nf
+    gen = torch.Generator(device="cuda").manual_seed(9)
+    xs = [(torch.randn(r, c, generator=gen, device="cuda") * 2.0 ** i).to(dt) for i, (r, c, dt) in
+          enumerate([(64, 1024, torch.bfloat16), (131, 512, torch.float16), (300, 4096, torch.bfloat16), (1000, 2048, torch.float16), (2048, 4096, torch.bfloat16)])]
+    L.lib.nvfp4a_b200_set_quant_fused(0)
+    try:
+        want = [nf.quantize(x, swizzled=True) for x in xs]
+    finally:
+        L.lib.nvfp4a_b200_set_quant_fused(1)
+    streams = [torch.cuda.Stream() for _ in range(4)]
+    torch.cuda.synchronize()
+    got = []
+    for rep in range(40):
+        for i in range(len(xs)):
+            with torch.cuda.stream(streams[(rep + i) % 4]):
+                got.append((i, nf.quantize(xs[i], swizzled=True)))
+    torch.cuda.synchronize()
+    for i, q in got:
+        w = want[i]
+        assert torch.equal(q.data.view(torch.uint8), w.data.view(torch.uint8)) and torch.equal(q.scales.view(torch.uint8), w.scales.view(torch.uint8))
+        assert torch.equal(q.amax, w.amax)
