@@ -159,7 +159,8 @@ static BOperand make_b(const nvfp4a_tensor *B, int ldb, int ldsb, int k, bool im
 // nvfp4a_gemm / nvfp4a_gemm_ex
 static nvfp4a_status gemm_run(const char *fn, int m, int n, int k, float alpha, const nvfp4a_tensor *A, int lda, const nvfp4a_tensor *B, int ldb,
                               float beta, const nvfp4a_tensor *C, int ldc, const nvfp4a_tensor *D, int ldd, const nvfp4a_tensor *bias,
-                              const EpilogueEx &ex, cudaStream_t stream, bool validate_only = false, int a_groups = 1, GemmArgs *args_out = nullptr) {
+                              const EpilogueEx &ex, cudaStream_t stream, bool validate_only = false, int a_groups = 1, GemmArgs *args_out = nullptr,
+                              bool whole_k = false) {
   // a_groups > 1 (nvfp4a_gemm_grouped): A holds a_groups stacked weights of m rows; nothing is launched, the arguments go to args_out
   if (!A || !B || !D || !A->data || !B->data || !D->data) return fail(NVFP4A_INVALID_VALUE, "%s: A, B or D (or its data pointer) is NULL", fn);
   if (m < 0 || n < 0 || k < 0) return fail(NVFP4A_INVALID_VALUE, "%s: negative size (m = %d, n = %d, k = %d)", fn, m, n, k);
@@ -201,6 +202,7 @@ static nvfp4a_status gemm_run(const char *fn, int m, int n, int k, float alpha, 
   g.e = make_epilogue(alpha, A, B, beta, C, ldc, D, ldd, bias);
   g.x = ex;
   g.no_alloc = g_no_alloc;
+  g.whole_k = whole_k;
   if (args_out) *args_out = g;
   if (validate_only || args_out) return NVFP4A_OK;
   return dispatch(fn, g, stream);
@@ -375,7 +377,7 @@ extern "C" nvfp4a_status nvfp4a_gemm_ex(int m, int n, int k, float alpha, const 
   clear_error();
   EpilogueEx x;
   if (nvfp4a_status st = make_epilogue_ex("nvfp4a_gemm_ex", ex, m, beta, ldd, &x)) return st;
-  return gemm_run("nvfp4a_gemm_ex", m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, D, ldd, bias, x, stream);
+  return gemm_run("nvfp4a_gemm_ex", m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, D, ldd, bias, x, stream, false, 1, nullptr, true);
 }
 
 extern "C" nvfp4a_status nvfp4a_gemm_dual(int m, int n, int k, float alpha, const nvfp4a_dual_tensor *A, int trans_a, const nvfp4a_dual_tensor *B,

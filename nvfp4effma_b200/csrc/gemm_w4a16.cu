@@ -84,6 +84,7 @@ struct W4A16Args {
   int seg_stages;   // F16, GROUPED: stages per segment of k
   int unit;         // stages per unit: 1 or 2 (see the MMA issuer)
   const int *seg; int groups;   // GROUPED: m is the rows of ONE group's weight, n the bound on seg[groups]
+  int parts, part_stages; float *partial;   // kEpiPart: k in `parts` runs of part_stages stages, each one's sums in partial [part][n][m]
   const float *tscale;          // PLANES = 2: what each token's sums are multiplied by, then (word n) non-zero for three planes
 };
 
@@ -181,7 +182,8 @@ constexpr int kMaxGroups = 256;
 // which a plain call's instructions lie far apart: fetching them made a chunk of 32 columns take 5000 cycles, in which the tensor cores wait for the
 // accumulator or, at the end, the caller for the result.  28672 x 4096 with SwiGLU on 2048 tokens: 412 -> 344 us; FP16 4096 x 4096 on 333
 // tokens 37.5 -> 35.2; 5504 x 3584 with SwiGLU on 121 tokens 32.1 -> 27.0.
-enum { kEpiAny = 0, kEpiPlain = 1, kEpiSwiglu = 2 };
+// 3: no epilogue, the sums of a part of k as they are (see w4a16_join_kernel).
+enum { kEpiAny = 0, kEpiPlain = 1, kEpiSwiglu = 2, kEpiPart = 3 };
 template <int PLANES, bool F16, bool GROUPED, int EPI>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_b, const __grid_constant__ CUtensorMap tmap_d,
@@ -209,8 +211,11 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
   const int nA = 1 << lgA, nB = 1 << lgB, subA = kA >> lgA;
   constexpr int kSub = PLANES == 3 ? C::kBBytes / 2 : C::kBBytes;   // bytes of a stage of one plane (three planes: tiles of at most 128 tokens)
   const int slot_bytes = (kB * C::kBBytes) >> lgB;
-  const int tiles_m = (gm + 255) / 256, nk = gk / 64, nslots = (nk + 3) / 4;   // 256-row tiles
+  constexpr bool PART = EPI == kEpiPart;
   const int tile_first = blockIdx.x >> 1, tile_step = gridDim.x >> 1;
+  // (parts of k: a pair has one part of one tile, the stages [k0, k0 + nk))
+  const int parts = PART ? g.parts : 1, k0 = PART ? tile_first % parts * g.part_stages : 0;
+  const int tiles_m = (gm + 255) / 256, nk = PART ? min(g.part_stages, gk / 64 - k0) : gk / 64, nslots = (nk + 3) / 4;   // 256-row tiles
   const bool ue = g.A.ue != 0;
   unsigned *const status_word = g.status;
 
@@ -294,6 +299,7 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
       const int j0 = gseg[q] + (tt - gcum[q]) * W, left = gseg[q + 1] - j0;
       return Tile{t % tiles_m, j0, gseg[q + 1], left < W ? (left + 63) & ~63 : W, q * gm};
     }
+    if (PART) t /= parts;
     int w = W, part = 0;
     if (t >= nfull) { w = W / cut; part = (t - nfull) % cut; t = nfull + (t - nfull) / cut; }
     const int j0 = t / tiles_m * W + part * w, left = gn - j0;
@@ -322,7 +328,7 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
           if (rank == 0) mbar_arrive_expect_tx_elect(&b_full[s], nsub * sub_bytes);
           const uint32_t dst = smem_u32(sB) + (uint32_t)(s * slot_bytes), bar = mbar_addr_rank(&b_full[s], 0);
           for (int i = 0; i < nsub; ++i)
-            tma_load_3d_pair_elect(dst + i * kSub, &tmap_b, PLANES == 1 ? (ks + i) * 128 : (pl + i) * 2 * gk + ks * 128, row0, 0, bar);
+            tma_load_3d_pair_elect(dst + i * kSub, &tmap_b, PLANES == 1 ? (k0 + ks + i) * 128 : (pl + i) * 2 * gk + (k0 + ks) * 128, row0, 0, bar);
         }
       }
     }
@@ -397,8 +403,8 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
         mbar_arrive_expect_tx_elect(&raw_full[s], C::kRawBytes);
         const uint32_t dst = smem_u32(sRaw + (size_t)s * C::kRawBytes), bar = smem_u32(&raw_full[s]);
         // (rows past the matrix read zeros; their scales are those of its last row, and no row past it is stored)
-        if (img) tma_load_3d_elect(dst, &tmap_w, 0, 0, row_tile * ktiles + sl, bar);
-        else tma_load_3d_elect(dst, &tmap_w, sl * 128, p.ro + row_tile * 128, 0, bar);
+        if (img) tma_load_3d_elect(dst, &tmap_w, 0, 0, row_tile * ktiles + (k0 >> 2) + sl, bar);
+        else tma_load_3d_elect(dst, &tmap_w, ((k0 >> 2) + sl) * 128, p.ro + row_tile * 128, 0, bar);
       }
     }
   }
@@ -407,9 +413,9 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
     // ---------------- epilogue ----------------
     const int quad = warp & 3, half = (warp - 4) >> 2, bar_id = 2 + half;   // barrier 1: all eight warps; 2 and 3: the four of a half
     // (rarely used parameters are read from the constant bank where they are needed: the registers belong to the accumulator block)
-    const float gb0 = g.e.gb ? *g.e.gb : 1.f;   // B's global: dense B has none, INT8 B one for the tensor (a multiply by 1 is exact)
+    const float gb0 = !PART && g.e.gb ? *g.e.gb : 1.f;   // B's global: dense B has none, INT8 B one for the tensor (a multiply by 1 is exact)
     uint8_t *const dptr = (uint8_t *)g.e.d;
-    const int d_dtype = g.e.d_dtype, mask = EPI == kEpiSwiglu ? kExSwiglu : SEG || EPI == kEpiPlain ? 0 : g.x.mask;   // (segments: a 16-bit D and the plain epilogue)
+    const int d_dtype = g.e.d_dtype, mask = EPI == kEpiSwiglu ? kExSwiglu : SEG || EPI == kEpiPlain || PART ? 0 : g.x.mask;   // (segments: a 16-bit D and the plain epilogue)
     const bool d_tma = g.d_tma;
     // The accumulator is read as MMA fragments (16 lanes x 8 columns per register quad): a thread holds rows rb + 16 hh + 8 u (hh, u in
     // {0, 1}) of columns 8 gq + cp + e (e in {0, 1}) of a chunk of 32, register 16 hh + 4 gq + 2 u + e.  Gate and up rows of SwiGLU (8
@@ -474,8 +480,8 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
         const int i = rb + 8 * q;
-        rowp[q] = i < gm ? __fmul_rn(g.e.alpha, g.e.ga ? g.e.ga[(size_t)(p.ro + i) * g.e.ga_stride] : 1.f) : 0.f;
-        bias[q] = (i < gm && g.e.bias) ? load_dense(g.e.bias_dtype, g.e.bias, p.ro + i) : -0.f;   // (adding -0 changes nothing)
+        rowp[q] = !PART && i < gm ? __fmul_rn(g.e.alpha, g.e.ga ? g.e.ga[(size_t)(p.ro + i) * g.e.ga_stride] : 1.f) : 0.f;
+        bias[q] = (!PART && i < gm && g.e.bias) ? load_dense(g.e.bias_dtype, g.e.bias, p.ro + i) : -0.f;   // (adding -0 changes nothing)
         if (!(mask & kExNorm)) rowp[q] = __fmul_rn(__fmul_rn(rowp[q], gb0), g.e.gf);   // ((alpha gA) * gB) * gf
       }
       if (mask & kExNorm) {  // column scales of this token tile (the previous tile's are no longer in use: see the barrier below)
@@ -556,6 +562,21 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
         const int cc = half * hw + c * 32;   // first column of the chunk in the tile
         const int j0 = jt + cc;
         const int nvalid = min(32, jend - j0);
+        if constexpr (PART) {   // eight lanes write 32 contiguous bytes of a token's sums
+          float *const p32 = g.partial + ((size_t)(tile_first % parts) * gn + j0) * gm + rb;
+#pragma unroll
+          for (int ce = 0; ce < 8; ++ce) {
+            const int jj = 8 * (ce >> 1) + cp + (ce & 1);
+            if (jj >= nvalid) continue;
+            const float ts = PLANES == 2 ? tscale[j0 + jj] : 1.f;
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+              const float v = __uint_as_float(r[16 * (q >> 1) + 4 * (ce >> 1) + 2 * (q & 1) + (ce & 1)]);
+              if (rb + 8 * q < gm) p32[(size_t)jj * gm + 8 * q] = PLANES == 2 ? __fmul_rn(v, ts) : v;
+            }
+          }
+          continue;
+        }
         const bool tma = d_tma && (!GROUPED || nvalid == 32);   // (a group's last box would reach into the next group's tokens)
         // values before the output rounding, kept in r[] as FP32 bits
 #pragma unroll
@@ -719,7 +740,7 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
         const int ks = 4 * sl + 2 * group + h;
-        const size_t off = img ? (size_t)sl * kImgTileBytes + (ks & 3) * 512 : swz ? (size_t)ks * 512 : (size_t)ks * 4;
+        const size_t off = img ? (size_t)((k0 >> 2) + sl) * kImgTileBytes + (ks & 3) * 512 : swz ? (size_t)(k0 + ks) * 512 : (size_t)(k0 + ks) * 4;
         v[h] = ks < nk ? *(const uint32_t *)(scp + off) : 0u;
       }
     };
@@ -817,6 +838,25 @@ Plan make_plan(int rows256, int n, int planes, int pairs, int widest) {
   return best;
 }
 
+// Parts of k.  A problem with few tiles leaves most SM pairs idle while each tile is a serial chain over k (0.3 to 0.6 us per 64 values).  Up to eight pairs
+// take a run of at least 512 values each; their FP32 sums meet in memory, which is L2, and a small kernel adds them in order.  That kernel, its launch and
+// the memory cost 8 us of a caller's time and the traffic (0.5 ns per KB), so that k has to be long enough to gain more.  A call in eager mode: INT8
+// 4928 x 4608 on 35 tokens 47.8 -> 30.2 us, 832 x 4480 on 12 45.6 -> 28.2, BF16 2688 x 4736 on 46 25.3 -> 17.0; with less to gain, INT8 2594 x 1792 on
+// 12 tokens 26.3 -> 28.5 and BF16 872 x 5376 on 1030 29.6 -> 31.2, which this rule leaves whole.
+// Not for nvfp4a_gemm_ex (see GemmArgs::whole_k), nor for images of BF16 problems: the outputs of a tensor-parallel shard are those of the whole matrix bit for bit, however many tiles either has.
+int choose_parts(const GemmArgs &g, int planes, const Plan &p, int pairs) {
+  const bool tp_twin = g.A.image && g.B.dtype == NVFP4A_BF16;
+  if (tp_twin || g.no_alloc || g.whole_k || g.tp.world > 1 || g.x.mask || p.cut > 1 || 2 * p.tiles > pairs) return 1;
+  const int slots = (g.k + 255) / 256;
+  int parts = pairs / p.tiles;
+  if (parts > 8) parts = 8;
+  if (parts > slots / 2) parts = slots / 2;
+  if (parts < 2) return 1;
+  parts = (slots + (slots + parts - 1) / parts - 1) / ((slots + parts - 1) / parts);   // (equal runs: no empty part)
+  const int saved = (slots - (slots + parts - 1) / parts) * 4;   // stages
+  return saved * stage_cost(p.width, planes) > 8000 + 8ll * parts * g.n * g.m / 2000 ? parts : 1;
+}
+
 // Grouped: only the average number of tokens per group is known here, and each group ends in a tile as wide as its last tokens (in steps
 // of 64).  `tiles` bounds the grid, the kernel counts the tiles itself.
 Plan make_grouped_plan(int rows256, int n, int groups, int planes, int pairs, int widest) {
@@ -866,11 +906,21 @@ cudaError_t launch_epi(const CUtensorMap &tw, const CUtensorMap &tb, const CUten
 
 template <int PLANES, bool F16, bool GROUPED = false>
 cudaError_t launch_cfg(const CUtensorMap &tw, const CUtensorMap &tb, const CUtensorMap &td, const PeerMaps &pm, const W4A16Args &a, cudaStream_t s) {
+  if constexpr (!GROUPED)
+    if (a.parts > 1) return launch_epi<PLANES, F16, GROUPED, kEpiPart>(tw, tb, td, pm, a, s);
   const bool plain = a.e.beta == 0.f && !a.e.amax && a.e.d_dtype != NVFP4A_FP32;
   if constexpr (!F16 && !GROUPED)
     if (plain && a.x.mask == kExSwiglu) return launch_epi<PLANES, F16, GROUPED, kEpiSwiglu>(tw, tb, td, pm, a, s);
   if (plain && a.x.mask == 0) return launch_epi<PLANES, F16, GROUPED, kEpiPlain>(tw, tb, td, pm, a, s);
   return launch_epi<PLANES, F16, GROUPED, kEpiAny>(tw, tb, td, pm, a, s);
+}
+
+// the tile plan of one weight and the parts of k
+int plan_parts(const GemmArgs &g, int planes, bool f16, Plan *plan) {
+  const int rows256 = (g.m + 255) / 256, pairs = device_sms() / 2;
+  const Plan p = make_plan(rows256, g.n, planes, pairs, f16 || planes == 3 ? kSegmentWidth : 256);
+  if (plan) *plan = p;
+  return choose_parts(g, planes, p, pairs);
 }
 
 // what every launch of the kernel shares: arguments, the schedule, the maps of the weights, of the activations (`row_bytes` bytes per
@@ -883,12 +933,20 @@ bool set_up(const GemmArgs &g, int planes, bool f16, int groups, const void *act
   a->e = g.e; a->x = g.x;
   a->status = kernel_status_device_ptr();
   a->tag = next_launch_tag();
-  const int rows256 = (g.m + 255) / 256, pairs = device_sms() / 2, widest = f16 || planes == 3 ? kSegmentWidth : 256;
-  const Plan p = groups ? make_grouped_plan(rows256, g.n, groups, planes, pairs, widest) : make_plan(rows256, g.n, planes, pairs, widest);
+  const int rows256 = (g.m + 255) / 256, pairs = device_sms() / 2;
+  Plan p;
+  a->parts = 1;
+  if (groups) p = make_grouped_plan(rows256, g.n, groups, planes, pairs, kSegmentWidth);
+  else a->parts = plan_parts(g, planes, f16, &p);
   const uint64_t wrows = (uint64_t)g.m * (groups ? groups : 1);
   a->unit = planes == 1 && !(f16 && g.k < 512) ? 2 : 1;
   a->seg_stages = g.k >= 1024 ? 4 : g.k >= 512 ? 2 : 1;   // (the longest that keep the sums no less exact than the CUDA-core kernels': see the head of the file)
   a->width = p.width; a->nfull = p.nfull; a->cut = p.cut; a->tiles = p.tiles;
+  if (a->parts > 1) {
+    const int slots = (g.k + 255) / 256;
+    a->part_stages = (slots + a->parts - 1) / a->parts * 4;
+    a->nfull = a->tiles *= a->parts;
+  }
   const uint64_t wtiles = (uint64_t)((g.m + 127) / 128) * g.A.ktiles;
   if (g.A.image ? !make_tmap_bytes(tw, g.A.data, 128, 128, 128, 128, wtiles, kImgTileBytes)
                 : !make_tmap_bytes(tw, g.A.data, (uint64_t)g.k / 2, wrows, (uint64_t)g.A.ld / 2, 128, 1, (uint64_t)g.A.ld / 2 * wrows))
@@ -898,7 +956,7 @@ bool set_up(const GemmArgs &g, int planes, bool f16, int groups, const void *act
   const int esz = dense_bytes(g.e.d_dtype);
   const bool glu = (g.x.mask & kExSwiglu) != 0;
   const int drows = glu ? g.m / 2 : g.m;   // SwiGLU: the output has m / 2 rows, 64 per 128-row tile
-  a->d_tma = esz == 2 && ((uintptr_t)g.e.d & 15) == 0 && ((size_t)g.e.ldd * esz) % 16 == 0 && ((size_t)drows * esz) % 16 == 0 &&
+  a->d_tma = a->parts == 1 && esz == 2 && ((uintptr_t)g.e.d & 15) == 0 && ((size_t)g.e.ldd * esz) % 16 == 0 && ((size_t)drows * esz) % 16 == 0 &&
              make_tmap_dense(td, g.e.d, esz, (uint64_t)drows, (uint64_t)g.n, (uint64_t)g.e.ldd * esz, 64, 32, 128);
   return true;
 }
@@ -999,6 +1057,24 @@ __global__ void __launch_bounds__(256) w4a8_wide_planes_kernel(const int8_t *q_i
   }
 }
 
+// The parts' sums [parts][n][m] added in order, then the plain epilogue.
+__global__ void __launch_bounds__(256) w4a16_join_kernel(const float *partial_in, int parts, int m, int n, const Epilogue e) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const float *const p = behind_wait(partial_in);
+  const int i = blockIdx.x * 256 + threadIdx.x, j = blockIdx.y;
+  float amax = 0.f;
+  if (i < m) {
+    const size_t at = (size_t)j * m + i, step = (size_t)n * m;
+    float s = p[at];
+    for (int q = 1; q < parts; ++q) s = __fadd_rn(s, p[at + q * step]);
+    const float v = epi_value(e, i, j, s, epi_scale(e, epi_row_part(e, i), epi_col_part(e, j)));
+    store_dense(e.d_dtype, e.d, (size_t)j * e.ldd + i, v);
+    amax = fabsf(v);
+  }
+  if (e.amax) warp_amax_commit(e.amax, amax);
+}
+
 }  // namespace
 
 // tensor parallel: true when this kernel stores D into the peers' buffers itself (its output path is the TMA store)
@@ -1047,6 +1123,19 @@ static cudaError_t planes_pool(cudaMemPool_t *pool) {
   *pool = p;
   return cudaSuccess;
 }
+// the join behind a GEMM in parts of k
+static cudaError_t launch_join(const W4A16Args &a, cudaStream_t s) {
+  cudaLaunchConfig_t cfg;
+  memset(&cfg, 0, sizeof cfg);
+  cfg.gridDim = dim3((unsigned)((a.m + 255) / 256), (unsigned)a.n, 1);
+  cfg.blockDim = dim3(256, 1, 1);
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr; cfg.numAttrs = pdl_enabled() ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, w4a16_join_kernel, (const float *)a.partial, a.parts, a.m, a.n, a.e);
+}
 cudaError_t trim_planes_pool() {
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
@@ -1078,17 +1167,25 @@ bool gemm_w4a8_grouped_supports(const GemmArgs &g, int groups) {
 
 // seg == NULL: one weight; else `groups` stacked weights of g.m rows
 cudaError_t launch_gemm_w4a8_tc(const GemmArgs &g, const int *seg, int groups, cudaStream_t s) {
+  const bool three = seg || g.n < kW4A8ChainMinN;   // in segments
   uint16_t *planes = nullptr;
   cudaMemPool_t pool;
   cudaError_t e = planes_pool(&pool);
   if (e != cudaSuccess) return e;
-  // planes [n][3][k], n token scales and the word behind them, n marks
-  const size_t plane_bytes = (size_t)g.n * 3 * g.k * sizeof(uint16_t);
-  e = cudaMallocFromPoolAsync((void **)&planes, plane_bytes + (size_t)(g.n + 1) * sizeof(float) + g.n, pool, s);
+  // planes [n][3][k], n token scales and the word behind them, n marks; the sums of parts of k, if there are any
+  const size_t plane_bytes = (size_t)g.n * 3 * g.k * sizeof(uint16_t), small_bytes = (plane_bytes + (size_t)(g.n + 1) * sizeof(float) + g.n + 255) / 256 * 256;
+  GemmArgs w = g;
+  int parts = seg ? 1 : plan_parts(g, three ? 3 : 2, false, nullptr);
+  if (parts > 1 && cudaMallocFromPoolAsync((void **)&planes, small_bytes + (size_t)parts * g.n * g.m * sizeof(float), pool, s) != cudaSuccess) {
+    (void)cudaGetLastError();
+    planes = nullptr;
+    parts = 1;
+    w.no_alloc = 1;   // k stays whole
+  }
+  if (!planes) e = cudaMallocFromPoolAsync((void **)&planes, small_bytes, pool, s);
   if (e != cudaSuccess) return e;
   float *const tscale = (float *)((uint8_t *)planes + plane_bytes);
   uint8_t *const wide = (uint8_t *)(tscale + g.n + 1);
-  const bool three = seg || g.n < kW4A8ChainMinN;   // in segments
   const bool force = three || g.A.ue;   // three planes whatever the scales (products with UE5M3 scales leave FP16's range)
   // Each kernel starts while the one before it ends (a quantizer, usually) and waits for its results; the planes may still be in use by the GEMM before the
   // quantizer, which that one has waited for.
@@ -1114,11 +1211,13 @@ cudaError_t launch_gemm_w4a8_tc(const GemmArgs &g, const int *seg, int groups, c
     CUtensorMap tw, tb, td;
     PeerMaps pm;
     memset(&pm, 0, sizeof pm);
-    if (!set_up(g, three ? 3 : 2, false, seg ? groups : 0, planes, (uint64_t)g.k * 6, (uint64_t)g.k * 6, &a, &tw, &tb, &td)) e = cudaErrorInvalidValue;
+    if (!set_up(w, three ? 3 : 2, false, seg ? groups : 0, planes, (uint64_t)g.k * 6, (uint64_t)g.k * 6, &a, &tw, &tb, &td)) e = cudaErrorInvalidValue;
     else {
       a.tscale = tscale;
       a.seg = seg; a.groups = groups;
+      a.partial = (float *)((uint8_t *)planes + small_bytes);
       e = seg ? launch_cfg<3, false, true>(tw, tb, td, pm, a, s) : three ? launch_cfg<3, false>(tw, tb, td, pm, a, s) : launch_cfg<2, false>(tw, tb, td, pm, a, s);
+      if (e == cudaSuccess && a.parts > 1) e = launch_join(a, s);
     }
   }
   const cudaError_t ef = cudaFreeAsync(planes, s);
@@ -1142,7 +1241,24 @@ cudaError_t launch_gemm_w4a16(const GemmArgs &g, cudaStream_t s) {
       ++pm.n;
     }
   }
-  return g.B.dtype == NVFP4A_FP16 ? launch_cfg<1, true>(tw, tb, td, pm, a, s) : launch_cfg<1, false>(tw, tb, td, pm, a, s);
+  auto go = [&]() { return g.B.dtype == NVFP4A_FP16 ? launch_cfg<1, true>(tw, tb, td, pm, a, s) : launch_cfg<1, false>(tw, tb, td, pm, a, s); };
+  if (a.parts > 1) {
+    // Scratch from the pool; without it, or in a capture (a graph with memory nodes cannot be a child of another, nor be instantiated twice), k stays whole.
+    cudaMemPool_t pool;
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusActive;
+    if (cudaStreamIsCapturing(s, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone || planes_pool(&pool) != cudaSuccess ||
+        cudaMallocFromPoolAsync((void **)&a.partial, (size_t)a.parts * g.n * g.m * sizeof(float), pool, s) != cudaSuccess) {
+      (void)cudaGetLastError();
+      GemmArgs whole = g;
+      whole.no_alloc = 1;
+      if (!set_up(whole, 1, g.B.dtype == NVFP4A_FP16, 0, g.B.data, (uint64_t)g.k * 2, (uint64_t)g.B.ld * 2, &a, &tw, &tb, &td)) return cudaErrorInvalidValue;
+    }
+  }
+  if (a.parts == 1) return go();
+  cudaError_t e = go();
+  if (e == cudaSuccess) e = launch_join(a, s);
+  const cudaError_t ef = cudaFreeAsync(a.partial, s);
+  return e != cudaSuccess ? e : ef;
 }
 
 }  // namespace nvb

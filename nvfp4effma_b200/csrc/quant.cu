@@ -676,11 +676,12 @@ __global__ void __launch_bounds__(256) quant_dual_kernel(const uint8_t *__restri
     const bool words = (bpr & 3) == 0 && (orow.sld & 3) == 0 && ((uintptr_t)orow.sc & 3) == 0;
     const int blk = tid & 3, cb = (c0 >> 4) + blk;
     const uint64_t drop = l2_policy_evict_first();
+    const bool wide = ((uintptr_t)src & 31) == 0 && ((size_t)lds * EB & 31) == 0;
 #pragma unroll
     for (int h = 0; h < TR / 64; ++h) {
       const int lr = h * 64 + (tid >> 2), r = r0 + lr;
       const bool live = r < rows && cb < bpr;
-      const PackedBlock<T> b = load_block<T>(src + ((size_t)r * lds + 16 * cb) * EB, live, drop);
+      const PackedBlock<T> b = load_block<T>(src + ((size_t)r * lds + 16 * cb) * EB, live, drop, wide);
       uint4 *d = (uint4 *)(tile + (size_t)(lr * 64 + 16 * blk) * EB);
 #pragma unroll
       for (int q = 0; q < EB; ++q) d[q] = b.w[q];   // 16 values: EB 16-byte words

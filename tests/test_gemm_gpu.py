@@ -1090,3 +1090,48 @@ def test_w4a8_of_9_to_63_tokens_is_summed_in_segments(k):
     assert abs(float(amax.double()) / float(want.max()) - 1.0) <= (16 + 16 + 4) * 2.0 ** -24
     assert torch.allclose(D.double(), want, rtol=2.0 ** -8, atol=0.0)
     assert kernel_status() == 0
+
+
+@pytest.mark.parametrize("bt", [L.BF16, L.FP16, L.INT8])
+def test_long_reductions_of_few_tiles_in_parts_of_k(bt):
+    """Few tiles and a long k: several CTA pairs take a run of k each, a small kernel adds their sums and runs the plain epilogue.  Every layout, runs of unequal
+    length, odd numbers of stages, tails in m and n, bias, beta, every output type and amax; the same bytes on every call; and, captured in a graph
+    (where BF16 and FP16 keep k whole), the bound again."""
+    for i, (m, n, k) in enumerate([(512, 33, 8192), (130, 9, 4160), (300, 200, 6144 + 64), (700, 64, 4096 + 448), (128, 130, 16384)]):
+        for fa, out in ((0, L.BF16), (SW, L.FP16), (AM | PR, L.FP32)):
+            if bt == L.FP16 and out == L.FP32 or bt == L.INT8 and n < 64 and out == L.FP32:
+                continue      # (other kernels)
+            c = Case(m, n, k, bt, out, out if i % 2 else -1, L.BF16 if i % 2 else -1, 1.25, 0.5 if i % 2 else 0.0, fa=fa)
+            h = build_case(c, 5000 + i)
+            exp = oracle_case(c, h, want_ref=True)
+            got, amax = run_gemm(c, h)
+            assert L.lib.nvfp4a_b200_last_route() == (8 if bt == L.INT8 else 5), c
+            check_bound(c, h, got, amax, exp)
+            again, amax2 = run_gemm(c, h)
+            assert np.array_equal(got.view(np.uint8), again.view(np.uint8)) and amax == amax2, c
+            if bt == L.INT8:
+                got, amax = run_tc(c, h, gemv=False)
+                check_bound(c, h, got, amax, exp)
+    dA = DevFp4(h["A"])
+    keepB, tB = device_b(c, h)
+    dD = dev(h["Dinit"])
+    tA, tD = dA.tensor(), tensor(dD, c.dt)
+    dC = dev(h["C"]) if h["C"] is not None else None
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        assert L.lib.nvfp4a_gemm(c.m, c.n, c.k, c.alpha, ctypes.byref(tA), h["lda"], ctypes.byref(tB), h["ldb"], 0.0, None, 0, ctypes.byref(tD), h["ldd"], None, stream()) == 0
+    graph.replay()
+    torch.cuda.synchronize()
+    assert c.beta == 0.0 and c.bias < 0
+    if bt == L.BF16:      # nvfp4a_gemm_ex keeps k whole: the bytes of the entry that must not allocate
+        outs, ex = [], L.Epilogue()
+        for entry in (L.lib.nvfp4a_gemm_ex, L.lib.nvfp4a_b200_gemm_ex_static):
+            d = torch.zeros(c.n, c.m, dtype=torch.bfloat16, device="cuda")
+            td = tensor(d, L.BF16)
+            A0 = DevFp4(rand_fp4(np.random.default_rng(1), c.m, c.k, glob=0.375))
+            ta = A0.tensor()
+            L.check(entry(c.m, c.n, c.k, 1.0, ctypes.byref(ta), c.k, ctypes.byref(tB), h["ldb"], 0.0, None, 0, ctypes.byref(td), c.m, None, ctypes.byref(ex), stream()))
+            outs.append(d.view(torch.int16))
+        assert torch.equal(*outs) and bool(outs[0].any())
+    check_bound(c, h, host(dD).view(h["Dinit"].dtype), exp["amax"], exp)
+    assert kernel_status() == 0
