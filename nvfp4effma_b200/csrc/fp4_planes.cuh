@@ -1,4 +1,5 @@
-// BF16 activations -> FP4 digit planes, for the GEMVs on the FP4 tensor cores (gemv_fp4.cu, gemv_fp4_n8.cu).
+// What the GEMVs on the FP4 tensor cores (gemv_fp4.cu, gemv_fp4_n8.cu) share: BF16 activations as FP4 digit planes, and block scales that the
+// tensor cores do not take as this library does.
 //
 // An activation is the 32-bit integer X = |x| * 2^(158 - eb), eb the largest biased exponent of its token in the CTA's range of k; plane d holds
 // sign(x) * digit d of X to the base 4, the digits 0 .. 3 as the E2M1 codes of 0, 0.5, 1, 1.5.
@@ -9,7 +10,7 @@
 // an integer; the bytes of the even and of the odd values of a group of eight are transposed by byte permutes (8 each), after which the
 // digits of four values are a mask away from their places in the plane's word: nibble 2 j is even value j, nibble 2 j + 1 odd value j.
 #pragma once
-#include "common.cuh"
+#include "operands.cuh"
 
 namespace nvb {
 
@@ -54,6 +55,15 @@ __device__ __forceinline__ uint32_t planes_lost_bits(const uint4 &x, int eb) {
   return lost;
 }
 
+// what the planes drop of value i of the eight (0 if nothing): x less its bits from the last plane up
+__device__ __forceinline__ float planes_rest(const uint4 &x, int i, int eb) {
+  const uint32_t h = ((i < 2 ? x.x : i < 4 ? x.y : i < 6 ? x.z : x.w) >> (16 * (i & 1))) & 0xFFFFu;
+  const float v = __uint_as_float(h << 16), a = fabsf(v);
+  const uint32_t X = __float2uint_rz(__fmul_rn(a, __int_as_float((158 - eb + 127) << 23)));
+  const float rest = __fsub_rn(a, __fmul_rn(__fmul_rn((float)X, 0x1p-31f), __int_as_float(eb << 23)));   // (X below 2^8 or without lost bits: exact)
+  return v < 0.f ? -rest : rest;
+}
+
 // word d of the sixteen planes of eight consecutive values; scale = 2^(158 - eb)
 __device__ __forceinline__ void planes_of_8(const uint4 &x, float scale, uint32_t (&word)[16]) {
   const uint32_t w[4] = {x.x, x.y, x.z, x.w};
@@ -90,6 +100,40 @@ __device__ __forceinline__ void planes_of_8(const uint4 &x, float scale, uint32_
 __device__ __forceinline__ void store_planes(uint8_t *base, int b, const uint32_t (&word)[16]) {
 #pragma unroll
   for (int d = 0; d < 16; ++d) *(uint32_t *)(base + (d >> 3) * 1024 + (d & 7) * 128 + (b ^ ((d & 7) << 4))) = word[d];
+}
+
+// The tensor cores take block scales as unsigned: a negative code's sign moves into the block's sixteen weights.  `st`: a stage's nibbles, 256
+// rows of 128 bytes with the 128-byte swizzle; `sf`: this lane's 16 bytes of the stage's first scale tile (word q of tile (h, j): blocks 4 j ..
+// 4 j + 3 of row 128 h + 32 q + lane).
+__device__ __forceinline__ void move_signs(uint8_t *st, uint8_t *sf, int lane) {
+#pragma unroll 1
+  for (int i = 0; i < 32; ++i) {
+    uint32_t *const wp = (uint32_t *)(sf + (i >> 4) * 2048 + ((i >> 2) & 3) * 512) + (i & 3);
+    const uint32_t w = *wp;
+    const int row = (i >> 4) * 128 + (i & 3) * 32 + lane;
+    for (int b = 0; b < 4; ++b)
+      if (w >> (8 * b + 7) & 1u) {
+        const int jj = (i & 12) + b;   // block of 16 weights within the chunk
+        uint2 *const nib = (uint2 *)(st + (row >> 3) * 1024 + (row & 7) * 128 + (((jj >> 1) ^ (row & 7)) << 4) + (jj & 1) * 8);
+        *nib = make_uint2(nib->x ^ 0x88888888u, nib->y ^ 0x88888888u);
+      }
+    *wp = w & 0x7F7F7F7Fu;
+  }
+}
+
+// Block scale code 0x7F (with either sign) is 480 everywhere in this library, as in the reference's decode; the tensor cores take it for a NaN, which
+// reaches the partial sums of that weight row and of no other (activations and weights are finite here).  Such a row's sum over the CTA's
+// blocks [b0, b1) on the CUDA cores, from memory, in the order of the CUDA-core consumer below; never met in a matrix that a quantizer made from finite
+// values.  (Inlined: as a function it costs every launch 4 us.)
+__device__ __forceinline__ float code_7f_sum(const Fp4Operand &A, const uint16_t *x, int row, int b0, int b1) {
+  float acc = 0.f;
+  for (int b = b0; b < b1; ++b) {
+    const uint2 w = A.block(row, b);
+    float part = 0.f;
+    for (int i = 0; i < 16; ++i) part = __fmaf_rn((float)e2m1_x2(((i < 8 ? w.x : w.y) >> (4 * (i & 7))) & 15u), __uint_as_float((uint32_t)x[16 * b + i] << 16), part);
+    acc = __fmaf_rn(__fmul_rn(A.scale(row, b), 0.5f), part, acc);
+  }
+  return acc;
 }
 
 }  // namespace nvb

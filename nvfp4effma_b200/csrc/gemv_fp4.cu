@@ -7,7 +7,8 @@
 //
 // The BF16 activations become FP4 operands by an exact digit expansion.  For one token and the k range of one CTA let eb be
 // the largest biased exponent; every |x_i| is written as X_i * 2^(eb - 158) with the 32-bit integer X_i (for BF16, whose
-// significand has 8 bits, this is exact unless |x_i| < 2^-24 max|x|: such elements lose their bits below 2^-31 max|x|).
+// significand has 8 bits, this is exact unless |x_i| < 2^-24 max|x|: what the planes drop of such
+// elements -- a handful, usually -- each thread adds to its weight row by itself; more than 64 of them, Inf or NaN: the CUDA cores consume the weights).
 // X_i = sum over d of t_d(i) * 4^d with the base-4 digits t_d in {0, 1, 2, 3}; the E2M1 codes 0..3 are the values t / 2, so
 // "piece" d of the token is the FP4 vector sign(x_i) * t_d(i) / 2 and
 //     sum_i a_i x_i = 2^(eb - 157) * sum_d 4^d * (sum_i a_i * piece_d(i)).
@@ -32,7 +33,9 @@
 //
 // Semantics: FP32 accumulation in the tensor cores' order, within the FP32 accumulation bound of the exact definition
 // (reference include/nvfp4effma.h:82-92 there), as the reference's own tensor-core GEMV (src/tensors/gemv_tc.cuh there).
-// Block scales are consumed as unsigned E4M3.
+// Negative block scales keep their sign and the codes 0x7F / 0xFF are +-480, as in the mma.sync GEMV (gemv.cu) that takes the calls this kernel leaves:
+// the tensor cores know neither, and rows that have one are summed on the CUDA cores.
+#include <math.h>
 #include <atomic>
 #include "operands.cuh"
 #include "sm100.cuh"
@@ -48,6 +51,7 @@ namespace {
 struct GemvFp4Args {
   int m, n, k;
   int a_image;
+  Fp4Operand A;        // (weights by themselves: code_7f_sum, the rests of activations)
   const uint8_t *sa;   // plain: block scale base; image: image base
   int sa_ld, ktiles;
   int linear;          // plain operand with linear block scales: a TMA box brings [256 rows][16 bytes], four warps re-tile it
@@ -63,15 +67,16 @@ struct GemvFp4Args {
   int piece_bytes;     // shared memory of the activation pieces: chunks per CTA x piece rows x 128
 };
 
-constexpr int kThreads = 320, kDecompThreads = 256;
+constexpr int kThreads = 384, kDecompThreads = 256;         // warps 0, 1: copies, MMAs; 2-9: pieces and epilogue; 10, 11: signs of block scales
 constexpr int kRows = 256;                                  // weight rows per tile (the MMA's N)
 constexpr int kDataBytes = kRows * 128, kSfBytes = kRows * 16, kStageBytes = kDataBytes + kSfBytes;  // 36 KiB per 256-k chunk
 constexpr int kMaxChunks = 16;                              // 256-k chunks per CTA: 4096 values of k
 constexpr int kTmemCols = 512;                              // accumulator [0, 256), A scales (1.0) [256, 260), B scales [272, 272 + 32 * stages), stages <= 6
 constexpr int kMaxStages = 6;
-constexpr int kSmemLimit = 232448 - 1024;                   // dynamic shared memory of one CTA on sm_100, less the alignment slack
+constexpr int kSmemLimit = 232448 - 1024 - 1280;            // dynamic shared memory of one CTA on sm_100, less the alignment slack and the static arrays
 constexpr unsigned kStWaitFull = 0x201, kStWaitEmpty = 0x202, kStWaitAcc = 0x203, kStWaitPieces = 0x204, kStWaitRetile = 0x205;
 constexpr int kRawSfBytes = kRows * 16;                      // linear scales of one chunk as they lie in memory: [256 rows][16 bytes]
+constexpr int kRests = 64;
 
 // Shared memory of a CTA: [pieces | stages x 36 KiB | unit scales 512 | results splits x NTOK x 256 floats | barriers 256].
 // The MMA reads 16 KiB from the start of a pieces chunk (its M is 128 rows), which stays inside the stages.
@@ -95,11 +100,16 @@ gemv_fp4_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
   float *res = (float *)(unit_sf + 512);                   // [splits][NTOK][256]: slot p is written by the cluster's rank p (into rank 0's memory)
   uint64_t *bars = (uint64_t *)(unit_sf + 512 + splits * NTOK * 1024);
   uint64_t *full = bars, *empty = bars + kMaxStages, *sf_ready = bars + 2 * kMaxStages, *acc_full = bars + 3 * kMaxStages, *pieces_ready = acc_full + 1;
-  uint32_t *tmem_slot = (uint32_t *)(pieces_ready + 1);
+  uint64_t *scan_done = pieces_ready + 1;
+  uint32_t *tmem_slot = (uint32_t *)(scan_done + 1);
   volatile int *abort_flag = (volatile int *)(tmem_slot + 1);
   uint32_t *wmax = tmem_slot + 2;                          // [8 warps][NTOK] largest |x| bit pattern
   volatile int *inexact = (volatile int *)(wmax + 8 * NTOK);   // some activation of this CTA does not fit the digit planes
   int *consumed = (int *)(wmax + 8 * NTOK + 1);                // [stage] warps done with the stage (the CUDA-core consumer)
+  // Activations of which the planes drop bits, up to kRests of them: (token << 16 | k within the CTA) and what is dropped, as found and in order
+  __shared__ int rest_n, rest_key[2][kRests];
+  __shared__ float rest_val[2][kRests];
+  __shared__ uint32_t negative_row[8];   // rows with a negative block scale (not linear)
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int gm = g.m, gn = g.n;
@@ -143,11 +153,14 @@ gemv_fp4_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
   if (threadIdx.x == 0) {
     prefetch_tensormap(&tmap_a);
     if (a_image || linear) prefetch_tensormap(&tmap_s);
-    for (int s = 0; s < kStages; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); mbar_init(&sf_ready[s], 1); }
+    for (int s = 0; s < kStages; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], linear ? 1 : 2); mbar_init(&sf_ready[s], 1); }
+    mbar_init(scan_done, 2);
     mbar_init(acc_full, 1);
     mbar_init(pieces_ready, kDecompThreads / 32);
     *abort_flag = 0;
     *inexact = 0;
+    rest_n = 0;
+    for (int q = 0; q < 8; ++q) negative_row[q] = 0;
     for (int s = 0; s < kStages; ++s) consumed[s] = 0;
     fence_barrier_init();
   }
@@ -164,7 +177,7 @@ gemv_fp4_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
   // the decomposition warps ask for their activations first: the loads fly while the barrier below gathers the CTA
   const int t2 = threadIdx.x - 64, nvec = nloc * 32;  // vectors of 8 consecutive k; at most 2 per thread and token
   uint4 xq[NTOK][2];
-  if (warp >= 2) {
+  if (warp >= 2 && warp < 10) {
 #pragma unroll
     for (int t = 0; t < NTOK; ++t)
 #pragma unroll
@@ -191,10 +204,73 @@ gemv_fp4_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
 
   // rank 0 runs the epilogue, one thread per weight row; its operands are fetched once the pieces are built, far ahead of their use
   const int erow = t2, ei = tm * 256 + erow;
-  const bool erow_ok = warp >= 2 && rank == 0 && ei < gm;
+  const bool erow_ok = warp >= 2 && warp < 10 && rank == 0 && ei < gm;
   float e_rowp = 0.f, e_bias = 0.f, e_c[NTOK];
 #pragma unroll
   for (int t = 0; t < NTOK; ++t) e_c[t] = 0.f;
+
+  // Linear block scales [256 rows][16 bytes] of the stages w, w + 4, ... -> the eight 512-byte tiles of the stage; signs go to the weights (the tensor cores
+  // take scales as unsigned).  A stage belongs to one warp for the whole launch: a wait on the parity of fill f is only meaningful to a
+  // thread that has seen fill f - 1 complete (on a barrier still in its first phase, a wait for the second fill's parity returns at once).
+  auto retile = [&](int w) {
+    for (int it = 0; it < nloc; ++it) {
+      const int s = it % kStages;
+      if ((s & 3) != w) continue;
+      if (!__all_sync(0xFFFFFFFFu, wait(&full[s], (it / kStages) & 1, kStWaitRetile))) break;
+      uint8_t *st = stages + (size_t)s * stage_bytes;
+      const uint8_t *raw = st + kStageBytes;
+      uint8_t *sf = st + kDataBytes + lane * 16;
+      uint32_t any = 0;
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          uint32_t wd[4];
+#pragma unroll
+          for (int q = 0; q < 4; ++q) wd[q] = *(const uint32_t *)(raw + (h * 128 + 32 * q + lane) * 16 + 4 * j);
+          *(uint4 *)(sf + h * 2048 + j * 512) = make_uint4(wd[0], wd[1], wd[2], wd[3]);
+          any |= wd[0] | wd[1] | wd[2] | wd[3];
+        }
+      if (__any_sync(0xFFFFFFFFu, any & 0x80808080u)) move_signs(st, sf, lane);
+      fence_proxy_async_smem();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&sf_ready[s]);
+    }
+  };
+  // Tiled block scales go to the tensor cores as they are.  Two warps look for negative codes beside the MMAs (waiting for them cost 28672 x 4096 with one vector
+  // 0.6 us: a stage was held longer); a weight row that has one is summed on the CUDA cores at the end.
+  auto scan = [&](int w) {
+    for (int it = 0; it < nloc; ++it) {
+      const int s = it % kStages;
+      if ((s & 1) != w) continue;
+      if (!__all_sync(0xFFFFFFFFu, wait(&full[s], (it / kStages) & 1, kStWaitRetile))) break;
+      const uint8_t *sf = stages + (size_t)s * stage_bytes + kDataBytes + lane * 16;   // word q of tile (h, j): row 128 h + 32 q + lane
+      uint4 any[2];
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        any[h] = make_uint4(0, 0, 0, 0);
+        if (h == 0 || second || a_image) {   // (else nothing was copied here)
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const uint4 v = *(const uint4 *)(sf + h * 2048 + j * 512);
+            any[h].x |= v.x; any[h].y |= v.y; any[h].z |= v.z; any[h].w |= v.w;
+          }
+        }
+      }
+      if (__any_sync(0xFFFFFFFFu, (any[0].x | any[0].y | any[0].z | any[0].w | any[1].x | any[1].y | any[1].z | any[1].w) & 0x80808080u)) {
+        const uint32_t wd[8] = {any[0].x, any[0].y, any[0].z, any[0].w, any[1].x, any[1].y, any[1].z, any[1].w};
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+          const uint32_t rows = __ballot_sync(0xFFFFFFFFu, (wd[q] & 0x80808080u) != 0);
+          if (lane == 0 && rows) atomicOr(&negative_row[q], rows);
+        }
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&empty[s]);
+    }
+    __syncwarp();
+    if (lane == 0) mbar_arrive(scan_done);
+  };
 
   // The ring's first fill, one stage per warp: a copy instruction is slow to issue (see request_stage), and the decomposition
   // warps among these have nothing to do until their activations arrive.
@@ -242,6 +318,8 @@ gemv_fp4_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
         if (ok) tc_commit_elect(acc_full);
       }
     }
+  } else if (warp >= 10) {
+    if (!linear) scan(warp - 10);
   } else {
     // ---------------- 8 warps: activations -> FP4 pieces in shared memory ----------------
     const int w2 = warp - 2;
@@ -271,7 +349,16 @@ gemv_fp4_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
       const int eb = t ? ebs[NTOK - 1] : ebs[0];
       uint32_t word[16];
       planes_of_8(xv, pow2f(158 - eb), word);
-      lost |= planes_lost_bits(xv, eb);
+      if (eb != 255 && planes_lost_bits(xv, eb)) {
+#pragma unroll 1
+        for (int q = 0; q < 8; ++q) {
+          const float rest = planes_rest(xv, q, eb);
+          if (rest == 0.f) continue;
+          const int at = atomicAdd(&rest_n, 1);
+          if (at < kRests) { rest_key[0][at] = t << 16 | (8 * v + q); rest_val[0][at] = rest; }
+          else lost = 1;
+        }
+      }
       store_planes(pieces + (size_t)(v >> 5) * (PR * 128) + t * 2048, (v & 31) * 4, word);
     }
     if (lost) *inexact = 1;
@@ -280,6 +367,30 @@ gemv_fp4_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
     if (lane == 0) mbar_arrive(pieces_ready);
     named_barrier(3, kDecompThreads);   // every warp's verdict is in
     const bool exact = *inexact == 0;
+    // the rests in the order of k (they were found in any): a handful, met where activations spread over more than 2^24 (products, usually)
+    const int rests = exact ? rest_n : 0;
+    if (rests) {
+      if (t2 < rests) {
+        const int key = rest_key[0][t2];
+        int at = 0;
+        for (int q = 0; q < rests; ++q) at += rest_key[0][q] < key;
+        rest_key[1][at] = key;
+        rest_val[1][at] = rest_val[0][t2];
+      }
+      named_barrier(2, kDecompThreads);
+    }
+    auto rest_sum = [&](int t) {   // of this thread's weight row
+      float acc = 0.f;
+#pragma unroll 1
+      for (int q = 0; q < rests; ++q) {
+        const int kk = c0 * 256 + (rest_key[1][q] & 0xFFFF);
+        if (rest_key[1][q] >> 16 != t) continue;
+        const uint2 w = g.A.block(ei, kk >> 4);
+        const int nib = (kk & 8 ? w.y : w.x) >> (4 * (kk & 7)) & 15u;
+        acc = __fmaf_rn(__fmul_rn(__fmul_rn(g.A.scale(ei, kk >> 4), 0.5f), (float)e2m1_x2((uint32_t)nib)), rest_val[1][q], acc);
+      }
+      return acc;
+    };
     if (erow_ok) {
       e_rowp = epi_row_part(g.e, ei);
       if (g.e.bias) e_bias = load_dense(g.e.bias_dtype, g.e.bias, ei);
@@ -330,7 +441,7 @@ gemv_fp4_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
 #pragma unroll
           for (int b = 0; b < 2; ++b) {
             const int jj = 2 * u16 + b;   // block of 16 values within the chunk
-            const float sc = __fmul_rn(e4m3_to_f32((linear ? sfp[jj] : sfp[(jj >> 2) * 512 + (jj & 3)]) & 0x7Fu), 0.5f);
+            const float sc = __fmul_rn(e4m3_to_f32(linear ? sfp[jj] : sfp[(jj >> 2) * 512 + (jj & 3)]), 0.5f);
 #pragma unroll
             for (int t = 0; t < NTOK; ++t) {
               const float *xv = xs + (size_t)t * nloc * 256 + (size_t)it * 256 + jj * 16;
@@ -377,36 +488,13 @@ gemv_fp4_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
           }
       }
     }
-    if (exact && linear && (warp & 3) != 0 && warp >= 5) {
-      // ---------------- warps 5, 6, 7, 9: linear block scales [256 rows][16 bytes] -> the eight 512-byte tiles of the stage ----------------
-      // A stage belongs to one warp for the whole launch: a wait on the parity of fill f is only meaningful to a thread that
-      // has seen fill f - 1 complete (on a barrier still in its first phase, a wait for the second fill's parity returns at once).
-      const int w = warp == 9 ? 3 : warp - 5;
-      for (int it = 0; it < nloc; ++it) {
-        const int s = it % kStages;
-        if ((s & 3) != w) continue;
-        if (!wait(&full[s], (it / kStages) & 1, kStWaitRetile)) break;
-        uint8_t *st = stages + (size_t)s * stage_bytes;
-        const uint8_t *raw = st + kStageBytes;
-        uint8_t *sf = st + kDataBytes;
-#pragma unroll
-        for (int h = 0; h < 2; ++h)
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            uint32_t wd[4];
-#pragma unroll
-            for (int q = 0; q < 4; ++q) wd[q] = *(const uint32_t *)(raw + (h * 128 + 32 * q + lane) * 16 + 4 * j);
-            *(uint4 *)(sf + h * 2048 + j * 512 + lane * 16) = make_uint4(wd[0], wd[1], wd[2], wd[3]);
-          }
-        fence_proxy_async_smem();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&sf_ready[s]);
-      }
-    }
+    // linear block scales: warps 5, 6, 7, 9, once the verdict on the activations is in (the CUDA-core consumer reads the scales as they came)
+    if (exact && linear && (warp & 3) != 0 && warp >= 5) retile(warp == 9 ? 3 : warp - 5);
     if (exact) {
       // ---------------- all eight warps: each thread sums the sixteen pieces of its weight row and hands the result to rank 0 ----------------
       // (the order of the additions is that of a butterfly over the piece pairs)
       named_barrier(3, kDecompThreads);
+      const bool negative = !linear && wait(scan_done, 0, kStWaitRetile) && (negative_row[t2 >> 5] >> (t2 & 31) & 1u);
       if (nloc > 0 && !*abort_flag) {
 #pragma unroll
         for (int t = 0; t < NTOK; ++t) {
@@ -414,8 +502,10 @@ gemv_fp4_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
           const float sum = __fadd_rn(__fadd_rn(__fadd_rn(v[0], v[1]), __fadd_rn(v[2], v[3])), __fadd_rn(__fadd_rn(v[4], v[5]), __fadd_rn(v[6], v[7])));
           const int ex = ebs[t] - 157, e1 = max(ex, -100);
           const float s1 = pow2f(e1), s2 = pow2f(ex - e1);
-          const bool bad = ebs[t] == 255;  // Inf or NaN among the activations
-          st_peer_f32(&res[(rank * NTOK + t) * 256 + t2], 0, bad ? __int_as_float(0x7FC00000) : __fmul_rn(__fmul_rn(sum, s1), s2));
+          float r = __fmul_rn(__fmul_rn(sum, s1), s2);
+          if ((sum != sum || negative) && ei < gm) r = code_7f_sum(g.A, x + (size_t)t * g.ldx, ei, 16 * c0, 16 * c1);
+          else if (rests && ei < gm) r = __fadd_rn(r, rest_sum(t));   // (code_7f_sum is over the activations themselves)
+          st_peer_f32(&res[(rank * NTOK + t) * 256 + t2], 0, r);
         }
       }
     }
@@ -429,7 +519,7 @@ gemv_fp4_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
     cluster_arrive_release();
     if (rank == 0) cluster_wait_acquire();
   }
-  if (rank == 0 && warp >= 2 && !*abort_flag) {
+  if (rank == 0 && warp >= 2 && warp < 10 && !*abort_flag) {
     const Epilogue &e = g.e;
     const int mask = g.ex.mask, row = erow, i = ei;
     const bool row_ok = erow_ok;
@@ -492,22 +582,27 @@ static std::atomic<int> g_gemv_splits{0};  // 0 = automatic
 void set_gemv_fp4_splits(int s) { g_gemv_splits = s; }
 int gemv_fp4_pinned_splits() { return g_gemv_splits.load(); }
 
-// splits: power of two, at most 8 and nk; every CTA's k range is at most kMaxChunks chunks (its pieces' shared memory).
-// Pinned (nvfp4a_b200_set_gemv_splits): that value if the problem can use it.  Automatic: this kernel pays about 5 us of
-// set-up and tail per launch (pieces, cluster, two-step epilogue), so it takes only problems that stream at least 32 MB of
-// weights over at least 96 CTAs; smaller ones go to the mma.sync GEMV.  Returns 0 when the kernel should not run.
-static int choose_splits(int m, int k) {
-  const int nk = k >> 8, tiles = (m + kRows - 1) / kRows;
-  const int need = (nk + kMaxChunks - 1) / kMaxChunks;
-  int s = 1;
-  while (s < need) s *= 2;
-  if (const int f = g_gemv_splits.load()) {
-    return (f >= s && f <= 8 && f <= nk && !(f & (f - 1))) ? f : 0;
+// splits: power of two, at most 8 and nk; every CTA's k range is at most kMaxChunks chunks (its pieces' shared memory).  Returns 0 when the
+// kernel should not run.  Pinned (nvfp4a_b200_set_gemv_splits): that value if the problem can use it.  Automatic: the cut with the shortest
+// estimate, if that beats the mma.sync GEMV (3 us and 0.4 us per megabyte: it decodes weights on the CUDA cores).  The estimate: 3.4 us of set-up and tail,
+// 4.3 / 4.9 / 5.5 in a cluster of 2 / 4 / 8, and the stream, 36 KiB per chunk at 67 GB/s per CTA or 5.6 TB/s in all.  CUDA-graph timings of one
+// vector, here and there: 6144 x 4096 7.9 against 8.8 us, 4096 x 14336 12.5 against 17.5, 28672 x 4096 15.4 against 30.3; but 4096 x 4096 6.95 against 7.0 and 1024 x 1024 4.0 against 3.1: the first has no winner, so a tenth of
+// advantage is asked for.
+static int choose_splits(int m, int k, int n) {
+  const int nk = k >> 8, tiles = (m + kRows - 1) / kRows, sms = device_sms();
+  auto fits = [&](int s) { return s <= nk && (nk + s - 1) / s <= kMaxChunks; };
+  if (const int f = g_gemv_splits.load()) return fits(f) ? f : 0;
+  int best = 0;
+  double best_us = 0.9 * (3.0 + 0.405 * (m * (k * 0.5625e-6)));
+  for (int s = 1; s <= 8; s *= 2) {
+    if (!fits(s)) continue;
+    const int cap = s == 1 ? sms : s == 2 ? sms / 2 : s == 4 ? sms * 33 / 148 : sms * 15 / 148;   // clusters that run at once (see gemv_fp4_n8.cu)
+    const int rounds = (tiles + cap - 1) / cap, ctas = (tiles < cap ? tiles : cap) * s;
+    const double chunk = fmax(0.55, ctas * 36.9e3 / 5.6e6) + 0.08 * (n - 1);
+    const double us = (s == 1 ? 3.4 : s == 2 ? 4.3 : s == 4 ? 4.9 : 5.5) + rounds * ((nk + s - 1) / s) * chunk;
+    if (us < best_us) { best = s; best_us = us; }
   }
-  if (s > 4 || s > nk) return 0;
-  while (s * 2 <= 4 && nk / (s * 2) >= 8 && tiles * s * 2 <= device_sms()) s *= 2;
-  if (tiles * s < 96 || (double)m * k * 0.5625 < 32e6) return 0;
-  return s;
+  return best;
 }
 
 bool gemv_fp4_supports(const GemmArgs &g) {
@@ -515,7 +610,7 @@ bool gemv_fp4_supports(const GemmArgs &g) {
   if (((uintptr_t)g.B.data & 15) || g.B.ld % 8) return false;
   // plain operands: scales in aligned 512-byte tiles (the swizzled layout), or linear with a 16-byte aligned base and pitch (TMA)
   if (!g.A.image && (((uintptr_t)g.A.data & 15) || g.A.ld % 32 || ((uintptr_t)g.A.sc & 15) || (g.A.sld > 0 && g.A.sld % 16))) return false;
-  return choose_splits(g.m, g.k) > 0;
+  return choose_splits(g.m, g.k, g.n) > 0;
 }
 
 cudaError_t launch_gemv_fp4(const GemmArgs &g, cudaStream_t s) {
@@ -532,6 +627,7 @@ cudaError_t launch_gemv_fp4(const GemmArgs &g, cudaStream_t s) {
   }
   a.ktiles = (g.k + kImgK - 1) / kImgK;
   a.a_image = g.A.image;
+  a.A = g.A;
   CUtensorMap ta, ts;
   memset(&ts, 0, sizeof ts);
   if (g.A.image) {
@@ -544,7 +640,7 @@ cudaError_t launch_gemv_fp4(const GemmArgs &g, cudaStream_t s) {
     a.linear = g.A.sld > 0;
     if (a.linear && !make_tmap_dense(&ts, g.A.sc, 4, (uint64_t)g.k / 64, (uint64_t)g.m, (uint64_t)g.A.sld, 4, kRows)) return cudaErrorInvalidValue;
   }
-  const int splits = choose_splits(g.m, g.k);
+  const int splits = choose_splits(g.m, g.k, g.n);
   if (splits <= 0) return cudaErrorInvalidValue;
   void (*kern)(CUtensorMap, CUtensorMap, GemvFp4Args) = g.n == 1 ? gemv_fp4_kernel<1> : gemv_fp4_kernel<2>;
   static std::atomic<bool> attr_set[64][2];   // zero-initialised; set once per device and kernel

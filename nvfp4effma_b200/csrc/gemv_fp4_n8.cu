@@ -89,21 +89,6 @@ __host__ __device__ constexpr int fixed_bytes(int ntok, int buffers) { return 51
 
 __device__ __forceinline__ float pow2f(int e) { return __int_as_float((e + 127) << 23); }  // -126 <= e <= 127
 
-// Block scale code 0x7F (with either sign) is 480 everywhere in this library, as in the reference's decode; the tensor cores take it for a NaN, which
-// reaches the partial sums of that weight row and of no other (activations and weights are finite here).  Such a row's sum over the CTA's
-// blocks [b0, b1) on the CUDA cores, from memory, in the order of the CUDA-core consumer below; never met in a matrix that a quantizer made from finite
-// values.  (Inlined: as a function it costs every launch 4 us.)
-__device__ __forceinline__ float code_7f_sum(const Fp4Operand &A, const uint16_t *x, int row, int b0, int b1) {
-  float acc = 0.f;
-  for (int b = b0; b < b1; ++b) {
-    const uint2 w = A.block(row, b);
-    float part = 0.f;
-    for (int i = 0; i < 16; ++i) part = __fmaf_rn((float)e2m1_x2(((i < 8 ? w.x : w.y) >> (4 * (i & 7))) & 15u), __uint_as_float((uint32_t)x[16 * b + i] << 16), part);
-    acc = __fmaf_rn(__fmul_rn(A.scale(row, b), 0.5f), part, acc);
-  }
-  return acc;
-}
-
 template <int NTOK>
 __global__ void __launch_bounds__(kThreads, 1)
 gemv_fp4_n8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_s, const GemvN8Args g) {
@@ -304,21 +289,7 @@ gemv_fp4_n8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
             any |= w.x | w.y | w.z | w.w;
           }
         const bool negative = __any_sync(0xFFFFFFFFu, any & 0x80808080u);
-        if (negative) {
-#pragma unroll 1
-          for (int i = 0; i < 32; ++i) {
-            uint32_t *const wp = (uint32_t *)(sf + (i >> 4) * 2048 + ((i >> 2) & 3) * 512) + (i & 3);
-            const uint32_t w = *wp;
-            const int row = (i >> 4) * 128 + (i & 3) * 32 + lane;
-            for (int b = 0; b < 4; ++b)
-              if (w >> (8 * b + 7) & 1u) {
-                const int jj = (i & 12) + b;   // block of 16 weights within the chunk
-                uint2 *const nib = (uint2 *)(st + (row >> 3) * 1024 + (row & 7) * 128 + (((jj >> 1) ^ (row & 7)) << 4) + (jj & 1) * 8);
-                *nib = make_uint2(nib->x ^ 0x88888888u, nib->y ^ 0x88888888u);
-              }
-            *wp = w & 0x7F7F7F7Fu;
-          }
-        }
+        if (negative) move_signs(st, sf, lane);
         if (linear || negative) fence_proxy_async_smem();
         __syncwarp();
         if (lane == 0) mbar_arrive(&sf_ready[s]);

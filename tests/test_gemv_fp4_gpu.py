@@ -316,3 +316,73 @@ def test_digit_planes_at_the_edges_of_their_range(pin, spread):
         assert L.lib.nvfp4a_b200_last_route() == FP4_GEMV, c
         check_bound(c, h, got, amax, exp)
     assert kernel_status() == 0
+
+
+@pytest.mark.parametrize("layout", ["image", "swizzled", "linear"])
+def test_signed_and_largest_block_scale_codes_of_one_and_two_vectors(pin, layout):
+    """Negative block scales keep their sign and codes 0x7F / 0xFF are +-480, on the tensor cores and where the CUDA cores take over (the last size, a
+    vector spread over 2^-60 .. 1); row remainders with and without a second 128-row half."""
+    from util import rand_fp4
+    for i, (splits, m, n, k) in enumerate([(1, 300, 1, 768), (2, 515, 2, 1024), (4, 77, 2, 2048), (8, 1100, 1, 2048), (2, 300, 2, 1024)]):
+        pin(splits)
+        c = Case(m, n, k, L.BF16, L.FP32, -1, L.BF16, 1.25, 0.0, fa=SW if layout == "swizzled" else 0)
+        h = build_case(c, 1600 + i)
+        rng = np.random.default_rng(1600 + i)
+        if layout == "linear":
+            h["A"] = rand_fp4(rng, m, k, ld=h["lda"], ld_scale=k // 16, glob=0.375)
+        sc = h["A"].scales
+        sc[(rng.integers(0, 3 if i else 200, sc.size) == 0) & (sc != 0)] |= 0x80
+        if i % 2:
+            sc[rng.integers(0, sc.size, 1 + sc.size // 500)] = 0x7F
+            sc[rng.integers(0, sc.size, 1 + sc.size // 500)] = 0xFF
+        if i == 4:
+            x = rng.standard_normal((n, h["ldb"])).astype(np.float32)
+            x[1, :700] *= np.exp2(-rng.integers(0, 61, 700)).astype(np.float32)
+            h["B"] = O.Dense(L.BF16, O.from_f32(x.reshape(-1), L.BF16), h["ldb"])
+        exp = oracle_case(c, h, want_ref=True)
+        got, amax = run_tc(c, h, gemv=True) if layout == "image" else run_gemm(c, h)
+        assert L.lib.nvfp4a_b200_last_route() == FP4_GEMV, c
+        assert np.isfinite(exp["ref64"]).all()
+        check_bound(c, h, got, amax, exp)
+    assert kernel_status() == 0
+
+
+@pytest.mark.parametrize("few", [1, 7, 31, 32, 33, 40])
+def test_activations_of_which_the_planes_drop_bits(pin, few):
+    """`few` activations per vector far below the last digit plane and nothing else beside large ones that meet zero weights, so that the result is made of
+    what the planes drop: up to 64 a CTA adds by itself, more it leaves to the CUDA cores.  The same bytes on every launch."""
+    for i, (splits, n, layout) in enumerate([(1, 1, SW), (2, 2, 0), (4, 2, SW)]):
+        pin(splits)
+        m, k = 300, 4096
+        c = Case(m, n, k, L.BF16, L.FP32, -1, -1, 1.0, 0.0, fa=layout)
+        h = build_case(c, 1800 + few + i)
+        rng = np.random.default_rng(1801 + few)
+        if not layout:
+            from util import rand_fp4
+            h["A"] = rand_fp4(rng, m, k, ld=h["lda"], ld_scale=k // 16, glob=0.375)
+        big = rng.choice(k, 8, replace=False)
+        a = h["A"].data.reshape(m, h["lda"] // 2)
+        for kk in big:
+            a[:, kk // 2] &= 0xF0 if kk % 2 == 0 else 0x0F
+        x = np.zeros((n, h["ldb"]), dtype=np.float32)
+        x[:, big] = rng.choice([-1.0, 1.5], (n, big.size))
+        small = rng.choice(np.setdiff1d(np.arange(k), big), few, replace=False)
+        x[:, small] = rng.standard_normal((n, few)) * np.exp2(-rng.integers(22, 90, (n, few)))
+        h["B"] = O.Dense(L.BF16, O.from_f32(x.reshape(-1), L.BF16), h["ldb"])
+        exp = oracle_case(c, h, want_ref=True)
+        got, amax = run_gemm(c, h)
+        assert L.lib.nvfp4a_b200_last_route() == FP4_GEMV
+        check_bound(c, h, got, amax, exp)
+        for _ in range(5):
+            assert np.array_equal(run_gemm(c, h)[0].view(np.uint8), got.view(np.uint8))
+    assert kernel_status() == 0
+
+
+def test_one_vector_takes_the_tensor_cores_from_14_megabytes_up():
+    for m, k, route in ((6144, 4096, FP4_GEMV), (4096, 14336, FP4_GEMV), (1024, 1024, 2)):
+        c = Case(m, 1, k, L.BF16, L.BF16, -1, -1, 1.0, 0.0, fa=SW)
+        h = build_case(c, 1900)
+        exp = oracle_case(c, h, want_ref=True)
+        got, amax = run_gemm(c, h)
+        assert L.lib.nvfp4a_b200_last_route() == route, c
+        check_bound(c, h, got, amax, exp)
