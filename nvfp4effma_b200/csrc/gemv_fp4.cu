@@ -34,7 +34,8 @@
 // Semantics: FP32 accumulation in the tensor cores' order, within the FP32 accumulation bound of the exact definition
 // (reference include/nvfp4effma.h:82-92 there), as the reference's own tensor-core GEMV (src/tensors/gemv_tc.cuh there).
 // Negative block scales keep their sign and the codes 0x7F / 0xFF are +-480, as in the mma.sync GEMV (gemv.cu) that takes the calls this kernel leaves:
-// the tensor cores know neither, and rows that have one are summed on the CUDA cores.
+// the tensor cores know neither.  Linear scales are moved through registers anyway: their signs go into the weights there.  Rows of tiled scales that
+// have a negative code, and rows with 0x7F, are summed on the CUDA cores.
 #include <math.h>
 #include <atomic>
 #include "operands.cuh"
@@ -465,8 +466,8 @@ gemv_fp4_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
     } else if ((warp & 3) == 0) {
       // ---------------- warps 4 and 8 (tensor-memory lanes 0..31): accumulator -> shared memory, 128 weight rows each ----------------
       // A thread of the 16 x 256-bit load holds pieces d and d + 8 (d = lane / 4) of sixteen weight rows; it joins the two and
-      // leaves them in red[token][weight row][9] (the stage ring is free by now: every MMA has completed), from where all 256
-      // threads sum their row's eight values.
+      // leaves them in red[token][weight row][9] (the first stage's nibbles are free by now: every MMA has completed, and the scan
+      // reads scales only), from where all 256 threads sum their row's eight values.
       const int half = warp >> 3;  // 0: columns 0..127, 1: columns 128..255
       if (nloc > 0 && wait(acc_full, 0, kStWaitAcc)) {
         tc_fence_after();

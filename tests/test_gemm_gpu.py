@@ -1063,6 +1063,52 @@ def test_w4a16_epilogues_compiled_for_plain_calls_equal_the_general_one(bt, case
     assert kernel_status() == 0
 
 
+@pytest.mark.parametrize("bt", [L.BF16, L.INT8])
+@pytest.mark.parametrize("case", ["norm_swiglu", "out2"])
+def test_w4a16_epilogues_compiled_for_the_mlp_equal_the_general_one(bt, case):
+    """RMSNorm scale + SwiGLU and the second output with sums of squares have epilogues of their own where D has 16 bits; an FP32 D takes the general
+    one: the 16-bit D is its rounding, the other outputs and the amax are the same bytes.  With and without bias and amax, D that TMA stores or not, ragged tiles."""
+    m, n, k = 528, 300, 640
+    glu = case == "norm_swiglu"
+    gen = torch.Generator(device="cuda").manual_seed(18)
+    ints = lambda lo, hi, shape, t=torch.uint8: torch.randint(lo, hi, shape, generator=gen, device="cuda", dtype=t)
+    w, ws = ints(0, 256, (m, k // 2)), ints(0x28, 0x48, (m, k // 16))
+    ta = tensor(w, L.NVFP4, ws, k // 16)
+    if bt == L.INT8:
+        x, xs = ints(-127, 128, (n, k), torch.int8), torch.rand(n, k // 16, generator=gen, device="cuda") + 0.1
+        tb = tensor(x, L.INT8, xs, k // 16)
+    else:
+        x = torch.randn(n, k, generator=gen, device="cuda").to(torch.bfloat16)
+        tb = tensor(x, bt)
+    bias, w2 = (torch.randn(m, generator=gen, device="cuda").to(torch.bfloat16) for _ in range(2))
+    parts = torch.rand(n, 8, generator=gen, device="cuda")
+    mo = m // 2 if glu else m
+
+    def run(dt, ld, use_bias, use_amax):
+        D, amax = torch.zeros(n, ld, dtype=dt, device="cuda"), torch.zeros(1, dtype=torch.float32, device="cuda")
+        d2, sq = torch.zeros(n, m, dtype=torch.bfloat16, device="cuda"), torch.zeros(n, m // 16, dtype=torch.float32, device="cuda")
+        ex = L.Epilogue()
+        if glu:
+            ex.norm_parts, ex.norm_nparts, ex.norm_ld, ex.norm_inv_n, ex.norm_eps, ex.swiglu = parts.data_ptr(), 8, 8, 1.0 / 64.0, 1e-6, 1
+        else:
+            ex.d2, ex.d2_dtype, ex.ldd2, ex.w2, ex.w2_dtype, ex.sq, ex.ld_sq = d2.data_ptr(), L.BF16, m, w2.data_ptr(), L.BF16, sq.data_ptr(), m // 16
+        td = tensor(D, {torch.bfloat16: L.BF16, torch.float16: L.FP16, torch.float32: L.FP32}[dt], amax=amax if use_amax else None)
+        tbias = tensor(bias, L.BF16)
+        L.check(L.lib.nvfp4a_gemm_ex(m, n, k, -0.01, ctypes.byref(ta), k, ctypes.byref(tb), k, 0.0, None, 0, ctypes.byref(td), ld,
+                                     ctypes.byref(tbias) if use_bias else None, ctypes.byref(ex), stream()))
+        assert L.lib.nvfp4a_b200_last_route() == (8 if bt == L.INT8 else 5)
+        return D, d2.view(torch.int16), sq.view(torch.int32), amax.view(torch.int32)
+
+    for dt in (torch.bfloat16, torch.float16):
+        for ld in (mo, mo + 3):
+            for use in (False, True):
+                got, want = run(dt, ld, use, use), run(torch.float32, ld, use, use)
+                assert bool(want[0].any()) and torch.equal(got[0].view(torch.int16), want[0].to(dt).view(torch.int16))
+                for a, b in zip(got[1:], want[1:]):
+                    assert torch.equal(a, b)
+    assert kernel_status() == 0
+
+
 @pytest.mark.parametrize("k", [512, 576, 1088, 4096])
 def test_w4a8_of_9_to_63_tokens_is_summed_in_segments(k):
     """INT8 activations of fewer than 64 tokens (k >= 512, 16-bit D, plain epilogue): the tcgen05 kernel in segments (route 8), within the bound; sums of
