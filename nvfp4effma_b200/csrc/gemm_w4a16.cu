@@ -183,9 +183,10 @@ constexpr int kMaxGroups = 256;
 // accumulator or, at the end, the caller for the result.  28672 x 4096 with SwiGLU on 2048 tokens: 412 -> 344 us; FP16 4096 x 4096 on 333
 // tokens 37.5 -> 35.2; 5504 x 3584 with SwiGLU on 121 tokens 32.1 -> 27.0.
 // 3: no epilogue, the sums of a part of k as they are (see w4a16_join_kernel).
-// 4, 5: a transformer MLP's two calls with a 16-bit D and, at run time, an amax: RMSNorm scale and SwiGLU; second output and sums of squares.  28672 x 4096 on
-// 2048 tokens 400 -> 330 us (INT8 activations 679 -> 628), 4096 x 14336 214 -> 186.
-enum { kEpiAny = 0, kEpiPlain = 1, kEpiSwiglu = 2, kEpiPart = 3, kEpiNormGlu = 4, kEpiOut2 = 5 };
+// 4 .. 7: a 16-bit D, at run time an amax, and one of: RMSNorm scale and SwiGLU (28672 x 4096 on 2048 tokens 400 -> 330 us, INT8 activations 679 -> 628); second
+// output and sums of squares (4096 x 14336 214 -> 186); RMSNorm scale (6144 x 4096 103 -> 82; 4096 x 4096 on 100 tokens 30.3 -> 25.3); beta * C (131
+// -> 126, 32.9 -> 30.5: its two-byte loads of C remain).
+enum { kEpiAny = 0, kEpiPlain = 1, kEpiSwiglu = 2, kEpiPart = 3, kEpiNormGlu = 4, kEpiOut2 = 5, kEpiNorm = 6, kEpiAdd = 7 };
 template <int PLANES, bool F16, bool GROUPED, int EPI>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_b, const __grid_constant__ CUtensorMap tmap_d,
@@ -214,7 +215,7 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
   constexpr int kSub = PLANES == 3 ? C::kBBytes / 2 : C::kBBytes;   // bytes of a stage of one plane (three planes: tiles of at most 128 tokens)
   const int slot_bytes = (kB * C::kBBytes) >> lgB;
   constexpr bool PART = EPI == kEpiPart;
-  constexpr bool AMAX = EPI == kEpiAny || EPI == kEpiNormGlu || EPI == kEpiOut2;
+  constexpr bool AMAX = EPI == kEpiAny || EPI >= kEpiNormGlu, ADD = EPI == kEpiAny || EPI == kEpiAdd;
   const int tile_first = blockIdx.x >> 1, tile_step = gridDim.x >> 1;
   // (parts of k: a pair has one part of one tile, the stages [k0, k0 + nk))
   const int parts = PART ? g.parts : 1, k0 = PART ? tile_first % parts * g.part_stages : 0;
@@ -418,7 +419,7 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
     // (rarely used parameters are read from the constant bank where they are needed: the registers belong to the accumulator block)
     const float gb0 = !PART && g.e.gb ? *g.e.gb : 1.f;   // B's global: dense B has none, INT8 B one for the tensor (a multiply by 1 is exact)
     uint8_t *const dptr = (uint8_t *)g.e.d;
-    const int d_dtype = g.e.d_dtype, mask = EPI == kEpiSwiglu ? kExSwiglu : EPI == kEpiNormGlu ? kExNorm | kExSwiglu : EPI == kEpiOut2 ? kExOut2 : SEG || EPI == kEpiPlain || PART ? 0 : g.x.mask;   // (segments: a 16-bit D and the plain epilogue)
+    const int d_dtype = g.e.d_dtype, mask = EPI == kEpiSwiglu ? kExSwiglu : EPI == kEpiNormGlu ? kExNorm | kExSwiglu : EPI == kEpiOut2 ? kExOut2 : EPI == kEpiNorm ? kExNorm : SEG || EPI == kEpiPlain || EPI == kEpiAdd || PART ? 0 : g.x.mask;   // (segments: a 16-bit D and the plain epilogue)
     const bool d_tma = g.d_tma;
     // The accumulator is read as MMA fragments (16 lanes x 8 columns per register quad): a thread holds rows rb + 16 hh + 8 u (hh, u in
     // {0, 1}) of columns 8 gq + cp + e (e in {0, 1}) of a chunk of 32, register 16 hh + 4 gq + 2 u + e.  Gate and up rows of SwiGLU (8
@@ -600,7 +601,7 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
               float v = __fmul_rn(PLANES == 2 ? __fmul_rn(__uint_as_float(x), ts[e]) : __uint_as_float(x), sc);
               v = __fadd_rn(v, bias[q]);
               const int jj = 8 * gq + cp + e;
-              if (EPI == kEpiAny && g.e.beta != 0.f && rb + 8 * q < gm && jj < nvalid)
+              if (ADD && g.e.beta != 0.f && rb + 8 * q < gm && jj < nvalid)
                 v = __fmaf_rn(g.e.beta, load_dense(g.e.c_dtype, g.e.c, (size_t)(j0 + jj) * g.e.ldc + rb + 8 * q), v);
               x = __float_as_uint(v);
             }
@@ -914,6 +915,8 @@ cudaError_t launch_cfg(const CUtensorMap &tw, const CUtensorMap &tb, const CUten
   const bool scaled = a.e.beta == 0.f && a.e.d_dtype != NVFP4A_FP32, plain = scaled && !a.e.amax;
   if constexpr (!F16 && !GROUPED && PLANES < 3) {
     if (scaled && a.x.mask == (kExNorm | kExSwiglu)) return launch_epi<PLANES, F16, GROUPED, kEpiNormGlu>(tw, tb, td, pm, a, s);
+    if (scaled && a.x.mask == kExNorm) return launch_epi<PLANES, F16, GROUPED, kEpiNorm>(tw, tb, td, pm, a, s);
+    if (a.e.beta != 0.f && a.e.d_dtype != NVFP4A_FP32 && a.x.mask == 0) return launch_epi<PLANES, F16, GROUPED, kEpiAdd>(tw, tb, td, pm, a, s);
     if (scaled && a.x.mask == kExOut2) return launch_epi<PLANES, F16, GROUPED, kEpiOut2>(tw, tb, td, pm, a, s);
   }
   if constexpr (!F16 && !GROUPED)

@@ -1064,10 +1064,10 @@ def test_w4a16_epilogues_compiled_for_plain_calls_equal_the_general_one(bt, case
 
 
 @pytest.mark.parametrize("bt", [L.BF16, L.INT8])
-@pytest.mark.parametrize("case", ["norm_swiglu", "out2"])
+@pytest.mark.parametrize("case", ["norm_swiglu", "out2", "norm", "add"])
 def test_w4a16_epilogues_compiled_for_the_mlp_equal_the_general_one(bt, case):
-    """RMSNorm scale + SwiGLU and the second output with sums of squares have epilogues of their own where D has 16 bits; an FP32 D takes the general
-    one: the 16-bit D is its rounding, the other outputs and the amax are the same bytes.  With and without bias and amax, D that TMA stores or not, ragged tiles."""
+    """RMSNorm scale with or without SwiGLU, the second output with sums of squares, and beta * C have epilogues of their own where D has 16 bits; an FP32 D
+    takes the general one: the 16-bit D is its rounding, the other outputs and the amax are the same bytes.  With and without bias and amax, D that TMA stores or not, ragged tiles."""
     m, n, k = 528, 300, 640
     glu = case == "norm_swiglu"
     gen = torch.Generator(device="cuda").manual_seed(18)
@@ -1082,20 +1082,22 @@ def test_w4a16_epilogues_compiled_for_the_mlp_equal_the_general_one(bt, case):
         tb = tensor(x, bt)
     bias, w2 = (torch.randn(m, generator=gen, device="cuda").to(torch.bfloat16) for _ in range(2))
     parts = torch.rand(n, 8, generator=gen, device="cuda")
+    C = torch.randn(n, m, generator=gen, device="cuda").to(torch.bfloat16)
+    tc = tensor(C, L.BF16)
     mo = m // 2 if glu else m
 
     def run(dt, ld, use_bias, use_amax):
         D, amax = torch.zeros(n, ld, dtype=dt, device="cuda"), torch.zeros(1, dtype=torch.float32, device="cuda")
         d2, sq = torch.zeros(n, m, dtype=torch.bfloat16, device="cuda"), torch.zeros(n, m // 16, dtype=torch.float32, device="cuda")
         ex = L.Epilogue()
-        if glu:
-            ex.norm_parts, ex.norm_nparts, ex.norm_ld, ex.norm_inv_n, ex.norm_eps, ex.swiglu = parts.data_ptr(), 8, 8, 1.0 / 64.0, 1e-6, 1
-        else:
+        if case.startswith("norm"):
+            ex.norm_parts, ex.norm_nparts, ex.norm_ld, ex.norm_inv_n, ex.norm_eps, ex.swiglu = parts.data_ptr(), 8, 8, 1.0 / 64.0, 1e-6, int(glu)
+        elif case == "out2":
             ex.d2, ex.d2_dtype, ex.ldd2, ex.w2, ex.w2_dtype, ex.sq, ex.ld_sq = d2.data_ptr(), L.BF16, m, w2.data_ptr(), L.BF16, sq.data_ptr(), m // 16
         td = tensor(D, {torch.bfloat16: L.BF16, torch.float16: L.FP16, torch.float32: L.FP32}[dt], amax=amax if use_amax else None)
         tbias = tensor(bias, L.BF16)
-        L.check(L.lib.nvfp4a_gemm_ex(m, n, k, -0.01, ctypes.byref(ta), k, ctypes.byref(tb), k, 0.0, None, 0, ctypes.byref(td), ld,
-                                     ctypes.byref(tbias) if use_bias else None, ctypes.byref(ex), stream()))
+        L.check(L.lib.nvfp4a_gemm_ex(m, n, k, -0.01, ctypes.byref(ta), k, ctypes.byref(tb), k, *(ctypes.c_float(0.5), ctypes.byref(tc), m) if case == "add" else (0.0, None, 0),
+                                     ctypes.byref(td), ld, ctypes.byref(tbias) if use_bias else None, ctypes.byref(ex) if case != "add" else None, stream()))
         assert L.lib.nvfp4a_b200_last_route() == (8 if bt == L.INT8 else 5)
         return D, d2.view(torch.int16), sq.view(torch.int32), amax.view(torch.int32)
 
