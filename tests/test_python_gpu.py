@@ -449,3 +449,25 @@ def test_host_tensors_are_refused_before_any_launch():
         with pytest.raises(ValueError, match="lives on cpu"):
             call()
     assert torch.isfinite(nf.linear(x, w)).all()
+
+
+@pytest.mark.parametrize("shape", [(48, 64), (16, 16), (3, 16, 128)])
+def test_a_quantized_tensor_is_what_the_constructor_makes_of_its_parts(shape):
+    """``quantize`` builds its result without the constructor's checks: every attribute is the constructor's all the same, and a bound that it
+    refuses stays refused."""
+    x = torch.randn(*shape, device="cuda").to(torch.bfloat16)
+    for recipe in ({}, {"swizzled": True}, {"scale_dtype": "ue5m3"}, {"row_scaled": True}, {"columnwise": True, "swizzled": True}, {"four_over_six": "mse"},
+                   {"block": "16x16", "swizzled": 1}, {"scale_max": 448}):
+        q = nf.quantize(x, **recipe)
+        for t in (q, q.columnwise):
+            if t is None:
+                continue
+            want = nf.NVFP4Tensor(t.data, t.scales, amax=t.amax, scale_max=t.scale_max, swizzled=t.swizzled, ue5m3=t.ue5m3, cols=t.cols, block=t.block)
+            got, full = dict(vars(t)), dict(vars(want))
+            for name in ("data", "scales", "global_scale"):
+                a, b = got.pop(name), full.pop(name)
+                assert a.dtype == b.dtype and a.shape == b.shape and a.data_ptr() == b.data_ptr()
+            got.pop("columnwise"), full.pop("columnwise")
+            assert got == full and [type(got[n]) for n in got] == [type(full[n]) for n in got] and t.flags == want.flags and t.shape == want.shape
+    with pytest.raises(ValueError):
+        nf.quantize(x, scale_max=300)
