@@ -10,7 +10,8 @@
  *   - all pointers inside nvfp4a_tensor / nvfp4a_epilogue are DEVICE pointers of the current device; the structs
  *     themselves live on the host;
  *   - work is enqueued on `stream`; nothing is synchronised and no device memory is read on the host;
- *   - the library allocates no device memory in any entry point;
+ *   - the library allocates no device memory in any entry point but the GEMMs of 16-bit and INT8 activations on the tensor cores, which take scratch
+ *     (activation planes, partial sums) from a memory pool of the library's own, in stream order, for the duration of the call;
  *   - every argument is validated before anything is launched; a failed call launches nothing;
  *   - a status other than NVFP4A_OK leaves a message for nvfp4a_last_error() on the calling thread.
  */
@@ -80,8 +81,8 @@ typedef struct {
  * block-sum definition of the reference (ref include/nvfp4effma.h:78-92) within an FP32 accumulation bound.
  * Block scales on the tensor-core routes: the FP4 tensor cores read E4M3 block scales as UNSIGNED (UE4M3).  Codes with the sign bit
  * set -- which the reference decodes as negative factors (ref src/nvfp4effma.cuh:56-60) but which neither quantizer ever emits -- give
- * other results on the tcgen05 routes (NVFP4 B with n > 8, and the FP4 tensor-core GEMV) than the reference.  Tensors that carry such
- * codes must be run with nvfp4a_b200_set_route(1), whose CUDA-core kernels decode them exactly as the reference does.
+ * other results on the tcgen05 route of NVFP4 B with n > 8 than the reference (the GEMVs and the GEMMs of other B keep the sign).  Tensors
+ * that carry such codes must be run with nvfp4a_b200_set_route(1), whose CUDA-core kernels decode them exactly as the reference does.
  * ref include/nvfp4effma.h:93 */
 nvfp4a_status nvfp4a_gemm(int m, int n, int k, float alpha, const nvfp4a_tensor *A, int lda,
                           const nvfp4a_tensor *B, int ldb, float beta, const nvfp4a_tensor *C, int ldc,
