@@ -35,8 +35,8 @@
 // (reference include/nvfp4effma.h:82-92 there), as the reference's own tensor-core GEMV (src/tensors/gemv_tc.cuh there).
 // Negative block scales keep their sign and the codes 0x7F / 0xFF are +-480, as in the mma.sync GEMV (gemv.cu) that takes the calls this kernel leaves:
 // the tensor cores know neither.  Linear scales are moved through registers anyway: their signs go into the weights there.  Rows of tiled scales that
-// have a negative code, and rows with 0x7F, are summed on the CUDA cores.
-#include <math.h>
+// have a negative code, and rows with 0x7F, are summed on the CUDA cores.  (Looking for them and for dropped bits: 28672 x 4096 with one vector 15.0 -> 15.25 us, 8192 x
+// 8192 11.3 -> 11.6.)
 #include <atomic>
 #include "operands.cuh"
 #include "sm100.cuh"
@@ -584,26 +584,21 @@ void set_gemv_fp4_splits(int s) { g_gemv_splits = s; }
 int gemv_fp4_pinned_splits() { return g_gemv_splits.load(); }
 
 // splits: power of two, at most 8 and nk; every CTA's k range is at most kMaxChunks chunks (its pieces' shared memory).  Returns 0 when the
-// kernel should not run.  Pinned (nvfp4a_b200_set_gemv_splits): that value if the problem can use it.  Automatic: the cut with the shortest
-// estimate, if that beats the mma.sync GEMV (3 us and 0.4 us per megabyte: it decodes weights on the CUDA cores).  The estimate: 3.4 us of set-up and tail,
-// 4.3 / 4.9 / 5.5 in a cluster of 2 / 4 / 8, and the stream, 36 KiB per chunk at 67 GB/s per CTA or 5.6 TB/s in all.  CUDA-graph timings of one
-// vector, here and there: 6144 x 4096 7.9 against 8.8 us, 4096 x 14336 12.5 against 17.5, 28672 x 4096 15.4 against 30.3; but 4096 x 4096 6.95 against 7.0 and 1024 x 1024 4.0 against 3.1: the first has no winner, so a tenth of
-// advantage is asked for.
-static int choose_splits(int m, int k, int n) {
-  const int nk = k >> 8, tiles = (m + kRows - 1) / kRows, sms = device_sms();
+// kernel should not run.  Pinned (nvfp4a_b200_set_gemv_splits): that value if the problem can use it.  Automatic: problems that stream at
+// least 32 MB of weights over at least 96 CTAs.  One vector, CUDA-graph timings here and on the mma.sync GEMV: 28672 x 4096 15.3 against 30.0 us, 8192 x 8192
+// 11.6 against 19.5.  Smaller matrices belong to the mma.sync GEMV, whose time does not depend on the activations: 6144 x 4096 takes 7.2 us here and 8.5
+// there, 4096 x 14336 12.9 and 17.5, but with 1 / 8 / 64 activations of a CTA below the planes 9.2 / 11.6 / 25.7 and 15.0 / 18.2 / 36.7, and with
+// more of them 22.7 and 63.1 -- and the inputs of 4096 x 14336, a decoder's down projection, are products, which spread that far.  (28672 x 4096: 16.2 /
+// 19.6 / 42.9 and 69.9.)
+static int choose_splits(int m, int k) {
+  const int nk = k >> 8, tiles = (m + kRows - 1) / kRows;
   auto fits = [&](int s) { return s <= nk && (nk + s - 1) / s <= kMaxChunks; };
   if (const int f = g_gemv_splits.load()) return fits(f) ? f : 0;
-  int best = 0;
-  double best_us = 0.9 * (3.0 + 0.405 * (m * (k * 0.5625e-6)));
-  for (int s = 1; s <= 8; s *= 2) {
-    if (!fits(s)) continue;
-    const int cap = s == 1 ? sms : s == 2 ? sms / 2 : s == 4 ? sms * 33 / 148 : sms * 15 / 148;   // clusters that run at once (see gemv_fp4_n8.cu)
-    const int rounds = (tiles + cap - 1) / cap, ctas = (tiles < cap ? tiles : cap) * s;
-    const double chunk = fmax(0.55, ctas * 36.9e3 / 5.6e6) + 0.08 * (n - 1);
-    const double us = (s == 1 ? 3.4 : s == 2 ? 4.3 : s == 4 ? 4.9 : 5.5) + rounds * ((nk + s - 1) / s) * chunk;
-    if (us < best_us) { best = s; best_us = us; }
-  }
-  return best;
+  int s = 1;
+  while (s < 4 && !fits(s)) s *= 2;
+  if (!fits(s)) return 0;
+  while (s * 2 <= 4 && nk / (s * 2) >= 8 && tiles * s * 2 <= device_sms()) s *= 2;
+  return tiles * s < 96 || (double)m * k * 0.5625 < 32e6 ? 0 : s;
 }
 
 bool gemv_fp4_supports(const GemmArgs &g) {
@@ -611,7 +606,7 @@ bool gemv_fp4_supports(const GemmArgs &g) {
   if (((uintptr_t)g.B.data & 15) || g.B.ld % 8) return false;
   // plain operands: scales in aligned 512-byte tiles (the swizzled layout), or linear with a 16-byte aligned base and pitch (TMA)
   if (!g.A.image && (((uintptr_t)g.A.data & 15) || g.A.ld % 32 || ((uintptr_t)g.A.sc & 15) || (g.A.sld > 0 && g.A.sld % 16))) return false;
-  return choose_splits(g.m, g.k, g.n) > 0;
+  return choose_splits(g.m, g.k) > 0;
 }
 
 cudaError_t launch_gemv_fp4(const GemmArgs &g, cudaStream_t s) {
@@ -641,7 +636,7 @@ cudaError_t launch_gemv_fp4(const GemmArgs &g, cudaStream_t s) {
     a.linear = g.A.sld > 0;
     if (a.linear && !make_tmap_dense(&ts, g.A.sc, 4, (uint64_t)g.k / 64, (uint64_t)g.m, (uint64_t)g.A.sld, 4, kRows)) return cudaErrorInvalidValue;
   }
-  const int splits = choose_splits(g.m, g.k, g.n);
+  const int splits = choose_splits(g.m, g.k);
   if (splits <= 0) return cudaErrorInvalidValue;
   void (*kern)(CUtensorMap, CUtensorMap, GemvFp4Args) = g.n == 1 ? gemv_fp4_kernel<1> : gemv_fp4_kernel<2>;
   static std::atomic<bool> attr_set[64][2];   // zero-initialised; set once per device and kernel

@@ -378,11 +378,25 @@ def test_activations_of_which_the_planes_drop_bits(pin, few):
     assert kernel_status() == 0
 
 
-def test_one_vector_takes_the_tensor_cores_from_14_megabytes_up():
-    for m, k, route in ((6144, 4096, FP4_GEMV), (4096, 14336, FP4_GEMV), (1024, 1024, 2)):
-        c = Case(m, 1, k, L.BF16, L.BF16, -1, -1, 1.0, 0.0, fa=SW)
-        h = build_case(c, 1900)
-        exp = oracle_case(c, h, want_ref=True)
-        got, amax = run_gemm(c, h)
-        assert L.lib.nvfp4a_b200_last_route() == route, c
-        check_bound(c, h, got, amax, exp)
+def test_one_and_two_vectors_take_the_tensor_cores_from_32_megabytes_up():
+    """Below that the mma.sync GEMV, whose time and bytes do not depend on how far the activations spread: one vector whose tail lies 2^-30 below its
+    largest value, through the plain and the image entry, gives the bytes of the mma.sync GEMV asked for by name."""
+    for m, k, route in ((6144, 4096, 2), (4096, 14336, 2), (1024, 1024, 2), (8192, 8192, FP4_GEMV)):
+        for n in (1, 2):
+            c = Case(m, n, k, L.BF16, L.BF16, -1, -1, 1.0, 0.0, fa=SW)
+            h = build_case(c, 1900)
+            x = O.to_f32(h["B"].raw, L.BF16).reshape(n, -1).copy()
+            x[:, 1::2] *= np.float32(2.0 ** -30)
+            h["B"] = O.Dense(L.BF16, O.from_f32(x.reshape(-1), L.BF16), h["ldb"])
+            exp = oracle_case(c, h, want_ref=True) if n == 1 else None
+            for run in (run_gemm, lambda c, h: run_tc(c, h, gemv=True)):
+                got, amax = run(c, h)
+                assert L.lib.nvfp4a_b200_last_route() == route, c
+                if exp is not None:
+                    check_bound(c, h, got, amax, exp)
+                if route == 2:
+                    old = L.lib.nvfp4a_b200_set_route(2)
+                    named = run(c, h)[0]
+                    L.lib.nvfp4a_b200_set_route(old)
+                    assert np.array_equal(got.view(np.uint8), named.view(np.uint8))
+    assert kernel_status() == 0
