@@ -48,14 +48,16 @@
 // Grouped (mixture of experts): A stacks the weights of all groups, a group owns the tokens [seg[q], seg[q + 1]); the CTAs read seg
 // (device memory) into a table of tile counts and find a tile's group there.  (INT8 activations only, plain epilogue, 16-bit D.)
 //
-// INT8 activations (W4A8, FP32 scale s_b per 16 values) run on the same kernel as planes [token][3][k] that a small kernel makes first.
+// INT8 activations (W4A8, FP32 scale s_b per 16 values) run on the same kernel as planes [token][5 or 3][k] that small kernels make first.
 // PLANES = 2 (one weight): x = q * s_b is t1 + t2, two FP16 terms of 11 bits each, on a grid that puts the token's largest below 2^15 (the epilogue
 // takes that power of two back).  t2 is the exact remainder's rounding: together they are x to within 2^-23 of it, or 2^-25 on the grid, which the
-// (k + 2) 2^-24 of the accumulation bound covers for every value while a token's scales lie within 2^12 of each other.  If some token's do not, or its
-// scales are not near enough to one for the grid's power of two to be a float, or the weights' scales are UE5M3 (products leave FP16's range), all
-// tokens are three BF16 planes instead, t1 + t2 + t3 = fl(q * s_b) exactly (8 + 8 + 8 bits), and a word in memory tells this kernel so.  One chain in the
+// (k + 2) 2^-24 of the accumulation bound covers for every value while a token's scales lie within 2^12 of each other.  A token whose scales do not, or
+// are not near enough to one for the grid's power of two to be a float, is three BF16 planes instead, t1 + t2 + t3 = fl(q * s_b) exactly (8 + 8 + 8 bits),
+// and so are all tokens where the weights' scales are UE5M3 (products leave FP16's range).  In the planes of the other kind a token is zero: a tile with
+// tokens of both kinds goes over k twice, on the same accumulator, and no token's result depends on its neighbours.  One chain in the
 // tensor cores, 2-norm error at k = 512 / 1024 / 4096 / 8192: 0.97e-6, 1.9e-6, 8.2e-6, 1.69e-5 (three planes: 1.4e-6, 2.6e-6, 9.9e-6, 1.91e-5).
-// 6144 x 4096 on 1000 tokens 125 us with three planes and an MMA issue per plane, 93 with two.
+// Scales 2^0 / 2^6 / 2^12 apart, k = 1024: 1.82e-6, 2.25e-6, 2.47e-6 (three planes: 2.60e-6, 2.74e-6, 2.85e-6).
+// 6144 x 4096 on 1000 tokens 125 us with three planes and an MMA issue per plane, 93 with two, 76 with what followed; 124 with one token of BF16 planes.
 // PLANES = 3 (grouped): always three BF16 planes, the last two in an accumulator of their own (see Segments).  Two FP16 planes would be 94 us instead of 96
 // (8 experts of 2048 x 4096 on 1100 tokens), but 11-bit terms lose more to the truncation in the tensor cores than 8-bit ones, whose sums stay
 // on a coarse grid: 1.6e-7 instead of 0.74e-7 at k = 4096.
@@ -85,7 +87,8 @@ struct W4A16Args {
   int unit;         // stages per unit: 1 or 2 (see the MMA issuer)
   const int *seg; int groups;   // GROUPED: m is the rows of ONE group's weight, n the bound on seg[groups]
   int parts, part_stages; float *partial;   // kEpiPart: k in `parts` runs of part_stages stages, each one's sums in partial [part][n][m]
-  const float *tscale;          // PLANES = 2: what each token's sums are multiplied by, then (word n) non-zero for three planes
+  const float *tscale;          // PLANES = 2: what each token's sums are multiplied by; word n: 0 all tokens are two FP16 planes, 1 some, 2 none; behind it
+                                // a byte per token, non-zero for three BF16 planes
 };
 
 // tensor maps of D in the peers' buffers (tensor-parallel all-gather fused into the epilogue's TMA stores); n = 0: none
@@ -257,12 +260,20 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
   const uint32_t tmem_base = 0;
   pdl_wait();   // from here on the previous kernel has completed and its writes are visible
   const float *tscale = nullptr;
-  bool wide = false;   // three BF16 planes instead of two FP16 ones (see the head of the file)
+  int all_kinds = 1;   // kinds of tokens (see the head of the file): bit 0 two FP16 planes (or whatever PLANES says), bit 1 three BF16 planes
   if constexpr (PLANES == 2) {
     tscale = behind_wait(g.tscale);
-    wide = tscale[g.n] != 0.f;
+    const float w = tscale[gn];
+    all_kinds = w == 0.f ? 1 : w == 1.f ? 3 : 2;
   }
-  const int planes = PLANES == 2 && wide ? 3 : PLANES, per_slot = PLANES == 3 ? 3 : 2;   // planes of an activation, planes in a ring slot
+  auto kinds_of = [&](const Tile &p) -> int {   // those in a tile, each a pass over k (warp-wide)
+    if (PLANES != 2 || all_kinds != 3) return all_kinds;
+    const uint8_t *const three = (const uint8_t *)(tscale + gn + 1);
+    uint32_t f = 0;
+    for (int j = p.j0 + lane; j < min(p.j0 + p.width, gn); j += 32) f |= three[j] ? 2u : 1u;
+    return (int)__reduce_or_sync(0xFFFFFFFFu, f);
+  };
+  constexpr int kKinds = PLANES == 2 ? 2 : 1, per_slot = PLANES == 3 ? 3 : 2;   // (per_slot: planes in a ring slot)
 
   const unsigned tag = g.tag;
   auto wait = [abort_flag, status_word, tag](uint64_t *bar, uint32_t parity, unsigned code) -> bool {
@@ -322,18 +333,23 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
     for (int t = tile_first; t < ntiles; t += tile_step) {
       const Tile p = tile_of(t);
       if (p.width == 0) continue;
-      const int row0 = p.j0 + rank * (p.width >> 1);
+      const int row0 = p.j0 + rank * (p.width >> 1), kinds = kinds_of(p);
+#pragma unroll 1
+      for (int kind = 0; kind < kKinds; ++kind) {
+      if (kKinds == 2 && !(kinds >> kind & 1)) continue;
+      const int pl_end = PLANES == 2 ? (kind ? 5 : 2) : PLANES;   // (PLANES = 2: planes 0 and 1, then 2 to 4)
 #pragma unroll 1
       for (int ks = 0; ks < nk; ks += unit) {
 #pragma unroll 1
-        for (int pl = 0; pl < planes; pl += per_slot, ++it) {   // a slot: two stages, or two or three planes of one (plane pl of a token's row starts 2 k bytes after plane pl - 1)
-          const int s = it & (nB - 1), nsub = PLANES == 1 ? min(unit, nk - ks) : min(per_slot, planes - pl);
+        for (int pl = 2 * kind; pl < pl_end; pl += per_slot, ++it) {   // a slot: two stages, or two or three planes of one (plane pl of a token's row starts 2 k bytes after plane pl - 1)
+          const int s = it & (nB - 1), nsub = PLANES == 1 ? min(unit, nk - ks) : min(per_slot, pl_end - pl);
           if (!__all_sync(0xFFFFFFFFu, wait(&b_empty[s], (it >> lgB & 1) ^ 1, kStWaitEmpty))) goto done;
           if (rank == 0) mbar_arrive_expect_tx_elect(&b_full[s], nsub * sub_bytes);
           const uint32_t dst = smem_u32(sB) + (uint32_t)(s * slot_bytes), bar = mbar_addr_rank(&b_full[s], 0);
           for (int i = 0; i < nsub; ++i)
             tma_load_3d_pair_elect(dst + i * kSub, &tmap_b, PLANES == 1 ? (k0 + ks + i) * 128 : (pl + i) * 2 * gk + (k0 + ks) * 128, row0, 0, bar);
         }
+      }
       }
     }
   } else if (warp == 1) {
@@ -349,7 +365,7 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
       for (int t = tile_first; t < ntiles; t += tile_step) {
         const Tile p = tile_of(t);
         if (p.width == 0) continue;
-        const uint32_t idesc = idesc_f16(256, p.width, PLANES == 2 ? (wide ? 1 : 0) : F16 ? 0 : 1);
+        const int kinds = kinds_of(p);
         for (int ks0 = 0; ks0 < nk; ks0 += SEG ? seg_stages : nk, ++acc_i) {
           const int acc = nacc == 2 ? acc_i & 1 : 0, ks1 = SEG ? min(ks0 + seg_stages, nk) : nk;
           const uint32_t acc_par = (nacc == 2 ? acc_i >> 1 : acc_i) & 1;
@@ -358,6 +374,11 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
           if (SEG && PLANES != 1 && ks0 == 0 && !__all_sync(0xFFFFFFFFu, wait(&tmem_empty[acc ^ 1], (((acc_i + 1) >> 1) & 1) ^ 1, kStWaitTmemEmpty))) goto done;
           tc_fence_after();
           const uint32_t d_tmem = tmem_base + acc * 128;
+#pragma unroll 1
+          for (int kind = 0; kind < kKinds; ++kind) {
+          if (kKinds == 2 && !(kinds >> kind & 1)) continue;
+          const uint32_t idesc = idesc_f16(256, p.width, PLANES == 2 ? kind : F16 ? 0 : 1);
+          const bool second = kind && (kinds & 1);   // on the sums of the first pass
 #pragma unroll 1
           for (int ks = ks0; ks < ks1; ks += unit, ++ia, ++ib) {
             const int sa = ia & (nA - 1);
@@ -375,8 +396,8 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
               mma12_f16_commit_pair_elect(d_tmem, a_tmem, db, ks != ks0, tmem_base + kSmallCols, db + (kSub >> 4), ks != 0, db + 2 * (kSub >> 4), idesc, &b_empty[sb]);
               tc_commit_pair_elect(&a_empty[sa]);
             } else {
-              mma8_f16_commit_pair_elect(d_tmem, a_tmem, db, ks != ks0, d_tmem, a_tmem, db + (kSub >> 4), 1, idesc, &b_empty[sb]);
-              if (wide) {
+              mma8_f16_commit_pair_elect(d_tmem, a_tmem, db, second || ks != ks0, d_tmem, a_tmem, db + (kSub >> 4), 1, idesc, &b_empty[sb]);
+              if (kind) {
                 ++ib;
                 sb = ib & (nB - 1);
                 if (!__all_sync(0xFFFFFFFFu, wait(&b_full[sb], ib >> lgB & 1, kStWaitFullB))) goto done;
@@ -386,6 +407,7 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
               }
               tc_commit_pair_elect(&a_empty[sa]);
             }
+          }
           }
           tc_commit_pair_elect(&tmem_full[acc]);
         }
@@ -400,6 +422,7 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
       const Tile p = tile_of(t);
       if (p.width == 0) continue;
       const int row_tile = 2 * p.tm + rank;
+      for (int pass = kKinds == 2 ? __popc(kinds_of(p)) : 1; pass > 0; --pass) {
 #pragma unroll 1
       for (int sl = 0; sl < nslots; ++sl, ++it) {
         const int s = it % kRaw;
@@ -409,6 +432,7 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
         // (rows past the matrix read zeros; their scales are those of its last row, and no row past it is stored)
         if (img) tma_load_3d_elect(dst, &tmap_w, 0, 0, row_tile * ktiles + (k0 >> 2) + sl, bar);
         else tma_load_3d_elect(dst, &tmap_w, ((k0 >> 2) + sl) * 128, p.ro + row_tile * 128, 0, bar);
+      }
       }
     }
   }
@@ -738,7 +762,6 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
     const Fp4Operand A = g.A;
     const ScalePos sp{A.sld};
     const bool img = A.image, swz = A.sld < 0;
-    const uint4 *const table = lut + (wide ? 256 : 0);
     // scale words of this group's two stages of slot sl (stages past the end of k: zeros)
     auto fetch_scales = [&](const uint8_t *scp, int sl, uint32_t (&v)[2]) {
 #pragma unroll
@@ -749,13 +772,18 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
       }
     };
     const int tile_units = (nk + unit - 1) / unit;
-    uint32_t isl = 0, it0 = 0;   // slots so far; units of the finished tiles
-    for (int t = tile_first; t < ntiles; t += tile_step, it0 += tile_units) {
+    uint32_t isl = 0, it0 = 0;   // slots so far; units of the finished passes over k
+    for (int t = tile_first; t < ntiles; t += tile_step) {
       const Tile p = tile_of(t);
-      if (p.width == 0) { it0 -= tile_units; continue; }
+      if (p.width == 0) continue;
+      const int kinds = kinds_of(p);
       const int r = min((2 * p.tm + rank) * 128 + row, gm - 1);
       const uint8_t *scp = img ? A.data + (size_t)(r >> 7) * A.ktiles * kImgTileBytes + kImgDataBytes + (r & 31) * 16 + ((r & 127) >> 5) * 4
                                : A.sc + sp.row(p.ro + r);
+#pragma unroll 1
+      for (int kind = 0; kind < kKinds; ++kind) {
+      if (kKinds == 2 && !(kinds >> kind & 1)) continue;
+      const uint4 *const table = lut + 256 * kind;
       uint32_t sc[2], sc_next[2] = {0, 0};
       fetch_scales(scp, 0, sc);
 #pragma unroll 1
@@ -800,6 +828,8 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
         __syncwarp();
         if (lane == 0) mbar_arrive(&raw_empty[rs]);
         sc[0] = sc_next[0]; sc[1] = sc_next[1];
+      }
+      it0 += tile_units;
       }
     }
   }
@@ -971,9 +1001,9 @@ bool set_up(const GemmArgs &g, int planes, bool f16, int groups, const void *act
   return true;
 }
 
-// INT8 activations q [n][ld] with one FP32 scale s per 16 values -> two FP16 planes [n][3][k] (the third is left alone): t1 + t2 is q * s * 2^(7 - E) to
-// within 2^-23 of itself or 2^-25, E the exponent of the token's largest scale; tscale[token] = 2^(E - 7).  A token whose scales two planes do not
-// take (see the head of the file) is marked in wide[token].  One CTA per token, a thread per 8 values: 8 bytes in, two 16-byte stores out.
+// INT8 activations q [n][ld] with one FP32 scale s per 16 values -> planes 0 and 1 of [n][5][k], FP16: t1 + t2 is q * s * 2^(7 - E) to within 2^-23 of
+// itself or 2^-25, E the exponent of the token's largest scale; tscale[token] = 2^(E - 7).  A token whose scales two planes do not
+// take (see the head of the file) is zeros there, and marked in wide[token].  One CTA per token, a thread per 8 values: 8 bytes in, two 16-byte stores out.
 constexpr int kPlanesThreads = 256, kPlanesSpread = 12;
 __global__ void __launch_bounds__(kPlanesThreads) w4a8_planes_kernel(const int8_t *q_in, int ld, const float *sc_in, int lds, int k, uint16_t *planes, float *tscale,
                                                                      uint8_t *wide) {
@@ -1003,7 +1033,13 @@ __global__ void __launch_bounds__(kPlanesThreads) w4a8_planes_kernel(const int8_
     tscale[j] = __uint_as_float((uint32_t)(narrow ? eh - 7 : 127) << 23);
     wide[j] = !narrow;
   }
-  if (!narrow) return;
+  uint16_t *const row0 = planes + (size_t)j * 5 * k;
+  if (!narrow) {
+    for (int c = threadIdx.x; c < (k >> 3); c += kPlanesThreads)
+#pragma unroll
+      for (int p = 0; p < 2; ++p) *(uint4 *)(row0 + (size_t)p * k + 8 * c) = make_uint4(0, 0, 0, 0);
+    return;
+  }
   const float up = __uint_as_float((uint32_t)(261 - eh) << 23);   // 2^(7 - E), a normal number
   for (int c = threadIdx.x; c < (k >> 3); c += kPlanesThreads) {
     const uint2 raw = raw_next;
@@ -1021,16 +1057,16 @@ __global__ void __launch_bounds__(kPlanesThreads) w4a8_planes_kernel(const int8_
       t[0][i] = *reinterpret_cast<const uint32_t *>(&t1);
       t[1][i] = *reinterpret_cast<const uint32_t *>(&t2);
     }
-    uint16_t *const row = planes + (size_t)j * 3 * k + 8 * c;
+    uint16_t *const row = row0 + 8 * c;
 #pragma unroll
     for (int p = 0; p < 2; ++p) *(uint4 *)(row + (size_t)p * k) = make_uint4(t[p][0], t[p][1], t[p][2], t[p][3]);
   }
 }
 
-// Runs behind it: tells the GEMM which planes there are (tscale[n]), and if some token is wide (or all count as such: `force`) writes three BF16
-// planes [n][3][k] of every token instead, t1 + t2 + t3 = fl(q * s) exactly, tscale 1.
-__global__ void __launch_bounds__(256) w4a8_wide_planes_kernel(const int8_t *q_in, int ld, const float *sc_in, int lds, int n, int k, uint16_t *planes, float *tscale,
-                                                               const uint8_t *wide_in, int force) {
+// Runs behind it: tells the GEMM which planes there are (tscale[n], see W4A16Args), and if some token is wide, or all are (`force`), writes the last three of
+// each token's `per_token` planes, BF16: t1 + t2 + t3 = fl(q * s) exactly, tscale 1, of the wide ones, zeros of the others.
+__global__ void __launch_bounds__(256) w4a8_wide_planes_kernel(const int8_t *q_in, int ld, const float *sc_in, int lds, int n, int k, uint16_t *planes, int per_token,
+                                                               float *tscale, const uint8_t *wide_in, int force) {
   pdl_launch_dependents();
   pdl_wait();
   const uint8_t *const wide = behind_wait(wide_in);
@@ -1039,11 +1075,17 @@ __global__ void __launch_bounds__(256) w4a8_wide_planes_kernel(const int8_t *q_i
   int any = force;
   for (int j = threadIdx.x; j < n && !force; j += blockDim.x) any |= wide[j];
   any = __syncthreads_or(any);
-  if (blockIdx.x == 0 && threadIdx.x == 0) tscale[n] = any ? 1.f : 0.f;
+  if (blockIdx.x == 0 && threadIdx.x == 0) tscale[n] = force ? 2.f : any ? 1.f : 0.f;
   if (!any) return;
   const long long per_row = k >> 3;
   for (long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x; v < per_row * n; v += (long long)gridDim.x * blockDim.x) {
     const int j = (int)(v / per_row), c = (int)(v - (long long)j * per_row);   // token, group of 8 values
+    uint16_t *const row = planes + ((size_t)j * per_token + per_token - 3) * k + 8 * c;
+    if (!force && !wide[j]) {
+#pragma unroll
+      for (int p = 0; p < 3; ++p) *(uint4 *)(row + (size_t)p * k) = make_uint4(0, 0, 0, 0);
+      continue;
+    }
     if (c == 0) tscale[j] = 1.f;
     const uint2 raw = *(const uint2 *)(q + (size_t)j * ld + 8 * c);
     const float s = sc[(size_t)j * lds + (c >> 1)];
@@ -1061,7 +1103,6 @@ __global__ void __launch_bounds__(256) w4a8_wide_planes_kernel(const int8_t *q_i
         r = __fsub_rn(r, tp);   // exact: the remainder has at most 16, then 8 significant bits
       }
     }
-    uint16_t *row = planes + (size_t)j * 3 * k + 8 * c;
 #pragma unroll
     for (int p = 0; p < 3; ++p) *(uint4 *)(row + (size_t)p * k) = make_uint4(t[p][0], t[p][1], t[p][2], t[p][3]);
   }
@@ -1182,8 +1223,9 @@ cudaError_t launch_gemm_w4a8_tc(const GemmArgs &g, const int *seg, int groups, c
   cudaMemPool_t pool;
   cudaError_t e = planes_pool(&pool);
   if (e != cudaSuccess) return e;
-  // planes [n][3][k], n token scales and the word behind them, n marks; the sums of parts of k, if there are any
-  const size_t plane_bytes = (size_t)g.n * 3 * g.k * sizeof(uint16_t), small_bytes = (plane_bytes + (size_t)(g.n + 1) * sizeof(float) + g.n + 255) / 256 * 256;
+  // planes [n][3 or 5][k], n token scales and the word behind them, n marks; the sums of parts of k, if there are any
+  const int per_token = three ? 3 : 5;
+  const size_t plane_bytes = (size_t)g.n * per_token * g.k * sizeof(uint16_t), small_bytes = (plane_bytes + (size_t)(g.n + 1) * sizeof(float) + g.n + 255) / 256 * 256;
   GemmArgs w = g;
   int parts = seg ? 1 : plan_parts(g, three ? 3 : 2, false, nullptr);
   if (parts > 1 && cudaMallocFromPoolAsync((void **)&planes, small_bytes + (size_t)parts * g.n * g.m * sizeof(float), pool, s) != cudaSuccess) {
@@ -1196,7 +1238,7 @@ cudaError_t launch_gemm_w4a8_tc(const GemmArgs &g, const int *seg, int groups, c
   if (e != cudaSuccess) return e;
   float *const tscale = (float *)((uint8_t *)planes + plane_bytes);
   uint8_t *const wide = (uint8_t *)(tscale + g.n + 1);
-  const bool force = three || g.A.ue;   // three planes whatever the scales (products with UE5M3 scales leave FP16's range)
+  const bool force = three || g.A.ue;   // three BF16 planes whatever the scales (products with UE5M3 scales leave FP16's range)
   // Each kernel starts while the one before it ends (a quantizer, usually) and waits for its results; the planes may still be in use by the GEMM before the
   // quantizer, which that one has waited for.
   cudaLaunchConfig_t cfg;
@@ -1214,14 +1256,15 @@ cudaError_t launch_gemm_w4a8_tc(const GemmArgs &g, const int *seg, int groups, c
   if (e == cudaSuccess) {
     cfg.gridDim = dim3(force ? (unsigned)(((long long)g.n * (g.k >> 3) + 255) / 256) : (unsigned)device_sms(), 1, 1);
     cfg.blockDim = dim3(256, 1, 1);
-    e = cudaLaunchKernelEx(&cfg, w4a8_wide_planes_kernel, (const int8_t *)g.B.data, g.B.ld, g.B.s8, g.B.lds8, g.n, g.k, planes, tscale, (const uint8_t *)wide, force ? 1 : 0);
+    e = cudaLaunchKernelEx(&cfg, w4a8_wide_planes_kernel, (const int8_t *)g.B.data, g.B.ld, g.B.s8, g.B.lds8, g.n, g.k, planes, per_token, tscale, (const uint8_t *)wide, force ? 1 : 0);
   }
   if (e == cudaSuccess) {
     W4A16Args a;
     CUtensorMap tw, tb, td;
     PeerMaps pm;
     memset(&pm, 0, sizeof pm);
-    if (!set_up(w, three ? 3 : 2, false, seg ? groups : 0, planes, (uint64_t)g.k * 6, (uint64_t)g.k * 6, &a, &tw, &tb, &td)) e = cudaErrorInvalidValue;
+    const uint64_t row_bytes = (uint64_t)g.k * per_token * sizeof(uint16_t);
+    if (!set_up(w, three ? 3 : 2, false, seg ? groups : 0, planes, row_bytes, row_bytes, &a, &tw, &tb, &td)) e = cudaErrorInvalidValue;
     else {
       a.tscale = tscale;
       a.seg = seg; a.groups = groups;

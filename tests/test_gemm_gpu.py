@@ -990,6 +990,48 @@ def test_w4a8_planes_at_the_edges_of_their_range(grouped, spread, exponent):
     assert kernel_status() == 0
 
 
+@pytest.mark.parametrize("m,n,k,out", [(300, 64, 512, "bf16"), (512, 200, 1088, "fp16"), (640, 1000, 2048, "fp32"), (300, 130, 4096, "bf16"), (768, 449, 1024, "swiglu")])
+def test_w4a8_result_of_a_token_does_not_depend_on_its_neighbours(m, n, k, out):
+    """Tokens whose scales lie more than 2^12 apart are BF16 planes, the others FP16 planes: whichever tokens of a call are of which kind -- one, the first
+    and the last of a tile, every third, all -- a token's outputs are the bytes that it has among tokens of its own kind, and they keep the bound."""
+    gen = torch.Generator(device="cuda").manual_seed(m + n)
+    w = torch.randint(0, 16, (m, k), generator=gen, device="cuda", dtype=torch.uint8)
+    ws = torch.randint(0x28, 0x48, (m, k // 16), generator=gen, device="cuda", dtype=torch.uint8)
+    W = torch.tensor([0.0, 0.5, 1.0, 1.5, 2.0, 3.0, 4.0, 6.0], dtype=torch.float64, device="cuda")[(w & 7).long()] * (1.0 - 2.0 * (w >> 3).double())
+    W = (W.view(m, k // 16, 16) * ws.view(torch.float8_e4m3fn).double().unsqueeze(-1)).view(m, k)
+    packed = (w[:, 0::2] | (w[:, 1::2] << 4)).contiguous()
+    x = torch.randint(-127, 128, (n, k), generator=gen, device="cuda", dtype=torch.int8)
+    s = torch.exp2(-3.0 * torch.rand(n, k // 16, generator=gen, device="cuda")) * 2.0 ** -8
+    wide_s = s.clone()
+    wide_s[:, 3::7] *= 2.0 ** -14
+    dt = {"bf16": torch.bfloat16, "fp16": torch.float16, "fp32": torch.float32, "swiglu": torch.bfloat16}[out]
+    code = {"bf16": L.BF16, "fp16": L.FP16, "fp32": L.FP32, "swiglu": L.BF16}[out]
+    ta = tensor(packed, L.NVFP4, ws, k // 16)
+
+    def run(wide):
+        sc = torch.where(wide.unsqueeze(1), wide_s, s).contiguous()
+        d = torch.zeros(n, m // 2 if out == "swiglu" else m, dtype=dt, device="cuda")
+        tb, td = tensor(x, L.INT8, sc, k // 16), tensor(d, code)
+        if out == "swiglu":
+            ex = L.Epilogue()
+            ex.swiglu = 1
+            L.check(L.lib.nvfp4a_gemm_ex(m, n, k, 2.0 ** -6, ctypes.byref(ta), k, ctypes.byref(tb), k, 0.0, None, 0, ctypes.byref(td), m // 2, None, ctypes.byref(ex), stream()))
+        else:
+            L.check(L.lib.nvfp4a_gemm(m, n, k, 1.0, ctypes.byref(ta), k, ctypes.byref(tb), k, 0.0, None, 0, ctypes.byref(td), m, None, stream()))
+            X = (x.double().view(n, k // 16, 16) * sc.double().unsqueeze(-1)).view(n, k)
+            want, size = X @ W.t(), X.abs() @ W.abs().t()
+            assert bool(((d.double() - want).abs() <= (k + 2) * 2.0 ** -24 * size + (0.0 if out == "fp32" else 2.0 ** -8) * want.abs()).all())
+        assert L.lib.nvfp4a_b200_last_route() == 8
+        return d.view(torch.int32 if out == "fp32" else torch.int16)
+
+    index = torch.arange(n, device="cuda")
+    none, every = run(index < 0), run(index >= 0)
+    for wide in (index == 7, (index == 0) | (index == n - 1), index % 3 == 1, index >= n // 2, index != 63):
+        got = run(wide)
+        assert torch.equal(got[~wide], none[~wide]) and torch.equal(got[wide], every[wide])
+    assert kernel_status() == 0
+
+
 def test_w4a8_planes_with_ue5m3_weight_scales():
     """Products with UE5M3 scales do not fit FP16: three BF16 planes."""
     c = Case(256, 96, 512, L.INT8, L.FP32, -1, L.BF16, 1.25, 0.0, fa=UE)
