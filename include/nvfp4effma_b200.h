@@ -148,7 +148,8 @@ nvfp4a_status nvfp4a_b200_gemm_tc_tp(int m, int n, int k, float alpha, const nvf
 /* nvfp4a_gemm_ex that allocates nothing and still computes the RMSNorm column scales once per call: they are staged in a
  * 64 KiB device array inside the library image instead of a workspace.  No counterpart in the reference (its
  * nvfp4a_gemm_ex needs no scratch; its tensor-core entries take a caller workspace).  Same arguments and the same results,
- * bit for bit, as nvfp4a_gemm_ex.  For callers that cannot hand over or allocate scratch at the call: inside stream
+ * bit for bit, as nvfp4a_gemm_ex, except for INT8 activations of 64 and more tokens: those nvfp4a_gemm_ex takes to the tensor cores as
+ * planes, which need scratch (within the FP32 accumulation bound), and this entry to the exact DP4A kernel.  For callers that cannot hand over or allocate scratch at the call: inside stream
  * capture, or where a framework allocator holds all device memory.
  *   - n is limited to nvfp4a_b200_static_scratch_tokens() (16384); a larger n returns NVFP4A_INVALID_VALUE.
  *   - The first call on a device looks the array's address up (cudaGetSymbolAddress): make it before capturing a stream.

@@ -1198,12 +1198,12 @@ cudaError_t trim_planes_pool() {
 // W4A8 on the tensor cores (see the header): from 64 tokens and 128 weight rows up, where the planes' set-up pays whatever the rest.  The call
 // takes the planes from the pool above (stream-ordered: capturable, no synchronisation) and gives them back after the GEMM.
 // Fewer tokens came from the DP4A kernel, whose ordered sums are more exact than one chain: they are summed in segments (three planes, a 16-bit D, the
-// plain epilogue), and only where the reduction is long enough for that and for the planes to pay: 835 x 2176 on 30 tokens 158 us there, 30 here,
+// plain epilogue; nvfp4a_gemm_ex stays on the DP4A kernel, see GemmArgs::whole_k), and only where the reduction is long enough for that and for the planes to pay: 835 x 2176 on 30 tokens 158 us there, 30 here,
 // 640 x 3840 on 10 tokens 267 and 41, 1024 x 512 on 32 tokens 49 and 17.
 constexpr int kW4A8ChainMinN = 64;
 bool gemm_w4a8_tc_supports(const GemmArgs &g) {
   if (g.B.dtype != NVFP4A_INT8 || g.k < 64 || g.m < 128 || g.no_alloc || g.tp.world > 1 || g.e.gb_stride) return false;
-  if (g.n < kW4A8ChainMinN && (g.n <= 8 || g.k < 512 || g.e.d_dtype == NVFP4A_FP32 || g.x.mask || g.A.ue)) return false;
+  if (g.n < kW4A8ChainMinN && (g.n <= 8 || g.k < 512 || g.whole_k || g.e.d_dtype == NVFP4A_FP32 || g.x.mask || g.A.ue)) return false;
   if (((uintptr_t)g.B.data & 7) || g.B.ld % 8 || !g.B.s8 || ((uintptr_t)g.B.s8 & 3)) return false;
   if (!g.A.image && (((uintptr_t)g.A.data & 15) || g.A.ld % 32 || ((uintptr_t)g.A.sc & 1))) return false;
   return true;

@@ -59,7 +59,7 @@ struct GemmArgs {
   Epilogue e;
   EpilogueEx x;
   TpPush tp;   // tensor-parallel GEMV: D also goes to the peers, then the ranks' barrier (world <= 1: off)
-  int whole_k;    // nvfp4a_gemm_ex and its twin that must not allocate give the same bytes: no sums in parts of k
+  int whole_k;    // nvfp4a_gemm_ex gives the bytes of its twin that must not allocate: no sums in parts of k, no INT8 planes below 64 tokens
   int no_alloc;   // the call must not allocate (nvfp4a_b200_gemm_ex_static): routes that take scratch from the stream's memory pool step aside
 };
 

@@ -1183,6 +1183,24 @@ def test_w4a8_of_9_to_63_tokens_is_summed_in_segments(k):
 
 
 @pytest.mark.parametrize("bt", [L.BF16, L.FP16, L.INT8])
+def test_gemm_ex_and_its_twin_without_allocations_give_the_same_bytes(bt):
+    """Up to 63 tokens whatever the activations are, with a reduction that nvfp4a_gemm would cut into parts or take to the planes."""
+    for m, n, k in ((300, 16, 1024), (512, 33, 8192), (130, 63, 4096)):
+        c = Case(m, n, k, bt, L.BF16, -1, -1, 1.0, 0.0)
+        h = build_case(c, 5100 + n)
+        A = DevFp4(rand_fp4(np.random.default_rng(n), m, k, glob=0.375))
+        keep, tb = device_b(c, h)
+        ta, ex, outs = A.tensor(), L.Epilogue(), []
+        for entry in (L.lib.nvfp4a_gemm_ex, L.lib.nvfp4a_b200_gemm_ex_static):
+            d = torch.zeros(n, m, dtype=torch.bfloat16, device="cuda")
+            td = tensor(d, L.BF16)
+            L.check(entry(m, n, k, 1.0, ctypes.byref(ta), k, ctypes.byref(tb), h["ldb"], 0.0, None, 0, ctypes.byref(td), m, None, ctypes.byref(ex), stream()))
+            outs.append(d.view(torch.int16))
+        assert torch.equal(*outs) and bool(outs[0].any())
+    assert kernel_status() == 0
+
+
+@pytest.mark.parametrize("bt", [L.BF16, L.FP16, L.INT8])
 def test_long_reductions_of_few_tiles_in_parts_of_k(bt):
     """Few tiles and a long k: several CTA pairs take a run of k each, a small kernel adds their sums and runs the plain epilogue.  Every layout, runs of unequal
     length, odd numbers of stages, tails in m and n, bias, beta, every output type and amax; the same bytes on every call; and, captured in a graph
