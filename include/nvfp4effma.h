@@ -11,7 +11,8 @@
  *     themselves live on the host;
  *   - work is enqueued on `stream`; nothing is synchronised and no device memory is read on the host;
  *   - the library allocates no device memory in any entry point but the GEMMs of 16-bit and INT8 activations on the tensor cores, which take scratch
- *     (activation planes, partial sums) from a memory pool of the library's own, in stream order, for the duration of the call;
+ *     (activation planes, partial sums) from a memory pool of the library's own or from the caller (nvfp4a_b200_set_scratch_alloc), in stream order, for
+ *     the duration of the call;
  *   - every argument is validated before anything is launched; a failed call launches nothing;
  *   - a status other than NVFP4A_OK leaves a message for nvfp4a_last_error() on the calling thread.
  */

@@ -90,10 +90,21 @@ int nvfp4a_b200_set_swap(int mode);
 int nvfp4a_b200_last_route(void);
 
 /* The tensor-core W4A8 GEMM keeps the memory of its activation planes (10 bytes per INT8 activation of the largest call so far), and W4A16 /
- * W4A8 GEMMs with few tiles and a long k that of their FP32 sums over parts of k (at most 8 x 4 bytes per output, about 35 MB), in
+ * W4A8 GEMMs with few tiles and a long k that of their FP32 sums over parts of k (at most 19.4 MB), in
  * a memory pool of its own per device, so that later calls allocate in microseconds and without synchronising.  This call gives
  * the current device's pool memory that is not in use back to the system (no counterpart in the reference). */
 nvfp4a_status nvfp4a_b200_trim_scratch(void);
+
+/* From here on the calling thread's GEMM calls take that scratch from alloc(ctx, bytes) instead of the pool; alloc = NULL: from the pool again (no
+ * counterpart in the reference).  alloc returns memory of the current device on a 256-byte boundary that stays the call's until the work that the
+ * call enqueues has run -- the caller gives it back in the order of the call's stream -- or NULL, and must not throw.  At most two requests per call.
+ * For frameworks with an allocator of their own, and for stream capture, where memory of the pool would be an allocation node of the graph (a
+ * graph with such nodes cannot be a child of another, nor be instantiated twice).  Without scratch, and in a capture without an allocator, 16-bit
+ * activations keep k whole and 9 to 63 INT8 tokens take the exact DP4A kernel; 64 and more INT8 tokens take pool memory in a capture too. */
+void nvfp4a_b200_set_scratch_alloc(void *(*alloc)(void *ctx, size_t bytes), void *ctx);
+
+/* The number of parts that the calling thread's last W4A16 / W4A8 tensor-core GEMM cut k into (1: whole).  Test aid. */
+int nvfp4a_b200_last_parts(void);
 
 /* Pins the number of k ranges (CTAs per cluster) of the FP4 tensor-core GEMV: 0 = by problem size, else 1, 2, 4 or 8; a
  * value the problem cannot use (shared memory for the activation digit planes, k / 256) makes that GEMV step aside for the

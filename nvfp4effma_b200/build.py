@@ -39,7 +39,7 @@ def _compile(src, force):
 def _build_torch(force):
     """The torch operators' library; its C-ABI calls resolve to LIB beside it."""
     src = os.path.join(CSRC, "torch_ops.cpp")
-    newest = max(os.path.getmtime(src), os.path.getmtime(os.path.join(HERE, "..", "include", "nvfp4effma.h")))
+    newest = max(os.path.getmtime(f) for f in [src] + glob.glob(os.path.join(HERE, "..", "include", "*.h")))
     import torch
     out = os.path.join(HERE, f"libnvfp4effma_torch-{torch.__version__}.so")
     if not force and os.path.exists(out) and os.path.getmtime(out) > newest:

@@ -127,7 +127,11 @@ static nvfp4a_status dispatch(const char *fn, const GemmArgs &g, cudaStream_t st
   else if (gemv && g.k > 0 && gemv_blocked_supports(g)) { g_last_route = 6; err = launch_gemv_blocked(g, stream); }
   else if (!gemv && gemm_w4a4_supports(g)) { g_last_route = 4; err = launch_gemm_w4a4(g, stream); }
   else if ((!gemv || g.B.dtype == NVFP4A_FP16) && gemm_w4a16_supports(g)) { g_last_route = 5; err = launch_gemm_w4a16(g, stream); }
-  else if (!gemv && forced_route() != 3 && gemm_w4a8_tc_supports(g)) { g_last_route = 8; err = launch_gemm_w4a8_tc(g, nullptr, 0, stream); }
+  else if (!gemv && forced_route() != 3 && gemm_w4a8_tc_supports(g)) {
+    g_last_route = 8;
+    err = launch_gemm_w4a8_tc(g, nullptr, 0, stream);
+    if (err == cudaErrorMemoryAllocation && g.n < kW4A8ChainMinN && gemm_dp4a_supports(g)) { g_last_route = 7; err = launch_gemm_dp4a(g, stream); }
+  }
   else if (!gemv && gemm_dp4a_supports(g)) { g_last_route = 7; err = launch_gemm_dp4a(g, stream); }
   else { g_last_route = 1; err = launch_gemm_generic(g, stream); }
   if (err == cudaSuccess && g.tp.world > 1 && g_last_route != 2) {
@@ -351,6 +355,10 @@ extern "C" int nvfp4a_b200_set_route(int route) {
 }
 
 extern "C" int nvfp4a_b200_last_route(void) { return g_last_route; }
+
+extern "C" int nvfp4a_b200_last_parts(void) { return last_parts(); }
+
+extern "C" void nvfp4a_b200_set_scratch_alloc(void *(*alloc)(void *ctx, size_t bytes), void *ctx) { set_scratch_alloc({alloc, ctx}); }
 
 extern "C" nvfp4a_status nvfp4a_b200_trim_scratch(void) {
   clear_error();

@@ -1174,6 +1174,31 @@ static cudaError_t planes_pool(cudaMemPool_t *pool) {
   *pool = p;
   return cudaSuccess;
 }
+// The scratch of one call comes from the thread's allocator where it has set one (nvfp4a_b200_set_scratch_alloc: torch's, for the torch operators), else
+// from the pool.  In a capture memory of the pool would be a node of the caller's graph, which then cannot be a child of another graph nor be
+// instantiated twice: only calls that have no other kernel with a like result take it there (`in_capture`).
+static thread_local ScratchAlloc g_scratch_alloc = {nullptr, nullptr};
+void set_scratch_alloc(const ScratchAlloc &a) { g_scratch_alloc = a; }
+static thread_local int g_last_parts = 0;
+int last_parts() { return g_last_parts; }
+struct Scratch { void *p; bool pooled; };
+static Scratch take_scratch(size_t bytes, cudaStream_t s, bool in_capture) {
+  if (g_scratch_alloc.fn) {
+    void *const p = g_scratch_alloc.fn(g_scratch_alloc.ctx, bytes);
+    return {((uintptr_t)p & 255) ? nullptr : p, false};
+  }
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  cudaMemPool_t pool;
+  void *p = nullptr;
+  if ((!in_capture && (cudaStreamIsCapturing(s, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone)) || planes_pool(&pool) != cudaSuccess ||
+      cudaMallocFromPoolAsync(&p, bytes, pool, s) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return {nullptr, false};
+  }
+  return {p, true};
+}
+static cudaError_t give_scratch(const Scratch &t, cudaStream_t s) { return t.pooled ? cudaFreeAsync(t.p, s) : cudaSuccess; }
+
 // the join behind a GEMM in parts of k
 static cudaError_t launch_join(const W4A16Args &a, cudaStream_t s) {
   cudaLaunchConfig_t cfg;
@@ -1200,7 +1225,6 @@ cudaError_t trim_planes_pool() {
 // Fewer tokens came from the DP4A kernel, whose ordered sums are more exact than one chain: they are summed in segments (three planes, a 16-bit D, the
 // plain epilogue; nvfp4a_gemm_ex stays on the DP4A kernel, see GemmArgs::whole_k), and only where the reduction is long enough for that and for the planes to pay: 835 x 2176 on 30 tokens 158 us there, 30 here,
 // 640 x 3840 on 10 tokens 267 and 41, 1024 x 512 on 32 tokens 49 and 17.
-constexpr int kW4A8ChainMinN = 64;
 bool gemm_w4a8_tc_supports(const GemmArgs &g) {
   if (g.B.dtype != NVFP4A_INT8 || g.k < 64 || g.m < 128 || g.no_alloc || g.tp.world > 1 || g.e.gb_stride) return false;
   if (g.n < kW4A8ChainMinN && (g.n <= 8 || g.k < 512 || g.whole_k || g.e.d_dtype == NVFP4A_FP32 || g.x.mask || g.A.ue)) return false;
@@ -1216,26 +1240,25 @@ bool gemm_w4a8_grouped_supports(const GemmArgs &g, int groups) {
   return g.n >= kW4A8ChainMinN && gemm_w4a8_tc_supports(g) && !g.A.image && groups <= kMaxGroups && g.k >= 512 && g.e.d_dtype != NVFP4A_FP32;
 }
 
-// seg == NULL: one weight; else `groups` stacked weights of g.m rows
+// seg == NULL: one weight; else `groups` stacked weights of g.m rows.  Without scratch nothing is launched and cudaErrorMemoryAllocation returned; up to
+// 63 tokens, which the DP4A kernel takes as well, there is none from the pool in a capture.
 cudaError_t launch_gemm_w4a8_tc(const GemmArgs &g, const int *seg, int groups, cudaStream_t s) {
   const bool three = seg || g.n < kW4A8ChainMinN;   // in segments
-  uint16_t *planes = nullptr;
-  cudaMemPool_t pool;
-  cudaError_t e = planes_pool(&pool);
-  if (e != cudaSuccess) return e;
+  const bool in_capture = g.n >= kW4A8ChainMinN;
+  cudaError_t e = cudaSuccess;
   // planes [n][3 or 5][k], n token scales and the word behind them, n marks; the sums of parts of k, if there are any
   const int per_token = three ? 3 : 5;
   const size_t plane_bytes = (size_t)g.n * per_token * g.k * sizeof(uint16_t), small_bytes = (plane_bytes + (size_t)(g.n + 1) * sizeof(float) + g.n + 255) / 256 * 256;
   GemmArgs w = g;
-  int parts = seg ? 1 : plan_parts(g, three ? 3 : 2, false, nullptr);
-  if (parts > 1 && cudaMallocFromPoolAsync((void **)&planes, small_bytes + (size_t)parts * g.n * g.m * sizeof(float), pool, s) != cudaSuccess) {
-    (void)cudaGetLastError();
-    planes = nullptr;
-    parts = 1;
-    w.no_alloc = 1;   // k stays whole
+  const int parts = seg ? 1 : plan_parts(g, three ? 3 : 2, false, nullptr);
+  Scratch scratch = {nullptr, false};
+  if (parts > 1) {
+    scratch = take_scratch(small_bytes + (size_t)parts * g.n * g.m * sizeof(float), s, in_capture);
+    if (!scratch.p) w.no_alloc = 1;   // k stays whole
   }
-  if (!planes) e = cudaMallocFromPoolAsync((void **)&planes, small_bytes, pool, s);
-  if (e != cudaSuccess) return e;
+  if (!scratch.p) scratch = take_scratch(small_bytes, s, in_capture);
+  if (!scratch.p) return cudaErrorMemoryAllocation;
+  uint16_t *const planes = (uint16_t *)scratch.p;
   float *const tscale = (float *)((uint8_t *)planes + plane_bytes);
   uint8_t *const wide = (uint8_t *)(tscale + g.n + 1);
   const bool force = three || g.A.ue;   // three BF16 planes whatever the scales (products with UE5M3 scales leave FP16's range)
@@ -1269,11 +1292,12 @@ cudaError_t launch_gemm_w4a8_tc(const GemmArgs &g, const int *seg, int groups, c
       a.tscale = tscale;
       a.seg = seg; a.groups = groups;
       a.partial = (float *)((uint8_t *)planes + small_bytes);
+      g_last_parts = a.parts;
       e = seg ? launch_cfg<3, false, true>(tw, tb, td, pm, a, s) : three ? launch_cfg<3, false>(tw, tb, td, pm, a, s) : launch_cfg<2, false>(tw, tb, td, pm, a, s);
       if (e == cudaSuccess && a.parts > 1) e = launch_join(a, s);
     }
   }
-  const cudaError_t ef = cudaFreeAsync(planes, s);
+  const cudaError_t ef = give_scratch(scratch, s);
   return e != cudaSuccess ? e : ef;
 }
 
@@ -1295,22 +1319,21 @@ cudaError_t launch_gemm_w4a16(const GemmArgs &g, cudaStream_t s) {
     }
   }
   auto go = [&]() { return g.B.dtype == NVFP4A_FP16 ? launch_cfg<1, true>(tw, tb, td, pm, a, s) : launch_cfg<1, false>(tw, tb, td, pm, a, s); };
+  Scratch scratch = {nullptr, false};
   if (a.parts > 1) {
-    // Scratch from the pool; without it, or in a capture (a graph with memory nodes cannot be a child of another, nor be instantiated twice), k stays whole.
-    cudaMemPool_t pool;
-    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusActive;
-    if (cudaStreamIsCapturing(s, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone || planes_pool(&pool) != cudaSuccess ||
-        cudaMallocFromPoolAsync((void **)&a.partial, (size_t)a.parts * g.n * g.m * sizeof(float), pool, s) != cudaSuccess) {
-      (void)cudaGetLastError();
+    scratch = take_scratch((size_t)a.parts * g.n * g.m * sizeof(float), s, false);
+    a.partial = (float *)scratch.p;
+    if (!scratch.p) {   // k stays whole
       GemmArgs whole = g;
       whole.no_alloc = 1;
       if (!set_up(whole, 1, g.B.dtype == NVFP4A_FP16, 0, g.B.data, (uint64_t)g.k * 2, (uint64_t)g.B.ld * 2, &a, &tw, &tb, &td)) return cudaErrorInvalidValue;
     }
   }
+  g_last_parts = a.parts;
   if (a.parts == 1) return go();
   cudaError_t e = go();
   if (e == cudaSuccess) e = launch_join(a, s);
-  const cudaError_t ef = cudaFreeAsync(a.partial, s);
+  const cudaError_t ef = give_scratch(scratch, s);
   return e != cudaSuccess ? e : ef;
 }
 

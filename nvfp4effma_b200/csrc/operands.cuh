@@ -83,8 +83,12 @@ cudaError_t launch_gemm_w4a16(const GemmArgs &g, cudaStream_t s);    // tcgen05 
 bool gemm_w4a16_supports(const GemmArgs &g);
 bool gemm_w4a16_pushes(const GemmArgs &g);
 cudaError_t launch_gemm_w4a8_tc(const GemmArgs &g, const int *seg, int groups, cudaStream_t s);  // INT8 activations as two FP16 or three BF16 planes on the same tcgen05 kernel
+constexpr int kW4A8ChainMinN = 64;   // fewer INT8 tokens: the tensor cores sum in segments, and without scratch the DP4A kernel takes them
 bool gemm_w4a8_tc_supports(const GemmArgs &g);
 bool gemm_w4a8_grouped_supports(const GemmArgs &g, int groups);
+struct ScratchAlloc { void *(*fn)(void *ctx, size_t bytes); void *ctx; };
+void set_scratch_alloc(const ScratchAlloc &a);   // the calling thread's
+int last_parts();                 // parts of k of the calling thread's last W4A16 / W4A8 GEMM
 cudaError_t trim_planes_pool();   // gives the W4A8 planes' pool memory of the current device back to the system
 // s_j of every token (the RMSNorm column scale of the extended epilogue) -> out[0 .. n)
 cudaError_t launch_norm_scales(const EpilogueEx &x, int n, float *out, cudaStream_t s);

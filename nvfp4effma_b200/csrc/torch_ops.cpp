@@ -7,6 +7,7 @@
 #include <map>
 #include <mutex>
 #include <tuple>
+#include <vector>
 #include <ATen/core/Tensor.h>
 #include <ATen/ops/empty.h>
 #include <ATen/ops/zeros.h>
@@ -14,6 +15,7 @@
 #include <c10/cuda/CUDAStream.h>
 #include <torch/library.h>
 #include "../../include/nvfp4effma.h"
+#include "../../include/nvfp4effma_b200.h"
 
 namespace {
 
@@ -166,6 +168,25 @@ struct Bias {
 };
 void check_k(int64_t k) { TORCH_CHECK_VALUE(k % 64 == 0, "k = ", k, ": the reduction length must be a multiple of 64"); }
 
+// The scratch of one GEMM call comes from torch's allocator: no second pool beside it, and a captured call leaves no allocation in the graph and
+// does what it does outside.  Freed when the call is enqueued, to be used again in the order of its stream like any tensor.
+struct CallScratch {
+  const Tensor &like;
+  std::vector<Tensor> held;
+  explicit CallScratch(const Tensor &l) : like(l) { nvfp4a_b200_set_scratch_alloc(&alloc, this); }
+  ~CallScratch() { nvfp4a_b200_set_scratch_alloc(nullptr, nullptr); }
+  CallScratch(const CallScratch &) = delete;
+  static void *alloc(void *ctx, size_t bytes) {
+    CallScratch *const self = (CallScratch *)ctx;
+    try {
+      self->held.push_back(empty({(int64_t)bytes}, at::kByte, self->like));
+      return self->held.back().data_ptr();
+    } catch (...) {   // out of memory: the library does without
+      return nullptr;
+    }
+  }
+};
+
 // ---- linear -----------------------------------------------------------------------------------------------------------------------
 // One nvfp4a_gemm (or nvfp4a_gemv_tc on the weight's image up to 8 tokens) writing `out`; the amax tensor or none.
 OptTensor gemm_into(const Tensor &out, const Tensor &x, const OptTensor &xs, const OptTensor &xg, int64_t xf, int64_t xm, const Tensor &w, const Tensor &ws,
@@ -191,6 +212,7 @@ OptTensor gemm_into(const Tensor &out, const Tensor &x, const OptTensor &xs, con
     check(nvfp4a_gemv_tc((int)N, (int)T, (int)k, (float)alpha, &a, &b.t, (int)b.ld, (float)beta, c, ldc, &d, ldd, bi.p, stream()));
   } else {
     const Operand a = fp4_operand(w, ws, wg, wf, wm);
+    CallScratch scratch(out);
     check(nvfp4a_gemm((int)N, (int)T, (int)k, (float)alpha, &a.t, (int)a.ld, &b.t, (int)b.ld, (float)beta, c, ldc, &d, ldd, bi.p, stream()));
   }
   return amax;
@@ -225,6 +247,7 @@ OptTensor grouped_into(const Tensor &out, const Tensor &x, const OptTensor &xs, 
   const Bias bi(bias, w.size(0));
   const int ldd = (int)out.stride(0);
   const Tensor sg = seg.contiguous();
+  CallScratch scratch(out);
   check(nvfp4a_gemm_grouped((int)groups, (int)N, (int)k, (int)T, (float)alpha, &a.t, (int)a.ld, &b.t, (int)b.ld, (float)beta, beta != 0.0 ? &d : nullptr,
                             beta != 0.0 ? ldd : 0, &d, ldd, bi.p, (const int *)device_ptr(sg, "seg"), stream()));
   return amax;
@@ -288,6 +311,7 @@ OptTensor image_gemm_into(const Tensor &out, const Tensor &x_img, int64_t x_dtyp
   const Bias bi(bias, N);
   const int ldd = (int)out.stride(0);
   const cudaStream_t s = stream();
+  CallScratch scratch(out);
   check(nvfp4a_gemm_tc((int)N, (int)T, (int)K, (float)alpha, &a, &b, (float)beta, beta != 0.0 ? &d : nullptr, beta != 0.0 ? ldd : 0, &d, ldd, bi.p,
                        workspace(w_img, s), s));
   return amax;

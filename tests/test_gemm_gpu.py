@@ -1213,7 +1213,7 @@ def test_long_reductions_of_few_tiles_in_parts_of_k(bt):
             h = build_case(c, 5000 + i)
             exp = oracle_case(c, h, want_ref=True)
             got, amax = run_gemm(c, h)
-            assert L.lib.nvfp4a_b200_last_route() == (8 if bt == L.INT8 else 5), c
+            assert L.lib.nvfp4a_b200_last_route() == (8 if bt == L.INT8 else 5) and L.lib.nvfp4a_b200_last_parts() > 1, c
             check_bound(c, h, got, amax, exp)
             again, amax2 = run_gemm(c, h)
             assert np.array_equal(got.view(np.uint8), again.view(np.uint8)) and amax == amax2, c
@@ -1222,12 +1222,12 @@ def test_long_reductions_of_few_tiles_in_parts_of_k(bt):
                 check_bound(c, h, got, amax, exp)
     dA = DevFp4(h["A"])
     keepB, tB = device_b(c, h)
-    dD = dev(h["Dinit"])
-    tA, tD = dA.tensor(), tensor(dD, c.dt)
-    dC = dev(h["C"]) if h["C"] is not None else None
+    dD, damax = dev(h["Dinit"]), torch.zeros(1, device="cuda")
+    tA, tD = dA.tensor(), tensor(dD, c.dt, amax=damax)
     graph = torch.cuda.CUDAGraph()
     with torch.cuda.graph(graph):
         assert L.lib.nvfp4a_gemm(c.m, c.n, c.k, c.alpha, ctypes.byref(tA), h["lda"], ctypes.byref(tB), h["ldb"], 0.0, None, 0, ctypes.byref(tD), h["ldd"], None, stream()) == 0
+    assert (L.lib.nvfp4a_b200_last_parts() > 1) == (bt == L.INT8)
     graph.replay()
     torch.cuda.synchronize()
     assert c.beta == 0.0 and c.bias < 0
@@ -1239,7 +1239,107 @@ def test_long_reductions_of_few_tiles_in_parts_of_k(bt):
             A0 = DevFp4(rand_fp4(np.random.default_rng(1), c.m, c.k, glob=0.375))
             ta = A0.tensor()
             L.check(entry(c.m, c.n, c.k, 1.0, ctypes.byref(ta), c.k, ctypes.byref(tB), h["ldb"], 0.0, None, 0, ctypes.byref(td), c.m, None, ctypes.byref(ex), stream()))
+            assert L.lib.nvfp4a_b200_last_parts() == 1
             outs.append(d.view(torch.int16))
         assert torch.equal(*outs) and bool(outs[0].any())
-    check_bound(c, h, host(dD).view(h["Dinit"].dtype), exp["amax"], exp)
+    check_bound(c, h, host(dD).view(h["Dinit"].dtype), float(damax), exp)
+    assert kernel_status() == 0
+
+
+def graph_node_types(graph):
+    from cuda.bindings import runtime
+    raw = runtime.cudaGraph_t(graph.raw_cuda_graph())
+    err, nodes, count = runtime.cudaGraphGetNodes(raw)
+    err, nodes, count = runtime.cudaGraphGetNodes(raw, count)
+    assert err == runtime.cudaError_t.cudaSuccess and count > 0
+    return [runtime.cudaGraphNodeGetType(node)[1] for node in nodes], runtime, raw
+
+
+@pytest.mark.parametrize("bt,n", [(L.INT8, 9), (L.INT8, 40), (L.BF16, 46), (L.FP16, 33)])
+def test_captured_calls_leave_no_allocation_in_the_graph(bt, n):
+    """nvfp4a_gemm where eager calls take scratch from the library's pool: a capture has no allocation node, so that the graph can be instantiated twice and be a
+    child of another, and gives results within the bound.  INT8: the exact kernel's bytes."""
+    c = Case(512, n, 4096, bt, L.BF16, -1, -1, 1.0, 0.0)
+    h = build_case(c, 5200 + n)
+    exp = oracle_case(c, h, want_ref=True)
+    run_gemm(c, h)
+    assert L.lib.nvfp4a_b200_last_route() == (8 if bt == L.INT8 else 5)
+    dA, (keep, tB), dD, damax = DevFp4(h["A"]), device_b(c, h), dev(h["Dinit"]), torch.zeros(1, device="cuda")
+    tA, tD = dA.tensor(), tensor(dD, c.dt, amax=damax)
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(graph):
+        assert L.lib.nvfp4a_gemm(c.m, c.n, c.k, 1.0, ctypes.byref(tA), h["lda"], ctypes.byref(tB), h["ldb"], 0.0, None, 0, ctypes.byref(tD), h["ldd"], None, stream()) == 0
+    assert L.lib.nvfp4a_b200_last_route() == (7 if bt == L.INT8 else 5)
+    types, runtime, raw = graph_node_types(graph)
+    assert runtime.cudaGraphNodeType.cudaGraphNodeTypeMemAlloc not in types
+    execs = []
+    for _ in range(2):
+        err, ex = runtime.cudaGraphInstantiate(raw, 0)
+        assert err == runtime.cudaError_t.cudaSuccess
+        execs.append(ex)
+    err, parent = runtime.cudaGraphCreate(0)
+    err, node = runtime.cudaGraphAddChildGraphNode(parent, None, 0, raw)
+    assert err == runtime.cudaError_t.cudaSuccess
+    err, ex = runtime.cudaGraphInstantiate(parent, 0)
+    assert err == runtime.cudaError_t.cudaSuccess
+    for e in execs + [ex]:
+        dD.copy_(dev(h["Dinit"]))
+        damax.zero_()
+        assert runtime.cudaGraphLaunch(e, torch.cuda.current_stream().cuda_stream)[0] == runtime.cudaError_t.cudaSuccess
+        torch.cuda.synchronize()
+        check_bound(c, h, host(dD).view(h["Dinit"].dtype), float(damax), exp)
+        if bt == L.INT8:
+            old = L.lib.nvfp4a_b200_set_route(3)
+            exact = run_gemm(c, h)[0]
+            L.lib.nvfp4a_b200_set_route(old)
+            assert np.array_equal(host(dD).view(np.uint8), exact.view(np.uint8))
+    for e in execs + [ex]:
+        runtime.cudaGraphExecDestroy(e)
+    runtime.cudaGraphDestroy(parent)
+    assert kernel_status() == 0
+
+
+def test_scratch_from_the_callers_allocator_and_without_any():
+    """nvfp4a_b200_set_scratch_alloc: the bytes of the pool's calls, one request a call, nothing from the pool; where the allocator has nothing, 16-bit activations keep
+    k whole, 9 to 63 INT8 tokens take the exact kernel and 64 INT8 tokens report it."""
+    kind = ctypes.CFUNCTYPE(ctypes.c_void_p, ctypes.c_void_p, ctypes.c_size_t)
+    held, asked = [], []
+
+    def give(ctx, size):
+        asked.append(size)
+        held.append(torch.empty(size, dtype=torch.uint8, device="cuda"))
+        return held[-1].data_ptr()
+
+    def none(ctx, size):
+        asked.append(size)
+        return None
+
+    give_c, none_c = kind(give), kind(none)
+    for bt, n, route in ((L.INT8, 16, 8), (L.INT8, 130, 8), (L.BF16, 46, 5), (L.FP16, 33, 5)):
+        c = Case(512, n, 8192, bt, L.BF16, -1, -1, 1.0, 0.0)
+        h = build_case(c, 5300 + n)
+        exp = oracle_case(c, h, want_ref=True)
+        pool = run_gemm(c, h)
+        assert L.lib.nvfp4a_b200_last_route() == route and L.lib.nvfp4a_b200_last_parts() > 1
+        try:
+            L.lib.nvfp4a_b200_set_scratch_alloc(give_c, None)
+            del asked[:]
+            got = run_gemm(c, h)
+            assert len(asked) == 1 and L.lib.nvfp4a_b200_last_route() == route and L.lib.nvfp4a_b200_last_parts() > 1
+            assert np.array_equal(got[0].view(np.uint8), pool[0].view(np.uint8)) and got[1] == pool[1]
+            L.lib.nvfp4a_b200_set_scratch_alloc(none_c, None)
+            del asked[:]
+            if bt == L.INT8 and n >= 64:
+                with pytest.raises(AssertionError, match="memory"):
+                    run_gemm(c, h)
+            else:
+                got = run_gemm(c, h)
+                assert L.lib.nvfp4a_b200_last_route() == (7 if bt == L.INT8 else 5)
+                assert bt == L.INT8 or L.lib.nvfp4a_b200_last_parts() == 1
+                check_bound(c, h, got[0], got[1], exp)
+            assert 1 <= len(asked) <= 2
+        finally:
+            L.lib.nvfp4a_b200_set_scratch_alloc(None, None)
+        assert np.array_equal(run_gemm(c, h)[0].view(np.uint8), pool[0].view(np.uint8))
+        del held[:]
     assert kernel_status() == 0

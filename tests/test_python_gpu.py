@@ -471,3 +471,26 @@ def test_a_quantized_tensor_is_what_the_constructor_makes_of_its_parts(shape):
             assert got == full and [type(got[n]) for n in got] == [type(full[n]) for n in got] and t.flags == want.flags and t.shape == want.shape
     with pytest.raises(ValueError):
         nf.quantize(x, scale_max=300)
+
+
+@pytest.mark.parametrize("act,dtype,tokens,n,k", [("int8", torch.bfloat16, 16, 512, 4096), ("int8", torch.bfloat16, 150, 640, 4096), ("exact", torch.bfloat16, 46, 2688, 4736),
+                                                  ("exact", torch.float16, 33, 512, 8192)])
+def test_a_captured_linear_gives_the_bytes_of_an_eager_one(act, dtype, tokens, n, k):
+    """Scratch of a linear is torch's memory: a capture takes the kernels of an eager call, leaves no allocation in the graph, and its replays give the same bytes."""
+    from nvfp4effma_b200 import _lib as L
+    from test_gemm_gpu import graph_node_types
+    w = nf.quantize(normal((n, k), torch.bfloat16, seed=n))
+    x = normal((tokens, k), dtype, seed=tokens)
+    want = nf.linear(x, w, act=act)
+    route, parts = L.lib.nvfp4a_b200_last_route(), L.lib.nvfp4a_b200_last_parts()
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(graph):
+        y = nf.linear(x, w, act=act)
+    assert L.lib.nvfp4a_b200_last_route() == route and L.lib.nvfp4a_b200_last_parts() == parts > 1
+    types, runtime, raw = graph_node_types(graph)
+    assert runtime.cudaGraphNodeType.cudaGraphNodeTypeMemAlloc not in types
+    graph.instantiate()
+    for _ in range(2):
+        y.zero_()
+        graph.replay()
+        assert torch.equal(y, want)
