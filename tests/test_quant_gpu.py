@@ -343,6 +343,57 @@ def test_blocks_of_32_bytes_at_every_alignment(dtype, offset, pad):
         assert bool((back[: offset // esz] == 7).all()) and bool((out[:, cols:] == 7).all()) and bool((back[offset // esz + rows * ld:] == 7).all())
 
 
+@pytest.mark.parametrize("offset,pad", [(0, 0), (16, 0), (0, 16), (16, 48)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+def test_both_directions_at_every_alignment(dtype, offset, pad):
+    """The one-read kernel of both directions takes a block's 32 bytes in one load where base and pitch allow it: the same bytes as from an aligned copy, with
+    64-row and 256-row tiles and remainders of both."""
+    import nvfp4effma_b200.api as nf
+    esz, code = torch.empty(0, dtype=dtype).element_size(), {torch.bfloat16: L.BF16, torch.float16: L.FP16, torch.float32: L.FP32}[dtype]
+    for rows, cols in ((80, 208), (2064, 2320)):
+        ld = cols + pad
+        gen = torch.Generator(device="cuda").manual_seed(rows + 1)
+        base = torch.randn(rows * ld + 64, generator=gen, device="cuda").to(dtype)
+        x = base[offset // esz:][: rows * ld].view(rows, ld)
+        want = nf.quantize(x[:, :cols].contiguous(), columnwise=True)
+        out = []
+        for r, c in ((rows, cols), (cols, rows)):
+            data, sc = torch.zeros(r, c // 2, dtype=torch.uint8, device="cuda"), torch.zeros(r, (c // 16 + 3) // 4 * 4, dtype=torch.uint8, device="cuda")
+            out.append((data, sc, tensor(data, L.NVFP4, sc, sc.shape[1], torch.zeros(1, device="cuda"), None, L.GLOBAL_AMAX)))
+        S, cfg = tensor(x, code), L.QuantConfig(1, 0, 1)
+        L.check(L.lib.nvfp4a_quantize_ex(ctypes.byref(S), ld, rows, cols, ctypes.byref(out[0][2]), cols, ctypes.byref(out[1][2]), rows, ctypes.byref(cfg), stream()))
+        for (data, sc, _), w, c in ((out[0], want, cols), (out[1], want.columnwise, rows)):
+            assert torch.equal(data, w.data.view(torch.uint8)) and torch.equal(sc[:, : c // 16], w.scales.view(torch.uint8)[:, : c // 16])
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_one_launch_equals_two_on_infinities_nans_and_zeros(dtype):
+    """From 65536 values up the amax and the encoding are one launch: the bytes and the amax of the two-launch path for matrices of zeros, with a NaN of either sign, an
+    infinity, both, nothing but NaNs, subnormals and the largest finite value; rows that end inside a unit; linear and swizzled scales, E4M3 and UE5M3."""
+    import nvfp4effma_b200.api as nf
+    gen = torch.Generator(device="cuda").manual_seed(31)
+    top, tiny = torch.finfo(dtype).max, torch.finfo(dtype).smallest_normal / 4
+    for rows, cols in ((64, 1024), (300, 576), (1031, 2048)):
+        normal = torch.randn(rows, cols, generator=gen, device="cuda")
+        at = torch.randint(0, rows * cols, (5,), generator=gen, device="cuda")
+        cases = [torch.zeros(rows, cols, device="cuda"), torch.full((rows, cols), float("nan"), device="cuda"), normal * tiny, normal]
+        for values in ([float("nan")], [-float("nan"), float("nan")], [float("inf")], [-float("inf"), float("nan"), top], [-top, tiny, -0.0]):
+            x = normal.clone()
+            x.view(-1)[at[: len(values)]] = torch.tensor(values, device="cuda")
+            cases.append(x)
+        for i, x in enumerate(cases):
+            x = x.to(dtype)
+            out = []
+            try:
+                for fused in (1, 0):
+                    L.lib.nvfp4a_b200_set_quant_fused(fused)
+                    q = nf.quantize(x, swizzled=i % 2 == 0, scale_dtype="ue5m3" if i % 3 == 2 else "e4m3")
+                    out.append((q.data.view(torch.uint8), q.scales.view(torch.uint8), q.amax.view(torch.int32)))
+            finally:
+                L.lib.nvfp4a_b200_set_quant_fused(1)
+            assert all(torch.equal(a, b) for a, b in zip(*out)), (rows, cols, i)
+
+
 def test_small_matrices_quantize_in_one_launch_on_several_streams():
     """The cooperative kernel from 65536 values up, many launches on four streams at once (launches of it share a barrier counter and alternate between two
     arrays of maxima): every result has the bytes of the two-launch path."""
