@@ -541,7 +541,10 @@ int gemv_fp4_pinned_splits();   // (gemv_fp4.cu) nvfp4a_b200_set_gemv_splits: 0 
 // takes an SM; 148, 74, 33 and 15 clusters of 1, 2, 4 and 8 by cudaOccupancyMaxActiveClusters): more are not launched, a cluster takes
 // several tiles instead.  Automatic: the cut with the shortest estimate, fitted to CUDA-graph timings of 12 shapes from 1024 x 1024 to 28672 x
 // 4096 and up to 8 vectors (within about 10 %): 4.4 us of set-up and tail (4.8 in a cluster), the stream (36 KiB per chunk at 61 GB/s
-// per CTA or 5.4 TB/s in all), the pieces (0.11 us per chunk and vector past the first) and the tiles' ends, which clusters of eight pay most for.
+// per CTA or 5.4 TB/s in all), the pieces (0.14 us per chunk and vector past the first) and the tiles' ends, which clusters of eight pay most for.
+// The pieces now take 0.11 us.  The estimate keeps 0.14: with 0.11 8192 x 8192 with six to eight vectors would come here (eight: 18.0 us, mma.sync 23.7),
+// a middling gain for calls whose time would then depend on their data -- one activation outside the planes' range, and a CTA leaves the weights to
+// its CUDA cores: 150 us there, 23.7 on the mma.sync GEMV.
 struct GemvCut { int splits, clusters, rounds; double us; };
 static int ntok_of(int n) { return n <= 4 ? 4 : 8; }   // tokens of the kernel instance
 static GemvCut cut_for(int m, int k, int n, int splits) {
@@ -552,7 +555,7 @@ static GemvCut cut_for(int m, int k, int n, int splits) {
   const int rounds = (tiles + cap - 1) / cap, clusters = (tiles + rounds - 1) / rounds, ctas = clusters * splits;
   const double chunk = fmax(0.6, ctas * 36.9e3 / 5.4e6);
   const int more = ntok_of(n) - 1;
-  return {splits, clusters, rounds, (splits > 1 ? 4.8 : 4.4) + (0.1 + 0.11 * nloc) * more + (0.06 * more + (splits == 8 ? 1.2 : 0.05)) * (rounds - 1) + rounds * nloc * chunk};
+  return {splits, clusters, rounds, (splits > 1 ? 4.8 : 4.4) + (0.1 + 0.14 * nloc) * more + (0.06 * more + (splits == 8 ? 1.2 : 0.05)) * (rounds - 1) + rounds * nloc * chunk};
 }
 static GemvCut choose_cut(int m, int k, int n) {
   if (const int f = gemv_fp4_pinned_splits()) return cut_for(m, k, n, f);   // pinned (nvfp4a_b200_set_gemv_splits): that value if the problem can use it
@@ -562,8 +565,8 @@ static GemvCut choose_cut(int m, int k, int n) {
     if (c.splits && (!best.splits || c.us < best.us)) best = c;
   }
   // The mma.sync GEMV has less to set up and takes 3 us and 0.4 us per megabyte (same timings): it keeps small matrices, and middling ones
-  // as the number of vectors grows (28672 x 4096: 30.6 against 20.1 us for four vectors, 33.6 against 22.8 us for eight; 8192 x 8192, eight:
-  // 22.0 against 18.5, which the estimate misses; 4096 x 14336: 17.7 against 16.9 and 18.5 against 23.7; 4096 x 4096, eight: 7.6 against 10.8).
+  // as the number of vectors grows (28672 x 4096: 30.6 against 20.1 us for four vectors, 33.6 against 22.8 us for eight; 8192 x 8192: 19.8
+  // against 14.6 for four, which come here, 23.7 against 18.0 for eight, which do not; 4096 x 14336: 17.7 against 16.9 and 18.5 against 23.7; 4096 x 4096, eight: 7.6 against 10.8).
   if (best.us > 3.0 + 0.405 * (m * (k * 0.5625e-6)) * (1.0 + 0.012 * (n - 1))) best.splits = 0;
   return best;
 }

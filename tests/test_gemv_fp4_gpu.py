@@ -400,3 +400,15 @@ def test_one_and_two_vectors_take_the_tensor_cores_from_32_megabytes_up():
                     L.lib.nvfp4a_b200_set_route(old)
                     assert np.array_equal(got.view(np.uint8), named.view(np.uint8))
     assert kernel_status() == 0
+
+
+def test_which_matrices_several_vectors_take_to_the_tensor_cores():
+    """8192 x 8192 with up to four vectors, not with more: there the mma.sync GEMV, whose time does not depend on the activations, is near enough."""
+    for m, k, n, route in ((8192, 8192, 4, FP4_GEMV), (8192, 8192, 6, 2), (8192, 8192, 8, 2), (14336, 4096, 8, FP4_GEMV), (4096, 14336, 3, 2), (4096, 4096, 8, 2)):
+        A = DevFp4(O.Fp4(m, k, flags=SW))
+        x, y = torch.ones(n, k, dtype=torch.bfloat16, device="cuda"), torch.ones(n, m, dtype=torch.bfloat16, device="cuda")
+        ta, tb, td = A.tensor(), tensor(x, L.BF16), tensor(y, L.BF16)
+        L.check(L.lib.nvfp4a_gemm(m, n, k, 1.0, ctypes.byref(ta), k, ctypes.byref(tb), k, 0.0, None, 0, ctypes.byref(td), m, None, stream()))
+        assert L.lib.nvfp4a_b200_last_route() == route, (m, k, n)
+        assert not bool(y.any())
+    assert kernel_status() == 0
