@@ -22,7 +22,7 @@
 //               plain or extended epilogue (RMSNorm column scale, SwiGLU, second output + sums of squares), D through
 //               shared-memory staging tiles and TMA stores when its layout allows
 //   warps 12-19 weight expansion, two groups of four warps on alternate pairs of stages.  The eight magnitudes of E2M1 times a block scale
-//               are eight 16-bit floats (exact: 2 x 4 significant bits); a 4 KiB table holds their high and low bytes for each of
+//               are eight 16-bit floats (exact: 2 x 4 significant bits); a 4 KiB table (PLANES = 2: one for FP16 and one for BF16) holds their high and low bytes for each of
 //               the 256 scale codes, so a block costs one 16-byte table read and four values cost three byte permutes (the packed
 //               nibbles ARE the permute's selectors: high bytes, low bytes, signs), two of them again to interleave, and two
 //               logical operations -- 2 instructions per value where shifts, masks, the multiply and reordering took 3.
@@ -80,7 +80,7 @@ struct W4A16Args {
   unsigned *status;
   unsigned tag;  // this launch's tag in the status word
   int d_tma;     // the output goes through the staging tiles and TMA stores (SwiGLU: 64 output rows per tile)
-  int width;     // tokens per tile: 64, 128 or 256
+  int width;     // tokens per tile: 64, 128, 192 or 256
   int nfull, cut;   // tiles 0 .. nfull - 1 are `width` tokens wide; the rest (to `tiles`) are parts of width / cut tokens
   int tiles;
   int seg_stages;   // F16, GROUPED: stages per segment of k
@@ -466,7 +466,7 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
       const Tile p = tile_of(t);
       if (p.width == 0) continue;
       const int tm = 2 * p.tm + rank, jt = p.j0, jend = min(p.j0 + p.width, p.jend);
-      // this warp's block: width / 2 columns, one, two or four chunks of 32
+      // this warp's block: width / 2 columns, one to four chunks of 32
       const int hw = p.width >> 1, nchunks = min(hw, jend - jt - half * hw + 31) >> 5;   // (chunks past the last token are left alone)
       uint32_t r[32], rn[32];
       auto load_chunk = [&](uint32_t col, int c, uint32_t (&v)[32]) {
@@ -862,7 +862,7 @@ Plan make_plan(int rows256, int n, int planes, int pairs, int widest) {
     if (w > 64 && (w > 128 ? w - 64 : w / 2) >= n) continue;   // the next width covers every token
     const int tiles = rows256 * ((n + w - 1) / w), rest = tiles % pairs;
     int cut = 1;
-    while (w != 192 && tiles > pairs && rest && w / (2 * cut) >= kNarrow && rest * 2 * cut <= pairs) cut *= 2;
+    while (tiles > pairs && rest && w / (2 * cut) >= kNarrow && rest * 2 * cut <= pairs) cut *= 2;
     const long long c = tiles / pairs * stage_cost(w, planes) + (rest ? stage_cost(w / cut, planes) : 0);
     if (!best.width || c < best_cost) {
       best_cost = c;
@@ -873,11 +873,12 @@ Plan make_plan(int rows256, int n, int planes, int pairs, int widest) {
 }
 
 // Parts of k.  A problem with few tiles leaves most SM pairs idle while each tile is a serial chain over k (0.3 to 0.6 us per 64 values).  Up to eight pairs
-// take a run of at least 512 values each; their FP32 sums meet in memory, which is L2, and a small kernel adds them in order.  That kernel, its launch and
+// take a run of at least 512 values each (the last one what is left); their FP32 sums meet in memory, which is L2, and a small kernel adds them in order.  That kernel, its launch and
 // the memory cost 8 us of a caller's time and the traffic (0.5 ns per KB), so that k has to be long enough to gain more.  A call in eager mode: INT8
 // 4928 x 4608 on 35 tokens 47.8 -> 30.2 us, 832 x 4480 on 12 45.6 -> 28.2, BF16 2688 x 4736 on 46 25.3 -> 17.0; with less to gain, INT8 2594 x 1792 on
 // 12 tokens 26.3 -> 28.5 and BF16 872 x 5376 on 1030 29.6 -> 31.2, which this rule leaves whole.
-// Not for nvfp4a_gemm_ex (see GemmArgs::whole_k), nor for images of BF16 problems: the outputs of a tensor-parallel shard are those of the whole matrix bit for bit, however many tiles either has.
+// (The number of tiles decides: a plain weight's rows and a shard of them may be cut differently and then differ in the last bits.)  Not for nvfp4a_gemm_ex (see
+// GemmArgs::whole_k), nor for images of BF16 problems: the outputs of a tensor-parallel shard are those of the whole matrix bit for bit, however many tiles either has.
 int choose_parts(const GemmArgs &g, int planes, const Plan &p, int pairs) {
   const bool tp_twin = g.A.image && g.B.dtype == NVFP4A_BF16;
   if (tp_twin || g.no_alloc || g.whole_k || g.tp.world > 1 || g.x.mask || p.cut > 1 || 2 * p.tiles > pairs) return 1;

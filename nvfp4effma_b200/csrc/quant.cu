@@ -200,8 +200,8 @@ __global__ void __launch_bounds__(256) amax_rows_kernel(const uint8_t *__restric
 // four scales of a 64-value group are contiguous too.  Units are visited from the END of the matrix: after an amax pass
 // the tail of the matrix is what L2 still holds.
 template <int T> struct PackedBlock { uint4 w[T == NVFP4A_FP32 ? 4 : 2]; };
-// (wide: the address is a multiple of 32.  A block's 32 bytes in one load: two of 16 bytes touch every sector twice.  8192 x 8192 BF16 with the amax computed
-// 53.6 -> 51.6 us, 4096 x 8192 FP32 53.6 -> 46.9)
+// (wide: the address is a multiple of 32.  A block's 32 bytes in one load: two of 16 bytes touch every sector twice.  4096 x 8192 FP32 with the amax computed,
+// in a CUDA graph over three inputs, 54.6 -> 47.1 us; 8192 x 8192 BF16 55.2 and 55.4, over one input 51.5 and 50.2)
 template <int T>
 __device__ __forceinline__ PackedBlock<T> load_block(const uint8_t *p, bool live, uint64_t policy, bool wide = false) {
   PackedBlock<T> b;
@@ -329,8 +329,8 @@ __global__ void __launch_bounds__(256, 3) quant_rows_kernel(const uint8_t *__res
 // keeps its last four units in registers and the six before them in shared memory (10 x 2 KiB x 16 warps = 320 KiB per SM, 47 MB
 // over the chip: a third of an 8192 x 8192 BF16 matrix).  After the barrier every step of a warp encodes one on-chip unit and one
 // unit read again from memory (in descending order), whose load was issued a step earlier.
-// Measured on 8192 x 8192: HBM traffic 159 MB against 287 MB for the two launches, the same 55 us -- the encode arithmetic (about
-// 170 instructions per block of 16) at 16 warps per SM, not memory, is what bounds the second visit.
+// Measured on 8192 x 8192: HBM traffic 206 MB against 287 MB for the two launches, the same 55 us.  Not memory bounds the second visit but latency: an SM's 16 warps,
+// each with one chain of about 170 instructions per block of 16, fill 43 % of the issue slots, while quant_rows_kernel encodes the whole matrix in 28 us.
 // Per-CTA maxima meet in a device array (no atomics on floats, no memset launch): every CTA reads all of them after the barrier.
 // (A launch on another stream may begin while this one's last CTAs run -- a CTA takes a whole SM, so its own barrier opens only when they have left.  Launches
 // therefore alternate between two arrays of maxima: nobody writes what a late CTA of the launch before is still to read.)
@@ -1071,7 +1071,7 @@ extern "C" nvfp4a_status nvfp4a_quantize_ex(const nvfp4a_tensor *src, int lds, i
   const uint8_t *s = (const uint8_t *)src->data;
   const int bpr = cols / 16;
   // One-read path: the common recipe (rowwise 1 x 16 blocks, one amax for the tensor, no 4over6, 16-bit source) runs as ONE cooperative kernel
-  // that reads most of the source once (quant_fused_kernel) -- all of it up to 9.7 M values, and one launch where there were a fill, the amax pass and
+  // that reads most of the source once (quant_fused_kernel) -- all of it up to 24.2 M values (10 units of 1024 in each of 148 x 16 warps), and one launch where there were a fill, the amax pass and
   // the encode: 256 x 1024 7.9 -> 6.2 us, 1024 x 2048 9.8 -> 7.2, 1500 x 4096 12.5 -> 10.3 (2048 x 4096 and up as before).
   if (c.compute_amax && rowwise && !columnwise && c.tile_rows == 1 && c.four_over_six == NVFP4A_4OVER6_OFF &&
       !(rowwise->flags & NVFP4A_GLOBAL_PER_ROW) && src->dtype != NVFP4A_FP32 && (bpr & 3) == 0 && (long long)rows * cols >= (1ll << 16) &&
