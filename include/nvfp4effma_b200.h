@@ -102,6 +102,7 @@ nvfp4a_status nvfp4a_b200_trim_scratch(void);
  * graph with such nodes cannot be a child of another, nor be instantiated twice).  Without scratch, and in a capture without an allocator, 16-bit
  * activations keep k whole and 9 to 63 INT8 tokens take the exact DP4A kernel; 64 and more INT8 tokens take pool memory in a capture too. */
 void nvfp4a_b200_set_scratch_alloc(void *(*alloc)(void *ctx, size_t bytes), void *ctx);
+void nvfp4a_b200_get_scratch_alloc(void *(**alloc)(void *ctx, size_t bytes), void **ctx);   /* what the calling thread has set */
 
 /* The number of parts that the calling thread's last W4A16 / W4A8 tensor-core GEMM cut k into (1: whole).  Test aid. */
 int nvfp4a_b200_last_parts(void);

@@ -103,6 +103,7 @@ _PROTOS = {
     "nvfp4a_b200_set_pdl": (_i, [_i]),
     "nvfp4a_b200_trim_scratch": (_i, []),
     "nvfp4a_b200_set_scratch_alloc": (None, [_v, _v]),
+    "nvfp4a_b200_get_scratch_alloc": (None, [C.POINTER(_v), C.POINTER(_v)]),
     "nvfp4a_b200_last_parts": (_i, []),
 }
 EXPORTS = tuple(_PROTOS)

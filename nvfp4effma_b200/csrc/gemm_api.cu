@@ -360,6 +360,12 @@ extern "C" int nvfp4a_b200_last_parts(void) { return last_parts(); }
 
 extern "C" void nvfp4a_b200_set_scratch_alloc(void *(*alloc)(void *ctx, size_t bytes), void *ctx) { set_scratch_alloc({alloc, ctx}); }
 
+extern "C" void nvfp4a_b200_get_scratch_alloc(void *(**alloc)(void *ctx, size_t bytes), void **ctx) {
+  const ScratchAlloc a = get_scratch_alloc();
+  if (alloc) *alloc = a.fn;
+  if (ctx) *ctx = a.ctx;
+}
+
 extern "C" nvfp4a_status nvfp4a_b200_trim_scratch(void) {
   clear_error();
   return cuda_fail(trim_planes_pool(), "nvfp4a_b200_trim_scratch");

@@ -1180,6 +1180,7 @@ static cudaError_t planes_pool(cudaMemPool_t *pool) {
 // instantiated twice: only calls that have no other kernel with a like result take it there (`in_capture`).
 static thread_local ScratchAlloc g_scratch_alloc = {nullptr, nullptr};
 void set_scratch_alloc(const ScratchAlloc &a) { g_scratch_alloc = a; }
+ScratchAlloc get_scratch_alloc() { return g_scratch_alloc; }
 static thread_local int g_last_parts = 0;
 int last_parts() { return g_last_parts; }
 struct Scratch { void *p; bool pooled; };

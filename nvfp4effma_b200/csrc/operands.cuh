@@ -88,6 +88,7 @@ bool gemm_w4a8_tc_supports(const GemmArgs &g);
 bool gemm_w4a8_grouped_supports(const GemmArgs &g, int groups);
 struct ScratchAlloc { void *(*fn)(void *ctx, size_t bytes); void *ctx; };
 void set_scratch_alloc(const ScratchAlloc &a);   // the calling thread's
+ScratchAlloc get_scratch_alloc();
 int last_parts();                 // parts of k of the calling thread's last W4A16 / W4A8 GEMM
 cudaError_t trim_planes_pool();   // gives the W4A8 planes' pool memory of the current device back to the system
 // s_j of every token (the RMSNorm column scale of the extended epilogue) -> out[0 .. n)

@@ -169,17 +169,22 @@ struct Bias {
 void check_k(int64_t k) { TORCH_CHECK_VALUE(k % 64 == 0, "k = ", k, ": the reduction length must be a multiple of 64"); }
 
 // The scratch of one GEMM call comes from torch's allocator: no second pool beside it, and a captured call leaves no allocation in the graph and
-// does what it does outside.  Freed when the call is enqueued, to be used again in the order of its stream like any tensor.
+// does what it does outside.  Of the current device (the output may be pinned host memory).  Freed when the call is enqueued, to be used again in the
+// order of its stream like any tensor.  An allocator that the thread has set for itself is back afterwards.
 struct CallScratch {
-  const Tensor &like;
   std::vector<Tensor> held;
-  explicit CallScratch(const Tensor &l) : like(l) { nvfp4a_b200_set_scratch_alloc(&alloc, this); }
-  ~CallScratch() { nvfp4a_b200_set_scratch_alloc(nullptr, nullptr); }
+  void *(*old)(void *, size_t) = nullptr;
+  void *old_ctx = nullptr;
+  CallScratch() {
+    nvfp4a_b200_get_scratch_alloc(&old, &old_ctx);
+    nvfp4a_b200_set_scratch_alloc(&alloc, this);
+  }
+  ~CallScratch() { nvfp4a_b200_set_scratch_alloc(old, old_ctx); }
   CallScratch(const CallScratch &) = delete;
   static void *alloc(void *ctx, size_t bytes) {
     CallScratch *const self = (CallScratch *)ctx;
     try {
-      self->held.push_back(empty({(int64_t)bytes}, at::kByte, self->like));
+      self->held.push_back(at::empty({(int64_t)bytes}, at::TensorOptions().dtype(at::kByte).device(at::kCUDA)));
       return self->held.back().data_ptr();
     } catch (...) {   // out of memory: the library does without
       return nullptr;
@@ -212,7 +217,7 @@ OptTensor gemm_into(const Tensor &out, const Tensor &x, const OptTensor &xs, con
     check(nvfp4a_gemv_tc((int)N, (int)T, (int)k, (float)alpha, &a, &b.t, (int)b.ld, (float)beta, c, ldc, &d, ldd, bi.p, stream()));
   } else {
     const Operand a = fp4_operand(w, ws, wg, wf, wm);
-    CallScratch scratch(out);
+    CallScratch scratch;
     check(nvfp4a_gemm((int)N, (int)T, (int)k, (float)alpha, &a.t, (int)a.ld, &b.t, (int)b.ld, (float)beta, c, ldc, &d, ldd, bi.p, stream()));
   }
   return amax;
@@ -247,7 +252,7 @@ OptTensor grouped_into(const Tensor &out, const Tensor &x, const OptTensor &xs, 
   const Bias bi(bias, w.size(0));
   const int ldd = (int)out.stride(0);
   const Tensor sg = seg.contiguous();
-  CallScratch scratch(out);
+  CallScratch scratch;
   check(nvfp4a_gemm_grouped((int)groups, (int)N, (int)k, (int)T, (float)alpha, &a.t, (int)a.ld, &b.t, (int)b.ld, (float)beta, beta != 0.0 ? &d : nullptr,
                             beta != 0.0 ? ldd : 0, &d, ldd, bi.p, (const int *)device_ptr(sg, "seg"), stream()));
   return amax;
@@ -311,7 +316,7 @@ OptTensor image_gemm_into(const Tensor &out, const Tensor &x_img, int64_t x_dtyp
   const Bias bi(bias, N);
   const int ldd = (int)out.stride(0);
   const cudaStream_t s = stream();
-  CallScratch scratch(out);
+  CallScratch scratch;
   check(nvfp4a_gemm_tc((int)N, (int)T, (int)K, (float)alpha, &a, &b, (float)beta, beta != 0.0 ? &d : nullptr, beta != 0.0 ? ldd : 0, &d, ldd, bi.p,
                        workspace(w_img, s), s));
   return amax;

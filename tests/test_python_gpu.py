@@ -494,3 +494,26 @@ def test_a_captured_linear_gives_the_bytes_of_an_eager_one(act, dtype, tokens, n
         y.zero_()
         graph.replay()
         assert torch.equal(y, want)
+
+
+@pytest.mark.parametrize("act,dtype,tokens", [("int8", torch.bfloat16, 16), ("int8", torch.bfloat16, 150), ("exact", torch.bfloat16, 46), ("exact", torch.float16, 33)])
+def test_linear_into_pinned_host_memory(act, dtype, tokens):
+    """The output may be pinned host memory; the call's scratch is the device's all the same.  An allocator that the thread has set stays set, and unused."""
+    import ctypes
+    from nvfp4effma_b200 import _lib as L
+    w, x = nf.quantize(normal((512, 4096), torch.bfloat16, seed=1)), normal((tokens, 4096), dtype, seed=tokens)
+    want = nf.linear(x, w, act=act)
+    assert L.lib.nvfp4a_b200_last_parts() > 1
+    asked = []
+    own = ctypes.CFUNCTYPE(ctypes.c_void_p, ctypes.c_void_p, ctypes.c_size_t)(lambda ctx, size: asked.append(size))
+    fn, ctx = ctypes.c_void_p(), ctypes.c_void_p()
+    try:
+        L.lib.nvfp4a_b200_set_scratch_alloc(own, 77)
+        out = torch.zeros(tokens, 512, dtype=dtype).pin_memory()
+        assert nf.linear(x, w, act=act, out=out) is out
+        L.lib.nvfp4a_b200_get_scratch_alloc(ctypes.byref(fn), ctypes.byref(ctx))
+    finally:
+        L.lib.nvfp4a_b200_set_scratch_alloc(None, None)
+    torch.cuda.synchronize()
+    assert torch.equal(out, want.cpu()) and not asked
+    assert fn.value == ctypes.cast(own, ctypes.c_void_p).value and ctx.value == 77
