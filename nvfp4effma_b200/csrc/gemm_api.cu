@@ -3,6 +3,7 @@
 // reference's host layer (src/gemm_nvfp4effma.cu:465-557, :614-930 there); everything is checked before anything is launched.
 //
 // Routing on sm_100a:
+//   n <= 2, BF16 x, E4M3 scales                         -> mma.sync GEMV on FP16 (gemv_stream.cu), from 32 MB of weights the FP4 GEMV (gemv_fp4.cu)
 //   n <= kGemvMaxN (or k == 0)                          -> streaming split-k GEMV (gemv.cu) when it takes the operand types
 //   NVFP4 x NVFP4, E4M3 scales on both                  -> tcgen05 kind::mxf4nvf4 block-scaled GEMM (gemm_w4a4.cu)
 //   NVFP4 x BF16                                        -> tcgen05 kind::f16 GEMM on weights expanded to exact BF16 (gemm_w4a16.cu)
@@ -118,11 +119,12 @@ static nvfp4a_status dispatch(const char *fn, const GemmArgs &g, cudaStream_t st
     if (!(g.tp.deferred & 2) && g.k > 0 && forced_route() != 2 && gemv_fp4_supports(g)) { g_last_route = 3; return cuda_fail(launch_gemv_fp4(g, stream), fn); }
     if (!(g.tp.deferred & 2) && g.k > 0 && forced_route() != 2 && gemv_fp4_n8_supports(g)) { g_last_route = 3; return cuda_fail(launch_gemv_fp4_n8(g, stream), fn); }
     g_last_route = 2;
-    return cuda_fail(launch_gemv(g, stream), fn);
+    return cuda_fail(gemv_stream_supports(g) ? launch_gemv_stream(g, stream) : launch_gemv(g, stream), fn);
   }
   if (forced_route() == 1) { g_last_route = 1; err = launch_gemm_generic(g, stream); }
   else if (gemv && g.k > 0 && forced_route() != 2 && gemv_fp4_supports(g)) { g_last_route = 3; err = launch_gemv_fp4(g, stream); }
   else if (gemv && g.k > 0 && forced_route() != 2 && gemv_fp4_n8_supports(g)) { g_last_route = 3; err = launch_gemv_fp4_n8(g, stream); }
+  else if (gemv && gemv_stream_supports(g)) { g_last_route = 2; err = launch_gemv_stream(g, stream); }
   else if (gemv && gemv_supports(g)) { g_last_route = 2; err = launch_gemv(g, stream); }
   else if (gemv && g.k > 0 && gemv_blocked_supports(g)) { g_last_route = 6; err = launch_gemv_blocked(g, stream); }
   else if (!gemv && gemm_w4a4_supports(g)) { g_last_route = 4; err = launch_gemm_w4a4(g, stream); }

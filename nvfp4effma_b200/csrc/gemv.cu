@@ -1,4 +1,5 @@
-// Streaming GEMV for decoding: D[m x n] = A[m x k] (NVFP4) * B[n x k]^T with 1 <= n <= 8 and BF16 activations (W4A16).
+// Streaming GEMV for decoding: D[m x n] = A[m x k] (NVFP4) * B[n x k]^T with 1 <= n <= 8 and BF16 activations (W4A16).  (One and two vectors
+// against E4M3 scales have a kernel of their own, gemv_stream.cu.)
 //
 // The kernel is bound by reading A once from HBM (0.5625 bytes per weight), so it is built around 16-byte loads and as
 // few instructions per weight as an exact decode allows:
