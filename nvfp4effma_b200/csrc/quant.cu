@@ -11,6 +11,7 @@
 #include <atomic>
 #include <type_traits>
 #include "common.cuh"
+#include "sm100.cuh"
 
 namespace nvb {
 
@@ -325,12 +326,13 @@ __global__ void __launch_bounds__(256, 3) quant_rows_kernel(const uint8_t *__res
 // The global amax must be known before the first block scale, so the matrix is visited twice; this kernel keeps part of it on the
 // chip between the visits instead of paying a second full trip to HBM.  One CTA per SM (cooperative launch: all CTAs are resident,
 // so the grid barrier between the visits cannot starve), each with a contiguous share of the matrix in units of 64 blocks of one
-// row (2 KiB of 16-bit values), dealt to its 16 warps in turn.  Visit 1 takes the amax, four units per warp in flight.  A warp
-// keeps its last four units in registers and the six before them in shared memory (10 x 2 KiB x 16 warps = 320 KiB per SM, 47 MB
-// over the chip: a third of an 8192 x 8192 BF16 matrix).  After the barrier every step of a warp encodes one on-chip unit and one
+// row (2 KiB of 16-bit values), dealt to its warps in turn.  Visit 1 takes the amax, several units per warp in flight.  For a large matrix there are 24 warps; each
+// keeps its last four units in shared memory and the five before them in tensor memory, which is 256 KiB per SM that nothing else uses here (9 x 2 KiB x
+// 24 warps = 432 KiB per SM, 65 MB over the chip: half of an 8192 x 8192 BF16 matrix).  After the barrier every step of a warp encodes one on-chip unit and one
 // unit read again from memory (in descending order), whose load was issued a step earlier.
-// Measured on 8192 x 8192: HBM traffic 206 MB against 287 MB for the two launches, the same 55 us.  Not memory bounds the second visit but latency: an SM's 16 warps,
-// each with one chain of about 170 instructions per block of 16, fill 43 % of the issue slots, while quant_rows_kernel encodes the whole matrix in 28 us.
+// What bounds it: the second visit is instruction issue (about 150 per block of 16 values, many of them conversions at half rate), so warps count: 16 of them
+// with four more units each in registers (127 registers a thread) take 53.1 us for 8192 x 8192 BF16 where 24 take 49.1 and 32 take 50.0; without tensor memory 16
+// took 56.8.  8192 x 4096 30.0 -> 25.9, 4096 x 4096 17.6 -> 16.8 (CUDA graph, rotating inputs; quant_rows_kernel, one visit, 28.5 us for 8192 x 8192).
 // Per-CTA maxima meet in a device array (no atomics on floats, no memset launch): every CTA reads all of them after the barrier.
 // (A launch on another stream may begin while this one's last CTAs run -- a CTA takes a whole SM, so its own barrier opens only when they have left.  Launches
 // therefore alternate between two arrays of maxima: nobody writes what a late CTA of the launch before is still to read.)
@@ -341,24 +343,30 @@ constexpr int kQfMaxGrid = 1024;
 static __device__ unsigned long long g_qf_arrivals;   // arrivals of every launch so far on this device (each launch adds its grid size, which never changes)
 static __device__ float g_qf_max[2][kQfMaxGrid];   // per-CTA maxima of the current launch and of the one before it
 
-// max |x| of a block of 16-bit values taken on the packed words (bit patterns of non-negative BF16 / FP16 values order like the values)
-template <int T>
-__device__ __forceinline__ float packed_block_max(const PackedBlock<T> &a) {
-  uint32_t pm = 0;
-#pragma unroll
-  for (int q = 0; q < 2; ++q) pm = packed_absmax<T>(packed_absmax<T>(packed_absmax<T>(packed_absmax<T>(pm, a.w[q].x), a.w[q].y), a.w[q].z), a.w[q].w);
-  if (T == NVFP4A_BF16) return fmaxf(__uint_as_float(pm << 16), __uint_as_float(pm & 0xFFFF0000u));
-  const float2 f = __half22float2(*reinterpret_cast<const __half2 *>(&pm));
-  return fmaxf(f.x, f.y);
+// max(m, |a|, |b|): one instruction (NaN counts as nothing, as in fmaxf)
+__device__ __forceinline__ float absmax3(float m, float a, float b) {
+  float d;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(m), "f"(fabsf(a)), "f"(fabsf(b)));
+  return d;
 }
-// quant_block16 with the block's maximum already known
-// (the factor 1 / (scale * S_dec) depends on the scale code only: it comes from a 256-entry table the CTA fills once)
-template <bool UE>
-__device__ __forceinline__ uint2 quant_block16_given_max(float v[16], float bmax, float enc6, const float *inv_of_code, uint32_t &code) {
-  code = UE ? f32_to_ue5m3_sw(fminf(__fmul_rn(bmax, enc6), kFltMax)) : e4m3_encode(fminf(__fmul_rn(bmax, enc6), kFltMax));
-  const float inv = inv_of_code[code];
+__device__ __forceinline__ float absmax16(const float v[16]) {
+  float m0 = 0.f, m1 = 0.f;   // (a block of NaNs has the maximum 0)
 #pragma unroll
-  for (int k = 0; k < 16; ++k) v[k] = __fmul_rn(v[k], inv);
+  for (int k = 0; k < 16; k += 4) { m0 = absmax3(m0, v[k], v[k + 1]); m1 = absmax3(m1, v[k + 2], v[k + 3]); }
+  return fmaxf(m0, m1);
+}
+// v *= f, two values an instruction; each product rounded by itself as __fmul_rn does
+__device__ __forceinline__ void scale16(float v[16], float f) {
+#pragma unroll
+  for (int k = 0; k < 16; k += 2)
+    asm("{\n\t.reg .b64 a, b, d;\n\tmov.b64 a, {%0, %1};\n\tmov.b64 b, {%2, %2};\n\tmul.rn.f32x2 d, a, b;\n\tmov.b64 {%0, %1}, d;\n\t}" : "+f"(v[k]), "+f"(v[k + 1]) : "f"(f));
+}
+// quant_block16 with the factor 1 / (scale * S_dec), which depends on the scale code only, from a 256-entry table that the CTA fills once
+template <bool UE>
+__device__ __forceinline__ uint2 quant_block16_by_table(float v[16], float enc6, const float *inv_of_code, uint32_t &code, float &bmax) {
+  bmax = absmax16(v);
+  code = UE ? f32_to_ue5m3_sw(fminf(__fmul_rn(bmax, enc6), kFltMax)) : e4m3_encode(fminf(__fmul_rn(bmax, enc6), kFltMax));
+  scale16(v, inv_of_code[code]);
   return make_uint2(e2m1_pack8(v), e2m1_pack8(v + 8));
 }
 // the two blocks (lane and lane + 32 of a 64-block unit) a lane owns, encoded and stored: nibbles, and the scale bytes as words
@@ -366,12 +374,12 @@ __device__ __forceinline__ uint2 quant_block16_given_max(float v[16], float bmax
 template <int T, bool UE>
 __device__ __forceinline__ void emit_two_blocks(const PackedBlock<T> a0, const PackedBlock<T> a1, int r, int c0, int c1, bool live0, bool live1,
                                              float enc6, const float *inv_of_code, uint8_t *data, int ldq, uint8_t *sc, const ScalePos sp, bool words, int lane) {
-  float v[16];
+  float v[16], bmax;
   uint32_t code0, code1;
   unpack_block<T>(a0, v);
-  const uint2 q0 = quant_block16_given_max<UE>(v, packed_block_max<T>(a0), enc6, inv_of_code, code0);
+  const uint2 q0 = quant_block16_by_table<UE>(v, enc6, inv_of_code, code0, bmax);
   unpack_block<T>(a1, v);
-  const uint2 q1 = quant_block16_given_max<UE>(v, packed_block_max<T>(a1), enc6, inv_of_code, code1);
+  const uint2 q1 = quant_block16_by_table<UE>(v, enc6, inv_of_code, code1, bmax);
   uint8_t *drow = data + (size_t)r * ldq;
   if (live0) __stcs((uint2 *)(drow + 8 * c0), q0);
   if (live1) __stcs((uint2 *)(drow + 8 * c1), q1);
@@ -392,10 +400,12 @@ __device__ __forceinline__ void emit_two_blocks(const PackedBlock<T> a0, const P
 
 template <int T, bool UE, int WARPS>
 __global__ void __launch_bounds__(WARPS * 32, 1)
-quant_fused_kernel(const uint8_t *__restrict__ src, int lds, int rows, int bpr, QOut o, float *gout, float *stat, unsigned *status, unsigned tag) {
+quant_fused_kernel(const uint8_t *__restrict__ src, int lds, int rows, int bpr, unsigned div_mul, int div_shift, QOut o, float *gout, float *stat, unsigned *status, unsigned tag) {
   static_assert(T != NVFP4A_FP32, "16-bit sources");
   extern __shared__ uint4 qf_keep[];   // [warp][unit][4 words][32 lanes]
-  constexpr int kQfWarps = WARPS, kQfRegUnits = WARPS == 16 ? 4 : 0, kQfSmemUnits = 96 / WARPS, kFlight = WARPS == 16 ? 4 : 2;
+  constexpr bool kTmem = WARPS == 24;               // 24 warps: tensor memory; 16: registers
+  constexpr int kQfWarps = WARPS, kQfRegUnits = kTmem ? 0 : 4, kQfSmemUnits = 96 / WARPS, kFlight = kTmem ? 2 : 4;
+  constexpr int kQfTmemUnits = kTmem ? 32 / (WARPS / 4) : 0;    // 512 columns of tensor memory, 16 to a unit; a warp reaches a quarter of the lanes, WARPS / 4 warps share a quarter
   __shared__ float warp_max[kQfWarps];
   __shared__ float gmax_s;
   __shared__ float inv_of_code[256];
@@ -405,9 +415,18 @@ quant_fused_kernel(const uint8_t *__restrict__ src, int lds, int rows, int bpr, 
   const unsigned u_begin = (unsigned)(U * blockIdx.x / gridDim.x), u_end = (unsigned)(U * (blockIdx.x + 1) / gridDim.x);
   const int n_cta = (int)(u_end - u_begin);
   const int n_w = n_cta > warp ? (n_cta - warp + kQfWarps - 1) / kQfWarps : 0;   // this warp's units: u_begin + warp + 16 j
-  // of a warp's units the last n_rg stay in registers, the n_sm before them in shared memory; the first n_glob are read again
-  const int n_ret = n_w < kQfRegUnits + kQfSmemUnits ? n_w : kQfRegUnits + kQfSmemUnits;
-  const int n_rg = n_ret < kQfRegUnits ? n_ret : kQfRegUnits, n_sm = n_ret - n_rg, n_glob = n_w - n_ret;
+  // of a warp's units the last n_rg stay in registers, the n_sm before them in shared memory, the n_tm before those in tensor memory; the first n_glob are read again
+  const int n_ret = min(n_w, kQfRegUnits + kQfSmemUnits + kQfTmemUnits);
+  const int n_rg = min(n_ret, kQfRegUnits), n_sm = min(n_ret - n_rg, kQfSmemUnits), n_tm = n_ret - n_rg - n_sm, n_glob = n_w - n_ret;
+  const bool use_tmem = kTmem && n_cta > kQfWarps * kQfSmemUnits;   // (of the CTA)
+  __shared__ uint32_t tmem_slot;
+  if (use_tmem) {
+    if (warp == 0) sm100::tmem_alloc(&tmem_slot, 512);
+    sm100::tc_fence_before();
+    __syncthreads();
+    sm100::tc_fence_after();
+  }
+  const uint32_t my_tmem = (use_tmem ? tmem_slot : 0u) + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)(warp >> 2) * (16 * kQfTmemUnits);
   const size_t row_bytes = (size_t)lds * 2;
   const bool wide = ((uintptr_t)src & 31) == 0 && (row_bytes & 31) == 0;
   // every load tells L2 to drop the line early: asking it to keep lines (evict_last) slowed the first visit from 22 to 28 us and
@@ -416,7 +435,7 @@ quant_fused_kernel(const uint8_t *__restrict__ src, int lds, int rows, int bpr, 
   uint4 *const my_smem = qf_keep + (size_t)warp * kQfSmemUnits * 128;
   struct Unit { int r, c0; };
   auto unit_of = [&](int j) {
-    const unsigned u = u_begin + warp + (unsigned)(kQfWarps * j), r = u / (unsigned)upr;
+    const unsigned u = u_begin + warp + (unsigned)(kQfWarps * j), r = (unsigned)(((unsigned long long)u * div_mul) >> div_shift);
     return Unit{(int)r, (int)(u - r * (unsigned)upr) * 64 + lane};
   };
   auto load_unit = [&](int j, uint64_t pol, PackedBlock<T> &a0, PackedBlock<T> &a1) {
@@ -445,16 +464,30 @@ quant_fused_kernel(const uint8_t *__restrict__ src, int lds, int rows, int bpr, 
 #pragma unroll
     for (int q = 0; q < 2 * kFlight; ++q) pm = absmax_of(pm, x[q]);
   }
-  for (; j < n_glob + n_sm; ++j) {    // the rest of those, then the units that stay in shared memory
-    PackedBlock<T> a0, a1;
-    load_unit(j, drop_pol, a0, a1);
-    pm = absmax_of(absmax_of(pm, a0), a1);
-    if (j >= n_glob) {
-      uint4 *d = my_smem + (j - n_glob) * 128 + lane;
-      d[0] = a0.w[0]; d[32] = a0.w[1]; d[64] = a1.w[0]; d[96] = a1.w[1];
+  for (; j < n_glob + n_tm + n_sm; j += 2) {    // the rest of those, then the units that stay in tensor memory and in shared memory; two in flight
+    PackedBlock<T> x[4];
+    const bool two = j + 1 < n_glob + n_tm + n_sm;
+    load_unit(j, drop_pol, x[0], x[1]);
+    if (two) load_unit(j + 1, drop_pol, x[2], x[3]);
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      if (h && !two) break;
+      const PackedBlock<T> &a0 = x[2 * h], &a1 = x[2 * h + 1];
+      pm = absmax_of(absmax_of(pm, a0), a1);
+      const int k = j + h - n_glob;
+      if (k >= n_tm) {
+        uint4 *d = my_smem + (k - n_tm) * 128 + lane;
+        d[0] = a0.w[0]; d[32] = a0.w[1]; d[64] = a1.w[0]; d[96] = a1.w[1];
+      } else if (kTmem && k >= 0) {
+        const uint32_t r[16] = {a0.w[0].x, a0.w[0].y, a0.w[0].z, a0.w[0].w, a0.w[1].x, a0.w[1].y, a0.w[1].z, a0.w[1].w,
+                                a1.w[0].x, a1.w[0].y, a1.w[0].z, a1.w[0].w, a1.w[1].x, a1.w[1].y, a1.w[1].z, a1.w[1].w};
+        sm100::tmem_st16(my_tmem + 16 * k, r);
+      }
     }
   }
-  // the last units stay in registers (named, not an array: they must not end up in local memory); all four loads fly together
+  j = n_glob + n_tm + n_sm;
+  if (use_tmem) sm100::tmem_st_wait();
+  // sixteen warps: the last units stay in registers (named, not an array: they must not end up in local memory); all four loads fly together
   PackedBlock<T> rk0_0, rk1_0, rk0_1, rk1_1, rk0_2, rk1_2, rk0_3, rk1_3;
   rk0_0.w[0] = rk0_0.w[1] = make_uint4(0, 0, 0, 0);
   rk1_0 = rk0_1 = rk1_1 = rk0_2 = rk1_2 = rk0_3 = rk1_3 = rk0_0;
@@ -522,7 +555,7 @@ quant_fused_kernel(const uint8_t *__restrict__ src, int lds, int rows, int bpr, 
     const Unit t = unit_of(j);
     emit_two_blocks<T, UE>(x0, x1, t.r, t.c0, t.c0 + 32, t.c0 < bpr, t.c0 + 32 < bpr, enc6, inv_of_code, data, ldq, sc, sp, words, lane);
   };
-  // Interleaved: every step encodes one on-chip unit (registers first, then shared memory) and one re-read unit whose load was
+  // Interleaved: every step encodes one on-chip unit (registers or shared memory first, then tensor memory) and one re-read unit whose load was
   // issued a step earlier, so the arithmetic of the on-chip units hides the latency of the re-reads.  The encoder is a long
   // stretch of code: it appears at two places only (one loop), so that it stays in the instruction cache.
   PackedBlock<T> n0, n1;
@@ -535,11 +568,19 @@ quant_fused_kernel(const uint8_t *__restrict__ src, int lds, int rows, int bpr, 
       if (kQfRegUnits && i < n_rg) {   // (i is the same for the whole warp)
         x0 = i == 0 ? rk0_0 : i == 1 ? rk0_1 : i == 2 ? rk0_2 : rk0_3;
         x1 = i == 0 ? rk1_0 : i == 1 ? rk1_1 : i == 2 ? rk1_2 : rk1_3;
-        j = n_glob + n_sm + i;
-      } else {
+        j = n_glob + n_tm + n_sm + i;
+      } else if (!kTmem || i < n_sm) {
         const uint4 *d = my_smem + (i - n_rg) * 128 + lane;
         x0.w[0] = d[0]; x0.w[1] = d[32]; x1.w[0] = d[64]; x1.w[1] = d[96];
-        j = n_glob + i - n_rg;
+        j = n_glob + n_tm + i - n_rg;
+      } else {
+        uint32_t r[16];
+        const int k = i - n_sm;
+        sm100::tmem_ld16(my_tmem + 16 * k, r);
+        sm100::tmem_ld_wait16(r);
+        x0.w[0] = make_uint4(r[0], r[1], r[2], r[3]); x0.w[1] = make_uint4(r[4], r[5], r[6], r[7]);
+        x1.w[0] = make_uint4(r[8], r[9], r[10], r[11]); x1.w[1] = make_uint4(r[12], r[13], r[14], r[15]);
+        j = n_glob + k;
       }
       emit(j, x0, x1);
     }
@@ -550,7 +591,12 @@ quant_fused_kernel(const uint8_t *__restrict__ src, int lds, int rows, int bpr, 
       --jg;
     }
   }
+  sm100::tc_fence_before();
   __syncthreads();
+  if (use_tmem && warp == 0) {
+    sm100::tc_fence_after();
+    sm100::tmem_dealloc(tmem_slot, 512);
+  }
 }
 
 // ---- pass 2, general path ----------------------------------------------------------------------------------------------
@@ -1011,17 +1057,24 @@ static cudaError_t launch_quant_fused_w(const uint8_t *src, int lds, int rows, i
     (void)cudaGetLastError();
   }
   if (st < 0 || device_sms() > kQfMaxGrid) return cudaErrorNotSupported;
-  if (cudaError_t e = cudaFuncSetAttribute(quant_fused_kernel<T, UE, WARPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, kQfSmemBytes)) return e;
   float *gout = (float *)dst->global_scale, *stat = dst->amax;
   unsigned *status = kernel_status_device_ptr();
   unsigned tag = next_launch_tag();
-  void *args[] = {(void *)&src, (void *)&lds, (void *)&rows, (void *)&bpr, (void *)&o, (void *)&gout, (void *)&stat, (void *)&status, (void *)&tag};
+  // u / upr as a product (upr: units per row): with L = ceil(log2 upr) and M = ceil(2^(31 + L) / upr) < 2^32, floor(u M / 2^(31 + L)) = floor(u / upr) for every u < 2^31
+  const unsigned upr = (unsigned)(bpr + 63) / 64;
+  int div_shift = 31;
+  while ((1u << (div_shift - 31)) < upr) ++div_shift;
+  unsigned div_mul = (unsigned)(((1ull << div_shift) + upr - 1) / upr);
+  void *args[] = {(void *)&src, (void *)&lds, (void *)&rows, (void *)&bpr, (void *)&div_mul, (void *)&div_shift, (void *)&o, (void *)&gout, (void *)&stat, (void *)&status, (void *)&tag};
   return cudaLaunchCooperativeKernel((const void *)quant_fused_kernel<T, UE, WARPS>, dim3(device_sms()), dim3(WARPS * 32), args, kQfSmemBytes, stream);
 }
 template <int T, bool UE>
 static cudaError_t launch_quant_fused(const uint8_t *src, int lds, int rows, int bpr, QOut o, const nvfp4a_tensor *dst, cudaStream_t stream) {
   if ((long long)rows * ((bpr + 63) / 64) >= (1ll << 31)) return cudaErrorNotSupported;
-  return launch_quant_fused_w<T, UE, 16>(src, lds, rows, bpr, o, dst, stream);
+  // Sixteen warps hold four units each in registers, whose loads fly together: what fits there (9.7 M values) takes 0.2 to 1 us less than with 24 warps.
+  // Beyond it those have more on chip and more to issue: 4096 x 4096 16.8 against 17.4 us, 8192 x 8192 49.1 against 53.1.
+  if ((long long)rows * ((bpr + 63) / 64) <= 64ll * device_sms()) return launch_quant_fused_w<T, UE, 16>(src, lds, rows, bpr, o, dst, stream);
+  return launch_quant_fused_w<T, UE, 24>(src, lds, rows, bpr, o, dst, stream);
 }
 
 }  // namespace nvb
@@ -1071,7 +1124,7 @@ extern "C" nvfp4a_status nvfp4a_quantize_ex(const nvfp4a_tensor *src, int lds, i
   const uint8_t *s = (const uint8_t *)src->data;
   const int bpr = cols / 16;
   // One-read path: the common recipe (rowwise 1 x 16 blocks, one amax for the tensor, no 4over6, 16-bit source) runs as ONE cooperative kernel
-  // that reads most of the source once (quant_fused_kernel) -- all of it up to 24.2 M values (10 units of 1024 in each of 148 x 16 warps), and one launch where there were a fill, the amax pass and
+  // that reads most of the source once (quant_fused_kernel) -- all of it up to 32.7 M values (9 units of 1024 in each of 148 x 24 warps), and one launch where there were a fill, the amax pass and
   // the encode: 256 x 1024 7.9 -> 6.2 us, 1024 x 2048 9.8 -> 7.2, 1500 x 4096 12.5 -> 10.3 (2048 x 4096 and up as before).
   if (c.compute_amax && rowwise && !columnwise && c.tile_rows == 1 && c.four_over_six == NVFP4A_4OVER6_OFF &&
       !(rowwise->flags & NVFP4A_GLOBAL_PER_ROW) && src->dtype != NVFP4A_FP32 && (bpr & 3) == 0 && (long long)rows * cols >= (1ll << 16) &&
