@@ -520,7 +520,7 @@ def run_ours(args, rank, world, local_rank):
                                           kernel=routes.get(route_image), timing="CUDA graph of 48 calls, median of 7 replays",
                                           plain_operand={"entry": "nvfp4a_gemm (linear scales)", "us_per_call": ms_gp * 1e3,
                                                          "gbs": gbytes / (ms_gp * 1e-3) / 1e9, "kernel": routes.get(route_plain)})
-        # W4A8 decode beside it: 4096 x 4096 weights, 8 INT8 activation vectors (gemv_blocked_kernel: exact DP4A block sums)
+        # W4A8 decode beside it: 4096 x 4096 weights, 8 INT8 activation vectors (gemv_q8_kernel: exact block sums)
         m8 = k8 = 4096
         w8 = [W.quantize_decode_factor(W.randn_bf16(m8, k8, 0.02, 330 + s + 1000 * rank, dev)) for s in range(16)]   # 151 MB > L2
         x8 = W.randn_bf16(8, k8, 1.0, 401 + rank, dev)
@@ -539,7 +539,7 @@ def run_ours(args, rank, world, local_rank):
         ms_g8, n3 = time_graph(gemv_int8, 48, 7, 8, dist, world)
         launches += n3
         b8 = m8 * k8 // 2 + m8 * k8 // 16
-        extra["gemv_8192_b1"]["w4a8_4096_b8"] = {"entry": "nvfp4a_gemm, INT8 activations, 8 vectors, 4096 x 4096", "kernel": "gemv_blocked_kernel (DP4A, exact block sums)",
+        extra["gemv_8192_b1"]["w4a8_4096_b8"] = {"entry": "nvfp4a_gemm, INT8 activations, 8 vectors, 4096 x 4096", "kernel": "gemv_q8_kernel (exact block sums)",
                                                  "us_per_call": ms_g8 * 1e3, "gbs": b8 / (ms_g8 * 1e-3) / 1e9, "frac": b8 / (ms_g8 * 1e-3) / 1e9 / peaks["hbm_gbs"]}
         del ws, tws, imgs, w8, t_w8
     # ---- quantization 8192^2 BF16 -> NVFP4, swizzled scales: 3 inputs = 403 MB > L2 ----

@@ -112,6 +112,12 @@ int nvfp4a_b200_last_parts(void);
  * mma.sync one.  A pinned value also lifts the size threshold below which the automatic choice prefers the mma.sync GEMV.  Tuning / test aid, no counterpart in the reference.  Returns 0, or -1 for another value. */
 int nvfp4a_b200_set_gemv_splits(int splits);
 
+/* nvfp4a_gemm (image != 0: nvfp4a_gemv_tc, A->data is the weight's image and lda is not looked at) on up to 8 dense activation vectors that the kernel itself makes
+ * INT8 with one FP32 scale per 16 values: the bytes of nvfp4a_quantize to INT8 followed by that call, in one launch and without buffers between the two (no counterpart
+ * in the reference).  More vectors, and what the INT8 GEMV does not take (nvfp4a_b200_set_route(1) among it): NVFP4A_NOT_SUPPORTED, and nothing is launched. */
+nvfp4a_status nvfp4a_b200_gemv_w4a8(int m, int n, int k, float alpha, const nvfp4a_tensor *A, int lda, int image, const nvfp4a_tensor *B, int ldb, float beta,
+                                    const nvfp4a_tensor *C, int ldc, const nvfp4a_tensor *D, int ldd, const nvfp4a_tensor *bias, cudaStream_t stream);
+
 /* All-gather of a tensor-parallel layer's output over peer memory (no counterpart in the reference, which is single-GPU).
  * buffers[p] / flags[p], p < world <= 8: the activation buffer [rows][row_pitch_bytes] and a flag array of 16 64-bit words
  * (zero before the first use) as mapped on this GPU for every rank of the node (peer mappings of symmetric allocations;

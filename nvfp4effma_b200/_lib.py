@@ -105,6 +105,7 @@ _PROTOS = {
     "nvfp4a_b200_set_scratch_alloc": (None, [_v, _v]),
     "nvfp4a_b200_get_scratch_alloc": (None, [C.POINTER(_v), C.POINTER(_v)]),
     "nvfp4a_b200_last_parts": (_i, []),
+    "nvfp4a_b200_gemv_w4a8": (_i, [_i, _i, _i, _f, _T, _i, _i, _T, _i, _f, _T, _i, _T, _i, _T, _s]),
 }
 EXPORTS = tuple(_PROTOS)
 

@@ -20,6 +20,7 @@ constexpr int kGemvMaxN = 8;
 
 static bool dense_t(const nvfp4a_tensor *t) { return t->dtype >= NVFP4A_BF16 && t->dtype <= NVFP4A_FP32; }
 static bool blocked_t(const nvfp4a_tensor *t) { return t->dtype == NVFP4A_NVFP4 || t->dtype == NVFP4A_INT8; }
+static bool blocked_dt(int t) { return t == NVFP4A_NVFP4 || t == NVFP4A_INT8; }
 static bool aligned(const void *p, unsigned a) { return ((uintptr_t)p & (a - 1)) == 0; }
 static bool dense_dt(nvfp4a_dtype t) { return t >= NVFP4A_BF16 && t <= NVFP4A_FP32; }
 
@@ -126,7 +127,7 @@ static nvfp4a_status dispatch(const char *fn, const GemmArgs &g, cudaStream_t st
   else if (gemv && g.k > 0 && forced_route() != 2 && gemv_fp4_n8_supports(g)) { g_last_route = 3; err = launch_gemv_fp4_n8(g, stream); }
   else if (gemv && gemv_stream_supports(g)) { g_last_route = 2; err = launch_gemv_stream(g, stream); }
   else if (gemv && gemv_supports(g)) { g_last_route = 2; err = launch_gemv(g, stream); }
-  else if (gemv && g.k > 0 && gemv_blocked_supports(g)) { g_last_route = 6; err = launch_gemv_blocked(g, stream); }
+  else if (gemv && g.k > 0 && blocked_dt(g.B.dtype) && gemv_q8_supports(g)) { g_last_route = 6; err = launch_gemv_q8(g, stream); }
   else if (!gemv && gemm_w4a4_supports(g)) { g_last_route = 4; err = launch_gemm_w4a4(g, stream); }
   else if ((!gemv || g.B.dtype == NVFP4A_FP16) && gemm_w4a16_supports(g)) { g_last_route = 5; err = launch_gemm_w4a16(g, stream); }
   else if (!gemv && forced_route() != 3 && gemm_w4a8_tc_supports(g)) {
@@ -385,6 +386,36 @@ extern "C" nvfp4a_status nvfp4a_gemm(int m, int n, int k, float alpha, const nvf
   EpilogueEx x;
   memset(&x, 0, sizeof x);
   return gemm_run("nvfp4a_gemm", m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, D, ldd, bias, x, stream);
+}
+
+// Up to 8 dense activation vectors made INT8 (one FP32 scale per 16 values) inside the GEMV: the bytes of nvfp4a_quantize to INT8 and nvfp4a_gemm (image: nvfp4a_gemv_tc).
+extern "C" nvfp4a_status nvfp4a_b200_gemv_w4a8(int m, int n, int k, float alpha, const nvfp4a_tensor *A, int lda, int image, const nvfp4a_tensor *B, int ldb, float beta,
+                                               const nvfp4a_tensor *C, int ldc, const nvfp4a_tensor *D, int ldd, const nvfp4a_tensor *bias, cudaStream_t stream) {
+  const char *fn = "nvfp4a_b200_gemv_w4a8";
+  clear_error();
+  if (!B || !dense_t(B)) return fail(NVFP4A_INVALID_VALUE, "%s: B must be BF16, FP16 or FP32", fn);
+  if (n > kGemvMaxN) return fail(NVFP4A_NOT_SUPPORTED, "%s: n = %d (at most %d)", fn, n, kGemvMaxN);
+  GemmArgs g;
+  memset(&g, 0, sizeof g);
+  const EpilogueEx none = {};
+  nvfp4a_tensor a;
+  if (image && A) {   // (an image has the scales inside; the checks of a plain operand are about memory that is not there)
+    if (!aligned(A->data, 16)) return fail(NVFP4A_INVALID_VALUE, "%s: the image must be 16-byte aligned", fn);
+    if (nvfp4a_status st = check_flags_only(fn, A)) return st;
+    a = *A;
+    a.block_scale = A->data; a.ld_scale = 0;
+    A = &a;
+    lda = k;
+  }
+  if (nvfp4a_status st = gemm_run(fn, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, D, ldd, bias, none, stream, false, 1, &g)) return st;
+  if (m <= 0 || n <= 0) return NVFP4A_OK;
+  if (image) {
+    g.A.image = 1; g.A.ktiles = (k + kImgK - 1) / kImgK; g.A.sc = nullptr;
+  }
+  // Every CTA quantizes all activations: up to 32768 values that takes 0.6 to 1.6 us (k = 4096, one to eight vectors) where a launch of its own takes 1.9; 8 x 8000 take 9.
+  if (forced_route() == 1 || (long long)n * k > 32768 || !gemv_q8_supports(g)) return fail(NVFP4A_NOT_SUPPORTED, "%s: quantize first (k = %d)", fn, k);
+  g_last_route = 6;
+  return cuda_fail(launch_gemv_q8(g, stream), fn);
 }
 
 extern "C" nvfp4a_status nvfp4a_gemm_ex(int m, int n, int k, float alpha, const nvfp4a_tensor *A, int lda, const nvfp4a_tensor *B, int ldb, float beta,

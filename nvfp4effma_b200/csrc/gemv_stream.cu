@@ -27,15 +27,13 @@
 // A long k (more than 128 KiB of FP16 activations): a cluster of 2, 4 or 8 CTAs takes a section of k each; the sections' sums go to the first CTA (DSMEM),
 // which adds them in order.
 #include <atomic>
-#include "operands.cuh"
-#include "sm100.cuh"
+#include "gemv_stream.cuh"
 
 namespace nvb {
 
 namespace {
 
 constexpr int kWarps = 16, kThreads = 32 * kWarps;
-constexpr int kUnitK = 128;                                       // a warp's unit: 16 rows x 128 values
 constexpr int kAhead = 2;                                         // units of a warp in flight
 constexpr int kSmemMax = 226 * 1024;
 constexpr int kXLimit = 128 * 1024;                                // activations of a CTA at most
@@ -54,53 +52,16 @@ struct StreamArgs {
   int round;                       // slices whose sums fit shared memory
 };
 
-__device__ __forceinline__ void prefetch_line(const void *p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
-
-// eight E2M1 nibbles -> four pairs of FP16 values, in the order of k
-__device__ __forceinline__ void e2m1_to_f16(uint32_t w, uint32_t (&o)[4]) {
-  asm("{\n\t.reg .b8 b0, b1, b2, b3;\n\tmov.b32 {b0, b1, b2, b3}, %4;\n\tcvt.rn.f16x2.e2m1x2 %0, b0;\n\tcvt.rn.f16x2.e2m1x2 %1, b1;\n\t"
-      "cvt.rn.f16x2.e2m1x2 %2, b2;\n\tcvt.rn.f16x2.e2m1x2 %3, b3;\n\t}"
-      : "=r"(o[0]), "=r"(o[1]), "=r"(o[2]), "=r"(o[3]) : "r"(w));
-}
 __device__ __forceinline__ uint32_t mul2(uint32_t a, uint32_t b) {
   uint32_t d;
   asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
   return d;
 }
-__device__ __forceinline__ void mma16(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-  asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
-      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-// the first of a chain: nothing to add to
-__device__ __forceinline__ void mma16_first(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-  asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%10, %10, %10, %10};"
-      : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.f));
-}
-// two E4M3 codes -> their values * 2^-8 as a pair of FP16 values (0x7F: 480 * 2^-8)
-__device__ __forceinline__ uint32_t scale_pair(uint32_t v) {
-  const uint32_t t = byte_perm(v, 0u, 0x1404u);
-  return ((t >> 1) & 0x3F803F80u) | (t & 0x80008000u);
-}
-__device__ __forceinline__ uint4 lds16(uint32_t a) {
-  uint4 v;
-  asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a));
-  return v;
-}
-__device__ __forceinline__ uint32_t ld2(const uint8_t *p) {
-  uint16_t v;
-  asm("ld.global.u16 %0, [%1];" : "=h"(v) : "l"(p));
-  return v;
-}
-__device__ __forceinline__ uint32_t word(const uint4 &v, int i) { return i == 0 ? v.x : i == 1 ? v.y : i == 2 ? v.z : v.w; }
 __device__ __forceinline__ float pow2i(int e) { return __int_as_float((e + 127) << 23); }   // -126 <= e <= 127
 // v * 2^e for any e that a vector's scale can be, by two exact factors
 __device__ __forceinline__ float scale2(float v, int e) {
   const int a = max(min(e, 100), -100);
   return __fmul_rn(__fmul_rn(v, pow2i(a)), pow2i(max(min(e - a, 127), -126)));
-}
-// slices of 16 rows in the order a matrix is dealt out: the four slices of a 128-row tile whose scale codes share 16-byte lines follow one another
-__device__ __forceinline__ int slice_row(int s, int m) {
-  return s < ((m >> 7) << 3) ? (s >> 3) * 128 + (s & 3) * 32 + ((s >> 2) & 1) * 16 : s * 16;
 }
 // eight BF16 values of plane p > 0 of a vector whose largest biased exponent is eb, as FP16 values scaled by 2^(141 - eb + 32 p); values of other planes are 0
 __device__ __forceinline__ uint4 plane_values(const uint4 &v, int eb, int p) {
@@ -136,7 +97,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemv_stream_kernel(const StreamAr
   const int S = g.sections, rank = S > 1 ? (int)sm100::cluster_ctarank() : 0, cluster = blockIdx.x / S;
   const int KG = g.kgroups, SG = kWarps / KG, kg = warp & (KG - 1), sg = warp / KG;
   const int sec = g.sec_chunks, c_first = rank * sec, kloc = max(min(gk - c_first * 256, sec * 256), 0);   // values of this CTA's range of k
-  const int nloc = (kloc + 255) >> 8, units = (kloc + kUnitK - 1) / kUnitK;
+  const int nloc = (kloc + 255) >> 8, units = (kloc + kStreamUnitK - 1) / kStreamUnitK;
   const int s_first = cluster * g.per, s_count = min(g.per, ((gm + 15) >> 4) - s_first);
   uint8_t *const xs = smem;                                                            // FP16 activations [chunk][8][n][4 lanes][8 values]
   const int chunk_x = 512 * n;
@@ -146,72 +107,16 @@ __global__ void __launch_bounds__(kThreads, 1) gemv_stream_kernel(const StreamAr
   float *const part = (float *)(more + sec);                                           // [slice of a round][KG warps][n][16 rows]
   float *const res = part + g.round * KG * n * 16;                                     // [section][slice of a round][n][16 rows] (first CTA of a cluster)
 
-  // ---- the warp's units: every KG-th of a slice, every SG-th slice ----
-  struct Unit { uint4 wa, wb; uint32_t ca, cb; };  // rows gq and gq + 8: 32 values of k and two scale codes each
-  const bool lin = !IMG && g.A.sld > 0;
-  int f_slice = sg, f_unit = kg;                   // the next unit to be requested
-  const uint8_t *f_w = g.A.data, *f_s = g.A.data;  // where it is for row gq
-  uint32_t f_w8 = 0, f_s8 = 0;                             // from there to row gq + 8
-  const uint32_t step_w = IMG ? (uint32_t)(KG >> 1) * kImgTileBytes : (uint32_t)KG * 64;      // (whole tiles, or a slice has one unit)
-  const uint32_t step_s = IMG ? (uint32_t)(KG >> 1) * kImgTileBytes : (uint32_t)KG * (lin ? 8 : 1024);
-  auto start_slice = [&]() {
-    const int row0 = slice_row(s_first + f_slice, gm);
-    if (IMG) {
-      const int rr = (row0 & 127) + gq;
-      const uint8_t *t = g.A.data + ((size_t)(row0 >> 7) * g.A.ktiles + c_first + (kg >> 1)) * kImgTileBytes;
-      f_w = t + rr * 128 + (kg & 1) * 64 + q * 16;
-      f_s = t + kImgDataBytes + (kg & 1) * 1024 + (q >> 1) * 512 + (rr & 31) * 16 + (rr >> 5) * 4 + (q & 1) * 2;
-      f_w8 = 1024; f_s8 = 128;
-    } else {
-      const int r0 = min(row0 + gq, gm - 1), r1 = min(row0 + gq + 8, gm - 1);
-      const ScalePos sp{g.A.sld};
-      f_w = g.A.data + (size_t)r0 * (g.A.ld >> 1) + (size_t)c_first * 128 + kg * 64 + q * 16;
-      f_w8 = (uint32_t)(r1 - r0) * (uint32_t)(g.A.ld >> 1);
-      f_s = g.A.sc + sp.row(r0) + (lin ? (size_t)c_first * 16 + kg * 8 + q * 2 : (size_t)c_first * 2048 + kg * 1024 + (q >> 1) * 512 + (q & 1) * 2);
-      f_s8 = (uint32_t)(sp.row(r1) - sp.row(r0));
-    }
-  };
-  auto in_k = [&]() { return IMG || f_unit * kUnitK + q * 32 < kloc; };   // (the last unit of a plain operand may be short)
-  auto advance = [&]() {
-    f_unit += KG; f_w += step_w; f_s += step_s;
-    if (f_unit >= units) {
-      f_unit = kg; f_slice += SG;
-      if (f_slice < s_count) start_slice();
-    }
-  };
-  auto fetch = [&]() {
-    Unit v;
-    v.wa = v.wb = make_uint4(0, 0, 0, 0);
-    v.ca = v.cb = 0;
-    if (f_slice < s_count) {
-      if (in_k()) {
-        v.wa = ld16((const uint4 *)f_w);
-        v.wb = ld16((const uint4 *)(f_w + f_w8));
-        v.ca = ld2(f_s);
-        v.cb = ld2(f_s + f_s8);
-      }
-      advance();
-    }
-    return v;
-  };
-  if (kg >= units) f_slice = s_count;              // (nothing for this warp)
-  if (f_slice < s_count) {                         // the first units' lines into L2 (a prefetch reads nothing: a predecessor may still be writing the weights)
-    start_slice();
-    for (int i = 0; i < kAhead && f_slice < s_count; ++i) {
-      if (in_k()) { prefetch_line(f_w); prefetch_line(f_w + f_w8); prefetch_line(f_s); }
-      advance();
-    }
-    f_slice = sg; f_unit = kg;
-    start_slice();
-  }
+  UnitStream<IMG> f(g.A, gm, s_first, s_count, c_first, kloc, KG, warp, kWarps, lane);
+  f.prefetch(kAhead);
   if (S > 1) sm100::cluster_arrive_release();
   sm100::pdl_wait();
   // tensor-parallel layers in the deferred form: the activations are complete once every peer has posted the previous gather
   if (g.tp.world > 1 && (g.tp.deferred & 1)) tp_wait_posts(g.tp.flags, g.tp.world, g.tp.rank, g.tp.status, g.tp.tag, g.tp.wait_cycles);
-  f_w = behind_wait(f_w); f_s = behind_wait(f_s);
-  Unit ahead[kAhead];
+  f.w = behind_wait(f.w); f.s = behind_wait(f.s);
+  WeightUnit ahead[kAhead];
 #pragma unroll
-  for (int i = 0; i < kAhead; ++i) ahead[i] = fetch();
+  for (int i = 0; i < kAhead; ++i) ahead[i] = f.fetch();
   if (tid == 0) any_more_s = 0;
   for (int i = tid; i < sec; i += kThreads) more[i] = 0;
   for (int i = tid; i < chunk_x / 16; i += kThreads) ((uint4 *)zeros)[i] = make_uint4(0, 0, 0, 0);
@@ -239,7 +144,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemv_stream_kernel(const StreamAr
       uint32_t a = __vmaxu2(__vmaxu2(w[0] & 0x7FFF7FFFu, w[1] & 0x7FFF7FFFu), __vmaxu2(w[2] & 0x7FFF7FFFu, w[3] & 0x7FFF7FFFu));
       a = __reduce_max_sync(0xFFFFFFFFu, max(a & 0xFFFFu, a >> 16));
       const int eb = (int)max(min(a >> 7, 254u), kMinExp);               // the biased exponent this chunk of the vector is scaled by
-      const float f = pow2i(141 - eb);
+      const float up = pow2i(141 - eb);
       const uint32_t least = eb <= 32 ? 1u : (uint32_t)(eb - 31) << 7;    // smallest magnitude of plane 0
       // (zeros count as the largest value here: 0 - 1 wraps)
       const uint32_t lo = __vminu2(__vminu2(__vsub2(w[0] & 0x7FFF7FFFu, 0x00010001u), __vsub2(w[1] & 0x7FFF7FFFu, 0x00010001u)),
@@ -265,7 +170,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemv_stream_kernel(const StreamAr
       uint32_t o[4];
 #pragma unroll
       for (int i = 0; i < 4; ++i)
-        asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(o[i]) : "f"(__fmul_rn(__uint_as_float(w[i] & 0xFFFF0000u), f)), "f"(__fmul_rn(__uint_as_float(w[i] << 16), f)));
+        asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(o[i]) : "f"(__fmul_rn(__uint_as_float(w[i] & 0xFFFF0000u), up)), "f"(__fmul_rn(__uint_as_float(w[i] << 16), up)));
       // value k = 128 h + 32 q + 8 i of a chunk: lane q's operand of the MMAs of word i, half h
       const int at = ((lane >> 4) * 4 + (lane & 3)) * n * 4 + j * 4 + ((lane >> 2) & 3);
       *(uint4 *)(xs + (size_t)c * chunk_x + at * 16) = make_uint4(o[0], o[1], o[2], o[3]);
@@ -286,7 +191,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemv_stream_kernel(const StreamAr
   float acc[4] = {0, 0, 0, 0};   // [2 row + vector] of the lane's blocks, true scale
   const bool diag = (gq >> 1) == q && (gq & 1) < N;
   const uint32_t xa0 = diag ? sm100::smem_u32(xs) + ((gq & 1) * 4 + q) * 16 : sm100::smem_u32(zeros), xa_step = diag ? 256 * N : 0;   // per 128 values of k
-  auto compute = [&](const Unit &w) {
+  auto compute = [&](const WeightUnit &w) {
     float sum[4] = {0, 0, 0, 0};   // of this unit
     const uint32_t xa = xa0 + u * xa_step;
     const uint32_t sa = scale_pair(w.ca), sb = scale_pair(w.cb);
@@ -312,14 +217,14 @@ __global__ void __launch_bounds__(kThreads, 1) gemv_stream_kernel(const StreamAr
       }
     }
     const int c = u >> 1;
-    const float *const f = factor + c * N;
+    const float *const fc = factor + c * N;
 #pragma unroll
     for (int j = 0; j < N; ++j) {
-      acc[j] = __fmaf_rn(sum[j], f[j], acc[j]);
-      acc[2 + j] = __fmaf_rn(sum[2 + j], f[j], acc[2 + j]);
+      acc[j] = __fmaf_rn(sum[j], fc[j], acc[j]);
+      acc[2 + j] = __fmaf_rn(sum[2 + j], fc[j], acc[2 + j]);
     }
     if (any_more && more[c]) {   // (the same for every lane) values that plane 0 could not hold
-      const int planes = more[c], col = gq < N ? gq : 0, eb = (__float_as_int(f[col]) >> 23) + 6;   // (the exponent of 2^(eb - 133), biased, is eb - 6)
+      const int planes = more[c], col = gq < N ? gq : 0, eb = (__float_as_int(fc[col]) >> 23) + 6;   // (the exponent of 2^(eb - 133), biased, is eb - 6)
       const uint4 *row = (const uint4 *)(x + (size_t)col * g.ldx) + (size_t)(c_first + c) * 32;
       const int vec_left = kvec - c * 32;
 #pragma unroll 1
@@ -339,7 +244,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemv_stream_kernel(const StreamAr
         if (q == 0)       // columns 0 and 1 are the vectors here; lane 0 of a quad has them, and its sums join the others'
 #pragma unroll
           for (int j = 0; j < N; ++j) {
-            const int ex = (__float_as_int(f[j]) >> 23) - 127 - 32 * p;
+            const int ex = (__float_as_int(fc[j]) >> 23) - 127 - 32 * p;
             acc[j] = __fadd_rn(acc[j], scale2(d[j], ex));
             acc[2 + j] = __fadd_rn(acc[2 + j], scale2(d[2 + j], ex));
           }
@@ -380,18 +285,17 @@ __global__ void __launch_bounds__(kThreads, 1) gemv_stream_kernel(const StreamAr
     const int end = min(base + g.round, s_count);
     if (kg < units) {
       if (base > 0 && slice < s_count) {
-        f_slice = slice; f_unit = kg;
-        start_slice();
+        f.restart(slice);
 #pragma unroll
-        for (int i = 0; i < kAhead; ++i) ahead[i] = fetch();
+        for (int i = 0; i < kAhead; ++i) ahead[i] = f.fetch();
       }
 #pragma unroll 1
       while (slice < end) {
 #pragma unroll
         for (int i = 0; i < kAhead; ++i) {
           if (slice >= end) break;
-          const Unit w = ahead[i];
-          ahead[i] = fetch();
+          const WeightUnit w = ahead[i];
+          ahead[i] = f.fetch();
           compute(w);
           u += KG;
           if (u >= units) { put(slice - base); u = kg; slice += SG; }
@@ -402,43 +306,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemv_stream_kernel(const StreamAr
     }
     __syncthreads();
     const int outs = (end - base) * n * 16;
-    auto epilogue = [&](auto sum_of) {
-      for (int o0 = 0; o0 < outs; o0 += kThreads) {
-        const int o = o0 + tid;
-        if ((o & ~31) >= outs) break;                       // (whole warps)
-        const int ri = o & 15, cj = (o >> 4) % n, s = base + (o >> 4) / n;
-        const int row0 = slice_row(s_first + s, gm), i = row0 + ri;
-        const bool live = o < outs && i < gm;
-        float v = 0.f;
-        if (live) {
-          float colp = epi_col_part(e, cj);
-          if (g.ex.mask & kExNorm) colp = __fmul_rn(colp, colscale[cj]);
-          v = epi_value(e, i, cj, sum_of(o), epi_scale(e, __fmul_rn(e.alpha, e.ga_stride ? e.ga[i] : ga0), colp));
-        }
-        if (g.ex.mask & kExSwiglu) {
-          const float up = __shfl_down_sync(0xFFFFFFFFu, v, 8);
-          if (live && ri < 8) {
-            const float h = silu_mul(v, up);
-            store_dense(e.d_dtype, e.d, (size_t)cj * e.ldd + (row0 >> 1) + ri, h);
-            amax = fmaxf(amax, fabsf(h));
-          }
-        } else if (live) {
-          store_dense(e.d_dtype, e.d, (size_t)cj * e.ldd + i, v);
-          amax = fmaxf(amax, fabsf(v));
-        }
-        if (g.ex.mask & kExOut2) {
-          float sq = 0.f;
-#pragma unroll
-          for (int r = 0; r < 16; ++r) {
-            const float w = __shfl_sync(0xFFFFFFFFu, v, (lane & 16) + r);
-            sq = __fadd_rn(sq, __fmul_rn(w, w));
-          }
-          if (live) store_dense(g.ex.d2_dtype, g.ex.d2, (size_t)cj * g.ex.ldd2 + i, __fmul_rn(v, load_dense(g.ex.w2_dtype, g.ex.w2, i)));
-          if (live && ri == 0) g.ex.sq[(size_t)cj * g.ex.ld_sq + (i >> 4)] = sq;
-        }
-      }
-      __syncwarp();
-    };
+    auto epilogue = [&](auto sum_of) { slices_epilogue(e, g.ex, n, s_first + base, outs, gm, ga0, colscale, amax, sum_of); };
     if (S == 1) {
       epilogue(own_sum);
       if (end < s_count) __syncthreads();
@@ -549,7 +417,7 @@ cudaError_t launch_gemv_stream(const GemmArgs &g, cudaStream_t s) {
   const int chunks = (g.k + 255) >> 8;
   a.sections = sections_for(g.k, g.n);
   a.sec_chunks = (chunks + a.sections - 1) / a.sections;
-  const int units = min(2 * a.sec_chunks, (g.k + kUnitK - 1) / kUnitK);
+  const int units = min(2 * a.sec_chunks, (g.k + kStreamUnitK - 1) / kStreamUnitK);
   a.kgroups = 1;
   while (a.kgroups < kWarps && a.kgroups * 2 <= units) a.kgroups *= 2;
   // (half as many where more than an eighth of the turns would be idle; an even number, so that a warp stays in the same half of an image's tiles)

@@ -75,8 +75,8 @@ bool gemv_fp4_supports(const GemmArgs &g);
 cudaError_t launch_gemv_fp4_n8(const GemmArgs &g, cudaStream_t s);   // the same for 3 <= n <= 8
 bool gemv_fp4_n8_supports(const GemmArgs &g);
 void set_gemv_fp4_splits(int s);
-cudaError_t launch_gemv_blocked(const GemmArgs &g, cudaStream_t s);  // n <= 8, INT8 or NVFP4 activations: exact integer block sums (mma.sync s8)
-bool gemv_blocked_supports(const GemmArgs &g);
+cudaError_t launch_gemv_q8(const GemmArgs &g, cudaStream_t s);       // n <= 8, INT8 / NVFP4 activations, or dense ones that it makes INT8: exact block sums (mma.sync on FP16)
+bool gemv_q8_supports(const GemmArgs &g);
 cudaError_t launch_gemm_w4a4(const GemmArgs &g, cudaStream_t s);     // tcgen05 kind::mxf4nvf4 (E4M3 scales)
 bool gemm_w4a4_supports(const GemmArgs &g);
 cudaError_t launch_gemm_dp4a(const GemmArgs &g, cudaStream_t s);     // W4A8, n > 8: DP4A block sums in the reference's tiled order
