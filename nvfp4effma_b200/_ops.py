@@ -1,5 +1,5 @@
 """The torch operator layer: ``torch.ops.nvfp4effma.*`` with the schemas of the reference's extension
-(binds/python/csrc/nvfp4effma_torch.cpp:721-743 there), a CUDA implementation that calls the C ABI of
+(binds/python/csrc/nvfp4effma_torch.cpp:721-743 there; ``linear_w4a8``, ``quantize_int8`` and ``linear`` in one, is this library's own), a CUDA implementation that calls the C ABI of
 ``libnvfp4effma.so`` and a Meta implementation (shapes and dtypes only), so that code written against the reference's
 operators -- or traced through them by ``torch.compile`` / ``torch.library.opcheck`` -- runs unchanged.  The CUDA
 implementations are in csrc/torch_ops.cpp (``transpose`` and ``swizzle_scales``, which no hot path calls, here through ctypes).
@@ -31,6 +31,7 @@ SCHEMAS = {
     "swizzle_scales": "(Tensor scales, int rows, int cols, bool to_swizzled) -> Tensor",
     "linear": f"({_X}, {_W}, int k, Tensor? bias, ScalarType? out_dtype, float alpha, bool want_amax, Tensor? w_img) -> (Tensor, Tensor?)",
     "linear_out": f"({_X}, {_W}, int k, Tensor? bias, Tensor(a!) out, float alpha, float beta, bool want_amax, Tensor? w_img) -> Tensor?",
+    "linear_w4a8": f"(Tensor x, {_W}, int k, Tensor? bias, ScalarType? out_dtype, float alpha, bool want_amax, Tensor? w_img) -> (Tensor, Tensor?)",
     "grouped_linear": f"({_X}, Tensor seg, {_W}, int k, int groups, Tensor? bias, ScalarType? out_dtype, float alpha, bool want_amax) -> (Tensor, Tensor?)",
     "grouped_linear_out": f"({_X}, Tensor seg, {_W}, int k, int groups, Tensor? bias, Tensor(a!) out, float alpha, float beta, bool want_amax) -> Tensor?",
     "tc_image": "(int operand, Tensor x, Tensor? scales, int flags, int k) -> Tensor",
@@ -170,6 +171,13 @@ def _check_out(out, T, N):
 
 @_op("linear").meta
 def _linear_meta(x, x_scales, x_global, x_flags, x_smax, w, w_scales, w_global, w_flags, w_smax, k, bias, out_dtype, alpha, want_amax, w_img):
+    out = torch.empty((x.shape[0], w.shape[0]), dtype=_result_dtype(x, out_dtype), device=w.device)
+    return out, (_one_float(out) if want_amax else None)
+
+
+@_op("linear_w4a8").meta
+def _linear_w4a8_meta(x, w, w_scales, w_global, w_flags, w_smax, k, bias, out_dtype, alpha, want_amax, w_img):
+    _quantize_int8_meta(x)
     out = torch.empty((x.shape[0], w.shape[0]), dtype=_result_dtype(x, out_dtype), device=w.device)
     return out, (_one_float(out) if want_amax else None)
 

@@ -230,6 +230,15 @@ def _run(a: _Activations, w: Fp4Operand, image, N, K, bias, out_dtype, out, alph
     return out if out is not None else y if len(a.lead) == 1 else y.reshape(*a.lead, N)
 
 
+def _run_w4a8(x, w: Fp4Operand, image, N, K, bias, out_dtype, alpha, amax_out):
+    """Dense activations, INT8 on the way into the product, a result of its own: one operator."""
+    matrix = _as_matrix(x)
+    _dense_input(matrix)
+    y, seen = ops.linear_w4a8(matrix, w.data, w.scales, w.glob, w.flags, w.scale_max, K, bias, out_dtype, alpha, amax_out is not None, image)
+    _raise_amax(amax_out, seen)
+    return y if x.dim() == 2 else y.reshape(*x.shape[:-1], N)
+
+
 def linear(x: Union[torch.Tensor, NVFP4Tensor, Int8Tensor], weight, bias: Optional[torch.Tensor] = None, *, act: str = "auto",
            out_dtype: Optional[torch.dtype] = None, out: Optional[torch.Tensor] = None, alpha: float = 1.0, beta: float = 0.0,
            amax_out: Optional[torch.Tensor] = None) -> torch.Tensor:
@@ -252,6 +261,8 @@ def linear(x: Union[torch.Tensor, NVFP4Tensor, Int8Tensor], weight, bias: Option
         _check_mode(act, ("auto",) + _ACT_MODES)
         if mode == "auto":
             mode = "exact" if math.prod(x.shape[:-1]) <= AUTO_EXACT_MAX_ROWS else "int8"
+        if mode == "int8" and out is None and beta == 0.0:
+            return _run_w4a8(x, weight._operand(), None, N, K, bias, out_dtype, alpha, amax_out)
     return _run(_activations(x, K, mode), weight._operand(), None, N, K, bias, out_dtype, out, alpha, beta, amax_out)
 
 
@@ -268,6 +279,8 @@ def _linear_on_image(x, weight: TCWeight, bias, act, out_dtype, out, alpha, beta
             raise ValueError(f"act = {mode!r} cannot use an image built for act = {weight.act!r}")
         if mode == "exact" and x.dtype != torch.bfloat16:
             raise TypeError(f"the W4A16 image path multiplies bfloat16 activations; x is {x.dtype}")
+        if mode == "int8" and out is None and beta == 0.0 and math.prod(x.shape[:-1]) <= 8:
+            return _run_w4a8(x, weight.weight._operand(), weight.image, N, K, bias, out_dtype, alpha, amax_out)
     return _run(_activations(x, K, mode), weight.weight._operand(), weight.image, N, K, bias, out_dtype, out, alpha, beta, amax_out)
 
 

@@ -403,6 +403,45 @@ std::tuple<Tensor, Tensor> quantize_int8(const Tensor &x0) {
   return {q, s};
 }
 
+// quantize_int8 and linear in one call: up to 8 tokens in one kernel too, which makes the activations INT8 itself (the same bytes)
+std::tuple<Tensor, OptTensor> linear_w4a8(const Tensor &x0, const Tensor &w, const Tensor &ws, const OptTensor &wg, int64_t wf, int64_t wm, int64_t k,
+                                          const OptTensor &bias, std::optional<ScalarType> out_dtype, double alpha, bool want_amax, const OptTensor &w_img) {
+  check_matrix16(x0, "linear_w4a8");
+  check_k(k);
+  const int64_t T = x0.size(0), N = w.size(0);
+  if (T >= 1 && T <= 8 && x0.size(1) == k && x0.device() == w.device()) {
+    const c10::cuda::CUDAGuard guard(w.device());
+    const Tensor x = matrix(x0, 16, "x");
+    if (x.stride(0) % 64 == 0) {
+      const nvfp4a_tensor b = dense_tensor(x, "x");
+      const Tensor out = empty({T, N}, result_dtype(x0, out_dtype), w);
+      const OptTensor amax = amax_buffer(want_amax, out);
+      const nvfp4a_tensor d = dense_tensor(out, "out", amax);
+      const Bias bi(bias, N);
+      Operand a;
+      if (w_img) {
+        a.t.data = device_ptr(*w_img, "the weight's image");
+        a.t.dtype = NVFP4A_NVFP4;
+        a.t.global_scale = (const float *)addr(wg, "global");
+        a.t.flags = (unsigned)wf;
+        a.t.scale_max = (int)wm;
+      } else {
+        a = fp4_operand(w, ws, wg, wf, wm);
+      }
+      const nvfp4a_status st = nvfp4a_b200_gemv_w4a8((int)N, (int)T, (int)k, (float)alpha, &a.t, (int)a.ld, w_img ? 1 : 0, &b, (int)x.stride(0), 0.f, nullptr, 0, &d,
+                                                     (int)out.stride(0), bi.p, stream());
+      if (st != NVFP4A_NOT_SUPPORTED) {
+        check(st);
+        return {out, amax};
+      }
+    }
+  }
+  const auto [q, s] = quantize_int8(x0);
+  const c10::cuda::CUDAGuard guard(w.device());
+  const Tensor out = empty({T, N}, result_dtype(x0, out_dtype), w);
+  return {out, gemm_into(out, q, s, std::nullopt, 0, 0, w, ws, wg, wf, wm, k, bias, alpha, 0.0, want_amax, w_img)};
+}
+
 Tensor dequantize(const Tensor &data, const Tensor &scales, const OptTensor &glob, int64_t flags, int64_t smax, int64_t cols, ScalarType dtype) {
   dense_code(dtype);
   const c10::cuda::CUDAGuard guard(data.device());
@@ -421,6 +460,7 @@ TORCH_LIBRARY_IMPL(nvfp4effma, CUDA, m) {
   m.impl("dequantize", &dequantize);
   m.impl("linear", &linear);
   m.impl("linear_out", &linear_out);
+  m.impl("linear_w4a8", &linear_w4a8);
   m.impl("grouped_linear", &grouped_linear);
   m.impl("grouped_linear_out", &grouped_linear_out);
   m.impl("tc_image", &tc_image);

@@ -517,3 +517,24 @@ def test_linear_into_pinned_host_memory(act, dtype, tokens):
     torch.cuda.synchronize()
     assert torch.equal(out, want.cpu()) and not asked
     assert fn.value == ctypes.cast(own, ctypes.c_void_p).value and ctx.value == 77
+
+
+@pytest.mark.parametrize("tokens,k", [(1, 128), (5, 320), (8, 8192), (20, 256)])
+def test_w4a8_in_one_operator_gives_the_bytes_of_two(tokens, k):
+    """linear on dense activations with act="int8" is one operator; views and other dtypes, the amax, leading dimensions, image weights; traced like the others."""
+    w = nf.quantize(normal((96, k), torch.bfloat16, seed=61))
+    wo = w._operand()
+    for dtype in (torch.bfloat16, torch.float16, torch.float32):
+        wide = normal((tokens, k + 64), dtype, seed=62)
+        for x in (wide[:, :k].contiguous(), wide[:, :k], wide[:, 16:k + 16]):
+            bias = normal((96,), dtype, seed=63)
+            a, b = torch.zeros(1, device=GPU), torch.zeros(1, device=GPU)
+            y = nf.linear(x, w, bias, act="int8", amax_out=a)
+            q = nf.quantize_int8(x)
+            assert torch.equal(y, nf.linear(q, w, bias, amax_out=b)) and y.dtype == dtype and torch.equal(a, b)
+    x = normal((tokens, k), torch.bfloat16, seed=64)
+    image = nf.TCWeight(w, "int8")
+    assert torch.equal(nf.linear(x, image, out_dtype=torch.float32), nf.linear(nf.quantize_int8(x), image, out_dtype=torch.float32))
+    assert nf.linear(x.view(1, tokens, k), w, act="int8").shape == (1, tokens, 96)
+    head = (x, wo.data, wo.scales, wo.glob, wo.flags, wo.scale_max, k, None, None, 1.0, True, None)
+    torch.library.opcheck(torch.ops.nvfp4effma.linear_w4a8, head, test_utils=("test_schema", "test_faketensor"))
