@@ -140,6 +140,8 @@ __device__ __forceinline__ uint32_t mbar_addr_rank(uint64_t *own_bar, uint32_t r
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(addr) : "r"(smem_u32(own_bar)), "r"(rank));
   return addr;
 }
+// contiguous memory into L2: address 16-byte aligned, bytes a multiple of 16
+__device__ __forceinline__ void prefetch_l2(const void *p, uint32_t bytes) { asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes)); }
 // contiguous copy: both addresses 16-byte aligned, bytes a multiple of 16
 __device__ __forceinline__ void bulk_load(void *dst, const void *src, uint32_t bytes, uint64_t *bar) {
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
