@@ -89,6 +89,13 @@ def test_quantize_ex_recipes(spec, dtype):
     run_quant(dtype, 256, 320, spec, 12)
 
 
+@pytest.mark.parametrize("spec", [SPECS[1], SPECS[11]], ids=["e4m3", "ue5m3"])
+@pytest.mark.parametrize("dtype,rows,cols", [(L.BF16, 2064, 2128), (L.FP32, 2064, 2128), (L.FP32, 2177, 2112), (L.FP32, 17, 18944)])
+def test_both_halves_of_many_tiles(spec, dtype, rows, cols):
+    """The sizes from which a CTA takes a tall tile of rows (128 of FP32, 256 of 16-bit values): a last tile of a few rows, of part of a block, and nothing else."""
+    run_quant(dtype, rows, cols, spec, 17)
+
+
 def test_quantize_ex_small_and_fp16():
     run_quant(L.FP16, 40, 48, SPECS[8], 13)
     for dtype in (L.BF16, L.FP16, L.FP32):
