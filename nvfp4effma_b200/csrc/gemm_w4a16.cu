@@ -28,7 +28,7 @@
 //               logical operations -- 2 instructions per value where shifts, masks, the multiply and reordering took 3.
 // Instruction issue, not the tensor pipe, bounded the former kernel (a thread-per-row expansion through shared memory with a proxy
 // fence per stage: 1240 cycles per stage of 512 cycles of MMAs, 41 % of the tensor pipe).
-// The last round of tiles over the SM pairs is cut along the tokens when it would leave pairs idle, and a tile at the end of the
+// The last round of tiles over the SM pairs is cut along the tokens, or into parts of k (see choose_tail), when it would leave pairs idle, and a tile at the end of the
 // tokens is only as wide (in steps of 64) as the tokens left.
 // Every wait is bounded; a wait that gives up raises the CTA's abort flag and the kernel status word.
 //
@@ -86,7 +86,8 @@ struct W4A16Args {
   int seg_stages;   // F16, GROUPED: stages per segment of k
   int unit;         // stages per unit: 1 or 2 (see the MMA issuer)
   const int *seg; int groups;   // GROUPED: m is the rows of ONE group's weight, n the bound on seg[groups]
-  int parts, part_stages; float *partial;   // kEpiPart: k in `parts` runs of part_stages stages, each one's sums in partial [part][n][m]
+  // kEpiPart, kEpiTail: the tiles from nfull on take k in `parts` runs of part_stages stages, each one's sums in partial [tile - nfull][part][width tokens][256 rows]
+  int parts, part_stages; float *partial;
   const float *tscale;          // PLANES = 2: what each token's sums are multiplied by; word n: 0 all tokens are two FP16 planes, 1 some, 2 none; behind it
                                 // a byte per token, non-zero for three BF16 planes
 };
@@ -178,18 +179,19 @@ __device__ __forceinline__ void mma12_f16_commit_pair_elect(uint32_t d0, uint32_
 
 // A tile of the schedule: 128-row tiles 2 * tm and 2 * tm + 1 (one per CTA of the pair) against the tokens [j0, j0 + width), of which
 // those below jend exist (width: a multiple of 64; 0: nothing to do).  Grouped: ro = the group's first row in the stacked weights.
-struct Tile { int tm, j0, jend, width, ro; };
+// A part of k: the stages [k0, k0 + nk), `unit` its place in the partial sums; -1: a whole tile.
+struct Tile { int tm, j0, jend, width, ro, unit, k0, nk; };
 constexpr int kMaxGroups = 256;
 
 // EPI: what the epilogue is compiled for.  0: everything; 1: a 16-bit D, alpha, globals and bias; 2: the same and SwiGLU.  The whole of it is 150 KiB of code in
 // which a plain call's instructions lie far apart: fetching them made a chunk of 32 columns take 5000 cycles, in which the tensor cores wait for the
 // accumulator or, at the end, the caller for the result.  28672 x 4096 with SwiGLU on 2048 tokens: 412 -> 344 us; FP16 4096 x 4096 on 333
 // tokens 37.5 -> 35.2; 5504 x 3584 with SwiGLU on 121 tokens 32.1 -> 27.0.
-// 3: no epilogue, the sums of a part of k as they are (see w4a16_join_kernel).
+// 3: no epilogue, the sums of a part of k as they are (see w4a16_join_kernel); 8: as 1 for whole tiles, as 3 for the parts of the last ones.
 // 4 .. 7: a 16-bit D, at run time an amax, and one of: RMSNorm scale and SwiGLU (28672 x 4096 on 2048 tokens 400 -> 330 us, INT8 activations 679 -> 628); second
 // output and sums of squares (4096 x 14336 214 -> 186); RMSNorm scale (6144 x 4096 103 -> 82; 4096 x 4096 on 100 tokens 30.3 -> 25.3); beta * C (131
 // -> 126, 32.9 -> 30.5: its two-byte loads of C remain).
-enum { kEpiAny = 0, kEpiPlain = 1, kEpiSwiglu = 2, kEpiPart = 3, kEpiNormGlu = 4, kEpiOut2 = 5, kEpiNorm = 6, kEpiAdd = 7 };
+enum { kEpiAny = 0, kEpiPlain = 1, kEpiSwiglu = 2, kEpiPart = 3, kEpiNormGlu = 4, kEpiOut2 = 5, kEpiNorm = 6, kEpiAdd = 7, kEpiTail = 8 };
 template <int PLANES, bool F16, bool GROUPED, int EPI>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_b, const __grid_constant__ CUtensorMap tmap_d,
@@ -217,12 +219,10 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
   const int nA = 1 << lgA, nB = 1 << lgB, subA = kA >> lgA;
   constexpr int kSub = PLANES == 3 ? C::kBBytes / 2 : C::kBBytes;   // bytes of a stage of one plane (three planes: tiles of at most 128 tokens)
   const int slot_bytes = (kB * C::kBBytes) >> lgB;
-  constexpr bool PART = EPI == kEpiPart;
-  constexpr bool AMAX = EPI == kEpiAny || EPI >= kEpiNormGlu, ADD = EPI == kEpiAny || EPI == kEpiAdd;
+  constexpr bool PART = EPI == kEpiPart, TAIL = EPI == kEpiTail, CUT_K = PART || TAIL;
+  constexpr bool AMAX = EPI == kEpiAny || (EPI >= kEpiNormGlu && !TAIL), ADD = EPI == kEpiAny || EPI == kEpiAdd;
   const int tile_first = blockIdx.x >> 1, tile_step = gridDim.x >> 1;
-  // (parts of k: a pair has one part of one tile, the stages [k0, k0 + nk))
-  const int parts = PART ? g.parts : 1, k0 = PART ? tile_first % parts * g.part_stages : 0;
-  const int tiles_m = (gm + 255) / 256, nk = PART ? min(g.part_stages, gk / 64 - k0) : gk / 64, nslots = (nk + 3) / 4;   // 256-row tiles
+  const int tiles_m = (gm + 255) / 256, nk_all = gk / 64, nslots_all = (nk_all + 3) / 4;   // 256-row tiles
   const bool ue = g.A.ue != 0;
   unsigned *const status_word = g.status;
 
@@ -312,13 +312,17 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
       int q = 0, hi = g.groups;   // the last q with gcum[q] <= tt (the group holding token tile tt has gcum[q + 1] > tt)
       while (hi - q > 1) { const int mid = (q + hi) >> 1; if (gcum[mid] <= tt) q = mid; else hi = mid; }
       const int j0 = gseg[q] + (tt - gcum[q]) * W, left = gseg[q + 1] - j0;
-      return Tile{t % tiles_m, j0, gseg[q + 1], left < W ? (left + 63) & ~63 : W, q * gm};
+      return Tile{t % tiles_m, j0, gseg[q + 1], left < W ? (left + 63) & ~63 : W, q * gm, -1, 0, nk_all};
     }
-    if (PART) t /= parts;
-    int w = W, part = 0;
-    if (t >= nfull) { w = W / cut; part = (t - nfull) % cut; t = nfull + (t - nfull) / cut; }
+    int w = W, part = 0, u = -1, k0 = 0, nk = nk_all;
+    if (CUT_K && t >= nfull) {
+      u = t - nfull;
+      k0 = u % g.parts * g.part_stages;
+      nk = min(g.part_stages, nk_all - k0);
+      t = nfull + u / g.parts;
+    } else if (!TAIL && t >= nfull) { w = W / cut; part = (t - nfull) % cut; t = nfull + (t - nfull) / cut; }
     const int j0 = t / tiles_m * W + part * w, left = gn - j0;
-    return Tile{t % tiles_m, j0, gn, left <= 0 ? 0 : left < w ? (left + 63) & ~63 : w, 0};
+    return Tile{t % tiles_m, j0, gn, left <= 0 ? 0 : left < w ? (left + 63) & ~63 : w, 0, u, k0, nk};
   };
   // accumulators: two of 128 columns while tiles are that narrow, else one of 256
   const int nacc = W > 128 ? 1 : 2;
@@ -333,7 +337,7 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
     for (int t = tile_first; t < ntiles; t += tile_step) {
       const Tile p = tile_of(t);
       if (p.width == 0) continue;
-      const int row0 = p.j0 + rank * (p.width >> 1), kinds = kinds_of(p);
+      const int row0 = p.j0 + rank * (p.width >> 1), kinds = kinds_of(p), nk = CUT_K ? p.nk : nk_all, k0 = CUT_K ? p.k0 : 0;
 #pragma unroll 1
       for (int kind = 0; kind < kKinds; ++kind) {
       if (kKinds == 2 && !(kinds >> kind & 1)) continue;
@@ -365,7 +369,7 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
       for (int t = tile_first; t < ntiles; t += tile_step) {
         const Tile p = tile_of(t);
         if (p.width == 0) continue;
-        const int kinds = kinds_of(p);
+        const int kinds = kinds_of(p), nk = CUT_K ? p.nk : nk_all;
         for (int ks0 = 0; ks0 < nk; ks0 += SEG ? seg_stages : nk, ++acc_i) {
           const int acc = nacc == 2 ? acc_i & 1 : 0, ks1 = SEG ? min(ks0 + seg_stages, nk) : nk;
           const uint32_t acc_par = (nacc == 2 ? acc_i >> 1 : acc_i) & 1;
@@ -421,7 +425,7 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
     for (int t = tile_first; t < ntiles; t += tile_step) {
       const Tile p = tile_of(t);
       if (p.width == 0) continue;
-      const int row_tile = 2 * p.tm + rank;
+      const int row_tile = 2 * p.tm + rank, k0 = CUT_K ? p.k0 : 0, nslots = CUT_K ? (p.nk + 3) / 4 : nslots_all;
       for (int pass = kKinds == 2 ? __popc(kinds_of(p)) : 1; pass > 0; --pass) {
 #pragma unroll 1
       for (int sl = 0; sl < nslots; ++sl, ++it) {
@@ -443,7 +447,7 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
     // (rarely used parameters are read from the constant bank where they are needed: the registers belong to the accumulator block)
     const float gb0 = !PART && g.e.gb ? *g.e.gb : 1.f;   // B's global: dense B has none, INT8 B one for the tensor (a multiply by 1 is exact)
     uint8_t *const dptr = (uint8_t *)g.e.d;
-    const int d_dtype = g.e.d_dtype, mask = EPI == kEpiSwiglu ? kExSwiglu : EPI == kEpiNormGlu ? kExNorm | kExSwiglu : EPI == kEpiOut2 ? kExOut2 : EPI == kEpiNorm ? kExNorm : SEG || EPI == kEpiPlain || EPI == kEpiAdd || PART ? 0 : g.x.mask;   // (segments: a 16-bit D and the plain epilogue)
+    const int d_dtype = g.e.d_dtype, mask = EPI == kEpiSwiglu ? kExSwiglu : EPI == kEpiNormGlu ? kExNorm | kExSwiglu : EPI == kEpiOut2 ? kExOut2 : EPI == kEpiNorm ? kExNorm : SEG || EPI == kEpiPlain || EPI == kEpiAdd || PART || TAIL ? 0 : g.x.mask;   // (segments: a 16-bit D and the plain epilogue)
     const bool d_tma = g.d_tma;
     // The accumulator is read as MMA fragments (16 lanes x 8 columns per register quad): a thread holds rows rb + 16 hh + 8 u (hh, u in
     // {0, 1}) of columns 8 gq + cp + e (e in {0, 1}) of a chunk of 32, register 16 hh + 4 gq + 2 u + e.  Gate and up rows of SwiGLU (8
@@ -465,7 +469,7 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
     for (int t = tile_first; t < ntiles; t += tile_step) {
       const Tile p = tile_of(t);
       if (p.width == 0) continue;
-      const int tm = 2 * p.tm + rank, jt = p.j0, jend = min(p.j0 + p.width, p.jend);
+      const int tm = 2 * p.tm + rank, jt = p.j0, jend = min(p.j0 + p.width, p.jend), nk = CUT_K ? p.nk : nk_all;
       // this warp's block: width / 2 columns, one to four chunks of 32
       const int hw = p.width >> 1, nchunks = min(hw, jend - jt - half * hw + 31) >> 5;   // (chunks past the last token are left alone)
       uint32_t r[32], rn[32];
@@ -590,8 +594,8 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
         const int cc = half * hw + c * 32;   // first column of the chunk in the tile
         const int j0 = jt + cc;
         const int nvalid = min(32, jend - j0);
-        if constexpr (PART) {   // eight lanes write 32 contiguous bytes of a token's sums
-          float *const p32 = g.partial + ((size_t)(tile_first % parts) * gn + j0) * gm + rb;
+        if (PART || (TAIL && p.unit >= 0)) {   // eight lanes write 32 contiguous bytes of a token's sums
+          float *const p32 = g.partial + ((size_t)p.unit * W + cc) * 256 + rank * 128 + quad * 32 + (lane >> 2);
 #pragma unroll
           for (int ce = 0; ce < 8; ++ce) {
             const int jj = 8 * (ce >> 1) + cp + (ce & 1);
@@ -600,7 +604,7 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
               const float v = __uint_as_float(r[16 * (q >> 1) + 4 * (ce >> 1) + 2 * (q & 1) + (ce & 1)]);
-              if (rb + 8 * q < gm) p32[(size_t)jj * gm + 8 * q] = PLANES == 2 ? __fmul_rn(v, ts) : v;
+              if (rb + 8 * q < gm) p32[jj * 256 + 8 * q] = PLANES == 2 ? __fmul_rn(v, ts) : v;
             }
           }
           continue;
@@ -763,7 +767,7 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
     const ScalePos sp{A.sld};
     const bool img = A.image, swz = A.sld < 0;
     // scale words of this group's two stages of slot sl (stages past the end of k: zeros)
-    auto fetch_scales = [&](const uint8_t *scp, int sl, uint32_t (&v)[2]) {
+    auto fetch_scales = [&](const uint8_t *scp, int k0, int nk, int sl, uint32_t (&v)[2]) {
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
         const int ks = 4 * sl + 2 * group + h;
@@ -771,12 +775,13 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
         v[h] = ks < nk ? *(const uint32_t *)(scp + off) : 0u;
       }
     };
-    const int tile_units = (nk + unit - 1) / unit;
+    const int tile_units_all = (nk_all + unit - 1) / unit;
     uint32_t isl = 0, it0 = 0;   // slots so far; units of the finished passes over k
     for (int t = tile_first; t < ntiles; t += tile_step) {
       const Tile p = tile_of(t);
       if (p.width == 0) continue;
-      const int kinds = kinds_of(p);
+      const int kinds = kinds_of(p), k0 = CUT_K ? p.k0 : 0, nk = CUT_K ? p.nk : nk_all, nslots = CUT_K ? (nk + 3) / 4 : nslots_all,
+                tile_units = CUT_K ? (nk + unit - 1) / unit : tile_units_all;
       const int r = min((2 * p.tm + rank) * 128 + row, gm - 1);
       const uint8_t *scp = img ? A.data + (size_t)(r >> 7) * A.ktiles * kImgTileBytes + kImgDataBytes + (r & 31) * 16 + ((r & 127) >> 5) * 4
                                : A.sc + sp.row(p.ro + r);
@@ -785,10 +790,10 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
       if (kKinds == 2 && !(kinds >> kind & 1)) continue;
       const uint4 *const table = lut + 256 * kind;
       uint32_t sc[2], sc_next[2] = {0, 0};
-      fetch_scales(scp, 0, sc);
+      fetch_scales(scp, k0, nk, 0, sc);
 #pragma unroll 1
       for (int sl = 0; sl < nslots; ++sl, ++isl) {
-        if (sl + 1 < nslots) fetch_scales(scp, sl + 1, sc_next);
+        if (sl + 1 < nslots) fetch_scales(scp, k0, nk, sl + 1, sc_next);
         const int rs = isl % kRaw;
         if (!__all_sync(0xFFFFFFFFu, wait(&raw_full[rs], (isl / kRaw) & 1, kStWaitRaw))) goto done;
         const uint8_t *src = sRaw + (size_t)rs * C::kRawBytes + row * 128;
@@ -879,18 +884,53 @@ Plan make_plan(int rows256, int n, int planes, int pairs, int widest) {
 // 12 tokens 26.3 -> 28.5 and BF16 872 x 5376 on 1030 29.6 -> 31.2, which this rule leaves whole.
 // (The number of tiles decides: a plain weight's rows and a shard of them may be cut differently and then differ in the last bits.)  Not for nvfp4a_gemm_ex (see
 // GemmArgs::whole_k), nor for images of BF16 problems: the outputs of a tensor-parallel shard are those of the whole matrix bit for bit, however many tiles either has.
-int choose_parts(const GemmArgs &g, int planes, const Plan &p, int pairs) {
+bool parts_allowed(const GemmArgs &g) {
   const bool tp_twin = g.A.image && g.B.dtype == NVFP4A_BF16;
-  if (tp_twin || g.no_alloc || g.whole_k || g.tp.world > 1 || g.x.mask || p.cut > 1 || 2 * p.tiles > pairs) return 1;
-  const int slots = (g.k + 255) / 256;
-  int parts = pairs / p.tiles;
+  return !(tp_twin || g.no_alloc || g.whole_k || g.tp.world > 1 || g.x.mask);
+}
+// parts of k, and the slots of 256 values in each but the last, for `tiles` tiles that have the pairs to themselves
+int most_parts(int k, int tiles, int pairs, int *run) {
+  const int slots = (k + 255) / 256;
+  int parts = pairs / tiles;
   if (parts > 8) parts = 8;
   if (parts > slots / 2) parts = slots / 2;
   if (parts < 2) return 1;
-  parts = (slots + (slots + parts - 1) / parts - 1) / ((slots + parts - 1) / parts);   // (equal runs: no empty part)
-  const int saved = (slots - (slots + parts - 1) / parts) * 4;   // stages
+  *run = (slots + parts - 1) / parts;
+  return (slots + *run - 1) / *run;   // (equal runs: no empty part)
+}
+int choose_parts(const GemmArgs &g, int planes, const Plan &p, int pairs) {
+  int run = 0;
+  if (!parts_allowed(g) || p.cut > 1 || p.tiles > pairs) return 1;
+  const int parts = most_parts(g.k, p.tiles, pairs, &run);
+  if (parts < 2) return 1;
+  const int saved = ((g.k + 255) / 256 - run) * 4;   // stages
   return saved * stage_cost(p.width, planes) > 8000 + 8ll * parts * g.n * g.m / 2000 ? parts : 1;
 }
+// The same for the last round of a problem of several: at a width whose last round has at most half as many tiles as there are pairs, those run in parts beside the whole ones.
+// The sums' way through memory and the join took 7 to 9 us up to 9000 tokens x parts of tiles (17000 of them 12 and more: there the last round is better left half as
+// wide), which the model's 5 us and 0.4 ns each stand for; the four per cent that a tail has to gain are what it does not know.  In a graph, INT8 2500 x 4288 on 1793 tokens 92.1 -> 78.1 us,
+// BF16 18997 x 7168 on 250 81.5 -> 61.6, FP16 4864 x 6208 on 600 85 - 95 -> 70 - 78, 4096 x 4096 on 700 51.0 -> 45.6, 3584 x 3584 on 1500 64.6 -> 61.3; forced, INT8 6144 x 4096
+// on 1000 80.8 -> 92.8 and BF16 49.0 -> 53.2, which the rule leaves whole.
+int choose_tail(const GemmArgs &g, int planes, int rows256, int pairs, int widest, Plan *p) {
+  if (!parts_allowed(g) || p->tiles <= pairs || g.e.beta != 0.f || g.e.d_dtype == NVFP4A_FP32 || g.e.amax) return 1;   // (whole tiles beside parts: the plain epilogue)
+  const int stages = (g.k + 63) / 64;
+  const long long last = p->cut > 1 || p->tiles % pairs ? stage_cost(p->width / p->cut, planes) : 0;
+  const long long whole = (p->nfull / pairs * stage_cost(p->width, planes) + last) * stages;
+  long long best = whole - whole / 25;
+  int parts = 1;
+  for (int w = widest; w >= 64; w -= w > 128 ? 64 : w / 2) {
+    const int tiles = rows256 * ((g.n + w - 1) / w), tail = tiles % pairs;
+    int run = 0;
+    const int q = tiles > pairs && tail ? most_parts(g.k, tail, pairs, &run) : 1;
+    const long long c = (tiles / pairs * stages + run * 4) * stage_cost(w, planes) + 5000 + (long long)q * tail * w * 2 / 5;
+    if (q < 2 || c >= best) continue;
+    best = c;
+    parts = q;
+    *p = Plan{w, tiles - tail, 1, tiles};
+  }
+  return parts;
+}
+size_t partial_bytes(int tiles, int parts, int width) { return (size_t)tiles * parts * width * 256 * sizeof(float); }
 
 // Grouped: only the average number of tokens per group is known here, and each group ends in a tile as wide as its last tokens (in steps
 // of 64).  `tiles` bounds the grid, the kernel counts the tiles itself.
@@ -941,8 +981,10 @@ cudaError_t launch_epi(const CUtensorMap &tw, const CUtensorMap &tb, const CUten
 
 template <int PLANES, bool F16, bool GROUPED = false>
 cudaError_t launch_cfg(const CUtensorMap &tw, const CUtensorMap &tb, const CUtensorMap &td, const PeerMaps &pm, const W4A16Args &a, cudaStream_t s) {
-  if constexpr (!GROUPED)
+  if constexpr (!GROUPED) {
+    if (a.parts > 1 && a.nfull) return launch_epi<PLANES, F16, GROUPED, kEpiTail>(tw, tb, td, pm, a, s);
     if (a.parts > 1) return launch_epi<PLANES, F16, GROUPED, kEpiPart>(tw, tb, td, pm, a, s);
+  }
   const bool scaled = a.e.beta == 0.f && a.e.d_dtype != NVFP4A_FP32, plain = scaled && !a.e.amax;
   if constexpr (!F16 && !GROUPED && PLANES < 3) {
     if (scaled && a.x.mask == (kExNorm | kExSwiglu)) return launch_epi<PLANES, F16, GROUPED, kEpiNormGlu>(tw, tb, td, pm, a, s);
@@ -956,12 +998,15 @@ cudaError_t launch_cfg(const CUtensorMap &tw, const CUtensorMap &tb, const CUten
   return launch_epi<PLANES, F16, GROUPED, kEpiAny>(tw, tb, td, pm, a, s);
 }
 
-// the tile plan of one weight and the parts of k
-int plan_parts(const GemmArgs &g, int planes, bool f16, Plan *plan) {
+// the tile plan of one weight; *parts: the parts of k, of all its tiles (nfull = 0) or of those from nfull on
+Plan plan_parts(const GemmArgs &g, int planes, bool f16, int *parts) {
   const int rows256 = (g.m + 255) / 256, pairs = device_sms() / 2;
-  const Plan p = make_plan(rows256, g.n, planes, pairs, f16 || planes == 3 ? kSegmentWidth : 256);
-  if (plan) *plan = p;
-  return choose_parts(g, planes, p, pairs);
+  const int widest = f16 || planes == 3 ? kSegmentWidth : 256;
+  Plan p = make_plan(rows256, g.n, planes, pairs, widest);
+  *parts = choose_parts(g, planes, p, pairs);
+  if (*parts > 1) p.nfull = 0;
+  else *parts = choose_tail(g, planes, rows256, pairs, widest, &p);
+  return p;
 }
 
 // what every launch of the kernel shares: arguments, the schedule, the maps of the weights, of the activations (`row_bytes` bytes per
@@ -974,11 +1019,8 @@ bool set_up(const GemmArgs &g, int planes, bool f16, int groups, const void *act
   a->e = g.e; a->x = g.x;
   a->status = kernel_status_device_ptr();
   a->tag = next_launch_tag();
-  const int rows256 = (g.m + 255) / 256, pairs = device_sms() / 2;
-  Plan p;
   a->parts = 1;
-  if (groups) p = make_grouped_plan(rows256, g.n, groups, planes, pairs, kSegmentWidth);
-  else a->parts = plan_parts(g, planes, f16, &p);
+  const Plan p = groups ? make_grouped_plan((g.m + 255) / 256, g.n, groups, planes, device_sms() / 2, kSegmentWidth) : plan_parts(g, planes, f16, &a->parts);
   const uint64_t wrows = (uint64_t)g.m * (groups ? groups : 1);
   a->unit = planes == 1 && !(f16 && g.k < 512) ? 2 : 1;
   a->seg_stages = g.k >= 1024 ? 4 : g.k >= 512 ? 2 : 1;   // (the longest that keep the sums no less exact than the CUDA-core kernels': see the head of the file)
@@ -986,7 +1028,7 @@ bool set_up(const GemmArgs &g, int planes, bool f16, int groups, const void *act
   if (a->parts > 1) {
     const int slots = (g.k + 255) / 256;
     a->part_stages = (slots + a->parts - 1) / a->parts * 4;
-    a->nfull = a->tiles *= a->parts;
+    a->tiles = p.nfull + (p.tiles - p.nfull) * a->parts;
   }
   const uint64_t wtiles = (uint64_t)((g.m + 127) / 128) * g.A.ktiles;
   if (g.A.image ? !make_tmap_bytes(tw, g.A.data, 128, 128, 128, 128, wtiles, kImgTileBytes)
@@ -997,7 +1039,7 @@ bool set_up(const GemmArgs &g, int planes, bool f16, int groups, const void *act
   const int esz = dense_bytes(g.e.d_dtype);
   const bool glu = (g.x.mask & kExSwiglu) != 0;
   const int drows = glu ? g.m / 2 : g.m;   // SwiGLU: the output has m / 2 rows, 64 per 128-row tile
-  a->d_tma = a->parts == 1 && esz == 2 && ((uintptr_t)g.e.d & 15) == 0 && ((size_t)g.e.ldd * esz) % 16 == 0 && ((size_t)drows * esz) % 16 == 0 &&
+  a->d_tma = (a->parts == 1 || a->nfull) && esz == 2 && ((uintptr_t)g.e.d & 15) == 0 && ((size_t)g.e.ldd * esz) % 16 == 0 && ((size_t)drows * esz) % 16 == 0 &&
              make_tmap_dense(td, g.e.d, esz, (uint64_t)drows, (uint64_t)g.n, (uint64_t)g.e.ldd * esz, 64, 32, 128);
   return true;
 }
@@ -1109,17 +1151,19 @@ __global__ void __launch_bounds__(256) w4a8_wide_planes_kernel(const int8_t *q_i
   }
 }
 
-// The parts' sums [parts][n][m] added in order, then the plain epilogue.
-__global__ void __launch_bounds__(256) w4a16_join_kernel(const float *partial_in, int parts, int m, int n, const Epilogue e) {
+// The parts' sums of the tiles from nfull on (one per blockIdx.x) added in order, then the plain epilogue: a thread per row, a token per blockIdx.y.
+__global__ void __launch_bounds__(256) w4a16_join_kernel(const float *partial_in, int parts, int width, int nfull, int m, int n, const Epilogue e) {
   pdl_launch_dependents();
   pdl_wait();
-  const float *const p = behind_wait(partial_in);
-  const int i = blockIdx.x * 256 + threadIdx.x, j = blockIdx.y;
+  const int tiles_m = (m + 255) / 256, t = nfull + blockIdx.x;
+  const int i = t % tiles_m * 256 + threadIdx.x, j = t / tiles_m * width + blockIdx.y;
+  if (j >= n) return;
+  const size_t step = (size_t)width * 256;
+  const float *const p = behind_wait(partial_in) + (size_t)blockIdx.x * parts * step + blockIdx.y * 256 + threadIdx.x;
   float amax = 0.f;
   if (i < m) {
-    const size_t at = (size_t)j * m + i, step = (size_t)n * m;
-    float s = p[at];
-    for (int q = 1; q < parts; ++q) s = __fadd_rn(s, p[at + q * step]);
+    float s = p[0];
+    for (int q = 1; q < parts; ++q) s = __fadd_rn(s, p[q * step]);
     const float v = epi_value(e, i, j, s, epi_scale(e, epi_row_part(e, i), epi_col_part(e, j)));
     store_dense(e.d_dtype, e.d, (size_t)j * e.ldd + i, v);
     amax = fabsf(v);
@@ -1205,14 +1249,14 @@ static cudaError_t give_scratch(const Scratch &t, cudaStream_t s) { return t.poo
 static cudaError_t launch_join(const W4A16Args &a, cudaStream_t s) {
   cudaLaunchConfig_t cfg;
   memset(&cfg, 0, sizeof cfg);
-  cfg.gridDim = dim3((unsigned)((a.m + 255) / 256), (unsigned)a.n, 1);
+  cfg.gridDim = dim3((unsigned)((a.tiles - a.nfull) / a.parts), (unsigned)(a.width < a.n ? a.width : a.n), 1);
   cfg.blockDim = dim3(256, 1, 1);
   cfg.stream = s;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr; cfg.numAttrs = pdl_enabled() ? 1 : 0;
-  return cudaLaunchKernelEx(&cfg, w4a16_join_kernel, (const float *)a.partial, a.parts, a.m, a.n, a.e);
+  return cudaLaunchKernelEx(&cfg, w4a16_join_kernel, (const float *)a.partial, a.parts, a.width, a.nfull, a.m, a.n, a.e);
 }
 cudaError_t trim_planes_pool() {
   int dev = 0;
@@ -1252,10 +1296,11 @@ cudaError_t launch_gemm_w4a8_tc(const GemmArgs &g, const int *seg, int groups, c
   const int per_token = three ? 3 : 5;
   const size_t plane_bytes = (size_t)g.n * per_token * g.k * sizeof(uint16_t), small_bytes = (plane_bytes + (size_t)(g.n + 1) * sizeof(float) + g.n + 255) / 256 * 256;
   GemmArgs w = g;
-  const int parts = seg ? 1 : plan_parts(g, three ? 3 : 2, false, nullptr);
+  int parts = 1;
+  const Plan p = seg ? Plan{} : plan_parts(g, three ? 3 : 2, false, &parts);
   Scratch scratch = {nullptr, false};
   if (parts > 1) {
-    scratch = take_scratch(small_bytes + (size_t)parts * g.n * g.m * sizeof(float), s, in_capture);
+    scratch = take_scratch(small_bytes + partial_bytes(p.tiles - p.nfull, parts, p.width), s, in_capture);
     if (!scratch.p) w.no_alloc = 1;   // k stays whole
   }
   if (!scratch.p) scratch = take_scratch(small_bytes, s, in_capture);
@@ -1323,7 +1368,7 @@ cudaError_t launch_gemm_w4a16(const GemmArgs &g, cudaStream_t s) {
   auto go = [&]() { return g.B.dtype == NVFP4A_FP16 ? launch_cfg<1, true>(tw, tb, td, pm, a, s) : launch_cfg<1, false>(tw, tb, td, pm, a, s); };
   Scratch scratch = {nullptr, false};
   if (a.parts > 1) {
-    scratch = take_scratch((size_t)a.parts * g.n * g.m * sizeof(float), s, false);
+    scratch = take_scratch(partial_bytes(a.tiles - a.nfull, 1, a.width), s, false);
     a.partial = (float *)scratch.p;
     if (!scratch.p) {   // k stays whole
       GemmArgs whole = g;

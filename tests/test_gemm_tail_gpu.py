@@ -1,0 +1,42 @@
+"""The tensor-core kernel's last round of tiles in parts of k beside whole tiles, against the oracle."""
+import ctypes
+
+import numpy as np
+import pytest
+
+from nvfp4effma_b200 import _lib as L
+from test_gemm_gpu import Case, DevFp4, build_case, check_bound, dev, device_b, host, kernel_status, oracle_case, stream, tensor
+
+pytestmark = pytest.mark.gpu
+SW = L.SCALES_SWIZZLED
+
+
+def run_plain(c, h):
+    """nvfp4a_gemm without an amax (the plain epilogue)."""
+    dA, (keep, tB), dD = DevFp4(h["A"]), device_b(c, h), dev(h["Dinit"])
+    bias = dev(h["bias"]) if h["bias"] is not None else None
+    tA, tD, tbias = dA.tensor(), tensor(dD, c.dt), tensor(bias, c.bias) if bias is not None else None
+    L.check(L.lib.nvfp4a_gemm(c.m, c.n, c.k, c.alpha, ctypes.byref(tA), h["lda"], ctypes.byref(tB), h["ldb"], 0.0, None, 0, ctypes.byref(tD), h["ldd"],
+                              ctypes.byref(tbias) if tbias is not None else None, stream()))
+    return host(dD).view(h["Dinit"].dtype)
+
+
+# (74 SM pairs; tiles of 256 rows and at most 256 tokens, 128 with FP16; an output pitch that TMA stores take and one that they do not)
+@pytest.mark.parametrize("bt,m,n,k", [
+    (L.INT8, 2500, 1793, 4096 + 192),  # a last token alone in its tile, rows past the matrix, an odd number of stages
+    (L.BF16, 18997, 250, 7168),       # one tile more than a round
+    (L.FP16, 4864, 600, 6144 + 64),
+])
+@pytest.mark.parametrize("fa,out,bias,pitch", [(0, L.BF16, -1, 8), (SW, L.FP16, L.BF16, 3)])
+def test_last_round_in_parts_of_k(bt, m, n, k, fa, out, bias, pitch):
+    """Whole tiles and parts both within the bound of one sum over k, every output written, the same bytes on every call."""
+    c = Case(m, n, k, bt, out, -1, bias, 2.0 ** -12 if out == L.FP16 else 1.25, 0.0, fa=fa)   # (FP16: inside its range)
+    h = build_case(c, 5400)
+    h["ldd"] = (m + 7) // 8 * 8 + pitch
+    h["Dinit"] = np.resize(h["Dinit"], n * h["ldd"])
+    exp = oracle_case(c, h, want_ref=True)
+    got = run_plain(c, h)
+    assert L.lib.nvfp4a_b200_last_route() == (8 if bt == L.INT8 else 5) and L.lib.nvfp4a_b200_last_parts() > 1
+    check_bound(c, h, got, float(exp["amax"]), exp)
+    assert np.array_equal(got.view(np.uint8), run_plain(c, h).view(np.uint8))
+    assert kernel_status() == 0
