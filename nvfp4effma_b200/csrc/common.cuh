@@ -120,6 +120,18 @@ __device__ __forceinline__ void e2m1_expand4(uint32_t w, const uint4 &t, uint32_
   o1 = byte_perm(lo, hi, 0x7362u);
 }
 
+// eight E2M1 nibbles -> four pairs of FP16 values, in the order of k
+__device__ __forceinline__ void e2m1_to_f16(uint32_t w, uint32_t (&o)[4]) {
+  asm("{\n\t.reg .b8 b0, b1, b2, b3;\n\tmov.b32 {b0, b1, b2, b3}, %4;\n\tcvt.rn.f16x2.e2m1x2 %0, b0;\n\tcvt.rn.f16x2.e2m1x2 %1, b1;\n\t"
+      "cvt.rn.f16x2.e2m1x2 %2, b2;\n\tcvt.rn.f16x2.e2m1x2 %3, b3;\n\t}"
+      : "=r"(o[0]), "=r"(o[1]), "=r"(o[2]), "=r"(o[3]) : "r"(w));
+}
+// two E4M3 codes -> their values * 2^-8 as a pair of FP16 values (0x7F: 480 * 2^-8)
+__device__ __forceinline__ uint32_t scale_pair(uint32_t v) {
+  const uint32_t t = byte_perm(v, 0u, 0x1404u);
+  return ((t >> 1) & 0x3F803F80u) | (t & 0x80008000u);
+}
+
 // Data that another kernel (programmatic dependent launch) or a peer writes until a wait of this kernel returns: `p` after the wait is a value the
 // compiler cannot have known before, so no load through it moves up across the wait.  ld16 is an ordinary load (not ld.global.nc, which
 // promises that nobody writes during the kernel's lifetime) that the compiler may otherwise schedule as freely as a read-only one.

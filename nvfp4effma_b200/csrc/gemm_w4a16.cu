@@ -22,10 +22,10 @@
 //               plain or extended epilogue (RMSNorm column scale, SwiGLU, second output + sums of squares), D through
 //               shared-memory staging tiles and TMA stores when its layout allows
 //   warps 12-19 weight expansion, two groups of four warps on alternate pairs of stages.  The eight magnitudes of E2M1 times a block scale
-//               are eight 16-bit floats (exact: 2 x 4 significant bits); a 4 KiB table (PLANES = 2: one for FP16 and one for BF16) holds their high and low bytes for each of
+//               are eight 16-bit floats (exact: 2 x 4 significant bits); for BF16 a 4 KiB table holds their high and low bytes for each of
 //               the 256 scale codes, so a block costs one 16-byte table read and four values cost three byte permutes (the packed
 //               nibbles ARE the permute's selectors: high bytes, low bytes, signs), two of them again to interleave, and two
-//               logical operations -- 2 instructions per value where shifts, masks, the multiply and reordering took 3.
+//               logical operations -- 2 instructions per value where shifts, masks, the multiply and reordering took 3.  (FP16: see below.)
 // Instruction issue, not the tensor pipe, bounded the former kernel (a thread-per-row expansion through shared memory with a proxy
 // fence per stage: 1240 cycles per stage of 512 cycles of MMAs, 41 % of the tensor pipe).
 // The last round of tiles over the SM pairs is cut along the tokens, or into parts of k (see choose_tail), when it would leave pairs idle, and a tile at the end of the
@@ -33,7 +33,9 @@
 // Every wait is bounded; a wait that gives up raises the CTA's abort flag and the kernel status word.
 //
 // FP16 activations (F16): e2m1 x E4M3 is a multiple of 2^-10 up to 2880 with at most 6 significant bits, exact in FP16, so the same
-// kernel runs on FP16 operands.
+// kernel runs on FP16 operands.  FP16 weights come from the hardware's conversions of E2M1 pairs and one packed multiply by the block's scale, both exact: 1.4
+// instructions per value and no table, whose sixteen-byte reads at 32 unrelated addresses also met in the banks (in a graph, FP16 4096 x 4096 on 700 tokens 45.8 -> 41.6 us,
+// 3584 x 3584 on 1500 61 -> 56, 4864 x 6208 on 600 70 -> 57; INT8, whose first pass runs on them too and which the MMAs bound, 6144 x 4096 on 1000 80.6 -> 79.5).
 //
 // Segments.  The tensor cores truncate the running sum at every instruction, so that one chain over all of k drifts towards zero: at k = 4096 its
 // error against 64 bits is 1.3e-6 (BF16 / FP16 activations) and 9.9e-6 (INT8, three chains in one) where the ordered FP32 sums of the
@@ -104,7 +106,7 @@ struct Cfg {
   static constexpr int kA = PLANES == 3 ? 4 : 8, kB = 8, kRaw = 3;
   static constexpr int kACols = 512 - 32 * kA;   // first tensor memory column of the weight stages (32 columns each)
   static constexpr int kBBytes = 128 * 128, kRawBytes = 128 * 128, kStagingBytes = 8192;
-  static constexpr int kSmemBytes = 1024 + kB * kBBytes + kRaw * kRawBytes + 4 * kStagingBytes + (PLANES == 2 ? 8192 : 4096) /* expansion tables */ + 256 * 4 /* column scales */ +
+  static constexpr int kSmemBytes = 1024 + kB * kBBytes + kRaw * kRawBytes + 4 * kStagingBytes + 4096 /* expansion table */ + 256 * 4 /* column scales */ +
                                     512 /* barriers */ + 2 * 257 * 4 + 8 /* groups */;
 };
 static_assert(Cfg<1, false>::kSmemBytes <= 232448 && Cfg<2, false>::kSmemBytes <= 232448, "shared memory budget");
@@ -115,6 +117,11 @@ static_assert(128 * kRegsRest + 256 * kRegsEpi + 256 * kRegsConv <= kThreads * 9
 constexpr unsigned kStWaitFullA = 0x301, kStWaitFullB = 0x302, kStWaitEmpty = 0x303, kStWaitTmemFull = 0x304, kStWaitTmemEmpty = 0x305,
                    kStWaitConv = 0x306, kStWaitRaw = 0x307;
 
+__device__ __forceinline__ uint32_t h2mul(uint32_t a, uint32_t b) {
+  uint32_t d;
+  asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+  return d;
+}
 __device__ __forceinline__ uint32_t bf16x2_rn(float lo, float hi) {
   uint32_t d;
   asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(d) : "f"(hi), "f"(lo));
@@ -203,7 +210,7 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
   uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint8_t *const sB = smem, *const sRaw = sB + kB * C::kBBytes, *const staging = sRaw + kRaw * C::kRawBytes;
   uint4 *lut = (uint4 *)(staging + 4 * C::kStagingBytes);           // scale code -> bytes of the eight products (see e2m1_expand4)
-  float *colscale = (float *)(lut + (PLANES == 2 ? 512 : 256));                           // RMSNorm column scales of the current token tile
+  float *colscale = (float *)(lut + 256);                           // RMSNorm column scales of the current token tile
   uint64_t *bars = (uint64_t *)(colscale + 256);
   uint64_t *a_full = bars, *b_full = a_full + kA, *b_empty = b_full + kB, *a_empty = PLANES == 1 ? b_empty : b_empty + kB,
            *raw_full = b_empty + kB + kA, *raw_empty = raw_full + kRaw, *tmem_full = raw_empty + kRaw, *tmem_empty = tmem_full + 2;
@@ -239,14 +246,12 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
     prefetch_tensormap(&tmap_w);
     prefetch_tensormap(&tmap_b);
   }
-  for (int i = threadIdx.x; i < (PLANES == 2 ? 512 : 256); i += kThreads) {   // (PLANES = 2: a table for FP16, then one for BF16)
-    const bool half = PLANES == 2 ? i < 256 : F16;
-    const float sc = scale_to_f32((uint32_t)i & 255u, ue);
+  for (int i = threadIdx.x; i < (F16 ? 0 : 256); i += kThreads) {   // (FP16 weights come from conversions)
+    const float sc = scale_to_f32((uint32_t)i, ue);
     uint32_t hi[2] = {0, 0}, lo[2] = {0, 0};
 #pragma unroll
     for (int c = 0; c < 8; ++c) {
-      const float v = __fmul_rn(e2m1_to_f32(c), sc);   // exact in 16 bits
-      const uint32_t h = half ? (uint32_t)__half_as_ushort(__float2half_rn(v)) : __float_as_uint(v) >> 16;
+      const uint32_t h = __float_as_uint(__fmul_rn(e2m1_to_f32(c), sc)) >> 16;   // exact in 16 bits
       hi[c >> 2] |= (h >> 8) << (8 * (c & 3));
       lo[c >> 2] |= (h & 0xFFu) << (8 * (c & 3));
     }
@@ -788,7 +793,6 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
 #pragma unroll 1
       for (int kind = 0; kind < kKinds; ++kind) {
       if (kKinds == 2 && !(kinds >> kind & 1)) continue;
-      const uint4 *const table = lut + 256 * kind;
       uint32_t sc[2], sc_next[2] = {0, 0};
       fetch_scales(scp, k0, nk, 0, sc);
 #pragma unroll 1
@@ -814,9 +818,22 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
           for (int u = 0; u < 2; ++u) {   // 32 values: two blocks, 16 columns
             const uint32_t wv[4] = {w[2 * h + u].x, w[2 * h + u].y, w[2 * h + u].z, w[2 * h + u].w};
             uint32_t o[16];
+            if (F16 || (PLANES == 2 && kind == 0)) {   // (E4M3 scales) conversions to FP16 and one multiply per pair of values, exact
+              const uint32_t s2 = h2mul(scale_pair(sc[h] >> (16 * u)), 0x5C005C00u);   // (2^8: scale_pair's are that much smaller)
+#pragma unroll
+              for (int q = 0; q < 4; ++q) {
+                uint32_t v[4];
+                e2m1_to_f16(wv[q], v);
+                const uint32_t sb = byte_perm(s2, s2, q >> 1 ? 0x3232u : 0x1010u);
+#pragma unroll
+                for (int e = 0; e < 4; ++e) o[4 * q + e] = h2mul(v[e], sb);
+              }
+              tmem_st16(dst + 16 * u, o);
+              continue;
+            }
 #pragma unroll
             for (int q = 0; q < 4; ++q) {  // 8 values per word
-              const uint4 t4 = table[(sc[h] >> (16 * u + 8 * (q >> 1))) & 0xFF];
+              const uint4 t4 = lut[(sc[h] >> (16 * u + 8 * (q >> 1))) & 0xFF];
               e2m1_expand4(wv[q], t4, o[4 * q], o[4 * q + 1]);
               e2m1_expand4(wv[q] >> 16, t4, o[4 * q + 2], o[4 * q + 3]);
             }

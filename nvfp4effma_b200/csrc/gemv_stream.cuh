@@ -10,12 +10,6 @@ constexpr int kStreamUnitK = 128;      // a warp's unit: 16 rows x 128 values
 
 __device__ __forceinline__ void prefetch_line(const void *p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 
-// eight E2M1 nibbles -> four pairs of FP16 values, in the order of k
-__device__ __forceinline__ void e2m1_to_f16(uint32_t w, uint32_t (&o)[4]) {
-  asm("{\n\t.reg .b8 b0, b1, b2, b3;\n\tmov.b32 {b0, b1, b2, b3}, %4;\n\tcvt.rn.f16x2.e2m1x2 %0, b0;\n\tcvt.rn.f16x2.e2m1x2 %1, b1;\n\t"
-      "cvt.rn.f16x2.e2m1x2 %2, b2;\n\tcvt.rn.f16x2.e2m1x2 %3, b3;\n\t}"
-      : "=r"(o[0]), "=r"(o[1]), "=r"(o[2]), "=r"(o[3]) : "r"(w));
-}
 __device__ __forceinline__ void mma16(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
   asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
       : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
@@ -24,11 +18,6 @@ __device__ __forceinline__ void mma16(float (&c)[4], uint32_t a0, uint32_t a1, u
 __device__ __forceinline__ void mma16_first(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
   asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%10, %10, %10, %10};"
       : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.f));
-}
-// two E4M3 codes -> their values * 2^-8 as a pair of FP16 values (0x7F: 480 * 2^-8)
-__device__ __forceinline__ uint32_t scale_pair(uint32_t v) {
-  const uint32_t t = byte_perm(v, 0u, 0x1404u);
-  return ((t >> 1) & 0x3F803F80u) | (t & 0x80008000u);
 }
 __device__ __forceinline__ uint4 lds16(uint32_t a) {
   uint4 v;
