@@ -591,8 +591,8 @@ int gemv_fp4_pinned_splits() { return g_gemv_splits.load(); }
 
 // splits: power of two, at most 8 and nk; every CTA's k range is at most kMaxChunks chunks (its pieces' shared memory).  Returns 0 when the
 // kernel should not run.  Pinned (nvfp4a_b200_set_gemv_splits): that value if the problem can use it.  Automatic: problems that stream at
-// least 32 MB of weights over at least 96 CTAs.  One vector, CUDA-graph timings here and on the mma.sync GEMV (gemv_stream.cu): 28672 x 4096 14.9 against 21.3 us, 8192 x
-// 8192 11.2 against 14.0.  Smaller matrices belong to the mma.sync GEMV, whose time hardly depends on the activations: 6144 x 4096 takes 7.2 us here and 7.1
+// least 32 MB of weights over at least 96 CTAs.  One vector, CUDA-graph timings here and on the mma.sync GEMV (gemv_stream.cu): 28672 x 4096 14.4 against 21.3 us, 8192 x
+// 8192 10.4 against 14.0.  Smaller matrices belong to the mma.sync GEMV, whose time hardly depends on the activations: 6144 x 4096 takes 7.2 us here and 7.1
 // there, 4096 x 14336 12.9 and 13.2, but with 1 / 8 / 64 activations of a CTA below the planes 9.2 / 11.6 / 25.7 and 15.0 / 18.2 / 36.7 here, and with
 // more of them 22.7 and 63.1 -- and the inputs of 4096 x 14336, a decoder's down projection, are products, which spread that far.  (28672 x 4096: 16.2 /
 // 19.6 / 42.9 and 69.9.)
