@@ -90,7 +90,7 @@ int nvfp4a_b200_set_swap(int mode);
 int nvfp4a_b200_last_route(void);
 
 /* The tensor-core W4A8 GEMM keeps the memory of its activation planes (10 bytes per INT8 activation of the largest call so far), and W4A16 /
- * W4A8 GEMMs with few tiles and a long k that of their FP32 sums over parts of k (at most 19.4 MB), in
+ * W4A8 GEMMs with few tiles (in all, or in their last round) and a long k that of their FP32 sums over parts of k (at most 19.4 MB), in
  * a memory pool of its own per device, so that later calls allocate in microseconds and without synchronising.  This call gives
  * the current device's pool memory that is not in use back to the system (no counterpart in the reference). */
 nvfp4a_status nvfp4a_b200_trim_scratch(void);

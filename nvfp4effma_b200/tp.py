@@ -7,8 +7,8 @@ shard's swizzled block scales are a contiguous range of the tensor's (128-row ti
 SwiGLU weight stay whole.  A tensor is quantized BEFORE it is sharded: the per-tensor global is shared by all shards and a
 rank's outputs equal the corresponding outputs of the one-GPU call bit for bit wherever both run the same kernel in the same number
 of parts of k.  A decode shard may be too small for the FP4 tensor-core GEMVs, which add in another order (``nvfp4a_b200_set_route(2)``
-leaves those out).  The layers here keep k whole; ``linear`` on ``shard_rows`` of a plain weight with more than 8 tokens may cut k where
-a shard has few tiles and the whole matrix many (``nvfp4a_b200_last_parts``), and the sums then differ in their last bits.
+leaves those out).  The layers here keep k whole; ``linear`` on ``shard_rows`` of a plain weight with more than 8 tokens may cut k, in
+all tiles or in those of the last round, where the whole matrix is cut otherwise (``nvfp4a_b200_last_parts``), and the sums then differ in their last bits.
 
 One process per GPU (``torch.distributed``).  The layout functions (``shard_bounds``, ``shard_rows``, ``gather_features``)
 work on tensors of any device and with any backend, which is how the host logic is tested on CPU ranks over gloo; the
