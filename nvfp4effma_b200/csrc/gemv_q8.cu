@@ -130,7 +130,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemv_q8_kernel(const GemvQArgs g)
   f.prefetch(kAhead);
   if (S > 1) sm100::cluster_arrive_release();
   sm100::pdl_wait();
-  f.w = behind_wait(f.w); f.s = behind_wait(f.s);
+  f.start_behind_wait();
   WeightUnit ahead[kAhead];
 #pragma unroll
   for (int i = 0; i < kAhead; ++i) ahead[i] = f.fetch();

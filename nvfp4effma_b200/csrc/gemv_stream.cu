@@ -111,12 +111,12 @@ __global__ void __launch_bounds__(kThreads, 1) gemv_stream_kernel(const StreamAr
   f.prefetch(kAhead);
   if (S > 1) sm100::cluster_arrive_release();
   sm100::pdl_wait();
-  // tensor-parallel layers in the deferred form: the activations are complete once every peer has posted the previous gather
-  if (g.tp.world > 1 && (g.tp.deferred & 1)) tp_wait_posts(g.tp.flags, g.tp.world, g.tp.rank, g.tp.status, g.tp.tag, g.tp.wait_cycles);
-  f.w = behind_wait(f.w); f.s = behind_wait(f.s);
+  f.start_behind_wait();
   WeightUnit ahead[kAhead];
 #pragma unroll
   for (int i = 0; i < kAhead; ++i) ahead[i] = f.fetch();
+  // tensor-parallel layers in the deferred form: the activations are complete once every peer has posted the previous gather (the weights are on their way)
+  if (g.tp.world > 1 && (g.tp.deferred & 1)) tp_wait_posts(g.tp.flags, g.tp.world, g.tp.rank, g.tp.status, g.tp.tag, g.tp.wait_cycles);
   if (tid == 0) any_more_s = 0;
   for (int i = tid; i < sec; i += kThreads) more[i] = 0;
   for (int i = tid; i < chunk_x / 16; i += kThreads) ((uint4 *)zeros)[i] = make_uint4(0, 0, 0, 0);

@@ -40,8 +40,11 @@ struct WeightUnit { uint4 wa, wb; uint32_t ca, cb; };
 
 // The units of one warp: of every SG-th slice of a CTA's run, every KG-th unit of the CTA's range of k [256 c_first, 256 c_first + kloc).  KG is even, or a slice
 // has one unit: a warp then stays in the same half of an image's tiles.
+// Every address comes from `data` and `sc`: start_behind_wait() makes them values that the compiler cannot have known before the programmatic wait, so that no load
+// of any slice moves up across it (see behind_wait).
 template <bool IMG> struct UnitStream {
   const Fp4Operand &A;
+  const uint8_t *data, *sc;   // A's
   int gm, s_first, s_count, c_first, kloc, units, KG, SG, kg, sg, gq, q;
   bool lin;
   int slice, unit;            // the next unit to be requested
@@ -49,7 +52,7 @@ template <bool IMG> struct UnitStream {
   uint32_t w8, s8;            // from there to row gq + 8
   uint32_t step_w, step_s;
   __device__ __forceinline__ UnitStream(const Fp4Operand &a, int gm_, int s_first_, int s_count_, int c_first_, int kloc_, int KG_, int warp, int warps, int lane)
-      : A(a), gm(gm_), s_first(s_first_), s_count(s_count_), c_first(c_first_), kloc(kloc_), units((kloc_ + kStreamUnitK - 1) / kStreamUnitK), KG(KG_),
+      : A(a), data(a.data), sc(a.sc), gm(gm_), s_first(s_first_), s_count(s_count_), c_first(c_first_), kloc(kloc_), units((kloc_ + kStreamUnitK - 1) / kStreamUnitK), KG(KG_),
         SG(warps / KG_), kg(warp & (KG_ - 1)), sg(warp / KG_), gq(lane >> 2), q(lane & 3), lin(!IMG && a.sld > 0), w(a.data), s(a.data), w8(0), s8(0) {
     step_w = IMG ? (uint32_t)(KG >> 1) * kImgTileBytes : (uint32_t)KG * 64;
     step_s = IMG ? (uint32_t)(KG >> 1) * kImgTileBytes : (uint32_t)KG * (lin ? 8 : 1024);
@@ -59,16 +62,16 @@ template <bool IMG> struct UnitStream {
     const int row0 = slice_row(s_first + slice, gm);
     if (IMG) {
       const int rr = (row0 & 127) + gq;
-      const uint8_t *t = A.data + ((size_t)(row0 >> 7) * A.ktiles + c_first + (kg >> 1)) * kImgTileBytes;
+      const uint8_t *t = data + ((size_t)(row0 >> 7) * A.ktiles + c_first + (kg >> 1)) * kImgTileBytes;
       w = t + rr * 128 + (kg & 1) * 64 + q * 16;
       s = t + kImgDataBytes + (kg & 1) * 1024 + (q >> 1) * 512 + (rr & 31) * 16 + (rr >> 5) * 4 + (q & 1) * 2;
       w8 = 1024; s8 = 128;
     } else {
       const int r0 = min(row0 + gq, gm - 1), r1 = min(row0 + gq + 8, gm - 1);
       const ScalePos sp{A.sld};
-      w = A.data + (size_t)r0 * (A.ld >> 1) + (size_t)c_first * 128 + kg * 64 + q * 16;
+      w = data + (size_t)r0 * (A.ld >> 1) + (size_t)c_first * 128 + kg * 64 + q * 16;
       w8 = (uint32_t)(r1 - r0) * (uint32_t)(A.ld >> 1);
-      s = A.sc + sp.row(r0) + (lin ? (size_t)c_first * 16 + kg * 8 + q * 2 : (size_t)c_first * 2048 + kg * 1024 + (q >> 1) * 512 + (q & 1) * 2);
+      s = sc + sp.row(r0) + (lin ? (size_t)c_first * 16 + kg * 8 + q * 2 : (size_t)c_first * 2048 + kg * 1024 + (q >> 1) * 512 + (q & 1) * 2);
       s8 = (uint32_t)(sp.row(r1) - sp.row(r0));
     }
   }
@@ -76,6 +79,12 @@ template <bool IMG> struct UnitStream {
     slice = kg < units ? at : s_count;
     unit = kg;
     if (slice < s_count) start_slice();
+  }
+  // after the programmatic wait: the first unit again
+  __device__ __forceinline__ void start_behind_wait() {
+    data = behind_wait(data);
+    if (!IMG) sc = behind_wait(sc);
+    restart(sg);
   }
   __device__ __forceinline__ bool in_k() const { return IMG || unit * kStreamUnitK + q * 32 < kloc; }   // (the last unit of a plain operand may be short)
   __device__ __forceinline__ void advance() {
@@ -85,13 +94,12 @@ template <bool IMG> struct UnitStream {
       if (slice < s_count) start_slice();
     }
   }
-  // the first units' lines into L2 (a prefetch reads nothing: a predecessor may still be writing the weights)
+  // the first units' lines into L2 (a prefetch reads nothing: a predecessor may still be writing the weights); start_behind_wait() follows
   __device__ __forceinline__ void prefetch(int count) {
     for (int i = 0; i < count && slice < s_count; ++i) {
       if (in_k()) { prefetch_line(w); prefetch_line(w + w8); prefetch_line(s); }
       advance();
     }
-    restart(sg);
   }
   __device__ __forceinline__ WeightUnit fetch() {
     WeightUnit v;

@@ -37,6 +37,9 @@ def test_kernels_that_start_before_their_producer_ends_use_no_read_only_loads():
         if "pdl_wait()" in text:
             early.append(name)
             assert "__ldg(" not in text and "ld.global.nc" not in text, name
+            for header in re.findall(r'#include "(\w+\.cuh)"', text):    # (and what it takes its loads from)
+                included = re.sub(r"//.*", "", open(os.path.join(csrc, header)).read())
+                assert "__ldg(" not in included and "ld.global.nc" not in included, (name, header)
         elif "tp_wait_posts(" in text:
             assert "__ldg(xrow" not in text and "__ldg(g.x" not in text, name
     assert len(early) >= 4, early
@@ -45,10 +48,26 @@ def test_kernels_that_start_before_their_producer_ends_use_no_read_only_loads():
 def test_deferred_tensor_parallel_gemvs_read_activations_behind_a_cta_barrier():
     """tp_wait_posts is executed by `world` threads of a CTA; the others know that the peers have posted only after a CTA barrier."""
     csrc = os.path.join(ROOT, "nvfp4effma_b200", "csrc")
-    for name in ("gemv.cu", "gemv_fp4.cu", "gemv_fp4_n8.cu"):
+    for name in ("gemv.cu", "gemv_fp4.cu", "gemv_fp4_n8.cu", "gemv_stream.cu"):
         text = re.sub(r"//.*", "", open(os.path.join(csrc, name)).read())
         after = text[text.index("tp_wait_posts("):]
         assert after.index("__syncthreads()") < after.index("behind_wait(") <= after.index("ld16("), name
+
+
+def test_streamed_weights_are_addressed_behind_the_programmatic_wait():
+    """Before the wait a predecessor may still be writing the weights.  Loads are free to move up to where their address is known, so UnitStream's addresses -- of
+    every slice, not of the first alone -- come from bases that pass through behind_wait after the wait."""
+    csrc = os.path.join(ROOT, "nvfp4effma_b200", "csrc")
+    text = re.sub(r"//.*", "", open(os.path.join(csrc, "gemv_stream.cuh")).read())
+    stream = text[text.index("struct UnitStream"):text.index("};", text.index("WeightUnit fetch()"))]
+    methods = stream[stream.index("void start_slice()"):]
+    assert "A.data" not in methods and "A.sc" not in methods
+    start = methods[methods.index("void start_behind_wait()"):]
+    start = start[:start.index("}")]
+    assert start.index("data = behind_wait(data)") < start.index("restart(") and start.index("sc = behind_wait(sc)") < start.index("restart(")
+    for name in ("gemv_stream.cu", "gemv_q8.cu"):
+        kernel = re.sub(r"//.*", "", open(os.path.join(csrc, name)).read())
+        assert kernel.index("pdl_wait()") < kernel.index("start_behind_wait()") < kernel.index(".fetch()"), name
 
 
 def test_the_torch_operators_library_belongs_to_one_version_of_torch(monkeypatch):
