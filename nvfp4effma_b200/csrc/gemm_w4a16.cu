@@ -194,11 +194,12 @@ constexpr int kMaxGroups = 256;
 // which a plain call's instructions lie far apart: fetching them made a chunk of 32 columns take 5000 cycles, in which the tensor cores wait for the
 // accumulator or, at the end, the caller for the result.  28672 x 4096 with SwiGLU on 2048 tokens: 412 -> 344 us; FP16 4096 x 4096 on 333
 // tokens 37.5 -> 35.2; 5504 x 3584 with SwiGLU on 121 tokens 32.1 -> 27.0.
-// 3: no epilogue, the sums of a part of k as they are (see w4a16_join_kernel); 8: as 1 for whole tiles, as 3 for the parts of the last ones.
+// 3: no epilogue, the sums of a part of k as they are (see w4a16_join_kernel); 8: as 1 for whole tiles, as 3 for the parts of the last ones; 9: the same with everything
+// for the whole ones (a row's sums are cut the same way whatever is asked for beside them).
 // 4 .. 7: a 16-bit D, at run time an amax, and one of: RMSNorm scale and SwiGLU (28672 x 4096 on 2048 tokens 400 -> 330 us, INT8 activations 679 -> 628); second
 // output and sums of squares (4096 x 14336 214 -> 186); RMSNorm scale (6144 x 4096 103 -> 82; 4096 x 4096 on 100 tokens 30.3 -> 25.3); beta * C (131
 // -> 126, 32.9 -> 30.5: its two-byte loads of C remain).
-enum { kEpiAny = 0, kEpiPlain = 1, kEpiSwiglu = 2, kEpiPart = 3, kEpiNormGlu = 4, kEpiOut2 = 5, kEpiNorm = 6, kEpiAdd = 7, kEpiTail = 8 };
+enum { kEpiAny = 0, kEpiPlain = 1, kEpiSwiglu = 2, kEpiPart = 3, kEpiNormGlu = 4, kEpiOut2 = 5, kEpiNorm = 6, kEpiAdd = 7, kEpiTail = 8, kEpiTailAny = 9 };
 template <int PLANES, bool F16, bool GROUPED, int EPI>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_b, const __grid_constant__ CUtensorMap tmap_d,
@@ -226,8 +227,8 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
   const int nA = 1 << lgA, nB = 1 << lgB, subA = kA >> lgA;
   constexpr int kSub = PLANES == 3 ? C::kBBytes / 2 : C::kBBytes;   // bytes of a stage of one plane (three planes: tiles of at most 128 tokens)
   const int slot_bytes = (kB * C::kBBytes) >> lgB;
-  constexpr bool PART = EPI == kEpiPart, TAIL = EPI == kEpiTail, CUT_K = PART || TAIL;
-  constexpr bool AMAX = EPI == kEpiAny || (EPI >= kEpiNormGlu && !TAIL), ADD = EPI == kEpiAny || EPI == kEpiAdd;
+  constexpr bool PART = EPI == kEpiPart, TAIL = EPI == kEpiTail || EPI == kEpiTailAny, CUT_K = PART || TAIL, ANY = EPI == kEpiAny || EPI == kEpiTailAny;
+  constexpr bool AMAX = ANY || (EPI >= kEpiNormGlu && !TAIL), ADD = ANY || EPI == kEpiAdd;
   const int tile_first = blockIdx.x >> 1, tile_step = gridDim.x >> 1;
   const int tiles_m = (gm + 255) / 256, nk_all = gk / 64, nslots_all = (nk_all + 3) / 4;   // 256-row tiles
   const bool ue = g.A.ue != 0;
@@ -682,7 +683,7 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
                 amax = fmaxf(amax, fabsf(__uint_as_float(r[16 * (q >> 1) + 4 * (ce >> 1) + 2 * (q & 1) + (ce & 1)])));
         }
         const int orow = glu ? tm * 64 : tm * 128, orows = glu ? gm >> 1 : gm;   // the tile's first output row, rows of D
-        if (!SEG && EPI == kEpiAny && d_dtype == NVFP4A_FP32) {   // eight lanes write 32 contiguous bytes of a column
+        if (!SEG && ANY && d_dtype == NVFP4A_FP32) {   // eight lanes write 32 contiguous bytes of a column
           float *const d32 = (float *)dptr + (size_t)j0 * g.e.ldd + orow + (lane >> 2);
 #pragma unroll
           for (int q = 0; q < 4; ++q) {
@@ -929,7 +930,7 @@ int choose_parts(const GemmArgs &g, int planes, const Plan &p, int pairs) {
 // BF16 18997 x 7168 on 250 81.5 -> 61.6, FP16 4864 x 6208 on 600 85 - 95 -> 70 - 78, 4096 x 4096 on 700 51.0 -> 45.6, 3584 x 3584 on 1500 64.6 -> 61.3; forced, INT8 6144 x 4096
 // on 1000 80.8 -> 92.8 and BF16 49.0 -> 53.2, which the rule leaves whole.
 int choose_tail(const GemmArgs &g, int planes, int rows256, int pairs, int widest, Plan *p) {
-  if (!parts_allowed(g) || p->tiles <= pairs || g.e.beta != 0.f || g.e.d_dtype == NVFP4A_FP32 || g.e.amax) return 1;   // (whole tiles beside parts: the plain epilogue)
+  if (!parts_allowed(g) || p->tiles <= pairs) return 1;
   const int stages = (g.k + 63) / 64;
   const long long last = p->cut > 1 || p->tiles % pairs ? stage_cost(p->width / p->cut, planes) : 0;
   const long long whole = (p->nfull / pairs * stage_cost(p->width, planes) + last) * stages;
@@ -998,11 +999,11 @@ cudaError_t launch_epi(const CUtensorMap &tw, const CUtensorMap &tb, const CUten
 
 template <int PLANES, bool F16, bool GROUPED = false>
 cudaError_t launch_cfg(const CUtensorMap &tw, const CUtensorMap &tb, const CUtensorMap &td, const PeerMaps &pm, const W4A16Args &a, cudaStream_t s) {
+  const bool scaled = a.e.beta == 0.f && a.e.d_dtype != NVFP4A_FP32, plain = scaled && !a.e.amax;
   if constexpr (!GROUPED) {
-    if (a.parts > 1 && a.nfull) return launch_epi<PLANES, F16, GROUPED, kEpiTail>(tw, tb, td, pm, a, s);
+    if (a.parts > 1 && a.nfull) return plain ? launch_epi<PLANES, F16, GROUPED, kEpiTail>(tw, tb, td, pm, a, s) : launch_epi<PLANES, F16, GROUPED, kEpiTailAny>(tw, tb, td, pm, a, s);
     if (a.parts > 1) return launch_epi<PLANES, F16, GROUPED, kEpiPart>(tw, tb, td, pm, a, s);
   }
-  const bool scaled = a.e.beta == 0.f && a.e.d_dtype != NVFP4A_FP32, plain = scaled && !a.e.amax;
   if constexpr (!F16 && !GROUPED && PLANES < 3) {
     if (scaled && a.x.mask == (kExNorm | kExSwiglu)) return launch_epi<PLANES, F16, GROUPED, kEpiNormGlu>(tw, tb, td, pm, a, s);
     if (scaled && a.x.mask == kExNorm) return launch_epi<PLANES, F16, GROUPED, kEpiNorm>(tw, tb, td, pm, a, s);

@@ -3,7 +3,9 @@ import ctypes
 
 import numpy as np
 import pytest
+import torch
 
+import nvfp4effma_b200.api as nf
 from nvfp4effma_b200 import _lib as L
 from test_gemm_gpu import Case, DevFp4, build_case, check_bound, dev, device_b, host, kernel_status, oracle_case, stream, tensor
 
@@ -39,4 +41,30 @@ def test_last_round_in_parts_of_k(bt, m, n, k, fa, out, bias, pitch):
     assert L.lib.nvfp4a_b200_last_route() == (8 if bt == L.INT8 else 5) and L.lib.nvfp4a_b200_last_parts() > 1
     check_bound(c, h, got, float(exp["amax"]), exp)
     assert np.array_equal(got.view(np.uint8), run_plain(c, h).view(np.uint8))
+    assert kernel_status() == 0
+
+
+TAILS = [(torch.bfloat16, "int8", 2504, 1793, 4288), (torch.bfloat16, "exact", 19000, 250, 7168), (torch.float16, "exact", 4864, 600, 6208)]
+
+
+def operands(dtype, m, n, k):
+    gen = torch.Generator(device="cuda").manual_seed(54)
+    w = nf.quantize((torch.randn(m, k, generator=gen, device="cuda") * 0.02).to(torch.bfloat16), swizzled=True)
+    return torch.randn(n, k, generator=gen, device="cuda").to(dtype), w
+
+
+@pytest.mark.parametrize("dtype,act,m,n,k", TAILS)
+def test_what_is_asked_for_beside_the_product_changes_no_bits(dtype, act, m, n, k):
+    """The amax, beta * out and (where this kernel writes it) an FP32 result: the same sums as the plain call, in parts of k for the same outputs."""
+    x, w = operands(dtype, m, n, k)
+    y = nf.linear(x, w, act=act)
+    assert L.lib.nvfp4a_b200_last_parts() > 1
+    amax = torch.zeros(1, device="cuda")
+    assert torch.equal(nf.linear(x, w, act=act, amax_out=amax), y)
+    out = torch.zeros_like(y)
+    assert torch.equal(nf.linear(x, w, act=act, out=out, beta=1.0), y)
+    assert L.lib.nvfp4a_b200_last_parts() > 1
+    if dtype == torch.bfloat16:
+        wide = nf.linear(x, w, act=act, out_dtype=torch.float32)
+        assert torch.equal(wide.to(dtype), y) and float(amax) == float(wide.abs().max())
     assert kernel_status() == 0
