@@ -52,11 +52,6 @@ struct StreamArgs {
   int round;                       // slices whose sums fit shared memory
 };
 
-__device__ __forceinline__ uint32_t mul2(uint32_t a, uint32_t b) {
-  uint32_t d;
-  asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
-  return d;
-}
 __device__ __forceinline__ float pow2i(int e) { return __int_as_float((e + 127) << 23); }   // -126 <= e <= 127
 // v * 2^e for any e that a vector's scale can be, by two exact factors
 __device__ __forceinline__ float scale2(float v, int e) {
@@ -238,8 +233,8 @@ __global__ void __launch_bounds__(kThreads, 1) gemv_stream_kernel(const StreamAr
           e2m1_to_f16(word(w.wb, i), pb);
           const int v = (u & 1) * 16 + q * 4 + i;
           const uint4 xv = gq < N && v < vec_left ? plane_values(ld16(row + v), eb, p) : make_uint4(0, 0, 0, 0);
-          mma16(d, mul2(pa[0], s0), mul2(pb[0], s1), mul2(pa[1], s0), mul2(pb[1], s1), xv.x, xv.y);
-          mma16(d, mul2(pa[2], s0), mul2(pb[2], s1), mul2(pa[3], s0), mul2(pb[3], s1), xv.z, xv.w);
+          mma16(d, h2mul(pa[0], s0), h2mul(pb[0], s1), h2mul(pa[1], s0), h2mul(pb[1], s1), xv.x, xv.y);
+          mma16(d, h2mul(pa[2], s0), h2mul(pb[2], s1), h2mul(pa[3], s0), h2mul(pb[3], s1), xv.z, xv.w);
         }
         if (q == 0)       // columns 0 and 1 are the vectors here; lane 0 of a quad has them, and its sums join the others'
 #pragma unroll

@@ -29,6 +29,12 @@ __device__ __forceinline__ uint32_t ld2(const uint8_t *p) {
   asm("ld.global.u16 %0, [%1];" : "=h"(v) : "l"(p));
   return v;
 }
+// products of FP16 pairs
+__device__ __forceinline__ uint32_t h2mul(uint32_t a, uint32_t b) {
+  uint32_t d;
+  asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+  return d;
+}
 __device__ __forceinline__ uint32_t word(const uint4 &v, int i) { return i == 0 ? v.x : i == 1 ? v.y : i == 2 ? v.z : v.w; }
 // slices of 16 rows in the order a matrix is dealt out: the four slices of a 128-row tile whose scale codes share 16-byte lines follow one another
 __device__ __forceinline__ int slice_row(int s, int m) {

@@ -98,3 +98,25 @@ def test_what_the_fused_entry_leaves_to_two_calls():
     assert call(2) == L.NOT_SUPPORTED
     L.lib.nvfp4a_b200_set_route(old)
     assert not bool(y.any()) and call(4) == L.OK and bool(y[:4].all()) and not bool(y[4:].any())
+
+
+@pytest.mark.parametrize("flags,one", [(0, 0x38), (UE, 0x78)])
+@pytest.mark.parametrize("n", [1, 4, 7])
+def test_sums_of_the_smallest_activations_keep_their_bits(n, flags, one):
+    """INT8 activations whose scales are 2^-140: every product with a weight and its block scale is a whole number of 2^-144, so that FP32, whose smallest number is
+    2^-149, holds every sum exactly, and the weight's decode factor of 2^100 brings the result back.  No tolerance."""
+    m, k = 40, 192
+    rng = np.random.default_rng(63)
+    codes, scodes = rng.integers(0, 16, (m, k)).astype(np.uint8), rng.integers(one, one + 16, (m, k // 16)).astype(np.uint8)     # (scales of 1 to 3.75)
+    q = rng.integers(-127, 128, (n, k)).astype(np.int8)
+    e2m1 = np.array([0.0, 0.5, 1.0, 1.5, 2.0, 3.0, 4.0, 6.0])
+    w = np.where(codes & 8, -1.0, 1.0) * e2m1[codes & 7] * np.repeat((1.0 + (scodes & 7) / 8.0) * 2.0 ** ((scodes >> 3) - float(one >> 3)), 16, axis=1)
+    want = q.astype(np.float64) @ w.T * 2.0 ** -40
+    data, scales, glob = dev((codes[:, 0::2] | codes[:, 1::2] << 4).reshape(-1)), dev(scodes.reshape(-1)), dev(np.array([2.0 ** 100], np.float32))
+    values8, scales8, ones = dev(q.reshape(-1)), dev(np.full(n * k // 16, 2.0 ** -140, np.float32)), dev(np.ones(1, np.float32))
+    ta, tb = tensor(data, L.NVFP4, scales, k // 16, glob, flags=flags), tensor(values8, L.INT8, scales8, k // 16, ones)
+    y = torch.zeros(n, m, device="cuda")
+    td = tensor(y, L.FP32)
+    L.check(L.lib.nvfp4a_gemm(m, n, k, 1.0, ctypes.byref(ta), k, ctypes.byref(tb), k, 0.0, None, 0, ctypes.byref(td), m, None, stream()))
+    assert L.lib.nvfp4a_b200_last_route() == 6
+    assert np.array_equal(host(y).astype(np.float64).reshape(n, m), want)
