@@ -114,7 +114,9 @@ int nvfp4a_b200_set_gemv_splits(int splits);
 
 /* nvfp4a_gemm (image != 0: nvfp4a_gemv_tc, A->data is the weight's image and lda is not looked at) on up to 8 dense activation vectors that the kernel itself makes
  * INT8 with one FP32 scale per 16 values: the bytes of nvfp4a_quantize to INT8 followed by that call, in one launch and without buffers between the two (no counterpart
- * in the reference).  More vectors, and what the INT8 GEMV does not take (nvfp4a_b200_set_route(1) among it): NVFP4A_NOT_SUPPORTED, and nothing is launched. */
+ * in the reference).  More vectors, more than NVFP4A_B200_GEMV_W4A8_VALUES activations in all (n * k: every CTA quantizes them for itself, which then takes longer than a
+ * launch that does it once), and what the INT8 GEMV does not take (nvfp4a_b200_set_route(1) among it): NVFP4A_NOT_SUPPORTED, and nothing is launched. */
+#define NVFP4A_B200_GEMV_W4A8_VALUES 32768
 nvfp4a_status nvfp4a_b200_gemv_w4a8(int m, int n, int k, float alpha, const nvfp4a_tensor *A, int lda, int image, const nvfp4a_tensor *B, int ldb, float beta,
                                     const nvfp4a_tensor *C, int ldc, const nvfp4a_tensor *D, int ldd, const nvfp4a_tensor *bias, cudaStream_t stream);
 

@@ -13,6 +13,7 @@
 #include <stdlib.h>
 #include <atomic>
 #include "operands.cuh"
+#include "../../include/nvfp4effma_b200.h"
 
 namespace nvb {
 
@@ -413,7 +414,7 @@ extern "C" nvfp4a_status nvfp4a_b200_gemv_w4a8(int m, int n, int k, float alpha,
     g.A.image = 1; g.A.ktiles = (k + kImgK - 1) / kImgK; g.A.sc = nullptr;
   }
   // Every CTA quantizes all activations: up to 32768 values that takes 0.6 to 1.6 us (k = 4096, one to eight vectors) where a launch of its own takes 1.9; 8 x 8000 take 9.
-  if (forced_route() == 1 || (long long)n * k > 32768 || !gemv_q8_supports(g)) return fail(NVFP4A_NOT_SUPPORTED, "%s: quantize first (k = %d)", fn, k);
+  if (forced_route() == 1 || (long long)n * k > NVFP4A_B200_GEMV_W4A8_VALUES || !gemv_q8_supports(g)) return fail(NVFP4A_NOT_SUPPORTED, "%s: quantize first (k = %d)", fn, k);
   g_last_route = 6;
   return cuda_fail(launch_gemv_q8(g, stream), fn);
 }

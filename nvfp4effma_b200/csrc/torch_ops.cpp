@@ -409,7 +409,7 @@ std::tuple<Tensor, OptTensor> linear_w4a8(const Tensor &x0, const Tensor &w, con
   check_matrix16(x0, "linear_w4a8");
   check_k(k);
   const int64_t T = x0.size(0), N = w.size(0);
-  if (T >= 1 && T <= 8 && x0.size(1) == k && x0.device() == w.device()) {
+  if (T >= 1 && T <= 8 && T * k <= NVFP4A_B200_GEMV_W4A8_VALUES && x0.size(1) == k && x0.device() == w.device()) {
     const c10::cuda::CUDAGuard guard(w.device());
     const Tensor x = matrix(x0, 16, "x");
     if (x.stride(0) % 64 == 0) {

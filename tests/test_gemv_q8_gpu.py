@@ -120,3 +120,14 @@ def test_sums_of_the_smallest_activations_keep_their_bits(n, flags, one):
     L.check(L.lib.nvfp4a_gemm(m, n, k, 1.0, ctypes.byref(ta), k, ctypes.byref(tb), k, 0.0, None, 0, ctypes.byref(td), m, None, stream()))
     assert L.lib.nvfp4a_b200_last_route() == 6
     assert np.array_equal(host(y).astype(np.float64).reshape(n, m), want)
+
+
+def test_activations_that_the_fused_entry_leaves_to_two_calls_cost_no_try():
+    """Five vectors of 8192 values: the INT8 values, their scales, the result and the amax are all that a call allocates."""
+    gen = torch.Generator(device="cuda").manual_seed(64)
+    w, x, amax = nf.quantize(torch.randn(64, 8192, generator=gen, device="cuda")), torch.randn(5, 8192, generator=gen, device="cuda").to(torch.bfloat16), torch.zeros(1, device="cuda")
+    y = nf.linear(x, w, act="int8", amax_out=amax)
+    before = torch.cuda.memory_stats()["allocation.all.allocated"]
+    again = nf.linear(x, w, act="int8", amax_out=amax)
+    assert torch.cuda.memory_stats()["allocation.all.allocated"] - before == 4
+    assert torch.equal(y, again) and torch.equal(y, nf.linear(nf.quantize_int8(x), w, out_dtype=torch.bfloat16)) and float(amax.to(torch.bfloat16)) == float(y.abs().max())
