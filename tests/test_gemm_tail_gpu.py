@@ -7,7 +7,7 @@ import torch
 
 import nvfp4effma_b200.api as nf
 from nvfp4effma_b200 import _lib as L
-from test_gemm_gpu import Case, DevFp4, build_case, check_bound, dev, device_b, host, kernel_status, oracle_case, stream, tensor
+from test_gemm_gpu import Case, DevFp4, build_case, check_bound, dev, device_b, host, kernel_status, oracle_case, run_tc, stream, tensor
 
 pytestmark = pytest.mark.gpu
 SW = L.SCALES_SWIZZLED
@@ -23,7 +23,8 @@ def run_plain(c, h):
     return host(dD).view(h["Dinit"].dtype)
 
 
-# (74 SM pairs; tiles of 256 rows and at most 256 tokens, 128 with FP16; an output pitch that TMA stores take and one that they do not)
+# (74 SM pairs; tiles of 256 rows and at most 256 tokens, 128 with FP16.  FP16: an output pitch that TMA stores take and one that they do not; the other rows are no whole 16
+# bytes and take plain stores)
 @pytest.mark.parametrize("bt,m,n,k", [
     (L.INT8, 2500, 1793, 4096 + 192),  # a last token alone in its tile, rows past the matrix, an odd number of stages
     (L.BF16, 18997, 250, 7168),       # one tile more than a round
@@ -67,4 +68,26 @@ def test_what_is_asked_for_beside_the_product_changes_no_bits(dtype, act, m, n, 
     if dtype == torch.bfloat16:
         wide = nf.linear(x, w, act=act, out_dtype=torch.float32)
         assert torch.equal(wide.to(dtype), y) and float(amax) == float(wide.abs().max())
+    assert kernel_status() == 0
+
+
+@pytest.mark.parametrize("bt,m,n,k,form", [
+    (L.INT8, 2504, 1793, 4096 + 192, "plain"),
+    (L.INT8, 2504, 1793, 4096 + 192, "image"),
+    (L.INT8, 2504, 1793, 4096 + 192, "wide tokens"),   # every third token is three BF16 planes, the others two FP16 planes
+    (L.INT8, 2504, 1793, 4096 + 192, "ue5m3"),         # three planes for all of them
+    (L.BF16, 19000, 250, 7168, "plain"),
+])
+def test_last_round_in_parts_of_k_beside_tiles_that_tma_stores(bt, m, n, k, form):
+    """A pitch and rows of whole 16 bytes: TMA stores the whole tiles, whose last tokens do not fill a tile; image tiles and scales at a part's first stage."""
+    c = Case(m, n, k, bt, L.BF16, -1, L.BF16, 1.25, 0.0, fa=L.SCALES_UE5M3 if form == "ue5m3" else SW)
+    h = build_case(c, 5450)
+    h["ldd"] = m
+    h["Dinit"] = np.resize(h["Dinit"], n * m)
+    if form == "wide tokens":
+        h["B"].scales.reshape(n, -1)[1::3, 3::7] *= np.float32(2.0 ** -14)
+    exp = oracle_case(c, h, want_ref=True)
+    got, amax = run_tc(c, h, gemv=False) if form == "image" else (run_plain(c, h), float(exp["amax"]))
+    assert L.lib.nvfp4a_b200_last_route() == (8 if bt == L.INT8 else 5) and L.lib.nvfp4a_b200_last_parts() > 1
+    check_bound(c, h, got, amax, exp)
     assert kernel_status() == 0
