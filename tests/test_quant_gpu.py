@@ -425,3 +425,60 @@ def test_small_matrices_quantize_in_one_launch_on_several_streams():
         w = want[i]
         assert torch.equal(q.data.view(torch.uint8), w.data.view(torch.uint8)) and torch.equal(q.scales.view(torch.uint8), w.scales.view(torch.uint8))
         assert torch.equal(q.amax, w.amax)
+
+
+@pytest.mark.parametrize("dtype,flags,rows,cols,pad,offset", [
+    (torch.float16, AM | SW, 4100, 8256, 0, 0),      # 33.8 M values: units in shared memory, in tensor memory and read again; the last unit of a row is ragged
+    (torch.bfloat16, AM | UE, 8190, 4160, 16, 0),
+    (torch.float16, AM | UE, 6001, 8192, 16, 8),     # rows on 16-byte boundaries only: two loads for a block
+    (torch.bfloat16, AM | SW, 4100, 4160, 0, 0),     # tensor memory, nothing read again
+])
+def test_quantizer_that_keeps_units_in_tensor_memory_equals_the_two_launch_path(dtype, flags, rows, cols, pad, offset):
+    gen = torch.Generator(device="cuda").manual_seed(rows)
+    lds = cols + pad
+    base = torch.randn(rows * lds + offset, generator=gen, device="cuda").mul_(3.0)
+    base[torch.randint(0, rows * lds, (1000,), generator=gen, device="cuda")] *= 100.0
+    x = base.to(dtype)[offset:]
+    code = L.FP16 if dtype == torch.float16 else L.BF16
+    sbytes = O.scale_bytes(bool(flags & SW), 0 if flags & SW else cols // 16, rows, cols)
+    outs = []
+    try:
+        for fused in (1, 0, 1):
+            assert L.lib.nvfp4a_b200_set_quant_fused(fused) == 0
+            d, s = torch.full((rows * cols // 2,), 0xEE, dtype=torch.uint8, device="cuda"), torch.full((sbytes,), 0xEE, dtype=torch.uint8, device="cuda")
+            glob, amax = torch.zeros(1, device="cuda"), torch.zeros(1, device="cuda")
+            S, R = tensor(x, code), tensor(d, L.NVFP4, s, 0 if flags & SW else cols // 16, glob, amax, flags, 0)
+            cfg = L.QuantConfig(1, 0, 1)
+            L.check(L.lib.nvfp4a_quantize_ex(ctypes.byref(S), lds, rows, cols, ctypes.byref(R), cols, None, 0, ctypes.byref(cfg), stream()))
+            outs.append((d, s, glob, amax))
+    finally:
+        L.lib.nvfp4a_b200_set_quant_fused(1)
+    assert float(outs[0][2]) == float(x[: rows * lds].view(rows, lds)[:, :cols].abs().max())
+    for other in outs[1:]:
+        assert all(torch.equal(a, b) for a, b in zip(outs[0], other))
+
+
+def test_both_quantizers_of_one_launch_take_turns_on_several_streams():
+    """The sixteen-warp kernel and the one with tensor memory share the barrier's counter and the arrays of maxima: matrices of both, with and without tensor memory and a
+    second read, on four streams at once."""
+    import nvfp4effma_b200.api as nf
+    gen = torch.Generator(device="cuda").manual_seed(10)
+    xs = [(torch.randn(r, c, generator=gen, device="cuda") * 2.0 ** i).to(dt) for i, (r, c, dt) in
+          enumerate([(64, 1024, torch.bfloat16), (3000, 4096, torch.bfloat16), (300, 4096, torch.float16), (4100, 4096, torch.float16), (8200, 4160, torch.bfloat16)])]
+    L.lib.nvfp4a_b200_set_quant_fused(0)
+    try:
+        want = [nf.quantize(x, swizzled=True) for x in xs]
+    finally:
+        L.lib.nvfp4a_b200_set_quant_fused(1)
+    streams = [torch.cuda.Stream() for _ in range(4)]
+    torch.cuda.synchronize()
+    got = []
+    for rep in range(16):
+        for i in range(len(xs)):
+            with torch.cuda.stream(streams[(rep + i) % 4]):
+                got.append((i, nf.quantize(xs[i], swizzled=True)))
+    torch.cuda.synchronize()
+    for i, q in got:
+        w = want[i]
+        assert torch.equal(q.data.view(torch.uint8), w.data.view(torch.uint8)) and torch.equal(q.scales.view(torch.uint8), w.scales.view(torch.uint8))
+        assert torch.equal(q.amax, w.amax)
