@@ -94,6 +94,48 @@ def test_a_barrier_whose_peer_never_arrives_gives_up_and_reports_it():
     assert st.value == 0 and bool(torch.isfinite(y.float()).all())
 
 
+@pytest.mark.parametrize("rank", [0, 1])
+@pytest.mark.parametrize("T", [1, 2, 5])
+def test_decode_gemvs_push_their_outputs_to_a_peer_that_is_ahead(T, rank):
+    """The fused forms of the GEMVs (one and two vectors: csrc/gemv_stream.cu, more: csrc/gemv.cu) on ONE GPU, with nobody to wait for: the "peer" is a second
+    buffer and a flag array in which it has posted every epoch that the calls can ask for.  Both buffers get the shard of the plain call and nothing else, and every call
+    that posts raises the rank's epoch at the peer."""
+    import ctypes
+    import nvfp4effma_b200 as nf
+    from nvfp4effma_b200 import _lib as L
+    m, k = 1040, 1088
+    image = nf.TCWeight(nf.quantize(rand((m, k), torch.bfloat16, seed=21)), "exact")
+    op = image.weight._operand()
+    x = rand((T, k), torch.bfloat16, seed=22)
+    ta, tx = L.Tensor(image.image.data_ptr(), L.NVFP4, None, 0, op.glob.data_ptr(), None, op.flags, op.scale_max), L.Tensor(x.data_ptr(), L.BF16)
+    stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    bufs = [torch.full((T, 2 * m), 3.0, dtype=torch.bfloat16, device="cuda") for _ in range(2)]
+    flags = [torch.zeros(16, dtype=torch.int64, device="cuda") for _ in range(2)]
+    flags[rank][1 - rank] = 1 << 40
+    pb, pf = (ctypes.c_void_p * 2)(*[b.data_ptr() for b in bufs]), (ctypes.c_void_p * 2)(*[f.data_ptr() for f in flags])
+    want = torch.empty(T, m, dtype=torch.bfloat16, device="cuda")
+    tw = L.Tensor(want.data_ptr(), L.BF16)
+    old = L.lib.nvfp4a_b200_set_route(2)
+    try:
+        L.check(L.lib.nvfp4a_gemv_tc(m, T, k, 1.0, ctypes.byref(ta), ctypes.byref(tx), k, 0.0, None, 0, ctypes.byref(tw), m, None, stream))
+        for call, (entry, push) in enumerate([("gemv_tc_tp", ()), ("gemv_tc_tp_deferred", (1,)), ("gemv_tc_tp_deferred", (1,)), ("gemv_tc_tp", ())]):
+            for b in bufs:
+                b.fill_(3.0)
+            td = L.Tensor(bufs[rank].data_ptr() + 2 * rank * m, L.BF16)
+            L.check(getattr(L.lib, "nvfp4a_b200_" + entry)(m, T, k, 1.0, ctypes.byref(ta), ctypes.byref(tx), k, ctypes.byref(td), 2 * m, None, None, pb, pf, 2, rank, *push,
+                                                           stream))
+            assert L.lib.nvfp4a_b200_last_route() == 2
+            for b in bufs:
+                halves = b.view(T, 2, m)
+                assert torch.equal(halves[:, rank], want) and bool((halves[:, 1 - rank] == 3.0).all()), (call, entry)
+            assert int(flags[1 - rank][rank]) == call + 1 and int(flags[rank][9]) == 0
+    finally:
+        L.lib.nvfp4a_b200_set_route(old)
+    st = ctypes.c_uint(0)
+    L.check(L.lib.nvfp4a_b200_kernel_status(ctypes.byref(st), 1))
+    assert st.value == 0
+
+
 @pytest.mark.parametrize("T", [1, 4, 8])
 def test_shard_rows_are_the_rows_of_the_whole_on_the_same_kernel(T):
     """A shard's decode outputs equal the whole matrix's bit for bit where both run one kernel: on the mma.sync GEMV (nvfp4a_b200_set_route(2)),
