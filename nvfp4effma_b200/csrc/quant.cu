@@ -338,7 +338,7 @@ __global__ void __launch_bounds__(256, 3) quant_rows_kernel(const uint8_t *__res
 // therefore alternate between two arrays of maxima: nobody writes what a late CTA of the launch before is still to read.)
 // The barrier's wait is bounded like every wait of this library; on expiry the status word gets 0x601 and the kernel goes on
 // (with whatever maxima have arrived) so that it always terminates.
-constexpr int kQfSmemBytes = 96 * 2048;            // 96 units of 2 KiB stay in shared memory per CTA
+constexpr int kQfSmemBytes = 96 * 2048;            // 96 units of 2 KiB stay in shared memory per CTA; of sixteen warps none, but a CTA has to take a whole SM (see below)
 constexpr int kQfMaxGrid = 1024;
 static __device__ unsigned long long g_qf_arrivals;   // arrivals of every launch so far on this device (each launch adds its grid size, which never changes)
 static __device__ float g_qf_max[2][kQfMaxGrid];   // per-CTA maxima of the current launch and of the one before it
@@ -363,8 +363,8 @@ __device__ __forceinline__ void scale16(float v[16], float f) {
 }
 // quant_block16 with the factor 1 / (scale * S_dec), which depends on the scale code only, from a 256-entry table that the CTA fills once
 template <bool UE>
-__device__ __forceinline__ uint2 quant_block16_by_table(float v[16], float enc6, const float *inv_of_code, uint32_t &code, float &bmax) {
-  bmax = absmax16(v);
+__device__ __forceinline__ uint2 quant_block16_by_table(float v[16], float enc6, const float *inv_of_code, uint32_t &code) {
+  const float bmax = absmax16(v);
   code = UE ? f32_to_ue5m3_sw(fminf(__fmul_rn(bmax, enc6), kFltMax)) : e4m3_encode(fminf(__fmul_rn(bmax, enc6), kFltMax));
   scale16(v, inv_of_code[code]);
   return make_uint2(e2m1_pack8(v), e2m1_pack8(v + 8));
@@ -374,12 +374,12 @@ __device__ __forceinline__ uint2 quant_block16_by_table(float v[16], float enc6,
 template <int T, bool UE>
 __device__ __forceinline__ void emit_two_blocks(const PackedBlock<T> a0, const PackedBlock<T> a1, int r, int c0, int c1, bool live0, bool live1,
                                              float enc6, const float *inv_of_code, uint8_t *data, int ldq, uint8_t *sc, const ScalePos sp, bool words, int lane) {
-  float v[16], bmax;
+  float v[16];
   uint32_t code0, code1;
   unpack_block<T>(a0, v);
-  const uint2 q0 = quant_block16_by_table<UE>(v, enc6, inv_of_code, code0, bmax);
+  const uint2 q0 = quant_block16_by_table<UE>(v, enc6, inv_of_code, code0);
   unpack_block<T>(a1, v);
-  const uint2 q1 = quant_block16_by_table<UE>(v, enc6, inv_of_code, code1, bmax);
+  const uint2 q1 = quant_block16_by_table<UE>(v, enc6, inv_of_code, code1);
   uint8_t *drow = data + (size_t)r * ldq;
   if (live0) __stcs((uint2 *)(drow + 8 * c0), q0);
   if (live1) __stcs((uint2 *)(drow + 8 * c1), q1);
@@ -403,8 +403,8 @@ __global__ void __launch_bounds__(WARPS * 32, 1)
 quant_fused_kernel(const uint8_t *__restrict__ src, int lds, int rows, int bpr, unsigned div_mul, int div_shift, QOut o, float *gout, float *stat, unsigned *status, unsigned tag) {
   static_assert(T != NVFP4A_FP32, "16-bit sources");
   extern __shared__ uint4 qf_keep[];   // [warp][unit][4 words][32 lanes]
-  constexpr bool kTmem = WARPS == 24;               // 24 warps: tensor memory; 16: registers
-  constexpr int kQfWarps = WARPS, kQfRegUnits = kTmem ? 0 : 4, kQfSmemUnits = 96 / WARPS, kFlight = kTmem ? 2 : 4;
+  constexpr bool kTmem = WARPS == 24;               // 24 warps: shared and tensor memory, the rest read again; 16: registers, which hold all of it (the host sees to that)
+  constexpr int kQfWarps = WARPS, kQfSmemUnits = 96 / WARPS, kFlight = 2;
   constexpr int kQfTmemUnits = kTmem ? 32 / (WARPS / 4) : 0;    // 512 columns of tensor memory, 16 to a unit; a warp reaches a quarter of the lanes, WARPS / 4 warps share a quarter
   __shared__ float warp_max[kQfWarps];
   __shared__ float gmax_s;
@@ -414,10 +414,9 @@ quant_fused_kernel(const uint8_t *__restrict__ src, int lds, int rows, int bpr, 
   const long long U = (long long)rows * upr;   // (below 2^31: the host checks)
   const unsigned u_begin = (unsigned)(U * blockIdx.x / gridDim.x), u_end = (unsigned)(U * (blockIdx.x + 1) / gridDim.x);
   const int n_cta = (int)(u_end - u_begin);
-  const int n_w = n_cta > warp ? (n_cta - warp + kQfWarps - 1) / kQfWarps : 0;   // this warp's units: u_begin + warp + 16 j
-  // of a warp's units the last n_rg stay in registers, the n_sm before them in shared memory, the n_tm before those in tensor memory; the first n_glob are read again
-  const int n_ret = min(n_w, kQfRegUnits + kQfSmemUnits + kQfTmemUnits);
-  const int n_rg = min(n_ret, kQfRegUnits), n_sm = min(n_ret - n_rg, kQfSmemUnits), n_tm = n_ret - n_rg - n_sm, n_glob = n_w - n_ret;
+  const int n_w = n_cta > warp ? (n_cta - warp + kQfWarps - 1) / kQfWarps : 0;   // this warp's units: u_begin + warp + kQfWarps j
+  // of a warp's units the last n_rg (all, at most four) stay in registers or the last n_sm in shared memory, the n_tm before those in tensor memory; the first n_glob are read again
+  const int n_rg = kTmem ? 0 : n_w, n_sm = kTmem ? min(n_w, kQfSmemUnits) : 0, n_tm = kTmem ? min(n_w - n_sm, kQfTmemUnits) : 0, n_ret = n_rg + n_sm + n_tm, n_glob = kTmem ? n_w - n_ret : 0;
   const bool use_tmem = kTmem && n_cta > kQfWarps * kQfSmemUnits;   // (of the CTA)
   __shared__ uint32_t tmem_slot;
   if (use_tmem) {
@@ -491,7 +490,7 @@ quant_fused_kernel(const uint8_t *__restrict__ src, int lds, int rows, int bpr, 
   PackedBlock<T> rk0_0, rk1_0, rk0_1, rk1_1, rk0_2, rk1_2, rk0_3, rk1_3;
   rk0_0.w[0] = rk0_0.w[1] = make_uint4(0, 0, 0, 0);
   rk1_0 = rk0_1 = rk1_1 = rk0_2 = rk1_2 = rk0_3 = rk1_3 = rk0_0;
-  if (kQfRegUnits) {
+  if (!kTmem) {
     if (n_rg > 0) load_unit(j, drop_pol, rk0_0, rk1_0);
     if (n_rg > 1) load_unit(j + 1, drop_pol, rk0_1, rk1_1);
     if (n_rg > 2) load_unit(j + 2, drop_pol, rk0_2, rk1_2);
@@ -565,14 +564,14 @@ quant_fused_kernel(const uint8_t *__restrict__ src, int lds, int rows, int bpr, 
     if (i < n_ret) {
       PackedBlock<T> x0, x1;
       int j;
-      if (kQfRegUnits && i < n_rg) {   // (i is the same for the whole warp)
+      if (!kTmem) {                // (i is the same for the whole warp)
         x0 = i == 0 ? rk0_0 : i == 1 ? rk0_1 : i == 2 ? rk0_2 : rk0_3;
         x1 = i == 0 ? rk1_0 : i == 1 ? rk1_1 : i == 2 ? rk1_2 : rk1_3;
-        j = n_glob + n_tm + n_sm + i;
-      } else if (!kTmem || i < n_sm) {
-        const uint4 *d = my_smem + (i - n_rg) * 128 + lane;
+        j = i;
+      } else if (i < n_sm) {
+        const uint4 *d = my_smem + i * 128 + lane;
         x0.w[0] = d[0]; x0.w[1] = d[32]; x1.w[0] = d[64]; x1.w[1] = d[96];
-        j = n_glob + n_tm + i - n_rg;
+        j = n_glob + n_tm + i;
       } else {
         uint32_t r[16];
         const int k = i - n_sm;
