@@ -104,7 +104,9 @@ nvfp4a_status nvfp4a_b200_trim_scratch(void);
 void nvfp4a_b200_set_scratch_alloc(void *(*alloc)(void *ctx, size_t bytes), void *ctx);
 void nvfp4a_b200_get_scratch_alloc(void *(**alloc)(void *ctx, size_t bytes), void **ctx);   /* what the calling thread has set */
 
-/* The number of parts that the calling thread's last W4A16 / W4A8 tensor-core GEMM cut k into (1: whole).  Test aid. */
+/* The number of parts that the calling thread's last W4A16 / W4A8 tensor-core GEMM cut k into, in all its tiles or in those of its last round (1: whole).  The plan
+ * depends on sizes and operand types alone.  With only the last round cut, the last tokens of a call are summed in parts and the others whole: the same token, given early and
+ * late in one call, may differ in its last bits.  Test aid. */
 int nvfp4a_b200_last_parts(void);
 
 /* Pins the number of k ranges (CTAs per cluster) of the FP4 tensor-core GEMV: 0 = by problem size, else 1, 2, 4 or 8; a
@@ -114,8 +116,7 @@ int nvfp4a_b200_set_gemv_splits(int splits);
 
 /* nvfp4a_gemm (image != 0: nvfp4a_gemv_tc, A->data is the weight's image and lda is not looked at) on up to 8 dense activation vectors that the kernel itself makes
  * INT8 with one FP32 scale per 16 values: the bytes of nvfp4a_quantize to INT8 followed by that call, in one launch and without buffers between the two (no counterpart
- * in the reference).  More vectors, more than NVFP4A_B200_GEMV_W4A8_VALUES activations in all (n * k: every CTA quantizes them for itself, which then takes longer than a
- * launch that does it once), and what the INT8 GEMV does not take (nvfp4a_b200_set_route(1) among it): NVFP4A_NOT_SUPPORTED, and nothing is launched. */
+ * in the reference).  More vectors, more than NVFP4A_B200_GEMV_W4A8_VALUES activations in all (n * k: every CTA quantizes all of them for itself), and what the INT8 GEMV does not take (nvfp4a_b200_set_route(1) among it): NVFP4A_NOT_SUPPORTED, and nothing is launched. */
 #define NVFP4A_B200_GEMV_W4A8_VALUES 32768
 nvfp4a_status nvfp4a_b200_gemv_w4a8(int m, int n, int k, float alpha, const nvfp4a_tensor *A, int lda, int image, const nvfp4a_tensor *B, int ldb, float beta,
                                     const nvfp4a_tensor *C, int ldc, const nvfp4a_tensor *D, int ldd, const nvfp4a_tensor *bias, cudaStream_t stream);

@@ -413,7 +413,9 @@ extern "C" nvfp4a_status nvfp4a_b200_gemv_w4a8(int m, int n, int k, float alpha,
   if (image) {
     g.A.image = 1; g.A.ktiles = (k + kImgK - 1) / kImgK; g.A.sc = nullptr;
   }
-  // Every CTA quantizes all activations: up to 32768 values that takes 0.6 to 1.6 us (k = 4096, one to eight vectors) where a launch of its own takes 1.9; 8 x 8000 take 9.
+  // Every CTA quantizes all activations, so the gain shrinks with their number (CUDA graph, here and with a launch of its own): 4096 x 4096 with 1 / 4 / 8 vectors 6.9 / 8.5 / 12.0 and
+  // 8.9 / 10.0 / 12.8 us, 14336 x 4096 14.1 / 17.6 / 27.4 and 15.9 / 19.1 / 28.3, 4096 x 8192 with 4 (32768 values) 12.9 and 13.6.  The line is on the safe side: 4096 x 8192 with 6
+  // takes 17.1 and 17.3, 4096 x 14336 with 4 18.1 and 19.1; with eight, 4096 x 8192 takes 19.9 and 19.4, 4096 x 14336 27.4 and 27.1.
   if (forced_route() == 1 || (long long)n * k > NVFP4A_B200_GEMV_W4A8_VALUES || !gemv_q8_supports(g)) return fail(NVFP4A_NOT_SUPPORTED, "%s: quantize first (k = %d)", fn, k);
   g_last_route = 6;
   return cuda_fail(launch_gemv_q8(g, stream), fn);

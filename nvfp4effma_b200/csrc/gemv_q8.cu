@@ -10,7 +10,8 @@
 // holds vector j's values in the k positions of lane l's block and zeros elsewhere; four MMAs give lane l the sums of ITS block for two vectors.
 // The order of a row's additions depends on k alone: its bits depend neither on the matrix around it nor on the other vectors.
 //
-// What bounds it: instruction issue and load latency.  CUDA graph, INT8 vectors given, int8 MMAs on weights decoded by byte permutes (11 instructions per 8 weights, 7
+// What bounds it: instruction issue and the chains between instructions (14336 x 4096, four vectors made INT8 here: 322 instructions per unit with all set-up, 57 % of the issue slots; per
+// instruction warps wait 2.5 cycles for their own arithmetic, 0.8 for shared memory, 0.4 for weights).  CUDA graph, INT8 vectors given, int8 MMAs on weights decoded by byte permutes (11 instructions per 8 weights, 7
 // here) with one unit ahead and then: 14336 x 4096 with 1 / 4 / 8 vectors 15.8 / 19.8 / 27.6 and 13.6 / 16.5 / 25.8 us, 4096 x 4096 7.5 / 8.6 / 11.2 and 6.1 / 7.4 / 10.3,
 // 4096 x 14336 15.2 / 18.7 / 26.8 and 14.0 / 16.6 / 24.5, 1024 x 1024 2.9 / 3.1 / 3.6 and 3.1 / 3.3 / 4.0.  Dense BF16 vectors, quantized by a launch of their own and
 // then here: 14336 x 4096 18.0 / 21.7 / 29.1 and 14.2 / 17.5 / 27.4, 1024 x 1024 4.4 / 4.5 / 5.7 and 3.6 / 3.8 / 4.8.

@@ -16,8 +16,8 @@
 // far (gemv_kernel: 1.2e-7 and 5.5e-7).  The order of a row's additions depends on k and n alone: a row's bits do not depend on
 // the matrix (or tensor-parallel shard) around it.
 //
-// What bounds it: launch and one memory round trip for the activations, then instruction issue (175 instructions per unit, half of the slots filled by 16 warps)
-// and load latency.  CUDA graph, one vector, before (gemv_kernel) and now: 1024 x 1024 3.1 and 2.8 us, 512 x 4096 4.65 and 3.75, 4096 x 4096 6.9 and 5.6, 6144 x
+// What bounds it: launch and one memory round trip for the activations, then load latency and instruction issue
+// (4096 x 14336: 187 instructions per unit with all set-up, 45 % of the issue slots; per instruction warps wait 3.2 cycles for memory and 1.6 for their own arithmetic).  CUDA graph, one vector, before (gemv_kernel) and now: 1024 x 1024 3.1 and 2.8 us, 512 x 4096 4.65 and 3.75, 4096 x 4096 6.9 and 5.6, 6144 x
 // 4096 8.6 and 7.1, 4096 x 14336 17.4 and 13.2; two vectors 3.1 and 3.1, 4.7 and 4.4, 6.95 and 6.1, 9.0 and 7.6, 17.4 and 14.5.  Starting under the
 // previous kernel's tail is 1.1 us of each.  Slower: units of 16 x 256 (registers spill), three units ahead (5.7 / 7.1 / 13.0), CTAs of eight warps two
 // of which fit an SM (7.4 / 9.2 / 18.1), bulk copies into a ring of shared memory with a cluster of four per k (6.9 / 8.0 / 16.0).

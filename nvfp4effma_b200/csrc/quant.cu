@@ -330,7 +330,8 @@ __global__ void __launch_bounds__(256, 3) quant_rows_kernel(const uint8_t *__res
 // keeps its last four units in shared memory and the five before them in tensor memory, which is 256 KiB per SM that nothing else uses here (9 x 2 KiB x
 // 24 warps = 432 KiB per SM, 65 MB over the chip: half of an 8192 x 8192 BF16 matrix).  After the barrier every step of a warp encodes one on-chip unit and one
 // unit read again from memory (in descending order), whose load was issued a step earlier.
-// What bounds it: the second visit is instruction issue (about 150 per block of 16 values, many of them conversions at half rate), so warps count: 16 of them
+// What bounds it: latency and issue (about 150 instructions per block of 16 values in the second visit, many of them conversions at half rate; over both visits 45 % of the
+// issue slots are taken, and per instruction warps wait 4.7 cycles for memory, 1.9 at barriers, 1.7 for a slot, 1.6 for their own arithmetic, 1.2 for its pipe), so warps count: 16 of them
 // with four more units each in registers (127 registers a thread) take 53.1 us for 8192 x 8192 BF16 where 24 take 49.1 and 32 take 50.0; without tensor memory 16
 // took 56.8.  8192 x 4096 30.0 -> 25.9, 4096 x 4096 17.6 -> 16.8 (CUDA graph, rotating inputs; quant_rows_kernel, one visit, 28.5 us for 8192 x 8192).
 // Per-CTA maxima meet in a device array (no atomics on floats, no memset launch): every CTA reads all of them after the barrier.
